@@ -765,6 +765,7 @@ int cc_check_async_error(cc_device* dev) {
     *(volatile unsigned*)dev->err_host = 0u;
     if (dev->err_dev) cudaMemset(dev->err_dev, 0, 256);
     if (dev->lz && dev->lz->bar_dev) cudaMemset(dev->lz->bar_dev, 0, 4096);
+    if (code == 5u) return cc_fail(dev, CC_ERR_CUDA, "split product: its pipeline timed out");
     return cc_fail(dev, CC_ERR_CUDA, "%s timeout (%s): the grid was not co-resident or a peer GPU stopped responding",
                    code == 3u ? "exchange kernel" : "megakernel barrier", code == 1u ? "grid barrier" : code == 4u ? "weight ring" : "cross-GPU handshake");
 }

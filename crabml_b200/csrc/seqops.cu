@@ -13,6 +13,7 @@
 #include "act.cuh"
 #include "capi_checks.cuh"
 #include "layer_norm.cuh"
+#include "split_gemm.cuh"
 
 #define SEQ_ENTER(dev, what)                                                                                          \
     if (!(dev)) return CC_ERR_ARG;                                                                                    \
@@ -720,23 +721,21 @@ extern "C" CC_API int cc_kv_ring_append(cc_device* dev, const cc_view* kring, co
     return CC_OK;
 }
 
-// Three kernels (plus the query norm), all plain 32-bit arithmetic, shaped as banded tile products so that keys and values are read once
-// per TILE of queries and once for all query heads of a key/value head, not once per (query, head):
-//   1. wa_scores_kernel : S[row][c] = (q_row . k_j) * scale - r1 ln(1 + r2 (i - j)) for the visible j = lo_i + c, a 64 x 64 tile product over dk
-//   2. wa_softmax_kernel: one warp per row: max, exp, sum, normalise (in place)
-//   3. wa_values_kernel : out[row][d] = sum_c S[row][c] v[lo_i + c][d], a 64 x 64 tile product over the keys of the tile's band
-// A row is one (query, head); a tile's 64 rows are the R = n_heads / n_kv heads of one key/value head for 64 / R consecutive queries.
-// Every dot product runs over its index in ascending order inside ONE thread, the softmax sums depend on the row alone, and the value sum
-// has one order per kernel (ascending keys in the tile kernel, masked keys adding an exact 0; ascending slices in the kernel that serves calls
-// of few rows): a query's result does not depend on where the call starts or what else it carries, and differs between a
-// prompt pass and a decoded token only by the rounding of that last sum.
-#define WA_TILE 64
-#define WA_K 16
-#define WA_THREADS 256
+// A pass of many rows is two products of 32-bit operands on the tensor cores (split_gemm.cuh), tiles of 128 rows:
+//   1. WaScores: S[row][j] = (q_row . k_j) * scale - r1 ln(1 + r2 (i - j)), -inf where masked, and the largest score of each row of the tile
+//   2. WaValues: out[row][d] = sum_j exp(S[row][j] - top) v[j][d] / (sum_j exp(S[row][j] - top) + sink); the weights are made while the operand is staged
+// A row is one (query, head); a tile's rows are the R = n_heads / n_kv heads of one key/value head for 128 / R consecutive queries, so that keys and
+// values are read once per tile and not once per (query, head).  A decoded token takes the two kernels for few rows below.
+// The keys of a tile start at a multiple of 64 positions, a score is one sum over dk, a row's weights are added in an order that the positions of the keys
+// alone decide (masked keys add an exact 0), and the value sum goes by steps of 64 positions, even ones and odd ones: a query's result does not
+// depend on where the call starts or what else it carries, and differs between a prompt pass and a decoded token only by the rounding of those sums.
+#define WA_ROWS 128
+#define WA_LOG2E 1.44269504f
 struct WaGeom {
     int T, H, G, R, dk, dv, window, block, ring, QT, cap;      // QT queries per tile; cap = row stride of S; block > 0: a query sees only its own block of positions
     int krs, vrs, vhs;                                  // floats between two rows of the key / value ring (vhs: between two heads' values inside a row)
     float softcap;                                      // > 0: score <- softcap * tanh(score / softcap), after the scale
+    int pos0_row;                                       // pos0 % ring
     int64_t pos0;
 };
 __host__ __device__ __forceinline__ int64_t wa_lo(const WaGeom& g, int64_t i) {
@@ -757,83 +756,187 @@ __global__ void head_rms_norm_kernel(float* __restrict__ x, const float* __restr
     for (int c = lane; c < hs; c += 32) xr[c] = xr[c] * inv * w[c];
 }
 
-// grid (key tiles of the band, query tiles, G)
-__global__ void __launch_bounds__(WA_THREADS) wa_scores_kernel(const float* __restrict__ q, const float* __restrict__ kring, float* __restrict__ S, WaGeom g, float scale,
-                                                               const float* __restrict__ r1, const float* __restrict__ r2) {
-    __shared__ float sq[WA_K][WA_TILE + 4];
-    __shared__ float sk[WA_K][WA_TILE + 4];
-    const int t0 = blockIdx.y * g.QT, kvh = blockIdx.z;
-    const int tq_n = min(g.QT, g.T - t0);
-    const int64_t i_first = g.pos0 + t0, i_last = i_first + tq_n - 1;
-    const int64_t band_lo = wa_lo(g, i_first);
-    const int64_t j0 = band_lo + (int64_t)blockIdx.x * WA_TILE;
-    if (j0 > i_last) return;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = 0.0f;
-    // the next 16 coordinates of queries and keys are fetched into registers while the current ones are multiplied; a thread's rows stay the same
-    float pq[4], pk[4];
-    const float *qp[4], *kp[4];
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const int r = (threadIdx.x + e * WA_THREADS) >> 4;
-        const int tq = r / g.R, hr = r - tq * g.R;
-        const int64_t j = j0 + r;
-        qp[e] = tq < tq_n ? q + ((int64_t)(t0 + tq) * g.H + kvh * g.R + hr) * g.dk : nullptr;
-        kp[e] = j <= i_last ? kring + (j % g.ring) * g.krs + kvh * g.dk : nullptr;
-    }
-    auto fetch = [&](int d0) {
-        const int d = d0 + (threadIdx.x & 15);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            pq[e] = (d < g.dk && qp[e]) ? qp[e][d] : 0.0f;
-            pk[e] = (d < g.dk && kp[e]) ? kp[e][d] : 0.0f;
-        }
-    };
-    fetch(0);
-    for (int d0 = 0; d0 < g.dk; d0 += WA_K) {
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int idx = threadIdx.x + e * WA_THREADS;
-            sq[idx & 15][idx >> 4] = pq[e];
-            sk[idx & 15][idx >> 4] = pk[e];
-        }
-        __syncthreads();
-        if (d0 + WA_K < g.dk) fetch(d0 + WA_K);
-#pragma unroll
-        for (int dd = 0; dd < WA_K; dd++) {
-            const float4 qv = *(const float4*)&sq[dd][ty * 4];
-            const float4 kv = *(const float4*)&sk[dd][tx * 4];
-            const float qr[4] = {qv.x, qv.y, qv.z, qv.w}, kr[4] = {kv.x, kv.y, kv.z, kv.w};
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = fmaf(qr[a], kr[b], acc[a][b]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-        const int r = ty * 4 + a;
-        const int tq = r / g.R, hr = r - tq * g.R;
-        if (tq >= tq_n) continue;
-        const int h = kvh * g.R + hr;
-        const int64_t i = i_first + tq, lo = wa_lo(g, i);
-        float* Sr = S + ((int64_t)(t0 + tq) * g.H + h) * g.cap;
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int64_t j = j0 + tx * 4 + b;
-            if (j < lo || j > i) continue;
-            float sc = acc[a][b] * scale;
-            if (g.softcap > 0.0f) sc = g.softcap * tanhf(sc / g.softcap);
-            if (r1) sc -= r1[h] * log1pf(r2[h] * (float)(i - j));
-            Sr[j - lo] = sc;
-        }
-    }
+// what the two products share: the tile's queries and the band of keys they can see
+struct WaTile {
+    int steps, t0, tq_n, kvh, c0, qt;                   // c0: first key (from `base` on) / first value column of the tile ; qt: which tile of queries
+    int band_lo, last;                                  // first and last key any of the tile's queries sees, counted from base
+    int ring0;                                          // the ring's row of position base
+    int step0;                                          // values: the first 64-key step of this CTA (it takes every second one)
+    int64_t base;                                       // a multiple of 64
+};
+__device__ __forceinline__ void wa_tile(const WaGeom& g, int qt, int kvh, WaTile& t) {
+    t.qt = qt; t.t0 = qt * g.QT; t.kvh = kvh; t.step0 = 0;
+    t.tq_n = min(g.QT, g.T - t.t0);
+    const int64_t i_first = g.pos0 + t.t0, lo = wa_lo(g, i_first);
+    t.base = lo & ~(int64_t)63;
+    t.band_lo = (int)(lo - t.base); t.last = (int)(i_first + t.tq_n - 1 - t.base);
+    // the ring holds every visible position, so base lies at most ring + 62 positions before pos0
+    t.ring0 = (int)((unsigned)((int)(t.base - g.pos0) + g.pos0_row + 64 + 2 * g.ring - 64 % g.ring) % (unsigned)g.ring);
 }
+struct WaFixed { int tq, hr; };                         // row r of a tile: its query and its head
+// -> its index among the T * H rows, or -1
+__device__ __forceinline__ int64_t wa_row(const WaGeom& g, const WaTile& t, WaFixed f) {
+    return f.tq < t.tq_n ? (int64_t)(t.t0 + f.tq) * g.H + t.kvh * g.R + f.hr : -1;
+}
+// the scores of a tile of queries: groups of 4 keys x 128 rows, so that the writer (a thread per row) and the reader (likewise) both move whole lines
+__device__ __forceinline__ int64_t wa_score_at(const WaTile& t, int q_tiles, int cap, int key, int r) {
+    return ((int64_t)t.kvh * q_tiles + t.qt) * WA_ROWS * cap + (int64_t)(key >> 2) * (4 * WA_ROWS) + r * 4;
+}
+// tiles: key tiles of the band (fastest), query tiles, G
+struct WaScores {
+    static constexpr int HALVES = 2, N = 128;
+    static constexpr bool A_TRANSPOSED = false, B_TRANSPOSED = false, SHARED = false;
+    typedef WaTile Tile;
+    typedef WaFixed Fixed;
+    struct Shared {};
+    typedef const float* ARow;
+    typedef const float* BCol;
+    const float *q, *kring, *r1, *r2;
+    float *S, *tops;                                    // tops: [G][query tiles][key tiles][4 quarters][WA_ROWS]
+    WaGeom g;
+    float scale;
+    int key_tiles, q_tiles, vec;                        // vec: rows may be read 16 bytes at a time
+    __device__ bool tile(int i, int, Tile& t) const {
+        const int rest = (unsigned)i / (unsigned)key_tiles, kvh = (unsigned)rest / (unsigned)q_tiles;
+        wa_tile(g, rest - kvh * q_tiles, kvh, t);
+        t.c0 = (i - rest * key_tiles) * N; t.steps = (g.dk + 63) >> 6;
+        return t.c0 <= t.last;
+    }
+    __device__ Fixed fixed(int r) const { const int tq = r / g.R; return Fixed{tq, r - tq * g.R}; }
+    __device__ void setup(const Tile&, Shared&) const {}
+    __device__ ARow a_row(const Tile& t, const Shared&, Fixed f, int) const {
+        const int64_t row = wa_row(g, t, f);
+        return row < 0 ? nullptr : q + row * g.dk;
+    }
+    __device__ void load_a(const Tile&, ARow a, int s, int c, float (&v)[8]) const { if (a) sg_load8(a, s * 64 + c * 8, g.dk, vec, v); else sg_zero8(v); }
+    __device__ void prep_a(const Tile&, ARow&, float (&)[8]) const {}
+    __device__ BCol b_col(const Tile& t, int n) const {
+        const int j = t.c0 + n;
+        return j < t.band_lo || j > t.last ? nullptr : kring + (int64_t)((unsigned)(t.ring0 + j) % (unsigned)g.ring) * g.krs + t.kvh * g.dk;
+    }
+    __device__ void load_b(const Tile&, BCol b, int s, int c, float (&v)[8]) const { if (b) sg_load8(b, s * 64 + c * 8, g.dk, vec, v); else sg_zero8(v); }
+    __device__ void end_a(const Tile&, Shared&, ARow&, int, int) const {}
+    __device__ void give(const Shared&, Shared&, int) const {}
+    template <int COUNT>
+    __device__ void emit(const Tile& t, const Shared&, Fixed f, int r, int col0, float (&v)[COUNT], float*) const {
+        int lo = 0, hi = -1;                            // visible keys, counted from the first of the COUNT
+        const int h = t.kvh * g.R + f.hr;
+        float a1 = 0.0f, a2 = 0.0f, top = -INFINITY;
+        if (f.tq < t.tq_n) {
+            const int64_t i = g.pos0 + t.t0 + f.tq;
+            lo = (int)(wa_lo(g, i) - t.base) - t.c0 - col0; hi = (int)(i - t.base) - t.c0 - col0;
+            if (r1) { a1 = r1[h]; a2 = r2[h]; }
+        }
+#pragma unroll
+        for (int c = 0; c < COUNT; c++) v[c] *= scale;
+        if (g.softcap > 0.0f) {
+#pragma unroll
+            for (int c = 0; c < COUNT; c++) v[c] = g.softcap * tanhf(v[c] / g.softcap);
+        }
+        if (r1) {
+#pragma unroll
+            for (int c = 0; c < COUNT; c++) v[c] -= a1 * log1pf(a2 * (float)(hi - c));
+        }
+#pragma unroll
+        for (int c = 0; c < COUNT; c++) {
+            v[c] = c < lo || c > hi ? -INFINITY : v[c];
+            top = fmaxf(top, v[c]);
+        }
+        float* s = S + wa_score_at(t, q_tiles, g.cap, t.c0 + col0, r);
+#pragma unroll
+        for (int c = 0; c < COUNT; c += 4) *(float4*)(s + c * WA_ROWS) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        tops[((((int64_t)t.kvh * q_tiles + t.qt) * key_tiles + t.c0 / N) * 4 + col0 / COUNT) * WA_ROWS + r] = top;
+    }
+};
+// tiles: value columns (fastest), query tiles, G; the two CTAs of a cluster take the 64-key steps whose position is an even / odd multiple of 64
+// sink != NULL: the denominator also holds exp(sink[head]), a key without a value whose score is sink[head] as it stands (no scale)
+// exp(s - top) is taken as 2^(s log2e - top log2e): one rounding, and that of the second term is common to a row's weights and its denominator
+template <int TILE_HALVES>
+struct WaValues {
+    static constexpr int HALVES = TILE_HALVES, N = 64 * HALVES;
+    static constexpr bool A_TRANSPOSED = true, B_TRANSPOSED = true, SHARED = true;
+    typedef WaTile Tile;
+    typedef WaFixed Fixed;
+    struct Shared { float top[WA_ROWS], sum[8][WA_ROWS]; };     // top: times log2e ; sum: of each quarter of the threads, of this CTA and of the other
+    struct ARow { const float* s; float top, sum; };
+    typedef const float* BCol;
+    const float *S, *tops, *vring, *sink;
+    float* o;
+    WaGeom g;
+    int key_tiles, q_tiles;                             // of the scores
+    __device__ bool tile(int i, int rank, Tile& t) const {
+        const int per = (g.dv + N - 1) / N, rest = (unsigned)i / (unsigned)per, kvh = (unsigned)rest / (unsigned)q_tiles;
+        wa_tile(g, rest - kvh * q_tiles, kvh, t);
+        t.c0 = (i - rest * per) * N;
+        t.step0 = (int)(((t.base >> 6) & 1) ^ rank);
+        t.steps = ((t.last >> 6) + 2 - t.step0) >> 1;
+        return true;
+    }
+    __device__ Fixed fixed(int r) const { const int tq = r / g.R; return Fixed{tq, r - tq * g.R}; }
+    __device__ float sink_of(const Tile& t, int r) const { return sink[t.kvh * g.R + r % g.R]; }
+    __device__ void setup(const Tile& t, Shared& ps) const {
+        const int r = threadIdx.x;
+        if (r >= WA_ROWS) return;
+        const float* p = tops + ((int64_t)t.kvh * q_tiles + t.qt) * key_tiles * 4 * WA_ROWS + r;
+        float top = -INFINITY;
+#pragma unroll 8
+        for (int n = 0; n < 4 * (t.last / WaScores::N + 1); n++) top = fmaxf(top, p[n * WA_ROWS]);
+        if (sink) top = fmaxf(top, sink_of(t, r));
+        ps.top[r] = top * WA_LOG2E;
+    }
+    __device__ float weight(float s, float top) const {
+        float e;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(fmaf(s, WA_LOG2E, -top)));
+        return e;
+    }
+    __device__ ARow a_row(const Tile& t, const Shared& ps, Fixed f, int r) const {
+        return ARow{f.tq < t.tq_n ? S + wa_score_at(t, q_tiles, g.cap, 0, r) : nullptr, ps.top[r], 0.0f};
+    }
+    __device__ void load_a(const Tile& t, const ARow& a, int s, int c, float (&v)[8]) const {
+        if (!a.s) { sg_zero8(v); return; }
+        const float* p = a.s + ((t.step0 + 2 * s) * 16 + c * 2) * (4 * WA_ROWS);
+        const float4 x = *(const float4*)p, y = *(const float4*)(p + 4 * WA_ROWS);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+    }
+    __device__ void prep_a(const Tile&, ARow& a, float (&v)[8]) const {
+        if (!a.s) return;
+#pragma unroll
+        for (int i = 0; i < 8; i++) { v[i] = weight(v[i], a.top); a.sum += v[i]; }
+    }
+    __device__ BCol b_col(const Tile& t, int n) const { return t.c0 + n < g.dv ? vring + t.kvh * g.vhs + t.c0 + n : nullptr; }
+    __device__ void load_b(const Tile& t, BCol b, int s, int c, float (&v)[8]) const {
+        const int k = (t.step0 + 2 * s) * 64 + c * 8;
+        unsigned row = (unsigned)(t.ring0 + k);
+        while (row >= (unsigned)g.ring) row -= (unsigned)g.ring;
+        if (b && k >= t.band_lo && k + 7 <= t.last && row + 8 <= (unsigned)g.ring) {
+            const float* at = b + (int64_t)row * g.vrs;
+#pragma unroll
+            for (int i = 0; i < 8; i++) { v[i] = *at; at += g.vrs; }
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            v[i] = b && k + i >= t.band_lo && k + i <= t.last ? b[(int64_t)row * g.vrs] : 0.0f;
+            if (++row == (unsigned)g.ring) row = 0;
+        }
+    }
+    __device__ void end_a(const Tile&, Shared& ps, const ARow& a, int r, int part) const { ps.sum[part][r] = a.sum; }
+    // a CTA's sums of weights to the other
+    __device__ void give(const Shared& mine, Shared& theirs, int tid) const { theirs.sum[4 + (tid >> 7)][tid & 127] = mine.sum[tid >> 7][tid & 127]; }
+    template <int COUNT>
+    __device__ void emit(const Tile& t, const Shared& ps, Fixed f, int r, int col0, float (&v)[COUNT], float* buf) const {
+        float a = 0.0f, b = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) { a += ps.sum[i][r]; b += ps.sum[4 + i][r]; }
+        float total = a + b;                            // of the two CTAs, the same number in both
+        if (sink) total += weight(sink_of(t, r), ps.top[r]);
+        const float inv = 1.0f / total;
+#pragma unroll
+        for (int c = 0; c < COUNT; c++) v[c] *= inv;
+        const int64_t row = wa_row(g, t, f);
+        sg_store_rows<COUNT, false>(buf, row < 0 ? nullptr : o + row * g.dv + t.c0 + col0, g.dv - t.c0 - col0, v);
+    }
+};
 // few rows (decoding): grid (ceil(keys / 16), T, G * head blocks), 256 threads.  The CTA stages up to WS_HEADS queries of (token, key/value head); a
 // warp owns two visible keys and takes their dot products with each of them: lane-strided partial sums, then the butterfly.  A key row is
 // read into registers once for the block's heads (rows longer than WS_KEEP * 32: as far as they fit), and the keys spread over the whole device
@@ -879,27 +982,6 @@ __global__ void __launch_bounds__(256) wa_scores_row_kernel(const float* __restr
             S[((int64_t)t * g.H + h) * g.cap + (j - lo)] = sc;
         }
     }
-}
-// one warp per row
-// sink != NULL: the denominator also holds exp(sink[head]), a key without a value whose score is sink[head] as it stands (no scale)
-__global__ void wa_softmax_kernel(float* __restrict__ S, WaGeom g, const float* __restrict__ sink) {
-    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= (int64_t)g.T * g.H) return;
-    const int64_t i = g.pos0 + row / g.H;
-    const int n = (int)(i - wa_lo(g, i) + 1);
-    float* Sr = S + row * g.cap;
-    float mx = -INFINITY;
-    for (int c = lane; c < n; c += 32) mx = fmaxf(mx, Sr[c]);
-    mx = warp_max(mx);
-    const float sk = sink ? sink[row % g.H] : -INFINITY;
-    mx = fmaxf(mx, sk);
-    float sum = 0.0f;
-    for (int c = lane; c < n; c += 32) { const float e = expf(Sr[c] - mx); Sr[c] = e; sum += e; }
-    sum = warp_sum(sum);
-    if (sink) sum += expf(sk - mx);
-    const float inv = 1.0f / sum;
-    for (int c = lane; c < n; c += 32) Sr[c] *= inv;
 }
 // few rows (decoding): grid (T * G * head blocks, ceil(dv / 32), WV_SPLIT) in clusters of WV_SPLIT CTAs along z.  A cluster owns 32 value columns of
 // RB query heads of one (token, key/value head), each of its CTAs one contiguous slice of the visible keys: raw scores of the slice -> its
@@ -994,87 +1076,6 @@ static cudaError_t wa_launch_slices(cc_device* dev, const float* S, const float*
     wa_values_slices_kernel<RB><<<dim3((unsigned)(g.T * g.G * ((g.R + RB - 1) / RB)), (unsigned)((g.dv + 31) / 32), WV_SPLIT), WV_THREADS, smem, dev->stream>>>(S, v, out, g, sink, slice_cap);
     return cudaSuccess;
 }
-// grid (dv tiles, query tiles, G)
-__global__ void __launch_bounds__(WA_THREADS) wa_values_kernel(const float* __restrict__ S, const float* __restrict__ vring, float* __restrict__ out, WaGeom g) {
-    __shared__ float sp[WA_K][WA_TILE + 4];       // [key][row]
-    __shared__ float sv[WA_K][WA_TILE + 4];       // [key][dv column]
-    const int t0 = blockIdx.y * g.QT, kvh = blockIdx.z, c0 = blockIdx.x * WA_TILE;
-    const int tq_n = min(g.QT, g.T - t0);
-    const int64_t i_first = g.pos0 + t0, i_last = i_first + tq_n - 1;
-    const int64_t band_lo = wa_lo(g, i_first);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = 0.0f;
-    // the next block of 16 keys (probabilities and values) is fetched into registers while the current one is multiplied: the loads' latency
-    // hides behind the arithmetic of a CTA that often has its SM to itself
-    // keys are counted from the band's first one; a thread's rows, its column and its keys inside a block of 16 stay the same
-    float pp[4], pv[4];
-    const float *Sp[4], *vp[4];
-    int p_lo[4], p_hi[4], vrow[4];
-    const int last_rel = (int)(i_last - band_lo);
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const int idx = threadIdx.x + e * WA_THREADS;
-        {   // probabilities: consecutive threads read consecutive keys of one row
-            const int r = idx >> 4, tq = r / g.R, hr = r - tq * g.R;
-            const int64_t i = i_first + tq, lo = wa_lo(g, i);
-            const bool on = tq < tq_n;
-            p_lo[e] = (int)(lo - band_lo); p_hi[e] = on ? (int)(i - band_lo) : -1;
-            Sp[e] = on ? S + ((int64_t)(t0 + tq) * g.H + kvh * g.R + hr) * g.cap - p_lo[e] : S;
-        }
-        {   // values: consecutive threads read consecutive columns of one key
-            const int kk = idx >> 6, c = c0 + (idx & 63);
-            vrow[e] = (int)((band_lo + kk) % g.ring);
-            vp[e] = c < g.dv ? vring + kvh * g.vhs + c : nullptr;
-        }
-    }
-    auto fetch = [&](int j_rel) {                                // called with 0, 16, 32, ...
-        const int jp = j_rel + (threadIdx.x & 15);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            pp[e] = (jp >= p_lo[e] && jp <= p_hi[e]) ? Sp[e][jp] : 0.0f;
-            pv[e] = (vp[e] && j_rel + ((threadIdx.x + e * WA_THREADS) >> 6) <= last_rel) ? vp[e][(int64_t)vrow[e] * g.vrs] : 0.0f;
-            vrow[e] += WA_K;
-            while (vrow[e] >= g.ring) vrow[e] -= g.ring;
-        }
-    };
-    fetch(0);
-    for (int j0 = 0; j0 <= last_rel; j0 += WA_K) {
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int idx = threadIdx.x + e * WA_THREADS;
-            sp[idx & 15][idx >> 4] = pp[e];
-            sv[idx >> 6][idx & 63] = pv[e];
-        }
-        __syncthreads();
-        if (j0 + WA_K <= last_rel) fetch(j0 + WA_K);
-#pragma unroll
-        for (int kk = 0; kk < WA_K; kk++) {
-            const float4 pv4 = *(const float4*)&sp[kk][ty * 4];
-            const float4 vv = *(const float4*)&sv[kk][tx * 4];
-            const float pr[4] = {pv4.x, pv4.y, pv4.z, pv4.w}, vr[4] = {vv.x, vv.y, vv.z, vv.w};
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = fmaf(pr[a], vr[b], acc[a][b]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-        const int r = ty * 4 + a;
-        const int tq = r / g.R, hr = r - tq * g.R;
-        if (tq >= tq_n) continue;
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int c = c0 + tx * 4 + b;
-            if (c < g.dv) out[((int64_t)(t0 + tq) * g.H + kvh * g.R + hr) * g.dv + c] = acc[a][b];
-        }
-    }
-}
 static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view* qnw, float eps, const cc_view* kring, const cc_view* vring, int64_t pos0, int32_t H, int32_t G,
                                  int32_t dk, int32_t dv, int32_t window, int32_t block, float scale, const cc_view* r1, const cc_view* r2, const cc_view* sink, cc_buf** out,
                                  float softcap = 0.0f) {
@@ -1112,9 +1113,21 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
     if (block > 0 && block < reach) reach = block;
     const int64_t maxn = reach;
     const int R = H / G;
-    CC_REQUIRE(dev, R <= WA_TILE, "window_attention: %d query heads per key/value head (at most %d)", R, WA_TILE);
-    g.T = (int)T; g.H = H; g.G = G; g.R = R; g.dk = dk; g.dv = dv; g.ring = (int)ring; g.QT = WA_TILE / R; g.cap = (int)maxn; g.pos0 = pos0;
+    CC_REQUIRE(dev, R <= 64, "window_attention: %d query heads per key/value head (at most %d)", R, 64);
+    g.T = (int)T; g.H = H; g.G = G; g.R = R; g.dk = dk; g.dv = dv; g.ring = (int)ring; g.QT = WA_ROWS / R; g.pos0 = pos0; g.pos0_row = (int)(pos0 % ring);
     g.krs = G * dk; g.vrs = vring ? G * dv : G * dk; g.vhs = vring ? dv : dk;
+    const float *r1p = r1 ? fptr(r1) : nullptr, *r2p = r2 ? fptr(r2) : nullptr, *sinkp = sink ? fptr(sink) : nullptr;
+    // few rows: keys spread over the whole device; what its kernels keep in shared memory has to fit
+    const int s_heads = R < WS_HEADS ? R : WS_HEADS;
+    const int RB = R >= 8 ? 8 : R >= 3 ? 4 : R;              // query heads a cluster of the few-row value kernel takes together
+    int slice_cap = 0;
+    const size_t rows_smem = (size_t)s_heads * dk * 4, slices_smem = wa_slices_smem(RB, maxn, &slice_cap);
+    const bool few_rows = T * H <= 64 && rows_smem <= 160 * 1024 && slices_smem <= 160 * 1024;
+    const int q_tiles = (int)((T + g.QT - 1) / g.QT);
+    // keys a query tile can see, counted from the multiple of 64 below the first of them
+    const int64_t band = reach - 1 + g.QT + 63, band_max = band < last + 64 ? band : last + 64;
+    const int key_tiles = (int)((band_max + WaScores::N - 1) / WaScores::N);
+    g.cap = few_rows ? (int)maxn : key_tiles * WaScores::N;
     float* qp = fptr(q);
     if (qnw) {             // the query norm, in place: q is this call's private projection output in every caller of the runner; a caller that
                            // needs its q untouched passes a copy
@@ -1122,42 +1135,27 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
         dev->launches++;
     }
     void* Sp = nullptr; size_t cls = 0;
-    rc = cc_pool_alloc(dev, (size_t)T * H * maxn * 4, &Sp, &cls);
+    const size_t scores = few_rows ? (size_t)T * H * g.cap : (size_t)G * q_tiles * WA_ROWS * g.cap;
+    rc = cc_pool_alloc(dev, (scores + (few_rows ? 0 : (size_t)G * q_tiles * key_tiles * 4 * WA_ROWS)) * 4, &Sp, &cls);
     if (rc) return rc;
-    const int q_tiles = (int)((T + g.QT - 1) / g.QT);
-    const int64_t band = reach - 1 + g.QT;                                             // keys a query tile can see
-    const int64_t band_max = band < last + 1 ? band : last + 1;
-    const bool few_rows = T * H <= 64;
-    const int s_heads = R < WS_HEADS ? R : WS_HEADS;
-    if (few_rows && (size_t)s_heads * dk * 4 <= 160 * 1024) {
-        const size_t smem = (size_t)s_heads * dk * 4;
-        if (smem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(wa_scores_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) { cc_pool_free(dev, Sp, cls); return cc_fail(dev, CC_ERR_CUDA, "window_attention: %s", cudaGetErrorString(e)); } }
-        wa_scores_row_kernel<<<dim3((unsigned)((maxn + 15) / 16), (unsigned)T, (unsigned)(G * ((R + WS_HEADS - 1) / WS_HEADS))), 256, smem, dev->stream>>>(qp, fptr(kring), (float*)Sp, g, scale, r1 ? fptr(r1) : nullptr,
-                                                                                                                      r2 ? fptr(r2) : nullptr);
-    } else {
-        dim3 g1((unsigned)((band_max + WA_TILE - 1) / WA_TILE), (unsigned)q_tiles, (unsigned)G);
-        wa_scores_kernel<<<g1, WA_THREADS, 0, dev->stream>>>(qp, fptr(kring), (float*)Sp, g, scale, r1 ? fptr(r1) : nullptr, r2 ? fptr(r2) : nullptr);
+    if (!few_rows) {
+        float* tops = (float*)Sp + scores;
+        const int vec = dk % 4 == 0 && (((uintptr_t)qp | (uintptr_t)fptr(kring)) & 15) == 0;
+        rc = sg_launch(dev, WaScores{qp, fptr(kring), r1p, r2p, (float*)Sp, tops, g, scale, key_tiles, q_tiles, vec}, (int64_t)key_tiles * q_tiles * G);
+        if (rc == CC_OK)
+            rc = dv > 64 ? sg_launch<WaValues<2>, true>(dev, WaValues<2>{(const float*)Sp, tops, vptr, sinkp, (float*)o->base, g, key_tiles, q_tiles}, (int64_t)((dv + 127) / 128) * q_tiles * G)
+                         : sg_launch<WaValues<1>, true>(dev, WaValues<1>{(const float*)Sp, tops, vptr, sinkp, (float*)o->base, g, key_tiles, q_tiles}, (int64_t)q_tiles * G);
+        cc_pool_free(dev, Sp, cls);
+        return rc;
     }
+    if (rows_smem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(wa_scores_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem); if (e != cudaSuccess) { cc_pool_free(dev, Sp, cls); return cc_fail(dev, CC_ERR_CUDA, "window_attention: %s", cudaGetErrorString(e)); } }
+    wa_scores_row_kernel<<<dim3((unsigned)((maxn + 15) / 16), (unsigned)T, (unsigned)(G * ((R + WS_HEADS - 1) / WS_HEADS))), 256, rows_smem, dev->stream>>>(qp, fptr(kring), (float*)Sp, g, scale, r1p, r2p);
     dev->launches++;
-    const int RB = R >= 8 ? 8 : R >= 3 ? 4 : R;              // query heads a cluster of the few-row value kernel takes together
-    int slice_cap = 0;
-    const size_t slices_smem = wa_slices_smem(RB, maxn, &slice_cap);
-    const bool row_values = few_rows && slices_smem <= 160 * 1024;
-    if (!row_values) {
-        wa_softmax_kernel<<<(unsigned)((T * H + 7) / 8), 256, 0, dev->stream>>>((float*)Sp, g, sink ? fptr(sink) : nullptr);
-        dev->launches++;
-    }
-    if (row_values) {
-        const float* sp = sink ? fptr(sink) : nullptr;
-        cudaError_t e = RB == 8 ? wa_launch_slices<8>(dev, (const float*)Sp, vptr, (float*)o->base, g, sp, slices_smem, slice_cap)
-                      : RB == 4 ? wa_launch_slices<4>(dev, (const float*)Sp, vptr, (float*)o->base, g, sp, slices_smem, slice_cap)
-                      : RB == 2 ? wa_launch_slices<2>(dev, (const float*)Sp, vptr, (float*)o->base, g, sp, slices_smem, slice_cap)
-                                : wa_launch_slices<1>(dev, (const float*)Sp, vptr, (float*)o->base, g, sp, slices_smem, slice_cap);
-        if (e != cudaSuccess) { cc_pool_free(dev, Sp, cls); return cc_fail(dev, CC_ERR_CUDA, "window_attention: %s", cudaGetErrorString(e)); }
-    } else {
-        dim3 g3((unsigned)((dv + WA_TILE - 1) / WA_TILE), (unsigned)q_tiles, (unsigned)G);
-        wa_values_kernel<<<g3, WA_THREADS, 0, dev->stream>>>((const float*)Sp, vptr, (float*)o->base, g);
-    }
+    cudaError_t e = RB == 8 ? wa_launch_slices<8>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap)
+                  : RB == 4 ? wa_launch_slices<4>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap)
+                  : RB == 2 ? wa_launch_slices<2>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap)
+                            : wa_launch_slices<1>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap);
+    if (e != cudaSuccess) { cc_pool_free(dev, Sp, cls); return cc_fail(dev, CC_ERR_CUDA, "window_attention: %s", cudaGetErrorString(e)); }
     cc_pool_free(dev, Sp, cls);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;

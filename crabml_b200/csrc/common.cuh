@@ -218,6 +218,8 @@ int cc_launch_matvec(cc_device* dev, const cc_buf* w, const void* act_scratch, c
 bool cc_prefill_supported(int wtype, int64_t m, int64_t k, int64_t b);
 int cc_launch_prefill_matmul(cc_device* dev, const cc_buf* w, const void* act, const float* x_f32, float* out, int64_t m, int64_t k, int64_t b);
 void cc_prefill_release(cc_device* dev);
+// tensor map (CUtensorMap) of a bfloat16 matrix [rows][k], box 64 columns x box_rows rows, 128-byte swizzle
+int cc_make_tmap_bf16(cc_device* dev, void* tm, const void* base, int64_t rows, int64_t k, int box_rows);
 
 // ---- dense.cu: plain F32 / BF16 weight matrices with a batch of activation rows -------------------
 bool cc_dense_supported(int wtype, int64_t b);

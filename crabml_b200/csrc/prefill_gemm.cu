@@ -228,6 +228,8 @@ static int pg_make_tmap(cc_device* dev, CUtensorMap* tm, const void* base, int64
     return CC_OK;
 }
 
+int cc_make_tmap_bf16(cc_device* dev, void* tm, const void* base, int64_t rows, int64_t k, int box_rows) { return pg_make_tmap(dev, (CUtensorMap*)tm, base, rows, k, box_rows, true); }
+
 struct PgScratch { void* w = nullptr; size_t w_bytes = 0; void* x = nullptr; size_t x_bytes = 0; };
 static PgScratch* pg_scratch(cc_device* dev) {
     static std::mutex mu;

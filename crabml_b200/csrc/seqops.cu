@@ -7,6 +7,7 @@
 // (a warp's lane-strided partial sums and the xor butterfly, or one thread's sequential loop), so prefill, chunked prefill and
 // token-by-token decoding give the same bits for the recurrent layers and the same bits per (query, key set) for attention.
 #include <cooperative_groups.h>
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include "../../include/crabml_seqops.h"
@@ -721,7 +722,8 @@ extern "C" CC_API int cc_kv_ring_append(cc_device* dev, const cc_view* kring, co
     return CC_OK;
 }
 
-// A pass of many rows is two products of 32-bit operands on the tensor cores (split_gemm.cuh), tiles of 128 rows:
+// A pass of many rows is two products of 32-bit operands on the tensor cores (split_gemm.cuh), tiles of 128 rows, after one kernel that cuts what many
+// tiles read: queries in the order of the tiles' rows, keys and (transposed) values in the order of their positions:
 //   1. WaScores: S[row][j] = (q_row . k_j) * scale - r1 ln(1 + r2 (i - j)), -inf where masked, and the largest score of each row of the tile
 //   2. WaValues: out[row][d] = sum_j exp(S[row][j] - top) v[j][d] / (sum_j exp(S[row][j] - top) + sink); the weights are made while the operand is staged
 // A row is one (query, head); a tile's rows are the R = n_heads / n_kv heads of one key/value head for 128 / R consecutive queries, so that keys and
@@ -736,6 +738,8 @@ struct WaGeom {
     int krs, vrs, vhs;                                  // floats between two rows of the key / value ring (vhs: between two heads' values inside a row)
     float softcap;                                      // > 0: score <- softcap * tanh(score / softcap), after the scale
     int pos0_row;                                       // pos0 % ring
+    int span, dkp, dvp;                                 // keys in the cut planes ; dk and dv in whole tiles
+    int64_t base0;                                      // position of the planes' first key, a multiple of 64
     int64_t pos0;
 };
 __host__ __device__ __forceinline__ int64_t wa_lo(const WaGeom& g, int64_t i) {
@@ -761,6 +765,7 @@ struct WaTile {
     int steps, t0, tq_n, kvh, c0, qt;                   // c0: first key (from `base` on) / first value column of the tile ; qt: which tile of queries
     int band_lo, last;                                  // first and last key any of the tile's queries sees, counted from base
     int ring0;                                          // the ring's row of position base
+    int at;                                             // base, counted from the first key of the cut planes
     int step0;                                          // values: the first 64-key step of this CTA (it takes every second one)
     int64_t base;                                       // a multiple of 64
 };
@@ -770,6 +775,7 @@ __device__ __forceinline__ void wa_tile(const WaGeom& g, int qt, int kvh, WaTile
     const int64_t i_first = g.pos0 + t.t0, lo = wa_lo(g, i_first);
     t.base = lo & ~(int64_t)63;
     t.band_lo = (int)(lo - t.base); t.last = (int)(i_first + t.tq_n - 1 - t.base);
+    t.at = (int)(t.base - g.base0);
     // the ring holds every visible position, so base lies at most ring + 62 positions before pos0
     t.ring0 = (int)((unsigned)((int)(t.base - g.pos0) + g.pos0_row + 64 + 2 * g.ring - 64 % g.ring) % (unsigned)g.ring);
 }
@@ -782,13 +788,63 @@ __device__ __forceinline__ int64_t wa_row(const WaGeom& g, const WaTile& t, WaFi
 __device__ __forceinline__ int64_t wa_score_at(const WaTile& t, int q_tiles, int cap, int key, int r) {
     return ((int64_t)t.kvh * q_tiles + t.qt) * WA_ROWS * cap + (int64_t)(key >> 2) * (4 * WA_ROWS) + r * 4;
 }
+// what many tiles read, cut once into three planes of bfloat16 (split_gemm.cuh).  Blocks 0 .. row_blocks: eight elements of a query or key row per
+// thread; the rest: 64 keys x 64 columns of the values, turned through shared memory.  Rows of no query, positions nobody sees and columns
+// behind dk / dv are zeros.  Bound by memory: 10 bytes per element.
+__global__ void __launch_bounds__(256) wa_cut_kernel(const float* __restrict__ q, const float* __restrict__ kring, const float* __restrict__ vring, uint8_t* __restrict__ qc,
+                                                     uint8_t* __restrict__ kc, uint8_t* __restrict__ vc, WaGeom g, int q_tiles, unsigned row_blocks, int64_t lo0, int vec) {
+    const int64_t last = g.pos0 + g.T - 1;
+    const int64_t q_rows = (int64_t)g.G * q_tiles * WA_ROWS, k_rows = (int64_t)g.G * g.span;
+    float v[8];
+    if (blockIdx.x < row_blocks) {
+        const int per = g.dkp >> 3;
+        const int64_t u = (int64_t)blockIdx.x * 256 + threadIdx.x, row = u / per;
+        const int c = (int)(u - row * per) * 8;
+        if (row >= q_rows + k_rows) return;
+        const float* src = nullptr;
+        if (row < q_rows) {
+            const int r = (int)(row % WA_ROWS), tq = r / g.R;
+            const int64_t qt = row / WA_ROWS % q_tiles, t = qt * g.QT + tq;
+            if (tq < g.QT && t < g.T) src = q + (t * g.H + row / WA_ROWS / q_tiles * g.R + (r - tq * g.R)) * g.dk;
+        } else {
+            const int64_t kvh = (row - q_rows) / g.span, j = g.base0 + (row - q_rows) % g.span;
+            if (j >= lo0 && j <= last) src = kring + (j % g.ring) * g.krs + kvh * g.dk;
+        }
+        if (src) sg_load8(src, c, g.dk, vec, v); else sg_zero8(v);
+        if (row < q_rows) sg_cut(qc + (row * g.dkp + c) * 2, (size_t)q_rows * g.dkp * 2, v);
+        else sg_cut(kc + ((row - q_rows) * g.dkp + c) * 2, (size_t)k_rows * g.dkp * 2, v);
+        return;
+    }
+    __shared__ float turn[64][65];
+    const unsigned b = blockIdx.x - row_blocks, key_blocks = g.span >> 6, col_blocks = g.dvp >> 6;
+    const int j0 = (int)(b % key_blocks) * 64, d0 = (int)(b / key_blocks % col_blocks) * 64, kvh = (int)(b / key_blocks / col_blocks);
+#pragma unroll 4
+    for (int i = threadIdx.x >> 6; i < 64; i += 4) {
+        const int64_t j = g.base0 + j0 + i;
+        const int d = d0 + (threadIdx.x & 63);
+        turn[i][threadIdx.x & 63] = j >= lo0 && j <= last && d < g.dv ? vring[(j % g.ring) * g.vrs + kvh * g.vhs + d] : 0.0f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int d = (threadIdx.x >> 3) + 32 * i, k = (threadIdx.x & 7) * 8;
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[e] = turn[k + e][d];
+        sg_cut(vc + (((int64_t)kvh * g.dvp + d0 + d) * g.span + j0 + k) * 2, (size_t)g.G * g.dvp * g.span * 2, v);
+    }
+}
 // tiles: key tiles of the band (fastest), query tiles, G
 struct WaScores {
     static constexpr int HALVES = 2, N = 128;
-    static constexpr bool A_TRANSPOSED = false, B_TRANSPOSED = false, SHARED = false;
+    static constexpr bool A_TRANSPOSED = false, B_TRANSPOSED = false, SHARED = false, A_TMA = true, B_TMA = true;
     typedef WaTile Tile;
     typedef WaFixed Fixed;
     struct Shared {};
+    CUtensorMap maps[2];                                // queries [3][G][query tiles][128][dkp], keys [3][G][span][dkp]
+    __device__ const void* map_a() const { return &maps[0]; }
+    __device__ const void* map_b() const { return &maps[1]; }
+    __device__ void at_a(const Tile& t, int s, int plane, int& x, int& y) const { x = s * 64; y = ((plane * g.G + t.kvh) * q_tiles + t.qt) * WA_ROWS; }
+    __device__ void at_b(const Tile& t, int s, int plane, int& x, int& y) const { x = s * 64; y = (plane * g.G + t.kvh) * g.span + t.at + t.c0; }
     typedef const float* ARow;
     typedef const float* BCol;
     const float *q, *kring, *r1, *r2;
@@ -854,9 +910,14 @@ struct WaScores {
 template <int TILE_HALVES>
 struct WaValues {
     static constexpr int HALVES = TILE_HALVES, N = 64 * HALVES;
-    static constexpr bool A_TRANSPOSED = true, B_TRANSPOSED = true, SHARED = true;
+    static constexpr bool A_TRANSPOSED = true, B_TRANSPOSED = true, SHARED = true, A_TMA = false, B_TMA = true;
     typedef WaTile Tile;
     typedef WaFixed Fixed;
+    CUtensorMap maps[1];                                // values [3][G][dvp][span]
+    __device__ const void* map_a() const { return nullptr; }
+    __device__ const void* map_b() const { return &maps[0]; }
+    __device__ void at_a(const Tile&, int, int, int&, int&) const {}
+    __device__ void at_b(const Tile& t, int s, int plane, int& x, int& y) const { x = t.at + (t.step0 + 2 * s) * 64; y = (plane * g.G + t.kvh) * g.dvp + t.c0; }
     struct Shared { float top[WA_ROWS], sum[8][WA_ROWS]; };     // top: times log2e ; sum: of each quarter of the threads, of this CTA and of the other
     struct ARow { const float* s; float top, sum; };
     typedef const float* BCol;
@@ -1135,19 +1196,41 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
         dev->launches++;
     }
     void* Sp = nullptr; size_t cls = 0;
-    const size_t scores = few_rows ? (size_t)T * H * g.cap : (size_t)G * q_tiles * WA_ROWS * g.cap;
-    rc = cc_pool_alloc(dev, (scores + (few_rows ? 0 : (size_t)G * q_tiles * key_tiles * 4 * WA_ROWS)) * 4, &Sp, &cls);
-    if (rc) return rc;
     if (!few_rows) {
-        float* tops = (float*)Sp + scores;
+        const int vtile = dv > 64 ? 128 : 64;
+        g.base0 = oldest & ~(int64_t)63;
+        g.span = (int)((last - g.base0 + 64) & ~(int64_t)63) + 64;          // in whole steps, and one more: a tile of 128 keys may start at any step
+        g.dkp = (dk + 63) & ~63; g.dvp = (dv + vtile - 1) / vtile * vtile;
+        const size_t q_rows = (size_t)G * q_tiles * WA_ROWS, scores = q_rows * g.cap * 4, tops = (size_t)G * q_tiles * key_tiles * 4 * WA_ROWS * 4;
+        const size_t qc = 3 * q_rows * g.dkp * 2, kc = 3 * (size_t)G * g.span * g.dkp * 2, vc = 3 * (size_t)G * g.dvp * g.span * 2;
+        CC_REQUIRE(dev, 3 * q_rows < ((size_t)1 << 31) && (size_t)3 * G * g.span < ((size_t)1 << 31), "window_attention: too many rows");
+        rc = cc_pool_alloc(dev, scores + tops + qc + kc + vc, &Sp, &cls);   // every part is a multiple of 512 bytes
+        if (rc) return rc;
+        uint8_t *base = (uint8_t*)Sp, *qp3 = base + scores + tops, *kp3 = qp3 + qc, *vp3 = kp3 + kc;
         const int vec = dk % 4 == 0 && (((uintptr_t)qp | (uintptr_t)fptr(kring)) & 15) == 0;
-        rc = sg_launch(dev, WaScores{qp, fptr(kring), r1p, r2p, (float*)Sp, tops, g, scale, key_tiles, q_tiles, vec}, (int64_t)key_tiles * q_tiles * G);
-        if (rc == CC_OK)
-            rc = dv > 64 ? sg_launch<WaValues<2>, true>(dev, WaValues<2>{(const float*)Sp, tops, vptr, sinkp, (float*)o->base, g, key_tiles, q_tiles}, (int64_t)((dv + 127) / 128) * q_tiles * G)
-                         : sg_launch<WaValues<1>, true>(dev, WaValues<1>{(const float*)Sp, tops, vptr, sinkp, (float*)o->base, g, key_tiles, q_tiles}, (int64_t)q_tiles * G);
+        const int64_t row_blocks = ((int64_t)(q_rows + (size_t)G * g.span) * (g.dkp >> 3) + 255) / 256, blocks = row_blocks + (int64_t)(g.span >> 6) * (g.dvp >> 6) * G;
+        WaScores ws{};
+        ws.q = qp; ws.kring = fptr(kring); ws.r1 = r1p; ws.r2 = r2p; ws.S = (float*)base; ws.tops = (float*)(base + scores); ws.g = g; ws.scale = scale;
+        ws.key_tiles = key_tiles; ws.q_tiles = q_tiles; ws.vec = vec;
+        CUtensorMap vmap;
+        rc = cc_make_tmap_bf16(dev, &ws.maps[0], qp3, 3 * (int64_t)q_rows, g.dkp, WA_ROWS);
+        if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &ws.maps[1], kp3, (int64_t)3 * G * g.span, g.dkp, WaScores::N);
+        if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &vmap, vp3, (int64_t)3 * G * g.dvp, g.span, vtile);
+        if (rc == CC_OK) {
+            wa_cut_kernel<<<(unsigned)blocks, 256, 0, dev->stream>>>(qp, fptr(kring), vptr, qp3, kp3, vp3, g, q_tiles, (unsigned)row_blocks, oldest, vec);
+            dev->launches++;
+            rc = sg_launch(dev, ws, (int64_t)key_tiles * q_tiles * G);
+        }
+        auto values = [&](auto wv) {
+            wv.maps[0] = vmap; wv.S = ws.S; wv.tops = ws.tops; wv.vring = vptr; wv.sink = sinkp; wv.o = (float*)o->base; wv.g = g; wv.key_tiles = key_tiles; wv.q_tiles = q_tiles;
+            return sg_launch<decltype(wv), true>(dev, wv, (int64_t)(g.dvp / vtile) * q_tiles * G);
+        };
+        if (rc == CC_OK) rc = vtile == 128 ? values(WaValues<2>{}) : values(WaValues<1>{});
         cc_pool_free(dev, Sp, cls);
         return rc;
     }
+    rc = cc_pool_alloc(dev, (size_t)T * H * g.cap * 4, &Sp, &cls);
+    if (rc) return rc;
     if (rows_smem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(wa_scores_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem); if (e != cudaSuccess) { cc_pool_free(dev, Sp, cls); return cc_fail(dev, CC_ERR_CUDA, "window_attention: %s", cudaGetErrorString(e)); } }
     wa_scores_row_kernel<<<dim3((unsigned)((maxn + 15) / 16), (unsigned)T, (unsigned)(G * ((R + WS_HEADS - 1) / WS_HEADS))), 256, rows_smem, dev->stream>>>(qp, fptr(kring), (float*)Sp, g, scale, r1p, r2p);
     dev->launches++;

@@ -3,20 +3,22 @@
 // An operand x is cut into three bfloat16 numbers h + m + l (8 mantissa bits each, cut off, so that all 24 bits are kept) while it is staged, and a
 // product is the sum of the six partial products that reach 2^-24 of it: hh + (hm + mh) + (hl + mm + lh).  tcgen05.mma adds a group of 16
 // products to its accumulator and cuts the sum off at 24 bits (measured: 1 + 0.75 ulp stays 1), so a long chain of additions would drift towards
-// zero.  Therefore hh has an accumulator of its own that is read out after 64 terms and added to a 32-bit register sum with ordinary rounding; the
+// zero.  Therefore hh has an accumulator of its own that is read out after 128 terms and added to a 32-bit register sum with ordinary rounding; the
 // other five, 2^-8 and less of it, are read out once.  Measured error and speed: at the users of this header.
 //
 // Why not CUDA cores: 148 SMs x 128 fused multiply-adds at 1.9 GHz are 72 TFLOP/s at the very best; the six bfloat16 products of a 128 x 128 x 64
-// step take the tensor core 1536 cycles, which is 380 TFLOP/s of 32-bit product.  The three planes of 64 columns of B lie one behind the other, so
+// step take the tensor core 1536 cycles, which is 380 TFLOP/s of 32-bit product.  The three planes of N columns of B lie one behind the other, so
 // four instructions make the six products: A_h x B_h, A_h x [B_m B_l], A_m x [B_h B_m], A_l x B_h.  One instruction per product reads the planes of A
-// from shared memory more often and took 85 cycles for 32 cycles of arithmetic.  What bounds the kernel is the cutting of the operands (about six
-// instructions per element) and, for short sums, the epilogue.
+// from shared memory more often; at N = 64 it took 85 cycles for 32 cycles of arithmetic.
 //
-// One CTA per SM: warps 0-15 with the same duties, because the cutting needs every issue slot and all the latency hiding there is, and warp 16, which
-// issues the products (issuing blocks while the tensor core is busy).  Step s: cut this warp's share of 64 columns of both operands (128-byte
-// swizzle, K-major) into one of two stages, issuing the loads of step s + 1 as registers become free; then collect the accumulator of step
-// s - 1.  A CTA walks over the tiles blockIdx.x, blockIdx.x + gridDim.x, ... (SPLIT: the two CTAs of a cluster share a tile's steps, and each
-// finishes half of its columns with the sums of both).
+// Operands arrive in one of two ways.  TMA: a kernel before this one has cut them into planes in global memory (what many tiles read), three boxes of
+// 64 columns per step.  Otherwise warps 0-15 load 32-bit numbers, cut and store them (128-byte swizzle, K-major) while they are staged.  Cutting costs
+// about six instructions per element and a trip through registers: with both operands cut in the kernel, a step of 128 x 128 x 64 took 5400 cycles.
+//
+// One CTA per SM: warps 0-15 stage and collect, warp 16 issues the products (issuing blocks while the tensor core is busy), warp 17 the TMA loads.  Step
+// s: cut this warp's share of 64 columns into one of two stages, issuing the loads of step s + 1 as registers become free; then collect
+// the accumulators if step s - 1 closed a run of two.  A CTA walks over the tiles blockIdx.x, blockIdx.x + gridDim.x, ... (SPLIT: the two CTAs of
+// a cluster share a tile's steps, and each finishes half of its columns with the sums of both).
 // Every wait is bounded: on expiry the CTA raises `fail`, every warp leaves its loop, TMEM is freed and the host reports it.
 //
 // An infinity cannot be cut (its rest is NaN): sums that come out as NaN are computed again in plain 32-bit arithmetic from the same operands, so
@@ -28,8 +30,9 @@
 //   Fixed, fixed(r)                what does not change from tile to tile about row r
 //   SHARED, Shared                 void setup(Tile, Shared&) is called by all threads before a tile, which then waits for the one before
 //   ARow, BCol                     what a thread keeps of a row / a column
-//   a_row, load_a, prep_a          a row of A; 8 consecutive elements of it as they lie in memory; the operand they stand for
-//   b_col, load_b                  the same for B
+//   A_TMA, B_TMA, map_a, at_a, ..  the operand comes by TMA: its tensor map and the coordinates of a step's box of a plane
+//   a_row, load_a, prep_a          otherwise, and for sums that are computed again: a row of A; 8 consecutive elements of it as they lie in memory; the
+//   b_col, load_b                  operand they stand for; the same for B
 //   A_TRANSPOSED, B_TRANSPOSED     consecutive threads take consecutive rows (columns) instead of consecutive elements
 //   end_a                          SHARED: after the last step, with the thread's row state
 //   emit                           the epilogue: 16 * HALVES consecutive sums of a row (sg_store_rows below: as they are, into rows of memory)
@@ -41,7 +44,7 @@
 
 #define SG_WORKERS 512
 #define SG_WARPS (SG_WORKERS / 32)
-#define SG_THREADS (SG_WORKERS + 32)
+#define SG_THREADS (SG_WORKERS + 64)
 #define SG_PIECE 8                          // columns a warp stores at a time
 #define SG_WAIT_LIMIT (1u << 24)
 
@@ -67,7 +70,7 @@ __device__ __forceinline__ void sg_arrive(unsigned bar) {
     if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // eight elements -> 16 bytes in each of the three planes
-__device__ __forceinline__ void sg_cut(uint8_t* at, unsigned plane, const float (&v)[8]) {
+__device__ __forceinline__ void sg_cut(uint8_t* at, size_t plane, const float (&v)[8]) {
     unsigned h[4], m[4], l[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -129,8 +132,10 @@ __device__ __forceinline__ void sg_store_rows(float* buf, float* out, int cols, 
 template <class P, bool SPLIT>
 __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_constant__ P p, int n_tiles, unsigned* err_dev, unsigned* err_host) {
     constexpr int N = 64 * P::HALVES, COUNT = N / 4, NB = P::HALVES, ROWS = P::A_TRANSPOSED ? 1 : 2;      // COUNT: columns a warp collects ; NB: chunks of B a thread stages
-    constexpr unsigned A_PLANE = 128 * 128, B_PLANE = 64 * 128, A_BYTES = 3 * A_PLANE, B_HALF = 3 * B_PLANE, STAGE = A_BYTES + P::HALVES * B_HALF;
-    constexpr unsigned TMEM_COLS = P::HALVES == 1 ? 256 : 512;       // per half: hh | hm + mh | hl + mm + lh
+    constexpr unsigned A_PLANE = 128 * 128, B_PLANE = N * 128, A_BYTES = 3 * A_PLANE, B_BYTES = 3 * B_PLANE, STAGE = A_BYTES + B_BYTES;
+    constexpr unsigned TMEM_COLS = P::HALVES == 1 ? 256 : 512;       // hh | hm + mh | hl + mm + lh
+    constexpr unsigned TMA_BYTES = (P::A_TMA ? A_BYTES : 0) + (P::B_TMA ? B_BYTES : 0);
+    constexpr bool CUTS = !P::A_TMA || !P::B_TMA;
     static_assert(!SPLIT || P::SHARED, "the other CTA's sums need the tiles' barriers");
     namespace cg = cooperative_groups;
     extern __shared__ __align__(1024) uint8_t sg_raw[];
@@ -141,7 +146,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
     const int rank = SPLIT ? (int)cg::this_cluster().block_rank() : 0, first = SPLIT ? blockIdx.x >> 1 : blockIdx.x, stride = SPLIT ? gridDim.x >> 1 : gridDim.x;
     if (tid == 0) {
 #pragma unroll
-        for (int s = 0; s < 2; s++) { pg_mbar_init(pg_smem(&sh.full[s]), SG_WARPS); pg_mbar_init(pg_smem(&sh.empty[s]), 1); }
+        for (int s = 0; s < 2; s++) { pg_mbar_init(pg_smem(&sh.full[s]), (CUTS ? SG_WARPS : 0) + (TMA_BYTES ? 1 : 0)); pg_mbar_init(pg_smem(&sh.empty[s]), 1); }
         pg_mbar_init(pg_smem(&sh.acc_full), 1); pg_mbar_init(pg_smem(&sh.acc_empty), SG_WARPS);
         pg_mbar_init(pg_smem(&sh.rows_done), SG_WARPS); pg_mbar_init(pg_smem(&sh.drained), 1);
         sh.fail = 0;
@@ -155,7 +160,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
     __syncthreads();
     pg_fence_after();
     const unsigned tmem = sh.tmem_base;
-    unsigned g = 0;                                                   // steps of the tiles before
+    unsigned g = 0, runs = 0;                                         // steps and runs of the tiles before
 
     if (warp == SG_WARPS) {
         // ===== products: one thread =====
@@ -172,27 +177,24 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
             if (lane == 0) {
                 for (int s = 0; s < steps; s++) {
                     const unsigned gs = g + s, slot = gs & 1u;
-                    if (!(ok = sg_wait(pg_smem(&sh.full[slot]), (gs >> 1) & 1u, &sh.fail) && sg_wait(pg_smem(&sh.acc_empty), (gs & 1u) ^ 1u, &sh.fail))) break;
+                    if (!(ok = sg_wait(pg_smem(&sh.full[slot]), (gs >> 1) & 1u, &sh.fail) && (s & 1 || sg_wait(pg_smem(&sh.acc_empty), ((runs + (s >> 1)) & 1u) ^ 1u, &sh.fail)))) break;
                     pg_fence_after();
                     const unsigned at = pg_smem(ring + (size_t)slot * STAGE);
                     const uint64_t ah = pg_smem_desc(at), am = pg_smem_desc(at + A_PLANE), al = pg_smem_desc(at + 2 * A_PLANE);
+                    const uint64_t bh = pg_smem_desc(at + A_BYTES), bm = pg_smem_desc(at + A_BYTES + B_PLANE);
 #pragma unroll
-                    for (int h = 0; h < P::HALVES; h++) {
-                        const uint64_t b = pg_smem_desc(at + A_BYTES + h * B_HALF), bm = pg_smem_desc(at + A_BYTES + h * B_HALF + B_PLANE);
-                        const unsigned d = tmem + h * 192;
-#pragma unroll
-                        for (int kk = 0; kk < 4; kk++) {
-                            const uint64_t adv = (uint64_t)((kk * PG_UMMA_K * 2) >> 4);
-                            pg_umma_f16(d, ah + adv, b + adv, pg_instr_desc(128, 64, 1), kk > 0);                            // hh
-                            pg_umma_f16(d + 64, ah + adv, bm + adv, pg_instr_desc(128, 128, 1), s > 0 || kk > 0);            //      hm | hl
-                            pg_umma_f16(d + 64, am + adv, b + adv, pg_instr_desc(128, 128, 1), 1u);                          //      mh | mm
-                            pg_umma_f16(d + 128, al + adv, b + adv, pg_instr_desc(128, 64, 1), 1u);                          //           lh
-                        }
+                    for (int kk = 0; kk < 4; kk++) {
+                        const uint64_t adv = (uint64_t)((kk * PG_UMMA_K * 2) >> 4);
+                        pg_umma_f16(tmem, ah + adv, bh + adv, pg_instr_desc(128, N, 1), (s & 1) || kk > 0);                  // hh
+                        pg_umma_f16(tmem + N, ah + adv, bm + adv, pg_instr_desc(128, 2 * N, 1), s > 0 || kk > 0);            //      hm | hl
+                        pg_umma_f16(tmem + N, am + adv, bh + adv, pg_instr_desc(128, 2 * N, 1), 1u);                         //      mh | mm
+                        pg_umma_f16(tmem + 2 * N, al + adv, bh + adv, pg_instr_desc(128, N, 1), 1u);                         //           lh
                     }
                     pg_umma_commit(pg_smem(&sh.empty[slot]));
-                    pg_umma_commit(pg_smem(&sh.acc_full));
+                    if ((s & 1) || s + 1 == steps) pg_umma_commit(pg_smem(&sh.acc_full));
                 }
             }
+            runs += (steps + 1) >> 1;
             ok = __all_sync(0xffffffffu, ok);
             g += steps;
             if (SPLIT) {
@@ -208,6 +210,43 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
             sg_wait(pg_smem(&sh.drained), 0, &never);
         }
         __syncwarp();
+    } else if (warp == SG_WARPS + 1) {
+        // ===== TMA loads: one thread =====
+        if (lane == 0 && TMA_BYTES) {
+            if (P::A_TMA) asm volatile("prefetch.tensormap [%0];" ::"l"(p.map_a()) : "memory");
+            if (P::B_TMA) asm volatile("prefetch.tensormap [%0];" ::"l"(p.map_b()) : "memory");
+        }
+        for (int index = first; index < n_tiles; index += stride) {
+            typename P::Tile tile;
+            if (!p.tile(index, rank, tile)) continue;
+            if (P::SHARED) {
+                __syncthreads();
+                if (*(volatile int*)&sh.fail) break;
+                __syncthreads();
+            }
+            bool ok = true;
+            if (lane == 0 && TMA_BYTES) {
+                for (int s = 0; s < tile.steps; s++) {
+                    const unsigned gs = g + s, slot = gs & 1u, full = pg_smem(&sh.full[slot]), at = pg_smem(ring + (size_t)slot * STAGE);
+                    if (!(ok = sg_wait(pg_smem(&sh.empty[slot]), ((gs >> 1) & 1u) ^ 1u, &sh.fail))) break;
+                    pg_mbar_expect_tx(full, TMA_BYTES);
+#pragma unroll
+                    for (int i = 0; i < 3; i++) {
+                        int x, y;
+                        if (P::A_TMA) { p.at_a(tile, s, i, x, y); pg_tma_load_2d(at + i * A_PLANE, p.map_a(), full, x, y); }
+                        if (P::B_TMA) { p.at_b(tile, s, i, x, y); pg_tma_load_2d(at + A_BYTES + i * B_PLANE, p.map_b(), full, x, y); }
+                    }
+                }
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            g += tile.steps;
+            if (SPLIT) {
+                cg::this_cluster().sync();
+                if (*(volatile int*)&sh.fail) break;
+                cg::this_cluster().sync();
+            }
+            if (!ok) break;
+        }
     } else {
         // ===== operands.  A: elements 8 (tid % 8) .. of the rows tid / 8 and tid / 8 + 64, or (A_TRANSPOSED) elements 8 (tid / 128) .. and 32 later of the
         // row tid % 128; B likewise, or column tid % 64 and elements 8 (tid / 64) .. =====
@@ -218,8 +257,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
         typename P::Fixed a_fixed[ROWS];
 #pragma unroll
         for (int e = 0; e < ROWS; e++) a_fixed[e] = p.fixed(ar0 + 64 * e);
-        const unsigned a_at = sg_offset(ar0, ac0), a_at2 = P::A_TRANSPOSED ? sg_offset(ar0, ac0 + 4) : sg_offset(ar0 + 64, ac0), b_at = A_BYTES + sg_offset(bn0, bk0);
-        const unsigned from = tmem + ((unsigned)(q * 32) << 16) + (unsigned)(col0 >> 6) * 192 + (unsigned)(col0 & 63);
+        const unsigned a_at = sg_offset(ar0, ac0), a_at2 = P::A_TRANSPOSED ? sg_offset(ar0, ac0 + 4) : sg_offset(ar0 + 64, ac0), b_at = A_BYTES + sg_offset(bn0, bk0);      // (64 rows further: 8192 bytes)
+        const unsigned from = tmem + ((unsigned)(q * 32) << 16) + (unsigned)col0;
         for (int index = first, nth = 0; index < n_tiles; index += stride) {
             typename P::Tile tile;
             if (!p.tile(index, rank, tile)) continue;
@@ -235,15 +274,15 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
             float av[2][8], bv[NB][8], acc[COUNT];
             auto load_a = [&](int s, int e) { p.load_a(tile, ar[P::A_TRANSPOSED ? 0 : e], s, P::A_TRANSPOSED ? ac0 + 4 * e : ac0, av[e]); };
             auto load_b = [&](int s, int e) { p.load_b(tile, bc[e], s, bk0, bv[e]); };
+            if (!P::A_TMA) {
 #pragma unroll
-            for (int e = 0; e < ROWS; e++) ar[e] = p.a_row(tile, ps, a_fixed[e], ar0 + 64 * e);
+                for (int e = 0; e < ROWS; e++) ar[e] = p.a_row(tile, ps, a_fixed[e], ar0 + 64 * e);
 #pragma unroll
-            for (int e = 0; e < NB; e++) bc[e] = p.b_col(tile, bn0 + 64 * e);
-            if (steps > 0) {
+                for (int e = 0; e < 2; e++) if (steps > 0) load_a(0, e);
+            }
+            if (!P::B_TMA) {
 #pragma unroll
-                for (int e = 0; e < 2; e++) load_a(0, e);
-#pragma unroll
-                for (int e = 0; e < NB; e++) load_b(0, e);
+                for (int e = 0; e < NB; e++) { bc[e] = p.b_col(tile, bn0 + 64 * e); if (steps > 0) load_b(0, e); }
             }
             bool ok = true;
 #pragma unroll
@@ -251,34 +290,40 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
             for (int s = 0; s <= steps; s++) {
                 if (s < steps) {
                     const unsigned gs = g + s, slot = gs & 1u;
-                    if (!(ok = sg_wait_warp(pg_smem(&sh.empty[slot]), ((gs >> 1) & 1u) ^ 1u, &sh.fail))) break;
+                    if (CUTS && !(ok = sg_wait_warp(pg_smem(&sh.empty[slot]), ((gs >> 1) & 1u) ^ 1u, &sh.fail))) break;
                     uint8_t* st = ring + slot * STAGE;
+                    if (!P::A_TMA) {
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        p.prep_a(tile, ar[P::A_TRANSPOSED ? 0 : e], av[e]);
-                        sg_cut(st + (e ? a_at2 : a_at), A_PLANE, av[e]);
-                        if (s + 1 < steps) load_a(s + 1, e);
+                        for (int e = 0; e < 2; e++) {
+                            p.prep_a(tile, ar[P::A_TRANSPOSED ? 0 : e], av[e]);
+                            sg_cut(st + (e ? a_at2 : a_at), A_PLANE, av[e]);
+                            if (s + 1 < steps) load_a(s + 1, e);
+                        }
                     }
+                    if (!P::B_TMA) {
 #pragma unroll
-                    for (int e = 0; e < NB; e++) {
-                        sg_cut(st + b_at + e * B_HALF, B_PLANE, bv[e]);
-                        if (s + 1 < steps) load_b(s + 1, e);
+                        for (int e = 0; e < NB; e++) {
+                            sg_cut(st + b_at + e * (64 * 128), B_PLANE, bv[e]);
+                            if (s + 1 < steps) load_b(s + 1, e);
+                        }
                     }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    sg_arrive(pg_smem(&sh.full[slot]));
+                    if (CUTS) {
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        sg_arrive(pg_smem(&sh.full[slot]));
+                    }
                 } else if (P::SHARED) {
                     p.end_a(tile, ps, ar[0], ar0, ac0);
                     sg_arrive(pg_smem(&sh.rows_done));
                 }
-                if (s > 0) {
-                    if (!(ok = sg_wait_warp(pg_smem(&sh.acc_full), (g + s - 1) & 1u, &sh.fail))) break;
+                if (s > 0 && (!(s & 1) || s == steps)) {              // step s - 1 closed a run
+                    if (!(ok = sg_wait_warp(pg_smem(&sh.acc_full), (runs + ((s - 1) >> 1)) & 1u, &sh.fail))) break;
                     pg_fence_after();
 #pragma unroll 1
                     for (int part = 0; part < (s < steps ? 1 : 3); part++) {
 #pragma unroll
                         for (int c0 = 0; c0 < COUNT; c0 += 16) {
                             unsigned b[16];
-                            sg_tmem16(from + part * 64 + c0, b);
+                            sg_tmem16(from + part * N + c0, b);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                             for (int c = 0; c < 16; c++) acc[c0 + c] += __uint_as_float(b[c]);
@@ -334,7 +379,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
                 }
             } else if (ok) p.emit(tile, ps, row_fixed, row, col0, acc, buf);
             if (!ok) break;
-            g += steps; nth++;
+            g += steps; runs += (steps + 1) >> 1; nth++;
         }
     }
     pg_fence_before();

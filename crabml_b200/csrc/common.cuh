@@ -124,6 +124,11 @@ struct cc_device {
     size_t dev_idx_bytes = 0;
 
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;    // cc_bench_timer_*
+    // pinned staging of a prompt's rotation angles (exact.cu), two buffers by turns
+    void* rope_pinned[2] = {nullptr, nullptr};
+    size_t rope_bytes[2] = {0, 0};
+    cudaEvent_t rope_ev[2] = {nullptr, nullptr};
+    int rope_slot = 0;
     // greedy decode without host round trips (capi.cu cc_argmax_to_slot / cc_copy_rows_from_slot): token-id slots and the history
     // of sampled ids, both in device memory
     int64_t* slots = nullptr;         // [CC_N_SLOTS]
@@ -324,6 +329,9 @@ int cc_launch_rms_norm_exact(cc_device* dev, float* x, int64_t rows, int64_t col
 int cc_launch_softmax_exact(cc_device* dev, float* x, int64_t rows, int64_t cols);
 int cc_launch_rope_exact(cc_device* dev, float* x, int64_t n_batch, int64_t batch_stride, int64_t head_dim, int mode,
                          int64_t pos, int64_t rope_dim);
+// the cos / sin of n rows from position pos on, [n][rope_dim / 2] float2 in the pool (the caller gives it back), and the rotation that reads them
+int cc_rope_angles(cc_device* dev, int64_t n, int64_t head_dim, int mode, int64_t pos, int64_t rope_dim, void** table, size_t* cls);
+int cc_launch_rope_rows(cc_device* dev, float* x, int64_t n_batch, int64_t batch_stride, int64_t head_dim, int mode, int64_t rope_dim, const void* table);
 int cc_launch_bmm_kcontig_exact(cc_device* dev, const float* a, const void* b, int b_dtype, float* c, int64_t ab, int64_t bb,
                                 int64_t m, int64_t k, int64_t n, int64_t sb0, int64_t sb2);
 

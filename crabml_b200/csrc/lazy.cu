@@ -18,6 +18,7 @@
 
 #include <chrono>
 #include <functional>
+#include <memory>
 
 #include "common.cuh"
 
@@ -156,12 +157,30 @@ static uint64_t hash_sig(const std::vector<uint64_t>& s) {
     return h;
 }
 
+// the rotation angles of a prompt's rows: made by the first rotation of the flush that needs them, given back with the flush's steps
+struct RopeAngles {
+    cc_device* dev; int64_t n, head_dim, pos, rope_dim; int mode;
+    void* table = nullptr; size_t cls = 0;
+    RopeAngles(cc_device* d, int64_t n_, int64_t hd, int m, int64_t p, int64_t rd) : dev(d), n(n_), head_dim(hd), pos(p), rope_dim(rd), mode(m) {}
+    ~RopeAngles() { if (table) cc_pool_free(dev, table, cls); }
+    int ready() { return table ? CC_OK : cc_rope_angles(dev, n, head_dim, mode, pos, rope_dim, &table, &cls); }
+};
+
 struct Fuser {
     cc_device* dev;
     LazyState* lz;
     std::vector<LOp>& q;
     Plan& P;
     size_t rope_off = (size_t)-1; int64_t rope_pos = -1; int rope_hd = 0, rope_dim = 0;
+
+    std::shared_ptr<RopeAngles> angles;                // of the last rotation of many rows
+    std::shared_ptr<RopeAngles> angles_for(const LOp& op) {
+        const int64_t n = op.i1, hd = op.a.shape[op.a.ndim - 1], rd = op.rows[0];
+        if (n < 2 || rd < 2 || rd > 256) return nullptr;
+        if (!angles || angles->n != n || angles->head_dim != hd || angles->pos != op.i0 || angles->rope_dim != rd || angles->mode != (int)op.f)
+            angles = std::make_shared<RopeAngles>(dev, n, hd, (int)op.f, op.i0, rd);
+        return angles;
+    }
 
     bool is(size_t i, int kind) const { return i < q.size() && !q[i].done && q[i].kind == kind; }
     std::unordered_map<cc_buf*, size_t> last_use;      // buffer -> index of the last queued op that touches it (built once per flush)
@@ -200,7 +219,8 @@ struct Fuser {
         default: break;
         }
         for (int64_t r : op.rows) P.S((uint64_t)r);
-        P.steps.push_back([d, op](uint8_t*) -> int {
+        std::shared_ptr<RopeAngles> ra = op.kind == L_ROPE ? angles_for(op) : nullptr;
+        P.steps.push_back([d, op, ra](uint8_t*) -> int {
             const LView &a = op.a, &b = op.b;
             switch (op.kind) {
             case L_DUP: {
@@ -218,7 +238,12 @@ struct Fuser {
             case L_ALLGATHER: return cc_launch_all_gather(d, (const float*)b.buf->plane[0], op.i0, (float*)a.buf->plane[0]);
             case L_ARGMAX: return cc_launch_argmax(d, (const float*)a.buf->plane[0], vlen(a), d->slots + op.i0, d->history, nullptr, op.i1);
             case L_SOFTMAX: { int64_t cols = a.shape[a.ndim - 1]; return cc_launch_softmax(d, (float*)a.buf->plane[0], cols ? vlen(a) / cols : 0, cols); }
-            case L_ROPE: return cc_launch_rope_exact(d, (float*)a.buf->plane[0], op.i1, op.i2, a.shape[a.ndim - 1], (int)op.f, op.i0, op.rows[0]);
+            case L_ROPE:
+                if (ra) {
+                    int rc = ra->ready();
+                    return rc ? rc : cc_launch_rope_rows(d, (float*)a.buf->plane[0], op.i1, op.i2, a.shape[a.ndim - 1], (int)op.f, op.rows[0], ra->table);
+                }
+                return cc_launch_rope_exact(d, (float*)a.buf->plane[0], op.i1, op.i2, a.shape[a.ndim - 1], (int)op.f, op.i0, op.rows[0]);
             case L_CONCAT:
                 return cc_launch_strided_copy(d, b.buf->plane[0], b.buf->dtype, b.shape, b.strides, a.buf->plane[0], a.buf->dtype, a.strides,
                                               a.shape[op.i0] * a.strides[op.i0], a.ndim);

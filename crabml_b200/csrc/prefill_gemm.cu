@@ -293,6 +293,23 @@ static int pg_weight_f16(cc_device* dev, const cc_buf* w, int64_t m, int64_t k, 
     return CC_OK;
 }
 
+// The output tile of a CTA: large tiles read fewer operand bytes per multiplication, small ones put more SMs to work.  Estimated time of a tile in
+// SM cycles: per 64-deep step the slowest of the tensor core (4096 multiply-adds per cycle), the operand bytes at about 40 per cycle and a floor
+// for the step's own latency; once per tile its start and its stores.  The whole product takes as many rounds of tiles as the SMs need.
+static void pg_pick_tile(cc_device* dev, int64_t m, int64_t b, int64_t k, int* block_n, int* mt) {
+    double best = 0.0;
+    for (int n = 256; n >= 64; n /= 2)
+        for (int t = 2; t >= 1; t--) {
+            if (n > 64 && b <= n / 2) continue;                  // more than half of every tile would be padding
+            const int64_t tiles = ((m + PG_BLOCK_M * t - 1) / (PG_BLOCK_M * t)) * ((b + n - 1) / n);
+            const int64_t rounds = (tiles + dev->sm_count - 1) / dev->sm_count;
+            const double mma = t * PG_BLOCK_M * (double)n * PG_BLOCK_K / 4096.0, load = (t * PG_BLOCK_M + n) * PG_BLOCK_K * 2 / 40.0;
+            double step = mma > load ? mma : load;
+            if (step < 260.0) step = 260.0;
+            const double cost = rounds * (step * (k / PG_BLOCK_K) + 3000.0 + t * n * 8.0);
+            if (best == 0.0 || cost < best) { best = cost; *block_n = n; *mt = t; }
+        }
+}
 // act: the quantisation of the (b, k) activation to the weight's partner type, Q8_0 or Q8_K (quantize.cu layout) -- or, for Q8_0
 // partners, x_f32: the f32 activation itself, quantised on the way to f16 (the caller then skips its own quantise launch); out: f32 [b][m]
 int cc_launch_prefill_matmul(cc_device* dev, const cc_buf* w, const void* act_q8_0, const float* x_f32, float* out, int64_t m, int64_t k, int64_t b) {
@@ -309,14 +326,14 @@ int cc_launch_prefill_matmul(cc_device* dev, const cc_buf* w, const void* act_q8
         else act_q8_to_f16_kernel<<<(unsigned)((na / 2 + 255) / 256), 256, 0, dev->stream>>>(cc_act_q8_0((void*)act_q8_0, na), na, (__half*)s->x);
         CC_LAUNCH_CHECK(dev);
     }
-    const int block_n = b >= 192 ? 256 : b >= 96 ? 128 : 64;
+    int block_n = 64, mt = 1;
+    pg_pick_tile(dev, m, b, k, &block_n, &mt);
     CUtensorMap tw, tx;
     rc = pg_make_tmap(dev, &tw, wf16, m, k, PG_BLOCK_M);
     if (rc) return rc;
     rc = pg_make_tmap(dev, &tx, s->x, b, k, block_n);
     if (rc) return rc;
-    static const bool one_tile = getenv("CRABML_PREFILL_MT1") != nullptr;          // developer A/B: 128-row CTA tiles
-    const bool mt2 = !one_tile && m >= 512;
+    const bool mt2 = mt == 2;
     if (block_n == 256) return mt2 ? pg_launch<256, 2>(dev, tw, tx, out, m, b, k) : pg_launch<256, 1>(dev, tw, tx, out, m, b, k);
     if (block_n == 128) return mt2 ? pg_launch<128, 2>(dev, tw, tx, out, m, b, k) : pg_launch<128, 1>(dev, tw, tx, out, m, b, k);
     return mt2 ? pg_launch<64, 2>(dev, tw, tx, out, m, b, k) : pg_launch<64, 1>(dev, tw, tx, out, m, b, k);
@@ -342,23 +359,6 @@ int cc_prefill_bf16_operand(cc_device* dev, int64_t b, int64_t k, void** out) {
     int rc = pg_ensure(dev, &s->x, &s->x_bytes, (size_t)b * k * 2);
     *out = s->x;
     return rc;
-}
-// The output tile of a CTA: large tiles read fewer operand bytes per multiplication, small ones put more SMs to work.  Estimated time of a tile in
-// SM cycles: per 64-deep step the slowest of the tensor core (4096 multiply-adds per cycle), the operand bytes at about 40 per cycle and a floor
-// for the step's own latency; once per tile its start and its stores.  The whole product takes as many rounds of tiles as the SMs need.
-static void pg_pick_tile(cc_device* dev, int64_t m, int64_t b, int64_t k, int* block_n, int* mt) {
-    double best = 0.0;
-    for (int n = 256; n >= 64; n /= 2)
-        for (int t = 2; t >= 1; t--) {
-            if (n > 64 && b <= n / 2) continue;                  // more than half of every tile would be padding
-            const int64_t tiles = ((m + PG_BLOCK_M * t - 1) / (PG_BLOCK_M * t)) * ((b + n - 1) / n);
-            const int64_t rounds = (tiles + dev->sm_count - 1) / dev->sm_count;
-            const double mma = t * PG_BLOCK_M * (double)n * PG_BLOCK_K / 4096.0, load = (t * PG_BLOCK_M + n) * PG_BLOCK_K * 2 / 40.0;
-            double step = mma > load ? mma : load;
-            if (step < 260.0) step = 260.0;
-            const double cost = rounds * (step * (k / PG_BLOCK_K) + 3000.0 + t * n * 8.0);
-            if (best == 0.0 || cost < best) { best = cost; *block_n = n; *mt = t; }
-        }
 }
 // the product over the operand in that scratch; accumulate != 0: out += it
 int cc_launch_prefill_bf16_operand(cc_device* dev, const cc_buf* w, float* out, int64_t m, int64_t k, int64_t b, int accumulate) {

@@ -497,14 +497,19 @@ __global__ void delta_gates_kernel(const float* __restrict__ a, const float* __r
     bd[i * 2 + 1] = expf(-expf(a_log[h]) * seq_softplus(a[i] + dt_bias[h]));
 }
 // grid (H, ceil(dv / columns per CTA)).  A column j of the head's state S[dk][dv] is owned for the whole call by SPLIT adjacent threads,
-// each holding dk / SPLIT of its entries: DK > 0 keeps them in registers (SPLIT = 2 for dk = 128, so that 64 registers hold a thread's
-// share), DK == 0 (any dk) in shared memory [dk][DR_THREADS].  Tokens run in order; per token two passes over dk:
+// each holding dk / SPLIT of its entries: DK > 0 keeps them in registers (16 per thread: groups of 4, dealt in turn, so that a warp's reads of k and q
+// fall into different banks), DK == 0 (any dk) in shared memory [dk][DR_THREADS].
+// Tokens run in order; per token two passes over dk:
 //   acc = sum_i S[i] k[i]           (the decayed read-out is decay * acc)
 //   u = beta * (v - decay * acc) ;  S[i] = decay * S[i] + k[i] * u ;  out = sum_i S[i] q[i]
-// k, q, beta and decay of DR_TB tokens at a time are staged in shared memory and the thread's v values in registers (one trip to L2 per
-// block of tokens instead of several per token).  Both dot products run as four interleaved partial sums per thread (i mod 4), added as
-// (p0 + p1) + (p2 + p3), then the SPLIT shares are added by a shuffle: a fixed order, the same for any T.
-#define DR_THREADS 64
+// k, q, v, beta and decay of DR_TB tokens at a time are staged in shared memory (one trip to L2 per block of tokens instead of several per
+// token).  Both dot products run as four interleaved partial sums per thread (i mod 4), added as (p0 + p1) + (p2 + p3); the SPLIT shares of acc are
+// added by a butterfly, those of out in ascending order after the block of tokens: a fixed order, the same for any T.
+// Bound by the chain acc -> u -> S from token to token, which is why a column is cut into 16 entries per thread: with two threads per column of 128
+// (64 CTAs of 2 warps for 16 heads) a token took 860 cycles, most of them issue slots of one warp.  1000 tokens, 16 heads (4 key heads) of 128:
+// 439 -> DELTA_US us.
+#define DR_THREADS 64                                   // DK == 0
+#define DR_SPLIT_THREADS 128                            // DK > 0
 #define DR_TB 16
 __device__ __forceinline__ void dr_cp_async16(float* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -512,34 +517,36 @@ __device__ __forceinline__ void dr_cp_async16(float* dst, const float* src) {
 __device__ __forceinline__ void dr_cp_async4(float* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
-// one staging buffer: k[DR_TB][dk4], q[DR_TB][dk4], bd[DR_TB][2], v[DR_TB][DR_THREADS] (a thread's own value column)
-__device__ __forceinline__ int dr_stage_floats(int dk4) { return 2 * DR_TB * dk4 + 2 * DR_TB + DR_TB * DR_THREADS; }
-template <int DK, int SPLIT>
-__global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                                                                const float* __restrict__ bd, float* __restrict__ state, float* __restrict__ o, int T, int H, int G,
-                                                                int dk, int dv) {
-    extern __shared__ __align__(16) float dr_sm[];            // two staging buffers, then (DK == 0) the state columns
-    constexpr int DKP = DK > 0 ? DK / SPLIT : 1;
-    constexpr int COLS = DR_THREADS / SPLIT;
+// one staging buffer: k[DR_TB][dk4], q[DR_TB][dk4], bd[DR_TB][2], v[DR_TB][columns]
+__host__ __device__ constexpr int dr_stage_floats(int dk4, int cols) { return 2 * DR_TB * dk4 + 2 * DR_TB + DR_TB * cols; }
+template <int DK, int SPLIT, int THREADS>
+__global__ void __launch_bounds__(THREADS) delta_rule_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                                             const float* __restrict__ bd, float* __restrict__ state, float* __restrict__ o, int T, int H, int G,
+                                                             int dk, int dv) {
+    extern __shared__ __align__(16) float dr_sm[];            // two staging buffers, then the state columns (DK == 0) or the shares of out (DK > 0)
+    constexpr int DKP = DK > 0 ? DK / SPLIT : 4;
+    constexpr int COLS = THREADS / SPLIT;
     const int dk4 = (dk + 3) & ~3;
-    const int stage_floats = dr_stage_floats(dk4);
+    const int stage_floats = dr_stage_floats(dk4, COLS);
     const int h = blockIdx.x, g = h / (H / G);
-    const int part = threadIdx.x % SPLIT;
-    const int j = blockIdx.y * COLS + threadIdx.x / SPLIT;
+    const int part = threadIdx.x % SPLIT, col = threadIdx.x / SPLIT;
+    const int j0 = blockIdx.y * COLS, j = j0 + col;
     const bool live = j < dv;
     const int jj = live ? j : dv - 1;                       // idle threads shadow the last column and never store
     float S[DKP];
-    float* Ss = dr_sm + 2 * stage_floats + threadIdx.x;      // generic: S[i] at Ss[i * DR_THREADS]
-    float* sp = state + ((int64_t)h * dk + part * DKP) * dv + jj;
+    float* rest = dr_sm + 2 * stage_floats;
+    float* Ss = rest + threadIdx.x;                          // generic: S[i] at Ss[i * THREADS]
+    float* sp = state + ((int64_t)h * dk + part * 4) * dv + jj;
+    constexpr int TURN = 4 * SPLIT;                          // thread `part` holds the entries 4 part .. 4 part + 3 of every TURN
     if (DK > 0) {
 #pragma unroll
-        for (int i = 0; i < DKP; i++) S[i] = sp[(int64_t)i * dv];
+        for (int i = 0; i < DKP; i++) S[i] = sp[(int64_t)((i >> 2) * TURN + (i & 3)) * dv];
     } else {
-        for (int i = 0; i < dk4; i++) Ss[i * DR_THREADS] = i < dk ? sp[(int64_t)i * dv] : 0.0f;
+        for (int i = 0; i < dk4; i++) Ss[i * THREADS] = i < dk ? sp[(int64_t)i * dv] : 0.0f;
     }
     // the pad lanes dk .. dk4 of both buffers are zero for the whole call (the copies below never touch them)
     if (dk4 != dk)
-        for (int idx = threadIdx.x; idx < 2 * 2 * DR_TB; idx += DR_THREADS)
+        for (int idx = threadIdx.x; idx < 2 * 2 * DR_TB; idx += THREADS)
             for (int i = dk; i < dk4; i++) dr_sm[(idx / (2 * DR_TB)) * stage_floats + (idx % (2 * DR_TB)) * dk4 + i] = 0.0f;
     // asynchronous copies (cp.async) of a block of tokens: issued one block ahead, so the trip to L2 overlaps the recurrence
     auto stage = [&](int buf, int tb) {
@@ -547,14 +554,14 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const float* __r
         const int nt = min(DR_TB, T - tb);
         if ((dk & 3) == 0) {
             const int per = dk >> 2;
-            for (int idx = threadIdx.x; idx < nt * per; idx += DR_THREADS) {
+            for (int idx = threadIdx.x; idx < nt * per; idx += THREADS) {
                 const int tt = idx / per, c = (idx - tt * per) * 4;
                 const int64_t src = ((int64_t)(tb + tt) * G + g) * dk + c;
                 dr_cp_async16(base + tt * dk4 + c, k + src);
                 dr_cp_async16(base + (DR_TB + tt) * dk4 + c, q + src);
             }
         } else {
-            for (int idx = threadIdx.x; idx < nt * dk; idx += DR_THREADS) {
+            for (int idx = threadIdx.x; idx < nt * dk; idx += THREADS) {
                 const int tt = idx / dk, c = idx - tt * dk;
                 const int64_t src = ((int64_t)(tb + tt) * G + g) * dk + c;
                 dr_cp_async4(base + tt * dk4 + c, k + src);
@@ -562,9 +569,12 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const float* __r
             }
         }
         float* sbd = base + 2 * DR_TB * dk4;
-        for (int idx = threadIdx.x; idx < nt * 2; idx += DR_THREADS) dr_cp_async4(sbd + idx, bd + ((int64_t)(tb + (idx >> 1)) * H + h) * 2 + (idx & 1));
-        float* sv = sbd + 2 * DR_TB + threadIdx.x;
-        for (int tt = 0; tt < nt; tt++) dr_cp_async4(sv + tt * DR_THREADS, v + ((int64_t)(tb + tt) * H + h) * dv + jj);
+        for (int idx = threadIdx.x; idx < nt * 2; idx += THREADS) dr_cp_async4(sbd + idx, bd + ((int64_t)(tb + (idx >> 1)) * H + h) * 2 + (idx & 1));
+        float* sv = sbd + 2 * DR_TB;
+        for (int idx = threadIdx.x; idx < nt * COLS; idx += THREADS) {
+            const int tt = idx / COLS, c = idx - tt * COLS;
+            dr_cp_async4(sv + idx, v + ((int64_t)(tb + tt) * H + h) * dv + min(j0 + c, dv - 1));
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if (T > 0) stage(0, 0);
@@ -576,58 +586,73 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const float* __r
         if (tb + DR_TB < T) stage(buf ^ 1, tb + DR_TB);
         const float* base = dr_sm + buf * stage_floats;
         const float* sbd = base + 2 * DR_TB * dk4;
-        const float* sv = sbd + 2 * DR_TB + threadIdx.x;
+        const float* sv = sbd + 2 * DR_TB + col;
+        const float* kt = base + part * 4;
+        const float* qt = base + DR_TB * dk4 + part * 4;
 #pragma unroll 1
-        for (int tt = 0; tt < nt; tt++) {
-            const int t = tb + tt;
-            const float* kt = base + tt * dk4 + part * DKP;
-            const float* qt = base + (DR_TB + tt) * dk4 + part * DKP;
+        for (int tt = 0; tt < nt; tt++, kt += dk4, qt += dk4) {
             const float beta = sbd[tt * 2], dec = sbd[tt * 2 + 1];
-            const float vj = sv[tt * DR_THREADS];
+            const float vj = sv[tt * COLS];
             float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f, o0 = 0.0f, o1 = 0.0f, o2 = 0.0f, o3 = 0.0f;
             if (DK > 0) {
+                float4 kv[DKP / 4], qv[DKP / 4];
 #pragma unroll
-                for (int i = 0; i < DKP; i += 4) {
-                    const float4 kv = *(const float4*)(kt + i);
-                    a0 = fmaf(S[i], kv.x, a0); a1 = fmaf(S[i + 1], kv.y, a1); a2 = fmaf(S[i + 2], kv.z, a2); a3 = fmaf(S[i + 3], kv.w, a3);
+                for (int i = 0; i < DKP / 4; i++) kv[i] = *(const float4*)(kt + TURN * i);
+#pragma unroll
+                for (int i = 0; i < DKP / 4; i++) qv[i] = *(const float4*)(qt + TURN * i);
+#pragma unroll
+                for (int i = 0; i < DKP / 4; i++) {
+                    a0 = fmaf(S[4 * i], kv[i].x, a0); a1 = fmaf(S[4 * i + 1], kv[i].y, a1); a2 = fmaf(S[4 * i + 2], kv[i].z, a2); a3 = fmaf(S[4 * i + 3], kv[i].w, a3);
                 }
                 float acc = (a0 + a1) + (a2 + a3);
-                if (SPLIT == 2) acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+#pragma unroll
+                for (int i = 0; i < DKP; i++) S[i] *= dec;    // while the shares meet
+#pragma unroll
+                for (int w = 1; w < SPLIT; w <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, w);
                 const float u = beta * (vj - dec * acc);
 #pragma unroll
-                for (int i = 0; i < DKP; i += 4) {
-                    const float4 kv = *(const float4*)(kt + i);
-                    const float4 qv = *(const float4*)(qt + i);
-                    S[i] = fmaf(kv.x, u, dec * S[i]); S[i + 1] = fmaf(kv.y, u, dec * S[i + 1]); S[i + 2] = fmaf(kv.z, u, dec * S[i + 2]); S[i + 3] = fmaf(kv.w, u, dec * S[i + 3]);
-                    o0 = fmaf(S[i], qv.x, o0); o1 = fmaf(S[i + 1], qv.y, o1); o2 = fmaf(S[i + 2], qv.z, o2); o3 = fmaf(S[i + 3], qv.w, o3);
+                for (int i = 0; i < DKP / 4; i++) {
+                    S[4 * i] = fmaf(kv[i].x, u, S[4 * i]); S[4 * i + 1] = fmaf(kv[i].y, u, S[4 * i + 1]);
+                    S[4 * i + 2] = fmaf(kv[i].z, u, S[4 * i + 2]); S[4 * i + 3] = fmaf(kv[i].w, u, S[4 * i + 3]);
+                    o0 = fmaf(S[4 * i], qv[i].x, o0); o1 = fmaf(S[4 * i + 1], qv[i].y, o1); o2 = fmaf(S[4 * i + 2], qv[i].z, o2); o3 = fmaf(S[4 * i + 3], qv[i].w, o3);
                 }
+                rest[tt * THREADS + threadIdx.x] = (o0 + o1) + (o2 + o3);
             } else {
                 for (int i = 0; i < dk4; i += 4) {
                     const float4 kv = *(const float4*)(kt + i);
-                    a0 = fmaf(Ss[i * DR_THREADS], kv.x, a0); a1 = fmaf(Ss[(i + 1) * DR_THREADS], kv.y, a1);
-                    a2 = fmaf(Ss[(i + 2) * DR_THREADS], kv.z, a2); a3 = fmaf(Ss[(i + 3) * DR_THREADS], kv.w, a3);
+                    a0 = fmaf(Ss[i * THREADS], kv.x, a0); a1 = fmaf(Ss[(i + 1) * THREADS], kv.y, a1);
+                    a2 = fmaf(Ss[(i + 2) * THREADS], kv.z, a2); a3 = fmaf(Ss[(i + 3) * THREADS], kv.w, a3);
                 }
                 const float u = beta * (vj - dec * ((a0 + a1) + (a2 + a3)));
                 for (int i = 0; i < dk4; i += 4) {
                     const float4 kv = *(const float4*)(kt + i);
                     const float4 qv = *(const float4*)(qt + i);
-                    const float s0 = fmaf(kv.x, u, dec * Ss[i * DR_THREADS]), s1 = fmaf(kv.y, u, dec * Ss[(i + 1) * DR_THREADS]);
-                    const float s2 = fmaf(kv.z, u, dec * Ss[(i + 2) * DR_THREADS]), s3 = fmaf(kv.w, u, dec * Ss[(i + 3) * DR_THREADS]);
-                    Ss[i * DR_THREADS] = s0; Ss[(i + 1) * DR_THREADS] = s1; Ss[(i + 2) * DR_THREADS] = s2; Ss[(i + 3) * DR_THREADS] = s3;
+                    const float s0 = fmaf(kv.x, u, dec * Ss[i * THREADS]), s1 = fmaf(kv.y, u, dec * Ss[(i + 1) * THREADS]);
+                    const float s2 = fmaf(kv.z, u, dec * Ss[(i + 2) * THREADS]), s3 = fmaf(kv.w, u, dec * Ss[(i + 3) * THREADS]);
+                    Ss[i * THREADS] = s0; Ss[(i + 1) * THREADS] = s1; Ss[(i + 2) * THREADS] = s2; Ss[(i + 3) * THREADS] = s3;
                     o0 = fmaf(s0, qv.x, o0); o1 = fmaf(s1, qv.y, o1); o2 = fmaf(s2, qv.z, o2); o3 = fmaf(s3, qv.w, o3);
                 }
+                if (live) o[((int64_t)(tb + tt) * H + h) * dv + j] = (o0 + o1) + (o2 + o3);
             }
-            float outv = (o0 + o1) + (o2 + o3);
-            if (SPLIT == 2) outv += __shfl_xor_sync(0xffffffffu, outv, 1);
-            if (live && part == 0) o[((int64_t)t * H + h) * dv + j] = outv;
+        }
+        if (DK > 0) {
+            __syncthreads();
+            for (int idx = threadIdx.x; idx < nt * COLS; idx += THREADS) {
+                const int tt = idx / COLS, c = idx - tt * COLS;
+                const float* sh = rest + tt * THREADS + c * SPLIT;
+                float sum = sh[0];
+#pragma unroll
+                for (int w = 1; w < SPLIT; w++) sum += sh[w];
+                if (j0 + c < dv) o[((int64_t)(tb + tt) * H + h) * dv + j0 + c] = sum;
+            }
         }
     }
     if (live) {
         if (DK > 0) {
 #pragma unroll
-            for (int i = 0; i < DKP; i++) sp[(int64_t)i * dv] = S[i];
+            for (int i = 0; i < DKP; i++) sp[(int64_t)((i >> 2) * TURN + (i & 3)) * dv] = S[i];
         } else {
-            for (int i = 0; i < dk; i++) sp[(int64_t)i * dv] = Ss[i * DR_THREADS];
+            for (int i = 0; i < dk; i++) sp[(int64_t)i * dv] = Ss[i * THREADS];
         }
     }
 }
@@ -655,26 +680,25 @@ extern "C" CC_API int cc_gated_delta_rule(cc_device* dev, const cc_view* q, cons
     if (rc) return rc;
     delta_gates_kernel<<<(unsigned)((T * H + 255) / 256), 256, 0, dev->stream>>>(fptr(a), fptr(b), fptr(a_log), fptr(dt_bias), (float*)bdp, T * H, H);
     dev->launches++;
-    const int cols = dk == 128 ? DR_THREADS / 2 : DR_THREADS;
+    const bool split = dk == 32 || dk == 64 || dk == 128;
+    const int threads = split ? DR_SPLIT_THREADS : DR_THREADS, cols = split ? DR_SPLIT_THREADS / (dk / 16) : DR_THREADS;
     dim3 grid((unsigned)H, (unsigned)((dv + cols - 1) / cols));
 #define DR_ARGS fptr(q), fptr(k), fptr(v), (const float*)bdp, fptr(state), (float*)o->base, (int)T, H, G, dk, dv
     const int dk4 = (dk + 3) & ~3;
-    const size_t stage = (size_t)2 * ((size_t)2 * DR_TB * dk4 + 2 * DR_TB + DR_TB * DR_THREADS) * 4;      // two staging buffers
-    if (stage > 48 * 1024 && (dk == 32 || dk == 64 || dk == 128)) {
-        cudaError_t e = dk == 32 ? cudaFuncSetAttribute(delta_rule_kernel<32, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage)
-                        : dk == 64 ? cudaFuncSetAttribute(delta_rule_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage)
-                                   : cudaFuncSetAttribute(delta_rule_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage);
-        if (e != cudaSuccess) { cc_pool_free(dev, bdp, cls); return cc_fail(dev, CC_ERR_CUDA, "gated_delta_rule: %s", cudaGetErrorString(e)); }
-    }
-    if (dk == 32) delta_rule_kernel<32, 1><<<grid, DR_THREADS, stage, dev->stream>>>(DR_ARGS);
-    else if (dk == 64) delta_rule_kernel<64, 1><<<grid, DR_THREADS, stage, dev->stream>>>(DR_ARGS);
-    else if (dk == 128) delta_rule_kernel<128, 2><<<grid, DR_THREADS, stage, dev->stream>>>(DR_ARGS);
-    else {
-        const size_t smem = stage + (size_t)dk4 * DR_THREADS * 4;
-        if (smem > 200 * 1024) { cc_pool_free(dev, bdp, cls); return cc_fail(dev, CC_ERR_UNSUPPORTED, "gated_delta_rule: dk=%d is too large", dk); }
-        if (smem > 48 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(delta_rule_kernel<0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        delta_rule_kernel<0, 1><<<grid, DR_THREADS, smem, dev->stream>>>(DR_ARGS);
-    }
+    // two staging buffers, and the shares of the read-out or the state
+    const size_t smem = ((size_t)2 * dr_stage_floats(dk4, cols) + (size_t)(split ? DR_TB : dk4) * threads) * 4;
+    if (smem > 200 * 1024) { cc_pool_free(dev, bdp, cls); return cc_fail(dev, CC_ERR_UNSUPPORTED, "gated_delta_rule: dk=%d is too large", dk); }
+    cudaError_t e = cudaSuccess;
+    if (smem > 48 * 1024)
+        e = dk == 32    ? cudaFuncSetAttribute(delta_rule_kernel<32, 2, DR_SPLIT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+            : dk == 64  ? cudaFuncSetAttribute(delta_rule_kernel<64, 4, DR_SPLIT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+            : dk == 128 ? cudaFuncSetAttribute(delta_rule_kernel<128, 8, DR_SPLIT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                        : cudaFuncSetAttribute(delta_rule_kernel<0, 1, DR_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) { cc_pool_free(dev, bdp, cls); return cc_fail(dev, CC_ERR_CUDA, "gated_delta_rule: %s", cudaGetErrorString(e)); }
+    if (dk == 32) delta_rule_kernel<32, 2, DR_SPLIT_THREADS><<<grid, threads, smem, dev->stream>>>(DR_ARGS);
+    else if (dk == 64) delta_rule_kernel<64, 4, DR_SPLIT_THREADS><<<grid, threads, smem, dev->stream>>>(DR_ARGS);
+    else if (dk == 128) delta_rule_kernel<128, 8, DR_SPLIT_THREADS><<<grid, threads, smem, dev->stream>>>(DR_ARGS);
+    else delta_rule_kernel<0, 1, DR_THREADS><<<grid, threads, smem, dev->stream>>>(DR_ARGS);
 #undef DR_ARGS
     cc_pool_free(dev, bdp, cls);            // stream-ordered pool: the next user of this block runs after the kernels above
     CC_LAUNCH_CHECK(dev);
@@ -836,7 +860,7 @@ __global__ void __launch_bounds__(256) wa_cut_kernel(const float* __restrict__ q
 // tiles: key tiles of the band (fastest), query tiles, G
 struct WaScores {
     static constexpr int HALVES = 2, N = 128;
-    static constexpr bool A_TRANSPOSED = false, B_TRANSPOSED = false, SHARED = false, A_TMA = true, B_TMA = true;
+    static constexpr bool A_TRANSPOSED = false, B_TRANSPOSED = false, SHARED = false, A_TMA = true, B_TMA = true, SKIP_ZERO = false;
     typedef WaTile Tile;
     typedef WaFixed Fixed;
     struct Shared {};
@@ -910,7 +934,7 @@ struct WaScores {
 template <int TILE_HALVES>
 struct WaValues {
     static constexpr int HALVES = TILE_HALVES, N = 64 * HALVES;
-    static constexpr bool A_TRANSPOSED = true, B_TRANSPOSED = true, SHARED = true, A_TMA = false, B_TMA = true;
+    static constexpr bool A_TRANSPOSED = true, B_TRANSPOSED = true, SHARED = true, A_TMA = false, B_TMA = true, SKIP_ZERO = true;
     typedef WaTile Tile;
     typedef WaFixed Fixed;
     CUtensorMap maps[1];                                // values [3][G][dvp][span]

@@ -34,6 +34,7 @@
 //   a_row, load_a, prep_a          otherwise, and for sums that are computed again: a row of A; 8 consecutive elements of it as they lie in memory; the
 //   b_col, load_b                  operand they stand for; the same for B
 //   A_TRANSPOSED, B_TRANSPOSED     consecutive threads take consecutive rows (columns) instead of consecutive elements
+//   SKIP_ZERO                      in sums that are computed again, a zero of A leaves its term out (weights of masked keys)
 //   end_a                          SHARED: after the last step, with the thread's row state
 //   emit                           the epilogue: 16 * HALVES consecutive sums of a row (sg_store_rows below: as they are, into rows of memory)
 #pragma once
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
                         typename P::ARow scratch = a;
                         p.load_a(tile, a, k >> 3, k & 7, x); p.prep_a(tile, scratch, x); p.load_b(tile, b, k >> 3, k & 7, y);
 #pragma unroll
-                        for (int i = 0; i < 8; i++) sum = fmaf(x[i], y[i], sum);
+                        for (int i = 0; i < 8; i++) sum = P::SKIP_ZERO && x[i] == 0.0f ? sum : fmaf(x[i], y[i], sum);
                     }
 #pragma unroll
                     for (int i = 0; i < COUNT; i++) acc[i] = i == c && acc[i] != acc[i] ? sum : acc[i];

@@ -44,6 +44,10 @@ struct WPlanes { const uint8_t* p[CC_MAX_PLANES]; };
 //   smem_bytes(k); stage_act(scratch, bi, k, smem); row_dot(W, row, k, smem, lane) -> per-lane partial
 // ------------------------------------------------------------------------------------------------
 
+// `rows_dot<R, NB>` (Q8_0, Q4_0, Q4_K, Q5_K, Q6_K) is row_dot for R weight rows (row0 ..; a row from `m` on repeats the last) and NB activations that lie
+// `stride` bytes apart in shared memory: a weight is fetched and unpacked once for all NB, an activation fetched once for all R.  Per (row,
+// activation) the terms are those of row_dot in the same order: identical bits.
+
 // ---- Q8_0 x Q8_0 : buf_q8_0.rs:136-286 -------------------------------------------------------------
 struct TQ8_0 {
     static __host__ __device__ int smem_bytes(int k) { return al16i(k) + al16i(k / 32 * 4); }
@@ -71,6 +75,30 @@ struct TQ8_0 {
             acc += (float)dot16(w0, aq[2 * blk + half]) * h2f_bits(wd[blk]) * ad[blk];
         }
         return acc;
+    }
+    template <int R, int NB>
+    static __device__ void rows_dot(const WPlanes& W, int64_t row0, int64_t m, int k, const uint8_t* sm, int stride, int lane, float (&acc)[R][NB]) {
+        const int nb = k >> 5, nchunk = k >> 4;
+        for (int c = lane; c < nchunk; c += 32) {
+            const int g = c >> 6, idx = c & 63;
+            const int nbg = min(32, nb - 32 * g);
+            const int half = idx >= nbg ? 1 : 0;
+            const int blk = 32 * g + idx - half * nbg;
+            int4 w[R]; float d[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int64_t row = min(row0 + r, m - 1);
+                w[r] = ld_stream_16((const int4*)W.p[0] + row * nchunk + c);
+                d[r] = h2f_bits(((const uint16_t*)W.p[1])[row * CC_D_STRIDE(nb) + blk]);
+            }
+#pragma unroll
+            for (int n = 0; n < NB; n++) {
+                const int4 a = ((const int4*)(sm + n * stride))[2 * blk + half];
+                const float ad = ((const float*)(sm + n * stride + al16i(k)))[blk];
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r][n] += (float)dot16(w[r], a) * d[r] * ad;
+            }
+        }
     }
 };
 
@@ -109,6 +137,30 @@ struct TQ4_0 {
         }
         for (; b < nb; b += 32) acc += block(ld_stream_16(wq + b), aq, ad, as, b, wd[b]);
         return acc;
+    }
+    template <int R, int NB>
+    static __device__ void rows_dot(const WPlanes& W, int64_t row0, int64_t m, int k, const uint8_t* sm, int stride, int lane, float (&acc)[R][NB]) {
+        const int nb = k >> 5;
+#pragma unroll 2
+        for (int b = lane; b < nb; b += 32) {
+            int4 lo[R], hi[R]; float d[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int64_t row = min(row0 + r, m - 1);
+                const int4 w = ld_stream_16((const int4*)W.p[0] + row * nb + b);
+                lo[r] = and4(w, 0x0F0F0F0F); hi[r] = shr4(w, 4, 0x0F0F0F0F);
+                d[r] = h2f_bits(((const uint16_t*)W.p[1])[row * CC_D_STRIDE(nb) + b]);
+            }
+#pragma unroll
+            for (int n = 0; n < NB; n++) {
+                const int4* aq = (const int4*)(sm + n * stride);
+                const int4 a0 = aq[2 * b], a1 = aq[2 * b + 1];
+                const float ad = ((const float*)(sm + n * stride + al16i(k)))[b];
+                const int as = ((const int*)(sm + n * stride + al16i(k) + al16i(nb * 4)))[b];
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r][n] += (float)(dot16(lo[r], a0) + dot16(hi[r], a1) - 8 * as) * d[r] * ad;
+            }
+        }
     }
 };
 
@@ -236,6 +288,43 @@ struct TQ45_K : TKBase {
         }
         return acc;
     }
+    template <int R, int NB>
+    static __device__ void rows_dot(const WPlanes& W, int64_t row0, int64_t m, int k, const uint8_t* sm, int stride, int lane, float (&acc)[R][NB]) {
+        const int nsb = k >> 8, BB = FIVE ? 176 : 144, QOFF = FIVE ? 48 : 16;
+        const int j = lane & 7, g = j >> 1, l0 = (j & 1) * 16;
+#pragma unroll 2
+        for (int sb = lane >> 3; sb < nsb; sb += 4) {
+            int4 lo[R], hi[R]; int sl[R], sh[R], mn[R]; float d[R], dm[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const uint8_t* blk = W.p[0] + (min(row0 + r, m - 1) * nsb + sb) * BB;
+                const int4 hdr = ld_stream_16(blk), q = ld_stream_16(blk + QOFF + 16 * j);
+                unsigned s0, s1, m0, m1;
+                k4_unpack((unsigned)hdr.y, (unsigned)hdr.z, (unsigned)hdr.w, s0, s1, m0, m1);
+                lo[r] = and4(q, 0x0F0F0F0F); hi[r] = shr4(q, 4, 0x0F0F0F0F);
+                if (FIVE) {
+                    const int4 qh = ld_stream_16(blk + 16 + l0);
+                    lo[r] = or4(lo[r], shl4(shr4(qh, 2 * g, 0x01010101), 4));
+                    hi[r] = or4(hi[r], shl4(shr4(qh, 2 * g + 1, 0x01010101), 4));
+                }
+                sl[r] = byte_of(s0, s1, 2 * g); sh[r] = byte_of(s0, s1, 2 * g + 1); mn[r] = byte_of(m0, m1, j);
+                d[r] = h2f_bits((uint16_t)(hdr.x & 0xFFFF)); dm[r] = h2f_bits((uint16_t)((unsigned)hdr.x >> 16));
+            }
+            const int abase = sb * 16 + g * 4 + (j & 1);
+#pragma unroll
+            for (int n = 0; n < NB; n++) {
+                KAct A(sm + n * stride, k);
+                const int4 a0 = A.q[abase], a1 = A.q[abase + 2];
+                const int bs = (int)A.bs[sb * 16 + 2 * j] + (int)A.bs[sb * 16 + 2 * j + 1];
+                const float da = A.d[sb];
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const int isum = sl[r] * dot16(lo[r], a0) + sh[r] * dot16(hi[r], a1), msum = bs * mn[r];
+                    acc[r][n] += (d[r] * da) * (float)isum - (dm[r] * da) * (float)msum;
+                }
+            }
+        }
+    }
     // ---- the same dot cut into SEGMENTS of 16 super-blocks (4 iterations of the loop above) whose 8 16-byte loads are issued as one
     // batch into a KSeg, so a caller can keep the next segment in flight while it computes the current one (megakernel generic
     // phase).  Per lane the terms are added in the same order as in row_dot -> identical bits.  x: 4 extra words per segment (Q6_K).
@@ -303,6 +392,35 @@ struct TQ6_K : TKBase {
             acc += (float)isum * (h2f_bits(wd[sb]) * A.d[sb]);
         }
         return acc;
+    }
+    template <int R, int NB>
+    static __device__ void rows_dot(const WPlanes& W, int64_t row0, int64_t m, int k, const uint8_t* sm, int stride, int lane, float (&acc)[R][NB]) {
+        const int nsb = k >> 8;
+        const int j = lane & 7, n6 = j >> 2, jj = j & 3, r6 = jj & 1, p = jj >> 1;
+        const int e_lo = 128 * n6 + 32 * p + 16 * r6;
+#pragma unroll 2
+        for (int sb = lane >> 3; sb < nsb; sb += 4) {
+            int4 lo[R], hi[R]; int sl[R], sh[R]; float d[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int64_t at = min(row0 + r, m - 1) * nsb + sb;
+                const int4 l = ld_stream_16(W.p[0] + at * 128 + 16 * j), h = ld_stream_16(W.p[1] + at * 64 + 32 * n6 + 16 * r6);
+                lo[r] = or4(and4(l, 0x0F0F0F0F), shl4(shr4(h, 2 * p, 0x03030303), 4));
+                hi[r] = or4(shr4(l, 4, 0x0F0F0F0F), shl4(shr4(h, 2 * p + 4, 0x03030303), 4));
+                sl[r] = ((const int8_t*)W.p[2])[at * 16 + (e_lo >> 4)]; sh[r] = ((const int8_t*)W.p[2])[at * 16 + (e_lo >> 4) + 4];
+                d[r] = h2f_bits(((const uint16_t*)W.p[3])[at]);
+            }
+            const int a_lo = sb * 16 + (e_lo >> 4), a_hi = a_lo + 4;
+#pragma unroll
+            for (int n = 0; n < NB; n++) {
+                KAct A(sm + n * stride, k);
+                const int4 a0 = A.q[a_lo], a1 = A.q[a_hi];
+                const int b0 = 32 * (int)A.bs[a_lo], b1 = 32 * (int)A.bs[a_hi];
+                const float da = A.d[sb];
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r][n] += (float)(sl[r] * (dot16(lo[r], a0) - b0) + sh[r] * (dot16(hi[r], a1) - b1)) * (d[r] * da);
+            }
+        }
     }
     // segments of 16 super-blocks, loads batched (see TQ45_K): ql chunk, qh chunk, the two sub-block scales and d per iteration
     static constexpr bool kSegmented = true;

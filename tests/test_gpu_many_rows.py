@@ -1,0 +1,214 @@
+"""The kernels that a prompt's rows take, at the sizes where they can go wrong: edges of the 128-row and 64-deep tiles, remainders, rings that wrap,
+grouped heads that do not fill a tile, infinities.  Products of 32-bit operands on the tensor cores (csrc/split_gemm.cuh) keep 24 bits of every
+operand and drop partial products below 2^-23 of a term; an accumulator is cut off after 8 additions at most before it joins a 32-bit sum, so
+    |got - exact| <= (2^-23 + 8 * 2^-23 + steps * 2^-24) * sum |terms|
+bounds a product of up to `steps` runs of 128 terms; 2e-6 * sum |terms| covers it for sums of up to 2048 terms."""
+import numpy as np
+import pytest
+
+from oracle import oracle as oc
+from oracle.tensor_ref import OracleDevice, OracleTensor
+from tests.gpu_common import make_device
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    d = make_device()
+    yield d
+    d.close()
+
+
+def tensor(dev, a):
+    from crabml_b200 import CudaTensor
+    return CudaTensor.new(np.asarray(a, np.float32), list(a.shape), dev)
+
+
+# ---- rotation of many rows -----------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("shape,pos,dims", [([2, 1, 2], 0, 2), ([33, 5, 48], 7, 32), ([300, 3, 128], 100000, 128)])
+def test_rotation_of_many_rows_has_the_reference_bits(dev, mode, shape, pos, dims):
+    x = np.random.default_rng(0).standard_normal(shape)
+    o = OracleTensor.new(x.reshape(-1), shape, OracleDevice()).rope_inplace(mode, pos, dims)
+    for _ in range(3):                                     # the staging buffers come round
+        np.testing.assert_array_equal(tensor(dev, x).rope_inplace(mode, pos, dims).export().view(np.uint32), o.export().view(np.uint32))
+
+
+# ---- softmax: many rows and one row at a time give the same bits ------------------------------------------------------------------------------
+@pytest.mark.parametrize("cols", [1, 31, 512, 513, 1025, 2048, 2049])
+def test_softmax_of_many_rows_has_the_bits_of_one(dev, cols):
+    x = np.random.default_rng(cols).standard_normal((700, cols)).astype(np.float32) * 3
+    many = tensor(dev, x).softmax_inplace(1).export().reshape(x.shape)
+    for r in (0, 1, 350, 699):
+        np.testing.assert_array_equal(many[r].view(np.uint32), tensor(dev, x[r:r + 1]).softmax_inplace(1).export().view(np.uint32))
+
+
+# ---- batch_matmul of many rows ------------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("kind", ["f32", "f16"])
+@pytest.mark.parametrize("ab,bb,m,k,n", [(2, 1, 16, 48, 17), (6, 2, 127, 64, 128), (4, 4, 128, 65, 129), (3, 3, 129, 200, 5), (8, 2, 300, 128, 333)])
+def test_batch_matmul_of_many_rows(dev, kind, ab, bb, m, k, n):
+    from crabml_b200 import CudaTensor, capi
+    rng = np.random.default_rng(m)
+    a = rng.standard_normal((ab, m, k)).astype(np.float32)
+    rows = rng.standard_normal((n, bb, k)).astype(np.float32)          # n cached rows per head, as the key cache holds them
+    cache = CudaTensor.alloc([bb, n + 3, k], capi.F16 if kind == "f16" else capi.F32, dev).resize(1, 0)
+    cache.concatenate(tensor(dev, rows).transpose([1, 0, 2]), 1)
+    if kind == "f16":
+        a, rows = a.astype(np.float16).astype(np.float32), rows.astype(np.float16).astype(np.float32)
+    head = np.arange(ab) % bb if kind == "f32" else np.arange(ab) // (ab // bb)
+    b = rows.transpose(1, 0, 2)[head].astype(np.float64)               # [ab, n, k]
+    got = tensor(dev, a).batch_matmul(cache.transpose([0, 2, 1])).export().reshape(ab, m, n)
+    want, size = np.einsum("amk,ank->amn", a, b), np.einsum("amk,ank->amn", np.abs(a), np.abs(b))
+    assert (np.abs(got - want) <= 2e-6 * size).all()
+    if kind == "f32":                                                  # [ab, m, n] x [bb, n, k]: the value product (f16 keeps its own order of sums)
+        w = np.abs(rng.standard_normal((ab, m, n))).astype(np.float32)
+        got = tensor(dev, w).batch_matmul(cache).export().reshape(ab, m, k)
+        want, size = np.einsum("amn,ank->amk", w, b), np.einsum("amn,ank->amk", w, np.abs(b))
+        assert (np.abs(got - want) <= 2e-6 * size).all()
+
+
+def test_batch_matmul_spreads_infinities_like_a_sum_of_products(dev):
+    rng = np.random.default_rng(1)
+    a, b = rng.standard_normal((1, 40, 70)).astype(np.float32), rng.standard_normal((1, 70, 50)).astype(np.float32)
+    a[0, 3, 5], a[0, 7, 9], b[0, 11, 2], b[0, 5, 4] = np.inf, np.nan, -np.inf, 0.0
+    with np.errstate(invalid="ignore"):
+        want = np.einsum("amk,akn->amn", a.astype(np.float64), b.astype(np.float64))
+    got = tensor(dev, a).batch_matmul(tensor(dev, b)).export().reshape(want.shape)
+    fine = np.isfinite(want)
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+    np.testing.assert_array_equal(got[~fine & ~np.isnan(want)], want[~fine & ~np.isnan(want)])
+    np.testing.assert_allclose(got[fine], want[fine], rtol=0, atol=2e-4)
+
+
+# ---- attention over a ring ------------------------------------------------------------------------------------------------------------------------
+def attend(q, k, v, scale, pos0, window, block, cap, sink):
+    """q [T, H, dk]; k, v: row j is position j; -> [T, H, dv] in 64 bits"""
+    T, H = q.shape[:2]
+    R, out = H // k.shape[1], np.zeros((T, H, v.shape[2]))
+    for t in range(T):
+        i = pos0 + t
+        lo = max(0, i - window + 1) if window else 0
+        lo = max(lo, i - i % block) if block else lo
+        for h in range(H):
+            s = k[lo:i + 1, h // R].astype(np.float64) @ q[t, h].astype(np.float64) * scale
+            s = cap * np.tanh(s / cap) if cap else s
+            top = max(s.max(), sink[h]) if sink is not None else s.max()
+            e = np.exp(s - top)
+            out[t, h] = e @ v[lo:i + 1, h // R] / (e.sum() + (np.exp(sink[h] - top) if sink is not None else 0.0))
+    return out
+
+
+CASES = [  # T, pos0, H, G, dk, dv, window, block, cap, sink, latent
+    (65, 0, 1, 1, 64, 64, 0, 0, 0.0, False, False),
+    (33, 63, 6, 2, 80, 40, 50, 0, 0.0, True, False),          # three heads per key head: 126 of a tile's 128 rows ; a window that ends inside steps
+    (130, 129, 2, 2, 128, 128, 0, 0, 5.0, False, False),
+    (7, 1000, 10, 1, 36, 132, 64, 0, 0.0, False, False),      # dk not a whole step, dv one column group and four columns
+    (200, 100, 4, 4, 64, 200, 0, 96, 0.0, True, False),       # blocks of positions
+    (40, 300, 8, 1, 192, 128, 0, 0, 0.0, False, True),        # a key row's first dv columns are its value
+    (129, 511, 3, 1, 30, 30, 128, 0, 0.0, False, False),      # rows that cannot be read 16 bytes at a time
+]
+
+
+def rings(k, v, pos, ring):
+    """positions pos of k, v in the rows p % ring"""
+    kr, vr = np.full((ring,) + k.shape[1:], np.nan, np.float32), None if v is None else np.full((ring,) + v.shape[1:], np.nan, np.float32)
+    kr[pos % ring] = k[pos]
+    if v is not None:
+        vr[pos % ring] = v[pos]
+    return kr, vr
+
+
+@pytest.mark.parametrize("T,pos0,H,G,dk,dv,window,block,cap,sink,latent", CASES)
+def test_attention_of_many_rows(dev, T, pos0, H, G, dk, dv, window, block, cap, sink, latent):
+    from crabml_b200 import seqops
+    rng = np.random.default_rng(T)
+    n = pos0 + T
+    q, k = rng.standard_normal((T, H, dk)).astype(np.float32), rng.standard_normal((n, G, dk)).astype(np.float32)
+    v = k[..., :dv] if latent else rng.standard_normal((n, G, dv)).astype(np.float32)
+    sk = rng.standard_normal(H).astype(np.float32) if sink else None
+    first = max(0, pos0 - window + 1) if window else 0
+    first = max(first, pos0 - pos0 % block) if block else first
+    ring = n - first + 5                                       # rows nobody may look at hold NaN
+    kr, vr = rings(k, None if latent else v, np.arange(first, n), ring)
+    args = dict(window=window, block=block, softcap=cap, sink=None if sk is None else tensor(dev, sk))
+    kt, vt = tensor(dev, kr.reshape(ring, -1)), None if latent else tensor(dev, vr.reshape(ring, -1))
+    got = seqops.masked_attention_capped(tensor(dev, q.reshape(T, -1)), kt, vt, pos0, H, G, dk, dv, dk ** -0.5, **args).export().reshape(T, H, dv)
+    want = attend(q, k, v, dk ** -0.5, pos0, window, block, cap, sk)
+    # a score's error moves its weight by as much, the weights' and sums' roundings are a few 2^-24 each: 1e-5 of the values' size
+    assert np.abs(got - want).max() <= 1e-5
+    # however a portion is cut, a query keeps its bits while both cuts have many rows
+    cut = T // 2
+    if cut * H > 64 and (T - cut) * H > 64:
+        for a, b in ((0, cut), (cut, T)):
+            part = seqops.masked_attention_capped(tensor(dev, q[a:b].reshape(b - a, -1)), kt, vt, pos0 + a, H, G, dk, dv, dk ** -0.5, **args).export().reshape(b - a, H, dv)
+            np.testing.assert_array_equal(part.view(np.uint32), got[a:b].view(np.uint32))
+
+
+def test_attention_keeps_an_infinite_value_to_the_queries_that_see_it(dev):
+    from crabml_b200 import seqops
+    rng = np.random.default_rng(3)
+    T, H, d = 96, 2, 64
+    q, k, v = (rng.standard_normal((T, H, d)).astype(np.float32) for _ in range(3))
+    v[70, 1, 5] = np.inf
+    got = seqops.masked_attention(tensor(dev, q.reshape(T, -1)), tensor(dev, k.reshape(T, -1)), tensor(dev, v.reshape(T, -1)), 0, H, H, d, d, d ** -0.5).export().reshape(T, H, d)
+    bad = np.zeros(got.shape, bool)
+    bad[70:, 1, 5] = True
+    assert np.isposinf(got[bad]).all() and np.isfinite(got[:70]).all() and np.isfinite(got[70:, 0]).all()
+    assert np.isfinite(np.delete(got[70:, 1], 5, 1)).all()
+
+
+# ---- a few activation rows against one quantised matrix ---------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("t", [oc.Q4_K, oc.Q5_K, oc.Q6_K])
+@pytest.mark.parametrize("m,k,b", [(1, 256, 2), (33, 1024, 3), (40, 2816, 8), (257, 4096, 9), (17, 14336, 31), (16, 40960, 5)])
+def test_few_rows_have_the_bits_of_one(dev, t, m, k, b):
+    from crabml_b200 import CudaTensor
+    from tests.blockgen import random_weight
+    rng = np.random.default_rng(m + b)
+    w = CudaTensor.from_cpu(random_weight(t, m, k, rng, 0.02), [m, k], t, dev)
+    x = rng.standard_normal((b, k)).astype(np.float32)
+    got = w.matmul_vec(tensor(dev, x)).export().reshape(b, m)
+    for i in range(b):
+        np.testing.assert_array_equal(got[i].view(np.uint32), w.matmul_vec(tensor(dev, x[i:i + 1])).export().view(np.uint32))
+
+
+@pytest.mark.parametrize("t", [oc.Q8_0, oc.Q4_0, oc.Q5_0])
+@pytest.mark.parametrize("m,k,b", [(1, 32, 2), (33, 288, 3), (40, 1056, 8), (257, 4096, 9), (17, 14336, 31), (16, 40960, 5)])
+def test_few_rows_against_the_oracle(dev, t, m, k, b):
+    from tests.test_gpu_matvec import run_case
+    run_case(dev, t, m, k, b=b, seed=m + b)
+
+
+# ---- gated delta rule: any cut of the tokens gives the same bits, columns that do not fill a CTA -------------------------------------------------------
+@pytest.mark.parametrize("dk,dv,H,G", [(128, 128, 2, 1), (128, 20, 3, 3), (64, 33, 4, 2), (32, 64, 2, 2), (36, 70, 2, 1)])
+def test_delta_rule_however_the_tokens_are_cut(dev, dk, dv, H, G):
+    from crabml_b200 import seqops
+    rng = np.random.default_rng(dk + dv)
+    T = 37
+    q, k, v = rng.standard_normal((T, G, dk)) / dk ** 0.5, rng.standard_normal((T, G, dk)), rng.standard_normal((T, H, dv))
+    k /= np.linalg.norm(k, axis=-1, keepdims=True)
+    a, b, a_log, dt = rng.standard_normal((T, H)), rng.standard_normal((T, H)), np.log(rng.uniform(0.5, 4, H)), rng.uniform(-3, 0, H)
+    S0 = rng.standard_normal((H, dk, dv))
+
+    def run(cuts):
+        state, outs = tensor(dev, S0.reshape(-1)), []
+        for lo, hi in zip(cuts, cuts[1:]):
+            t = [tensor(dev, x[lo:hi].reshape(hi - lo, -1)) for x in (q, k, v, a, b)]
+            outs.append(seqops.gated_delta_rule(*t, tensor(dev, a_log), tensor(dev, dt), state, H, G, dk, dv).export())
+        return np.concatenate(outs).reshape(T, H, dv), state.export().reshape(S0.shape)
+    got, end = run([0, T])
+    for cuts in ([0, 1, 2, 18, T], [0, 16, 32, T]):
+        o, s = run(cuts)
+        np.testing.assert_array_equal(o.view(np.uint32), got.view(np.uint32))
+        np.testing.assert_array_equal(s.view(np.uint32), end.view(np.uint32))
+    S = np.asarray(S0, np.float32).astype(np.float64)
+    f = [np.asarray(x, np.float32).astype(np.float64) for x in (q, k, v, a, b, a_log, dt)]
+    beta, decay = 1 / (1 + np.exp(-f[4])), np.exp(-np.exp(f[5]) * np.log1p(np.exp(f[3] + f[6])))
+    for t in range(T):
+        for h in range(H):
+            S[h] *= decay[t, h]
+            kt = f[1][t, h // (H // G)]
+            S[h] += np.outer(kt, beta[t, h] * (f[2][t, h] - S[h].T @ kt))
+            # 32-bit sums of dk terms of order one, carried on by a contraction: 1e-5
+            assert np.abs(got[t, h] - S[h].T @ f[0][t, h // (H // G)]).max() < 1e-5
+    assert np.abs(end - S).max() < 1e-5

@@ -156,6 +156,40 @@ __global__ void strided_copy_kernel(const void* src, int src_dtype, void* dst, i
     else if (src_dtype == CC_F32 && dst_dtype == CC_F16) ((__half*)dst)[dof] = __float2half_rn(((const float*)src)[so]);   // f16::from_f32
     else ((float*)dst)[dof] = __half2float(((const __half*)src)[so]);
 }
+// the case of every cache append and head turn: f32 to f32, rows of unit stride, whose starts are 16-byte aligned on both sides -- a thread moves 16 bytes and
+// finds its place with 32-bit divisions.  [512, 32, 128] -> [32, 512, 128] (8 MB): 35 -> COPY_US us
+struct CopyDims32 { unsigned shape[CC_MAX_DIMS], sstr[CC_MAX_DIMS], dstr[CC_MAX_DIMS]; int ndim; };      // last axis and strides in units of 4 elements
+__global__ void __launch_bounds__(256) strided_copy16_kernel(const float4* __restrict__ src, float4* __restrict__ dst, CopyDims32 d, unsigned total) {
+    const unsigned i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= total) return;
+    unsigned rem = i, so = 0, dof = 0;
+#pragma unroll
+    for (int ax = CC_MAX_DIMS - 1; ax >= 0; ax--) {
+        if (ax >= d.ndim) continue;
+        const unsigned q = rem / d.shape[ax], c = rem - q * d.shape[ax];
+        rem = q;
+        so += c * d.sstr[ax];
+        dof += c * d.dstr[ax];
+    }
+    dst[dof] = src[so];
+}
+// whether the copy above may take it; fills d
+static bool copy16(const void* src, int src_dtype, const int64_t* sshape, const int64_t* sstrides, const void* dst, int dst_dtype, const int64_t* dstrides, int64_t dst_offset, int ndim,
+                   CopyDims32* d) {
+    if (src_dtype != CC_F32 || dst_dtype != CC_F32 || ndim < 1 || sstrides[ndim - 1] != 1 || dstrides[ndim - 1] != 1 || sshape[ndim - 1] % 4) return false;
+    if ((((uintptr_t)src | (uintptr_t)((const float*)dst + dst_offset)) & 15) != 0) return false;
+    int64_t smax = 0, dmax = 0;
+    d->ndim = ndim;
+    for (int i = 0; i < ndim; i++) {
+        if (sstrides[i] < 0 || dstrides[i] < 0) return false;
+        if (i + 1 < ndim && sshape[i] > 1 && (sstrides[i] % 4 || dstrides[i] % 4)) return false;
+        smax += (sshape[i] - 1) * sstrides[i]; dmax += (sshape[i] - 1) * dstrides[i];
+        d->shape[i] = (unsigned)(i + 1 < ndim ? sshape[i] : sshape[i] / 4);
+        d->sstr[i] = i + 1 < ndim ? (unsigned)(sstrides[i] / 4) : 1u;
+        d->dstr[i] = i + 1 < ndim ? (unsigned)(dstrides[i] / 4) : 1u;
+    }
+    return smax < ((int64_t)1 << 31) && dmax < ((int64_t)1 << 31);
+}
 int cc_launch_strided_copy(cc_device* dev, const void* src, int src_dtype, const int64_t* sshape, const int64_t* sstrides,
                            void* dst, int dst_dtype, const int64_t* dstrides, int64_t dst_offset, int ndim) {
     CopyDims d;
@@ -163,6 +197,13 @@ int cc_launch_strided_copy(cc_device* dev, const void* src, int src_dtype, const
     int64_t total = 1;
     for (int i = 0; i < ndim; i++) { d.shape[i] = sshape[i]; d.sstr[i] = sstrides[i]; d.dstr[i] = dstrides[i]; total *= sshape[i]; }
     if (total == 0) return CC_OK;
+    CopyDims32 d32;
+    if (total < ((int64_t)1 << 31) && copy16(src, src_dtype, sshape, sstrides, dst, dst_dtype, dstrides, dst_offset, ndim, &d32)) {
+        const unsigned n = (unsigned)(total / 4);
+        strided_copy16_kernel<<<(n + 255) / 256, 256, 0, dev->stream>>>((const float4*)src, (float4*)((float*)dst + dst_offset), d32, n);
+        CC_LAUNCH_CHECK(dev);
+        return CC_OK;
+    }
     strided_copy_kernel<<<(unsigned)((total + 255) / 256), 256, 0, dev->stream>>>(src, src_dtype, dst, dst_dtype, d, dst_offset, total);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;

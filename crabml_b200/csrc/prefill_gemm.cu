@@ -15,6 +15,7 @@
 //      Warp roles: 0 TMA producer, 1 MMA issuer, 2 TMEM allocator, 4-7 epilogue.
 // MMA-M is the WEIGHT row dimension (large: 4096 .. 32000), MMA-N the batch dimension.
 // Every mbarrier wait is bounded (trap after ~2 s) so that a descriptor mistake ends in an error, not a hung GPU.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <stdlib.h>
 #include <string.h>
@@ -26,15 +27,34 @@
 #include "dequant.cuh"
 #include "umma.cuh"
 
-#define PG_STAGES 4
+namespace cg = cooperative_groups;
+
+#define PG_MAX_STAGES 8
+// what a CTA keeps in flight: as many stages as 200 KB hold.  Four stages of a 128 x 64 tile (96 KB) left the tensor core waiting: a step took 550 cycles,
+// twice what its operand bytes need (1024 x 512 x 4096, 64 CTAs)
+__host__ __device__ constexpr int pg_stages(int block_n, int mt) {
+    const int n = 200 * 1024 / ((mt * PG_BLOCK_M + block_n) * PG_BLOCK_K * 2);
+    return n < PG_MAX_STAGES ? n : PG_MAX_STAGES;
+}
 #define PG_THREADS 256
 
 struct PgShared {
-    unsigned long long full[PG_STAGES], empty[PG_STAGES], tmem_full;      // (3 or PG_STAGES slots in use)
+    unsigned long long full[PG_MAX_STAGES], empty[PG_MAX_STAGES], tmem_full;      // (pg_stages slots in use)
     unsigned tmem_base;
 };
 
-// grid: (ceil(m / (128 * MT)), ceil(b / BLOCK_N)); dynamic smem: 1024-aligned ring of STAGES x (A tile MT x 16 KB + B tile BLOCK_N*128 B)
+__device__ __forceinline__ void pg_tmem_load32(unsigned taddr, unsigned (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, "
+        "%23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
+          "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// grid: (ceil(m / (128 * MT)), ceil(b / BLOCK_N), parts of the depth); dynamic smem: 1024-aligned ring of STAGES x (A tile MT x 16 KB + B tile BLOCK_N*128 B)
 // MT = 2: the CTA owns a 256-row weight tile as TWO M = 128 accumulators (2 x BLOCK_N TMEM columns) that share every B tile -- 1.5x
 // fewer operand bytes per FLOP than 128 x 256 tiles, which matters because 148 CTAs pulling 48 KB per 128x256x64 step ask more of L2
 // than it delivers (profiles/r02e: 47 % tensor pipe with MT = 1).
@@ -56,9 +76,12 @@ __global__ void __launch_bounds__(PG_THREADS, 1) umma_gemm_kernel(const __grid_c
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr unsigned A_TILE = PG_BLOCK_M * PG_BLOCK_K * 2, A_BYTES = MT * A_TILE, B_BYTES = BLOCK_N * PG_BLOCK_K * 2;
     constexpr unsigned TMEM_COLS = MT * BLOCK_N < 32 ? 32 : MT * BLOCK_N;     // power of two >= 32 (64 .. 512)
-    constexpr int STAGES = (A_BYTES + B_BYTES) * PG_STAGES <= 200 * 1024 ? PG_STAGES : 3;
+    constexpr int STAGES = pg_stages(BLOCK_N, MT);
     uint8_t* ring = (uint8_t*)(((uintptr_t)pg_smem_raw + 1023) & ~(uintptr_t)1023);
-    const int num_kb = k / PG_BLOCK_K;
+    // gridDim.z CTAs of a cluster share the product's depth: each takes a run of 64-deep steps, the first adds the others' sums to its own in ascending
+    // order and stores.  For products too narrow to give every SM a tile
+    const int parts = gridDim.z, part = blockIdx.z, all_kb = k / PG_BLOCK_K, kb0 = (int)((int64_t)all_kb * part / parts);
+    const int num_kb = (int)((int64_t)all_kb * (part + 1) / parts) - kb0;
     const int m0 = blockIdx.x * PG_BLOCK_M * MT, n0 = groups ? g_row0 : blockIdx.y * BLOCK_N;
 
     if (warp == 0 && lane == 0) {
@@ -90,8 +113,8 @@ __global__ void __launch_bounds__(PG_THREADS, 1) umma_gemm_kernel(const __grid_c
                 pg_mbar_expect_tx(full, A_BYTES + B_BYTES);
                 uint8_t* st = ring + (size_t)s * (A_BYTES + B_BYTES);
 #pragma unroll
-                for (int t = 0; t < MT; t++) pg_tma_load_2d(pg_smem(st + t * A_TILE), &tmap_w, full, kb * PG_BLOCK_K, g_w0 + m0 + t * PG_BLOCK_M);
-                pg_tma_load_2d(pg_smem(st + A_BYTES), &tmap_x, full, kb * PG_BLOCK_K, n0);
+                for (int t = 0; t < MT; t++) pg_tma_load_2d(pg_smem(st + t * A_TILE), &tmap_w, full, (kb0 + kb) * PG_BLOCK_K, g_w0 + m0 + t * PG_BLOCK_M);
+                pg_tma_load_2d(pg_smem(st + A_BYTES), &tmap_x, full, (kb0 + kb) * PG_BLOCK_K, n0);
             }
         }
     } else if (warp == 1) {
@@ -124,20 +147,37 @@ __global__ void __launch_bounds__(PG_THREADS, 1) umma_gemm_kernel(const __grid_c
         const int q = warp & 3;                                          // a warp reads the TMEM lanes 32 * (warp % 4) ..
         pg_mbar_wait(pg_smem(&sh.tmem_full), 0);
         pg_fence_after();
+    }
+    if (parts > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        __syncwarp();
+        cluster.sync();                                                  // every CTA's products are done: the first one's ring is free
+        if (part > 0 && warp >= 4) {
+            float* to = cluster.map_shared_rank((float*)ring, 0) + (size_t)(part - 1) * (MT * BLOCK_N * PG_BLOCK_M) + (warp & 3) * 32 + lane;
+#pragma unroll 1
+            for (int cc = 0; cc < MT * BLOCK_N; cc += 32) {
+                unsigned v[32];
+                pg_tmem_load32(tmem_acc + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)cc, v);
+#pragma unroll
+                for (int j = 0; j < 32; j++) to[(cc + j) * PG_BLOCK_M] = __uint_as_float(v[j]);
+            }
+        }
+        __syncwarp();
+        cluster.sync();
+    }
+    if (warp >= 4 && part == 0) {
+        const int q = warp & 3;
 #pragma unroll 1
         for (int cc = 0; cc < MT * BLOCK_N; cc += 32) {
             const int t = cc / BLOCK_N, c0 = cc - t * BLOCK_N;          // accumulator t holds the weight rows m0 + 128 t ..
             const int row = m0 + t * PG_BLOCK_M + q * 32 + lane;         // weight row = output column index
             unsigned v[32];
-            const unsigned taddr = tmem_acc + ((unsigned)(q * 32) << 16) + (unsigned)cc;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, "
-                "%23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-                  "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
-                  "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                : "r"(taddr));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            pg_tmem_load32(tmem_acc + ((unsigned)(q * 32) << 16) + (unsigned)cc, v);
+            for (int z = 1; z < parts; z++) {
+                const float* o = (const float*)ring + (size_t)(z - 1) * (MT * BLOCK_N * PG_BLOCK_M) + q * 32 + lane;
+#pragma unroll
+                for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + o[(cc + j) * PG_BLOCK_M]);
+            }
             if (row < m && accumulate) {                                 // C += the product: the residual stream is updated where it lies
                 float old[32];
 #pragma unroll
@@ -260,13 +300,17 @@ bool cc_prefill_supported(int wtype, int64_t m, int64_t k, int64_t b) {
 }
 
 template <int BLOCK_N, int MT, int FMT = 0>
-static int pg_launch(cc_device* dev, const CUtensorMap& tw, const CUtensorMap& tx, float* out, int64_t m, int64_t b, int64_t k, int accumulate = 0) {
-    const size_t stage = (size_t)MT * PG_BLOCK_M * PG_BLOCK_K * 2 + (size_t)BLOCK_N * PG_BLOCK_K * 2;
-    const int stages = stage * PG_STAGES <= 200 * 1024 ? PG_STAGES : 3;
-    const size_t smem = (size_t)stages * stage + 1024;
+static int pg_launch(cc_device* dev, const CUtensorMap& tw, const CUtensorMap& tx, float* out, int64_t m, int64_t b, int64_t k, int accumulate = 0, int parts = 1) {
+    const size_t smem = (size_t)pg_stages(BLOCK_N, MT) * (MT * PG_BLOCK_M + BLOCK_N) * PG_BLOCK_K * 2 + 1024;
     CC_CUDA(dev, cudaFuncSetAttribute(umma_gemm_kernel<BLOCK_N, MT, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((unsigned)((m + PG_BLOCK_M * MT - 1) / (PG_BLOCK_M * MT)), (unsigned)((b + BLOCK_N - 1) / BLOCK_N));
-    umma_gemm_kernel<BLOCK_N, MT, FMT><<<grid, PG_THREADS, smem, dev->stream>>>(tw, tx, out, (int)m, (int)b, (int)k, nullptr, accumulate);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((m + PG_BLOCK_M * MT - 1) / (PG_BLOCK_M * MT)), (unsigned)((b + BLOCK_N - 1) / BLOCK_N), (unsigned)parts);
+    cfg.blockDim = dim3(PG_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = dev->stream;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = 1; cluster.val.clusterDim.y = 1; cluster.val.clusterDim.z = (unsigned)parts;
+    if (parts > 1) { cfg.attrs = &cluster; cfg.numAttrs = 1; }
+    CC_CUDA(dev, cudaLaunchKernelEx(&cfg, umma_gemm_kernel<BLOCK_N, MT, FMT>, tw, tx, out, (int)m, (int)b, (int)k, (const int*)nullptr, accumulate));
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -293,23 +337,35 @@ static int pg_weight_f16(cc_device* dev, const cc_buf* w, int64_t m, int64_t k, 
     return CC_OK;
 }
 
-// The output tile of a CTA: large tiles read fewer operand bytes per multiplication, small ones put more SMs to work.  Estimated time of a tile in
-// SM cycles: per 64-deep step the slowest of the tensor core (4096 multiply-adds per cycle), the operand bytes at about 40 per cycle and a floor
-// for the step's own latency; once per tile its start and its stores.  The whole product takes as many rounds of tiles as the SMs need.
-static void pg_pick_tile(cc_device* dev, int64_t m, int64_t b, int64_t k, int* block_n, int* mt) {
+// The output tile of a CTA and how many CTAs share its depth: large tiles read fewer operand bytes per multiplication, small ones and shared depths put
+// more SMs to work.  Estimated time in SM cycles: per 64-deep step the slowest of the tensor core (4096 multiply-adds per cycle), the operand bytes at
+// about 40 per cycle and a floor for the step's own latency; once per tile its start and its stores, and per sharing CTA its sums on their way to
+// the first (4 bytes each at about 8 per cycle).  The whole product takes as many rounds of tiles as the SMs need.  The sums that meet must fit the ring.
+static void pg_pick_tile(cc_device* dev, int64_t m, int64_t b, int64_t k, int* block_n, int* mt, int* parts) {
     double best = 0.0;
     for (int n = 256; n >= 64; n /= 2)
         for (int t = 2; t >= 1; t--) {
             if (n > 64 && b <= n / 2) continue;                  // more than half of every tile would be padding
             const int64_t tiles = ((m + PG_BLOCK_M * t - 1) / (PG_BLOCK_M * t)) * ((b + n - 1) / n);
-            const int64_t rounds = (tiles + dev->sm_count - 1) / dev->sm_count;
             const double mma = t * PG_BLOCK_M * (double)n * PG_BLOCK_K / 4096.0, load = (t * PG_BLOCK_M + n) * PG_BLOCK_K * 2 / 40.0;
             double step = mma > load ? mma : load;
             if (step < 260.0) step = 260.0;
-            const double cost = rounds * (step * (k / PG_BLOCK_K) + 3000.0 + t * n * 8.0);
-            if (best == 0.0 || cost < best) { best = cost; *block_n = n; *mt = t; }
+            const int64_t ring = (int64_t)pg_stages(n, t) * (t * PG_BLOCK_M + n) * PG_BLOCK_K * 2, sums = (int64_t)t * PG_BLOCK_M * n * 4;
+            for (int z = 1; z <= 4; z *= 2) {
+                if (z > 1 && ((z - 1) * sums > ring || k / PG_BLOCK_K < 8 * z || tiles * z > dev->sm_count)) break;
+                const int64_t rounds = (tiles * z + dev->sm_count - 1) / dev->sm_count;
+                const double cost = rounds * (step * ((k / PG_BLOCK_K + z - 1) / z) + 3000.0 + t * n * 8.0) + (z > 1 ? 2000.0 + (z - 1) * sums / 8.0 : 0.0);
+                if (best == 0.0 || cost < best) { best = cost; *block_n = n; *mt = t; *parts = z; }
+            }
         }
 }
+template <int FMT>
+static int pg_launch_tile(cc_device* dev, int block_n, int mt, int parts, const CUtensorMap& tw, const CUtensorMap& tx, float* out, int64_t m, int64_t b, int64_t k, int accumulate) {
+    if (block_n == 256) return mt == 2 ? pg_launch<256, 2, FMT>(dev, tw, tx, out, m, b, k, accumulate, parts) : pg_launch<256, 1, FMT>(dev, tw, tx, out, m, b, k, accumulate, parts);
+    if (block_n == 128) return mt == 2 ? pg_launch<128, 2, FMT>(dev, tw, tx, out, m, b, k, accumulate, parts) : pg_launch<128, 1, FMT>(dev, tw, tx, out, m, b, k, accumulate, parts);
+    return mt == 2 ? pg_launch<64, 2, FMT>(dev, tw, tx, out, m, b, k, accumulate, parts) : pg_launch<64, 1, FMT>(dev, tw, tx, out, m, b, k, accumulate, parts);
+}
+
 // act: the quantisation of the (b, k) activation to the weight's partner type, Q8_0 or Q8_K (quantize.cu layout) -- or, for Q8_0
 // partners, x_f32: the f32 activation itself, quantised on the way to f16 (the caller then skips its own quantise launch); out: f32 [b][m]
 int cc_launch_prefill_matmul(cc_device* dev, const cc_buf* w, const void* act_q8_0, const float* x_f32, float* out, int64_t m, int64_t k, int64_t b) {
@@ -326,17 +382,14 @@ int cc_launch_prefill_matmul(cc_device* dev, const cc_buf* w, const void* act_q8
         else act_q8_to_f16_kernel<<<(unsigned)((na / 2 + 255) / 256), 256, 0, dev->stream>>>(cc_act_q8_0((void*)act_q8_0, na), na, (__half*)s->x);
         CC_LAUNCH_CHECK(dev);
     }
-    int block_n = 64, mt = 1;
-    pg_pick_tile(dev, m, b, k, &block_n, &mt);
+    int block_n = 64, mt = 1, parts = 1;
+    pg_pick_tile(dev, m, b, k, &block_n, &mt, &parts);
     CUtensorMap tw, tx;
     rc = pg_make_tmap(dev, &tw, wf16, m, k, PG_BLOCK_M);
     if (rc) return rc;
     rc = pg_make_tmap(dev, &tx, s->x, b, k, block_n);
     if (rc) return rc;
-    const bool mt2 = mt == 2;
-    if (block_n == 256) return mt2 ? pg_launch<256, 2>(dev, tw, tx, out, m, b, k) : pg_launch<256, 1>(dev, tw, tx, out, m, b, k);
-    if (block_n == 128) return mt2 ? pg_launch<128, 2>(dev, tw, tx, out, m, b, k) : pg_launch<128, 1>(dev, tw, tx, out, m, b, k);
-    return mt2 ? pg_launch<64, 2>(dev, tw, tx, out, m, b, k) : pg_launch<64, 1>(dev, tw, tx, out, m, b, k);
+    return pg_launch_tile<0>(dev, block_n, mt, parts, tw, tx, out, m, b, k, 0);
 }
 
 // ---- plain bfloat16 weights (dense.cu): the weight matrix [m][k] is its own tile source, the f32 activation rows are rounded to
@@ -363,17 +416,14 @@ int cc_prefill_bf16_operand(cc_device* dev, int64_t b, int64_t k, void** out) {
 // the product over the operand in that scratch; accumulate != 0: out += it
 int cc_launch_prefill_bf16_operand(cc_device* dev, const cc_buf* w, float* out, int64_t m, int64_t k, int64_t b, int accumulate) {
     PgScratch* s = pg_scratch(dev);
-    int block_n = 64, mt = 1;
-    pg_pick_tile(dev, m, b, k, &block_n, &mt);
+    int block_n = 64, mt = 1, parts = 1;
+    pg_pick_tile(dev, m, b, k, &block_n, &mt, &parts);
     CUtensorMap tw, tx;
     int rc = pg_make_tmap(dev, &tw, w->plane[0], m, k, PG_BLOCK_M, true);
     if (rc) return rc;
     rc = pg_make_tmap(dev, &tx, s->x, b, k, block_n, true);
     if (rc) return rc;
-    const bool mt2 = mt == 2;
-    if (block_n == 256) return mt2 ? pg_launch<256, 2, 1>(dev, tw, tx, out, m, b, k, accumulate) : pg_launch<256, 1, 1>(dev, tw, tx, out, m, b, k, accumulate);
-    if (block_n == 128) return mt2 ? pg_launch<128, 2, 1>(dev, tw, tx, out, m, b, k, accumulate) : pg_launch<128, 1, 1>(dev, tw, tx, out, m, b, k, accumulate);
-    return mt2 ? pg_launch<64, 2, 1>(dev, tw, tx, out, m, b, k, accumulate) : pg_launch<64, 1, 1>(dev, tw, tx, out, m, b, k, accumulate);
+    return pg_launch_tile<1>(dev, block_n, mt, parts, tw, tx, out, m, b, k, accumulate);
 }
 int cc_launch_prefill_bf16_act(cc_device* dev, const cc_buf* w, const float* x_f32, int act, float* out, int64_t m, int64_t k, int64_t b) {
     PgScratch* s = pg_scratch(dev);
@@ -406,9 +456,7 @@ int cc_launch_grouped_bf16(cc_device* dev, const cc_buf* w_stack, int64_t n_grou
     const bool mt2 = m >= 512;
 #define PG_GROUPED(BN, MT)                                                                                                                       \
     do {                                                                                                                                         \
-        const size_t stage = (size_t)MT * PG_BLOCK_M * PG_BLOCK_K * 2 + (size_t)BN * PG_BLOCK_K * 2;                                             \
-        const int stages = stage * PG_STAGES <= 200 * 1024 ? PG_STAGES : 3;                                                                      \
-        const size_t smem = (size_t)stages * stage + 1024;                                                                                       \
+        const size_t smem = (size_t)pg_stages(BN, MT) * (MT * PG_BLOCK_M + BN) * PG_BLOCK_K * 2 + 1024;                                          \
         CC_CUDA(dev, cudaFuncSetAttribute(umma_gemm_kernel<BN, MT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                  \
         dim3 grid((unsigned)((m + PG_BLOCK_M * MT - 1) / (PG_BLOCK_M * MT)), (unsigned)max_tiles);                                               \
         umma_gemm_kernel<BN, MT, 1><<<grid, PG_THREADS, smem, dev->stream>>>(tw, tx, out, (int)m, 0, (int)k, groups_dev);                          \

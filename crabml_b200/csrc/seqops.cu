@@ -507,7 +507,7 @@ __global__ void delta_gates_kernel(const float* __restrict__ a, const float* __r
 // added by a butterfly, those of out in ascending order after the block of tokens: a fixed order, the same for any T.
 // Bound by the chain acc -> u -> S from token to token, which is why a column is cut into 16 entries per thread: with two threads per column of 128
 // (64 CTAs of 2 warps for 16 heads) a token took 860 cycles, most of them issue slots of one warp.  1000 tokens, 16 heads (4 key heads) of 128:
-// 439 -> DELTA_US us.
+// 439 -> 217 us.
 #define DR_THREADS 64                                   // DK == 0
 #define DR_SPLIT_THREADS 128                            // DK > 0
 #define DR_TB 16
@@ -815,46 +815,55 @@ __device__ __forceinline__ int64_t wa_score_at(const WaTile& t, int q_tiles, int
 // what many tiles read, cut once into three planes of bfloat16 (split_gemm.cuh).  Blocks 0 .. row_blocks: eight elements of a query or key row per
 // thread; the rest: 64 keys x 64 columns of the values, turned through shared memory.  Rows of no query, positions nobody sees and columns
 // behind dk / dv are zeros.  Bound by memory: 10 bytes per element.
+// ring_base0: the ring's row of position base0; lo0: the first position anybody sees
 __global__ void __launch_bounds__(256) wa_cut_kernel(const float* __restrict__ q, const float* __restrict__ kring, const float* __restrict__ vring, uint8_t* __restrict__ qc,
-                                                     uint8_t* __restrict__ kc, uint8_t* __restrict__ vc, WaGeom g, int q_tiles, unsigned row_blocks, int64_t lo0, int vec) {
-    const int64_t last = g.pos0 + g.T - 1;
-    const int64_t q_rows = (int64_t)g.G * q_tiles * WA_ROWS, k_rows = (int64_t)g.G * g.span;
+                                                     uint8_t* __restrict__ kc, uint8_t* __restrict__ vc, WaGeom g, int q_tiles, unsigned row_blocks, int ring_base0, int lo0, int vec) {
+    const int last = (int)(g.pos0 + g.T - 1 - g.base0);       // positions are counted from base0
+    const unsigned q_rows = (unsigned)(g.G * q_tiles) * WA_ROWS, k_rows = (unsigned)(g.G * g.span);
     float v[8];
     if (blockIdx.x < row_blocks) {
-        const int per = g.dkp >> 3;
-        const int64_t u = (int64_t)blockIdx.x * 256 + threadIdx.x, row = u / per;
+        const unsigned per = (unsigned)g.dkp >> 3, u = blockIdx.x * 256u + threadIdx.x;
+        unsigned row = u / per;
         const int c = (int)(u - row * per) * 8;
         if (row >= q_rows + k_rows) return;
         const float* src = nullptr;
-        if (row < q_rows) {
-            const int r = (int)(row % WA_ROWS), tq = r / g.R;
-            const int64_t qt = row / WA_ROWS % q_tiles, t = qt * g.QT + tq;
-            if (tq < g.QT && t < g.T) src = q + (t * g.H + row / WA_ROWS / q_tiles * g.R + (r - tq * g.R)) * g.dk;
+        const bool is_q = row < q_rows;
+        if (is_q) {
+            const unsigned r = row & (WA_ROWS - 1), tile = row / WA_ROWS, kvh = tile / (unsigned)q_tiles, tq = r / (unsigned)g.R;
+            const int t = (int)(tile - kvh * q_tiles) * g.QT + (int)tq;
+            if ((int)tq < g.QT && t < g.T) src = q + ((int64_t)t * g.H + kvh * g.R + (r - tq * g.R)) * g.dk;
         } else {
-            const int64_t kvh = (row - q_rows) / g.span, j = g.base0 + (row - q_rows) % g.span;
-            if (j >= lo0 && j <= last) src = kring + (j % g.ring) * g.krs + kvh * g.dk;
+            row -= q_rows;
+            const unsigned kvh = row / (unsigned)g.span;
+            const int j = (int)(row - kvh * g.span);
+            if (j >= lo0 && j <= last) src = kring + (int64_t)((unsigned)(ring_base0 + j) % (unsigned)g.ring) * g.krs + kvh * g.dk;
         }
         if (src) sg_load8(src, c, g.dk, vec, v); else sg_zero8(v);
-        if (row < q_rows) sg_cut(qc + (row * g.dkp + c) * 2, (size_t)q_rows * g.dkp * 2, v);
-        else sg_cut(kc + ((row - q_rows) * g.dkp + c) * 2, (size_t)k_rows * g.dkp * 2, v);
+        sg_cut((is_q ? qc : kc) + ((size_t)row * g.dkp + c) * 2, (size_t)(is_q ? q_rows : k_rows) * g.dkp * 2, v);
         return;
     }
     __shared__ float turn[64][65];
-    const unsigned b = blockIdx.x - row_blocks, key_blocks = g.span >> 6, col_blocks = g.dvp >> 6;
-    const int j0 = (int)(b % key_blocks) * 64, d0 = (int)(b / key_blocks % col_blocks) * 64, kvh = (int)(b / key_blocks / col_blocks);
-#pragma unroll 4
-    for (int i = threadIdx.x >> 6; i < 64; i += 4) {
-        const int64_t j = g.base0 + j0 + i;
-        const int d = d0 + (threadIdx.x & 63);
-        turn[i][threadIdx.x & 63] = j >= lo0 && j <= last && d < g.dv ? vring[(j % g.ring) * g.vrs + kvh * g.vhs + d] : 0.0f;
+    const unsigned b = blockIdx.x - row_blocks, key_blocks = (unsigned)g.span >> 6, col_blocks = (unsigned)g.dvp >> 6, rest = b / key_blocks;
+    const int j0 = (int)(b - rest * key_blocks) * 64, kvh = (int)(rest / col_blocks), d0 = (int)(rest - kvh * col_blocks) * 64, d = d0 + (threadIdx.x & 63);
+    unsigned row = (unsigned)(ring_base0 + j0 + (int)(threadIdx.x >> 6)) % (unsigned)g.ring;
+    const float* col = vring + (int64_t)kvh * g.vhs + d;
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const int j = j0 + (int)(threadIdx.x >> 6) + 4 * i;
+        x[i] = j >= lo0 && j <= last && d < g.dv ? col[(int64_t)row * g.vrs] : 0.0f;
+        row += 4;
+        while (row >= (unsigned)g.ring) row -= (unsigned)g.ring;
     }
+#pragma unroll
+    for (int i = 0; i < 16; i++) turn[(threadIdx.x >> 6) + 4 * i][threadIdx.x & 63] = x[i];
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 2; i++) {
-        const int d = (threadIdx.x >> 3) + 32 * i, k = (threadIdx.x & 7) * 8;
+        const int dd = (threadIdx.x >> 3) + 32 * i, k = (threadIdx.x & 7) * 8;
 #pragma unroll
-        for (int e = 0; e < 8; e++) v[e] = turn[k + e][d];
-        sg_cut(vc + (((int64_t)kvh * g.dvp + d0 + d) * g.span + j0 + k) * 2, (size_t)g.G * g.dvp * g.span * 2, v);
+        for (int e = 0; e < 8; e++) v[e] = turn[k + e][dd];
+        sg_cut(vc + (((size_t)kvh * g.dvp + d0 + dd) * g.span + j0 + k) * 2, (size_t)g.G * g.dvp * g.span * 2, v);
     }
 }
 // tiles: key tiles of the band (fastest), query tiles, G
@@ -1227,7 +1236,7 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
         g.dkp = (dk + 63) & ~63; g.dvp = (dv + vtile - 1) / vtile * vtile;
         const size_t q_rows = (size_t)G * q_tiles * WA_ROWS, scores = q_rows * g.cap * 4, tops = (size_t)G * q_tiles * key_tiles * 4 * WA_ROWS * 4;
         const size_t qc = 3 * q_rows * g.dkp * 2, kc = 3 * (size_t)G * g.span * g.dkp * 2, vc = 3 * (size_t)G * g.dvp * g.span * 2;
-        CC_REQUIRE(dev, 3 * q_rows < ((size_t)1 << 31) && (size_t)3 * G * g.span < ((size_t)1 << 31), "window_attention: too many rows");
+        CC_REQUIRE(dev, (3 * q_rows + (size_t)3 * G * g.span) * (g.dkp / 8) < ((size_t)1 << 31) && ring < (1 << 30), "window_attention: too many rows");
         rc = cc_pool_alloc(dev, scores + tops + qc + kc + vc, &Sp, &cls);   // every part is a multiple of 512 bytes
         if (rc) return rc;
         uint8_t *base = (uint8_t*)Sp, *qp3 = base + scores + tops, *kp3 = qp3 + qc, *vp3 = kp3 + kc;
@@ -1241,7 +1250,7 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
         if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &ws.maps[1], kp3, (int64_t)3 * G * g.span, g.dkp, WaScores::N);
         if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &vmap, vp3, (int64_t)3 * G * g.dvp, g.span, vtile);
         if (rc == CC_OK) {
-            wa_cut_kernel<<<(unsigned)blocks, 256, 0, dev->stream>>>(qp, fptr(kring), vptr, qp3, kp3, vp3, g, q_tiles, (unsigned)row_blocks, oldest, vec);
+            wa_cut_kernel<<<(unsigned)blocks, 256, 0, dev->stream>>>(qp, fptr(kring), vptr, qp3, kp3, vp3, g, q_tiles, (unsigned)row_blocks, (int)(g.base0 % ring), (int)(oldest - g.base0), vec);
             dev->launches++;
             rc = sg_launch(dev, ws, (int64_t)key_tiles * q_tiles * G);
         }

@@ -223,6 +223,11 @@ int cc_launch_matvec(cc_device* dev, const cc_buf* w, const void* act_scratch, c
 bool cc_prefill_supported(int wtype, int64_t m, int64_t k, int64_t b);
 int cc_launch_prefill_matmul(cc_device* dev, const cc_buf* w, const void* act, const float* x_f32, float* out, int64_t m, int64_t k, int64_t b);
 void cc_prefill_release(cc_device* dev);
+// the same product in two halves: an elementwise step that leaves the quantised f16 operand [rows][cols] in the device's scratch, and products over it
+int cc_prefill_rows_norm(cc_device* dev, float* x, float* orig, const float* w, float eps, int64_t rows, int64_t cols, bool write_back);
+int cc_prefill_rows_unit(cc_device* dev, const float* g, const float* u, bool gelu, int64_t n, int64_t rows, int64_t cols);
+int cc_prefill_rows_plain(cc_device* dev, const float* x, int64_t rows, int64_t cols);
+int cc_launch_prefill_operand(cc_device* dev, const cc_buf* w, float* out, int64_t m, int64_t k, int64_t b, const float* res);
 // tensor map (CUtensorMap) of a bfloat16 matrix [rows][k], box 64 columns x box_rows rows, 128-byte swizzle
 int cc_make_tmap_bf16(cc_device* dev, void* tm, const void* base, int64_t rows, int64_t k, int box_rows);
 

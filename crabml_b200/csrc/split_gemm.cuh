@@ -365,17 +365,20 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
                 if (*(volatile int*)&sh.fail) break;
                 // columns of the lower half are finished by CTA 0, the others by CTA 1: each sends what the other needs
                 const bool send = (warp >= SG_WARPS / 2) == (rank == 0);
-                float* sums = (float*)ring + (size_t)(warp & (SG_WARPS / 2 - 1)) * COUNT * 32 + lane;
+                float4* sums = (float4*)ring + (size_t)(warp & (SG_WARPS / 2 - 1)) * (COUNT / 4) * 32 + lane;
                 if (send) {
-                    float* to = cluster.map_shared_rank(sums, rank ^ 1);
+                    float4* to = cluster.map_shared_rank(sums, rank ^ 1);
 #pragma unroll
-                    for (int c = 0; c < COUNT; c++) to[c * 32] = acc[c];
+                    for (int c = 0; c < COUNT; c += 4) to[c * 8] = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
                 }
                 p.give(ps, *cluster.map_shared_rank(&ps, rank ^ 1), tid);
                 cluster.sync();
                 if (!send) {
 #pragma unroll
-                    for (int c = 0; c < COUNT; c++) acc[c] += sums[c * 32];
+                    for (int c = 0; c < COUNT; c += 4) {
+                        const float4 x = sums[c * 8];
+                        acc[c] += x.x; acc[c + 1] += x.y; acc[c + 2] += x.z; acc[c + 3] += x.w;
+                    }
                     p.emit(tile, ps, row_fixed, row, col0, acc, buf);
                 }
             } else if (ok) p.emit(tile, ps, row_fixed, row, col0, acc, buf);

@@ -212,3 +212,33 @@ def test_delta_rule_however_the_tokens_are_cut(dev, dk, dv, H, G):
             # 32-bit sums of dk terms of order one, carried on by a contraction: 1e-5
             assert np.abs(got[t, h] - S[h].T @ f[0][t, h // (H // G)]).max() < 1e-5
     assert np.abs(end - S).max() < 1e-5
+
+
+# ---- a prompt in one call: the joined steps of a recording device give the bits of the separate ones ----------------------------------------------------
+@pytest.mark.parametrize("arch", ["llama", "qwen2"])
+@pytest.mark.parametrize("wtype", ["Q8_0", "Q4_0", "Q4_K"])
+@pytest.mark.parametrize("tokens", [33, 200])
+def test_prompt_recorded_and_eager_agree(arch, wtype, tokens):
+    from crabml_b200 import CudaTensor, CudaTensorDevice, capi
+    from crabml_b200 import runner as R
+    conf = R.LlamaConfig(4, 2, 2, 512, 768, 512, 1000, 1e-5, 128, arch)
+    ids = np.random.default_rng(tokens).integers(0, 1000, tokens).tolist()
+    got = []
+    for lazy in (0, 1, 2):
+        d = CudaTensorDevice(0, lazy=lazy)
+        w = R.synthetic_weights(d, conf, getattr(capi, wtype), capi.Q8_0, seed=5)
+        if arch == "qwen2":
+            rng = np.random.default_rng(9)
+            for name, n in (("bq", 512), ("bk", 256), ("bv", 256)):
+                w[name] = [CudaTensor.from_cpu(rng.standard_normal(n).astype(np.float32), [n], capi.F32, d) for _ in range(2)]
+        r = R.LlamaRunner(d, conf, w, 256)
+        a = r.forward(ids, 0).copy()
+        b = r.forward(ids[:3], tokens).copy()                 # a short portion behind it, and a token
+        c = r.forward(ids[:1], tokens + 3).copy()
+        got.append(np.stack([a, b, c]))
+        r.close()
+        del w
+        d.close()
+    assert np.isfinite(got[0]).all()
+    for g in got[1:]:
+        np.testing.assert_array_equal(g.view(np.uint32), got[0].view(np.uint32))

@@ -322,7 +322,7 @@ struct BmmTile {
     __device__ void give(const Shared&, Shared&, int) const {}
     template <int COUNT>
     __device__ void emit(const Tile& t, const Shared&, Fixed, int r, int col0, float (&v)[COUNT], float* buf) const {
-        sg_store_rows<COUNT, false>(buf, t.m0 + r < m ? t.c + (int64_t)(t.m0 + r) * n + t.n0 + col0 : nullptr, n - t.n0 - col0, v);
+        sg_store_rows<COUNT, false>(buf, t.m0 + r < m ? t.c + (int64_t)(t.m0 + r) * n + t.n0 + col0 : nullptr, n - t.n0 - col0, n % 4 == 0, v);
     }
 };
 template <bool B_F16, bool N_CONTIG>

@@ -361,7 +361,7 @@ static int pg_weight_f16(cc_device* dev, const cc_buf* w, int64_t m, int64_t k, 
 // The output tile of a CTA and how many CTAs share its depth: large tiles read fewer operand bytes per multiplication, small ones and shared depths put
 // more SMs to work.  Estimated time in SM cycles: per 64-deep step the slowest of the tensor core (4096 multiply-adds per cycle), the operand bytes at
 // about 40 per cycle and a floor for the step's own latency; once per tile its start and its stores, and for CTAs that share a depth the
-// sums on their way to each other (4 bytes each at about 16 per cycle).  The whole product takes as many rounds of tiles as the SMs need.  The sums that
+// sums on their way to each other (4 bytes each at about 8 per cycle).  The whole product takes as many rounds of tiles as the SMs need.  The sums that
 // meet must fit the ring.
 static void pg_pick_tile(cc_device* dev, int64_t m, int64_t b, int64_t k, int* block_n, int* mt, int* parts) {
     double best = 0.0;
@@ -376,7 +376,7 @@ static void pg_pick_tile(cc_device* dev, int64_t m, int64_t b, int64_t k, int* b
             for (int z = 1; z <= 4; z *= 2) {
                 if (z > 1 && (sums * (z - 1) / z > ring || t * n / 32 < z || k / PG_BLOCK_K < 4 * z || tiles * z > dev->sm_count)) break;
                 const int64_t rounds = (tiles * z + dev->sm_count - 1) / dev->sm_count;
-                const double cost = rounds * (step * ((k / PG_BLOCK_K + z - 1) / z) + 3000.0 + t * n * 8.0 / z) + (z > 1 ? 1500.0 + sums * (z - 1) / z / 16.0 : 0.0);
+                const double cost = rounds * (step * ((k / PG_BLOCK_K + z - 1) / z) + 3000.0 + t * n * 8.0 / z) + (z > 1 ? 1500.0 + sums * (z - 1) / z / 8.0 : 0.0);
                 if (best == 0.0 || cost < best) { best = cost; *block_n = n; *mt = t; *parts = z; }
             }
         }

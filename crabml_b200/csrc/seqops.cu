@@ -951,7 +951,8 @@ struct WaValues {
     __device__ const void* map_b() const { return &maps[0]; }
     __device__ void at_a(const Tile&, int, int, int&, int&) const {}
     __device__ void at_b(const Tile& t, int s, int plane, int& x, int& y) const { x = t.at + (t.step0 + 2 * s) * 64; y = (plane * g.G + t.kvh) * g.dvp + t.c0; }
-    struct Shared { float top[WA_ROWS], sum[8][WA_ROWS]; };     // top: times log2e ; sum: of each quarter of the threads, of this CTA and of the other
+    struct Shared { float top[WA_ROWS], sum[12][WA_ROWS]; };    // top: times log2e ; sum: before the steps the quarters' largest scores (0 ..), behind them the sums of each quarter
+                                                                // of the threads, of this CTA (4 ..) and of the other (8 ..)
     struct ARow { const float* s; float top, sum; };
     typedef const float* BCol;
     const float *S, *tops, *vring, *sink;
@@ -968,15 +969,19 @@ struct WaValues {
     }
     __device__ Fixed fixed(int r) const { const int tq = r / g.R; return Fixed{tq, r - tq * g.R}; }
     __device__ float sink_of(const Tile& t, int r) const { return sink[t.kvh * g.R + r % g.R]; }
+    // the rows' largest scores, a quarter of the threads for each quarter of a key tile
     __device__ void setup(const Tile& t, Shared& ps) const {
-        const int r = threadIdx.x;
-        if (r >= WA_ROWS) return;
-        const float* p = tops + ((int64_t)t.kvh * q_tiles + t.qt) * key_tiles * 4 * WA_ROWS + r;
+        const int r = threadIdx.x & 127, quarter = threadIdx.x >> 7;
+        const float* p = tops + (((int64_t)t.kvh * q_tiles + t.qt) * key_tiles * 4 + quarter) * WA_ROWS + r;
         float top = -INFINITY;
 #pragma unroll 8
-        for (int n = 0; n < 4 * (t.last / WaScores::N + 1); n++) top = fmaxf(top, p[n * WA_ROWS]);
+        for (int n = 0; n <= t.last / WaScores::N; n++) top = fmaxf(top, p[n * 4 * WA_ROWS]);
+        ps.sum[quarter][r] = top;
+    }
+    __device__ float top_of(const Tile& t, const Shared& ps, int r) const {
+        float top = fmaxf(fmaxf(ps.sum[0][r], ps.sum[1][r]), fmaxf(ps.sum[2][r], ps.sum[3][r]));
         if (sink) top = fmaxf(top, sink_of(t, r));
-        ps.top[r] = top * WA_LOG2E;
+        return top * WA_LOG2E;
     }
     __device__ float weight(float s, float top) const {
         float e;
@@ -984,7 +989,7 @@ struct WaValues {
         return e;
     }
     __device__ ARow a_row(const Tile& t, const Shared& ps, Fixed f, int r) const {
-        return ARow{f.tq < t.tq_n ? S + wa_score_at(t, q_tiles, g.cap, 0, r) : nullptr, ps.top[r], 0.0f};
+        return ARow{f.tq < t.tq_n ? S + wa_score_at(t, q_tiles, g.cap, 0, r) : nullptr, top_of(t, ps, r), 0.0f};
     }
     __device__ void load_a(const Tile& t, const ARow& a, int s, int c, float (&v)[8]) const {
         if (!a.s) { sg_zero8(v); return; }
@@ -1014,21 +1019,24 @@ struct WaValues {
             if (++row == (unsigned)g.ring) row = 0;
         }
     }
-    __device__ void end_a(const Tile&, Shared& ps, const ARow& a, int r, int part) const { ps.sum[part][r] = a.sum; }
+    __device__ void end_a(const Tile&, Shared& ps, const ARow& a, int r, int part) const {
+        ps.sum[4 + part][r] = a.sum;
+        if (part == 0) ps.top[r] = a.top;
+    }
     // a CTA's sums of weights to the other
-    __device__ void give(const Shared& mine, Shared& theirs, int tid) const { theirs.sum[4 + (tid >> 7)][tid & 127] = mine.sum[tid >> 7][tid & 127]; }
+    __device__ void give(const Shared& mine, Shared& theirs, int tid) const { theirs.sum[8 + (tid >> 7)][tid & 127] = mine.sum[4 + (tid >> 7)][tid & 127]; }
     template <int COUNT>
     __device__ void emit(const Tile& t, const Shared& ps, Fixed f, int r, int col0, float (&v)[COUNT], float* buf) const {
         float a = 0.0f, b = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 4; i++) { a += ps.sum[i][r]; b += ps.sum[4 + i][r]; }
+        for (int i = 0; i < 4; i++) { a += ps.sum[4 + i][r]; b += ps.sum[8 + i][r]; }
         float total = a + b;                            // of the two CTAs, the same number in both
         if (sink) total += weight(sink_of(t, r), ps.top[r]);
         const float inv = 1.0f / total;
 #pragma unroll
         for (int c = 0; c < COUNT; c++) v[c] *= inv;
         const int64_t row = wa_row(g, t, f);
-        sg_store_rows<COUNT, false>(buf, row < 0 ? nullptr : o + row * g.dv + t.c0 + col0, g.dv - t.c0 - col0, v);
+        sg_store_rows<COUNT, false>(buf, row < 0 ? nullptr : o + row * g.dv + t.c0 + col0, g.dv - t.c0 - col0, g.dv % 4 == 0, v);
     }
 };
 // few rows (decoding): grid (ceil(keys / 16), T, G * head blocks), 256 threads.  The CTA stages up to WS_HEADS queries of (token, key/value head); a

@@ -108,10 +108,21 @@ __device__ __forceinline__ void sg_tmem16(unsigned addr, unsigned (&v)[16]) {
                    "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                  : "r"(addr));
 }
-// a warp's 32 rows x COUNT columns into rows of memory, through shared memory so that a warp stores whole lines.  out: the row's first number (NULL: no
-// such row); columns from `cols` on are dropped
+// a warp's 32 rows x COUNT columns into rows of memory.  out: the row's first number (NULL: no such row); columns from `cols` on are dropped.  vec (rows start
+// at multiples of 16 bytes): a thread stores its own row 16 bytes at a time -- eight stores and nothing else, where the way through shared memory, for rows
+// that start anywhere, is a chain of some 500 instructions in two warps per scheduler (5000 cycles)
 template <int COUNT, bool ADD>
-__device__ __forceinline__ void sg_store_rows(float* buf, float* out, int cols, const float (&v)[COUNT]) {
+__device__ __forceinline__ void sg_store_rows(float* buf, float* out, int cols, bool vec, const float (&v)[COUNT]) {
+    if (vec) {
+#pragma unroll
+        for (int c = 0; c < COUNT; c += 4)
+            if (out && c < cols) {
+                float4 x = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+                if (ADD) { const float4 y = *(const float4*)(out + c); x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w; }
+                *(float4*)(out + c) = x;
+            }
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const unsigned long long at = (unsigned long long)out;
 #pragma unroll

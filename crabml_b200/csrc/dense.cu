@@ -23,6 +23,7 @@ __device__ __forceinline__ float dn_load_w(const uint16_t* w, int64_t i) { retur
 // grid: (ceil(m / 64), ceil(b / 64)).  Thread (ty, tx) of a 16 x 16 layout owns batch rows ty*4.. and weight rows tx*4.. of the tile.
 template <class WT, bool ROUND_X>
 __global__ void __launch_bounds__(DN_THREADS) dense_tile_kernel(const WT* __restrict__ W, const float* __restrict__ X, float* __restrict__ C, int m, int b, int k, int accumulate) {
+    pdl_enter();
     __shared__ float sw[DN_K][DN_TILE + 4];       // [kk][weight row]
     __shared__ float sx[DN_K][DN_TILE + 4];       // [kk][batch row]
     const int m0 = blockIdx.x * DN_TILE, b0 = blockIdx.y * DN_TILE;
@@ -85,8 +86,8 @@ int cc_launch_dense(cc_device* dev, const cc_buf* w, const float* x, float* out,
 int cc_launch_dense_tile(cc_device* dev, const cc_buf* w, const float* x, float* out, int64_t m, int64_t k, int64_t b, int accumulate) {
     if (m == 0 || b == 0) return CC_OK;
     dim3 grid((unsigned)((m + DN_TILE - 1) / DN_TILE), (unsigned)((b + DN_TILE - 1) / DN_TILE));
-    if (w->dtype == CC_F32) dense_tile_kernel<float, false><<<grid, DN_THREADS, 0, dev->stream>>>((const float*)w->plane[0], x, out, (int)m, (int)b, (int)k, accumulate);
-    else if (w->dtype == CC_BF16) dense_tile_kernel<uint16_t, true><<<grid, DN_THREADS, 0, dev->stream>>>((const uint16_t*)w->plane[0], x, out, (int)m, (int)b, (int)k, accumulate);
+    if (w->dtype == CC_F32) cc_launch_pdl(dev, dense_tile_kernel<float, false>, grid, DN_THREADS, 0, (const float*)w->plane[0], x, out, (int)m, (int)b, (int)k, accumulate);
+    else if (w->dtype == CC_BF16) cc_launch_pdl(dev, dense_tile_kernel<uint16_t, true>, grid, DN_THREADS, 0, (const uint16_t*)w->plane[0], x, out, (int)m, (int)b, (int)k, accumulate);
     else return cc_fail(dev, CC_ERR_UNSUPPORTED, "dense matmul: weight type %d", w->dtype);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;

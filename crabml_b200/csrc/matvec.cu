@@ -18,6 +18,7 @@
 template <class T>
 __global__ void __launch_bounds__(MV_THREADS) matvec_kernel(WPlanes W, const void* act, int64_t n_total,
                                                             float* __restrict__ out, int m, int k) {
+    pdl_enter();
     extern __shared__ __align__(16) uint8_t smem[];
     const int bi = blockIdx.y;
     T::stage_act(act, n_total, bi, k, smem);
@@ -36,6 +37,7 @@ __global__ void __launch_bounds__(MV_THREADS) matvec_kernel(WPlanes W, const voi
 // activation reads from shared memory (a 16-byte weight chunk meets 2 x NB 16-byte activation chunks)
 template <class T, int NB>
 __global__ void __launch_bounds__(MV_THREADS) matvec_few_kernel(WPlanes W, const void* act, int64_t n_total, float* __restrict__ out, int m, int k, int b) {
+    pdl_enter();
     extern __shared__ __align__(16) uint8_t smem[];
     const int b0 = blockIdx.y * NB, stride = T::smem_bytes(k);
     for (int n = 0; n < NB; n++) T::stage_act(act, n_total, min(b0 + n, b - 1), k, smem + n * stride);       // activations behind the last repeat it
@@ -60,7 +62,7 @@ static int launch_few(cc_device* dev, const WPlanes& W, const void* act, int64_t
     const int64_t groups = (b + NB - 1) / NB, need = (m + 2 * MV_WARPS - 1) / (2 * MV_WARPS), most = smem > 100 * 1024 ? dev->sm_count : 2 * (int64_t)dev->sm_count;
     int64_t ctas = most / groups > 0 ? most / groups : 1;
     if (ctas > need) ctas = need;
-    matvec_few_kernel<T, NB><<<dim3((unsigned)ctas, (unsigned)groups), MV_THREADS, smem, dev->stream>>>(W, act, n_total, out, (int)m, (int)k, (int)b);
+    cc_launch_pdl(dev, matvec_few_kernel<T, NB>, dim3((unsigned)ctas, (unsigned)groups), MV_THREADS, smem, W, act, n_total, out, (int)m, (int)k, (int)b);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -77,7 +79,7 @@ static int launch(cc_device* dev, const cc_buf* w, const void* act, int64_t n_to
     int64_t cap = (int64_t)dev->sm_count * 8;
     if (ctas > cap) ctas = cap;
     dim3 grid((unsigned)ctas, (unsigned)b);
-    matvec_kernel<T><<<grid, MV_THREADS, smem, dev->stream>>>(W, act, n_total, out, (int)m, (int)k);
+    cc_launch_pdl(dev, matvec_kernel<T>, grid, MV_THREADS, smem, W, act, n_total, out, (int)m, (int)k);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }

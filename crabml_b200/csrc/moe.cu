@@ -50,6 +50,7 @@ struct RouteArgs {
 // logit's sum does not depend on TOK.
 template <int TOK>
 __global__ void __launch_bounds__(TOK == 1 ? 1024 : 512) moe_route_kernel(RouteArgs a) {
+    pdl_enter();
     extern __shared__ float rt_sm[];
     __shared__ float sg_sm[TOK];                           // the shared gate's logit: row E of the same products
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
@@ -200,8 +201,8 @@ extern "C" CC_API int cc_moe_route_shared(cc_device* dev, const cc_view* x, cons
     const int64_t rows = E + (shared_gate ? 1 : 0), most = tiled ? 16 : 32, rounds = (rows + most - 1) / most;
     const int64_t even = (rows + rounds - 1) / rounds;
     const unsigned threads = 32 * (unsigned)(even < 4 ? 4 : even);
-    if (tiled) moe_route_kernel<4><<<(unsigned)((T + 3) / 4), threads, 4 * one, dev->stream>>>(a);
-    else moe_route_kernel<1><<<(unsigned)T, threads, one, dev->stream>>>(a);
+    if (tiled) cc_launch_pdl(dev, moe_route_kernel<4>, (unsigned)((T + 3) / 4), threads, 4 * one, a);
+    else cc_launch_pdl(dev, moe_route_kernel<1>, (unsigned)T, threads, one, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -254,6 +255,7 @@ template <class WT, bool VEC> __device__ __forceinline__ float moe_dot(const WT*
 template <class WT, bool VEC>
 __global__ void __launch_bounds__(256) moe_gate_up_kernel(const float* __restrict__ x, const int* __restrict__ ids, const WT* __restrict__ wg, const WT* __restrict__ wu,
                                                           float* __restrict__ hid, int D, int ff, int top, cc_glu_params act, int E) {
+    pdl_enter();
     extern __shared__ __align__(16) float mg_sm[];
     const int ts = blockIdx.x, t = ts / top;
     const int e = ids ? moe_clamp(ids[ts], E) : 0;
@@ -271,6 +273,7 @@ __global__ void __launch_bounds__(256) moe_gate_up_kernel(const float* __restric
 template <class WT, bool VEC>
 __global__ void __launch_bounds__(256) moe_down_kernel(const float* __restrict__ hid, const int* __restrict__ ids, const float* __restrict__ wts, const WT* __restrict__ wd,
                                                        float* __restrict__ out, int D, int ff, int top, int E) {
+    pdl_enter();
     extern __shared__ __align__(16) float md_sm[];
     const int t = blockIdx.x;
     for (int i = threadIdx.x; i < top * ff; i += 256) md_sm[i] = moe_round<WT>(hid[(int64_t)t * top * ff + i]);
@@ -295,9 +298,9 @@ static int moe_launch_vec(cc_device* dev, const float* x, const int* ids, const 
     if (s1 > 200 * 1024 || s2 > 200 * 1024) return cc_fail(dev, CC_ERR_UNSUPPORTED, "moe_experts: row does not fit shared memory");
     if (s1 > 48 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(moe_gate_up_kernel<WT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1));
     if (s2 > 48 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(moe_down_kernel<WT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2));
-    moe_gate_up_kernel<WT, VEC><<<dim3((unsigned)(T * top), (unsigned)((ff + 7) / 8)), 256, s1, dev->stream>>>(x, ids, wg, wu, hid, D, ff, top, act, E);
+    cc_launch_pdl(dev, moe_gate_up_kernel<WT, VEC>, dim3((unsigned)(T * top), (unsigned)((ff + 7) / 8)), 256, s1, x, ids, wg, wu, hid, D, ff, top, act, E);
     CC_LAUNCH_CHECK(dev);
-    moe_down_kernel<WT, VEC><<<dim3((unsigned)T, (unsigned)((D + 7) / 8)), 256, s2, dev->stream>>>(hid, ids, wts, wd, out, D, ff, top, E);
+    cc_launch_pdl(dev, moe_down_kernel<WT, VEC>, dim3((unsigned)T, (unsigned)((D + 7) / 8)), 256, s2, hid, ids, wts, wd, out, D, ff, top, E);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -320,6 +323,7 @@ int cc_launch_grouped_bf16(cc_device* dev, const cc_buf* w_stack, int64_t n_grou
 // one CTA: counts per expert (shared-memory atomics), exclusive offsets, the tile table {n_tiles | expert, first row, rows, 0 ...}, and
 // pos[i] = sorted row of entry i = (token, slot).  The order of the rows INSIDE an expert is arbitrary; no value depends on it.
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ ids, int n, int E, int block_n, int* __restrict__ pos, int* __restrict__ table) {
+    pdl_enter();
     extern __shared__ int ms_sm[];            // counts[E], offsets[E]
     int* cnt = ms_sm;
     int* off = ms_sm + E;
@@ -344,6 +348,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
 }
 // xs[pos[i]][:] = bf16(x[i / top][:]) ; one warp per entry
 __global__ void moe_gather_bf16_kernel(const float* __restrict__ x, const int* __restrict__ pos, __nv_bfloat16* __restrict__ xs, int n, int top, int D) {
+    pdl_enter();
     const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i >= n) return;
     const float* src = x + (int64_t)(i / top) * D;
@@ -351,6 +356,7 @@ __global__ void moe_gather_bf16_kernel(const float* __restrict__ x, const int* _
     for (int d = lane * 2; d < D; d += 64) *(__nv_bfloat162*)(dst + d) = __floats2bfloat162_rn(src[d], src[d + 1]);
 }
 __global__ void moe_glu_bf16_kernel(const float* __restrict__ g, const float* __restrict__ u, __nv_bfloat16* __restrict__ h, int64_t n, cc_glu_params act) {
+    pdl_enter();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (i >= n) return;
     const float2 uv = *(const float2*)(u + i);
@@ -362,11 +368,13 @@ __global__ void moe_glu_bf16_kernel(const float* __restrict__ g, const float* __
     }
 }
 __global__ void moe_activate_kernel(float* __restrict__ x, int64_t n, int act) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = act_apply(x[i], act);
 }
 // out[t][d] = sum over the slots, in slot order, of weights[t][s] * y[pos[t * top + s]][d]
 __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ pos, const float* __restrict__ wts, float* __restrict__ out, int64_t T, int top, int D) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= T * D) return;
     const int64_t t = i / D; const int d = (int)(i % D);
@@ -390,19 +398,19 @@ static int moe_grouped(cc_device* dev, const float* x, const int* ids, const flo
     int* pos = (int*)(base + o_pos); int* table = (int*)(base + o_tab);
     __nv_bfloat16* xs = (__nv_bfloat16*)(base + o_xs); float* g = wg ? (float*)(base + o_g) : nullptr; float* u = (float*)(base + o_u);
     __nv_bfloat16* h = (__nv_bfloat16*)(base + o_h); float* y = (float*)(base + o_y);
-    moe_sort_kernel<<<1, 1024, (size_t)2 * E * 4, dev->stream>>>(ids, (int)n, E, block_n, pos, table);
+    cc_launch_pdl(dev, moe_sort_kernel, 1, 1024, (size_t)2 * E * 4, ids, (int)n, E, block_n, pos, table);
     dev->launches++;
-    moe_gather_bf16_kernel<<<(unsigned)((n + 7) / 8), 256, 0, dev->stream>>>(x, pos, xs, (int)n, top, D);
+    cc_launch_pdl(dev, moe_gather_bf16_kernel, (unsigned)((n + 7) / 8), 256, 0, x, pos, xs, (int)n, top, D);
     dev->launches++;
     if (wg) rc = cc_launch_grouped_bf16(dev, wg, E, ff, D, xs, n, table, max_tiles, block_n, g);
     if (!rc) rc = cc_launch_grouped_bf16(dev, wu, E, ff, D, xs, n, table, max_tiles, block_n, u);
     if (!rc) {
-        moe_glu_bf16_kernel<<<(unsigned)((n * ff / 2 + 255) / 256), 256, 0, dev->stream>>>(g, u, h, n * ff, act);
+        cc_launch_pdl(dev, moe_glu_bf16_kernel, (unsigned)((n * ff / 2 + 255) / 256), 256, 0, g, u, h, n * ff, act);
         dev->launches++;
         rc = cc_launch_grouped_bf16(dev, wd, E, D, ff, h, n, table, max_tiles, block_n, y);
     }
     if (!rc) {
-        moe_combine_kernel<<<(unsigned)((T * D + 255) / 256), 256, 0, dev->stream>>>(y, pos, wts, out, T, top, D);
+        cc_launch_pdl(dev, moe_combine_kernel, (unsigned)((T * D + 255) / 256), 256, 0, y, pos, wts, out, T, top, D);
         CC_LAUNCH_CHECK(dev);
     }
     cc_pool_free(dev, base, cls);
@@ -496,7 +504,7 @@ extern "C" CC_API int cc_feed_forward_act(cc_device* dev, const cc_view* x, cons
             rc = cc_launch_prefill_bf16_act(dev, w_down->buf, (const float*)hid, act, (float*)o->base, D, ff, T);          // the activation rides in the operand's conversion
         } else {
             const int64_t n = T * ff;
-            moe_activate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>((float*)hid, n, act);
+            cc_launch_pdl(dev, moe_activate_kernel, (unsigned)((n + 255) / 256), 256, 0, (float*)hid, n, act);
             dev->launches++;
             rc = cc_launch_dense(dev, w_down->buf, (const float*)hid, (float*)o->base, D, ff, T);
         }

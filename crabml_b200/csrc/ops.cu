@@ -7,6 +7,7 @@
 // ---- rms_norm_inplace: primitives/rms_norm.rs:32-47  x /= sqrt(sum(x^2)/n + eps), no weight ------------
 // canonical 512-thread order (common.cuh); cols % 4 == 0 is implied by the reference's own assert (cols % 32 == 0)
 __global__ void __launch_bounds__(CC_RED_THREADS) rms_norm_kernel(float* x, int64_t cols, float eps) {
+    pdl_enter();
     __shared__ float sh[CC_RED_WARPS];
     float* v = x + (int64_t)blockIdx.x * cols;
     float s = 0.0f;
@@ -19,7 +20,7 @@ __global__ void __launch_bounds__(CC_RED_THREADS) rms_norm_kernel(float* x, int6
 }
 int cc_launch_rms_norm(cc_device* dev, float* x, int64_t rows, int64_t cols, float eps) {
     if (rows == 0 || cols == 0) return CC_OK;
-    rms_norm_kernel<<<(unsigned)rows, CC_RED_THREADS, 0, dev->stream>>>(x, cols, eps);
+    cc_launch_pdl(dev, rms_norm_kernel, (unsigned)rows, CC_RED_THREADS, 0, x, cols, eps);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -30,6 +31,7 @@ int cc_launch_rms_norm(cc_device* dev, float* x, int64_t rows, int64_t cols, flo
 __device__ __forceinline__ float exp_cached(float v, const uint16_t* lut) { return h2f_bits(lut[f2h_bits(v)]); }
 
 __global__ void __launch_bounds__(CC_RED_THREADS) softmax_kernel(float* x, int64_t cols, const uint16_t* __restrict__ lut) {
+    pdl_enter();
     __shared__ float sh[CC_RED_WARPS];
     float* v = x + (int64_t)blockIdx.x * cols;
     float m = -INFINITY;
@@ -49,6 +51,7 @@ __global__ void __launch_bounds__(CC_RED_THREADS) softmax_kernel(float* x, int64
 #define SM_MAX_COLS 2048
 #define SM_WARPS 4
 __global__ void __launch_bounds__(SM_WARPS * 32) softmax_rows_kernel(float* x, int64_t rows, int cols, const uint16_t* __restrict__ lut) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * SM_WARPS + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -80,17 +83,18 @@ int cc_launch_softmax(cc_device* dev, float* x, int64_t rows, int64_t cols) {
     if (rows == 0 || cols == 0) return CC_OK;
     // a CTA per row is the faster one while its rows leave SMs idle, and where a row is long
     if (rows >= 4 * (int64_t)dev->sm_count && cols <= SM_MAX_COLS) {
-        softmax_rows_kernel<<<(unsigned)((rows + SM_WARPS - 1) / SM_WARPS), SM_WARPS * 32, 0, dev->stream>>>(x, rows, (int)cols, dev->exp_lut);
+        cc_launch_pdl(dev, softmax_rows_kernel, (unsigned)((rows + SM_WARPS - 1) / SM_WARPS), SM_WARPS * 32, 0, x, rows, (int)cols, dev->exp_lut);
         CC_LAUNCH_CHECK(dev);
         return CC_OK;
     }
-    softmax_kernel<<<(unsigned)rows, CC_RED_THREADS, 0, dev->stream>>>(x, cols, dev->exp_lut);
+    cc_launch_pdl(dev, softmax_kernel, (unsigned)rows, CC_RED_THREADS, 0, x, cols, dev->exp_lut);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 
 // ---- silu / gelu: primitives/silu.rs:6-13, gelu.rs:10-15 -----------------------------------------------------
 __global__ void silu_kernel(float* x, int64_t n, const uint16_t* __restrict__ lut) {
+    pdl_enter();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         float v = x[i];
@@ -98,24 +102,26 @@ __global__ void silu_kernel(float* x, int64_t n, const uint16_t* __restrict__ lu
     }
 }
 __global__ void gelu_kernel(float* x, int64_t n, const uint16_t* __restrict__ lut) {
+    pdl_enter();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = h2f_bits(lut[f2h_bits(x[i])]);
 }
 int cc_launch_silu(cc_device* dev, float* x, int64_t n) {
     if (n == 0) return CC_OK;
-    silu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(x, n, dev->exp_lut);
+    cc_launch_pdl(dev, silu_kernel, (unsigned)((n + 255) / 256), 256, 0, x, n, dev->exp_lut);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 int cc_launch_gelu(cc_device* dev, float* x, int64_t n) {
     if (n == 0) return CC_OK;
-    gelu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(x, n, dev->gelu_lut);
+    cc_launch_pdl(dev, gelu_kernel, (unsigned)((n + 255) / 256), 256, 0, x, n, dev->gelu_lut);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 
 // ---- add / mul with rhs cycling: primitives/arithmetic.rs:5-68 ---------------------------------------------------
 __global__ void binary_kernel(float* x, int64_t n, const float* __restrict__ y, int64_t ny, int op) {
+    pdl_enter();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float b = y[ny == 1 ? 0 : i % ny];
@@ -123,17 +129,18 @@ __global__ void binary_kernel(float* x, int64_t n, const float* __restrict__ y, 
 }
 int cc_launch_binary(cc_device* dev, float* x, int64_t n, const float* y, int64_t ny, int op) {
     if (n == 0) return CC_OK;
-    binary_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(x, n, y, ny, op);
+    cc_launch_pdl(dev, binary_kernel, (unsigned)((n + 255) / 256), 256, 0, x, n, y, ny, op);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 __global__ void scale_kernel(float* x, int64_t n, float s) {
+    pdl_enter();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = x[i] * s;
 }
 int cc_launch_scale(cc_device* dev, float* x, int64_t n, float s) {     // cpu_tensor.rs:404-410
     if (n == 0) return CC_OK;
-    scale_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(x, n, s);
+    cc_launch_pdl(dev, scale_kernel, (unsigned)((n + 255) / 256), 256, 0, x, n, s);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -142,6 +149,7 @@ int cc_launch_scale(cc_device* dev, float* x, int64_t n, float s) {     // cpu_t
 struct CopyDims { int64_t shape[CC_MAX_DIMS], sstr[CC_MAX_DIMS], dstr[CC_MAX_DIMS]; int ndim; };
 
 __global__ void strided_copy_kernel(const void* src, int src_dtype, void* dst, int dst_dtype, CopyDims d, int64_t dst_offset, int64_t total) {
+    pdl_enter();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     int64_t rem = i, so = 0, dof = dst_offset;
@@ -160,6 +168,7 @@ __global__ void strided_copy_kernel(const void* src, int src_dtype, void* dst, i
 // finds its place with 32-bit divisions.  [512, 32, 128] -> [32, 512, 128] (8 MB): 35 -> 6 us
 struct CopyDims32 { unsigned shape[CC_MAX_DIMS], sstr[CC_MAX_DIMS], dstr[CC_MAX_DIMS]; int ndim; };      // last axis and strides in units of 4 elements
 __global__ void __launch_bounds__(256) strided_copy16_kernel(const float4* __restrict__ src, float4* __restrict__ dst, CopyDims32 d, unsigned total) {
+    pdl_enter();
     const unsigned i = blockIdx.x * 256u + threadIdx.x;
     if (i >= total) return;
     unsigned rem = i, so = 0, dof = 0;
@@ -200,11 +209,11 @@ int cc_launch_strided_copy(cc_device* dev, const void* src, int src_dtype, const
     CopyDims32 d32;
     if (total < ((int64_t)1 << 31) && copy16(src, src_dtype, sshape, sstrides, dst, dst_dtype, dstrides, dst_offset, ndim, &d32)) {
         const unsigned n = (unsigned)(total / 4);
-        strided_copy16_kernel<<<(n + 255) / 256, 256, 0, dev->stream>>>((const float4*)src, (float4*)((float*)dst + dst_offset), d32, n);
+        cc_launch_pdl(dev, strided_copy16_kernel, (n + 255) / 256, 256, 0, (const float4*)src, (float4*)((float*)dst + dst_offset), d32, n);
         CC_LAUNCH_CHECK(dev);
         return CC_OK;
     }
-    strided_copy_kernel<<<(unsigned)((total + 255) / 256), 256, 0, dev->stream>>>(src, src_dtype, dst, dst_dtype, d, dst_offset, total);
+    cc_launch_pdl(dev, strided_copy_kernel, (unsigned)((total + 255) / 256), 256, 0, src, src_dtype, dst, dst_dtype, d, dst_offset, total);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -216,6 +225,7 @@ int cc_launch_strided_copy(cc_device* dev, const void* src, int src_dtype, const
 template <bool B_F16>
 __global__ void bmm_kcontig_kernel(const float* __restrict__ a, const void* __restrict__ b, float* __restrict__ c,
                                    int64_t ab, int64_t bb, int64_t m, int64_t k, int64_t n, int64_t sb0, int64_t sb2) {
+    pdl_enter();
     int64_t o = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (o >= ab * m * n) return;
@@ -238,6 +248,7 @@ __global__ void bmm_kcontig_kernel(const float* __restrict__ a, const void* __re
 template <bool B_F16>
 __global__ void bmm_ncontig_kernel(const float* __restrict__ a, const void* __restrict__ b, float* __restrict__ c,
                                    int64_t ab, int64_t bb, int64_t m, int64_t k, int64_t n, int64_t sb0, int64_t sb1) {
+    pdl_enter();
     int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= ab * m * n) return;
     int64_t ni = o % n, mi = (o / n) % m, bi = o / (m * n);
@@ -347,12 +358,12 @@ int cc_launch_batch_matmul(cc_device* dev, const float* a, const void* b, int b_
     }
     if (sb1 == 1) {
         unsigned grid = (unsigned)((outs * 32 + 255) / 256);
-        if (f16) bmm_kcontig_kernel<true><<<grid, 256, 0, dev->stream>>>(a, b, c, ab, bb, m, k, n, sb0, sb2);
-        else bmm_kcontig_kernel<false><<<grid, 256, 0, dev->stream>>>(a, b, c, ab, bb, m, k, n, sb0, sb2);
+        if (f16) cc_launch_pdl(dev, bmm_kcontig_kernel<true>, grid, 256, 0, a, b, c, ab, bb, m, k, n, sb0, sb2);
+        else cc_launch_pdl(dev, bmm_kcontig_kernel<false>, grid, 256, 0, a, b, c, ab, bb, m, k, n, sb0, sb2);
     } else {
         unsigned grid = (unsigned)((outs + 127) / 128);
-        if (f16) bmm_ncontig_kernel<true><<<grid, 128, 0, dev->stream>>>(a, b, c, ab, bb, m, k, n, sb0, sb1);
-        else bmm_ncontig_kernel<false><<<grid, 128, 0, dev->stream>>>(a, b, c, ab, bb, m, k, n, sb0, sb1);
+        if (f16) cc_launch_pdl(dev, bmm_ncontig_kernel<true>, grid, 128, 0, a, b, c, ab, bb, m, k, n, sb0, sb1);
+        else cc_launch_pdl(dev, bmm_ncontig_kernel<false>, grid, 128, 0, a, b, c, ab, bb, m, k, n, sb0, sb1);
     }
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
@@ -365,6 +376,7 @@ __device__ __forceinline__ void argmax_merge(float& bv, long long& bi, float ov,
 }
 __global__ void __launch_bounds__(CC_RED_THREADS) argmax_kernel(const float* __restrict__ x, long long n, long long* slot, long long* hist,
                                                                const long long* hist_index_dev, long long hist_index) {
+    pdl_enter();
     __shared__ float sv[CC_RED_WARPS];
     __shared__ long long si[CC_RED_WARPS];
     float bv = 0.0f; long long bi = -1;
@@ -386,7 +398,7 @@ __global__ void __launch_bounds__(CC_RED_THREADS) argmax_kernel(const float* __r
     }
 }
 int cc_launch_argmax(cc_device* dev, const float* x, int64_t n, int64_t* slot, int64_t* hist, const int64_t* hist_index_dev, int64_t hist_index) {
-    argmax_kernel<<<1, CC_RED_THREADS, 0, dev->stream>>>(x, (long long)n, (long long*)slot, (long long*)hist, (const long long*)hist_index_dev, (long long)hist_index);
+    cc_launch_pdl(dev, argmax_kernel, 1, CC_RED_THREADS, 0, x, (long long)n, (long long*)slot, (long long*)hist, (const long long*)hist_index_dev, (long long)hist_index);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }

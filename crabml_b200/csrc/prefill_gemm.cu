@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) umma_gemm_kernel(const __grid_c
     // per-group row count.  Rows a tile loads beyond its own (the next group's, or zero fill) are computed and never stored.
     int g_row0 = 0, g_w0 = 0;
     if (groups) {
+        pdl_enter();                                                     // the table is the kernel's before
         if ((int)blockIdx.y >= groups[0]) return;
         const int* gt = groups + 4 + 4 * blockIdx.y;
         g_w0 = gt[0] * m; g_row0 = gt[1]; b = gt[1] + gt[2];
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) umma_gemm_kernel(const __grid_c
     __syncthreads();
     pg_fence_after();
     const unsigned tmem_acc = sh.tmem_base;
+    if (!groups) pdl_enter();
 
     if (warp == 0) {
         // ===== TMA producer =====
@@ -225,6 +227,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) umma_gemm_kernel(const __grid_c
 // ---- operand preparation ---------------------------------------------------------------------------------------------------------
 // weights: device plane layout -> f16 [m][k]; one thread per 2 elements
 __global__ void dequant_w_f16_kernel(int dtype, DeqPlanes planes, int64_t nelems, __half* __restrict__ out) {
+    pdl_enter();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (i >= nelems) return;
     float a, b2;
@@ -235,6 +238,7 @@ __global__ void dequant_w_f16_kernel(int dtype, DeqPlanes planes, int64_t nelems
 }
 // activation: Q8_0 SoA (qs, f32(f16 d)) -> f16(q * d) [b][k]
 __global__ void act_q8_to_f16_kernel(ActQ8_0 act, int64_t nelems, __half* __restrict__ out) {
+    pdl_enter();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (i >= nelems) return;
     const float d = act.d[i >> 5];
@@ -243,6 +247,7 @@ __global__ void act_q8_to_f16_kernel(ActQ8_0 act, int64_t nelems, __half* __rest
 
 // activation of the K-quant weights: Q8_K SoA (qs, f32 d per 256) -> f16(q * d) [b][k]   (buf_q8_k.rs:84-131)
 __global__ void act_q8k_to_f16_kernel(ActQ8_K act, int64_t nelems, __half* __restrict__ out) {
+    pdl_enter();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (i >= nelems) return;
     const float d = act.d[i >> 8];
@@ -252,6 +257,7 @@ __global__ void act_q8k_to_f16_kernel(ActQ8_K act, int64_t nelems, __half* __res
 // f32 activation rows -> f16(q * d) in ONE pass (what quantize_q8_0_kernel + act_q8_to_f16_kernel produce together, same arithmetic:
 // d = max|x| / 127, q = trunc(x / d), stored scale f32(f16(d)); buf_q8_0.rs:87-134): one warp per 32-element block
 __global__ void act_f32_to_q8f16_kernel(const float* __restrict__ x, int64_t nblocks, __half* __restrict__ out) {
+    pdl_enter();
     const int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (b >= nblocks) return;
@@ -327,10 +333,12 @@ static int pg_launch(cc_device* dev, const CUtensorMap& tw, const CUtensorMap& t
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((m + PG_BLOCK_M * MT - 1) / (PG_BLOCK_M * MT)), (unsigned)((b + BLOCK_N - 1) / BLOCK_N), (unsigned)parts);
     cfg.blockDim = dim3(PG_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = dev->stream;
-    cudaLaunchAttribute cluster;
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = 1; cluster.val.clusterDim.y = 1; cluster.val.clusterDim.z = (unsigned)parts;
-    if (parts > 1) { cfg.attrs = &cluster; cfg.numAttrs = 1; }
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = dev->pdl ? 1 : 0;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = (unsigned)parts;
+    cfg.attrs = at; cfg.numAttrs = parts > 1 ? 2 : 1;
     CC_CUDA(dev, cudaLaunchKernelEx(&cfg, umma_gemm_kernel<BLOCK_N, MT, FMT>, tw, tx, out, (int)m, (int)b, (int)k, (const int*)nullptr, res));
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
@@ -351,7 +359,7 @@ static int pg_weight_f16(cc_device* dev, const cc_buf* w, int64_t m, int64_t k, 
     for (int i = 0; i < CC_MAX_PLANES; i++) pl.p[i] = w->plane[i];
     pl.cols = w->cols > 0 ? w->cols : k;
     const int64_t n = m * k;
-    dequant_w_f16_kernel<<<(unsigned)((n / 2 + 255) / 256), 256, 0, dev->stream>>>(w->dtype, pl, n, (__half*)dst);
+    cc_launch_pdl(dev, dequant_w_f16_kernel, (unsigned)((n / 2 + 255) / 256), 256, 0, w->dtype, pl, n, (__half*)dst);
     CC_LAUNCH_CHECK(dev);
     if (cacheable) wb->f16 = dst;
     *out = dst;
@@ -396,9 +404,9 @@ int cc_launch_prefill_matmul(cc_device* dev, const cc_buf* w, const void* act_q8
     if (rc) return rc;
     {
         const int64_t na = b * k;
-        if (cc_partner_type(w->dtype) == CC_Q8_K) act_q8k_to_f16_kernel<<<(unsigned)((na / 2 + 255) / 256), 256, 0, dev->stream>>>(cc_act_q8_k((void*)act_q8_0, na), na, (__half*)s->x);
-        else if (x_f32) act_f32_to_q8f16_kernel<<<(unsigned)((na / 32 + 7) / 8), 256, 0, dev->stream>>>(x_f32, na / 32, (__half*)s->x);      // quantise + f16 in one pass
-        else act_q8_to_f16_kernel<<<(unsigned)((na / 2 + 255) / 256), 256, 0, dev->stream>>>(cc_act_q8_0((void*)act_q8_0, na), na, (__half*)s->x);
+        if (cc_partner_type(w->dtype) == CC_Q8_K) cc_launch_pdl(dev, act_q8k_to_f16_kernel, (unsigned)((na / 2 + 255) / 256), 256, 0, cc_act_q8_k((void*)act_q8_0, na), na, (__half*)s->x);
+        else if (x_f32) cc_launch_pdl(dev, act_f32_to_q8f16_kernel, (unsigned)((na / 32 + 7) / 8), 256, 0, x_f32, na / 32, (__half*)s->x);      // quantise + f16 in one pass
+        else cc_launch_pdl(dev, act_q8_to_f16_kernel, (unsigned)((na / 2 + 255) / 256), 256, 0, cc_act_q8_0((void*)act_q8_0, na), na, (__half*)s->x);
         CC_LAUNCH_CHECK(dev);
     }
     return cc_launch_prefill_operand(dev, w, out, m, k, b, nullptr);
@@ -434,6 +442,7 @@ __device__ __forceinline__ uint2 q8f16_of(float4 v) {
 // replaces it.  512 rows of 4096: copy, norm, weight and three quantisations 50 us -> 9 us
 __global__ void __launch_bounds__(CC_RED_THREADS) prefill_norm_rows_kernel(float* x, float* __restrict__ orig, const float* __restrict__ w, float eps, int cols, int write_back,
                                                                            __half* __restrict__ out) {
+    pdl_enter();
     __shared__ float sh[CC_RED_WARPS];
     float4* v = (float4*)(x + (int64_t)blockIdx.x * cols);
     const int n4 = cols >> 2;
@@ -455,6 +464,7 @@ __global__ void __launch_bounds__(CC_RED_THREADS) prefill_norm_rows_kernel(float
 }
 // silu(g) * u or gelu(g) * u (the tables of silu_kernel / gelu_kernel) -> operand.  512 rows of 14336: 77 us in three passes -> 21 us
 __global__ void __launch_bounds__(256) prefill_unit_kernel(const float4* __restrict__ g, const float4* __restrict__ u, const uint16_t* __restrict__ lut, int gelu, int64_t n4, uint2* __restrict__ out) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const bool on = i < n4;
     const float4 a = on ? g[i] : make_float4(0, 0, 0, 0), b = on ? u[i] : make_float4(0, 0, 0, 0);
@@ -466,7 +476,7 @@ int cc_prefill_rows_norm(cc_device* dev, float* x, float* orig, const float* w, 
     PgScratch* s = pg_scratch(dev);
     int rc = pg_ensure(dev, &s->x, &s->x_bytes, (size_t)rows * cols * 2);
     if (rc) return rc;
-    prefill_norm_rows_kernel<<<(unsigned)rows, CC_RED_THREADS, 0, dev->stream>>>(x, orig, w, eps, (int)cols, write_back, (__half*)s->x);
+    cc_launch_pdl(dev, prefill_norm_rows_kernel, (unsigned)rows, CC_RED_THREADS, 0, x, orig, w, eps, (int)cols, write_back, (__half*)s->x);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -474,7 +484,7 @@ int cc_prefill_rows_unit(cc_device* dev, const float* g, const float* u, bool ge
     PgScratch* s = pg_scratch(dev);
     int rc = pg_ensure(dev, &s->x, &s->x_bytes, (size_t)rows * cols * 2);
     if (rc) return rc;
-    prefill_unit_kernel<<<(unsigned)((n / 4 + 255) / 256), 256, 0, dev->stream>>>((const float4*)g, (const float4*)u, gelu ? dev->gelu_lut : dev->exp_lut, gelu, n / 4, (uint2*)s->x);
+    cc_launch_pdl(dev, prefill_unit_kernel, (unsigned)((n / 4 + 255) / 256), 256, 0, (const float4*)g, (const float4*)u, gelu ? dev->gelu_lut : dev->exp_lut, gelu, n / 4, (uint2*)s->x);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -482,7 +492,7 @@ int cc_prefill_rows_plain(cc_device* dev, const float* x, int64_t rows, int64_t 
     PgScratch* s = pg_scratch(dev);
     int rc = pg_ensure(dev, &s->x, &s->x_bytes, (size_t)rows * cols * 2);
     if (rc) return rc;
-    act_f32_to_q8f16_kernel<<<(unsigned)((rows * cols / 32 + 7) / 8), 256, 0, dev->stream>>>(x, rows * cols / 32, (__half*)s->x);
+    cc_launch_pdl(dev, act_f32_to_q8f16_kernel, (unsigned)((rows * cols / 32 + 7) / 8), 256, 0, x, rows * cols / 32, (__half*)s->x);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -491,6 +501,7 @@ int cc_prefill_rows_plain(cc_device* dev, const float* x, int64_t rows, int64_t 
 // bfloat16 once, and the same pipeline runs with the bf16 operand format ---------------------------------------------------------------
 // act: an activation applied on the way (CC_ACT_NONE: none), before the rounding
 __global__ void act_f32_to_bf16_kernel(const float* __restrict__ x, int64_t nelems, __nv_bfloat16* __restrict__ out, int act) {
+    pdl_enter();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (i >= nelems) return;
     float a = x[i], b = x[i + 1];
@@ -525,7 +536,7 @@ int cc_launch_prefill_bf16_act(cc_device* dev, const cc_buf* w, const float* x_f
     int rc = pg_ensure(dev, &s->x, &s->x_bytes, (size_t)b * k * 2);
     if (rc) return rc;
     const int64_t na = b * k;
-    act_f32_to_bf16_kernel<<<(unsigned)((na / 2 + 255) / 256), 256, 0, dev->stream>>>(x_f32, na, (__nv_bfloat16*)s->x, act);
+    cc_launch_pdl(dev, act_f32_to_bf16_kernel, (unsigned)((na / 2 + 255) / 256), 256, 0, x_f32, na, (__nv_bfloat16*)s->x, act);
     CC_LAUNCH_CHECK(dev);
     return cc_launch_prefill_bf16_operand(dev, w, out, m, k, b, 0);
 }
@@ -554,7 +565,7 @@ int cc_launch_grouped_bf16(cc_device* dev, const cc_buf* w_stack, int64_t n_grou
         const size_t smem = (size_t)pg_stages(BN, MT) * (MT * PG_BLOCK_M + BN) * PG_BLOCK_K * 2 + 1024;                                          \
         CC_CUDA(dev, cudaFuncSetAttribute(umma_gemm_kernel<BN, MT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                  \
         dim3 grid((unsigned)((m + PG_BLOCK_M * MT - 1) / (PG_BLOCK_M * MT)), (unsigned)max_tiles);                                               \
-        umma_gemm_kernel<BN, MT, 1><<<grid, PG_THREADS, smem, dev->stream>>>(tw, tx, out, (int)m, 0, (int)k, groups_dev);                          \
+        cc_launch_pdl(dev, umma_gemm_kernel<BN, MT, 1>, grid, PG_THREADS, smem, tw, tx, out, (int)m, 0, (int)k, groups_dev, (const float*)nullptr);   \
     } while (0)
     if (block_n == 128) { if (mt2) PG_GROUPED(128, 2); else PG_GROUPED(128, 1); }
     else { if (mt2) PG_GROUPED(64, 2); else PG_GROUPED(64, 1); }

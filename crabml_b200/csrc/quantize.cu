@@ -44,6 +44,7 @@ ActQ8_K cc_act_q8_k(void* s, int64_t n) {
 
 // one warp per 32-element block, lane = element
 __global__ void quantize_q8_0_kernel(const float* __restrict__ x, int64_t nblocks, ActQ8_0 a) {
+    pdl_enter();
     int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (b >= nblocks) return;
@@ -60,6 +61,7 @@ __global__ void quantize_q8_0_kernel(const float* __restrict__ x, int64_t nblock
 }
 
 __global__ void quantize_q8_1_kernel(const float* __restrict__ x, int64_t nblocks, ActQ8_1 a) {
+    pdl_enter();
     int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (b >= nblocks) return;
@@ -76,6 +78,7 @@ __global__ void quantize_q8_1_kernel(const float* __restrict__ x, int64_t nblock
 
 // one warp per 256-element super-block; lane handles elements lane*8 .. lane*8+7 (cc_quant_q8k_sblock, quantize_dev.cuh)
 __global__ void quantize_q8_k_kernel(const float* __restrict__ x, int64_t nsb, ActQ8_K a) {
+    pdl_enter();
     int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (b >= nsb) return;
@@ -86,7 +89,7 @@ __global__ void quantize_q8_k_kernel(const float* __restrict__ x, int64_t nsb, A
     cc_quant_q8k_sblock(v, lane, a.qs + b * 256, a.d + b, a.bsums + b * 16);
 }
 
-__global__ void quantize_f16_kernel(const float* __restrict__ x, int64_t n, __half* out) {   // buf/api.rs:198
+__global__ void quantize_f16_kernel(const float* __restrict__ x, int64_t n, __half* out) { pdl_enter();   // buf/api.rs:198
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = __float2half_rn(x[i]);
 }
@@ -97,26 +100,26 @@ int cc_launch_quantize(cc_device* dev, const float* x, int64_t n, int act_type, 
         CC_REQUIRE(dev, n % 32 == 0, "quantize q8_0: length %lld %% 32 != 0", (long long)n);
         int64_t nb = n / 32;
         if (nb == 0) return CC_OK;
-        quantize_q8_0_kernel<<<(unsigned)((nb + 7) / 8), 256, 0, dev->stream>>>(x, nb, cc_act_q8_0(scratch, n));
+        cc_launch_pdl(dev, quantize_q8_0_kernel, (unsigned)((nb + 7) / 8), 256, 0, x, nb, cc_act_q8_0(scratch, n));
         break;
     }
     case CC_Q8_1: {
         CC_REQUIRE(dev, n % 32 == 0, "quantize q8_1: length %lld %% 32 != 0", (long long)n);
         int64_t nb = n / 32;
         if (nb == 0) return CC_OK;
-        quantize_q8_1_kernel<<<(unsigned)((nb + 7) / 8), 256, 0, dev->stream>>>(x, nb, cc_act_q8_1(scratch, n));
+        cc_launch_pdl(dev, quantize_q8_1_kernel, (unsigned)((nb + 7) / 8), 256, 0, x, nb, cc_act_q8_1(scratch, n));
         break;
     }
     case CC_Q8_K: {
         CC_REQUIRE(dev, n % 256 == 0, "quantize q8_k: length %lld %% 256 != 0", (long long)n);
         int64_t nb = n / 256;
         if (nb == 0) return CC_OK;
-        quantize_q8_k_kernel<<<(unsigned)((nb + 7) / 8), 256, 0, dev->stream>>>(x, nb, cc_act_q8_k(scratch, n));
+        cc_launch_pdl(dev, quantize_q8_k_kernel, (unsigned)((nb + 7) / 8), 256, 0, x, nb, cc_act_q8_k(scratch, n));
         break;
     }
     case CC_F16:
         if (n == 0) return CC_OK;
-        quantize_f16_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(x, n, (__half*)scratch);
+        cc_launch_pdl(dev, quantize_f16_kernel, (unsigned)((n + 255) / 256), 256, 0, x, n, (__half*)scratch);
         break;
     default:
         return cc_fail(dev, CC_ERR_TENSOR, "quantize to type %d is not supported", act_type);
@@ -128,6 +131,7 @@ int cc_launch_quantize(cc_device* dev, const float* x, int64_t n, int act_type, 
 // reassemble reference-layout blocks (for cc_test_quantize_activation): one thread per block
 __global__ void act_to_blocks_kernel(int t, const void* scratch, int64_t n, uint8_t* out,
                                      ActQ8_0 a0, ActQ8_1 a1, ActQ8_K ak) {
+    pdl_enter();
     int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t == CC_Q8_0) {
         if (b >= n / 32) return;
@@ -157,8 +161,7 @@ __global__ void act_to_blocks_kernel(int t, const void* scratch, int64_t n, uint
 int cc_launch_act_to_blocks(cc_device* dev, const void* scratch, int64_t n, int t, uint8_t* blocks_dev) {
     int64_t nb = n / (t == CC_Q8_K ? 256 : 32);
     if (nb == 0) return CC_OK;
-    act_to_blocks_kernel<<<(unsigned)((nb + 127) / 128), 128, 0, dev->stream>>>(
-        t, scratch, n, blocks_dev, cc_act_q8_0((void*)scratch, n), cc_act_q8_1((void*)scratch, n), cc_act_q8_k((void*)scratch, n));
+    cc_launch_pdl(dev, act_to_blocks_kernel, (unsigned)((nb + 127) / 128), 128, 0, t, scratch, n, blocks_dev, cc_act_q8_0((void*)scratch, n), cc_act_q8_1((void*)scratch, n), cc_act_q8_k((void*)scratch, n));
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }

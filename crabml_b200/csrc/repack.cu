@@ -119,6 +119,7 @@ int cc_launch_unrepack(cc_device* dev, const cc_buf* src, uint8_t* gguf_dev) {
 
 __global__ void dequant_rows_kernel(int t, DeqPlanes P, const int64_t* rows, int n_rows, int64_t cols,
                                     float* dst_f32, __half* dst_f16) {
+    pdl_enter();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)n_rows * cols) return;
     int64_t r = i / cols, c = i - r * cols;
@@ -137,8 +138,7 @@ int cc_launch_dequant_rows(cc_device* dev, const cc_buf* src, const int64_t* row
     P.cols = src->cols > 0 ? src->cols : cols;
     int64_t total = (int64_t)n_rows * cols;
     if (total == 0) return CC_OK;
-    dequant_rows_kernel<<<(unsigned)((total + 255) / 256), 256, 0, dev->stream>>>(
-        src->dtype, P, rows_dev, n_rows, cols, dst_dtype == CC_F32 ? (float*)dst : nullptr,
+    cc_launch_pdl(dev, dequant_rows_kernel, (unsigned)((total + 255) / 256), 256, 0, src->dtype, P, rows_dev, n_rows, cols, dst_dtype == CC_F32 ? (float*)dst : nullptr,
         dst_dtype == CC_F16 ? (__half*)dst : nullptr);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;

@@ -60,6 +60,7 @@ extern "C" CC_API int cc_tensor_zero(cc_device* dev, const cc_view* x) {
 // one warp per row: lane-strided sum of squares, butterfly, then the scaled write
 __global__ void rms_norm_gain_kernel(float* __restrict__ dst, const float* __restrict__ y, const float* __restrict__ gain, int gain_n, int rows, int cols,
                                      float eps, int accumulate, float mult) {
+    pdl_enter();
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= rows) return;
     const float* yr = y + (int64_t)r * cols;
@@ -78,6 +79,7 @@ __global__ void rms_norm_gain_kernel(float* __restrict__ dst, const float* __res
 #define RNG_THREADS 256
 __global__ void __launch_bounds__(RNG_THREADS) rms_norm_gain_wide_kernel(float* __restrict__ dst, const float* __restrict__ y, const float* __restrict__ gain, int gain_n, int cols,
                                                                          float eps, int accumulate, float mult) {
+    pdl_enter();
     __shared__ float red[RNG_THREADS / 32];
     const float* yr = y + (int64_t)blockIdx.x * cols;
     float* dr = dst + (int64_t)blockIdx.x * cols;
@@ -102,8 +104,8 @@ static int rms_norm_gain_impl(cc_device* dev, const cc_view* dst, const cc_view*
     const int64_t rows = y->shape[0], cols = y->shape[1], gn = view_len(gain);
     CC_REQUIRE(dev, gn == 1 || gn == cols, "rms_norm_gain: gain has %lld elements, need 1 or %lld", (long long)gn, (long long)cols);
     if (rows == 0) return CC_OK;
-    if (cols >= 512) rms_norm_gain_wide_kernel<<<(unsigned)rows, RNG_THREADS, 0, dev->stream>>>(fptr(dst), fptr(y), fptr(gain), (int)gn, (int)cols, eps, accumulate, mult);
-    else rms_norm_gain_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, dev->stream>>>(fptr(dst), fptr(y), fptr(gain), (int)gn, (int)rows, (int)cols, eps, accumulate, mult);
+    if (cols >= 512) cc_launch_pdl(dev, rms_norm_gain_wide_kernel, (unsigned)rows, RNG_THREADS, 0, fptr(dst), fptr(y), fptr(gain), (int)gn, (int)cols, eps, accumulate, mult);
+    else cc_launch_pdl(dev, rms_norm_gain_kernel, (unsigned)((rows + 7) / 8), 256, 0, fptr(dst), fptr(y), fptr(gain), (int)gn, (int)rows, (int)cols, eps, accumulate, mult);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -118,6 +120,7 @@ extern "C" CC_API int cc_rms_norm_gain_mult(cc_device* dev, const cc_view* dst, 
 // w_heads: how many heads have weights of their own (1: one vector for all)
 __global__ void gated_head_rms_norm_kernel(float* __restrict__ x, const float* __restrict__ gate, const float* __restrict__ w, int64_t n_units, int hs, float eps, int act,
                                            int w_heads) {
+    pdl_enter();
     const int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (u >= n_units) return;
@@ -149,13 +152,14 @@ extern "C" CC_API int cc_gated_head_rms_norm(cc_device* dev, const cc_view* x, c
     }
     const int64_t units = n / head_size;
     if (!units) return CC_OK;
-    gated_head_rms_norm_kernel<<<(unsigned)((units + 7) / 8), 256, 0, dev->stream>>>(fptr(x), gate ? fptr(gate) : nullptr, w ? fptr(w) : nullptr, units, head_size, eps, gate_act,
+    cc_launch_pdl(dev, gated_head_rms_norm_kernel, (unsigned)((units + 7) / 8), 256, 0, fptr(x), gate ? fptr(gate) : nullptr, w ? fptr(w) : nullptr, units, head_size, eps, gate_act,
                                                                                     w_heads);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 
 __global__ void glu_kernel(float* __restrict__ g, const float* __restrict__ u, int64_t n, int act) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) g[i] = seq_act(g[i], act) * u[i];
 }
@@ -165,11 +169,12 @@ extern "C" CC_API int cc_glu_inplace(cc_device* dev, const cc_view* gate, const 
     const int64_t n = view_len(gate);
     CC_REQUIRE(dev, view_len(up) == n, "glu_inplace: sizes differ");
     if (!n) return CC_OK;
-    glu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(gate), fptr(up), n, act);
+    cc_launch_pdl(dev, glu_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(gate), fptr(up), n, act);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 __global__ void activate_kernel(float* __restrict__ x, int64_t n, int act) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = seq_act(x[i], act);
 }
@@ -178,11 +183,12 @@ extern "C" CC_API int cc_activate_inplace(cc_device* dev, const cc_view* x, int3
     SEQ_F32(dev, x, "activate_inplace x");
     const int64_t n = view_len(x);
     if (!n) return CC_OK;
-    activate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(x), n, act);
+    cc_launch_pdl(dev, activate_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(x), n, act);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 __global__ void softcap_kernel(float* __restrict__ x, int64_t n, float cap) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = cap * tanhf(x[i] / cap);
 }
@@ -192,12 +198,13 @@ extern "C" CC_API int cc_softcap_inplace(cc_device* dev, const cc_view* x, float
     CC_REQUIRE(dev, cap > 0.0f, "softcap_inplace: the cap must be positive");
     const int64_t n = view_len(x);
     if (!n) return CC_OK;
-    softcap_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(x), n, cap);
+    cc_launch_pdl(dev, softcap_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(x), n, cap);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 // gate | up side by side in one product's rows
 __global__ void glu_halves_kernel(const float* __restrict__ src, const float* __restrict__ bias, float* __restrict__ out, int64_t n, int ff, int act) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t r = i / ff;
@@ -219,11 +226,12 @@ extern "C" CC_API int cc_glu_halves(cc_device* dev, const cc_view* src, const cc
     *out = o;
     const int64_t n = rows * ff;
     if (!n) return CC_OK;
-    glu_halves_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(src), bias ? fptr(bias) : nullptr, (float*)o->base, n, (int)ff, act);
+    cc_launch_pdl(dev, glu_halves_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(src), bias ? fptr(bias) : nullptr, (float*)o->base, n, (int)ff, act);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 __global__ void add_row_bias_kernel(float* __restrict__ x, const float* __restrict__ b, int64_t n, int cols) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] += b[i % cols];
 }
@@ -233,11 +241,12 @@ extern "C" CC_API int cc_add_row_bias(cc_device* dev, const cc_view* x, const cc
     CC_REQUIRE(dev, x->ndim == 2 && view_len(bias) == x->shape[1], "add_row_bias: x must be [rows, cols] and bias [cols]");
     const int64_t n = view_len(x);
     if (!n) return CC_OK;
-    add_row_bias_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(x), fptr(bias), n, (int)x->shape[1]);
+    cc_launch_pdl(dev, add_row_bias_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(x), fptr(bias), n, (int)x->shape[1]);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 __global__ void scaled_sum_kernel(float* __restrict__ dst, const float* __restrict__ a, float sa, const float* __restrict__ b, float sb, int64_t n) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = sa * a[i] + sb * b[i];
 }
@@ -247,13 +256,14 @@ extern "C" CC_API int cc_scaled_sum(cc_device* dev, const cc_view* dst, const cc
     const int64_t n = view_len(dst);
     CC_REQUIRE(dev, view_len(a) == n && view_len(b) == n, "scaled_sum: sizes differ");
     if (!n) return CC_OK;
-    scaled_sum_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(dst), fptr(a), sa, fptr(b), sb, n);
+    cc_launch_pdl(dev, scaled_sum_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(dst), fptr(a), sa, fptr(b), sb, n);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 
 __global__ void scaled_sum_accumulate_kernel(float* __restrict__ dst, const float* __restrict__ a, float sa, const float* __restrict__ b, float sb, const float* __restrict__ c,
                                              int64_t n) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float v = sa * a[i] + sb * b[i];
@@ -267,12 +277,13 @@ extern "C" CC_API int cc_scaled_sum_accumulate(cc_device* dev, const cc_view* ds
     const int64_t n = view_len(dst);
     CC_REQUIRE(dev, view_len(a) == n && view_len(b) == n && (!c || view_len(c) == n), "scaled_sum_accumulate: sizes differ");
     if (!n) return CC_OK;
-    scaled_sum_accumulate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(dst), fptr(a), sa, fptr(b), sb, c ? fptr(c) : nullptr, n);
+    cc_launch_pdl(dev, scaled_sum_accumulate_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(dst), fptr(a), sa, fptr(b), sb, c ? fptr(c) : nullptr, n);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
 // one gate number per (row, head): one thread per element
 __global__ void head_gate_kernel(float* __restrict__ x, const float* __restrict__ g, int64_t n, int hs, int heads, int64_t grs, int act) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t u = i / hs, t = u / heads;
@@ -285,7 +296,7 @@ static int head_gate_impl(cc_device* dev, const cc_view* x, const cc_view* g, in
                "head_gate: x must be [rows, heads * head_size] and g hold %d columns from column %d on", n_heads, col0);
     const int64_t n = view_len(x);
     if (!n) return CC_OK;
-    head_gate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(x), fptr(g) + col0, n, (int)(x->shape[1] / n_heads), n_heads, g->strides[0], act);
+    cc_launch_pdl(dev, head_gate_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(x), fptr(g) + col0, n, (int)(x->shape[1] / n_heads), n_heads, g->strides[0], act);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -299,6 +310,7 @@ extern "C" CC_API int cc_head_gate_cols(cc_device* dev, const cc_view* x, const 
 }
 // out = [a | b] row by row: one thread per element of out
 __global__ void concat_cols_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, int64_t n, int ca, int cb) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t r = i / (ca + cb);
@@ -317,7 +329,7 @@ extern "C" CC_API int cc_concat_cols(cc_device* dev, const cc_view* a, const cc_
     *out = o;
     const int64_t n = rows * (ca + cb);
     if (!n) return CC_OK;
-    concat_cols_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(a), fptr(b), (float*)o->base, n, (int)ca, (int)cb);
+    cc_launch_pdl(dev, concat_cols_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(a), fptr(b), (float*)o->base, n, (int)ca, (int)cb);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -326,6 +338,7 @@ extern "C" CC_API int cc_concat_cols(cc_device* dev, const cc_view* a, const cc_
 // one thread per (token, column); the hash is taken in 64-bit integers
 __global__ void pair_hash_rows_add_kernel(float* __restrict__ dst, const float* __restrict__ table, const int64_t* __restrict__ tok, const int32_t* __restrict__ last, int64_t n,
                                           int cols, int64_t mul_prev, int64_t mul_cur, int64_t buckets) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t t = i / cols;
@@ -334,7 +347,7 @@ __global__ void pair_hash_rows_add_kernel(float* __restrict__ dst, const float* 
     const int64_t row = prev < 0 ? buckets : (prev * mul_prev + tok[t] * mul_cur) % buckets;
     dst[i] += table[row * cols + c];
 }
-__global__ void pair_hash_last_kernel(const int64_t* __restrict__ tok, int32_t* __restrict__ last, int n) { last[0] = (int32_t)tok[n - 1] + 1; }
+__global__ void pair_hash_last_kernel(const int64_t* __restrict__ tok, int32_t* __restrict__ last, int n) { pdl_enter(); last[0] = (int32_t)tok[n - 1] + 1; }
 extern "C" CC_API int cc_pair_hash_rows_add(cc_device* dev, const cc_view* dst, const cc_view* table, const int64_t* tokens, int32_t n, int32_t slot, const cc_view* last,
                                             int64_t mul_prev, int64_t mul_cur, int64_t buckets) {
     SEQ_ENTER(dev, "pair_hash_rows_add");
@@ -359,9 +372,9 @@ extern "C" CC_API int cc_pair_hash_rows_add(cc_device* dev, const cc_view* dst, 
     }
     const int64_t total = (int64_t)n * dst->shape[1];
     int32_t* lp = (int32_t*)last->buf->plane[0];
-    pair_hash_rows_add_kernel<<<(unsigned)((total + 255) / 256), 256, 0, dev->stream>>>(fptr(dst), fptr(table), tok, lp, total, (int)dst->shape[1], mul_prev, mul_cur, buckets);
+    cc_launch_pdl(dev, pair_hash_rows_add_kernel, (unsigned)((total + 255) / 256), 256, 0, fptr(dst), fptr(table), tok, lp, total, (int)dst->shape[1], mul_prev, mul_cur, buckets);
     dev->launches++;
-    pair_hash_last_kernel<<<1, 1, 0, dev->stream>>>(tok, lp, n);
+    cc_launch_pdl(dev, pair_hash_last_kernel, 1, 1, 0, tok, lp, n);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -371,6 +384,7 @@ extern "C" CC_API int cc_pair_hash_rows_add(cc_device* dev, const cc_view* dst, 
 // in_bias (or NULL) is added to every input of x as it is read; the tail holds inputs that already carry it (or the zeros before a sequence)
 __global__ void short_conv_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ tail,
                                   float* __restrict__ y, int T, int C, int K, int hs, int act, int unit, float ueps, float uscale, const float* __restrict__ in_bias, int64_t xrs) {
+    pdl_enter();
     const int heads = C / hs;
     const int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -403,6 +417,7 @@ __device__ __forceinline__ void short_conv_new_tail(const float* x, float* tail,
     }
 }
 __global__ void short_conv_tail_kernel(const float* __restrict__ x, float* tail, int T, int C, int K, const float* __restrict__ in_bias, int64_t xrs) {
+    pdl_enter();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < C) short_conv_new_tail(x, tail, T, C, K, in_bias, xrs, c);
 }
@@ -411,6 +426,7 @@ __global__ void short_conv_tail_kernel(const float* __restrict__ x, float* tail,
 #define SC_FEW_ROWS 8
 __global__ void short_conv_few_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float* tail, float* __restrict__ y, int T, int C,
                                       int K, int act, const float* __restrict__ in_bias, int64_t xrs) {
+    pdl_enter();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     for (int t = 0; t < T; t++) {
@@ -454,16 +470,16 @@ static int short_conv_impl(cc_device* dev, const cc_view* x, const cc_view* w, c
     if (T == 0) return CC_OK;
     const float* tp = K > 1 ? fptr(tail) : nullptr;
     if (K > 1 && T <= SC_FEW_ROWS && !unit_norm) {
-        short_conv_few_kernel<<<(unsigned)((C + 127) / 128), 128, 0, dev->stream>>>(xp, fptr(w), bias ? fptr(bias) : nullptr, fptr(tail), (float*)y->base, (int)T, (int)C, (int)K, act, ibp, xrs);
+        cc_launch_pdl(dev, short_conv_few_kernel, (unsigned)((C + 127) / 128), 128, 0, xp, fptr(w), bias ? fptr(bias) : nullptr, fptr(tail), (float*)y->base, (int)T, (int)C, (int)K, act, ibp, xrs);
         CC_LAUNCH_CHECK(dev);
         return CC_OK;
     }
     const int64_t units = T * (C / hs);
-    short_conv_kernel<<<(unsigned)((units + 7) / 8), 256, 0, dev->stream>>>(xp, fptr(w), bias ? fptr(bias) : nullptr, tp, (float*)y->base, (int)T, (int)C, (int)K, hs, act, unit_norm,
+    cc_launch_pdl(dev, short_conv_kernel, (unsigned)((units + 7) / 8), 256, 0, xp, fptr(w), bias ? fptr(bias) : nullptr, tp, (float*)y->base, (int)T, (int)C, (int)K, hs, act, unit_norm,
                                                                         unit_eps, unit_scale, ibp, xrs);
     CC_LAUNCH_CHECK(dev);
     if (K > 1) {
-        short_conv_tail_kernel<<<(unsigned)((C + 127) / 128), 128, 0, dev->stream>>>(xp, fptr(tail), (int)T, (int)C, (int)K, ibp, xrs);
+        cc_launch_pdl(dev, short_conv_tail_kernel, (unsigned)((C + 127) / 128), 128, 0, xp, fptr(tail), (int)T, (int)C, (int)K, ibp, xrs);
         CC_LAUNCH_CHECK(dev);
     }
     return CC_OK;
@@ -490,6 +506,7 @@ extern "C" CC_API int cc_short_conv_cols(cc_device* dev, const cc_view* src, int
 // beta / decay of every (token, head): bd[(t * H + h) * 2] = {sigmoid(b), exp(-exp(a_log) * softplus(a + dt_bias))}
 __global__ void delta_gates_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                                    float* __restrict__ bd, int64_t n, int H) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int h = (int)(i % H);
@@ -523,6 +540,7 @@ template <int DK, int SPLIT, int THREADS>
 __global__ void __launch_bounds__(THREADS) delta_rule_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                                              const float* __restrict__ bd, float* __restrict__ state, float* __restrict__ o, int T, int H, int G,
                                                              int dk, int dv) {
+    pdl_enter();
     extern __shared__ __align__(16) float dr_sm[];            // two staging buffers, then the state columns (DK == 0) or the shares of out (DK > 0)
     constexpr int DKP = DK > 0 ? DK / SPLIT : 4;
     constexpr int COLS = THREADS / SPLIT;
@@ -678,7 +696,7 @@ extern "C" CC_API int cc_gated_delta_rule(cc_device* dev, const cc_view* q, cons
     void* bdp = nullptr; size_t cls = 0;
     rc = cc_pool_alloc(dev, (size_t)T * H * 2 * 4, &bdp, &cls);
     if (rc) return rc;
-    delta_gates_kernel<<<(unsigned)((T * H + 255) / 256), 256, 0, dev->stream>>>(fptr(a), fptr(b), fptr(a_log), fptr(dt_bias), (float*)bdp, T * H, H);
+    cc_launch_pdl(dev, delta_gates_kernel, (unsigned)((T * H + 255) / 256), 256, 0, fptr(a), fptr(b), fptr(a_log), fptr(dt_bias), (float*)bdp, T * H, H);
     dev->launches++;
     const bool split = dk == 32 || dk == 64 || dk == 128;
     const int threads = split ? DR_SPLIT_THREADS : DR_THREADS, cols = split ? DR_SPLIT_THREADS / (dk / 16) : DR_THREADS;
@@ -695,10 +713,10 @@ extern "C" CC_API int cc_gated_delta_rule(cc_device* dev, const cc_view* q, cons
             : dk == 128 ? cudaFuncSetAttribute(delta_rule_kernel<128, 8, DR_SPLIT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
                         : cudaFuncSetAttribute(delta_rule_kernel<0, 1, DR_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) { cc_pool_free(dev, bdp, cls); return cc_fail(dev, CC_ERR_CUDA, "gated_delta_rule: %s", cudaGetErrorString(e)); }
-    if (dk == 32) delta_rule_kernel<32, 2, DR_SPLIT_THREADS><<<grid, threads, smem, dev->stream>>>(DR_ARGS);
-    else if (dk == 64) delta_rule_kernel<64, 4, DR_SPLIT_THREADS><<<grid, threads, smem, dev->stream>>>(DR_ARGS);
-    else if (dk == 128) delta_rule_kernel<128, 8, DR_SPLIT_THREADS><<<grid, threads, smem, dev->stream>>>(DR_ARGS);
-    else delta_rule_kernel<0, 1, DR_THREADS><<<grid, threads, smem, dev->stream>>>(DR_ARGS);
+    if (dk == 32) cc_launch_pdl(dev, delta_rule_kernel<32, 2, DR_SPLIT_THREADS>, grid, threads, smem, DR_ARGS);
+    else if (dk == 64) cc_launch_pdl(dev, delta_rule_kernel<64, 4, DR_SPLIT_THREADS>, grid, threads, smem, DR_ARGS);
+    else if (dk == 128) cc_launch_pdl(dev, delta_rule_kernel<128, 8, DR_SPLIT_THREADS>, grid, threads, smem, DR_ARGS);
+    else cc_launch_pdl(dev, delta_rule_kernel<0, 1, DR_THREADS>, grid, threads, smem, DR_ARGS);
 #undef DR_ARGS
     cc_pool_free(dev, bdp, cls);            // stream-ordered pool: the next user of this block runs after the kernels above
     CC_LAUNCH_CHECK(dev);
@@ -709,6 +727,7 @@ extern "C" CC_API int cc_gated_delta_rule(cc_device* dev, const cc_view* q, cons
 // one warp per (token, kv head)
 __global__ void kv_ring_append_kernel(float* __restrict__ kring, float* __restrict__ vring, const float* __restrict__ k, const float* __restrict__ v,
                                       const float* __restrict__ knw, float eps, int64_t pos0, int ring, int T, int G, int dk, int dv) {
+    pdl_enter();
     const int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (u >= (int64_t)T * G) return;
@@ -740,7 +759,7 @@ extern "C" CC_API int cc_kv_ring_append(cc_device* dev, const cc_view* kring, co
                "kv_ring_append: operand sizes do not fit kv=%d dk=%d dv=%d", G, dk, dv);
     CC_REQUIRE(dev, T <= ring, "kv_ring_append: %lld tokens do not fit a ring of %lld", (long long)T, (long long)ring);
     if (T == 0) return CC_OK;
-    kv_ring_append_kernel<<<(unsigned)((T * G + 7) / 8), 256, 0, dev->stream>>>(fptr(kring), fptr(vring), fptr(k), fptr(v), knw ? fptr(knw) : nullptr, eps, pos0, (int)ring,
+    cc_launch_pdl(dev, kv_ring_append_kernel, (unsigned)((T * G + 7) / 8), 256, 0, fptr(kring), fptr(vring), fptr(k), fptr(v), knw ? fptr(knw) : nullptr, eps, pos0, (int)ring,
                                                                              (int)T, G, dk, dv);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
@@ -773,6 +792,7 @@ __host__ __device__ __forceinline__ int64_t wa_lo(const WaGeom& g, int64_t i) {
 }
 
 __global__ void head_rms_norm_kernel(float* __restrict__ x, const float* __restrict__ w, int64_t n_units, int hs, float eps) {
+    pdl_enter();
     const int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (u >= n_units) return;
@@ -818,6 +838,7 @@ __device__ __forceinline__ int64_t wa_score_at(const WaTile& t, int q_tiles, int
 // ring_base0: the ring's row of position base0; lo0: the first position anybody sees
 __global__ void __launch_bounds__(256) wa_cut_kernel(const float* __restrict__ q, const float* __restrict__ kring, const float* __restrict__ vring, uint8_t* __restrict__ qc,
                                                      uint8_t* __restrict__ kc, uint8_t* __restrict__ vc, WaGeom g, int q_tiles, unsigned row_blocks, int ring_base0, int lo0, int vec) {
+    pdl_enter();
     const int last = (int)(g.pos0 + g.T - 1 - g.base0);       // positions are counted from base0
     const unsigned q_rows = (unsigned)(g.G * q_tiles) * WA_ROWS, k_rows = (unsigned)(g.G * g.span);
     float v[8];
@@ -1047,6 +1068,7 @@ struct WaValues {
 #define WS_KEEP 20
 __global__ void __launch_bounds__(256) wa_scores_row_kernel(const float* __restrict__ q, const float* __restrict__ kring, float* __restrict__ S, WaGeom g, float scale,
                                                             const float* __restrict__ r1, const float* __restrict__ r2) {
+    pdl_enter();
     extern __shared__ float wsr_sm[];             // [heads of the block][dk]
     const int hblocks = (g.R + WS_HEADS - 1) / WS_HEADS;
     const int t = blockIdx.y, kvh = blockIdx.z / hblocks, h0 = (blockIdx.z % hblocks) * WS_HEADS, nh = min(WS_HEADS, g.R - h0);
@@ -1097,6 +1119,7 @@ __global__ void __launch_bounds__(256) wa_scores_row_kernel(const float* __restr
 template <int RB>
 __global__ void __cluster_dims__(1, 1, WV_SPLIT) __launch_bounds__(WV_THREADS) wa_values_slices_kernel(const float* __restrict__ S, const float* __restrict__ vring, float* __restrict__ out,
                                                                                                        WaGeom g, const float* __restrict__ sink, int slice_cap) {
+    pdl_enter();
     extern __shared__ float wv_sm[];
     float* pr = wv_sm;                                        // [RB][slice_cap]
     float* part = wv_sm + (size_t)RB * slice_cap;             // [WV_WARPS][RB][32]
@@ -1175,7 +1198,7 @@ static size_t wa_slices_smem(int RB, int64_t maxn, int* slice_cap) {
 template <int RB>
 static cudaError_t wa_launch_slices(cc_device* dev, const float* S, const float* v, float* out, const WaGeom& g, const float* sink, size_t smem, int slice_cap) {
     if (smem > 40 * 1024) { cudaError_t e = cudaFuncSetAttribute(wa_values_slices_kernel<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) return e; }
-    wa_values_slices_kernel<RB><<<dim3((unsigned)(g.T * g.G * ((g.R + RB - 1) / RB)), (unsigned)((g.dv + 31) / 32), WV_SPLIT), WV_THREADS, smem, dev->stream>>>(S, v, out, g, sink, slice_cap);
+    cc_launch_pdl(dev, wa_values_slices_kernel<RB>, dim3((unsigned)(g.T * g.G * ((g.R + RB - 1) / RB)), (unsigned)((g.dv + 31) / 32), WV_SPLIT), WV_THREADS, smem, S, v, out, g, sink, slice_cap);
     return cudaSuccess;
 }
 static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view* qnw, float eps, const cc_view* kring, const cc_view* vring, int64_t pos0, int32_t H, int32_t G,
@@ -1233,7 +1256,7 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
     float* qp = fptr(q);
     if (qnw) {             // the query norm, in place: q is this call's private projection output in every caller of the runner; a caller that
                            // needs its q untouched passes a copy
-        head_rms_norm_kernel<<<(unsigned)((T * H + 7) / 8), 256, 0, dev->stream>>>(qp, fptr(qnw), T * H, dk, eps);
+        cc_launch_pdl(dev, head_rms_norm_kernel, (unsigned)((T * H + 7) / 8), 256, 0, qp, fptr(qnw), T * H, dk, eps);
         dev->launches++;
     }
     void* Sp = nullptr; size_t cls = 0;
@@ -1258,7 +1281,7 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
         if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &ws.maps[1], kp3, (int64_t)3 * G * g.span, g.dkp, WaScores::N);
         if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &vmap, vp3, (int64_t)3 * G * g.dvp, g.span, vtile);
         if (rc == CC_OK) {
-            wa_cut_kernel<<<(unsigned)blocks, 256, 0, dev->stream>>>(qp, fptr(kring), vptr, qp3, kp3, vp3, g, q_tiles, (unsigned)row_blocks, (int)(g.base0 % ring), (int)(oldest - g.base0), vec);
+            cc_launch_pdl(dev, wa_cut_kernel, (unsigned)blocks, 256, 0, qp, fptr(kring), vptr, qp3, kp3, vp3, g, q_tiles, (unsigned)row_blocks, (int)(g.base0 % ring), (int)(oldest - g.base0), vec);
             dev->launches++;
             rc = sg_launch(dev, ws, (int64_t)key_tiles * q_tiles * G);
         }
@@ -1273,7 +1296,7 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
     rc = cc_pool_alloc(dev, (size_t)T * H * g.cap * 4, &Sp, &cls);
     if (rc) return rc;
     if (rows_smem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(wa_scores_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem); if (e != cudaSuccess) { cc_pool_free(dev, Sp, cls); return cc_fail(dev, CC_ERR_CUDA, "window_attention: %s", cudaGetErrorString(e)); } }
-    wa_scores_row_kernel<<<dim3((unsigned)((maxn + 15) / 16), (unsigned)T, (unsigned)(G * ((R + WS_HEADS - 1) / WS_HEADS))), 256, rows_smem, dev->stream>>>(qp, fptr(kring), (float*)Sp, g, scale, r1p, r2p);
+    cc_launch_pdl(dev, wa_scores_row_kernel, dim3((unsigned)((maxn + 15) / 16), (unsigned)T, (unsigned)(G * ((R + WS_HEADS - 1) / WS_HEADS))), 256, rows_smem, qp, fptr(kring), (float*)Sp, g, scale, r1p, r2p);
     dev->launches++;
     cudaError_t e = RB == 8 ? wa_launch_slices<8>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap)
                   : RB == 4 ? wa_launch_slices<4>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap)
@@ -1307,6 +1330,7 @@ extern "C" CC_API int cc_window_attention(cc_device* dev, const cc_view* q, cons
 // ---- RMS norm in groups ----------------------------------------------------------------------------------------------------------------
 // one warp per (row, group): the units are consecutive in memory, unit u covers x[u * gs, (u + 1) * gs)
 __global__ void group_rms_norm_kernel(float* __restrict__ dst, const float* __restrict__ x, const float* __restrict__ w, int64_t n_units, int groups, int gs, float eps) {
+    pdl_enter();
     const int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (u >= n_units) return;
@@ -1321,6 +1345,7 @@ __global__ void group_rms_norm_kernel(float* __restrict__ dst, const float* __re
 }
 // a wide group: one CTA per (row, group), the order of rms_norm_gain_wide_kernel
 __global__ void __launch_bounds__(RNG_THREADS) group_rms_norm_wide_kernel(float* __restrict__ dst, const float* __restrict__ x, const float* __restrict__ w, int groups, int gs, float eps) {
+    pdl_enter();
     __shared__ float red[RNG_THREADS / 32];
     const int64_t u = blockIdx.x;
     const float* xr = x + u * gs;
@@ -1345,8 +1370,8 @@ extern "C" CC_API int cc_group_rms_norm(cc_device* dev, const cc_view* dst, cons
     CC_REQUIRE(dev, groups >= 1 && cols % groups == 0 && view_len(w) == cols, "group_rms_norm: %lld columns, %d groups, %lld weights", (long long)cols, groups, (long long)view_len(w));
     if (rows == 0) return CC_OK;
     const int64_t units = rows * groups;
-    if (cols / groups >= 512) group_rms_norm_wide_kernel<<<(unsigned)units, RNG_THREADS, 0, dev->stream>>>(fptr(dst), fptr(x), fptr(w), groups, (int)(cols / groups), eps);
-    else group_rms_norm_kernel<<<(unsigned)((units + 7) / 8), 256, 0, dev->stream>>>(fptr(dst), fptr(x), fptr(w), units, groups, (int)(cols / groups), eps);
+    if (cols / groups >= 512) cc_launch_pdl(dev, group_rms_norm_wide_kernel, (unsigned)units, RNG_THREADS, 0, fptr(dst), fptr(x), fptr(w), groups, (int)(cols / groups), eps);
+    else cc_launch_pdl(dev, group_rms_norm_kernel, (unsigned)((units + 7) / 8), 256, 0, fptr(dst), fptr(x), fptr(w), units, groups, (int)(cols / groups), eps);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1355,6 +1380,7 @@ extern "C" CC_API int cc_group_rms_norm(cc_device* dev, const cc_view* dst, cons
 // one CTA per row (layer_norm.cuh)
 #define LN_THREADS 256
 __global__ void __launch_bounds__(LN_THREADS) layer_norm_kernel(float* dst, const float* x, const float* __restrict__ w, const float* __restrict__ b, int cols, float eps) {
+    pdl_enter();
     __shared__ float red[LN_THREADS / 32];
     float* dr = dst + (int64_t)blockIdx.x * cols;
     layer_norm_row<LN_THREADS>(x + (int64_t)blockIdx.x * cols, w, b, cols, eps, red, [&](int c, float v) { dr[c] = v; });
@@ -1367,7 +1393,7 @@ extern "C" CC_API int cc_layer_norm(cc_device* dev, const cc_view* dst, const cc
     const int64_t rows = x->shape[0], cols = x->shape[1];
     CC_REQUIRE(dev, cols >= 1 && view_len(w) == cols && (!b || view_len(b) == cols), "layer_norm: %lld columns need as many weights (and biases)", (long long)cols);
     if (rows == 0) return CC_OK;
-    layer_norm_kernel<<<(unsigned)rows, LN_THREADS, 0, dev->stream>>>(fptr(dst), fptr(x), fptr(w), b ? fptr(b) : nullptr, (int)cols, eps);
+    cc_launch_pdl(dev, layer_norm_kernel, (unsigned)rows, LN_THREADS, 0, fptr(dst), fptr(x), fptr(w), b ? fptr(b) : nullptr, (int)cols, eps);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1378,6 +1404,7 @@ extern "C" CC_API int cc_layer_norm(cc_device* dev, const cc_view* dst, const cc
 #define GGN_THREADS 256
 __global__ void gated_group_rms_norm_kernel(float* dst, const float* x, const float* __restrict__ gate, const float* __restrict__ w, int64_t n_units,
                                             int groups, int gs, float eps, int act, int64_t grs) {
+    pdl_enter();
     const int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (u >= n_units) return;
@@ -1393,6 +1420,7 @@ __global__ void gated_group_rms_norm_kernel(float* dst, const float* x, const fl
 }
 __global__ void __launch_bounds__(GGN_THREADS) gated_group_rms_norm_wide_kernel(float* dst, const float* x, const float* __restrict__ gate,
                                                                                 const float* __restrict__ w, int groups, int gs, float eps, int act, int64_t grs) {
+    pdl_enter();
     __shared__ float red[GGN_THREADS / 32];
     const int64_t u = blockIdx.x;
     const float* xr = x + u * gs;
@@ -1423,8 +1451,8 @@ extern "C" CC_API int cc_gated_group_rms_norm(cc_device* dev, const cc_view* dst
     if (rows == 0) return CC_OK;
     const int64_t units = rows * groups;
     const int gs = (int)(cols / groups);
-    if (gs >= 512) gated_group_rms_norm_wide_kernel<<<(unsigned)units, GGN_THREADS, 0, dev->stream>>>(fptr(dst), fptr(x), fptr(gate), fptr(w), groups, gs, eps, gate_act, grs);
-    else gated_group_rms_norm_kernel<<<(unsigned)((units + 7) / 8), 256, 0, dev->stream>>>(fptr(dst), fptr(x), fptr(gate), fptr(w), units, groups, gs, eps, gate_act, grs);
+    if (gs >= 512) cc_launch_pdl(dev, gated_group_rms_norm_wide_kernel, (unsigned)units, GGN_THREADS, 0, fptr(dst), fptr(x), fptr(gate), fptr(w), groups, gs, eps, gate_act, grs);
+    else cc_launch_pdl(dev, gated_group_rms_norm_kernel, (unsigned)((units + 7) / 8), 256, 0, fptr(dst), fptr(x), fptr(gate), fptr(w), units, groups, gs, eps, gate_act, grs);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1442,6 +1470,7 @@ __device__ __forceinline__ void rotate_pair(float u, float v, float pos, float f
 // halves of the rotated columns
 __global__ void rope_pairs_kernel(float* x, const float* __restrict__ freq, int64_t n, int heads, int hs, int off, int half, float mag, int64_t pos0, int step, int gap,
                                   float* x2) {
+    pdl_enter();
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (x2 ? 2 * n : n)) return;
     if (idx >= n) { idx -= n; x = x2; }                              // a second tensor of the same shape rides along
@@ -1476,7 +1505,7 @@ static int rope_table_impl(cc_device* dev, const cc_view* x, int32_t n_heads, in
     const int64_t n = x->shape[0] * n_heads * half;
     if (n == 0) return CC_OK;
     const int64_t items = x2 ? 2 * n : n;
-    rope_pairs_kernel<<<(unsigned)((items + 255) / 256), 256, 0, dev->stream>>>(fptr(x), fptr(freq), n, n_heads, head_size, offset, (int)half, mag, pos0, halves ? 1 : 2,
+    cc_launch_pdl(dev, rope_pairs_kernel, (unsigned)((items + 255) / 256), 256, 0, fptr(x), fptr(freq), n, n_heads, head_size, offset, (int)half, mag, pos0, halves ? 1 : 2,
                                                                                 halves ? (int)half : 1, x2 ? fptr(x2) : nullptr);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
@@ -1498,6 +1527,7 @@ struct QkPrepArgs {
 // column, which reads both raw values and writes both results; all raw values were read for the sums before the barrier, so q may be
 // overwritten in place.
 __global__ void __launch_bounds__(QKP_THREADS) qk_prepare_kernel(QkPrepArgs a) {
+    pdl_enter();
     extern __shared__ float qkp_sm[];               // inv[H + G], red[8]
     float* inv = qkp_sm;
     float* red = qkp_sm + a.H + a.G;
@@ -1592,7 +1622,7 @@ static int qk_prepare_impl(cc_device* dev, QkPrepArgs a, int64_t T, const cc_vie
     const size_t smem = (size_t)(H + G + QKP_THREADS / 32) * 4;
     CC_REQUIRE(dev, smem <= 48 * 1024, "qk_prepare_append: too many heads");
     const int blocks = qk_norm == CC_QK_NORM_ROW ? 1 : (H + G + QKP_THREADS / 32 - 1) / (QKP_THREADS / 32);       // a warp per head
-    qk_prepare_kernel<<<dim3((unsigned)T, (unsigned)blocks), QKP_THREADS, smem, dev->stream>>>(a);
+    cc_launch_pdl(dev, qk_prepare_kernel, dim3((unsigned)T, (unsigned)blocks), QKP_THREADS, smem, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1660,6 +1690,7 @@ __device__ __forceinline__ void latent_append_row(const LatAppend& a, int t, int
     for (int c = rank + 2 * half + lane; c < cols; c += 32) dst[c] = src[c];
 }
 __global__ void latent_ring_append_kernel(LatAppend a, int T) {
+    pdl_enter();
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t < T) latent_append_row(a, t, threadIdx.x & 31);
 }
@@ -1676,7 +1707,7 @@ extern "C" CC_API int cc_latent_ring_append(cc_device* dev, const cc_view* ring,
     CC_REQUIRE(dev, T <= ring->shape[0], "latent_ring_append: %lld tokens do not fit a ring of %lld", (long long)T, (long long)ring->shape[0]);
     if (T == 0) return CC_OK;
     const LatAppend a = {fptr(ring), fptr(ckv), norm_w ? fptr(norm_w) : nullptr, freq ? fptr(freq) : nullptr, cols, pos0, (int)ring->shape[0], rank, (int)(cols - rank), (int)half, 2, 1, eps, mag};
-    latent_ring_append_kernel<<<(unsigned)((T + 7) / 8), 256, 0, dev->stream>>>(a, (int)T);
+    cc_launch_pdl(dev, latent_ring_append_kernel, (unsigned)((T + 7) / 8), 256, 0, a, (int)T);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1696,6 +1727,7 @@ struct HpArgs {
 // lane-strided partial sums over n_in, then the butterfly -- one order per output, whatever T is.  W: [H * n_out, n_in], rows read
 // contiguously.  The `rest` columns behind a head's n_in inputs are copied behind its n_out outputs.
 __global__ void __launch_bounds__(128) head_project_kernel(HpArgs a) {
+    pdl_enter();
     extern __shared__ float hp_sm[];
     const int t0 = blockIdx.x * HP_TOK, h = blockIdx.y, T = a.T, H = a.H, n_in = a.n_in, rest = a.rest, n_out = a.n_out, half = a.half;
     const int z = (int)blockIdx.z - (a.app.ring ? 1 : 0);
@@ -1748,7 +1780,7 @@ static int head_project_few(cc_device* dev, const HpArgs& a) {
     const size_t smem = (size_t)HP_TOK * a.n_in * 4;
     CC_REQUIRE(dev, smem <= 160 * 1024, "head_project: %d inputs per head do not fit shared memory", a.n_in);
     if (smem > 48 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(head_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    head_project_kernel<<<dim3((unsigned)((a.T + HP_TOK - 1) / HP_TOK), (unsigned)a.H, (unsigned)((a.n_out + 3) / 4 + (a.app.ring ? 1 : 0))), 128, smem, dev->stream>>>(a);
+    cc_launch_pdl(dev, head_project_kernel, dim3((unsigned)((a.T + HP_TOK - 1) / HP_TOK), (unsigned)a.H, (unsigned)((a.n_out + 3) / 4 + (a.app.ring ? 1 : 0))), 128, smem, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1757,6 +1789,7 @@ static int head_project_few(cc_device* dev, const HpArgs& a) {
 #define HPT_TILE 64
 #define HPT_K 16
 __global__ void __launch_bounds__(256) head_project_tile_kernel(const float* __restrict__ x, const float* __restrict__ W, float* __restrict__ out, int T, int H, int n_in, int n_out) {
+    pdl_enter();
     __shared__ float sw[HPT_K][HPT_TILE + 4];
     __shared__ float sx[HPT_K][HPT_TILE + 4];
     const int o0 = blockIdx.x * HPT_TILE, t0 = blockIdx.y * HPT_TILE, h = blockIdx.z;
@@ -1818,8 +1851,7 @@ extern "C" CC_API int cc_head_project(cc_device* dev, const cc_view* x, const cc
     *out = o;
     if (T == 0) return CC_OK;
     if (rest == 0 && T >= 64) {          // a pass of many rows (a prompt): tiles; the sums differ from the few-row kernel's by their order only
-        head_project_tile_kernel<<<dim3((unsigned)((n_out + HPT_TILE - 1) / HPT_TILE), (unsigned)((T + HPT_TILE - 1) / HPT_TILE), (unsigned)n_heads), 256, 0, dev->stream>>>(
-            fptr(x), fptr(w), (float*)o->base, (int)T, n_heads, (int)n_in, (int)n_out);
+        cc_launch_pdl(dev, head_project_tile_kernel, dim3((unsigned)((n_out + HPT_TILE - 1) / HPT_TILE), (unsigned)((T + HPT_TILE - 1) / HPT_TILE), (unsigned)n_heads), 256, 0, fptr(x), fptr(w), (float*)o->base, (int)T, n_heads, (int)n_in, (int)n_out);
         CC_LAUNCH_CHECK(dev);
         return CC_OK;
     }
@@ -1895,6 +1927,7 @@ extern "C" CC_API int cc_latent_query_append_paired(cc_device* dev, const cc_vie
 // the same for a pass of many rows, whose queries are not folded: one CTA per token copies the queries out of their columns, rotating the last
 // `rest` columns of every head on the way (a pair by the thread of its first column), and warp 0 writes the token's cache row
 __global__ void __launch_bounds__(256) latent_prepare_kernel(const float* __restrict__ q, int64_t qrs, float* __restrict__ out, int H, int dim, LatAppend a) {
+    pdl_enter();
     const int t = blockIdx.x, hs = dim + a.rest;
     const float* qr = q + t * qrs;
     float* o = out + (int64_t)t * H * hs;
@@ -1941,7 +1974,7 @@ extern "C" CC_API int cc_latent_prepare_append(cc_device* dev, const cc_view* q_
     if (rc) return rc;
     *out = o;
     if (T == 0) return CC_OK;
-    latent_prepare_kernel<<<(unsigned)T, 256, 0, dev->stream>>>(fptr(q_src) + q_col0, q_src->strides[0], (float*)o->base, n_heads, dim, a);
+    cc_launch_pdl(dev, latent_prepare_kernel, (unsigned)T, 256, 0, fptr(q_src) + q_col0, q_src->strides[0], (float*)o->base, n_heads, dim, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1949,6 +1982,7 @@ extern "C" CC_API int cc_latent_prepare_append(cc_device* dev, const cc_view* q_
 // out[j, h] = [ a[j, h, :dim] | shared[j, col0 : col0 + rest] ]: every head's part followed by the columns all heads share.  One thread per element.
 __global__ void head_concat_shared_kernel(const float* __restrict__ a, const float* __restrict__ shared, float* __restrict__ out, int64_t n, int H, int dim, int rest, int scols,
                                           int col0) {
+    pdl_enter();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
     const int hs = dim + rest;
@@ -1970,7 +2004,7 @@ extern "C" CC_API int cc_head_concat_shared(cc_device* dev, const cc_view* a, co
     *out = o;
     const int64_t n = rows * n_heads * (dim + rest);
     if (n == 0) return CC_OK;
-    head_concat_shared_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(a), fptr(shared), (float*)o->base, n, n_heads, (int)dim, rest, (int)shared->shape[1], col0);
+    cc_launch_pdl(dev, head_concat_shared_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(a), fptr(shared), (float*)o->base, n, n_heads, (int)dim, rest, (int)shared->shape[1], col0);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1984,6 +2018,7 @@ struct SplitArgs {
 };
 // grid (ceil(cols / 256), about rows / 8): a thread owns one column (its part is found once) and walks the rows of its grid line
 __global__ void split_cols_kernel(const float* __restrict__ src, SplitArgs a, int64_t rows, int cols) {
+    pdl_enter();
     const int c = blockIdx.x * 256 + threadIdx.x;
     if (c >= cols) return;
     int p = 0;
@@ -2015,7 +2050,7 @@ extern "C" CC_API int cc_split_cols(cc_device* dev, const cc_view* src, int32_t 
     const int64_t total = rows * cols;
     if (total == 0) return CC_OK;
     const int64_t lines = (rows + 7) / 8;             // a thread copies about 8 rows of its column
-    split_cols_kernel<<<dim3((unsigned)((cols + 255) / 256), (unsigned)(lines < 65535 ? lines : 65535)), 256, 0, dev->stream>>>(fptr(src), a, rows, (int)cols);
+    cc_launch_pdl(dev, split_cols_kernel, dim3((unsigned)((cols + 255) / 256), (unsigned)(lines < 65535 ? lines : 65535)), 256, 0, fptr(src), a, rows, (int)cols);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -2023,6 +2058,7 @@ extern "C" CC_API int cc_split_cols(cc_device* dev, const cc_view* src, int32_t 
 // ---- PolyNorm ------------------------------------------------------------------------------------------------------------------------------
 // one CTA per row: thread-strided sums of z^2, z^4, z^6, a fixed tree over the 256 partial sums, then the weighted sum of the three unit powers
 __global__ void __launch_bounds__(256) poly_norm_kernel(float* __restrict__ z, const float* __restrict__ coef, int cols, float eps) {
+    pdl_enter();
     __shared__ float red[3][8];
     float* zr = z + (int64_t)blockIdx.x * cols;
     float s2 = 0.0f, s4 = 0.0f, s6 = 0.0f;
@@ -2049,7 +2085,7 @@ extern "C" CC_API int cc_poly_norm(cc_device* dev, const cc_view* z, const cc_vi
     SEQ_F32(dev, z, "poly_norm z"); SEQ_F32(dev, coef, "poly_norm coef");
     CC_REQUIRE(dev, z->ndim == 2 && view_len(coef) == 4, "poly_norm: z must be [rows, cols] and coef hold 4 numbers");
     if (z->shape[0] == 0) return CC_OK;
-    poly_norm_kernel<<<(unsigned)z->shape[0], 256, 0, dev->stream>>>(fptr(z), fptr(coef), (int)z->shape[1], eps);
+    cc_launch_pdl(dev, poly_norm_kernel, (unsigned)z->shape[0], 256, 0, fptr(z), fptr(coef), (int)z->shape[1], eps);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -2057,6 +2093,7 @@ extern "C" CC_API int cc_poly_norm(cc_device* dev, const cc_view* z, const cc_vi
 // ---- gated sum of sublayer results into the residual stream -----------------------------------------------------------------------------------
 __global__ void gated_sum_kernel(float* __restrict__ dst, const float* __restrict__ y1, const float* __restrict__ g1, const float* __restrict__ b1, const float* __restrict__ y2,
                                  const float* __restrict__ g2, const float* __restrict__ b2, int64_t n, int cols, int accumulate) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int c = (int)(i % cols);
@@ -2083,7 +2120,7 @@ extern "C" CC_API int cc_gated_sum(cc_device* dev, const cc_view* dst, int32_t a
         if (v) { SEQ_F32(dev, v, "gated_sum bias"); CC_REQUIRE(dev, view_len(v) == cols, "gated_sum: a bias needs one number per column"); }
     CC_REQUIRE(dev, (!b1 || g1) && (!b2 || g2) && (!g2 || y2), "gated_sum: a bias needs its gate, a gate its operand");
     if (n == 0) return CC_OK;
-    gated_sum_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(fptr(dst), fptr(y1), g1 ? fptr(g1) : nullptr, b1 ? fptr(b1) : nullptr, y2 ? fptr(y2) : nullptr,
+    cc_launch_pdl(dev, gated_sum_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(dst), fptr(y1), g1 ? fptr(g1) : nullptr, b1 ? fptr(b1) : nullptr, y2 ? fptr(y2) : nullptr,
                                                                            g2 ? fptr(g2) : nullptr, b2 ? fptr(b2) : nullptr, n, (int)cols, accumulate);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;

@@ -53,6 +53,7 @@ struct DgArgs {
 // gates while the other walks.  The walk over a block's tokens is done by the first 4 threads, one channel each: the operands of 16 tokens are
 // read from shared memory into registers at once (they do not depend on S), then the chain is one fmaf per token.
 __global__ void __launch_bounds__(DG_THREADS) gated_diag_kernel(DgArgs a) {
+    pdl_enter();
     __shared__ float s_a[DG_TB][DG_CH], s_b[DG_TB][DG_CH], s_s[DG_TB][DG_CH];
     const int l = threadIdx.x % DG_CH, row = threadIdx.x / DG_CH;
     const int ch = blockIdx.x * DG_CH + l;
@@ -140,7 +141,7 @@ extern "C" CC_API int cc_gated_diagonal_recurrence(cc_device* dev, const cc_view
     DgArgs a{};
     a.u = dptr(u); a.gates = dptr(gates); a.gate_bias = dptr(gate_bias); a.lam = dptr(lam); a.y = y ? dptr(y) : nullptr; a.y_bias = y_bias ? dptr(y_bias) : nullptr;
     a.state = dptr(state); a.out = (float*)o->base; a.T = (int)T; a.C = (int)C; a.bs = (int)(C / n_blocks); a.y_act = y_act; a.c = c;
-    gated_diag_kernel<<<(unsigned)((C + DG_CH - 1) / DG_CH), DG_THREADS, 0, dev->stream>>>(a);
+    cc_launch_pdl(dev, gated_diag_kernel, (unsigned)((C + DG_CH - 1) / DG_CH), DG_THREADS, 0, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }

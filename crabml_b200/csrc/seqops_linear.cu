@@ -72,6 +72,7 @@ static __host__ __device__ __forceinline__ int lr_stage_floats(int dk4, bool ade
 
 template <int DK, int SPLIT, bool ADEC>
 __global__ void __launch_bounds__(DK > 0 ? LR_COLS * SPLIT : LR_GENERIC_THREADS) lr_kernel(LrArgs a) {
+    pdl_enter();
     extern __shared__ __align__(16) float lr_sm[];           // two staging buffers, then (DK == 0) the state columns
     constexpr int THREADS = DK > 0 ? LR_COLS * SPLIT : LR_GENERIC_THREADS;
     constexpr int COLS = THREADS / SPLIT;
@@ -230,7 +231,7 @@ static cudaError_t lr_launch_one(cc_device* dev, const LrArgs& a, size_t smem) {
         if (e != cudaSuccess) return e;
     }
     const int threads = DK > 0 ? LR_COLS * SPLIT : LR_GENERIC_THREADS, cols = threads / SPLIT;
-    lr_kernel<DK, SPLIT, ADEC><<<dim3((unsigned)a.H, (unsigned)((a.dv + cols - 1) / cols)), threads, smem, dev->stream>>>(a);
+    cc_launch_pdl(dev, lr_kernel<DK, SPLIT, ADEC>, dim3((unsigned)a.H, (unsigned)((a.dv + cols - 1) / cols)), threads, smem, a);
     return cudaGetLastError();
 }
 template <bool ADEC>
@@ -262,6 +263,7 @@ static int lr_launch(cc_device* dev, LrArgs a, const char* what) {
 // its token's {exp(f + m - m'), exp(i - m')} and exp(-m').
 __global__ void __launch_bounds__(32) mm_gates_kernel(const float* __restrict__ gi, const float* __restrict__ gf, const float* __restrict__ bi, const float* __restrict__ bf,
                                                       float cap, float* __restrict__ mstate, float* __restrict__ sc, float* __restrict__ floor_out, int T, int H) {
+    pdl_enter();
     const int h = blockIdx.x, lane = threadIdx.x;
     float m = mstate[h];
     for (int t0 = 0; t0 < T; t0 += 32) {
@@ -290,6 +292,7 @@ __global__ void __launch_bounds__(32) mm_gates_kernel(const float* __restrict__ 
 }
 // raw: [T, H, dv + 1], the read-out of the state and, in the last column, of the normaliser; out = raw / (max(|n . q|, floor) + 1e-6)
 __global__ void mm_divide_kernel(const float* __restrict__ raw, const float* __restrict__ floor_in, float* __restrict__ out, int64_t n, int dv) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t th = i / dv;
@@ -322,7 +325,7 @@ extern "C" CC_API int cc_matrix_memory(cc_device* dev, const cc_view* q, const c
     float* sc = (float*)tmp;
     float* fl = sc + n_sc;
     float* raw = fl + n_floor;
-    mm_gates_kernel<<<(unsigned)H, 32, 0, dev->stream>>>(lptr(gi), lptr(gf), lptr(bi), lptr(bf), cap, lptr(mstate), sc, fl, (int)T, H);
+    cc_launch_pdl(dev, mm_gates_kernel, (unsigned)H, 32, 0, lptr(gi), lptr(gf), lptr(bi), lptr(bf), cap, lptr(mstate), sc, fl, (int)T, H);
     dev->launches++;
     LrArgs a{};
     a.q = lptr(q); a.k = lptr(k); a.v = lptr(v); a.adec = nullptr; a.sc = sc; a.skip = nullptr; a.state = lptr(state); a.out = raw;
@@ -330,7 +333,7 @@ extern "C" CC_API int cc_matrix_memory(cc_device* dev, const cc_view* q, const c
     rc = lr_launch(dev, a, "matrix_memory");
     if (rc == CC_OK) {
         const int64_t n = T * H * dv;
-        mm_divide_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(raw, fl, (float*)o->base, n, dv);
+        cc_launch_pdl(dev, mm_divide_kernel, (unsigned)((n + 255) / 256), 256, 0, raw, fl, (float*)o->base, n, dv);
     }
     cc_pool_free(dev, tmp, cls);
     if (rc) return rc;
@@ -341,6 +344,7 @@ extern "C" CC_API int cc_matrix_memory(cc_device* dev, const cc_view* q, const c
 // ---- linear attention with a decay per key channel ---------------------------------------------------------------------------------------------
 // alpha = sigmoid(z + b)^(1 / tau) = exp(-softplus(-(z + b)) / tau)
 __global__ void dla_decay_kernel(const float* __restrict__ z, const float* __restrict__ zb, float* __restrict__ adec, int64_t n, int cols, float inv_tau) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) adec[i] = expf(-lin_softplus(-(z[i] + zb[i % cols])) * inv_tau);
 }
@@ -364,7 +368,7 @@ extern "C" CC_API int cc_decayed_linear_attention(cc_device* dev, const cc_view*
     rc = cc_pool_alloc(dev, (size_t)T * H * dk * 4, &tmp, &cls);
     if (rc) return rc;
     const int64_t n = T * H * dk;
-    dla_decay_kernel<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(lptr(z), lptr(zb), (float*)tmp, n, H * dk, 1.0f / tau);
+    cc_launch_pdl(dev, dla_decay_kernel, (unsigned)((n + 255) / 256), 256, 0, lptr(z), lptr(zb), (float*)tmp, n, H * dk, 1.0f / tau);
     dev->launches++;
     LrArgs a{};
     a.q = lptr(q); a.k = lptr(k); a.v = lptr(v); a.adec = (const float*)tmp; a.sc = nullptr; a.skip = nullptr; a.state = lptr(state); a.out = (float*)o->base;
@@ -405,6 +409,7 @@ extern "C" CC_API int cc_retention(cc_device* dev, const cc_view* q, const cc_vi
 // sc[(t * H + h) * 2] = ss_step of the token and head
 __global__ void ss_steps_kernel(const float* __restrict__ dt, const float* __restrict__ dt_bias, const float* __restrict__ a_log, float* __restrict__ sc, int64_t n, int H,
                                 int64_t dt_rs) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int h = (int)(i % H);
@@ -440,7 +445,7 @@ static int state_space_scan_impl(cc_device* dev, const cc_view* xbc, const cc_vi
     } else {
         rc = cc_pool_alloc(dev, (size_t)T * H * 2 * 4, &tmp, &cls);
         if (rc) return rc;
-        ss_steps_kernel<<<(unsigned)((T * H + 255) / 256), 256, 0, dev->stream>>>(dtp, lptr(dt_bias), lptr(a_log), (float*)tmp, T * H, H, dt_rs);
+        cc_launch_pdl(dev, ss_steps_kernel, (unsigned)((T * H + 255) / 256), 256, 0, dtp, lptr(dt_bias), lptr(a_log), (float*)tmp, T * H, H, dt_rs);
         dev->launches++;
         a.sc = (const float*)tmp;
     }

@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
     __syncthreads();
     pg_fence_after();
     const unsigned tmem = sh.tmem_base;
+    pdl_enter();
     unsigned g = 0, runs = 0;                                         // steps and runs of the tiles before
 
     if (warp == SG_WARPS) {
@@ -415,11 +416,14 @@ static int sg_launch(cc_device* dev, const P& p, int64_t n_tiles) {
     int64_t at_once = SPLIT ? dev->sm_count / 2 : dev->sm_count;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2); cfg.blockDim = dim3(SG_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = dev->stream;
-    cudaLaunchAttribute pair;
-    pair.id = cudaLaunchAttributeClusterDimension;
-    pair.val.clusterDim.x = 2; pair.val.clusterDim.y = 1; pair.val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = SPLIT ? 2 : 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = dev->pdl ? 1 : 0;
+    cfg.attrs = at;
     if (SPLIT) {                                                      // pairs that fit the chip at a time: an SM without a partner in its group stays idle
-        cfg.attrs = &pair; cfg.numAttrs = 1;
+        cfg.numAttrs = 1;
         if (n_tiles > 64) {
             int pairs = 0;
             CC_CUDA(dev, cudaOccupancyMaxActiveClusters(&pairs, split_gemm_kernel<P, SPLIT>, &cfg));
@@ -428,6 +432,7 @@ static int sg_launch(cc_device* dev, const P& p, int64_t n_tiles) {
     }
     const unsigned ctas = (unsigned)(n_tiles < at_once ? n_tiles : at_once > 0 ? at_once : 1);
     cfg.gridDim = dim3(SPLIT ? 2 * ctas : ctas);
+    cfg.numAttrs = 2;
     CC_CUDA(dev, cudaLaunchKernelEx(&cfg, split_gemm_kernel<P, SPLIT>, p, (int)n_tiles, dev->err_dev, dev->err_host));
     CC_LAUNCH_CHECK(dev);
     return CC_OK;

@@ -17,11 +17,16 @@ extern "C" CC_API int cc_tensor_dup(cc_device* dev, const cc_view* src, cc_buf**
     int rc = cc_new_activation(dev, n, CC_F32, false, &b);
     if (rc) return rc;
     *out = b;
-    if (LAZY(dev)) return cc_lazy_record(dev, L_DUP, src, nullptr, b, 0, 0, 0, 0, nullptr, 0);
+    if (LAZY(dev)) {
+        rc = cc_lazy_record(dev, L_DUP, src, nullptr, b, 0, 0, 0, 0, nullptr, 0);      // may run what is queued: its error is this call's
+        if (rc) { cc_tensor_release(b); *out = nullptr; }
+        return rc;
+    }
     if (n) CC_CUDA(dev, cudaMemcpyAsync(b->base, src->buf->plane[0], (size_t)n * 4, cudaMemcpyDeviceToDevice, dev->stream));
     return CC_OK;
 }
 
+#define CC_EXPORT_STAGED ((size_t)1 << 20)
 extern "C" CC_API int cc_tensor_export_f32(cc_device* dev, const cc_view* src, float* dst, size_t n) {   // cpu_tensor.rs:339-349
     CHECK_VIEW(dev, src, "export");
     if (!dst) return cc_fail(dev, CC_ERR_ARG, "export: dst is NULL");
@@ -30,8 +35,11 @@ extern "C" CC_API int cc_tensor_export_f32(cc_device* dev, const cc_view* src, f
     FLUSH(dev);
     int64_t len = view_len(src);
     size_t cnt = n < (size_t)len ? n : (size_t)len;
-    if (cnt) CC_CUDA(dev, cudaMemcpyAsync(dst, src->buf->plane[0], cnt * 4, cudaMemcpyDeviceToHost, dev->stream));
+    // a row of logits goes through the device's pinned buffer: the driver's way into pageable memory takes some 20 us longer than the copy itself
+    const bool staged = cnt && cnt * 4 <= CC_EXPORT_STAGED && cc_ensure_pinned(dev, cnt * 4) == CC_OK;
+    if (cnt) CC_CUDA(dev, cudaMemcpyAsync(staged ? dev->pinned : dst, src->buf->plane[0], cnt * 4, cudaMemcpyDeviceToHost, dev->stream));
     CC_CUDA(dev, cudaStreamSynchronize(dev->stream));
+    if (staged) memcpy(dst, dev->pinned, cnt * 4);
     return cc_check_async_error(dev);
 }
 

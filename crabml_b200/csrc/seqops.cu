@@ -713,10 +713,10 @@ extern "C" CC_API int cc_gated_delta_rule(cc_device* dev, const cc_view* q, cons
             : dk == 128 ? cudaFuncSetAttribute(delta_rule_kernel<128, 8, DR_SPLIT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
                         : cudaFuncSetAttribute(delta_rule_kernel<0, 1, DR_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) { cc_pool_free(dev, bdp, cls); return cc_fail(dev, CC_ERR_CUDA, "gated_delta_rule: %s", cudaGetErrorString(e)); }
-    if (dk == 32) cc_launch_pdl(dev, delta_rule_kernel<32, 2, DR_SPLIT_THREADS>, grid, threads, smem, DR_ARGS);
-    else if (dk == 64) cc_launch_pdl(dev, delta_rule_kernel<64, 4, DR_SPLIT_THREADS>, grid, threads, smem, DR_ARGS);
-    else if (dk == 128) cc_launch_pdl(dev, delta_rule_kernel<128, 8, DR_SPLIT_THREADS>, grid, threads, smem, DR_ARGS);
-    else cc_launch_pdl(dev, delta_rule_kernel<0, 1, DR_THREADS>, grid, threads, smem, DR_ARGS);
+    if (dk == 32) cc_launch_alone(dev, delta_rule_kernel<32, 2, DR_SPLIT_THREADS>, grid, threads, smem, DR_ARGS);
+    else if (dk == 64) cc_launch_alone(dev, delta_rule_kernel<64, 4, DR_SPLIT_THREADS>, grid, threads, smem, DR_ARGS);
+    else if (dk == 128) cc_launch_alone(dev, delta_rule_kernel<128, 8, DR_SPLIT_THREADS>, grid, threads, smem, DR_ARGS);
+    else cc_launch_alone(dev, delta_rule_kernel<0, 1, DR_THREADS>, grid, threads, smem, DR_ARGS);
 #undef DR_ARGS
     cc_pool_free(dev, bdp, cls);            // stream-ordered pool: the next user of this block runs after the kernels above
     CC_LAUNCH_CHECK(dev);
@@ -1198,7 +1198,7 @@ static size_t wa_slices_smem(int RB, int64_t maxn, int* slice_cap) {
 template <int RB>
 static cudaError_t wa_launch_slices(cc_device* dev, const float* S, const float* v, float* out, const WaGeom& g, const float* sink, size_t smem, int slice_cap) {
     if (smem > 40 * 1024) { cudaError_t e = cudaFuncSetAttribute(wa_values_slices_kernel<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) return e; }
-    cc_launch_pdl(dev, wa_values_slices_kernel<RB>, dim3((unsigned)(g.T * g.G * ((g.R + RB - 1) / RB)), (unsigned)((g.dv + 31) / 32), WV_SPLIT), WV_THREADS, smem, S, v, out, g, sink, slice_cap);
+    cc_launch_alone(dev, wa_values_slices_kernel<RB>, dim3((unsigned)(g.T * g.G * ((g.R + RB - 1) / RB)), (unsigned)((g.dv + 31) / 32), WV_SPLIT), WV_THREADS, smem, S, v, out, g, sink, slice_cap);
     return cudaSuccess;
 }
 static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view* qnw, float eps, const cc_view* kring, const cc_view* vring, int64_t pos0, int32_t H, int32_t G,

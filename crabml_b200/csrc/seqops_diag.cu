@@ -141,7 +141,7 @@ extern "C" CC_API int cc_gated_diagonal_recurrence(cc_device* dev, const cc_view
     DgArgs a{};
     a.u = dptr(u); a.gates = dptr(gates); a.gate_bias = dptr(gate_bias); a.lam = dptr(lam); a.y = y ? dptr(y) : nullptr; a.y_bias = y_bias ? dptr(y_bias) : nullptr;
     a.state = dptr(state); a.out = (float*)o->base; a.T = (int)T; a.C = (int)C; a.bs = (int)(C / n_blocks); a.y_act = y_act; a.c = c;
-    cc_launch_pdl(dev, gated_diag_kernel, (unsigned)((C + DG_CH - 1) / DG_CH), DG_THREADS, 0, a);
+    cc_launch_alone(dev, gated_diag_kernel, (unsigned)((C + DG_CH - 1) / DG_CH), DG_THREADS, 0, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }

@@ -231,7 +231,7 @@ static cudaError_t lr_launch_one(cc_device* dev, const LrArgs& a, size_t smem) {
         if (e != cudaSuccess) return e;
     }
     const int threads = DK > 0 ? LR_COLS * SPLIT : LR_GENERIC_THREADS, cols = threads / SPLIT;
-    cc_launch_pdl(dev, lr_kernel<DK, SPLIT, ADEC>, dim3((unsigned)a.H, (unsigned)((a.dv + cols - 1) / cols)), threads, smem, a);
+    cc_launch_alone(dev, lr_kernel<DK, SPLIT, ADEC>, dim3((unsigned)a.H, (unsigned)((a.dv + cols - 1) / cols)), threads, smem, a);
     return cudaGetLastError();
 }
 template <bool ADEC>

@@ -308,6 +308,47 @@ static __device__ MK_GENERIC_ATTR void phase_matvec_generic(const MkPhase& ph, u
     int16_t* s_bs = (int16_t*)(smem + al16i(k) + al16i(k / 256 * 4));
     float* s_red = (float*)(smem + mk_generic_sx_offset(k) - 256);
     float* s_x = (float*)(smem + mk_generic_sx_offset(k));
+    // rows: the same warp-major dealing and epilogues as phase_matvec
+    const int gw = warp * gridDim.x + blockIdx.x, TW = gridDim.x * MK_WARPS;
+    const bool pair = A.epilogue == 2;
+    const int m_cat = pair ? M.m[0] : M.m[0] + (M.n > 1 ? M.m[1] : 0) + (M.n > 2 ? M.m[2] : 0);
+    const int n_rows = gw < m_cat ? (m_cat - gw + TW - 1) / TW : 0;
+    const int n_vrows = pair ? 2 * n_rows : n_rows;
+    auto locate = [&](int i, int& mat) -> int {                          // i-th virtual row of this warp -> (matrix, row)
+        int r;
+        mat = 0;
+        if (pair) { mat = i & 1; r = gw + (i >> 1) * TW; }
+        else {
+            r = gw + i * TW;
+            if (M.n > 1 && r >= M.m[0]) { r -= M.m[0]; mat = 1; if (M.n > 2 && r >= M.m[1]) { r -= M.m[1]; mat = 2; } }
+        }
+        return r;
+    };
+    auto planes = [&](int mat) -> WPlanes {
+        WPlanes W;
+        W.p[0] = mat == 0 ? M.qs[0] : mat == 1 ? M.qs[1] : M.qs[2];
+        W.p[1] = (const uint8_t*)(mat == 0 ? M.d[0] : mat == 1 ? M.d[1] : M.d[2]);
+        W.p[2] = mat == 0 ? M.p2[0] : mat == 1 ? M.p2[1] : M.p2[2];
+        W.p[3] = mat == 0 ? M.p3[0] : mat == 1 ? M.p3[1] : M.p3[2];
+        return W;
+    };
+    // rows cut into segments of 16 super-blocks; the loads of segment u + 2 are issued before segment u + 1 is consumed (two
+    // segments = 16-24 LDG.128 per lane in flight), across row boundaries.  The first two are on their way while the activation is prepared
+    const int NSEG = ((k >> 8) + 15) >> 4;
+    const int U = n_vrows * NSEG;
+#if MK_GENERIC_NOINLINE
+    KSeg S0, S1;
+#else
+    KSeg& S0 = P.buf0;                                                   // the weight pipe's registers (no streaming look-ahead is pending: caller)
+    KSeg& S1 = P.buf1;
+#endif
+    int x0[8] = {}, x1[8] = {};
+    int l_i = 0, l_seg = 0;
+    auto load = [&](KSeg& S, int (&x)[8], bool valid) {
+        if (valid) { int mat; const int r = locate(l_i, mat); T::seg_load(S, x, planes(mat), r, k, l_seg, lane); }
+        if (++l_seg == NSEG) { l_seg = 0; l_i++; }
+    };
+    if constexpr (T::kSegmented && !MK_GENERIC_NOINLINE) { load(S0, x0, U > 0); load(S1, x1, U > 1); }
     {   // one L2 round trip: the f32 row (unless requested right after the barrier) and the norm weights (unless staged before it)
         const int n4 = k >> 2;
         const unsigned sx = (unsigned)__cvta_generic_to_shared(s_x), sw = (unsigned)__cvta_generic_to_shared(s_w);
@@ -329,23 +370,24 @@ static __device__ MK_GENERIC_ATTR void phase_matvec_generic(const MkPhase& ph, u
     if (stamp1) stamp1[4] = globaltimer_ns();
     if (ph.orig && blockIdx.x == 0)                                     // Tensor::dup of the un-normalised row (llama2.rs:227,607)
         for (int i = threadIdx.x; i < (k >> 2); i += MK_THREADS) ((float4*)ph.orig)[i] = ((const float4*)s_x)[i];
+    const CcDivBy by_rms(rms);
+    const int q_at = T::act_at(lane >> 1) * 16 + (lane & 1) * 8;
     for (int sb = warp; sb < (k >> 8); sb += MK_WARPS) {                // one warp per 256-element super-block (buf_q8_k.rs:84-131)
-        float v[8];
+        float4 v4[2];
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            v[i] = s_x[sb * 256 + lane * 8 + i];
-            if (ph.norm_w) v[i] = (v[i] / rms) * s_w[sb * 256 + lane * 8 + i];
+        for (int i = 0; i < 2; i++) {
+            v4[i] = ((const float4*)s_x)[sb * 64 + lane * 2 + i];
+            if (ph.norm_w) {
+                const float4 w4 = ((const float4*)s_w)[sb * 64 + lane * 2 + i];
+                v4[i] = by_rms(v4[i]);
+                v4[i].x *= w4.x; v4[i].y *= w4.y; v4[i].z *= w4.z; v4[i].w *= w4.w;
+            }
         }
-        cc_quant_q8k_sblock(v, lane, s_q + sb * 256, s_d + sb, s_bs + sb * 16);
+        const float v[8] = {v4[0].x, v4[0].y, v4[0].z, v4[0].w, v4[1].x, v4[1].y, v4[1].z, v4[1].w};
+        cc_quant_q8k_sblock(v, lane, s_q + sb * 256 + q_at, s_d + sb, s_bs + sb * 16);
     }
     MK_SYNC();
     if (stamp1) *stamp1 = globaltimer_ns();
-    // rows: the same warp-major dealing and epilogues as phase_matvec
-    const int gw = warp * gridDim.x + blockIdx.x, TW = gridDim.x * MK_WARPS;
-    const bool pair = A.epilogue == 2;
-    const int m_cat = pair ? M.m[0] : M.m[0] + (M.n > 1 ? M.m[1] : 0) + (M.n > 2 ? M.m[2] : 0);
-    const int n_rows = gw < m_cat ? (m_cat - gw + TW - 1) / TW : 0;
-    const int n_vrows = pair ? 2 * n_rows : n_rows;
     float first = 0.0f, pend_a = 0.0f, pend_b = 0.0f, pend_res = 0.0f;
     unsigned short pend_lut = 0;
     int pend_row = -1;
@@ -355,24 +397,6 @@ static __device__ MK_GENERIC_ATTR void phase_matvec_generic(const MkPhase& ph, u
             else M.out[0][pend_row] = pend_a + pend_res;
         }
         pend_row = -1;
-    };
-    auto locate = [&](int i, int& mat) -> int {                          // i-th virtual row of this warp -> (matrix, row)
-        int r;
-        mat = 0;
-        if (pair) { mat = i & 1; r = gw + (i >> 1) * TW; }
-        else {
-            r = gw + i * TW;
-            if (M.n > 1 && r >= M.m[0]) { r -= M.m[0]; mat = 1; if (M.n > 2 && r >= M.m[1]) { r -= M.m[1]; mat = 2; } }
-        }
-        return r;
-    };
-    auto planes = [&](int mat) -> WPlanes {
-        WPlanes W;
-        W.p[0] = mat == 0 ? M.qs[0] : mat == 1 ? M.qs[1] : M.qs[2];
-        W.p[1] = (const uint8_t*)(mat == 0 ? M.d[0] : mat == 1 ? M.d[1] : M.d[2]);
-        W.p[2] = mat == 0 ? M.p2[0] : mat == 1 ? M.p2[1] : M.p2[2];
-        W.p[3] = mat == 0 ? M.p3[0] : mat == 1 ? M.p3[1] : M.p3[2];
-        return W;
     };
     auto emit = [&](int i, float v) {                                    // row i of this warp is reduced: epilogue
         int mat;
@@ -390,24 +414,7 @@ static __device__ MK_GENERIC_ATTR void phase_matvec_generic(const MkPhase& ph, u
         }
     };
     if constexpr (T::kSegmented) {
-        // rows cut into segments of 16 super-blocks; the loads of segment u + 2 are issued before segment u + 1 is consumed (two
-        // segments = 16-24 LDG.128 per lane in flight), across row boundaries
-        const int NSEG = ((k >> 8) + 15) >> 4;
-        const int U = n_vrows * NSEG;
-#if MK_GENERIC_NOINLINE
-        KSeg S0, S1;
-#else
-        KSeg& S0 = P.buf0;                                                   // the weight pipe's registers (no streaming look-ahead is pending: caller)
-        KSeg& S1 = P.buf1;
-#endif
-        int x0[4] = {0, 0, 0, 0}, x1[4] = {0, 0, 0, 0};
-        int l_i = 0, l_seg = 0;
-        auto load = [&](KSeg& S, int (&x)[4], bool valid) {
-            if (valid) { int mat; const int r = locate(l_i, mat); T::seg_load(S, x, planes(mat), r, k, l_seg, lane); }
-            if (++l_seg == NSEG) { l_seg = 0; l_i++; }
-        };
-        load(S0, x0, U > 0);
-        load(S1, x1, U > 1);
+        if constexpr (MK_GENERIC_NOINLINE) { load(S0, x0, U > 0); load(S1, x1, U > 1); }
         float acc = 0.0f;
         int c_i = 0, c_seg = 0;
         auto finish = [&]() { if (++c_seg < NSEG) return; c_seg = 0; const float v = warp_sum(acc); acc = 0.0f; emit(c_i++, v); };

@@ -86,7 +86,7 @@ __global__ void quantize_q8_k_kernel(const float* __restrict__ x, int64_t nsb, A
     float v[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = xb[i];
-    cc_quant_q8k_sblock(v, lane, a.qs + b * 256, a.d + b, a.bsums + b * 16);
+    cc_quant_q8k_sblock(v, lane, a.qs + b * 256 + lane * 8, a.d + b, a.bsums + b * 16);
 }
 
 __global__ void quantize_f16_kernel(const float* __restrict__ x, int64_t n, __half* out) { pdl_enter();   // buf/api.rs:198

@@ -232,16 +232,23 @@ struct TQx_1 {
 struct KAct {
     const int4* q; const float* d; const int16_t* bs;
     __device__ KAct(const uint8_t* sm, int k) : q((const int4*)sm), d((const float*)(sm + al16i(k))), bs((const int16_t*)(sm + al16i(k) + al16i(k / 256 * 4))) {}
+    __device__ __forceinline__ int bsum2(int i) const { const int w = ((const int*)bs)[i]; return (int)(int16_t)(w & 0xFFFF) + (w >> 16); }      // block sums 2 i and 2 i + 1
 };
 struct TKBase {
     static constexpr bool kSegmented = false;      // overridden by the types that offer seg_load / seg_dot (Q4_K, Q6_K)
-    static __device__ __forceinline__ void seg_load(KSeg&, int (&)[4], const WPlanes&, int64_t, int, int, int) {}
-    static __device__ __forceinline__ float seg_dot(const KSeg&, const int (&)[4], int, int, const uint8_t*, int, float acc) { return acc; }
+    static __device__ __forceinline__ void seg_load(KSeg&, int (&)[8], const WPlanes&, int64_t, int, int, int) {}
+    static __device__ __forceinline__ float seg_dot(const KSeg&, const int (&)[8], int, int, const uint8_t*, int, float acc) { return acc; }
     static __host__ __device__ int smem_bytes(int k) { return al16i(k) + al16i(k / 256 * 4) + al16i(k / 16 * 2); }
-    static __device__ void stage_act(const void* scratch, int64_t n_total, int bi, int k, uint8_t* sm) {
+    // where 16-byte chunk i of the activation lies in shared memory.  The types read 8 lanes to a super-block, a lane two of its 16 chunks: those of
+    // the 8 lanes' first reads go in front of those of the second, 128 consecutive bytes a read (in natural order half of the banks served all 8)
+    static __host__ __device__ __forceinline__ int act_at(int i) { return i; }
+    static __device__ void stage_act(const void* scratch, int64_t n_total, int bi, int k, uint8_t* sm) { stage_act_as<TKBase>(scratch, n_total, bi, k, sm); }
+    template <class T>
+    static __device__ void stage_act_as(const void* scratch, int64_t n_total, int bi, int k, uint8_t* sm) {
         const uint8_t* p = (const uint8_t*)scratch;
         int64_t o1 = (n_total + 15) & ~15ll, o2 = o1 + ((n_total / 256 * 4 + 15) & ~15ll);
-        stage(sm, p + (int64_t)bi * k, k);
+        const int4* q = (const int4*)(p + (int64_t)bi * k);
+        for (int i = threadIdx.x; i < (k >> 4); i += blockDim.x) ((int4*)sm)[T::act_at(i)] = q[i];
         stage(sm + al16i(k), p + o1 + (int64_t)bi * (k / 256) * 4, k / 256 * 4);
         stage(sm + al16i(k) + al16i(k / 256 * 4), p + o2 + (int64_t)bi * (k / 16) * 2, k / 16 * 2);
     }
@@ -259,6 +266,9 @@ __device__ __forceinline__ void k4_unpack(unsigned u0, unsigned u1, unsigned u2,
 // Q4_K: buf_q4_k.rs:192-277.  8 lanes per super-block, lane j owns the 16-byte qs chunk j.
 template <bool FIVE>
 struct TQ45_K : TKBase {
+    // chunk 4 g + 2 h + b of a super-block: the low (h = 0) or high nibbles of weight chunk j = 2 g + b
+    static __host__ __device__ __forceinline__ int act_at(int i) { return (i & ~15) | ((i & 2) << 2) | ((i & 12) >> 1) | (i & 1); }
+    static __device__ void stage_act(const void* scratch, int64_t n_total, int bi, int k, uint8_t* sm) { stage_act_as<TQ45_K>(scratch, n_total, bi, k, sm); }
     static __device__ float row_dot(const WPlanes& W, int64_t row, int k, const uint8_t* sm, int lane) {
         const int nsb = k >> 8, BB = FIVE ? 176 : 144, QOFF = FIVE ? 48 : 16;
         const uint8_t* wrow = W.p[0] + row * (int64_t)nsb * BB;
@@ -277,11 +287,11 @@ struct TQ45_K : TKBase {
                 lo = or4(lo, shl4(shr4(qh, 2 * g, 0x01010101), 4));
                 hi = or4(hi, shl4(shr4(qh, 2 * g + 1, 0x01010101), 4));
             }
-            const int abase = sb * 16 + g * 4 + (j & 1);               // int4 index of act elems 256 sb + 64 g + l0
-            int sum_lo = dot16(lo, A.q[abase]), sum_hi = dot16(hi, A.q[abase + 2]);
+            const int abase = sb * 16 + j;                              // = act_at of the chunk of elems 256 sb + 64 g + l0; the high nibbles' 8 behind
+            int sum_lo = dot16(lo, A.q[abase]), sum_hi = dot16(hi, A.q[abase + 8]);
             int isum = byte_of(s0, s1, 2 * g) * sum_lo + byte_of(s0, s1, 2 * g + 1) * sum_hi;
             // mins: lane j covers min index j  ->  (bsums[2j] + bsums[2j+1]) * mins[j]   (i32: B7 fixed)
-            int msum = ((int)A.bs[sb * 16 + 2 * j] + (int)A.bs[sb * 16 + 2 * j + 1]) * byte_of(m0, m1, j);
+            int msum = A.bsum2(sb * 8 + j) * byte_of(m0, m1, j);
             float da = A.d[sb];
             float d = h2f_bits((uint16_t)(hdr.x & 0xFFFF)) * da, dmin = h2f_bits((uint16_t)((unsigned)hdr.x >> 16)) * da;
             acc += d * (float)isum - dmin * (float)msum;
@@ -310,12 +320,12 @@ struct TQ45_K : TKBase {
                 sl[r] = byte_of(s0, s1, 2 * g); sh[r] = byte_of(s0, s1, 2 * g + 1); mn[r] = byte_of(m0, m1, j);
                 d[r] = h2f_bits((uint16_t)(hdr.x & 0xFFFF)); dm[r] = h2f_bits((uint16_t)((unsigned)hdr.x >> 16));
             }
-            const int abase = sb * 16 + g * 4 + (j & 1);
+            const int abase = sb * 16 + j;
 #pragma unroll
             for (int n = 0; n < NB; n++) {
                 KAct A(sm + n * stride, k);
-                const int4 a0 = A.q[abase], a1 = A.q[abase + 2];
-                const int bs = (int)A.bs[sb * 16 + 2 * j] + (int)A.bs[sb * 16 + 2 * j + 1];
+                const int4 a0 = A.q[abase], a1 = A.q[abase + 8];
+                const int bs = A.bsum2(sb * 8 + j);
                 const float da = A.d[sb];
 #pragma unroll
                 for (int r = 0; r < R; r++) {
@@ -327,9 +337,9 @@ struct TQ45_K : TKBase {
     }
     // ---- the same dot cut into SEGMENTS of 16 super-blocks (4 iterations of the loop above) whose 8 16-byte loads are issued as one
     // batch into a KSeg, so a caller can keep the next segment in flight while it computes the current one (megakernel generic
-    // phase).  Per lane the terms are added in the same order as in row_dot -> identical bits.  x: 4 extra words per segment (Q6_K).
+    // phase).  Per lane the terms are added in the same order as in row_dot -> identical bits.  x: 8 extra words per segment (Q6_K).
     static constexpr bool kSegmented = !FIVE;          // Q5_K would need 4 more 16-byte registers per segment (qh): plain loop
-    static __device__ __forceinline__ void seg_load(KSeg& S, int (&x)[4], const WPlanes& W, int64_t row, int k, int seg, int lane) {
+    static __device__ __forceinline__ void seg_load(KSeg& S, int (&x)[8], const WPlanes& W, int64_t row, int k, int seg, int lane) {
         const int nsb = k >> 8, BB = 144, QOFF = 16;
         const uint8_t* wrow = W.p[0] + row * (int64_t)nsb * BB;
         const int j = lane & 7;
@@ -343,7 +353,7 @@ struct TQ45_K : TKBase {
             }
         }
     }
-    static __device__ __forceinline__ float seg_dot(const KSeg& S, const int (&x)[4], int k, int seg, const uint8_t* sm, int lane, float acc) {
+    static __device__ __forceinline__ float seg_dot(const KSeg& S, const int (&x)[8], int k, int seg, const uint8_t* sm, int lane, float acc) {
         const int nsb = k >> 8;
         KAct A(sm, k);
         const int j = lane & 7, g = j >> 1;
@@ -355,10 +365,10 @@ struct TQ45_K : TKBase {
                 unsigned s0, s1, m0, m1;
                 k4_unpack((unsigned)hdr.y, (unsigned)hdr.z, (unsigned)hdr.w, s0, s1, m0, m1);
                 int4 lo = and4(q, 0x0F0F0F0F), hi = shr4(q, 4, 0x0F0F0F0F);
-                const int abase = sb * 16 + g * 4 + (j & 1);
-                int sum_lo = dot16(lo, A.q[abase]), sum_hi = dot16(hi, A.q[abase + 2]);
+                const int abase = sb * 16 + j;
+                int sum_lo = dot16(lo, A.q[abase]), sum_hi = dot16(hi, A.q[abase + 8]);
                 int isum = byte_of(s0, s1, 2 * g) * sum_lo + byte_of(s0, s1, 2 * g + 1) * sum_hi;
-                int msum = ((int)A.bs[sb * 16 + 2 * j] + (int)A.bs[sb * 16 + 2 * j + 1]) * byte_of(m0, m1, j);
+                int msum = A.bsum2(sb * 8 + j) * byte_of(m0, m1, j);
                 float da = A.d[sb];
                 float d = h2f_bits((uint16_t)(hdr.x & 0xFFFF)) * da, dmin = h2f_bits((uint16_t)((unsigned)hdr.x >> 16)) * da;
                 acc += d * (float)isum - dmin * (float)msum;
@@ -370,6 +380,9 @@ struct TQ45_K : TKBase {
 
 // Q6_K: buf_q6_k.rs:183-235.  8 lanes per super-block, lane j owns ql chunk j.
 struct TQ6_K : TKBase {
+    // chunk 8 n + 4 h + 2 p + r of a super-block: the low (h = 0) or high nibbles of weight chunk j = 4 n + 2 p + r
+    static __host__ __device__ __forceinline__ int act_at(int i) { return (i & ~15) | ((i & 4) << 1) | ((i & 8) >> 1) | (i & 3); }
+    static __device__ void stage_act(const void* scratch, int64_t n_total, int bi, int k, uint8_t* sm) { stage_act_as<TQ6_K>(scratch, n_total, bi, k, sm); }
     static __device__ float row_dot(const WPlanes& W, int64_t row, int k, const uint8_t* sm, int lane) {
         const int nsb = k >> 8;
         const uint8_t* ql = W.p[0] + row * (int64_t)nsb * 128;
@@ -386,8 +399,8 @@ struct TQ6_K : TKBase {
             int4 hi = or4(shr4(l, 4, 0x0F0F0F0F), shl4(shr4(h, 2 * p + 4, 0x03030303), 4));
             const int e_lo = 128 * n + 32 * p + 16 * r;                 // element offset inside the super-block
             const int a_lo = sb * 16 + (e_lo >> 4), a_hi = a_lo + 4;
-            int s_lo = dot16(lo, A.q[a_lo]) - 32 * (int)A.bs[a_lo];     // sum (q-32)*a
-            int s_hi = dot16(hi, A.q[a_hi]) - 32 * (int)A.bs[a_hi];
+            int s_lo = dot16(lo, A.q[sb * 16 + j]) - 32 * (int)A.bs[a_lo];     // sum (q-32)*a
+            int s_hi = dot16(hi, A.q[sb * 16 + j + 8]) - 32 * (int)A.bs[a_hi];
             int isum = (int)sc[sb * 16 + (e_lo >> 4)] * s_lo + (int)sc[sb * 16 + (e_lo >> 4) + 4] * s_hi;
             acc += (float)isum * (h2f_bits(wd[sb]) * A.d[sb]);
         }
@@ -414,7 +427,7 @@ struct TQ6_K : TKBase {
 #pragma unroll
             for (int n = 0; n < NB; n++) {
                 KAct A(sm + n * stride, k);
-                const int4 a0 = A.q[a_lo], a1 = A.q[a_hi];
+                const int4 a0 = A.q[sb * 16 + j], a1 = A.q[sb * 16 + j + 8];
                 const int b0 = 32 * (int)A.bs[a_lo], b1 = 32 * (int)A.bs[a_hi];
                 const float da = A.d[sb];
 #pragma unroll
@@ -424,7 +437,7 @@ struct TQ6_K : TKBase {
     }
     // segments of 16 super-blocks, loads batched (see TQ45_K): ql chunk, qh chunk, the two sub-block scales and d per iteration
     static constexpr bool kSegmented = true;
-    static __device__ __forceinline__ void seg_load(KSeg& S, int (&x)[4], const WPlanes& W, int64_t row, int k, int seg, int lane) {
+    static __device__ __forceinline__ void seg_load(KSeg& S, int (&x)[8], const WPlanes& W, int64_t row, int k, int seg, int lane) {
         const int nsb = k >> 8;
         const uint8_t* ql = W.p[0] + row * (int64_t)nsb * 128;
         const uint8_t* qh = W.p[1] + row * (int64_t)nsb * 64;
@@ -438,12 +451,13 @@ struct TQ6_K : TKBase {
             if (sb < nsb) {
                 S.a[it] = ld_stream_16(ql + (int64_t)sb * 128 + 16 * j);
                 S.b[it] = ld_stream_16(qh + (int64_t)sb * 64 + 32 * n + 16 * r);
-                x[it] = ((int)sc[sb * 16 + (e_lo >> 4)] & 0xFFFF) | ((int)sc[sb * 16 + (e_lo >> 4) + 4] << 16);     // the two sub-block scales
+                const int2 v = *(const int2*)(sc + sb * 16 + 8 * n);           // holds the lane's two sub-block scales; picked out when they are used: here
+                x[2 * it] = v.x; x[2 * it + 1] = v.y;                          // that would wait for the load and with it for every request ahead of it
                 S.s[it] = wd[sb];
             }
         }
     }
-    static __device__ __forceinline__ float seg_dot(const KSeg& S, const int (&x)[4], int k, int seg, const uint8_t* sm, int lane, float acc) {
+    static __device__ __forceinline__ float seg_dot(const KSeg& S, const int (&x)[8], int k, int seg, const uint8_t* sm, int lane, float acc) {
         const int nsb = k >> 8;
         KAct A(sm, k);
         const int j = lane & 7, n = j >> 2, jj = j & 3, r = jj & 1, p = jj >> 1;
@@ -456,9 +470,9 @@ struct TQ6_K : TKBase {
                 int4 lo = or4(and4(l, 0x0F0F0F0F), shl4(shr4(h, 2 * p, 0x03030303), 4));
                 int4 hi = or4(shr4(l, 4, 0x0F0F0F0F), shl4(shr4(h, 2 * p + 4, 0x03030303), 4));
                 const int a_lo = sb * 16 + (e_lo >> 4), a_hi = a_lo + 4;
-                int s_lo = dot16(lo, A.q[a_lo]) - 32 * (int)A.bs[a_lo];
-                int s_hi = dot16(hi, A.q[a_hi]) - 32 * (int)A.bs[a_hi];
-                int isum = (int)(int16_t)(x[it] & 0xFFFF) * s_lo + (x[it] >> 16) * s_hi;
+                int s_lo = dot16(lo, A.q[sb * 16 + j]) - 32 * (int)A.bs[a_lo];
+                int s_hi = dot16(hi, A.q[sb * 16 + j + 8]) - 32 * (int)A.bs[a_hi];
+                int isum = (int)(int8_t)(x[2 * it] >> (8 * (2 * p + r))) * s_lo + (int)(int8_t)(x[2 * it + 1] >> (8 * (2 * p + r))) * s_hi;
                 acc += (float)isum * (h2f_bits(S.s[it]) * A.d[sb]);
             }
         }

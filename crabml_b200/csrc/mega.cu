@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(MK_THREADS, MK_CTAS_PER_SM) mega_kernel(const 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
+    AtPre at_pre = {0, 0, 0.0f, 0.0f};
     MkPipe pipe;                             // weight prefetch registers, live across phases and barriers
     uint8_t* work = smem;                    // per-phase working area (activation arrays, attention tiles)
     float* s_w = (float*)(smem + wtop_off);  // norm weights of the next fused prologue (top of dynamic shared memory)
@@ -281,6 +282,7 @@ __global__ void __launch_bounds__(MK_THREADS, MK_CTAS_PER_SM) mega_kernel(const 
         if (stamp) { prof[p * MK_PROF_SLOTS] = globaltimer_ns(); prof[p * MK_PROF_SLOTS + 1] = 0; prof[p * MK_PROF_SLOTS + 4] = 0; prof[p * MK_PROF_SLOTS + 5] = 0; }
         __syncthreads();                     // descriptor p is in shared memory (stored one phase ago)
         const MkPhase& s_ph = s_phs[p & 1];
+        if (p == 0 && s_ph.type == MK_ATTN) at_pre = at_ask(s_ph, (float*)work, dyn, abar0, AT_CH);
         // Descriptor p+1 and the arguments of the next MATVEC phases (look-ahead prefetch) are LOADED now, into one register each,
         // and STORED to shared memory after the phase body: a load followed directly by its st.shared would block the thread for
         // an L2 round trip (in-order issue) before it could issue the phase's own loads.
@@ -328,7 +330,8 @@ __global__ void __launch_bounds__(MK_THREADS, MK_CTAS_PER_SM) mega_kernel(const 
                                                early ? s_next : nullptr, next_w));
             break;
         case MK_ATTN:
-            if (s_ph.at.kv_f16) phase_attn<true>(s_ph, (float*)work, s_red, dyn, exp_lut, abar0, apar, AT_CH); else phase_attn<false>(s_ph, (float*)work, s_red, dyn, exp_lut, abar0, apar, AT_CH);
+            if (s_ph.at.kv_f16) phase_attn<true>(s_ph, (float*)work, s_red, at_pre, exp_lut, abar0, apar, AT_CH); else phase_attn<false>(s_ph, (float*)work, s_red, at_pre, exp_lut, abar0, apar, AT_CH);
+            at_pre.jobs = 0;
             break;
         case MK_ROWS: phase_rows(s_ph, dyn); break;
         case MK_REDUCE: phase_reduce(s_ph, comm, xseq, false); break;
@@ -362,11 +365,12 @@ __global__ void __launch_bounds__(MK_THREADS, MK_CTAS_PER_SM) mega_kernel(const 
                 wstaged = nx;
             }
         }
+        if (more && s_phs[(p + 1) & 1].type == MK_ATTN) at_pre = at_ask(s_phs[(p + 1) & 1], (float*)work, dyn, abar0, AT_CH);
         if (stamp) prof[p * MK_PROF_SLOTS + 3] = globaltimer_ns();
         if (more) {
             grid_barrier_wait(bar, gridDim.x, gen, comm, xg ? xseq + 1u : 0u, (flags & MK_F_POLLCNT) != 0, &s_abort, err_host);
             gen++; if (xg) xseq++;
-            if (s_abort) break;              // a barrier timed out (a CTA never became resident, or a peer GPU died): bail out, host reports
+            if (s_abort) { if (threadIdx.x == 0) at_drain(at_pre.jobs, abar0, apar); break; }              // a barrier timed out (a CTA never became resident, or a peer GPU died): bail out, host reports
             // the barrier is open: the row the next fused prologue normalises is complete -- request it before anything else (descriptor
             // bookkeeping, geometry, look-ahead loads) so that its L2 round trip overlaps them
             const MkPhase& nph = s_phs[(p + 1) & 1];

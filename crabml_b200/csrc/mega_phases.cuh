@@ -111,56 +111,53 @@ __device__ __forceinline__ float mk_block_sum_512(float v, float* s_red /* [16] 
 
 
 // ---- NORMQ phase (fused.cu normq_kernel, grid-wide) -----------------------------------------------------------------
+// Run once or twice a token, so its instructions come from memory each time: a short loop over 16-byte chunks (8 lanes to a block of 32).  The row of
+// 4096 that one CTA keeps whole took 9.5 us as eight unrolled blocks a warp (12.5 with their loads batched), 4.7 us this way.
 static __device__ void phase_normq(const MkPhase& ph, float* s_red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = ph.n;
-    float* x = ph.x;
+    const int n4 = ph.n >> 2;
+    float4* x = (float4*)ph.x;
     float rms = 1.0f;
     // write_back: the normalised row must be materialised in place -> one CTA does the whole row (nobody else may
     // still be summing x while it is overwritten)
     if (ph.write_back && blockIdx.x != 0) return;
-    // this warp's blocks are requested first, so their latency overlaps the row pass below (one L2 round trip in total)
-    const int nb0 = n >> 5;
-    const int gw0 = ph.write_back ? warp : blockIdx.x * MK_WARPS + warp, tw0 = ph.write_back ? MK_WARPS : gridDim.x * MK_WARPS;
-    float pre[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) { const int b = gw0 + j * tw0; pre[j] = b < nb0 ? ldcg_f(x + b * 32 + lane) : 0.0f; }
     if (ph.norm_w) {
         float ss = 0.0f;
-        const float4* x4 = (const float4*)x;
-        const int n4 = n >> 2;
-        for (int i0 = 0; i0 < n4; i0 += MK_THREADS * 4) {
-            float4 v[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) { int i = i0 + j * MK_THREADS + threadIdx.x; v[j] = i < n4 ? __ldcg(x4 + i) : make_float4(0, 0, 0, 0); }
-#pragma unroll
-            for (int j = 0; j < 4; j++) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
-        }
+#pragma unroll 2
+        for (int i = threadIdx.x; i < n4; i += MK_THREADS) ss += cc_sq4(__ldcg(x + i));
         ss = warp_sum(ss);
         if (lane == 0) s_red[warp] = ss;
         MK_SYNC();
         float t = 0.0f;
 #pragma unroll
         for (int w = 0; w < MK_WARPS; w++) t += s_red[w];
-        rms = sqrtf(t / (float)n + ph.eps);
+        rms = sqrtf(t / (float)ph.n + ph.eps);
         MK_SYNC();
     }
     ActQ8_0 act = ph.act;
-    const int nb = n >> 5;
-    const int gw = ph.write_back ? warp : blockIdx.x * MK_WARPS + warp, tw = ph.write_back ? MK_WARPS : gridDim.x * MK_WARPS;
-    auto do_block = [&](int b, float v) {
-        if (ph.orig) ph.orig[b * 32 + lane] = v;
-        if (ph.norm_w) { v = (v / rms) * ph.norm_w[b * 32 + lane]; if (ph.write_back) x[b * 32 + lane] = v; }
-        float amax = warp_max(fabsf(v));
-        float d = amax / 127.0f;
-        int q = __float2int_rz(v / d);
-        act.qs[b * 32 + lane] = (int8_t)q;
-        int s = warp_sum_i(q);
-        if (lane == 0) { act.d[b] = __half2float(__float2half_rn(d)); act.isum[b] = s; }
-    };
+    const int step = ph.write_back ? MK_THREADS : (int)gridDim.x * MK_THREADS;
+    // (whole warps stay together: n is a multiple of 32, the lanes of a block are in or out as one)
+#pragma unroll 1
+    for (int i = (ph.write_back ? 0 : (int)blockIdx.x * MK_THREADS) + (int)threadIdx.x; i - lane < n4; i += step) {
+        const bool on = i < n4;
+        float4 v = on ? __ldcg(x + i) : make_float4(0, 0, 0, 0);
+        if (on && ph.orig) ((float4*)ph.orig)[i] = v;
+        if (on && ph.norm_w) {
+            const float4 w = ((const float4*)ph.norm_w)[i];
+            v.x = (v.x / rms) * w.x; v.y = (v.y / rms) * w.y; v.z = (v.z / rms) * w.z; v.w = (v.w / rms) * w.w;
+            if (ph.write_back) x[i] = v;
+        }
+        float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 #pragma unroll
-    for (int j = 0; j < 4; j++) { const int b = gw + j * tw; if (b < nb) do_block(b, pre[j]); }
-    for (int b = gw + 4 * tw; b < nb; b += tw) do_block(b, ldcg_f(x + b * 32 + lane));
+        for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        const float d = amax / 127.0f;
+        const int q0 = __float2int_rz(v.x / d), q1 = __float2int_rz(v.y / d), q2 = __float2int_rz(v.z / d), q3 = __float2int_rz(v.w / d);
+        int s = q0 + q1 + q2 + q3;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (on) ((int*)act.qs)[i] = (q0 & 255) | ((q1 & 255) << 8) | ((q2 & 255) << 16) | (q3 << 24);
+        if (on && (lane & 7) == 0) { act.d[i >> 3] = __half2float(__float2half_rn(d)); act.isum[i >> 3] = s; }
+    }
 }
 
 // ---- MATVEC phase: the body of matvec_stream_kernel (see matvec_stream.cu for the design notes) -------------------------
@@ -332,23 +329,6 @@ static __device__ MK_GENERIC_ATTR void phase_matvec_generic(const MkPhase& ph, u
         W.p[3] = mat == 0 ? M.p3[0] : mat == 1 ? M.p3[1] : M.p3[2];
         return W;
     };
-    // rows cut into segments of 16 super-blocks; the loads of segment u + 2 are issued before segment u + 1 is consumed (two
-    // segments = 16-24 LDG.128 per lane in flight), across row boundaries.  The first two are on their way while the activation is prepared
-    const int NSEG = ((k >> 8) + 15) >> 4;
-    const int U = n_vrows * NSEG;
-#if MK_GENERIC_NOINLINE
-    KSeg S0, S1;
-#else
-    KSeg& S0 = P.buf0;                                                   // the weight pipe's registers (no streaming look-ahead is pending: caller)
-    KSeg& S1 = P.buf1;
-#endif
-    int x0[8] = {}, x1[8] = {};
-    int l_i = 0, l_seg = 0;
-    auto load = [&](KSeg& S, int (&x)[8], bool valid) {
-        if (valid) { int mat; const int r = locate(l_i, mat); T::seg_load(S, x, planes(mat), r, k, l_seg, lane); }
-        if (++l_seg == NSEG) { l_seg = 0; l_i++; }
-    };
-    if constexpr (T::kSegmented && !MK_GENERIC_NOINLINE) { load(S0, x0, U > 0); load(S1, x1, U > 1); }
     {   // one L2 round trip: the f32 row (unless requested right after the barrier) and the norm weights (unless staged before it)
         const int n4 = k >> 2;
         const unsigned sx = (unsigned)__cvta_generic_to_shared(s_x), sw = (unsigned)__cvta_generic_to_shared(s_w);
@@ -414,7 +394,25 @@ static __device__ MK_GENERIC_ATTR void phase_matvec_generic(const MkPhase& ph, u
         }
     };
     if constexpr (T::kSegmented) {
-        if constexpr (MK_GENERIC_NOINLINE) { load(S0, x0, U > 0); load(S1, x1, U > 1); }
+        // rows cut into segments of 16 super-blocks; the loads of segment u + 2 are issued before segment u + 1 is consumed (two
+        // segments = 16-24 LDG.128 per lane in flight), across row boundaries
+        // (the first two ahead of the prologue: its own loads wait behind them, rows and prologue together take as long)
+        const int NSEG = ((k >> 8) + 15) >> 4;
+        const int U = n_vrows * NSEG;
+#if MK_GENERIC_NOINLINE
+        KSeg S0, S1;
+#else
+        KSeg& S0 = P.buf0;                                                   // the weight pipe's registers (no streaming look-ahead is pending: caller)
+        KSeg& S1 = P.buf1;
+#endif
+        int x0[8] = {}, x1[8] = {};
+        int l_i = 0, l_seg = 0;
+        auto load = [&](KSeg& S, int (&x)[8], bool valid) {
+            if (valid) { int mat; const int r = locate(l_i, mat); T::seg_load(S, x, planes(mat), r, k, l_seg, lane); }
+            if (++l_seg == NSEG) { l_seg = 0; l_i++; }
+        };
+        load(S0, x0, U > 0);
+        load(S1, x1, U > 1);
         float acc = 0.0f;
         int c_i = 0, c_seg = 0;
         auto finish = [&]() { if (++c_seg < NSEG) return; c_seg = 0; const float v = warp_sum(acc); acc = 0.0f; emit(c_i++, v); };
@@ -438,37 +436,69 @@ static __device__ MK_GENERIC_ATTR void phase_matvec_generic(const MkPhase& ph, u
 }
 
 // ---- ATTN phase: arithmetic of fused.cu attn_decode_kernel, heads dealt to CTAs.  The K (then V) rows of the head are
-// staged in shared memory in chunks of AT_CH positions with ALL loads of a chunk in flight at once: at decode the cost of
+// staged in shared memory in chunks of at_ch positions with ALL loads of a chunk in flight at once: at decode the cost of
 // this phase is HBM/L2 latency, not bandwidth, so round trips are what matters.
 #define AT_CH 64
 #define AT_NBUF 3
+// What does not depend on the phase before -- the length, the RoPE angles, the cached rows (written by earlier launches) -- is requested while the CTA waits
+// at the barrier in front of the phase (at_ask), so that the barrier covers those round trips.  jobs: chunks already under way for head blockIdx.x.
+struct AtPre { int kv_len, jobs; float c, s; };
+__device__ __forceinline__ uint8_t* at_buffers(const AttnArgs& a, float* sm) { return (uint8_t*)(sm + 3 * a.hd + ((a.max_len + 8 + 3) & ~3)); }
+// job j of the sequence K chunks 0 .. NC - 1, V chunks 0 .. NC - 1 of kv head g; one elected thread
+template <int ELT>
+__device__ __forceinline__ void at_issue(const AttnArgs& a, int g, int j, int NC, int kv_len, int at_ch, unsigned s_buf_smem, unsigned abar0) {
+    const int c = j < NC ? j : j - NC;
+    const int p0 = c * at_ch, cnt = min(at_ch, kv_len - p0);
+    const uint8_t* src = (const uint8_t*)(j < NC ? a.kcache : a.vcache) + ((int64_t)g * a.seq_stride + (int64_t)p0 * a.hd) * ELT;
+    const unsigned bytes = (unsigned)(cnt * a.hd * ELT), bar = abar0 + 8u * (unsigned)(j % AT_NBUF), dst = s_buf_smem + (unsigned)(j % AT_NBUF) * (unsigned)(at_ch * a.hd * ELT);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+// the caller's compute threads have left the working area (their barrier is behind them)
+__device__ __forceinline__ AtPre at_ask(const MkPhase& ph, float* sm, const uint8_t* dyn, unsigned abar0, int at_ch) {
+    AtPre pre = {0, 0, 0.0f, 0.0f};
+    const AttnArgs& a = ph.at;
+    if ((int)blockIdx.x >= a.n_heads) return pre;
+    pre.kv_len = (int)((const int64_t*)(dyn + ph.dyn_off))[1];
+    const float* rope_tab = (const float*)(dyn + ph.rope_off);
+    if ((int)threadIdx.x < a.rope_dim) { pre.c = rope_tab[threadIdx.x >> 1]; pre.s = rope_tab[(a.rope_dim >> 1) + (threadIdx.x >> 1)]; }
+    const int NC = (pre.kv_len + at_ch - 1) / at_ch, h = blockIdx.x;
+    pre.jobs = min(AT_NBUF, 2 * NC);
+    if (threadIdx.x == 0) {
+        const unsigned buf = (unsigned)__cvta_generic_to_shared(at_buffers(a, sm));
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");             // the last phase's stores to the same bytes
+        for (int j = 0; j < pre.jobs; j++) {
+            if (a.kv_f16) at_issue<2>(a, h / (a.n_heads / a.n_kv), j, NC, pre.kv_len, at_ch, buf, abar0);
+            else at_issue<4>(a, h % a.n_kv, j, NC, pre.kv_len, at_ch, buf, abar0);
+        }
+    }
+    return pre;
+}
+// a launch that gives up behind at_ask: its copies land before the CTA's shared memory goes (they need nobody; a second is far beyond their microseconds)
+__device__ __forceinline__ void at_drain(int jobs, unsigned abar0, unsigned apar) {
+    const unsigned long long t0 = globaltimer_ns();
+    for (int j = 0; j < jobs; j++) {
+        unsigned ok = 0;
+        while (!ok && globaltimer_ns() - t0 < 1000000000ull)
+            asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(abar0 + 8u * (unsigned)j), "r"((apar >> j) & 1u) : "memory");
+    }
+}
+// per layer of a 7B model at a short context, barrier included: 8.5 -> 7.3 us in the ring kernel, 7.5 -> 6.7 in the other
 template <bool KV_F16>
-static __device__ void phase_attn(const MkPhase& ph, float* sm, float* s_red, const uint8_t* dyn, const uint16_t* exp_lut, unsigned abar0, unsigned& apar, const int at_ch) {
+static __device__ void phase_attn(const MkPhase& ph, float* sm, float* s_red, const AtPre& pre, const uint16_t* exp_lut, unsigned abar0, unsigned& apar, const int at_ch) {
     const AttnArgs& a = ph.at;
     const int n_heads = a.n_heads, n_kv = a.n_kv, hd = a.hd, rope_dim = a.rope_dim;
     const int64_t seq_stride = a.seq_stride;
-    const int64_t* dynv = (const int64_t*)(dyn + ph.dyn_off);
-    const float* rope_tab = (const float*)(dyn + ph.rope_off);
-    const int kv_len = (int)dynv[1], L = kv_len + 1;
+    const int kv_len = pre.kv_len, L = kv_len + 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* s_q = sm; float* s_k = sm + hd; float* s_v = sm + 2 * hd; float* s_p = sm + 3 * hd;
     // AT_NBUF chunk buffers of at_ch cache rows each (raw bytes: f32 or f16), filled by TMA bulk copies -- the rows of one kv head
     // are contiguous -- in a K-chunks-then-V-chunks job sequence with AT_NBUF jobs in flight; one mbarrier per buffer.
-    uint8_t* s_buf = (uint8_t*)(sm + 3 * hd + ((a.max_len + 8 + 3) & ~3));
+    uint8_t* s_buf = at_buffers(a, sm);
     const unsigned s_buf_smem = (unsigned)__cvta_generic_to_shared(s_buf);
     constexpr int ELT = KV_F16 ? 2 : 4;
     const unsigned buf_bytes = (unsigned)(at_ch * hd * ELT);
-    const int pairs = rope_dim >> 1;
-    const int hd4 = hd >> 2;
     const int NC = (kv_len + at_ch - 1) / at_ch;                  // chunks per pass; jobs 0..NC-1 = K chunks, NC..2NC-1 = V chunks
-    auto issue_job = [&](int g, int j) {                            // one elected thread
-        const int c = j < NC ? j : j - NC;
-        const int p0 = c * at_ch, cnt = min(at_ch, kv_len - p0);
-        const uint8_t* src = (const uint8_t*)(j < NC ? a.kcache : a.vcache) + ((int64_t)g * seq_stride + (int64_t)p0 * hd) * ELT;
-        const unsigned bytes = (unsigned)(cnt * hd * ELT), bar = abar0 + 8u * (unsigned)(j % AT_NBUF), dst = s_buf_smem + (unsigned)(j % AT_NBUF) * buf_bytes;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-    };
     auto wait_job = [&](int j) {                                    // all threads, in job order
         const int bsel = j % AT_NBUF;
         mbar_wait(abar0 + 8u * (unsigned)bsel, (apar >> bsel) & 1u);
@@ -478,23 +508,22 @@ static __device__ void phase_attn(const MkPhase& ph, float* sm, float* s_red, co
     for (int h = blockIdx.x; h < n_heads; h += gridDim.x) {
         const int g = KV_F16 ? h / (n_heads / n_kv) : h % n_kv;
         // the first AT_NBUF jobs are requested up front; every later job is issued as soon as its buffer has been consumed
-        if (threadIdx.x == 0) for (int j = 0; j < min(AT_NBUF, 2 * NC); j++) issue_job(g, j);
-        for (int i = threadIdx.x; i < hd; i += MK_THREADS) {
+        if (threadIdx.x == 0 && h != (int)blockIdx.x) for (int j = 0; j < min(AT_NBUF, 2 * NC); j++) at_issue<ELT>(a, g, j, NC, kv_len, at_ch, s_buf_smem, abar0);
+        for (int i = threadIdx.x; i < hd; i += MK_THREADS) {      // hd <= MK_THREADS (the fuser): one element a thread
             float qv, kvv;
             if (i < rope_dim) {
                 const int j = i >> 1;
-                const float c = rope_tab[j], s = rope_tab[pairs + j];
                 const float q0 = ldcg_f(a.q + h * hd + 2 * j), q1 = ldcg_f(a.q + h * hd + 2 * j + 1);
                 const float k0 = ldcg_f(a.k + g * hd + 2 * j), k1 = ldcg_f(a.k + g * hd + 2 * j + 1);
-                qv = (i & 1) ? q0 * s + q1 * c : q0 * c - q1 * s;
-                kvv = (i & 1) ? k0 * s + k1 * c : k0 * c - k1 * s;
+                qv = (i & 1) ? q0 * pre.s + q1 * pre.c : q0 * pre.c - q1 * pre.s;
+                kvv = (i & 1) ? k0 * pre.s + k1 * pre.c : k0 * pre.c - k1 * pre.s;
             } else {
                 qv = ldcg_f(a.q + h * hd + i);
                 kvv = ldcg_f(a.k + g * hd + i);
             }
+            s_v[i] = ldcg_f(a.v + g * hd + i);
             s_q[i] = qv * a.scale;
             s_k[i] = kvv;
-            s_v[i] = ldcg_f(a.v + g * hd + i);
         }
         MK_SYNC();
         const bool owner = KV_F16 ? (h % (n_heads / n_kv) == 0) : (h < n_kv);
@@ -505,21 +534,7 @@ static __device__ void phase_attn(const MkPhase& ph, float* sm, float* s_red, co
                 else { ((float*)a.kcache)[off] = s_k[i]; ((float*)a.vcache)[off] = s_v[i]; }
             }
         }
-        // scores, chunk by chunk; per-lane summation order i = lane, lane+32, ... as in fused.cu
-        for (int j = 0; j < NC; j++) {
-            const int p0 = j * at_ch, cnt = min(at_ch, kv_len - p0);
-            const uint8_t* kb = s_buf + (size_t)(j % AT_NBUF) * buf_bytes;
-            wait_job(j);
-            for (int s = warp; s < cnt; s += MK_WARPS) {
-                float acc = 0.0f;
-                for (int i = lane; i < hd; i += 32) acc += (KV_F16 ? __half2float(__float2half_rn(s_q[i])) : s_q[i]) * ld_kv(kb, s * hd + i);
-                acc = warp_sum(acc);
-                if (lane == 0) s_p[p0 + s] = acc;
-            }
-            MK_SYNC();                                       // buffer consumed by every warp -> refill it
-            if (threadIdx.x == 0 && j + AT_NBUF < 2 * NC) issue_job(g, j + AT_NBUF);
-        }
-        if (warp == 0) {                                           // this token's own position
+        if (warp == MK_WARPS - 1) {                                // this token's own position
             float acc = 0.0f;
             for (int i = lane; i < hd; i += 32) {
                 if (KV_F16) acc += __half2float(__float2half_rn(s_q[i])) * __half2float(__float2half_rn(s_k[i]));
@@ -528,29 +543,64 @@ static __device__ void phase_attn(const MkPhase& ph, float* sm, float* s_red, co
             acc = warp_sum(acc);
             if (lane == 0) s_p[kv_len] = acc;
         }
+        // scores, chunk by chunk, two positions of a warp at a time; per-lane summation order i = lane, lane+32, ... as in fused.cu
+        for (int j = 0; j < NC; j++) {
+            const int p0 = j * at_ch, cnt = min(at_ch, kv_len - p0);
+            const uint8_t* kb = s_buf + (size_t)(j % AT_NBUF) * buf_bytes;
+            wait_job(j);
+            for (int s = warp; s < cnt; s += 2 * MK_WARPS) {
+                const int s2 = min(s + MK_WARPS, cnt - 1);          // behind the chunk: its last position once more, not stored
+                float acc = 0.0f, acc2 = 0.0f;
+                for (int i = lane; i < hd; i += 32) {
+                    const float qv = KV_F16 ? __half2float(__float2half_rn(s_q[i])) : s_q[i];
+                    acc += qv * ld_kv(kb, s * hd + i);
+                    acc2 += qv * ld_kv(kb, s2 * hd + i);
+                }
+                acc = warp_sum(acc); acc2 = warp_sum(acc2);
+                if (lane == 0) { s_p[p0 + s] = acc; if (s + MK_WARPS < cnt) s_p[p0 + s2] = acc2; }
+            }
+            if (j + AT_NBUF < 2 * NC) {
+                MK_SYNC();                                       // buffer consumed by every warp -> refill it
+                if (threadIdx.x == 0) at_issue<ELT>(a, g, j + AT_NBUF, NC, kv_len, at_ch, s_buf_smem, abar0);
+            }
+        }
         MK_SYNC();
         float m = -INFINITY;
-        for (int s = threadIdx.x; s < L; s += MK_THREADS) m = fmaxf(m, s_p[s]);
-        m = warp_max(m);
-        if (lane == 0) s_red[warp] = m;
-        MK_SYNC();
-        m = s_red[0];
+        if (L <= MK_THREADS) {                                     // every warp reads all scores: no exchange, and an exponential of its own per thread
+            for (int s = lane; s < L; s += 32) m = fmaxf(m, s_p[s]);
+            m = warp_max(m);
+            const bool on = (int)threadIdx.x < L;
+            const float e = on ? h2f_bits(exp_lut[f2h_bits(s_p[threadIdx.x] - m)]) : 0.0f;
+            const float part = warp_sum(e);
+            if (lane == 0) s_red[warp] = part;
+            MK_SYNC();
+            float sum = 0.0f;
 #pragma unroll
-        for (int w = 1; w < MK_WARPS; w++) m = fmaxf(m, s_red[w]);
-        MK_SYNC();
-        float sum = 0.0f;
-        for (int s = threadIdx.x; s < L; s += MK_THREADS) {
-            float e = h2f_bits(exp_lut[f2h_bits(s_p[s] - m)]);
-            s_p[s] = e;
-            sum += e;
+            for (int w = 0; w < MK_WARPS; w++) sum += s_red[w];
+            if (on) s_p[threadIdx.x] = e / sum;
+        } else {
+            for (int s = threadIdx.x; s < L; s += MK_THREADS) m = fmaxf(m, s_p[s]);
+            m = warp_max(m);
+            if (lane == 0) s_red[warp] = m;
+            MK_SYNC();
+            m = s_red[0];
+#pragma unroll
+            for (int w = 1; w < MK_WARPS; w++) m = fmaxf(m, s_red[w]);
+            MK_SYNC();
+            float sum = 0.0f;
+            for (int s = threadIdx.x; s < L; s += MK_THREADS) {
+                float e = h2f_bits(exp_lut[f2h_bits(s_p[s] - m)]);
+                s_p[s] = e;
+                sum += e;
+            }
+            sum = warp_sum(sum);
+            if (lane == 0) s_red[warp] = sum;
+            MK_SYNC();
+            sum = 0.0f;
+#pragma unroll
+            for (int w = 0; w < MK_WARPS; w++) sum += s_red[w];
+            for (int s = threadIdx.x; s < L; s += MK_THREADS) s_p[s] = s_p[s] / sum;
         }
-        sum = warp_sum(sum);
-        if (lane == 0) s_red[warp] = sum;
-        MK_SYNC();
-        sum = 0.0f;
-#pragma unroll
-        for (int w = 0; w < MK_WARPS; w++) sum += s_red[w];
-        for (int s = threadIdx.x; s < L; s += MK_THREADS) s_p[s] = s_p[s] / sum;
         MK_SYNC();
         // out[d] = sum_s p[s] * V[s][d], sequential over s (batch_matmul.rs:60-68 order); F16: f16 accumulation (buf_f16.rs:152-163)
         float accf = 0.0f;
@@ -561,38 +611,34 @@ static __device__ void phase_attn(const MkPhase& ph, float* sm, float* s_red, co
             const uint8_t* vb = s_buf + (size_t)(j % AT_NBUF) * buf_bytes;
             wait_job(j);
             if (d < hd) {
+#pragma unroll 8
                 for (int s = 0; s < cnt; s++) {
                     if (KV_F16) acch = __hadd(acch, __hmul(((const __half*)vb)[s * hd + d], __float2half_rn(s_p[p0 + s])));
                     else accf += s_p[p0 + s] * ((const float*)vb)[s * hd + d];
                 }
             }
-            MK_SYNC();
-            if (threadIdx.x == 0 && j + AT_NBUF < 2 * NC) issue_job(g, j + AT_NBUF);
+            if (j + AT_NBUF < 2 * NC) {
+                MK_SYNC();
+                if (threadIdx.x == 0) at_issue<ELT>(a, g, j + AT_NBUF, NC, kv_len, at_ch, s_buf_smem, abar0);
+            }
         }
-        float* s_o = s_k;
-        MK_SYNC();
+        float o = 0.0f;
         if (d < hd) {
-            float o;
             if (KV_F16) { acch = __hadd(acch, __hmul(__float2half_rn(s_v[d]), __float2half_rn(s_p[kv_len]))); o = __half2float(acch); }
             else { accf += s_p[kv_len] * s_v[d]; o = accf; }
             a.out[h * hd + d] = o;
-            s_o[d] = o;
         }
-        MK_SYNC();
-        if (a.act_scratch) {
+        if (a.act_scratch && warp < (hd >> 5)) {                   // block `warp` of the head's output lies in this warp's registers
             ActQ8_0 act = ph.act;
-            for (int b = warp; b < (hd >> 5); b += MK_WARPS) {
-                float v = s_o[b * 32 + lane];
-                float amax = warp_max(fabsf(v));
-                float dd = amax / 127.0f;
-                int qq = __float2int_rz(v / dd);
-                const int gb = h * (hd >> 5) + b;
-                act.qs[gb * 32 + lane] = (int8_t)qq;
-                int ss = warp_sum_i(qq);
-                if (lane == 0) { act.d[gb] = __half2float(__float2half_rn(dd)); act.isum[gb] = ss; }
-            }
+            const float amax = warp_max(fabsf(o));
+            const float dd = amax / 127.0f;
+            const int qq = __float2int_rz(o / dd);
+            const int gb = h * (hd >> 5) + warp;
+            act.qs[gb * 32 + lane] = (int8_t)qq;
+            const int ss = warp_sum_i(qq);
+            if (lane == 0) { act.d[gb] = __half2float(__float2half_rn(dd)); act.isum[gb] = ss; }
         }
-        MK_SYNC();
+        if (h + (int)gridDim.x < n_heads) MK_SYNC();               // the next head's rows go where this one's were
     }
 }
 

@@ -371,8 +371,9 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
             const float d = amax / 127.0f;
-            const int q0 = live ? __float2int_rz(v.x / d) : 0, q1 = live ? __float2int_rz(v.y / d) : 0;
-            const int q2 = live ? __float2int_rz(v.z / d) : 0, q3 = live ? __float2int_rz(v.w / d) : 0;
+            v = make_float4(v.x / d, v.y / d, v.z / d, v.w / d);
+            const int q0 = live ? __float2int_rz(v.x) : 0, q1 = live ? __float2int_rz(v.y) : 0;
+            const int q2 = live ? __float2int_rz(v.z) : 0, q3 = live ? __float2int_rz(v.w) : 0;
             s_q32[mr_act_word(i)] = (q0 & 255) | ((q1 & 255) << 8) | ((q2 & 255) << 16) | (q3 << 24);
             if constexpr (TYPE == CC_Q4_0) {
                 int sq = q0 + q1 + q2 + q3;
@@ -550,6 +551,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
     MrCons RC;
     RC.full0 = full0; RC.done0 = done0; RC.ring = smem + R.ring_off; RC.slot_bytes = R.slot_bytes; RC.nslots = R.nslots; RC.ent_base = 0u;
     RC.pairs = (flags & MK_F_RPAIR) != 0; RC.s_unit = &s_unit; RC.s_seq = s_seq; RC.s_dead = &s_ring_dead; RC.err_dev = &bar[MK_BAR_ERR]; RC.err_host = err_host;
+    AtPre at_pre = {0, 0, 0.0f, 0.0f};
     uint8_t* work = smem;
     float* s_w = (float*)(smem + wtop_off);  // generic phases: staging of the norm weights
     unsigned gen = 0;
@@ -561,6 +563,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
         if (stamp) { prof[p * MK_PROF_SLOTS] = globaltimer_ns(); prof[p * MK_PROF_SLOTS + 1] = 0; prof[p * MK_PROF_SLOTS + 4] = 0; prof[p * MK_PROF_SLOTS + 5] = 0; }
         MK_SYNC();                           // descriptor p is in shared memory (stored one phase ago)
         const MkPhase& s_ph = s_phs[p & 1];
+        if (p == 0 && s_ph.type == MK_ATTN) at_pre = at_ask(s_ph, (float*)work, dyn, abar0, R.at_ch);
         static_assert(sizeof(MkPhase) / 4 <= MK_THREADS, "descriptor does not fit one word per thread");
         int desc_w = 0;
         if (p + 1 < n_phases && threadIdx.x < sizeof(MkPhase) / 4) desc_w = ((const int*)(phases + p + 1))[threadIdx.x];
@@ -583,8 +586,9 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
             else phase_matvec_ring<CC_Q4_0>(s_ph, work, exp_lut, RC, comm, xseq, st1);
             break;
         case MK_ATTN:
-            if (s_ph.at.kv_f16) phase_attn<true>(s_ph, (float*)work, s_red, dyn, exp_lut, abar0, apar, R.at_ch);
-            else phase_attn<false>(s_ph, (float*)work, s_red, dyn, exp_lut, abar0, apar, R.at_ch);
+            if (s_ph.at.kv_f16) phase_attn<true>(s_ph, (float*)work, s_red, at_pre, exp_lut, abar0, apar, R.at_ch);
+            else phase_attn<false>(s_ph, (float*)work, s_red, at_pre, exp_lut, abar0, apar, R.at_ch);
+            at_pre.jobs = 0;
             break;
         case MK_ROWS: phase_rows(s_ph, dyn); break;
         case MK_REDUCE: phase_reduce(s_ph, comm, xseq, false); break;
@@ -597,6 +601,14 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
         const bool xg = s_ph.xgpu != 0;
         if ((flags & MK_F_TESTSTALL) && p == 2 && blockIdx.x == gridDim.x - 1) { if (threadIdx.x == 0) s_abort = 1; break; }     // test hook: this CTA deserts
         if (more) grid_barrier_arrive(bar, gridDim.x, gen, xg, (flags & MK_F_SYSFENCE) != 0);
+        if (more) {
+            const MkPhase& nx = s_phs[(p + 1) & 1];
+            if (nx.type == MK_ATTN) at_pre = at_ask(nx, (float*)work, dyn, abar0, R.at_ch);
+            // the norm weights of the next prologue were last read a token ago and come from HBM: a line of them per CTA into
+            // L2 now (0.8 % of a 7B token).  Its quotients stay divisions: without their branches (CcDivBy) the k = 11008 phases took 1 us longer
+            else if (nx.type == MK_MATVEC && nx.norm_w && threadIdx.x < 8)
+                for (int i = ((int)blockIdx.x * 8 + (int)threadIdx.x) * 32; i < nx.mv.k; i += (int)gridDim.x * 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx.norm_w + i));
+        }
         if (stamp) prof[p * MK_PROF_SLOTS + 3] = globaltimer_ns();
         if (more) {
             grid_barrier_wait(bar, gridDim.x, gen, comm, xg ? xseq + 1u : 0u, (flags & MK_F_POLLCNT) != 0, &s_abort, err_host);
@@ -610,6 +622,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
     // the CTA's shared memory goes away
     MK_SYNC();
     if (s_abort && threadIdx.x == 0) {
+        at_drain(at_pre.jobs, abar0, apar);
         while (*(volatile int*)&s_prod_done < MR_PRODUCER_WARPS) {}
         for (unsigned sl = 0; sl < (unsigned)R.nslots; sl++) {               // every slot's latest tenant has landed
             const unsigned q = *(volatile unsigned*)&s_seq[sl];

@@ -114,7 +114,8 @@ void cc_lazy_destroy(cc_device* dev) {
 }
 
 static int cc_lazy_flush_part(cc_device* dev, bool whole);
-#define LZ_HEAD_OPS 64                               // two or three layers: enough work for the GPU until the rest is recorded and fused
+#define LZ_HEAD_OPS 64                               // three layers: work for the GPU until the rest of a 7B token is recorded and fused.  16 tokens with 12 / 22 / 40 / 64 ops,
+                                                     // ms: 7B 41.2 / 40.6 / 40.5 / 39.8 (42.0 in one part), 15M 5.46 / 5.24 / 5.03 / 5.13 (5.93)
 static int64_t view_rows(const cc_view* v) { return v->ndim < 2 ? 1 : v->shape[0]; }
 
 // ---- recording ---------------------------------------------------------------------------------------------------
@@ -123,9 +124,9 @@ static void hold(LazyState* lz, cc_buf* b) { if (b) { cc_tensor_retain(b); lz->q
 int cc_lazy_record(cc_device* dev, int kind, const cc_view* a, const cc_view* b, cc_buf* out, float f, int64_t i0, int64_t i1, int64_t i2,
                    const int64_t* rows, int n_rows) {
     LazyState* lz = dev->lz;
-    // a long token starts while the rest of it is still being recorded: at the first layer boundary (a layer opens with the copy of its input) behind
-    // LZ_HEAD_OPS ops the queue so far runs, once per token -- the GPU used to wait some 180 us for the 840 ops of a 7B token.  What a fused pattern
-    // spans never crosses a layer's opening, so the phases are the same ones in two kernels
+    // a long token starts while the rest of it is still being recorded: at the first copy of a layer's input (attention's or the feed-forward's) behind
+    // LZ_HEAD_OPS ops the queue so far runs, once per token -- the GPU used to wait some 180 us for the 840 ops of a 7B token.  No fused
+    // pattern spans that copy, so the phases are the same ones in two kernels.  Ranks that exchange keep one part: their launches stay paired
     if (kind == L_DUP && !lz->head_done && lz->q.size() >= LZ_HEAD_OPS && !cc_comm_dev(dev) && a && a->ndim <= 2 && view_rows(a) == 1) {
         lz->head_done = true;
         int rc = cc_lazy_flush_part(dev, false);

@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(MV_THREADS) matvec_kernel(WPlanes W, const voi
 
 // a few activation rows (2 .. 31: several sequences' next tokens): the grid above fetches and unpacks the weights once per row.  Here a warp takes two weight
 // rows and NB activations at a time (vecdot.cuh rows_dot); a CTA stages its NB activations once and walks over the weight rows.
-// Q4_K, 11008 x 4096, 8 rows: 58 -> 35 us for 25 MB of weights (3.9 us at the copy rate); bound by the integer dot products and the
+// Q4_K, 11008 x 4096, 8 rows: 58 -> 37 us (whole call 77 -> 48) for 25 MB of weights (3.9 us at the copy rate); bound by the integer dot products and the
 // activation reads from shared memory (a 16-byte weight chunk meets 2 x NB 16-byte activation chunks)
 template <class T, int NB>
 __global__ void __launch_bounds__(MV_THREADS) matvec_few_kernel(WPlanes W, const void* act, int64_t n_total, float* __restrict__ out, int m, int k, int b) {

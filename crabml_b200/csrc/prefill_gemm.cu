@@ -9,7 +9,7 @@
 //      quantised value q * d is what enters the GEMM, so the only deviation from the reference is the f16 rounding of the two
 //      operands (relative 2^-11 each) and the f32 accumulation order
 //   3. umma_gemm_kernel     : TMA (cp.async.bulk.tensor.2d, 128-byte swizzle) stages [128 x 64] / [N x 64] f16 tiles into a
-//      4-deep shared-memory ring; ONE elected thread issues tcgen05.mma.cta_group::1.kind::f16 (M = 128, N = 64..256, K = 16)
+//      shared-memory ring (pg_stages); ONE elected thread issues tcgen05.mma.cta_group::1.kind::f16 (M = 128, N = 64..256, K = 16)
 //      with the f32 accumulator in TMEM; tcgen05.commit hands smem slots back to the TMA producer and the finished
 //      accumulator to four epilogue warps, which read it with tcgen05.ld and store C[b][m] (m contiguous across lanes).
 //      Warp roles: 0 TMA producer, 1 MMA issuer, 2 TMEM allocator, 4-7 epilogue.

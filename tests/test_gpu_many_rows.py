@@ -242,3 +242,32 @@ def test_prompt_recorded_and_eager_agree(arch, wtype, tokens):
     assert np.isfinite(got[0]).all()
     for g in got[1:]:
         np.testing.assert_array_equal(g.view(np.uint32), got[0].view(np.uint32))
+
+
+@pytest.mark.parametrize("wt,ct", [(oc.Q8_0, oc.Q8_0), (oc.Q4_K, oc.Q6_K)])
+@pytest.mark.parametrize("f16_kv", [False, True])
+def test_long_tokens_run_in_two_parts_with_the_same_bits(wt, ct, f16_kv):
+    """Six layers are recorded as more than one part; the cache's length crosses the 512 positions up to which the persistent kernels' attention keeps an
+    exponential per thread.  Every mode reduces in the same order, so the logits are the eager calls' bit for bit."""
+    from crabml_b200 import runner as R
+    conf = R.LlamaConfig(4, 2, 6, 256, 512, 600, 512, 1e-5, 64)
+    prompt = [1 + (7 * i) % 500 for i in range(506)]
+    res = {}
+    for lazy in (0, 1, 2):
+        dev = make_device(lazy=lazy)
+        try:
+            r = R.LlamaRunner(dev, conf, R.synthetic_weights(dev, conf, wt, ct, seed=3), 600, f16_kv=f16_kv)
+            first = [r.forward([t], p).copy() for p, t in enumerate([5, 6, 7])]
+            r.forward(prompt, 3)
+            before = dev.lazy_stats() if lazy else None
+            late = [r.forward([t], 3 + len(prompt) + p).copy() for p, t in enumerate(range(11, 19))]
+            res[lazy] = np.stack(first + late)
+            if lazy:
+                st = dev.lazy_stats()
+                assert st["uncached"] == before["uncached"] and st["graph_replays"] - before["graph_replays"] >= 4, (before, st)
+            r.close()
+        finally:
+            dev.close()
+    assert np.isfinite(res[0]).all() and np.abs(res[0]).max() > 0
+    for mode in (1, 2):
+        np.testing.assert_array_equal(res[mode].view(np.uint32), res[0].view(np.uint32), err_msg=f"lazy={mode} vs eager")

@@ -404,11 +404,12 @@ def run_b200(args, rank, world, local_rank):
         streams = 1 if sharded or world == 1 else world       # sharded: ONE token stream over N GPUs; replicas: N streams
         value = streams * K / (val_ms * 1e-3)
         e2e = streams * K / (e2e_ms * 1e-3)
-        if lazy == 2 and launches_val == K:
-            # the dominant kernel IS the step: one mega_kernel launch per token streams every weight byte of this rank once
+        mega = lazy == 2 and launches_val <= 2 * K and dev.mega_variant() != 0      # a token is one launch, or two when it starts while the rest is recorded
+        if mega:
+            # the dominant kernel IS the step: its one or two launches per token stream every weight byte of this rank once
             mega_gbs = bytes_per_token / (val_ms / K * 1e-3) / 1e9
             mk_name, mk_file = MEGA_NAMES.get(dev.mega_variant(), MEGA_NAMES[1])
-            roofline = {"bound": "hbm", "kernel": f"{mk_name} ({mk_file}): one persistent launch per decoded token, all matvec/attention/norm phases",
+            roofline = {"bound": "hbm", "kernel": f"{mk_name} ({mk_file}): {launches_val // K} persistent launch(es) per decoded token, all matvec/attention/norm phases",
                         "achieved": mega_gbs, "peak": peaks["hbm_gbs"], "peak_source": peak_src, "unit": "GB/s", "frac": mega_gbs / peaks["hbm_gbs"],
                         "traffic": TRAFFIC.get((args.workload, world)), "traffic_source": "profiles/ (ncu --set full, dram__bytes_read.sum + dram__bytes_write.sum per launch)" if TRAFFIC.get((args.workload, world)) else None,
                         "algorithmic_bytes_per_launch": bytes_per_token, "us_per_launch": val_ms / K * 1e3, "frac_of_8TBs_nominal": mega_gbs / 8000.0}
@@ -422,7 +423,7 @@ def run_b200(args, rank, world, local_rank):
             "ms_per_step": val_ms / K, "higher_is_better": True, "scaling": "strong" if sharded else "weak", "vs_baseline": None, "dtype": "int8",
             "data": "synthetic",
             "config": {"workload": f"{args.workload}-decode-synthetic", "weights": wt_name, "classifier": ct_name, "kv_cache": "f32",
-                       "start_pos": args.start_pos, "kv_positions": [int(p0), int(p0 + K)], "mode": "lazy: plan not megakernel-eligible (matvec types outside Q8_0/Q4_0 use the warp-per-row kernels): fused kernels, CUDA-graph replay" if (lazy == 2 and launches_val != K) else {0: "eager (one launch per trait call)", 1: "lazy: fused kernels, CUDA-graph replay", 2: "lazy: one persistent megakernel per token, CUDA-graph replay"}[args.lazy],
+                       "start_pos": args.start_pos, "kv_positions": [int(p0), int(p0 + K)], "mode": "lazy: plan not megakernel-eligible (matvec types outside Q8_0/Q4_0 use the warp-per-row kernels): fused kernels, CUDA-graph replay" if (lazy == 2 and not mega) else {0: "eager (one launch per trait call)", 1: "lazy: fused kernels, CUDA-graph replay", 2: f"lazy: persistent megakernel, {launches_val // K} launch(es) per token, CUDA-graph replay"}[args.lazy],
                        "multi_gpu": ("single GPU" if world == 1 else
                                      f"one token stream sharded over {world} GPUs: rows of wq/wk/wv/gate/up/classifier, block columns of wo/down; "
                                      f"exchange = {'one-shot NVLink peer stores fused into the megakernel' if transport == 'p2p' and lazy == 2 else 'one-shot NVLink peer-store kernel' if transport == 'p2p' else 'ncclAllReduce/ncclAllGather'} "

@@ -26,7 +26,7 @@ extern "C" CC_API int cc_tensor_dup(cc_device* dev, const cc_view* src, cc_buf**
     return CC_OK;
 }
 
-#define CC_EXPORT_STAGED ((size_t)1 << 20)
+#define CC_EXPORT_STAGED ((size_t)256 << 10)
 extern "C" CC_API int cc_tensor_export_f32(cc_device* dev, const cc_view* src, float* dst, size_t n) {   // cpu_tensor.rs:339-349
     CHECK_VIEW(dev, src, "export");
     if (!dst) return cc_fail(dev, CC_ERR_ARG, "export: dst is NULL");
@@ -35,11 +35,18 @@ extern "C" CC_API int cc_tensor_export_f32(cc_device* dev, const cc_view* src, f
     FLUSH(dev);
     int64_t len = view_len(src);
     size_t cnt = n < (size_t)len ? n : (size_t)len;
-    // a row of logits goes through the device's pinned buffer: the driver's way into pageable memory takes some 20 us longer than the copy itself
-    const bool staged = cnt && cnt * 4 <= CC_EXPORT_STAGED && cc_ensure_pinned(dev, cnt * 4) == CC_OK;
-    if (cnt) CC_CUDA(dev, cudaMemcpyAsync(staged ? dev->pinned : dst, src->buf->plane[0], cnt * 4, cudaMemcpyDeviceToHost, dev->stream));
+    // a row of logits goes through a pinned buffer: the driver's way into pageable memory takes some 20 us longer than the copy itself
+    if (cnt && cnt * 4 <= CC_EXPORT_STAGED) {
+        std::lock_guard<std::mutex> g(dev->export_mu);                 // as before, threads may export at the same time
+        const bool staged = dev->export_host || cudaMallocHost(&dev->export_host, CC_EXPORT_STAGED) == cudaSuccess;
+        if (!staged) { cudaGetLastError(); dev->export_host = nullptr; }
+        CC_CUDA(dev, cudaMemcpyAsync(staged ? dev->export_host : dst, src->buf->plane[0], cnt * 4, cudaMemcpyDeviceToHost, dev->stream));
+        CC_CUDA(dev, cudaStreamSynchronize(dev->stream));
+        if (staged) memcpy(dst, dev->export_host, cnt * 4);
+        return cc_check_async_error(dev);
+    }
+    if (cnt) CC_CUDA(dev, cudaMemcpyAsync(dst, src->buf->plane[0], cnt * 4, cudaMemcpyDeviceToHost, dev->stream));
     CC_CUDA(dev, cudaStreamSynchronize(dev->stream));
-    if (staged) memcpy(dst, dev->pinned, cnt * 4);
     return cc_check_async_error(dev);
 }
 

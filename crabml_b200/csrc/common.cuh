@@ -119,6 +119,7 @@ struct cc_device {
 
     // pinned staging for export / row indices
     void* pinned = nullptr;
+    std::mutex export_mu; void* export_host = nullptr;        // small results on their way to pageable memory (capi.cu), one export at a time
     size_t pinned_bytes = 0;
     void* dev_idx = nullptr;      // device copy of row indices
     size_t dev_idx_bytes = 0;

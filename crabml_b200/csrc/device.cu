@@ -118,6 +118,7 @@ extern "C" CC_API void cc_device_destroy(cc_device* dev) {
         for (uintptr_t p : kv.second) cudaFree((void*)p);
     if (dev->act_scratch) cudaFree(dev->act_scratch);
     if (dev->pinned) cudaFreeHost(dev->pinned);
+    if (dev->export_host) cudaFreeHost(dev->export_host);
     for (int i = 0; i < 2; i++) { if (dev->up_pinned[i]) cudaFreeHost(dev->up_pinned[i]); if (dev->up_ev[i]) cudaEventDestroy(dev->up_ev[i]); }
     for (int i = 0; i < 2; i++) { if (dev->rope_pinned[i]) cudaFreeHost(dev->rope_pinned[i]); if (dev->rope_ev[i]) cudaEventDestroy(dev->rope_ev[i]); }
     if (dev->err_host) cudaFreeHost(dev->err_host);

@@ -1,5 +1,6 @@
 """Profiling driver: the four Llama-2-7B matvec shapes, cycling over enough distinct matrices to defeat L2.
-Usage (under gpurun):  ncu --set full -k regex:matvec_kernel -s 8 -c 4 -o gpurun_out/mv python tools/prof_matvec.py Q8_0 11008 4096"""
+Usage, once `python tools/prof_matvec.py Q8_0 11008 4096` has run by itself:
+  ncu --section SpeedOfLight --section MemoryWorkloadAnalysis --clock-control none -k regex:matvec_kernel -s 1 -c 1 -o prof python tools/prof_matvec.py Q8_0 11008 4096"""
 import sys
 
 import numpy as np

@@ -1,5 +1,6 @@
 """Profiling driver of the dense (prefill) matmul_vec: one weight matrix against a (b, k) activation, a few repetitions.
-Usage (under gpurun):  ncu --set full -k regex:umma_gemm -s 1 -c 1 -o gpurun_out/gemm python tools/prof_prefill.py Q8_0 4096 4096 4096"""
+Usage, once `python tools/prof_prefill.py Q8_0 4096 4096 4096` has run by itself:
+  ncu --section SpeedOfLight --section MemoryWorkloadAnalysis --clock-control none -k regex:umma_gemm -s 1 -c 1 -o prof python tools/prof_prefill.py Q8_0 4096 4096 4096"""
 import sys
 
 import numpy as np

@@ -2,7 +2,6 @@
 // Compiled with -fmad=false / IEEE div+sqrt so that every op reproduces the reference's f32
 // arithmetic; only reduction ORDER differs (the canonical 512-thread tree of common.cuh instead of sequential).
 #include "common.cuh"
-#include "split_gemm.cuh"
 
 // ---- rms_norm_inplace: primitives/rms_norm.rs:32-47  x /= sqrt(sum(x^2)/n + eps), no weight ------------
 // canonical 512-thread order (common.cuh); cols % 4 == 0 is implied by the reference's own assert (cols % 32 == 0)
@@ -265,96 +264,199 @@ __global__ void bmm_ncontig_kernel(const float* __restrict__ a, const void* __re
         c[o] = acc;
     }
 }
-// (c) many rows (a prompt): tiles of 128 x 128 on the tensor cores, 32-bit operands and sums (split_gemm.cuh).  F16 B: A is rounded to f16 first, the
-//     products are exact and the sums 32-bit, as in (a).  The f16 SUMS of (b) with F16 B have an order of their own and stay there.
-// Tiles: columns (fastest), rows, batch.  A warp per output reads 1 KB for 128 products: 32 heads x 512 x 512 x 128 took 1963 us, and 45 us here
-template <bool B_F16, bool N_CONTIG>
-struct BmmTile {
-    static constexpr int HALVES = 2, N = 128;
-    static constexpr bool A_TRANSPOSED = false, B_TRANSPOSED = N_CONTIG, SHARED = false, A_TMA = false, B_TMA = false, SKIP_ZERO = false;
-    struct Tile { int steps, m0, n0; const float* a; const void* b; float* c; };
-    struct Fixed {};
-    struct Shared {};
-    typedef const float* ARow;
-    typedef const void* BCol;
-    const float* a;
-    const void* b;
-    float* c;
-    int ab, bb, m, k, n, a_vec, b_vec;
-    int64_t sb0, sb1, sb2;
-    __device__ bool tile(int i, int, Tile& t) const {
-        const int nt = (n + N - 1) / N, mt = (m + 127) >> 7, rest = (unsigned)i / (unsigned)nt, bi = (unsigned)rest / (unsigned)mt;
-        t.n0 = (i - rest * nt) * N; t.m0 = (rest - bi * mt) * 128; t.steps = (k + 63) >> 6;
-        t.a = a + (int64_t)bi * m * k; t.c = c + (int64_t)bi * m * n;
-        if (B_F16) t.b = (const __half*)b + (int64_t)(bi / (ab / bb)) * sb0;
-        else t.b = (const float*)b + (int64_t)(bi % bb) * sb0;
-        return true;
-    }
-    __device__ Fixed fixed(int) const { return Fixed{}; }
-    __device__ void setup(const Tile&, Shared&) const {}
-    __device__ const void* map_a() const { return nullptr; }
-    __device__ const void* map_b() const { return nullptr; }
-    __device__ void at_a(const Tile&, int, int, int&, int&) const {}
-    __device__ void at_b(const Tile&, int, int, int&, int&) const {}
-    __device__ ARow a_row(const Tile& t, const Shared&, Fixed, int r) const { return t.m0 + r < m ? t.a + (int64_t)(t.m0 + r) * k : nullptr; }
-    __device__ void load_a(const Tile&, ARow p, int s, int ch, float (&v)[8]) const { if (p) sg_load8(p, s * 64 + ch * 8, k, a_vec, v); else sg_zero8(v); }
-    __device__ void prep_a(const Tile&, ARow&, float (&v)[8]) const {
-        if (!B_F16) return;
+// two 32-bit numbers an instruction, each rounded as by itself.  nz: two times -0, which changes no product, as a value that the assembler does not know: it makes one
+// instruction with one rounding of a mul.rn.f32x2 (or an fma with a constant) and the addition behind it
+__device__ __forceinline__ uint64_t two(float a, float b) { uint64_t v; asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); return v; }
+__device__ __forceinline__ float2 apart(uint64_t v) { float2 x; asm("mov.b64 {%0, %1}, %2;" : "=f"(x.x), "=f"(x.y) : "l"(v)); return x; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b, uint64_t nz) { uint64_t v; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(nz)); return v; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t v; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b)); return v; }
+// (c) many rows: the sums of (a), bit for bit.  A thread makes 4 x 4 outputs of a 64 x 64 tile whose operands lie in shared memory for the whole depth (up to
+//     BK_DEPTH), so that it can take the 32 lanes' partial sums in the order in which the butterfly adds them -- lanes 0, 16, 8, 24, 4, .. -- and keep one
+//     unfinished sum per level of its tree.  Column k of 64 rows lies in 16 groups of 4, group g at place g ^ (k / 4): rows arrive along k and are read across.
+//     32 heads x 512 x 512 x 128, 1.1 G terms of two roundings (60 us at one a lane and cycle): 108 us ; a warp per output reads 1 KB for 128 terms: 1945 us
+#define BK_TILE 64
+#define BK_DEPTH 384
+__device__ __forceinline__ int bk_at(int k, int group) { return k * BK_TILE + ((group ^ ((k >> 2) & 15)) << 2); }
+template <bool B_F16>
+__global__ void __launch_bounds__(256, 2) bmm_kcontig_tile_kernel(const float* __restrict__ a, const void* __restrict__ b, float* __restrict__ c, int ab, int bb, int m, int k, int n,
+                                                                  int64_t sb0, int64_t sb2, int n_tiles, int m_tiles, int a_vec, int b_vec, uint64_t nz) {
+    pdl_enter();
+    extern __shared__ __align__(16) float bk_sm[];           // [depth][64] of A, [depth][64] of B
+    float *sa = bk_sm, *sb = bk_sm + ((k + 3) & ~3) * BK_TILE;
+    const int rest = blockIdx.x / (unsigned)n_tiles, bi = rest / m_tiles, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int m0 = (rest - bi * m_tiles) * BK_TILE, n0 = ((int)blockIdx.x - rest * n_tiles) * BK_TILE;
+    const float* pa = a + ((int64_t)bi * m + m0) * k;
+    const float* pf = (const float*)b + (int64_t)(bi % bb) * sb0 + n0 * sb2;
+    const __half* ph = (const __half*)b + (int64_t)(bi / (ab / bb)) * sb0 + n0 * sb2;
+    // a warp moves 4 rows x 32 of the depth at a time, rows outside as zeros ; the four runs of rows it has go together
+    for (int k0 = (lane >> 2) * 4; k0 < k; k0 += 32) {
+        float v[4][4];
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = __half2float(__float2half_rn(v[i]));
-    }
-    __device__ BCol b_col(const Tile& t, int col) const {
-        if (t.n0 + col >= n) return nullptr;
-        if (N_CONTIG) return (const float*)t.b + t.n0 + col;
-        if (B_F16) return (const __half*)t.b + (int64_t)(t.n0 + col) * sb2;
-        return (const float*)t.b + (int64_t)(t.n0 + col) * sb2;
-    }
-    __device__ void load_b(const Tile&, BCol p, int s, int ch, float (&v)[8]) const {
-        const int k0 = s * 64 + ch * 8;
-        if (!p) { sg_zero8(v); return; }
-        if (N_CONTIG) {
-            const float* at = (const float*)p + (int64_t)k0 * sb1;
+        for (int u = 0; u < 4; u++) {
+            const int r = (warp + (u & 1) * 8) * 4 + (lane & 3);
+            const bool left = u < 2, on = left ? m0 + r < m : n0 + r < n;
+            if (on && (left || !B_F16)) {
+                const float* p = left ? pa + (int64_t)r * k + k0 : pf + r * sb2 + k0;
+                if (left ? a_vec : b_vec) { const float4 x = *(const float4*)p; v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w; }
+                else {
 #pragma unroll
-            for (int i = 0; i < 8; i++) { v[i] = k0 + i < k ? *at : 0.0f; at += sb1; }
-        } else if (B_F16) {
-            const __half* at = (const __half*)p + k0;
-            if (b_vec && k0 + 8 <= k) {
-                const uint4 h = *(const uint4*)at;
-                const unsigned u[4] = {h.x, h.y, h.z, h.w};
-#pragma unroll
-                for (int i = 0; i < 4; i++) { v[2 * i] = h2f_bits((uint16_t)(u[i] & 0xffffu)); v[2 * i + 1] = h2f_bits((uint16_t)(u[i] >> 16)); }
+                    for (int i = 0; i < 4; i++) v[u][i] = k0 + i < k ? p[i] : 0.0f;
+                }
             } else {
 #pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = k0 + i < k ? __half2float(at[i]) : 0.0f;
+                for (int i = 0; i < 4; i++) v[u][i] = on && k0 + i < k ? __half2float(ph[r * sb2 + k0 + i]) : 0.0f;
             }
-        } else sg_load8((const float*)p, k0, k, b_vec, v);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            float* to = (u < 2 ? sa : sb) + bk_at(k0, warp + (u & 1) * 8) + (lane & 3);
+#pragma unroll
+            for (int i = 0; i < 4; i++) to[i * BK_TILE] = B_F16 && u < 2 ? __half2float(__float2half_rn(v[u][i])) : v[u][i];
+        }
     }
-    __device__ void end_a(const Tile&, Shared&, ARow&, int, int) const {}
-    __device__ void give(const Shared&, Shared&, int) const {}
-    template <int COUNT>
-    __device__ void emit(const Tile& t, const Shared&, Fixed, int r, int col0, float (&v)[COUNT], float* buf) const {
-        sg_store_rows<COUNT, false>(buf, t.m0 + r < m ? t.c + (int64_t)(t.m0 + r) * n + t.n0 + col0 : nullptr, n - t.n0 - col0, n % 4 == 0, v);
+    __syncthreads();
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15, row0 = m0 + ty * 4, col0 = n0 + tx * 4;
+    if (m0 + (warp * 2) * 4 >= m) return;                    // none of the warp's rows
+    uint64_t tree[5][8], sum[8];                             // [2 j + i]: rows 2 i and 2 i + 1 of column j
+#pragma unroll
+    for (int t = 0; t < 32; t++) {
+        const int l = (t & 1) << 4 | (t & 2) << 2 | (t & 4) | (t & 8) >> 2 | (t & 16) >> 4;
+#pragma unroll
+        for (int i = 0; i < 8; i++) sum[i] = 0;
+        // places of two steps of 32 differ in one bit of the group
+        const float *a0 = sa + bk_at(l, ty), *a1 = sa + bk_at(l + 32, ty), *b0 = sb + bk_at(l, tx), *b1 = sb + bk_at(l + 32, tx);
+        for (int ki = l; ki < k; ki += 64) {
+            const ulonglong2 x = *(const ulonglong2*)a0;
+            const float4 y = *(const float4*)b0;
+            const uint64_t xr[2] = {x.x, x.y}, yr[4] = {two(y.x, y.x), two(y.y, y.y), two(y.z, y.z), two(y.w, y.w)};
+#pragma unroll
+            for (int i = 0; i < 8; i++) sum[i] = add2(sum[i], mul2(xr[i & 1], yr[i >> 1], nz));
+            if (ki + 32 < k) {
+                const ulonglong2 x1 = *(const ulonglong2*)a1;
+                const float4 y1 = *(const float4*)b1;
+                const uint64_t xs[2] = {x1.x, x1.y}, ys[4] = {two(y1.x, y1.x), two(y1.y, y1.y), two(y1.z, y1.z), two(y1.w, y1.w)};
+#pragma unroll
+                for (int i = 0; i < 8; i++) sum[i] = add2(sum[i], mul2(xs[i & 1], ys[i >> 1], nz));
+            }
+            a0 += 64 * BK_TILE; a1 += 64 * BK_TILE; b0 += 64 * BK_TILE; b1 += 64 * BK_TILE;
+        }
+        int level = 0;
+#pragma unroll
+        for (; level < 5 && ((t >> level) & 1); level++)
+#pragma unroll
+            for (int i = 0; i < 8; i++) sum[i] = add2(tree[level][i], sum[i]);
+        if (level < 5) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) tree[level][i] = sum[i];
+        }
     }
-};
-template <bool B_F16, bool N_CONTIG>
-static int launch_bmm_tiles(cc_device* dev, const float* a, const void* b, float* c, int64_t ab, int64_t bb, int64_t m, int64_t k, int64_t n, int64_t sb0, int64_t sb1, int64_t sb2) {
-    BmmTile<B_F16, N_CONTIG> p{};
-    p.a = a; p.b = b; p.c = c; p.ab = (int)ab; p.bb = (int)bb; p.m = (int)m; p.k = (int)k; p.n = (int)n; p.sb0 = sb0; p.sb1 = sb1; p.sb2 = sb2;
-    const int per = B_F16 ? 8 : 4;                            // elements of 16 bytes
-    p.a_vec = k % 4 == 0 && ((uintptr_t)a & 15) == 0;
-    p.b_vec = sb0 % per == 0 && sb2 % per == 0 && ((uintptr_t)b & 15) == 0;
-    return sg_launch(dev, p, ((n + 127) / 128) * ((m + 127) / 128) * ab);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        if (row0 + i >= m) break;
+        float* o = c + ((int64_t)bi * m + row0 + i) * n + col0;
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) { const float2 x = apart(sum[2 * j + (i >> 1)]); v[j] = i & 1 ? x.y : x.x; }
+        if (n % 4 == 0 && col0 < n) *(float4*)o = make_float4(v[0], v[1], v[2], v[3]);
+        else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) if (col0 + j < n) o[j] = v[j];
+        }
+    }
+}
+// (d) many rows of (b), F32 B: the same sum per output in one thread, ascending k; 32 x 64 tiles staged 16 deep in two buffers of shared memory, 4 x 4 outputs a
+//     thread.  The f16 SUMS of (b) with F16 B stay there.  32 heads x 512 x 128 over 512: 300 -> 79 us
+#define BN_ROWS 32
+#define BN_TILE 64
+#define BN_K 16
+__global__ void __launch_bounds__(128) bmm_ncontig_tile_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c, int bb, int m, int k, int n,
+                                                               int64_t sb0, int64_t sb1, int n_tiles, int m_tiles, int a_vec, int b_vec, uint64_t nz) {
+    pdl_enter();
+    __shared__ __align__(16) float sa[2][BN_K][BN_ROWS + 4], sb[2][BN_K][BN_TILE];
+    const int rest = blockIdx.x / (unsigned)n_tiles, bi = rest / m_tiles;
+    const int m0 = (rest - bi * m_tiles) * BN_ROWS, n0 = ((int)blockIdx.x - rest * n_tiles) * BN_TILE;
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    const int ar = threadIdx.x >> 2, ak = (threadIdx.x & 3) * 4, bk = threadIdx.x >> 3, bn = (threadIdx.x & 7) * 8;      // what a thread stages: 4 of a row of A, 8 of B's
+    const float* pa = m0 + ar < m ? a + ((int64_t)bi * m + m0 + ar) * k : nullptr;
+    const float* pb = b + (int64_t)(bi % bb) * sb0 + n0;
+    float va[4], vb[8];
+    uint64_t acc[2][4];                                      // [i][j]: rows 2 i and 2 i + 1 of column j
+    auto four = [](const float* p, int at, int end, bool vec, float* v) {      // p[at ..], zeros from `end` on: they add exact zeros
+        if (p && vec && at + 4 <= end) {
+            const float4 x = *(const float4*)(p + at);
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = p && at + i < end ? p[at + i] : 0.0f;
+        }
+    };
+    auto fetch = [&](int k0) {
+        const float* row = k0 + bk < k ? pb + (int64_t)(k0 + bk) * sb1 : nullptr;
+        four(pa, k0 + ak, k, a_vec, va);
+        four(row, bn, n - n0, b_vec, vb);
+        four(row, bn + 4, n - n0, b_vec, vb + 4);
+    };
+    auto put = [&](int s) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) sa[s][ak + i][ar] = va[i];
+        *(float4*)&sb[s][bk][bn] = make_float4(vb[0], vb[1], vb[2], vb[3]);
+        *(float4*)&sb[s][bk][bn + 4] = make_float4(vb[4], vb[5], vb[6], vb[7]);
+    };
+#pragma unroll
+    for (int i = 0; i < 8; i++) acc[i >> 2][i & 3] = 0;
+    fetch(0);
+    put(0);
+    for (int k0 = 0, s = 0; k0 < k; k0 += BN_K, s ^= 1) {
+        __syncthreads();                                                 // this step's operands are there, the last one's have been read
+        if (k0 + BN_K < k) fetch(k0 + BN_K);                             // the next step's travel while this one is multiplied
+        if (m0 + (int)(threadIdx.x >> 5) * 8 < m) {                      // (a warp has rows 8 w ..)
+#pragma unroll
+            for (int kk = 0; kk < BN_K; kk++) {
+                const ulonglong2 x = *(const ulonglong2*)&sa[s][kk][ty * 4];
+                const float4 y = *(const float4*)&sb[s][kk][tx * 4];
+                const uint64_t xr[2] = {x.x, x.y}, yr[4] = {two(y.x, y.x), two(y.y, y.y), two(y.z, y.z), two(y.w, y.w)};
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[i >> 2][i & 3] = add2(acc[i >> 2][i & 3], mul2(xr[i >> 2], yr[i & 3], nz));
+            }
+        }
+        if (k0 + BN_K < k) put(s ^ 1);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int row = m0 + ty * 4 + i;
+        if (row >= m) break;
+        float* o = c + ((int64_t)bi * m + row) * n + n0 + tx * 4;
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) { const float2 x = apart(acc[i >> 1][j]); v[j] = i & 1 ? x.y : x.x; }
+        if (n % 4 == 0 && n0 + tx * 4 < n) *(float4*)o = make_float4(v[0], v[1], v[2], v[3]);
+        else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) if (n0 + tx * 4 + j < n) o[j] = v[j];
+        }
+    }
 }
 int cc_launch_batch_matmul(cc_device* dev, const float* a, const void* b, int b_dtype, float* c, int64_t ab, int64_t bb,
                            int64_t m, int64_t k, int64_t n, int64_t sb0, int64_t sb1, int64_t sb2) {
     int64_t outs = ab * m * n;
     if (outs == 0) return CC_OK;
     bool f16 = b_dtype == CC_F16;
-    // one row per batch entry (decoding) keeps the order of the fused kernels; the reference's order stays in exact mode.  From 16 rows on a tile that
-    // is mostly padding is still faster than reading B once per row
-    if (!dev->exact && m >= 16 && k > 0 && ab < 65536 && m < ((int64_t)1 << 24) && n < ((int64_t)1 << 24) && k < ((int64_t)1 << 24) && (sb1 == 1 || !f16)) {
-        if (sb1 == 1) return f16 ? launch_bmm_tiles<true, false>(dev, a, b, c, ab, bb, m, k, n, sb0, sb1, sb2) : launch_bmm_tiles<false, false>(dev, a, b, c, ab, bb, m, k, n, sb0, sb1, sb2);
-        return launch_bmm_tiles<false, true>(dev, a, b, c, ab, bb, m, k, n, sb0, sb1, sb2);
+    // a tile's time does not depend on how many of its rows there are, (a) and (b) go row by row.  us for 1 / 2 / 4 / 8 rows of 32 heads, K = 128, 512 columns: (a) 11, 11,
+    // 19, 34 beside 11 in tiles, 2048 columns: 19, 34, 64, 125 beside 38 ; 512 terms, 128 columns: (b) 35 beside 24
+    const int64_t m_tiles = sb1 == 1 ? (m + BK_TILE - 1) / BK_TILE : (m + BN_ROWS - 1) / BN_ROWS, n_tiles = (n + 63) / 64;
+    if (m >= 4 && (sb1 == 1 ? k <= BK_DEPTH : !f16) && ab < (1 << 24) && m < (1 << 24) && n < (1 << 24) && k < (1 << 24) && m_tiles * n_tiles * ab < ((int64_t)1 << 31)) {
+        static_assert(BK_TILE == 64 && BN_TILE == 64, "one count of column tiles");
+        const unsigned tiles = (unsigned)(m_tiles * n_tiles * ab);
+        const int a_vec = k % 4 == 0 && ((uintptr_t)a & 15) == 0, b_vec = !f16 && ((uintptr_t)b & 15) == 0 && sb0 % 4 == 0 && (sb1 == 1 ? sb2 % 4 == 0 && k % 4 == 0 : sb1 % 4 == 0);
+        if (sb1 != 1) cc_launch_pdl(dev, bmm_ncontig_tile_kernel, tiles, 128, 0, a, (const float*)b, c, (int)bb, (int)m, (int)k, (int)n, sb0, sb1, (int)n_tiles, (int)m_tiles, a_vec, b_vec, (uint64_t)0x8000000080000000ull);
+        else {
+            const int smem = 2 * (int)((k + 3) & ~3) * BK_TILE * 4;
+            auto kernel = f16 ? bmm_kcontig_tile_kernel<true> : bmm_kcontig_tile_kernel<false>;
+            if (smem > 48 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            cc_launch_pdl(dev, kernel, tiles, 256, smem, a, b, c, (int)ab, (int)bb, (int)m, (int)k, (int)n, sb0, sb2, (int)n_tiles, (int)m_tiles, a_vec, b_vec, (uint64_t)0x8000000080000000ull);
+        }
+        CC_LAUNCH_CHECK(dev);
+        return CC_OK;
     }
     if (sb1 == 1) {
         unsigned grid = (unsigned)((outs * 32 + 255) / 256);

@@ -890,7 +890,7 @@ __global__ void __launch_bounds__(256) wa_cut_kernel(const float* __restrict__ q
 // tiles: key tiles of the band (fastest), query tiles, G
 struct WaScores {
     static constexpr int HALVES = 2, N = 128;
-    static constexpr bool A_TRANSPOSED = false, B_TRANSPOSED = false, SHARED = false, A_TMA = true, B_TMA = true, SKIP_ZERO = false;
+    static constexpr bool SHARED = false, A_TMA = true, SKIP_ZERO = false;
     typedef WaTile Tile;
     typedef WaFixed Fixed;
     struct Shared {};
@@ -964,7 +964,7 @@ struct WaScores {
 template <int TILE_HALVES>
 struct WaValues {
     static constexpr int HALVES = TILE_HALVES, N = 64 * HALVES;
-    static constexpr bool A_TRANSPOSED = true, B_TRANSPOSED = true, SHARED = true, A_TMA = false, B_TMA = true, SKIP_ZERO = true;
+    static constexpr bool SHARED = true, A_TMA = false, SKIP_ZERO = true;
     typedef WaTile Tile;
     typedef WaFixed Fixed;
     CUtensorMap maps[1];                                // values [3][G][dvp][span]
@@ -1057,7 +1057,7 @@ struct WaValues {
 #pragma unroll
         for (int c = 0; c < COUNT; c++) v[c] *= inv;
         const int64_t row = wa_row(g, t, f);
-        sg_store_rows<COUNT, false>(buf, row < 0 ? nullptr : o + row * g.dv + t.c0 + col0, g.dv - t.c0 - col0, g.dv % 4 == 0, v);
+        sg_store_rows<COUNT>(buf, row < 0 ? nullptr : o + row * g.dv + t.c0 + col0, g.dv - t.c0 - col0, g.dv % 4 == 0, v);
     }
 };
 // few rows (decoding): grid (ceil(keys / 16), T, G * head blocks), 256 threads.  The CTA stages up to WS_HEADS queries of (token, key/value head); a

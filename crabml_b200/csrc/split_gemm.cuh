@@ -11,8 +11,8 @@
 // four instructions make the six products: A_h x B_h, A_h x [B_m B_l], A_m x [B_h B_m], A_l x B_h.  One instruction per product reads the planes of A
 // from shared memory more often; at N = 64 it took 85 cycles for 32 cycles of arithmetic.
 //
-// Operands arrive in one of two ways.  TMA: a kernel before this one has cut them into planes in global memory (what many tiles read), three boxes of
-// 64 columns per step.  Otherwise warps 0-15 load 32-bit numbers, cut and store them (128-byte swizzle, K-major) while they are staged.  Cutting costs
+// B, and A where A_TMA says so, arrive by TMA: a kernel before this one has cut them into planes in global memory (what many tiles read), three boxes of
+// 64 columns per step.  Otherwise warps 0-15 load A as 32-bit numbers, cut and store them (128-byte swizzle, K-major) while they are staged.  Cutting costs
 // about six instructions per element and a trip through registers: with both operands cut in the kernel, a step of 128 x 128 x 64 took 5400 cycles.
 //
 // One CTA per SM: warps 0-15 stage and collect, warp 16 issues the products (issuing blocks while the tensor core is busy), warp 17 the TMA loads.  Step
@@ -30,10 +30,9 @@
 //   Fixed, fixed(r)                what does not change from tile to tile about row r
 //   SHARED, Shared                 void setup(Tile, Shared&) is called by all threads before a tile, which then waits for the one before
 //   ARow, BCol                     what a thread keeps of a row / a column
-//   A_TMA, B_TMA, map_a, at_a, ..  the operand comes by TMA: its tensor map and the coordinates of a step's box of a plane
-//   a_row, load_a, prep_a          otherwise, and for sums that are computed again: a row of A; 8 consecutive elements of it as they lie in memory; the
-//   b_col, load_b                  operand they stand for; the same for B
-//   A_TRANSPOSED, B_TRANSPOSED     consecutive threads take consecutive rows (columns) instead of consecutive elements
+//   map_b, at_b (A_TMA: map_a ..)  the tensor map and the coordinates of a step's box of a plane
+//   a_row, load_a, prep_a          where A is cut here, and for sums that are computed again: a row of A; 8 consecutive elements of it as they lie in memory;
+//   b_col, load_b                  the operand they stand for; a column of B and 8 consecutive elements of it
 //   SKIP_ZERO                      in sums that are computed again, a zero of A leaves its term out (weights of masked keys)
 //   end_a                          SHARED: after the last step, with the thread's row state
 //   emit                           the epilogue: 16 * HALVES consecutive sums of a row (sg_store_rows below: as they are, into rows of memory)
@@ -111,16 +110,12 @@ __device__ __forceinline__ void sg_tmem16(unsigned addr, unsigned (&v)[16]) {
 // a warp's 32 rows x COUNT columns into rows of memory.  out: the row's first number (NULL: no such row); columns from `cols` on are dropped.  vec (rows start
 // at multiples of 16 bytes): a thread stores its own row 16 bytes at a time -- eight stores and nothing else, where the way through shared memory, for rows
 // that start anywhere, is a chain of some 500 instructions in two warps per scheduler (5000 cycles)
-template <int COUNT, bool ADD>
+template <int COUNT>
 __device__ __forceinline__ void sg_store_rows(float* buf, float* out, int cols, bool vec, const float (&v)[COUNT]) {
     if (vec) {
 #pragma unroll
         for (int c = 0; c < COUNT; c += 4)
-            if (out && c < cols) {
-                float4 x = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
-                if (ADD) { const float4 y = *(const float4*)(out + c); x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w; }
-                *(float4*)(out + c) = x;
-            }
+            if (out && c < cols) *(float4*)(out + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
         return;
     }
     const int lane = threadIdx.x & 31;
@@ -135,7 +130,7 @@ __device__ __forceinline__ void sg_store_rows(float* buf, float* out, int cols, 
         for (int r = lane / SG_PIECE; r < 32; r += 32 / SG_PIECE) {
             float* o = (float*)__shfl_sync(0xffffffffu, at, r);
             const float x = buf[r * (SG_PIECE + 1) + lane % SG_PIECE];
-            if (o && c < cols) o[c] = ADD ? o[c] + x : x;
+            if (o && c < cols) o[c] = x;
         }
         __syncwarp();
     }
@@ -143,11 +138,10 @@ __device__ __forceinline__ void sg_store_rows(float* buf, float* out, int cols, 
 
 template <class P, bool SPLIT>
 __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_constant__ P p, int n_tiles, unsigned* err_dev, unsigned* err_host) {
-    constexpr int N = 64 * P::HALVES, COUNT = N / 4, NB = P::HALVES, ROWS = P::A_TRANSPOSED ? 1 : 2;      // COUNT: columns a warp collects ; NB: chunks of B a thread stages
+    constexpr int N = 64 * P::HALVES, COUNT = N / 4;                  // COUNT: columns a warp collects
     constexpr unsigned A_PLANE = 128 * 128, B_PLANE = N * 128, A_BYTES = 3 * A_PLANE, B_BYTES = 3 * B_PLANE, STAGE = A_BYTES + B_BYTES;
     constexpr unsigned TMEM_COLS = P::HALVES == 1 ? 256 : 512;       // hh | hm + mh | hl + mm + lh
-    constexpr unsigned TMA_BYTES = (P::A_TMA ? A_BYTES : 0) + (P::B_TMA ? B_BYTES : 0);
-    constexpr bool CUTS = !P::A_TMA || !P::B_TMA;
+    constexpr unsigned TMA_BYTES = (P::A_TMA ? A_BYTES : 0) + B_BYTES;
     static_assert(!SPLIT || P::SHARED, "the other CTA's sums need the tiles' barriers");
     namespace cg = cooperative_groups;
     extern __shared__ __align__(1024) uint8_t sg_raw[];
@@ -158,7 +152,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
     const int rank = SPLIT ? (int)cg::this_cluster().block_rank() : 0, first = SPLIT ? blockIdx.x >> 1 : blockIdx.x, stride = SPLIT ? gridDim.x >> 1 : gridDim.x;
     if (tid == 0) {
 #pragma unroll
-        for (int s = 0; s < 2; s++) { pg_mbar_init(pg_smem(&sh.full[s]), (CUTS ? SG_WARPS : 0) + (TMA_BYTES ? 1 : 0)); pg_mbar_init(pg_smem(&sh.empty[s]), 1); }
+        for (int s = 0; s < 2; s++) { pg_mbar_init(pg_smem(&sh.full[s]), (P::A_TMA ? 0 : SG_WARPS) + 1); pg_mbar_init(pg_smem(&sh.empty[s]), 1); }
         pg_mbar_init(pg_smem(&sh.acc_full), 1); pg_mbar_init(pg_smem(&sh.acc_empty), SG_WARPS);
         pg_mbar_init(pg_smem(&sh.rows_done), SG_WARPS); pg_mbar_init(pg_smem(&sh.drained), 1);
         sh.fail = 0;
@@ -225,9 +219,9 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
         __syncwarp();
     } else if (warp == SG_WARPS + 1) {
         // ===== TMA loads: one thread =====
-        if (lane == 0 && TMA_BYTES) {
+        if (lane == 0) {
             if (P::A_TMA) asm volatile("prefetch.tensormap [%0];" ::"l"(p.map_a()) : "memory");
-            if (P::B_TMA) asm volatile("prefetch.tensormap [%0];" ::"l"(p.map_b()) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(p.map_b()) : "memory");
         }
         for (int index = first; index < n_tiles; index += stride) {
             typename P::Tile tile;
@@ -238,7 +232,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
                 __syncthreads();
             }
             bool ok = true;
-            if (lane == 0 && TMA_BYTES) {
+            if (lane == 0) {
                 for (int s = 0; s < tile.steps; s++) {
                     const unsigned gs = g + s, slot = gs & 1u, full = pg_smem(&sh.full[slot]), at = pg_smem(ring + (size_t)slot * STAGE);
                     if (!(ok = sg_wait(pg_smem(&sh.empty[slot]), ((gs >> 1) & 1u) ^ 1u, &sh.fail))) break;
@@ -247,7 +241,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
                     for (int i = 0; i < 3; i++) {
                         int x, y;
                         if (P::A_TMA) { p.at_a(tile, s, i, x, y); pg_tma_load_2d(at + i * A_PLANE, p.map_a(), full, x, y); }
-                        if (P::B_TMA) { p.at_b(tile, s, i, x, y); pg_tma_load_2d(at + A_BYTES + i * B_PLANE, p.map_b(), full, x, y); }
+                        p.at_b(tile, s, i, x, y);
+                        pg_tma_load_2d(at + A_BYTES + i * B_PLANE, p.map_b(), full, x, y);
                     }
                 }
             }
@@ -261,16 +256,11 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
             if (!ok) break;
         }
     } else {
-        // ===== operands.  A: elements 8 (tid % 8) .. of the rows tid / 8 and tid / 8 + 64, or (A_TRANSPOSED) elements 8 (tid / 128) .. and 32 later of the
-        // row tid % 128; B likewise, or column tid % 64 and elements 8 (tid / 64) .. =====
-        const int ar0 = P::A_TRANSPOSED ? tid & 127 : tid >> 3, ac0 = P::A_TRANSPOSED ? tid >> 7 : tid & 7;
-        const int bn0 = P::B_TRANSPOSED ? tid & 63 : tid >> 3, bk0 = P::B_TRANSPOSED ? tid >> 6 : tid & 7;
+        // ===== A, where it is cut here: elements 8 (tid / 128) .. and 32 later of the row tid % 128 =====
+        const int ar0 = tid & 127, ac0 = tid >> 7;
         const int q = warp & 3, col0 = (warp >> 2) * COUNT, row = q * 32 + lane;         // collected: TMEM lanes 32 (warp % 4) .., COUNT columns
-        const typename P::Fixed row_fixed = p.fixed(row);
-        typename P::Fixed a_fixed[ROWS];
-#pragma unroll
-        for (int e = 0; e < ROWS; e++) a_fixed[e] = p.fixed(ar0 + 64 * e);
-        const unsigned a_at = sg_offset(ar0, ac0), a_at2 = P::A_TRANSPOSED ? sg_offset(ar0, ac0 + 4) : sg_offset(ar0 + 64, ac0), b_at = A_BYTES + sg_offset(bn0, bk0);      // (64 rows further: 8192 bytes)
+        const typename P::Fixed row_fixed = p.fixed(row), a_fixed = p.fixed(ar0);
+        const unsigned a_at[2] = {sg_offset(ar0, ac0), sg_offset(ar0, ac0 + 4)};
         const unsigned from = tmem + ((unsigned)(q * 32) << 16) + (unsigned)col0;
         for (int index = first, nth = 0; index < n_tiles; index += stride) {
             typename P::Tile tile;
@@ -282,20 +272,12 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
                 p.setup(tile, ps);
                 __syncthreads();
             }
-            typename P::ARow ar[ROWS];
-            typename P::BCol bc[NB];
-            float av[2][8], bv[NB][8], acc[COUNT];
-            auto load_a = [&](int s, int e) { p.load_a(tile, ar[P::A_TRANSPOSED ? 0 : e], s, P::A_TRANSPOSED ? ac0 + 4 * e : ac0, av[e]); };
-            auto load_b = [&](int s, int e) { p.load_b(tile, bc[e], s, bk0, bv[e]); };
+            typename P::ARow ar;
+            float av[2][8], acc[COUNT];
             if (!P::A_TMA) {
+                ar = p.a_row(tile, ps, a_fixed, ar0);
 #pragma unroll
-                for (int e = 0; e < ROWS; e++) ar[e] = p.a_row(tile, ps, a_fixed[e], ar0 + 64 * e);
-#pragma unroll
-                for (int e = 0; e < 2; e++) if (steps > 0) load_a(0, e);
-            }
-            if (!P::B_TMA) {
-#pragma unroll
-                for (int e = 0; e < NB; e++) { bc[e] = p.b_col(tile, bn0 + 64 * e); if (steps > 0) load_b(0, e); }
+                for (int e = 0; e < 2; e++) if (steps > 0) p.load_a(tile, ar, 0, ac0 + 4 * e, av[e]);
             }
             bool ok = true;
 #pragma unroll
@@ -303,29 +285,20 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
             for (int s = 0; s <= steps; s++) {
                 if (s < steps) {
                     const unsigned gs = g + s, slot = gs & 1u;
-                    if (CUTS && !(ok = sg_wait_warp(pg_smem(&sh.empty[slot]), ((gs >> 1) & 1u) ^ 1u, &sh.fail))) break;
-                    uint8_t* st = ring + slot * STAGE;
                     if (!P::A_TMA) {
+                        if (!(ok = sg_wait_warp(pg_smem(&sh.empty[slot]), ((gs >> 1) & 1u) ^ 1u, &sh.fail))) break;
+                        uint8_t* st = ring + slot * STAGE;
 #pragma unroll
                         for (int e = 0; e < 2; e++) {
-                            p.prep_a(tile, ar[P::A_TRANSPOSED ? 0 : e], av[e]);
-                            sg_cut(st + (e ? a_at2 : a_at), A_PLANE, av[e]);
-                            if (s + 1 < steps) load_a(s + 1, e);
+                            p.prep_a(tile, ar, av[e]);
+                            sg_cut(st + a_at[e], A_PLANE, av[e]);
+                            if (s + 1 < steps) p.load_a(tile, ar, s + 1, ac0 + 4 * e, av[e]);
                         }
-                    }
-                    if (!P::B_TMA) {
-#pragma unroll
-                        for (int e = 0; e < NB; e++) {
-                            sg_cut(st + b_at + e * (64 * 128), B_PLANE, bv[e]);
-                            if (s + 1 < steps) load_b(s + 1, e);
-                        }
-                    }
-                    if (CUTS) {
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         sg_arrive(pg_smem(&sh.full[slot]));
                     }
                 } else if (P::SHARED) {
-                    p.end_a(tile, ps, ar[0], ar0, ac0);
+                    p.end_a(tile, ps, ar, ar0, ac0);
                     sg_arrive(pg_smem(&sh.rows_done));
                 }
                 if (s > 0 && (!(s & 1) || s == steps)) {              // step s - 1 closed a run

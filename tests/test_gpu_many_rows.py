@@ -68,6 +68,22 @@ def test_batch_matmul_of_many_rows(dev, kind, ab, bb, m, k, n):
         assert (np.abs(got - want) <= 2e-6 * size).all()
 
 
+@pytest.mark.parametrize("kind", ["f32", "f16"])
+@pytest.mark.parametrize("ab,bb,m,k,n", [(2, 1, 4, 1, 1), (2, 2, 9, 31, 33), (4, 2, 64, 128, 32), (6, 3, 65, 67, 63), (8, 2, 130, 160, 129)])
+def test_batch_matmul_of_many_rows_has_the_bits_of_one(dev, kind, ab, bb, m, k, n):
+    """32-bit sums in the order of a single row's, whatever the number of rows; numbers of very different size on both sides"""
+    from crabml_b200 import CudaTensor, capi
+    rng = np.random.default_rng(m + k)
+    a = (rng.standard_normal((ab, m, k)) * np.exp2(rng.integers(-12, 12, (ab, m, k)))).astype(np.float32)
+    cache = CudaTensor.alloc([bb, n + 3, k], capi.F16 if kind == "f16" else capi.F32, dev).resize(1, 0)
+    cache.concatenate(tensor(dev, np.abs(rng.standard_normal((n, bb, k)))).transpose([1, 0, 2]), 1)
+    for left, right in ((a, cache.transpose([0, 2, 1])), (rng.standard_normal((ab, m, n)), cache)):
+        got = tensor(dev, left).batch_matmul(right).export().reshape(ab, m, -1)
+        for r in sorted({0, 3, m // 2, m - 1}):
+            one = tensor(dev, left[:, r:r + 1]).batch_matmul(right).export().reshape(ab, -1)
+            np.testing.assert_array_equal(got[:, r].view(np.uint32), one.view(np.uint32))
+
+
 def test_batch_matmul_spreads_infinities_like_a_sum_of_products(dev):
     rng = np.random.default_rng(1)
     a, b = rng.standard_normal((1, 40, 70)).astype(np.float32), rng.standard_normal((1, 70, 50)).astype(np.float32)

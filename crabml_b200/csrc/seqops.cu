@@ -806,7 +806,7 @@ __global__ void head_rms_norm_kernel(float* __restrict__ x, const float* __restr
 
 // what the two products share: the tile's queries and the band of keys they can see
 struct WaTile {
-    int steps, t0, tq_n, kvh, c0, qt;                   // c0: first key (from `base` on) / first value column of the tile ; qt: which tile of queries
+    int steps, half, t0, tq_n, kvh, c0, qt;                   // c0: first key (from `base` on) / first value column of the tile ; qt: which tile of queries
     int band_lo, last;                                  // first and last key any of the tile's queries sees, counted from base
     int ring0;                                          // the ring's row of position base
     int at;                                             // base, counted from the first key of the cut planes
@@ -814,7 +814,7 @@ struct WaTile {
     int64_t base;                                       // a multiple of 64
 };
 __device__ __forceinline__ void wa_tile(const WaGeom& g, int qt, int kvh, WaTile& t) {
-    t.qt = qt; t.t0 = qt * g.QT; t.kvh = kvh; t.step0 = 0;
+    t.qt = qt; t.t0 = qt * g.QT; t.kvh = kvh; t.step0 = t.half = 0;
     t.tq_n = min(g.QT, g.T - t.t0);
     const int64_t i_first = g.pos0 + t.t0, lo = wa_lo(g, i_first);
     t.base = lo & ~(int64_t)63;
@@ -986,6 +986,7 @@ struct WaValues {
         t.c0 = (i - rest * per) * N;
         t.step0 = (int)(((t.base >> 6) & 1) ^ rank);
         t.steps = ((t.last >> 6) + 2 - t.step0) >> 1;
+        t.half = (int)((((t.base >> 6) + t.step0) >> 1) & 1);      // runs by position, not by where the tile's keys begin
         return true;
     }
     __device__ Fixed fixed(int r) const { const int tq = r / g.R; return Fixed{tq, r - tq * g.R}; }

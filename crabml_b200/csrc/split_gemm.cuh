@@ -3,8 +3,9 @@
 // An operand x is cut into three bfloat16 numbers h + m + l (8 mantissa bits each, cut off, so that all 24 bits are kept) while it is staged, and a
 // product is the sum of the six partial products that reach 2^-24 of it: hh + (hm + mh) + (hl + mm + lh).  tcgen05.mma adds a group of 16
 // products to its accumulator and cuts the sum off at 24 bits (measured: 1 + 0.75 ulp stays 1), so a long chain of additions would drift towards
-// zero.  Therefore hh has an accumulator of its own that is read out after 128 terms and added to a 32-bit register sum with ordinary rounding; the
-// other five, 2^-8 and less of it, are read out once.  Measured error and speed: at the users of this header.
+// zero.  Therefore hh has an accumulator of its own that is read out after 128 terms (a run of two steps) and added to a 32-bit register sum with
+// ordinary rounding; the other five, 2^-8 and less of it, are read out once.  Where the runs begin is the user's to say (Tile::half): a sum whose first
+// terms are zeros in one tile and absent in another keeps its bits when both tiles pair the same steps.  Measured error and speed: at the users of this header.
 //
 // Why not CUDA cores: 148 SMs x 128 fused multiply-adds at 1.9 GHz are 72 TFLOP/s at the very best; the six bfloat16 products of a 128 x 128 x 64
 // step take the tensor core 1536 cycles, which is 380 TFLOP/s of 32-bit product.  The three planes of N columns of B lie one behind the other, so
@@ -26,7 +27,8 @@
 //
 // The user is a struct P (a kernel argument) with
 //   static constexpr int HALVES    a tile has 64 * HALVES columns (1 or 2)
-//   struct Tile { int steps; ... } bool tile(i, rank, Tile&): the i-th tile, false = nothing to do; steps = ceil(K / 64); SPLIT: those of CTA `rank`
+//   struct Tile { int steps, half; ... } bool tile(i, rank, Tile&): the i-th tile, false = nothing to do; steps = ceil(K / 64); SPLIT: those of CTA `rank`;
+//                                  half: 1 = the first step is the second of its run
 //   Fixed, fixed(r)                what does not change from tile to tile about row r
 //   SHARED, Shared                 void setup(Tile, Shared&) is called by all threads before a tile, which then waits for the one before
 //   ARow, BCol                     what a thread keeps of a row / a column
@@ -136,6 +138,8 @@ __device__ __forceinline__ void sg_store_rows(float* buf, float* out, int cols, 
     }
 }
 
+__device__ __forceinline__ unsigned sg_runs(int steps, int half) { return steps ? (unsigned)(steps + half + 1) >> 1 : 0u; }
+
 template <class P, bool SPLIT>
 __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_constant__ P p, int n_tiles, unsigned* err_dev, unsigned* err_host) {
     constexpr int N = 64 * P::HALVES, COUNT = N / 4;                  // COUNT: columns a warp collects
@@ -174,7 +178,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
         for (int index = first; index < n_tiles; index += stride) {
             typename P::Tile tile;
             if (!p.tile(index, rank, tile)) continue;
-            const int steps = tile.steps;
+            const int steps = tile.steps, half = tile.half;
             if (P::SHARED) {
                 __syncthreads();
                 if (*(volatile int*)&sh.fail) break;
@@ -183,8 +187,9 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
             bool ok = true;
             if (lane == 0) {
                 for (int s = 0; s < steps; s++) {
-                    const unsigned gs = g + s, slot = gs & 1u;
-                    if (!(ok = sg_wait(pg_smem(&sh.full[slot]), (gs >> 1) & 1u, &sh.fail) && (s & 1 || sg_wait(pg_smem(&sh.acc_empty), ((runs + (s >> 1)) & 1u) ^ 1u, &sh.fail)))) break;
+                    const unsigned gs = g + s, slot = gs & 1u, in_run = (s + half) >> 1;
+                    const bool opens = s == 0 || !((s + half) & 1), closes = (s + half) & 1 || s + 1 == steps;
+                    if (!(ok = sg_wait(pg_smem(&sh.full[slot]), (gs >> 1) & 1u, &sh.fail) && (!opens || sg_wait(pg_smem(&sh.acc_empty), ((runs + in_run) & 1u) ^ 1u, &sh.fail)))) break;
                     pg_fence_after();
                     const unsigned at = pg_smem(ring + (size_t)slot * STAGE);
                     const uint64_t ah = pg_smem_desc(at), am = pg_smem_desc(at + A_PLANE), al = pg_smem_desc(at + 2 * A_PLANE);
@@ -192,16 +197,16 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {
                         const uint64_t adv = (uint64_t)((kk * PG_UMMA_K * 2) >> 4);
-                        pg_umma_f16(tmem, ah + adv, bh + adv, pg_instr_desc(128, N, 1), (s & 1) || kk > 0);                  // hh
+                        pg_umma_f16(tmem, ah + adv, bh + adv, pg_instr_desc(128, N, 1), !opens || kk > 0);                   // hh
                         pg_umma_f16(tmem + N, ah + adv, bm + adv, pg_instr_desc(128, 2 * N, 1), s > 0 || kk > 0);            //      hm | hl
                         pg_umma_f16(tmem + N, am + adv, bh + adv, pg_instr_desc(128, 2 * N, 1), 1u);                         //      mh | mm
                         pg_umma_f16(tmem + 2 * N, al + adv, bh + adv, pg_instr_desc(128, N, 1), 1u);                         //           lh
                     }
                     pg_umma_commit(pg_smem(&sh.empty[slot]));
-                    if ((s & 1) || s + 1 == steps) pg_umma_commit(pg_smem(&sh.acc_full));
+                    if (closes) pg_umma_commit(pg_smem(&sh.acc_full));
                 }
             }
-            runs += (steps + 1) >> 1;
+            runs += sg_runs(steps, half);
             ok = __all_sync(0xffffffffu, ok);
             g += steps;
             if (SPLIT) {
@@ -265,7 +270,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
         for (int index = first, nth = 0; index < n_tiles; index += stride) {
             typename P::Tile tile;
             if (!p.tile(index, rank, tile)) continue;
-            const int steps = tile.steps;
+            const int steps = tile.steps, half = tile.half;
             if (P::SHARED) {
                 __syncthreads();
                 if (*(volatile int*)&sh.fail) break;
@@ -301,8 +306,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
                     p.end_a(tile, ps, ar, ar0, ac0);
                     sg_arrive(pg_smem(&sh.rows_done));
                 }
-                if (s > 0 && (!(s & 1) || s == steps)) {              // step s - 1 closed a run
-                    if (!(ok = sg_wait_warp(pg_smem(&sh.acc_full), (runs + ((s - 1) >> 1)) & 1u, &sh.fail))) break;
+                if (s > 0 && (!((s + half) & 1) || s == steps)) {     // step s - 1 closed a run
+                    if (!(ok = sg_wait_warp(pg_smem(&sh.acc_full), (runs + ((s - 1 + half) >> 1)) & 1u, &sh.fail))) break;
                     pg_fence_after();
 #pragma unroll 1
                     for (int part = 0; part < (s < steps ? 1 : 3); part++) {
@@ -368,7 +373,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
                 }
             } else if (ok) p.emit(tile, ps, row_fixed, row, col0, acc, buf);
             if (!ok) break;
-            g += steps; runs += (steps + 1) >> 1; nth++;
+            g += steps; runs += sg_runs(steps, half); nth++;
         }
     }
     pg_fence_before();

@@ -174,6 +174,22 @@ def test_attention_keeps_an_infinite_value_to_the_queries_that_see_it(dev):
     assert np.isfinite(np.delete(got[70:, 1], 5, 1)).all()
 
 
+@pytest.mark.parametrize("window", [256, 512, 1024])
+def test_a_windowed_query_keeps_its_bits_wherever_its_call_starts(dev, window):
+    """Tiles of queries begin with the call, steps and runs of keys at positions: a query must not see which tile it fell into."""
+    from crabml_b200 import seqops
+    H, G, d, n = 4, 1, 128, 2012
+    rng = np.random.default_rng(window)
+    q, k, v = (rng.standard_normal((n, h * d)).astype(np.float32) for h in (H, G, G))
+    kt, vt = tensor(dev, k), tensor(dev, v)
+
+    def call(lo, hi):
+        return seqops.masked_attention(tensor(dev, q[lo:hi]), kt, vt, lo, H, G, d, d, d ** -0.5, window=window).export().reshape(hi - lo, H * d).view(np.uint32)
+    whole = call(1500, n)
+    for lo, hi in ((1501, n), (1531, n), (1564, 1700), (1627, n)):
+        np.testing.assert_array_equal(call(lo, hi), whole[lo - 1500:hi - 1500])
+
+
 # ---- a few activation rows against one quantised matrix ---------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("t", [oc.Q4_K, oc.Q5_K, oc.Q6_K])
 @pytest.mark.parametrize("m,k,b", [(1, 256, 2), (33, 1024, 3), (40, 2816, 8), (257, 4096, 9), (17, 14336, 31), (16, 40960, 5)])

@@ -775,7 +775,6 @@ extern "C" CC_API int cc_kv_ring_append(cc_device* dev, const cc_view* kring, co
 // alone decide (masked keys add an exact 0), and the value sum goes by steps of 64 positions, even ones and odd ones: a query's result does not
 // depend on where the call starts or what else it carries, and differs between a prompt pass and a decoded token only by the rounding of those sums.
 #define WA_ROWS 128
-#define WA_LOG2E 1.44269504f
 struct WaGeom {
     int T, H, G, R, dk, dv, window, block, ring, QT, cap;      // QT queries per tile; cap = row stride of S; block > 0: a query sees only its own block of positions
     int krs, vrs, vhs;                                  // floats between two rows of the key / value ring (vhs: between two heads' values inside a row)
@@ -960,7 +959,6 @@ struct WaScores {
 };
 // tiles: value columns (fastest), query tiles, G; the two CTAs of a cluster take the 64-key steps whose position is an even / odd multiple of 64
 // sink != NULL: the denominator also holds exp(sink[head]), a key without a value whose score is sink[head] as it stands (no scale)
-// exp(s - top) is taken as 2^(s log2e - top log2e): one rounding, and that of the second term is common to a row's weights and its denominator
 template <int TILE_HALVES>
 struct WaValues {
     static constexpr int HALVES = TILE_HALVES, N = 64 * HALVES;
@@ -972,7 +970,7 @@ struct WaValues {
     __device__ const void* map_b() const { return &maps[0]; }
     __device__ void at_a(const Tile&, int, int, int&, int&) const {}
     __device__ void at_b(const Tile& t, int s, int plane, int& x, int& y) const { x = t.at + (t.step0 + 2 * s) * 64; y = (plane * g.G + t.kvh) * g.dvp + t.c0; }
-    struct Shared { float top[WA_ROWS], sum[12][WA_ROWS]; };    // top: times log2e ; sum: before the steps the quarters' largest scores (0 ..), behind them the sums of each quarter
+    struct Shared { float top[WA_ROWS], sum[12][WA_ROWS]; };    // sum: before the steps the quarters' largest scores (0 ..), behind them the sums of each quarter
                                                                 // of the threads, of this CTA (4 ..) and of the other (8 ..)
     struct ARow { const float* s; float top, sum; };
     typedef const float* BCol;
@@ -1003,12 +1001,7 @@ struct WaValues {
     __device__ float top_of(const Tile& t, const Shared& ps, int r) const {
         float top = fmaxf(fmaxf(ps.sum[0][r], ps.sum[1][r]), fmaxf(ps.sum[2][r], ps.sum[3][r]));
         if (sink) top = fmaxf(top, sink_of(t, r));
-        return top * WA_LOG2E;
-    }
-    __device__ float weight(float s, float top) const {
-        float e;
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(fmaf(s, WA_LOG2E, -top)));
-        return e;
+        return top;
     }
     __device__ ARow a_row(const Tile& t, const Shared& ps, Fixed f, int r) const {
         return ARow{f.tq < t.tq_n ? S + wa_score_at(t, q_tiles, g.cap, 0, r) : nullptr, top_of(t, ps, r), 0.0f};
@@ -1022,7 +1015,7 @@ struct WaValues {
     __device__ void prep_a(const Tile&, ARow& a, float (&v)[8]) const {
         if (!a.s) return;
 #pragma unroll
-        for (int i = 0; i < 8; i++) { v[i] = weight(v[i], a.top); a.sum += v[i]; }
+        for (int i = 0; i < 8; i++) { v[i] = expf(v[i] - a.top); a.sum += v[i]; }
     }
     __device__ BCol b_col(const Tile& t, int n) const { return t.c0 + n < g.dv ? vring + t.kvh * g.vhs + t.c0 + n : nullptr; }
     __device__ void load_b(const Tile& t, BCol b, int s, int c, float (&v)[8]) const {
@@ -1053,7 +1046,7 @@ struct WaValues {
 #pragma unroll
         for (int i = 0; i < 4; i++) { a += ps.sum[4 + i][r]; b += ps.sum[8 + i][r]; }
         float total = a + b;                            // of the two CTAs, the same number in both
-        if (sink) total += weight(sink_of(t, r), ps.top[r]);
+        if (sink) total += expf(sink_of(t, r) - ps.top[r]);
         const float inv = 1.0f / total;
 #pragma unroll
         for (int c = 0; c < COUNT; c++) v[c] *= inv;

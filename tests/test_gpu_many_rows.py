@@ -190,6 +190,18 @@ def test_a_windowed_query_keeps_its_bits_wherever_its_call_starts(dev, window):
         np.testing.assert_array_equal(call(lo, hi), whole[lo - 1500:hi - 1500])
 
 
+def test_attention_weighs_scores_of_any_size(dev):
+    """Equal scores weigh the same however large they are: exp(score - largest) and no other form of it"""
+    from crabml_b200 import seqops
+    T, d = 80, 64
+    for size in (1.0, 1e10, 1.69e19):
+        q, k, v = np.zeros((T, 4), np.float32), np.zeros((T, 4), np.float32), np.random.default_rng(5).standard_normal((T, d)).astype(np.float32)
+        q[:, 1], k[:, 1] = size, size
+        got = seqops.masked_attention(tensor(dev, q), tensor(dev, k), tensor(dev, v), 0, 1, 1, 4, d, 1.0).export().reshape(T, d)
+        want = np.cumsum(v.astype(np.float64), 0) / np.arange(1, T + 1)[:, None]
+        assert np.abs(got - want).max() <= 2e-6, size
+
+
 # ---- a few activation rows against one quantised matrix ---------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("t", [oc.Q4_K, oc.Q5_K, oc.Q6_K])
 @pytest.mark.parametrize("m,k,b", [(1, 256, 2), (33, 1024, 3), (40, 2816, 8), (257, 4096, 9), (17, 14336, 31), (16, 40960, 5)])

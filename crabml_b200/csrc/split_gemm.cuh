@@ -1,7 +1,8 @@
 // split_gemm.cuh -- products of 32-bit operands on the tensor cores without giving up 32 bits.
 //
-// An operand x is cut into three bfloat16 numbers h + m + l (8 mantissa bits each, cut off, so that all 24 bits are kept) while it is staged, and a
-// product is the sum of the six partial products that reach 2^-24 of it: hh + (hm + mh) + (hl + mm + lh).  tcgen05.mma adds a group of 16
+// An operand x is cut into three bfloat16 numbers h + m + l (8 mantissa bits each, each the nearest to what is left, so that all 24 bits are kept), and a
+// product is the sum of six of the nine partial products: hh + (hm + mh) + (hl + mm + lh).  With x in [1, 2), |m| <= 2^-8 and |l| <= 2^-17, so that what is
+// left out, ml + lm + ll, stays below 2^-24 of the product, of either sign (cut off instead of rounded it reached 2^-21, always of the product's own sign).  tcgen05.mma adds a group of 16
 // products to its accumulator and cuts the sum off at 24 bits (measured: 1 + 0.75 ulp stays 1), so a long chain of additions would drift towards
 // zero.  Therefore hh has an accumulator of its own that is read out after 128 terms (a run of two steps) and added to a 32-bit register sum with
 // ordinary rounding; the other five, 2^-8 and less of it, are read out once.  Where the runs begin is the user's to say (Tile::half): a sum whose first
@@ -22,7 +23,7 @@
 // a cluster share a tile's steps, and each finishes half of its columns with the sums of both).
 // Every wait is bounded: on expiry the CTA raises `fail`, every warp leaves its loop, TMEM is freed and the host reports it.
 //
-// An infinity cannot be cut (its rest is NaN): sums that come out as NaN are computed again in plain 32-bit arithmetic from the same operands, so
+// An infinity cannot be cut (its rest is NaN), nor what rounds to one: sums that come out as NaN are computed again in plain 32-bit arithmetic from the same operands, so
 // that infinities spread exactly as far as they would in a sum of products.
 //
 // The user is a struct P (a kernel argument) with
@@ -76,13 +77,14 @@ __device__ __forceinline__ void sg_cut(uint8_t* at, size_t plane, const float (&
     unsigned h[4], m[4], l[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const unsigned a = __float_as_uint(v[2 * i]), b = __float_as_uint(v[2 * i + 1]);
-        const float a1 = v[2 * i] - __uint_as_float(a & 0xffff0000u), b1 = v[2 * i + 1] - __uint_as_float(b & 0xffff0000u);
-        const unsigned ua = __float_as_uint(a1), ub = __float_as_uint(b1);
-        const float a2 = a1 - __uint_as_float(ua & 0xffff0000u), b2 = b1 - __uint_as_float(ub & 0xffff0000u);
-        h[i] = __byte_perm(a, b, 0x7632);
-        m[i] = __byte_perm(ua, ub, 0x7632);
-        l[i] = __byte_perm(__float_as_uint(a2), __float_as_uint(b2), 0x7632);
+        auto high = [](float x) { return (__float_as_uint(x) + 0x8000u) & 0xffff0000u; };      // (an infinity stays one)
+        const float a = v[2 * i], b = v[2 * i + 1];
+        const unsigned ha = high(a), hb = high(b);
+        const float a1 = a - __uint_as_float(ha), b1 = b - __uint_as_float(hb);
+        const unsigned ma = high(a1), mb = high(b1);
+        h[i] = __byte_perm(ha, hb, 0x7632);
+        m[i] = __byte_perm(ma, mb, 0x7632);
+        l[i] = __byte_perm(__float_as_uint(a1 - __uint_as_float(ma)), __float_as_uint(b1 - __uint_as_float(mb)), 0x7632);
     }
     *(uint4*)at = make_uint4(h[0], h[1], h[2], h[3]);
     *(uint4*)(at + plane) = make_uint4(m[0], m[1], m[2], m[3]);

@@ -202,6 +202,23 @@ def test_attention_weighs_scores_of_any_size(dev):
         assert np.abs(got - want).max() <= 2e-6, size
 
 
+@pytest.mark.parametrize("bits", [0x3f80ffff, 0x3f807f7f, 0x3f807ebf, 0x3f8101ff, 0x3faaaaab, 0x3fff7fff, 0x3fd5c28f])
+def test_attention_scores_of_operands_that_use_all_their_bits(dev, bits):
+    """Keys of the odd positions are the nearest bfloat16 number to those of the even ones and lose nothing when they are cut.  A score s of one term: 2^-24 s at
+    most is left out, the accumulators cut off twice at 2^-23, the scale rounds once at 2^-24; a weight of two nearly equal ones moves by a quarter of that."""
+    from crabml_b200 import seqops
+    x = np.array([bits], np.uint32).view(np.float32)[0]
+    near = np.array([(bits + 0x8000) & 0xffff0000], np.uint32).view(np.float32)[0]
+    T, d = 130, 64
+    scale = np.float32(60.0)
+    q, k, v = np.full((T, 1), x, np.float32), np.full((T, 1), x, np.float32), np.zeros((T, d), np.float32)
+    k[1::2], v[::2] = near, 1.0
+    got = seqops.masked_attention(tensor(dev, q), tensor(dev, k), tensor(dev, v), 0, 1, 1, 1, d, scale).export().reshape(T, d)
+    want = attend(q[:, None], k[:, None], v[:, None], float(scale), 0, 0, 0, 0.0, None)[:, 0]
+    s = float(x) * float(x) * float(scale)
+    assert np.abs(got - want).max() <= 0.25 * s * (2.0 ** -24 + 2 * 2.0 ** -23 + 2.0 ** -24) + 4 * 2.0 ** -24
+
+
 # ---- a few activation rows against one quantised matrix ---------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("t", [oc.Q4_K, oc.Q5_K, oc.Q6_K])
 @pytest.mark.parametrize("m,k,b", [(1, 256, 2), (33, 1024, 3), (40, 2816, 8), (257, 4096, 9), (17, 14336, 31), (16, 40960, 5)])

@@ -75,16 +75,18 @@ __device__ __forceinline__ void sg_arrive(unsigned bar) {
 // eight elements -> 16 bytes in each of the three planes
 __device__ __forceinline__ void sg_cut(uint8_t* at, size_t plane, const float (&v)[8]) {
     unsigned h[4], m[4], l[4];
+    auto nearest = [](float a, float b) {
+        unsigned u;
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(u) : "f"(b), "f"(a));
+        return u;
+    };
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        auto high = [](float x) { return (__float_as_uint(x) + 0x8000u) & 0xffff0000u; };      // (an infinity stays one)
         const float a = v[2 * i], b = v[2 * i + 1];
-        const unsigned ha = high(a), hb = high(b);
-        const float a1 = a - __uint_as_float(ha), b1 = b - __uint_as_float(hb);
-        const unsigned ma = high(a1), mb = high(b1);
-        h[i] = __byte_perm(ha, hb, 0x7632);
-        m[i] = __byte_perm(ma, mb, 0x7632);
-        l[i] = __byte_perm(__float_as_uint(a1 - __uint_as_float(ma)), __float_as_uint(b1 - __uint_as_float(mb)), 0x7632);
+        h[i] = nearest(a, b);
+        const float a1 = a - __uint_as_float(h[i] << 16), b1 = b - __uint_as_float(h[i] & 0xffff0000u);
+        m[i] = nearest(a1, b1);
+        l[i] = nearest(a1 - __uint_as_float(m[i] << 16), b1 - __uint_as_float(m[i] & 0xffff0000u));
     }
     *(uint4*)at = make_uint4(h[0], h[1], h[2], h[3]);
     *(uint4*)(at + plane) = make_uint4(m[0], m[1], m[2], m[3]);

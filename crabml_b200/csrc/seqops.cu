@@ -1110,6 +1110,39 @@ __global__ void __launch_bounds__(256) wa_scores_row_kernel(const float* __restr
 #define WV_SPLIT 8
 #define WV_THREADS 256
 #define WV_WARPS (WV_THREADS / 32)
+// the slices meet: every warp's weighted values of a slice in acc, the slice's largest score and sum of weights in top and sum
+template <int RB>
+__device__ __forceinline__ void wv_finish(const float (&acc)[RB], float* part, float* top, float* sum, float* acc_sm, float* __restrict__ out, const WaGeom& g, const float* __restrict__ sink, int t, int kvh,
+                                          int h0, int nh, int lane, int w) {
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+#pragma unroll
+    for (int hr = 0; hr < RB; hr++) part[(w * RB + hr) * 32 + lane] = acc[hr];
+    __syncthreads();
+    for (int hr = w; hr < RB; hr += WV_WARPS) {
+        float a = 0.0f;
+#pragma unroll
+        for (int ww = 0; ww < WV_WARPS; ww++) a += part[(ww * RB + hr) * 32 + lane];
+        acc_sm[hr * 32 + lane] = a;
+    }
+    cluster.sync();
+    for (int hr = (int)blockIdx.z + WV_SPLIT * w; hr < nh; hr += WV_SPLIT * WV_WARPS) {
+        const int h = kvh * g.R + h0 + hr;
+        const float sk = sink ? sink[h] : -INFINITY;
+        float mx = sk;
+#pragma unroll
+        for (int z = 0; z < WV_SPLIT; z++) mx = fmaxf(mx, cluster.map_shared_rank(top, z)[hr]);
+        float tot = sink ? expf(sk - mx) : 0.0f, a = 0.0f;
+#pragma unroll
+        for (int z = 0; z < WV_SPLIT; z++) {
+            const float f = expf(cluster.map_shared_rank(top, z)[hr] - mx);                  // an empty slice: exp(-inf) = 0
+            tot = fmaf(f, cluster.map_shared_rank(sum, z)[hr], tot);
+            a = fmaf(f, cluster.map_shared_rank(acc_sm, z)[hr * 32 + lane], a);
+        }
+        const int col = blockIdx.y * 32 + lane;
+        if (col < g.dv) out[((int64_t)t * g.H + h) * g.dv + col] = a / tot;
+    }
+    cluster.sync();                                           // nobody leaves while its shared memory may still be read
+}
 template <int RB>
 __global__ void __cluster_dims__(1, 1, WV_SPLIT) __launch_bounds__(WV_THREADS) wa_values_slices_kernel(const float* __restrict__ S, const float* __restrict__ vring, float* __restrict__ out,
                                                                                                        WaGeom g, const float* __restrict__ sink, int slice_cap) {
@@ -1118,7 +1151,6 @@ __global__ void __cluster_dims__(1, 1, WV_SPLIT) __launch_bounds__(WV_THREADS) w
     float* pr = wv_sm;                                        // [RB][slice_cap]
     float* part = wv_sm + (size_t)RB * slice_cap;             // [WV_WARPS][RB][32]
     __shared__ float top[RB], sum[RB], acc_sm[RB * 32];       // what the cluster reads: the slice's largest score, sum of weights, weighted values
-    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int hblocks = (g.R + RB - 1) / RB;
     const int hb = blockIdx.x % hblocks, tk = blockIdx.x / hblocks;
     const int t = tk / g.G, kvh = tk % g.G, h0 = hb * RB, nh = min(RB, g.R - h0);
@@ -1157,43 +1189,169 @@ __global__ void __cluster_dims__(1, 1, WV_SPLIT) __launch_bounds__(WV_THREADS) w
             if (++r == g.ring) r = 0;
         }
     }
-#pragma unroll
-    for (int hr = 0; hr < RB; hr++) part[(w * RB + hr) * 32 + lane] = acc[hr];
-    __syncthreads();
-    for (int hr = w; hr < RB; hr += WV_WARPS) {
-        float a = 0.0f;
-#pragma unroll
-        for (int ww = 0; ww < WV_WARPS; ww++) a += part[(ww * RB + hr) * 32 + lane];
-        acc_sm[hr * 32 + lane] = a;
-    }
-    cluster.sync();
-    for (int hr = (int)blockIdx.z + WV_SPLIT * w; hr < nh; hr += WV_SPLIT * WV_WARPS) {
-        const int h = kvh * g.R + h0 + hr;
-        const float sk = sink ? sink[h] : -INFINITY;
-        float mx = sk;
-#pragma unroll
-        for (int z = 0; z < WV_SPLIT; z++) mx = fmaxf(mx, cluster.map_shared_rank(top, z)[hr]);
-        float tot = sink ? expf(sk - mx) : 0.0f, a = 0.0f;
-#pragma unroll
-        for (int z = 0; z < WV_SPLIT; z++) {
-            const float f = expf(cluster.map_shared_rank(top, z)[hr] - mx);                  // an empty slice: exp(-inf) = 0
-            tot = fmaf(f, cluster.map_shared_rank(sum, z)[hr], tot);
-            a = fmaf(f, cluster.map_shared_rank(acc_sm, z)[hr * 32 + lane], a);
-        }
-        const int col = blockIdx.y * 32 + lane;
-        if (col < g.dv) out[((int64_t)t * g.H + h) * g.dv + col] = a / tot;
-    }
-    cluster.sync();                                           // nobody leaves while its shared memory may still be read
+    wv_finish<RB>(acc, part, top, sum, acc_sm, out, g, sink, t, kvh, h0, nh, lane, w);
 }
-static size_t wa_slices_smem(int RB, int64_t maxn, int* slice_cap) {
-    *slice_cap = (int)((maxn + WV_SPLIT - 1) / WV_SPLIT);
-    return ((size_t)RB * *slice_cap + (size_t)WV_WARPS * RB * 32) * 4;
+// slices longer than shared memory holds, chunk by chunk: what is summed so far is scaled whenever the largest score grows.  A slice of one chunk gets the bits of
+// the kernel above, which stays for its loads in flight (one kernel for both: 155 us where that takes 108, a token of 32 heads over 16000 keys)
+__host__ __device__ constexpr int wv_chunk(int RB) { return 160 * 256 / RB - WV_WARPS * 32; }      // keys of a chunk: with the warps' parts 160 KB
+template <int RB>
+__global__ void __cluster_dims__(1, 1, WV_SPLIT) __launch_bounds__(WV_THREADS) wa_values_chunks_kernel(const float* __restrict__ S, const float* __restrict__ vring, float* __restrict__ out,
+                                                                                                       WaGeom g, const float* __restrict__ sink) {
+    pdl_enter();
+    extern __shared__ float wv_sm[];
+    constexpr int CHUNK = wv_chunk(RB);
+    float* pr = wv_sm;                                        // [RB][CHUNK]
+    float* part = wv_sm + (size_t)RB * CHUNK;                 // [WV_WARPS][RB][32]
+    __shared__ float top[RB], sum[RB], acc_sm[RB * 32], fac[RB];      // fac: what the sums of the chunks before are worth
+    const int hblocks = (g.R + RB - 1) / RB;
+    const int hb = blockIdx.x % hblocks, tk = blockIdx.x / hblocks;
+    const int t = tk / g.G, kvh = tk % g.G, h0 = hb * RB, nh = min(RB, g.R - h0);
+    const int64_t i = g.pos0 + t, lo = wa_lo(g, i);
+    const int n = (int)(i - lo + 1), per_slice = (n + WV_SPLIT - 1) / WV_SPLIT;
+    const int s0 = min(n, (int)blockIdx.z * per_slice), m = min(n, s0 + per_slice) - s0;      // this CTA's keys: s0 .. s0 + m of the visible ones
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.y * 32 + lane;
+    const float* vb = vring + (int64_t)kvh * g.vhs + d;
+    float acc[RB];
+#pragma unroll
+    for (int hr = 0; hr < RB; hr++) acc[hr] = 0.0f;
+    int c0 = 0;
+    do {                                                      // (an empty slice: once, for its -inf and zeros)
+        const int mc = min(CHUNK, m - c0);
+        for (int hr = w; hr < RB; hr += WV_WARPS) {
+            const float* Sr = S + ((int64_t)t * g.H + kvh * g.R + h0 + hr) * g.cap + s0 + c0;
+            float* p = pr + (size_t)hr * CHUNK;
+            const bool on = hr < nh;
+            const float before = c0 ? top[hr] : -INFINITY;
+            float mx = -INFINITY;
+            for (int c = lane; c < mc; c += 32) { const float v = on ? Sr[c] : 0.0f; p[c] = v; mx = fmaxf(mx, v); }
+            mx = fmaxf(warp_max(mx), before);
+            float tot = 0.0f;
+            for (int c = lane; c < mc; c += 32) { const float e = expf(p[c] - mx); p[c] = e; tot += e; }
+            tot = warp_sum(tot);
+            if (lane == 0) {
+                if (c0) { fac[hr] = expf(before - mx); tot = fmaf(fac[hr], sum[hr], tot); }
+                top[hr] = mx; sum[hr] = tot;
+            }
+        }
+        __syncthreads();
+        if (c0) {
+#pragma unroll
+            for (int hr = 0; hr < RB; hr++) acc[hr] *= fac[hr];
+        }
+        const int per = (mc + WV_WARPS - 1) / WV_WARPS;
+        const int c_begin = min(mc, w * per), c_end = min(mc, c_begin + per);
+        if (d < g.dv) {
+            int r = (int)((lo + s0 + c0 + c_begin) % g.ring);
+#pragma unroll 8
+            for (int c = c_begin; c < c_end; c++) {
+                const float v = vb[(int64_t)r * g.vrs];
+#pragma unroll
+                for (int hr = 0; hr < RB; hr++) acc[hr] = fmaf(pr[(size_t)hr * CHUNK + c], v, acc[hr]);
+                if (++r == g.ring) r = 0;
+            }
+        }
+        c0 += CHUNK;
+        __syncthreads();                                      // the chunk has been read
+    } while (c0 < m);
+    wv_finish<RB>(acc, part, top, sum, acc_sm, out, g, sink, t, kvh, h0, nh, lane, w);
 }
 template <int RB>
-static cudaError_t wa_launch_slices(cc_device* dev, const float* S, const float* v, float* out, const WaGeom& g, const float* sink, size_t smem, int slice_cap) {
-    if (smem > 40 * 1024) { cudaError_t e = cudaFuncSetAttribute(wa_values_slices_kernel<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) return e; }
-    cc_launch_alone(dev, wa_values_slices_kernel<RB>, dim3((unsigned)(g.T * g.G * ((g.R + RB - 1) / RB)), (unsigned)((g.dv + 31) / 32), WV_SPLIT), WV_THREADS, smem, S, v, out, g, sink, slice_cap);
-    return cudaSuccess;
+static int wa_launch_slices(cc_device* dev, const float* S, const float* v, float* out, const WaGeom& g, const float* sink, int64_t maxn) {
+    const int64_t slice = (maxn + WV_SPLIT - 1) / WV_SPLIT;
+    const bool whole = slice <= wv_chunk(RB);
+    const int smem = (int)((RB * (whole ? slice : wv_chunk(RB)) + WV_WARPS * RB * 32) * 4);
+    const dim3 grid((unsigned)(g.T * g.G * ((g.R + RB - 1) / RB)), (unsigned)((g.dv + 31) / 32), WV_SPLIT);
+    if (whole) {
+        if (smem > 40 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(wa_values_slices_kernel<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        cc_launch_alone(dev, wa_values_slices_kernel<RB>, grid, WV_THREADS, smem, S, v, out, g, sink, (int)slice);
+    } else {
+        CC_CUDA(dev, cudaFuncSetAttribute(wa_values_chunks_kernel<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        cc_launch_alone(dev, wa_values_chunks_kernel<RB>, grid, WV_THREADS, smem, S, v, out, g, sink);
+    }
+    CC_LAUNCH_CHECK(dev);
+    return CC_OK;
+}
+// what a call's two ways share
+struct WaCall {
+    float* q;
+    const float *k, *v, *r1, *r2, *sink;
+    float *o, scale;
+    int64_t last, oldest, reach;                        // last position; first one anybody sees; the most keys one query sees
+};
+static int64_t wa_rows_smem(const WaGeom& g) { return (int64_t)(g.R < WS_HEADS ? g.R : WS_HEADS) * g.dk * 4; }
+// few rows: keys spread over the whole device
+static int wa_by_rows(cc_device* dev, WaGeom g, const WaCall& c) {
+    const size_t smem = (size_t)wa_rows_smem(g);
+    const int RB = g.R >= 8 ? 8 : g.R >= 3 ? 4 : g.R;        // query heads a cluster of the value kernel takes together
+    if (smem > 48 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(wa_scores_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    g.cap = (int)c.reach;
+    void* S = nullptr; size_t cls = 0;
+    int rc = cc_pool_alloc(dev, (size_t)g.T * g.H * g.cap * 4, &S, &cls);
+    if (rc) return rc;
+    cc_launch_pdl(dev, wa_scores_row_kernel, dim3((unsigned)((c.reach + 15) / 16), (unsigned)g.T, (unsigned)(g.G * ((g.R + WS_HEADS - 1) / WS_HEADS))), 256, smem, c.q, c.k, (float*)S, g, c.scale, c.r1, c.r2);
+    dev->launches++;
+    rc = RB == 8 ? wa_launch_slices<8>(dev, (const float*)S, c.v, c.o, g, c.sink, c.reach) : RB == 4 ? wa_launch_slices<4>(dev, (const float*)S, c.v, c.o, g, c.sink, c.reach)
+         : RB == 2 ? wa_launch_slices<2>(dev, (const float*)S, c.v, c.o, g, c.sink, c.reach) : wa_launch_slices<1>(dev, (const float*)S, c.v, c.o, g, c.sink, c.reach);
+    cc_pool_free(dev, S, cls);
+    return rc;
+}
+// many rows: key/value heads in equal groups, so that the workspace -- scores and cut planes of a group -- is at most twice what the scores of all heads take
+// or WA_WORKSPACE, whichever is more (one head at least).  *room: false when the device had none and nothing was launched
+#define WA_WORKSPACE ((size_t)512 << 20)
+static int wa_by_tiles(cc_device* dev, WaGeom g, const WaCall& c, bool* room) {
+    const int G = g.G, q_tiles = (g.T + g.QT - 1) / g.QT, vtile = g.dv > 64 ? 128 : 64;
+    // keys a query tile can see, counted from the multiple of 64 below the first of them
+    const int64_t band = c.reach - 1 + g.QT + 63, band_max = band < c.last + 64 ? band : c.last + 64;
+    const int key_tiles = (int)((band_max + WaScores::N - 1) / WaScores::N);
+    g.cap = key_tiles * WaScores::N;
+    g.base0 = c.oldest & ~(int64_t)63;
+    g.span = (int)((c.last - g.base0 + 64) & ~(int64_t)63) + 64;              // in whole steps, and one more: a tile of 128 keys may start at any step
+    g.dkp = (g.dk + 63) & ~63; g.dvp = (g.dv + vtile - 1) / vtile * vtile;
+    // of one key/value head; every part is a multiple of 512 bytes
+    const size_t q_rows = (size_t)q_tiles * WA_ROWS, scores = q_rows * g.cap * 4, tops = (size_t)q_tiles * key_tiles * 4 * WA_ROWS * 4;
+    const size_t qc = 3 * q_rows * g.dkp * 2, kc = 3 * (size_t)g.span * g.dkp * 2, vc = 3 * (size_t)g.dvp * g.span * 2, one = scores + tops + qc + kc + vc;
+    const size_t scores_twice = 2 * (size_t)g.T * g.H * c.reach * 4, most = scores_twice > WA_WORKSPACE ? scores_twice : WA_WORKSPACE;
+    int groups = (int)((G * one + most - 1) / most);
+    if (groups > G) groups = G;
+    void* S = nullptr; size_t cls = 0;
+    int rc, n = 0;
+    for (;; groups = groups * 2 < G ? groups * 2 : G) {
+        n = (G + groups - 1) / groups;
+        if (3 * n * (q_rows + g.span) * (g.dkp / 8) >= (size_t)1 << 31) rc = cc_fail(dev, CC_ERR_UNSUPPORTED, "window_attention: too many rows");      // 32-bit indices
+        else rc = cc_pool_alloc(dev, n * one, &S, &cls);
+        if (rc == CC_OK) break;
+        cudaGetLastError();                                  // it has been taken note of
+        if (n == 1) { *room = false; return rc; }
+    }
+    uint8_t *base = (uint8_t*)S, *qp3 = base + n * (scores + tops), *kp3 = qp3 + n * qc, *vp3 = kp3 + n * kc;
+    WaScores ws{};
+    ws.S = (float*)base; ws.tops = (float*)(base + n * scores); ws.scale = c.scale; ws.key_tiles = key_tiles; ws.q_tiles = q_tiles;
+    ws.vec = g.dk % 4 == 0 && (((uintptr_t)c.q | (uintptr_t)c.k) & 15) == 0;
+    for (int g0 = 0; g0 < G && rc == CC_OK; g0 += n) {
+        const int h0 = g0 * g.R;
+        g.G = G - g0 < n ? G - g0 : n;
+        const float* v = c.v + (int64_t)g0 * g.vhs;
+        ws.q = c.q + (int64_t)h0 * g.dk; ws.kring = c.k + (int64_t)g0 * g.dk; ws.r1 = c.r1 ? c.r1 + h0 : nullptr; ws.r2 = c.r2 ? c.r2 + h0 : nullptr; ws.g = g;
+        const size_t rows = (size_t)g.G * q_rows;
+        const int64_t row_blocks = ((int64_t)(rows + (size_t)g.G * g.span) * (g.dkp >> 3) + 255) / 256, blocks = row_blocks + (int64_t)(g.span >> 6) * (g.dvp >> 6) * g.G;
+        CUtensorMap vmap;
+        rc = cc_make_tmap_bf16(dev, &ws.maps[0], qp3, 3 * (int64_t)rows, g.dkp, WA_ROWS);
+        if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &ws.maps[1], kp3, (int64_t)3 * g.G * g.span, g.dkp, WaScores::N);
+        if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &vmap, vp3, (int64_t)3 * g.G * g.dvp, g.span, vtile);
+        if (rc == CC_OK) {
+            cc_launch_pdl(dev, wa_cut_kernel, (unsigned)blocks, 256, 0, ws.q, ws.kring, v, qp3, kp3, vp3, g, q_tiles, (unsigned)row_blocks, (int)(g.base0 % g.ring), (int)(c.oldest - g.base0), ws.vec);
+            dev->launches++;
+            rc = sg_launch(dev, ws, (int64_t)key_tiles * q_tiles * g.G);
+        }
+        auto values = [&](auto wv) {
+            wv.maps[0] = vmap; wv.S = ws.S; wv.tops = ws.tops; wv.vring = v; wv.sink = c.sink ? c.sink + h0 : nullptr; wv.o = c.o + (int64_t)h0 * g.dv; wv.g = g;
+            wv.key_tiles = key_tiles; wv.q_tiles = q_tiles;
+            return sg_launch<decltype(wv), true>(dev, wv, (int64_t)(g.dvp / vtile) * q_tiles * g.G);
+        };
+        if (rc == CC_OK) rc = vtile == 128 ? values(WaValues<2>{}) : values(WaValues<1>{});
+    }
+    cc_pool_free(dev, S, cls);
+    return rc;
 }
 static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view* qnw, float eps, const cc_view* kring, const cc_view* vring, int64_t pos0, int32_t H, int32_t G,
                                  int32_t dk, int32_t dv, int32_t window, int32_t block, float scale, const cc_view* r1, const cc_view* r2, const cc_view* sink, cc_buf** out,
@@ -1230,76 +1388,26 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
     int64_t reach = last + 1;
     if (window > 0 && window < reach) reach = window;
     if (block > 0 && block < reach) reach = block;
-    const int64_t maxn = reach;
     const int R = H / G;
     CC_REQUIRE(dev, R <= 64, "window_attention: %d query heads per key/value head (at most %d)", R, 64);
     g.T = (int)T; g.H = H; g.G = G; g.R = R; g.dk = dk; g.dv = dv; g.ring = (int)ring; g.QT = WA_ROWS / R; g.pos0 = pos0; g.pos0_row = (int)(pos0 % ring);
     g.krs = G * dk; g.vrs = vring ? G * dv : G * dk; g.vhs = vring ? dv : dk;
-    const float *r1p = r1 ? fptr(r1) : nullptr, *r2p = r2 ? fptr(r2) : nullptr, *sinkp = sink ? fptr(sink) : nullptr;
-    // few rows: keys spread over the whole device; what its kernels keep in shared memory has to fit
-    const int s_heads = R < WS_HEADS ? R : WS_HEADS;
-    const int RB = R >= 8 ? 8 : R >= 3 ? 4 : R;              // query heads a cluster of the few-row value kernel takes together
-    int slice_cap = 0;
-    const size_t rows_smem = (size_t)s_heads * dk * 4, slices_smem = wa_slices_smem(RB, maxn, &slice_cap);
-    const bool few_rows = T * H <= 64 && rows_smem <= 160 * 1024 && slices_smem <= 160 * 1024;
-    const int q_tiles = (int)((T + g.QT - 1) / g.QT);
-    // keys a query tile can see, counted from the multiple of 64 below the first of them
-    const int64_t band = reach - 1 + g.QT + 63, band_max = band < last + 64 ? band : last + 64;
-    const int key_tiles = (int)((band_max + WaScores::N - 1) / WaScores::N);
-    g.cap = few_rows ? (int)maxn : key_tiles * WaScores::N;
-    float* qp = fptr(q);
+    const WaCall c = {fptr(q), fptr(kring), vptr, r1 ? fptr(r1) : nullptr, r2 ? fptr(r2) : nullptr, sink ? fptr(sink) : nullptr, (float*)o->base, scale, last, oldest, reach};
+    // Row by row the cache is read once per query and 8 heads of a key head; a tile's share of cutting it is the same up to 128 rows.  us by rows / by tiles, heads
+    // x queries over 300, 2000, 16000 keys: 16 x 4 (a key head each) 26 / 28, 65 / 57, 437 / 354 ; 16 x 8 42 / 27, 121 / 57, 817 / 353 ; 128 x 1 (keys of 192) 42 / 80,
+    // 139 / 320 ; 128 x 2 75 / 80, 254 / 320 ; 128 x 4 147 / 79, 499 / 320 ; 64 x 1 (32 a key head: 4 reads) 17 / 24, 28 / 38, 139 / 197 ; 64 x 2 18 / 20, 42 / 38, 239 / 197
+    const bool can_rows = T <= 65535 && wa_rows_smem(g) <= 160 * 1024;
+    const bool few_rows = can_rows && (T * H <= 64 || (T <= 2 && T * ((R + 7) / 8) <= 4) || ring >= (1 << 30));
     if (qnw) {             // the query norm, in place: q is this call's private projection output in every caller of the runner; a caller that
                            // needs its q untouched passes a copy
-        cc_launch_pdl(dev, head_rms_norm_kernel, (unsigned)((T * H + 7) / 8), 256, 0, qp, fptr(qnw), T * H, dk, eps);
+        cc_launch_pdl(dev, head_rms_norm_kernel, (unsigned)((T * H + 7) / 8), 256, 0, c.q, fptr(qnw), T * H, dk, eps);
         dev->launches++;
     }
-    void* Sp = nullptr; size_t cls = 0;
-    if (!few_rows) {
-        const int vtile = dv > 64 ? 128 : 64;
-        g.base0 = oldest & ~(int64_t)63;
-        g.span = (int)((last - g.base0 + 64) & ~(int64_t)63) + 64;          // in whole steps, and one more: a tile of 128 keys may start at any step
-        g.dkp = (dk + 63) & ~63; g.dvp = (dv + vtile - 1) / vtile * vtile;
-        const size_t q_rows = (size_t)G * q_tiles * WA_ROWS, scores = q_rows * g.cap * 4, tops = (size_t)G * q_tiles * key_tiles * 4 * WA_ROWS * 4;
-        const size_t qc = 3 * q_rows * g.dkp * 2, kc = 3 * (size_t)G * g.span * g.dkp * 2, vc = 3 * (size_t)G * g.dvp * g.span * 2;
-        CC_REQUIRE(dev, (3 * q_rows + (size_t)3 * G * g.span) * (g.dkp / 8) < ((size_t)1 << 31) && ring < (1 << 30), "window_attention: too many rows");
-        rc = cc_pool_alloc(dev, scores + tops + qc + kc + vc, &Sp, &cls);   // every part is a multiple of 512 bytes
-        if (rc) return rc;
-        uint8_t *base = (uint8_t*)Sp, *qp3 = base + scores + tops, *kp3 = qp3 + qc, *vp3 = kp3 + kc;
-        const int vec = dk % 4 == 0 && (((uintptr_t)qp | (uintptr_t)fptr(kring)) & 15) == 0;
-        const int64_t row_blocks = ((int64_t)(q_rows + (size_t)G * g.span) * (g.dkp >> 3) + 255) / 256, blocks = row_blocks + (int64_t)(g.span >> 6) * (g.dvp >> 6) * G;
-        WaScores ws{};
-        ws.q = qp; ws.kring = fptr(kring); ws.r1 = r1p; ws.r2 = r2p; ws.S = (float*)base; ws.tops = (float*)(base + scores); ws.g = g; ws.scale = scale;
-        ws.key_tiles = key_tiles; ws.q_tiles = q_tiles; ws.vec = vec;
-        CUtensorMap vmap;
-        rc = cc_make_tmap_bf16(dev, &ws.maps[0], qp3, 3 * (int64_t)q_rows, g.dkp, WA_ROWS);
-        if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &ws.maps[1], kp3, (int64_t)3 * G * g.span, g.dkp, WaScores::N);
-        if (rc == CC_OK) rc = cc_make_tmap_bf16(dev, &vmap, vp3, (int64_t)3 * G * g.dvp, g.span, vtile);
-        if (rc == CC_OK) {
-            cc_launch_pdl(dev, wa_cut_kernel, (unsigned)blocks, 256, 0, qp, fptr(kring), vptr, qp3, kp3, vp3, g, q_tiles, (unsigned)row_blocks, (int)(g.base0 % ring), (int)(oldest - g.base0), vec);
-            dev->launches++;
-            rc = sg_launch(dev, ws, (int64_t)key_tiles * q_tiles * G);
-        }
-        auto values = [&](auto wv) {
-            wv.maps[0] = vmap; wv.S = ws.S; wv.tops = ws.tops; wv.vring = vptr; wv.sink = sinkp; wv.o = (float*)o->base; wv.g = g; wv.key_tiles = key_tiles; wv.q_tiles = q_tiles;
-            return sg_launch<decltype(wv), true>(dev, wv, (int64_t)(g.dvp / vtile) * q_tiles * G);
-        };
-        if (rc == CC_OK) rc = vtile == 128 ? values(WaValues<2>{}) : values(WaValues<1>{});
-        cc_pool_free(dev, Sp, cls);
-        return rc;
-    }
-    rc = cc_pool_alloc(dev, (size_t)T * H * g.cap * 4, &Sp, &cls);
-    if (rc) return rc;
-    if (rows_smem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(wa_scores_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem); if (e != cudaSuccess) { cc_pool_free(dev, Sp, cls); return cc_fail(dev, CC_ERR_CUDA, "window_attention: %s", cudaGetErrorString(e)); } }
-    cc_launch_pdl(dev, wa_scores_row_kernel, dim3((unsigned)((maxn + 15) / 16), (unsigned)T, (unsigned)(G * ((R + WS_HEADS - 1) / WS_HEADS))), 256, rows_smem, qp, fptr(kring), (float*)Sp, g, scale, r1p, r2p);
-    dev->launches++;
-    cudaError_t e = RB == 8 ? wa_launch_slices<8>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap)
-                  : RB == 4 ? wa_launch_slices<4>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap)
-                  : RB == 2 ? wa_launch_slices<2>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap)
-                            : wa_launch_slices<1>(dev, (const float*)Sp, vptr, (float*)o->base, g, sinkp, slices_smem, slice_cap);
-    if (e != cudaSuccess) { cc_pool_free(dev, Sp, cls); return cc_fail(dev, CC_ERR_CUDA, "window_attention: %s", cudaGetErrorString(e)); }
-    cc_pool_free(dev, Sp, cls);
-    CC_LAUNCH_CHECK(dev);
-    return CC_OK;
+    if (few_rows) return wa_by_rows(dev, g, c);
+    CC_REQUIRE(dev, ring < (1 << 30), "window_attention: too many rows");
+    bool room = true;
+    rc = wa_by_tiles(dev, g, c, &room);
+    return !room && can_rows ? wa_by_rows(dev, g, c) : rc;
 }
 extern "C" CC_API int cc_window_attention_sink(cc_device* dev, const cc_view* q, const cc_view* qnw, float eps, const cc_view* kring, const cc_view* vring, int64_t pos0,
                                                int32_t H, int32_t G, int32_t dk, int32_t dv, int32_t window, float scale, const cc_view* r1, const cc_view* r2,

@@ -219,6 +219,49 @@ def test_attention_scores_of_operands_that_use_all_their_bits(dev, bits):
     assert np.abs(got - want).max() <= 0.25 * s * (2.0 ** -24 + 2 * 2.0 ** -23 + 2.0 ** -24) + 4 * 2.0 ** -24
 
 
+@pytest.mark.parametrize("T,pos0,H,G,d,window,sink", [
+    (1, 300, 80, 80, 64, 0, False),               # a decoded token of more heads than 64
+    (1, 500, 128, 4, 64, 200, True),              # .. of many heads a key head: four reads of the cache
+    (2, 250, 64, 8, 80, 0, False),                # two queries, the last count that goes row by row
+    (1, 40000, 8, 1, 64, 0, True),                # a slice of keys that shared memory does not hold: chunks
+    (2, 90000, 3, 1, 32, 0, False),               # .. of the kernel that takes four heads together; queries that see different numbers of keys
+])
+def test_attention_of_few_queries(dev, T, pos0, H, G, d, window, sink):
+    from crabml_b200 import seqops
+    rng = np.random.default_rng(H)
+    n = pos0 + T
+    q, k, v = (rng.standard_normal((r, h, d)).astype(np.float32) for r, h in ((T, H), (n, G), (n, G)))
+    k[n // 2:] *= 1.5                             # larger scores behind smaller ones
+    sk = rng.standard_normal(H).astype(np.float32) if sink else None
+    kt, vt, st = tensor(dev, k.reshape(n, -1)), tensor(dev, v.reshape(n, -1)), None if sk is None else tensor(dev, sk)
+
+    def call(a, b):
+        qt, launches = tensor(dev, q[a:b].reshape(b - a, -1)), dev.launch_count()
+        out = seqops.masked_attention(qt, kt, vt, pos0 + a, H, G, d, d, d ** -0.5, window=window, sink=st)
+        assert dev.launch_count() - launches == 2         # scores and values, and no cut of the cache in front of them
+        return out.export().reshape(b - a, H, d)
+    got = call(0, T)
+    # a score's error moves its weight by as much, the weights' and sums' roundings are a few 2^-24 each: 1e-5 of the values' size
+    assert np.abs(got - attend(q, k, v, d ** -0.5, pos0, window, 0, 0.0, sk)).max() <= 1e-5
+    for t in range(T):                            # a row's bits do not depend on what else the call carries
+        np.testing.assert_array_equal(call(t, t + 1)[0].view(np.uint32), got[t].view(np.uint32))
+
+
+def test_attention_of_many_rows_over_a_long_cache_takes_its_heads_in_groups(dev):
+    """16 heads over 40,000 keys: 820 MB of scores and cut planes where the scores of 33 queries take 84"""
+    from crabml_b200 import seqops
+    T, pos0, H, d = 33, 40000, 16, 64
+    rng = np.random.default_rng(0)
+    n = pos0 + T
+    q, k, v = (rng.standard_normal((r, H, d)).astype(np.float32) for r in (T, n, n))
+    t = [tensor(dev, x.reshape(x.shape[0], -1)) for x in (q, k, v)]
+    launches = dev.launch_count()
+    out = seqops.masked_attention(*t, pos0, H, H, d, d, d ** -0.5)
+    assert dev.launch_count() - launches == 6     # two groups: cut, scores, values
+    got = out.export().reshape(T, H, d)
+    assert np.abs(got - attend(q, k, v, d ** -0.5, pos0, 0, 0, 0.0, None)).max() <= 1e-5
+
+
 # ---- a few activation rows against one quantised matrix ---------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("t", [oc.Q4_K, oc.Q5_K, oc.Q6_K])
 @pytest.mark.parametrize("m,k,b", [(1, 256, 2), (33, 1024, 3), (40, 2816, 8), (257, 4096, 9), (17, 14336, 31), (16, 40960, 5)])

@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) split_gemm_kernel(const __grid_
             if (!p.tile(index, rank, tile)) continue;
             const int steps = tile.steps, half = tile.half;
             if (P::SHARED) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the sums that met in the stages, before TMA writes there again
                 __syncthreads();
                 if (*(volatile int*)&sh.fail) break;
                 p.setup(tile, ps);

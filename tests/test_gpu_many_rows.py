@@ -262,6 +262,24 @@ def test_attention_of_many_rows_over_a_long_cache_takes_its_heads_in_groups(dev)
     assert np.abs(got - attend(q, k, v, d ** -0.5, pos0, 0, 0, 0.0, None)).max() <= 1e-5
 
 
+@pytest.mark.parametrize("pos0,window", [(0, 0), (300, 0), (300, 257), (1000, 700)])
+def test_attention_of_more_tiles_than_ctas(dev, pos0, window):
+    """A CTA walks over several tiles of scores and of values, of odd and even numbers of steps, skipped ones among them; an infinity in a late one stays there."""
+    from crabml_b200 import seqops
+    T, H, dk, dv = 512, 16, 192, 200
+    rng = np.random.default_rng(pos0 + window)
+    n = pos0 + T
+    q, k, v = (rng.standard_normal((r, H, d)).astype(np.float32) for r, d in ((T, dk), (n, dk), (n, dv)))
+    v[n - 20, H - 1, 3] = np.inf
+    got = seqops.masked_attention(tensor(dev, q.reshape(T, -1)), tensor(dev, k.reshape(n, -1)), tensor(dev, v.reshape(n, -1)), pos0, H, H, dk, dv, dk ** -0.5, window=window).export().reshape(T, H, dv)
+    bad = np.zeros(got.shape, bool)
+    bad[T - 20:, H - 1, 3] = True
+    assert np.isposinf(got[bad]).all() and np.isfinite(got[~bad]).all()
+    v[n - 20, H - 1, 3] = 0.0
+    want = attend(q, k, v, dk ** -0.5, pos0, window, 0, 0.0, None)
+    assert np.abs(got - want)[~bad].max() <= 1e-5
+
+
 # ---- a few activation rows against one quantised matrix ---------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("t", [oc.Q4_K, oc.Q5_K, oc.Q6_K])
 @pytest.mark.parametrize("m,k,b", [(1, 256, 2), (33, 1024, 3), (40, 2816, 8), (257, 4096, 9), (17, 14336, 31), (16, 40960, 5)])

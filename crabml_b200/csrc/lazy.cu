@@ -45,7 +45,7 @@ struct GraphEntry { cudaGraphExec_t exec = nullptr; size_t dyn_bytes = 0; uint64
 struct LazyState {
     std::vector<LOp> q;
     std::unordered_map<cc_buf*, int> qrefs;
-#define LZ_DYN_SLOTS 8                               // tokens the host may run ahead of the GPU (absorbs host scheduling hiccups)
+#define LZ_DYN_SLOTS 16                              // the host may run eight tokens of two parts ahead of the GPU (absorbs host scheduling hiccups)
     uint8_t* dyn_host[LZ_DYN_SLOTS] = {nullptr};   // pinned, rotated so the host can build tokens t+1.. while t runs
     cudaEvent_t dyn_ev[LZ_DYN_SLOTS] = {nullptr};
     int dyn_slot = 0;

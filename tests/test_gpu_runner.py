@@ -135,6 +135,40 @@ def test_lazy_fused_graph_mode_golden_generation(fixture_path, fname, text, ids,
         dev.close()
 
 
+def test_the_host_runs_eight_long_tokens_ahead_of_the_gpu():
+    """Six layers run as two launches a token.  Eight tokens are recorded and submitted while the GPU is still at work on what was queued before them: had the host
+    waited for a slot of per-token values, that work and the first tokens would be over when it comes back."""
+    import time
+    from crabml_b200 import CudaTensor, runner as R
+    from tests.blockgen import random_weight
+    dev = make_device(lazy=2)
+    try:
+        r = R.LlamaRunner(dev, *(lambda c: (c, R.synthetic_weights(dev, c, oc.Q8_0, oc.Q8_0, seed=3)))(R.LlamaConfig(4, 2, 6, 256, 512, 600, 512, 1e-5, 64)), 64)
+        w = CudaTensor.from_cpu(random_weight(oc.Q8_0, 4096, 4096, np.random.default_rng(0), 0.02), [4096, 4096], oc.Q8_0, dev)
+        x = CudaTensor.new(np.ones((4096, 4096), np.float32), [4096, 4096], dev)
+
+        def ahead(products):
+            for _ in range(products):
+                w.matmul_vec(x)
+            dev.flush()
+            t0 = time.perf_counter()
+            for p in range(8):
+                r.forward([1 + p], p, export=False)
+            t1 = time.perf_counter()
+            dev.synchronize()
+            return t1 - t0, time.perf_counter() - t1
+        launches = dev.launch_count()
+        r.forward([1], 0, export=False)
+        assert dev.launch_count() - launches == 2
+        for _ in range(3):
+            ahead(20)                                      # plans, buffers and scratch are there now
+        submit, left = min((ahead(300) for _ in range(3)), key=lambda t: t[0])
+        assert submit < 0.5 * left, (submit, left)
+        r.close()
+    finally:
+        dev.close()
+
+
 def test_lazy_mode_matches_eager_ops_through_python_mirror(fixture_path):
     """The recorder is transparent for arbitrary call sequences: the Python replay (not the C++ runner), with debug
     taps forcing flushes at odd places, gives the reference's golden text."""

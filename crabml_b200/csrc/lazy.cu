@@ -40,7 +40,7 @@ struct LOp {
 // on every hit (a colliding key must re-capture, never replay another plan's baked pointers); `last_use` drives the LRU bound.
 struct GraphEntry { cudaGraphExec_t exec = nullptr; size_t dyn_bytes = 0; uint64_t launches = 0; MkPhase* phases_dev = nullptr;
                     std::vector<uint64_t> sig; uint64_t last_use = 0; int mega_variant = 0; };
-#define LZ_MAX_GRAPHS 64                             // cached token graphs per device (a decode loop needs 2-4)
+#define LZ_MAX_GRAPHS 128                            // cached token graphs per device: 64 token shapes (sequences with caches of their own) of two parts each
 
 struct LazyState {
     std::vector<LOp> q;

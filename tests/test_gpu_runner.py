@@ -169,6 +169,26 @@ def test_the_host_runs_eight_long_tokens_ahead_of_the_gpu():
         dev.close()
 
 
+def test_many_sequences_in_turn_replay_their_graphs():
+    """Forty runners with caches of their own, a token each in turn: every one has a plan per part of its token, and all of them stay cached."""
+    from crabml_b200 import runner as R
+    conf = R.LlamaConfig(4, 2, 6, 256, 512, 600, 512, 1e-5, 64)
+    dev = make_device(lazy=2)
+    try:
+        w = R.synthetic_weights(dev, conf, oc.Q8_0, oc.Q8_0, seed=3)
+        runners = [R.LlamaRunner(dev, conf, w, 16) for _ in range(40)]
+        captures = []
+        for p in range(4):
+            for r in runners:
+                r.forward([1 + p], p)
+            captures.append(dev.lazy_stats()["graph_captures"])
+        assert captures[3] == captures[1], captures
+        for r in runners:
+            r.close()
+    finally:
+        dev.close()
+
+
 def test_lazy_mode_matches_eager_ops_through_python_mirror(fixture_path):
     """The recorder is transparent for arbitrary call sequences: the Python replay (not the C++ runner), with debug
     taps forcing flushes at odd places, gives the reference's golden text."""

@@ -126,8 +126,8 @@ int cc_lazy_record(cc_device* dev, int kind, const cc_view* a, const cc_view* b,
     LazyState* lz = dev->lz;
     // a long token starts while the rest of it is still being recorded: at the first copy of a layer's input (attention's or the feed-forward's) behind
     // LZ_HEAD_OPS ops the queue so far runs, once per token -- the GPU used to wait some 180 us for the 840 ops of a 7B token.  No fused
-    // pattern spans that copy, so the phases are the same ones in two kernels.  Ranks that exchange keep one part: their launches stay paired
-    if (kind == L_DUP && !lz->head_done && lz->q.size() >= LZ_HEAD_OPS && !cc_comm_dev(dev) && a && a->ndim <= 2 && view_rows(a) == 1) {
+    // pattern spans that copy, so the phases are the same ones in two kernels.  Ranks that exchange keep one part: their launches stay paired.  So does a profiled token
+    if (kind == L_DUP && !lz->head_done && lz->q.size() >= LZ_HEAD_OPS && !cc_comm_dev(dev) && !lz->prof_dev && a && a->ndim <= 2 && view_rows(a) == 1) {
         lz->head_done = true;
         int rc = cc_lazy_flush_part(dev, false);
         if (rc) return rc;

@@ -2,6 +2,8 @@
 golden generations of the reference (llama2.rs:673-703), bit-identical logits in exact_order mode, and a
 Llama-2-7B-SHAPED layer on the synthetic weights bench.py uses (BASELINE.json configs 2-4 at full size)."""
 import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -187,6 +189,29 @@ def test_many_sequences_in_turn_replay_their_graphs():
             r.close()
     finally:
         dev.close()
+
+
+PROFILE_CHILD = r"""
+import ctypes as C, os, sys
+sys.path.insert(0, %r)
+os.environ["CRABML_MEGA_PROF"] = "1"
+from crabml_b200 import CudaTensorDevice, capi, runner as R
+dev = CudaTensorDevice(0, lazy=2)
+conf = R.LlamaConfig(4, 2, 6, 256, 512, 600, 512, 1e-5, 64)
+r = R.LlamaRunner(dev, conf, R.synthetic_weights(dev, conf, capi.Q8_0, capi.Q8_0, seed=3), 16)
+for p in range(4):
+    r.forward([1 + p], p)
+CAP = 8 * 4097
+ts, ty, n = (C.c_uint64 * CAP)(), (C.c_int32 * CAP)(), C.c_int32(0)
+dev.check(dev.lib.cc_lazy_mega_profile(dev.handle, ts, ty, CAP, C.byref(n)))
+print("attention phases", sum(t == 32 for t in ty[:n.value]))
+r.close(); dev.close()
+""" % os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def test_the_phase_profile_covers_a_whole_token():
+    p = subprocess.run([sys.executable, "-c", PROFILE_CHILD], capture_output=True, text=True, timeout=120)
+    assert "attention phases 6" in p.stdout, p.stdout + p.stderr
 
 
 def test_lazy_mode_matches_eager_ops_through_python_mirror(fixture_path):

@@ -350,7 +350,6 @@ static __device__ MK_GENERIC_ATTR void phase_matvec_generic(const MkPhase& ph, u
     if (stamp1) stamp1[4] = globaltimer_ns();
     if (ph.orig && blockIdx.x == 0)                                     // Tensor::dup of the un-normalised row (llama2.rs:227,607)
         for (int i = threadIdx.x; i < (k >> 2); i += MK_THREADS) ((float4*)ph.orig)[i] = ((const float4*)s_x)[i];
-    const CcDivBy by_rms(rms);
     const int q_at = T::act_at(lane >> 1) * 16 + (lane & 1) * 8;
     for (int sb = warp; sb < (k >> 8); sb += MK_WARPS) {                // one warp per 256-element super-block (buf_q8_k.rs:84-131)
         float4 v4[2];
@@ -359,8 +358,7 @@ static __device__ MK_GENERIC_ATTR void phase_matvec_generic(const MkPhase& ph, u
             v4[i] = ((const float4*)s_x)[sb * 64 + lane * 2 + i];
             if (ph.norm_w) {
                 const float4 w4 = ((const float4*)s_w)[sb * 64 + lane * 2 + i];
-                v4[i] = by_rms(v4[i]);
-                v4[i].x *= w4.x; v4[i].y *= w4.y; v4[i].z *= w4.z; v4[i].w *= w4.w;
+                v4[i] = make_float4(v4[i].x / rms * w4.x, v4[i].y / rms * w4.y, v4[i].z / rms * w4.z, v4[i].w / rms * w4.w);
             }
         }
         const float v[8] = {v4[0].x, v4[0].y, v4[0].z, v4[0].w, v4[1].x, v4[1].y, v4[1].z, v4[1].w};

@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
             const MkPhase& nx = s_phs[(p + 1) & 1];
             if (nx.type == MK_ATTN) at_pre = at_ask(nx, (float*)work, dyn, abar0, R.at_ch);
             // the norm weights of the next prologue were last read a token ago and come from HBM: a line of them per CTA into
-            // L2 now (0.8 % of a 7B token).  Its quotients stay divisions: without their branches (CcDivBy) the k = 11008 phases took 1 us longer
+            // L2 now (0.8 % of a 7B token)
             else if (nx.type == MK_MATVEC && nx.norm_w && threadIdx.x < 8)
                 for (int i = ((int)blockIdx.x * 8 + (int)threadIdx.x) * 32; i < nx.mv.k; i += (int)gridDim.x * 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx.norm_w + i));
         }

@@ -3,27 +3,6 @@
 #pragma once
 #include "common.cuh"
 
-// v / d rounded as IEEE asks, for many v and one d: y = 1 / d correctly rounded, then v y and twice q + (v - q d) y.  v y is 2 ulp off at most, the first
-// step makes it faithful, and a step from a faithful quotient with a correctly rounded reciprocal rounds correctly (P. Markstein, IBM J. Res. Dev. 34, 1990).
-// The remainders are exact while nothing leaves the normal range, so d and v outside 2^-60 .. 2^60 are divided.  5 instructions without a branch, which
-// overlap over the values; a division tests its operands and may branch, and its neighbours wait (tests/test_gpu_many_rows.py: the bits).
-struct CcDivBy {
-    float d, y;
-    bool ok;
-    __device__ __forceinline__ explicit CcDivBy(float by) : d(by), y(1.0f / by), ok(in_range(by)) {}
-    static __device__ __forceinline__ bool in_range(float v) { return fabsf(v) >= 0x1p-60f && fabsf(v) <= 0x1p60f; }
-    __device__ __forceinline__ float quotient(float v) const {
-        float q = v * y;
-        q = __fmaf_rn(__fmaf_rn(-q, d, v), y, q);
-        return __fmaf_rn(__fmaf_rn(-q, d, v), y, q);
-    }
-    // four quotients
-    __device__ __forceinline__ float4 operator()(const float4& v) const {
-        if (ok && in_range(v.x) && in_range(v.y) && in_range(v.z) && in_range(v.w)) return make_float4(quotient(v.x), quotient(v.y), quotient(v.z), quotient(v.w));
-        return make_float4(v.x / d, v.y / d, v.z / d, v.w / d);
-    }
-};
-
 // Q8_K (buf_q8_k.rs:84-131): one warp quantises one 256-element super-block; lane l holds the elements 8l .. 8l+7 in v.
 //   scale = -128 / x[first argmax |x|],  q = min(round_half_away(scale * x), 127),  d = 1 / scale,  bsums[j] = sum of 16 quants
 // qs: where this lane's 8 quants go, d: the super-block's scale, bsums: its 16 sums (global or shared memory).

@@ -115,7 +115,8 @@ void cc_lazy_destroy(cc_device* dev) {
 
 static int cc_lazy_flush_part(cc_device* dev, bool whole);
 #define LZ_HEAD_OPS 64                               // three layers: work for the GPU until the rest of a 7B token is recorded and fused.  16 tokens with 12 / 22 / 40 / 64 ops,
-                                                     // ms: 7B 41.2 / 40.6 / 40.5 / 39.8 (42.0 in one part), 15M 5.46 / 5.24 / 5.03 / 5.13 (5.93)
+                                                     // ms: 7B 41.2 / 40.6 / 40.5 / 39.8 (42.0 in one part), 15M 5.46 / 5.24 / 5.03 / 5.13 (5.93), four 7B layers of
+                                                     // K-quants 7.30 / 7.15 / 7.35 / 7.53 (7.97): a short token would go earlier, one count for all costs it 5 %
 static int64_t view_rows(const cc_view* v) { return v->ndim < 2 ? 1 : v->shape[0]; }
 
 // ---- recording ---------------------------------------------------------------------------------------------------

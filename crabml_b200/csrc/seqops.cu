@@ -1,11 +1,13 @@
 // seqops.cu -- sequence-mixing and normalisation ops of include/crabml_seqops.h: norms on the sublayer output, the short causal
 // convolution, the gated delta rule, and sliding-window attention over a ring cache.  Everything here is computed in 32-bit floats
-// (explicit fmaf; expf / logf / log1pf of the CUDA math library, not the fast intrinsics).
+// (explicit fmaf; expf / logf / log1pf of the CUDA math library, not the fast intrinsics); attention of many rows takes its two products on the tensor
+// cores from 32-bit operands cut into bfloat16 numbers, with an error no larger than 32-bit sums have (split_gemm.cuh).
 //
 // One property every kernel keeps: the value computed for a token depends only on that token's inputs and on the state / cache
 // contents, never on how many tokens the call carries or where the token sits in the call.  Sums run in a fixed order per output
-// (a warp's lane-strided partial sums and the xor butterfly, or one thread's sequential loop), so prefill, chunked prefill and
-// token-by-token decoding give the same bits for the recurrent layers and the same bits per (query, key set) for attention.
+// (a warp's lane-strided partial sums and the xor butterfly, one thread's sequential loop, or steps at fixed positions), so prefill, chunked prefill and
+// token-by-token decoding give the same bits for the recurrent layers.  Attention has two ways, for calls of many rows and of few: a (query, key set) has the
+// same bits in all calls that go one way, and differs between the two by the rounding of its sums.
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -770,7 +772,9 @@ extern "C" CC_API int cc_kv_ring_append(cc_device* dev, const cc_view* kring, co
 //   1. WaScores: S[row][j] = (q_row . k_j) * scale - r1 ln(1 + r2 (i - j)), -inf where masked, and the largest score of each row of the tile
 //   2. WaValues: out[row][d] = sum_j exp(S[row][j] - top) v[j][d] / (sum_j exp(S[row][j] - top) + sink); the weights are made while the operand is staged
 // A row is one (query, head); a tile's rows are the R = n_heads / n_kv heads of one key/value head for 128 / R consecutive queries, so that keys and
-// values are read once per tile and not once per (query, head).  A decoded token takes the two kernels for few rows below.
+// values are read once per tile and not once per (query, head).  Decoded tokens take the two kernels for few rows below.
+// Error against 64 bits, 512 queries of 16 heads over a window of 1024 keys of 128: 3.5e-7 of the values' size (32-bit sums on the CUDA cores: 7e-7); 58 us on
+// the device where those took 204.
 // The keys of a tile start at a multiple of 64 positions, a score is one sum over dk, a row's weights are added in an order that the positions of the keys
 // alone decide (masked keys add an exact 0), and the value sum goes by steps of 64 positions, even ones and odd ones: a query's result does not
 // depend on where the call starts or what else it carries, and differs between a prompt pass and a decoded token only by the rounding of those sums.

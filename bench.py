@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py -- decode tokens/s of the crabml CUDA backend on synthetic Llama-2-7B shapes (BASELINE.json metric).
+"""bench.py -- decode tokens/s of the crabml CUDA backend on synthetic Llama-2-7B shapes (the headline metric).
 
 One "step" = one decoded token = one pass of the hot path (225 quantized matvecs + the small ops around them).
   value : device-resident throughput (weights + KV in HBM, no host<->device traffic inside the timed region)
@@ -33,7 +33,7 @@ WORKLOADS = {
     "llama2-7b-q4_0-q6k": ("LLAMA2_7B", "Q4_0", "Q6_K"),
     "llama2-7b-q4_k": ("LLAMA2_7B", "Q4_K", "Q6_K"),
     "tinyllamas-15m-q8_0": ("TINYLLAMAS_15M", "Q8_0", "Q8_0"),
-    # BASELINE.json config 5: the dense matmuls of a 4096-token prefill (TMA + tcgen05 path, csrc/prefill_gemm.cu); see run_prefill
+    # the dense matmuls of a 4096-token prefill (TMA + tcgen05 path, csrc/prefill_gemm.cu); see run_prefill
     "mistral-7b-q8_0-prefill": ("MISTRAL_7B", "Q8_0", "Q8_0"),
     "llama2-7b-q8_0-prefill": ("LLAMA2_7B", "Q8_0", "Q8_0"),
     # the Zatorax family at layer sizes of a real model (random weights), beside a llama stack of equal size; see run_zatorax
@@ -471,7 +471,7 @@ def run_b200(args, rank, world, local_rank):
 
 
 def run_prefill(args, rank, world, local_rank):
-    """BASELINE.json config 5: every matmul_vec of a `--prefill-tokens`-token prompt pass (Tensor::matmul_vec with a (b, k) rhs) on the
+    """Every matmul_vec of a `--prefill-tokens`-token prompt pass (Tensor::matmul_vec with a (b, k) rhs) on the
     tensor-core path: per layer wq, wk, wv, wo, ffn_gate, ffn_up, ffn_down on (b, k) activations, then the classifier on the last row.
     A step = all 225 matmuls once.  This is the DENSE part of a prefill (58 of ~63 TFLOP for Mistral-7B at 4096 tokens); attention,
     norms and RoPE of a batched forward are not part of this workload (the reference has no batched forward: llama2.rs:111-139 walks

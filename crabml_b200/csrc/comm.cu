@@ -1,4 +1,4 @@
-// comm.cu -- the exchange step of the row/column-sharded decode path (SURVEY §8e): one allreduce(sum) of a [dim] f32
+// comm.cu -- the exchange step of the row/column-sharded decode path: one allreduce(sum) of a [dim] f32
 // row after `wo` and after `ffn_down`, one allgather of the classifier's logit slices.  One process per GPU.
 //
 // The reference has no multi-device path; what shards is its thread-pool split of output rows (matmul_vec.rs:41-76).

@@ -18,7 +18,7 @@ int cc_fail(cc_device* dev, int code, const char* fmt, ...) {
     return code;
 }
 
-// ---- type facts (crabml-core/src/gguf.rs:86-108; block sizes SURVEY Appendix A) ------------------
+// ---- type facts (crabml-core/src/gguf.rs:86-108) ------------------
 int cc_block_elems(int t) {
     switch (t) {
     case CC_F32: case CC_F16: case CC_BF16: case CC_I32: return 1;

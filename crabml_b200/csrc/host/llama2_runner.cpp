@@ -26,7 +26,7 @@ struct ccr_runner {
     std::string last_error;
     ~ccr_runner() { if (pinned_logits) cc_host_free(dev, pinned_logits); }
 
-    // Sharded decode (SURVEY 8e).  shard_world > 1: this process holds heads [rank*H/N, (rank+1)*H/N) of wq/wk/wv (rows), the
+    // Sharded decode.  shard_world > 1: this process holds heads [rank*H/N, (rank+1)*H/N) of wq/wk/wv (rows), the
     // matching COLUMNS of wo, hidden_local rows of gate/up and columns of down, vocab/N rows of the classifier; the replay is
     // the reference's op order with one all_reduce_sum after wo and after ffn_down and one all_gather of the logits.
     int world() const { return conf.shard_world > 1 ? conf.shard_world : 1; }

@@ -1,6 +1,6 @@
 // lazy.cu -- lazy mode: record the trait calls of one forward(), fuse, replay as a CUDA graph.
 //
-// The reference's Tensor API is eager: ~31 calls per layer, ~1000 per token (SURVEY §3.2), each a separate launch in
+// The reference's Tensor API is eager: ~31 calls per layer, ~1000 per token, each a separate launch in
 // eager mode.  profiles/r01c shows that per-launch overhead, not kernel bodies, is what caps decode.  In lazy mode the
 // SAME C-ABI calls only append to a queue (after the same argument checks); the queue is executed at the first call that
 // needs a result on the host (export / debug tap / synchronize -- the reference synchronises only there too, llama2.rs:209):

@@ -1,5 +1,5 @@
 // matvec.cu -- THE hot path: C[b,m] = sum_k W[m,k] * x[b,k] with W in GGUF quant blocks
-// (SURVEY §8a rows a1, a2, a6-a11;  reference: primitives/matmul_vec.rs:26-78 -> buf/buf_q*.rs vec_dot_*).
+// (reference: primitives/matmul_vec.rs:26-78 -> buf/buf_q*.rs vec_dot_*).
 //
 // Design (HBM-bound integer/byte work -- no tensor cores on purpose):
 //   * one warp per output row; weight bytes are streamed exactly once with 16-byte LDG.128

@@ -1,4 +1,4 @@
-// ops.cu -- the small ops around the matvec (SURVEY §8a rows a12-a19), one launch per trait call.
+// ops.cu -- the small ops around the matvec, one launch per trait call.
 // Compiled with -fmad=false / IEEE div+sqrt so that every op reproduces the reference's f32
 // arithmetic; only reduction ORDER differs (the canonical 512-thread tree of common.cuh instead of sequential).
 #include "common.cuh"

@@ -1,4 +1,4 @@
-// quantize.cu -- on-the-fly activation quantisation (SURVEY §8a rows a3-a5).
+// quantize.cu -- on-the-fly activation quantisation.
 //   Q8_0: buf_q8_0.rs:87-134   d = max|x|/127 (f32), q = trunc(x / d)   (TRUNCATION, quirk B1)
 //   Q8_1: buf_q8_1.rs:90-129   q = trunc(clamp(x/d,-128,127)), s = d * sum(q) stored f16
 //   Q8_K: buf_q8_k.rs:84-131   scale = -128/max_signed, q = min(round_half_away(scale*x),127), d = 1/scale

@@ -1,6 +1,6 @@
 // repack.cu -- GGUF AoS blocks <-> device planes, row dequantisation (copy_rows_from), synthetic weights.
 //
-// Block field orders follow the reference structs (SURVEY Appendix A):
+// Block field orders follow the reference structs:
 //   Q8_0 buf_q8_0.rs:8-13 | Q4_0 buf_q4_0.rs:10-15 | Q4_1 buf_q4_1.rs:10-16 | Q5_0 buf_q5_0.rs:13-19
 //   Q5_1 buf_q5_1.rs:10-17 | Q2_K buf_q2_k.rs:17-28 | Q3_K buf_q3_k.rs:19-30 | Q4_K buf_q4_k.rs:14-21
 //   Q5_K ggml order d,dmin,scales,qh,qs (the reference struct buf_q5_k.rs:15-21 is wrong, B9)
@@ -145,7 +145,7 @@ int cc_launch_dequant_rows(cc_device* dev, const cc_buf* src, const int64_t* row
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Synthetic weights (SURVEY §8d config 3/4): counter-based splitmix64 over (seed, tensor, byte index)
+// Synthetic weights: counter-based splitmix64 over (seed, tensor, byte index)
 // written in GGUF block layout, f16 scale fields overwritten with values uniform in [0.75,1.25)*scale.
 // oracle/synth.py holds the identical CPU generator (checked bit for bit in tests/test_gpu_synth.py).
 // ---------------------------------------------------------------------------------------------------

@@ -1,5 +1,5 @@
-// vecdot.cuh -- per-row dot products of every GGUF weight type against the on-the-fly quantised activation (SURVEY 8a rows a6-a11;
-// reference: buf/buf_q*.rs vec_dot_*).  One warp per output row: `T::row_dot` returns this lane's partial, the caller finishes with
+// vecdot.cuh -- per-row dot products of every GGUF weight type against the on-the-fly quantised activation
+// (reference: buf/buf_q*.rs vec_dot_*).  One warp per output row: `T::row_dot` returns this lane's partial, the caller finishes with
 // the xor-butterfly warp_sum.  Shared by the eager kernel (matvec.cu) and the generic MATVEC phase of the megakernel (mega.cu), so
 // both produce the same bits.  T::stage_act copies the activation scratch (quantize.cu layout) into shared memory.
 #pragma once

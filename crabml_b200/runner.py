@@ -1,6 +1,6 @@
 """Python handle on the C++ Llama2Runner replay (crabml_b200/csrc/host/llama2_runner.cpp) plus the two ways
 this repo builds a model: from a GGUF file (python `gguf` reader -> Tensor::from_cpu, the quantized relaxation of
-crabml-llama2/src/model.rs:817-837) and synthetic weights generated on the device (SURVEY §8d configs 3-5)."""
+crabml-llama2/src/model.rs:817-837) and synthetic weights generated on the device."""
 from __future__ import annotations
 
 import ctypes as C
@@ -34,7 +34,7 @@ LLAMA2_7B = LlamaConfig(32, 32, 32, 4096, 11008, 4096, 32000, 1e-5, 128)
 MISTRAL_7B = LlamaConfig(32, 8, 32, 4096, 14336, 4096, 32000, 1e-5, 128)
 TINYLLAMAS_15M = LlamaConfig(6, 6, 6, 288, 768, 256, 32000, 1e-5, 48)
 
-# GGUF block bytes / elements (SURVEY Appendix A) -- for algorithmic byte accounting
+# GGUF block bytes / elements -- for algorithmic byte accounting
 BLOCK = {capi.F32: (4, 1), capi.F16: (2, 1), capi.Q4_0: (18, 32), capi.Q4_1: (20, 32), capi.Q5_0: (22, 32), capi.Q5_1: (24, 32),
          capi.Q8_0: (34, 32), capi.Q2_K: (84, 256), capi.Q3_K: (110, 256), capi.Q4_K: (144, 256), capi.Q5_K: (176, 256),
          capi.Q6_K: (210, 256), capi.Q8_K: (292, 256)}
@@ -112,7 +112,7 @@ class LlamaRunner:
             self.device.lib.ccr_runner_destroy(self.handle)
             self.handle = None
 
-    # algorithmic weight bytes streamed per decoded token (SURVEY §8d): every matmul weight once (THIS rank's shards)
+    # algorithmic weight bytes streamed per decoded token: every matmul weight once (THIS rank's shards)
     def weight_bytes_per_token(self):
         w = self.weights
         total = 0
@@ -173,7 +173,7 @@ def load_gguf(path: str, device: CudaTensorDevice, shard=None, f16_kv=False):
     return conf, w, tok
 
 
-# central f16 scale of synthetic blocks so that a dequantized row has sigma_w ~ 1/sqrt(k) (SURVEY §8d-3)
+# central f16 scale of synthetic blocks so that a dequantized row has sigma_w ~ 1/sqrt(k)
 _Q_SIGMA = {capi.Q8_0: 73.9, capi.Q4_0: 4.61, capi.Q4_1: 4.61, capi.Q5_0: 9.23, capi.Q5_1: 9.23,
             capi.Q2_K: 1.12 * 8.0, capi.Q3_K: 2.29 * 18.5, capi.Q4_K: 4.61 * 31.5, capi.Q5_K: 9.23 * 31.5, capi.Q6_K: 18.5 * 73.9, capi.Q8_K: 73.9}
 

@@ -1,4 +1,4 @@
-"""Shard plan of the row/column-sharded decode path (SURVEY §8e) and the GGUF byte slicing that goes with it.
+"""Shard plan of the row/column-sharded decode path and the GGUF byte slicing that goes with it.
 
 The reference is single-device; its unit of parallelism is the output row of matmul_vec (matmul_vec.rs:41-76 deals rows
 to the thread pool).  Across N GPUs the same unit gives (Megatron pairing, in GGUF terms):
@@ -20,7 +20,7 @@ from dataclasses import dataclass
 
 import numpy as np
 
-# GGUF (bytes per block, elements per block), SURVEY Appendix A
+# GGUF (bytes per block, elements per block)
 BLOCK = {0: (4, 1), 1: (2, 1), 2: (18, 32), 3: (20, 32), 6: (22, 32), 7: (24, 32), 8: (34, 32), 9: (36, 32),
          10: (84, 256), 11: (110, 256), 12: (144, 256), 13: (176, 256), 14: (210, 256), 15: (292, 256)}
 

@@ -164,9 +164,9 @@ CC_API void cc_host_free(cc_device* dev, void* p);
 
 /* ---- test / bench hooks (not part of the trait) ---------------------------------------------- */
 /* quantize an F32 vector exactly as matmul_vec does internally and return the reference-layout
- * activation blocks (Q8_0 / Q8_1 / Q8_K bytes) to the host: parity tests of a3-a5 (SURVEY §8a). */
+ * activation blocks (Q8_0 / Q8_1 / Q8_K bytes) to the host: parity tests of a3-a5. */
 CC_API int cc_test_quantize_activation(cc_device* dev, const cc_view* x, int32_t act_type, void* dst, size_t nbytes);
-/* ---- sharded decode (SURVEY 8e): the exchange step ---------------------------------------------------------
+/* ---- sharded decode: the exchange step ---------------------------------------------------------
  * The reference is single-device; its unit of parallelism is the output row (matmul_vec.rs:41-76 splits rows over
  * the thread pool).  Across GPUs the same split leaves two exchanges per layer: a sum of [dim] partials after the
  * column-split `wo` and `ffn_down`, and a gather of the row-split classifier's logit slices.
@@ -192,7 +192,7 @@ CC_API int cc_tensor_synth_slice(cc_device* dev, const int64_t* shape, int32_t n
                                  uint64_t tensor_id, float scale, int64_t row0, int64_t nrows, int64_t col0,
                                  int64_t ncols, cc_buf** out);
 
-/* synthetic weights generated on device in the device layout (SURVEY §8d config 3): counter-based
+/* synthetic weights generated on device in the device layout: counter-based
  * RNG, identical bytes to tests/synth.py's CPU generator for the same (seed, tensor_id). */
 CC_API int cc_tensor_synth(cc_device* dev, const int64_t* shape, int32_t ndim, int32_t ggml_type,
                     uint64_t seed, uint64_t tensor_id, float scale, cc_buf** out);

@@ -30,7 +30,7 @@ enum oc_type {
 };
 
 /* flags */
-#define OC_BUGCOMPAT      1  /* reproduce reference bugs B7/B9/B10 (SURVEY Appendix B) */
+#define OC_BUGCOMPAT      1  /* reproduce reference bugs B7/B9/B10 */
 #define OC_ORDER_AVX2     2  /* f32 accumulation order of the reference's AVX2 kernels */
 
 int    oc_block_elems(int type);

@@ -1,7 +1,7 @@
 """CPU twin of the on-device synthetic weight generator (crabml_b200/csrc/repack.cu: synth_kernel /
 synth_scales_kernel), implemented in oracle/crabml_oracle.c (oc_synth_blocks).  TEST INFRASTRUCTURE: lets the
-oracle and the CPU baseline run on exactly the weights the GPU synthesised (SURVEY §8d configs 3-5) without
-shipping gigabytes through gpurun.  Bit-equality with the device generator: tests/test_gpu_synth.py."""
+oracle and the CPU baseline run on exactly the weights the GPU synthesised without
+shipping gigabytes to a GPU machine.  Bit-equality with the device generator: tests/test_gpu_synth.py."""
 from __future__ import annotations
 
 import numpy as np

@@ -1,4 +1,4 @@
-"""Per-phase parity of the megakernel (VERDICT r1, item 1b): one Llama-2-7B-shaped decode layer driven through the trait mirror in
+"""Per-phase parity of the megakernel: one Llama-2-7B-shaped decode layer driven through the trait mirror in
 lazy mode 2 with debug taps (`with_name`, cpu_tensor.rs:232-241 -- the reference's own cross-backend check works the same way,
 llama2.rs:768-784).  A tap forces a flush, so the token is cut into several megakernel launches whose outputs are visible:
 

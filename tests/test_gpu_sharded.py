@@ -1,6 +1,6 @@
-"""Sharded decode path on real GPUs (SURVEY §8e).  The one-process tests run the exchange protocol with a world of 1 (the
+"""Sharded decode path on real GPUs.  The one-process tests run the exchange protocol with a world of 1 (the
 peer stores, flag handshake and slot reduction all execute, against this GPU's own window), so they also run on a
-single-GPU box; the N-process test needs >= 2 GPUs (`gpurun --gpus 2 -- python -m pytest tests/test_gpu_sharded.py -m gpu`)."""
+single-GPU box; the N-process test needs >= 2 GPUs (`python -m pytest tests/test_gpu_sharded.py -m gpu`)."""
 import os
 import socket
 import subprocess
@@ -75,7 +75,7 @@ def _free_port():
 def test_two_gpus_sharded_llama_matches_single_gpu():
     import torch
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs >= 2 GPUs (gpurun --gpus 2)")
+        pytest.skip("needs >= 2 GPUs")
     n = min(int(os.environ.get("CRABML_TEST_WORLD", "2")), torch.cuda.device_count())
     cmd = [sys.executable, "-m", "torch.distributed.run", "--nnodes=1", "--nproc-per-node", str(n), "--master-addr", "127.0.0.1",
            "--master-port", str(_free_port()), os.path.join(ROOT, "tests", "sharded_worker.py"), "--mode", "gpu"]

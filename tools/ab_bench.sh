@@ -1,8 +1,8 @@
 #!/bin/bash
-# A/B two builds of libcrabml_cuda.so inside ONE gpurun call (boxes differ by up to 40 %: never compare across calls).
+# A/B two builds of libcrabml_cuda.so inside ONE session (machines differ by up to 40 %: never compare across calls).
 #   usage (on the GPU box):  tools/ab_bench.sh crabml_b200/lib/libcrabml_cuda_A.so crabml_b200/lib/libcrabml_cuda.so [workload] [rounds]
 # Build A from another commit here first:  git stash; python crabml_b200/build.py; cp crabml_b200/lib/libcrabml_cuda.so \
-#   crabml_b200/lib/libcrabml_cuda_A.so; git stash pop; python crabml_b200/build.py     (*.so travels with gpurun, stays out of git)
+#   crabml_b200/lib/libcrabml_cuda_A.so; git stash pop; python crabml_b200/build.py     (*.so stays out of git)
 # Prints value / e2e tok/s per run, alternating A B A B, then the in-kernel phase profile of each (stable to ~1 %).
 A=$1; B=$2; WL=${3:-llama2-7b-q8_0}; N=${4:-2}
 for i in $(seq $N); do

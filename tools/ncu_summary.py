@@ -1,4 +1,4 @@
-"""Key metrics of ncu reports (read here, without a GPU): python tools/ncu_summary.py gpurun_out/*.ncu-rep"""
+"""Key metrics of ncu reports (read here, without a GPU): python tools/ncu_summary.py *.ncu-rep"""
 import csv
 import io
 import subprocess

@@ -1058,223 +1058,7 @@ struct WaValues {
         sg_store_rows<COUNT>(buf, row < 0 ? nullptr : o + row * g.dv + t.c0 + col0, g.dv - t.c0 - col0, g.dv % 4 == 0, v);
     }
 };
-// few rows (decoding): grid (ceil(keys / 16), T, G * head blocks), 256 threads.  The CTA stages up to WS_HEADS queries of (token, key/value head); a
-// warp owns two visible keys and takes their dot products with each of them: lane-strided partial sums, then the butterfly.  A key row is
-// read into registers once for the block's heads (rows longer than WS_KEEP * 32: as far as they fit), and the keys spread over the whole device
-// however few rows the call has.
-#define WS_HEADS 8
-#define WS_KEEP 20
-__global__ void __launch_bounds__(256) wa_scores_row_kernel(const float* __restrict__ q, const float* __restrict__ kring, float* __restrict__ S, WaGeom g, float scale,
-                                                            const float* __restrict__ r1, const float* __restrict__ r2) {
-    pdl_enter();
-    extern __shared__ float wsr_sm[];             // [heads of the block][dk]
-    const int hblocks = (g.R + WS_HEADS - 1) / WS_HEADS;
-    const int t = blockIdx.y, kvh = blockIdx.z / hblocks, h0 = (blockIdx.z % hblocks) * WS_HEADS, nh = min(WS_HEADS, g.R - h0);
-    const int64_t i = g.pos0 + t, lo = wa_lo(g, i);
-    const int lane = threadIdx.x & 31;
-    if (lo + (int64_t)blockIdx.x * 16 > i) return;            // the whole CTA lies behind the last visible key
-    const int64_t ja = lo + (int64_t)blockIdx.x * 16 + (threadIdx.x >> 5), jb = ja + 8;
-    const float* ka = kring + ((ja < i ? ja : i) % g.ring) * g.krs + kvh * g.dk;
-    const float* kb = kring + ((jb < i ? jb : i) % g.ring) * g.krs + kvh * g.dk;
-    float xa[WS_KEEP], xb[WS_KEEP];
-#pragma unroll
-    for (int e = 0; e < WS_KEEP; e++) {
-        const int d = lane + e * 32;
-        xa[e] = d < g.dk ? ka[d] : 0.0f;
-        xb[e] = d < g.dk ? kb[d] : 0.0f;
-    }
-    for (int e = threadIdx.x; e < nh * g.dk; e += 256) wsr_sm[e] = q[((int64_t)t * g.H + kvh * g.R + h0) * g.dk + e];
-    __syncthreads();
-    for (int hr = 0; hr < nh; hr++) {
-        const float* qh = wsr_sm + hr * g.dk;
-        float sa = 0.0f, sb = 0.0f;
-#pragma unroll
-        for (int e = 0; e < WS_KEEP; e++) {
-            const int d = lane + e * 32;
-            if (d < g.dk) { sa = fmaf(qh[d], xa[e], sa); sb = fmaf(qh[d], xb[e], sb); }
-        }
-        for (int d = lane + WS_KEEP * 32; d < g.dk; d += 32) { sa = fmaf(qh[d], ka[d], sa); sb = fmaf(qh[d], kb[d], sb); }
-        sa = warp_sum(sa); sb = warp_sum(sb);
-        const int64_t j = lane ? jb : ja;                     // lane 0 finishes the first key, lane 1 the second
-        if (lane < 2 && j <= i) {
-            const int h = kvh * g.R + h0 + hr;
-            float sc = (lane ? sb : sa) * scale;
-            if (g.softcap > 0.0f) sc = g.softcap * tanhf(sc / g.softcap);
-            if (r1) sc -= r1[h] * log1pf(r2[h] * (float)(i - j));
-            S[((int64_t)t * g.H + h) * g.cap + (j - lo)] = sc;
-        }
-    }
-}
-// few rows (decoding): grid (T * G * head blocks, ceil(dv / 32), WV_SPLIT) in clusters of WV_SPLIT CTAs along z.  A cluster owns 32 value columns of
-// RB query heads of one (token, key/value head), each of its CTAs one contiguous slice of the visible keys: raw scores of the slice -> its
-// largest score, weights relative to it and their sum (a warp per head), then the slice's value rows, each read once for the RB heads
-// (warp w takes the w-th stretch of the slice in ascending order, the warps' sums are added in ascending order).  The slices meet through the
-// cluster's shared memory: rank r finishes the heads r, r + WV_SPLIT, ..., adding the slices in ascending order, each scaled from its own largest
-// score to the common one, the sink with them.  The order depends on the row alone (its number of visible keys), not on T.
-#define WV_SPLIT 8
-#define WV_THREADS 256
-#define WV_WARPS (WV_THREADS / 32)
-// the slices meet: every warp's weighted values of a slice in acc, the slice's largest score and sum of weights in top and sum
-template <int RB>
-__device__ __forceinline__ void wv_finish(const float (&acc)[RB], float* part, float* top, float* sum, float* acc_sm, float* __restrict__ out, const WaGeom& g, const float* __restrict__ sink, int t, int kvh,
-                                          int h0, int nh, int lane, int w) {
-    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-#pragma unroll
-    for (int hr = 0; hr < RB; hr++) part[(w * RB + hr) * 32 + lane] = acc[hr];
-    __syncthreads();
-    for (int hr = w; hr < RB; hr += WV_WARPS) {
-        float a = 0.0f;
-#pragma unroll
-        for (int ww = 0; ww < WV_WARPS; ww++) a += part[(ww * RB + hr) * 32 + lane];
-        acc_sm[hr * 32 + lane] = a;
-    }
-    cluster.sync();
-    for (int hr = (int)blockIdx.z + WV_SPLIT * w; hr < nh; hr += WV_SPLIT * WV_WARPS) {
-        const int h = kvh * g.R + h0 + hr;
-        const float sk = sink ? sink[h] : -INFINITY;
-        float mx = sk;
-#pragma unroll
-        for (int z = 0; z < WV_SPLIT; z++) mx = fmaxf(mx, cluster.map_shared_rank(top, z)[hr]);
-        float tot = sink ? expf(sk - mx) : 0.0f, a = 0.0f;
-#pragma unroll
-        for (int z = 0; z < WV_SPLIT; z++) {
-            const float f = expf(cluster.map_shared_rank(top, z)[hr] - mx);                  // an empty slice: exp(-inf) = 0
-            tot = fmaf(f, cluster.map_shared_rank(sum, z)[hr], tot);
-            a = fmaf(f, cluster.map_shared_rank(acc_sm, z)[hr * 32 + lane], a);
-        }
-        const int col = blockIdx.y * 32 + lane;
-        if (col < g.dv) out[((int64_t)t * g.H + h) * g.dv + col] = a / tot;
-    }
-    cluster.sync();                                           // nobody leaves while its shared memory may still be read
-}
-template <int RB>
-__global__ void __cluster_dims__(1, 1, WV_SPLIT) __launch_bounds__(WV_THREADS) wa_values_slices_kernel(const float* __restrict__ S, const float* __restrict__ vring, float* __restrict__ out,
-                                                                                                       WaGeom g, const float* __restrict__ sink, int slice_cap) {
-    pdl_enter();
-    extern __shared__ float wv_sm[];
-    float* pr = wv_sm;                                        // [RB][slice_cap]
-    float* part = wv_sm + (size_t)RB * slice_cap;             // [WV_WARPS][RB][32]
-    __shared__ float top[RB], sum[RB], acc_sm[RB * 32];       // what the cluster reads: the slice's largest score, sum of weights, weighted values
-    const int hblocks = (g.R + RB - 1) / RB;
-    const int hb = blockIdx.x % hblocks, tk = blockIdx.x / hblocks;
-    const int t = tk / g.G, kvh = tk % g.G, h0 = hb * RB, nh = min(RB, g.R - h0);
-    const int64_t i = g.pos0 + t, lo = wa_lo(g, i);
-    const int n = (int)(i - lo + 1), per_slice = (n + WV_SPLIT - 1) / WV_SPLIT;
-    const int s0 = min(n, (int)blockIdx.z * per_slice), m = min(n, s0 + per_slice) - s0;      // this CTA's keys: s0 .. s0 + m of the visible ones
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int hr = w; hr < RB; hr += WV_WARPS) {
-        const float* Sr = S + ((int64_t)t * g.H + kvh * g.R + h0 + hr) * g.cap + s0;
-        float* p = pr + (size_t)hr * slice_cap;
-        const bool on = hr < nh;
-        float mx = -INFINITY;
-        for (int c = lane; c < m; c += 32) { const float v = on ? Sr[c] : 0.0f; p[c] = v; mx = fmaxf(mx, v); }
-        mx = warp_max(mx);
-        float tot = 0.0f;
-        for (int c = lane; c < m; c += 32) { const float e = expf(p[c] - mx); p[c] = e; tot += e; }
-        tot = warp_sum(tot);
-        if (lane == 0) { top[hr] = mx; sum[hr] = tot; }
-    }
-    __syncthreads();
-    const int d = blockIdx.y * 32 + lane;
-    const int per = (m + WV_WARPS - 1) / WV_WARPS;
-    const int c_begin = min(m, w * per), c_end = min(m, c_begin + per);
-    float acc[RB];
-#pragma unroll
-    for (int hr = 0; hr < RB; hr++) acc[hr] = 0.0f;
-    if (d < g.dv) {
-        const float* vb = vring + (int64_t)kvh * g.vhs + d;
-        const int64_t rs = g.vrs;
-        int r = (int)((lo + s0 + c_begin) % g.ring);
-#pragma unroll 8
-        for (int c = c_begin; c < c_end; c++) {
-            const float v = vb[r * rs];
-#pragma unroll
-            for (int hr = 0; hr < RB; hr++) acc[hr] = fmaf(pr[(size_t)hr * slice_cap + c], v, acc[hr]);
-            if (++r == g.ring) r = 0;
-        }
-    }
-    wv_finish<RB>(acc, part, top, sum, acc_sm, out, g, sink, t, kvh, h0, nh, lane, w);
-}
-// slices longer than shared memory holds, chunk by chunk: what is summed so far is scaled whenever the largest score grows.  A slice of one chunk gets the bits of
-// the kernel above, which stays for its loads in flight (one kernel for both: 155 us where that takes 108, a token of 32 heads over 16000 keys)
-__host__ __device__ constexpr int wv_chunk(int RB) { return 160 * 256 / RB - WV_WARPS * 32; }      // keys of a chunk: with the warps' parts 160 KB
-template <int RB>
-__global__ void __cluster_dims__(1, 1, WV_SPLIT) __launch_bounds__(WV_THREADS) wa_values_chunks_kernel(const float* __restrict__ S, const float* __restrict__ vring, float* __restrict__ out,
-                                                                                                       WaGeom g, const float* __restrict__ sink) {
-    pdl_enter();
-    extern __shared__ float wv_sm[];
-    constexpr int CHUNK = wv_chunk(RB);
-    float* pr = wv_sm;                                        // [RB][CHUNK]
-    float* part = wv_sm + (size_t)RB * CHUNK;                 // [WV_WARPS][RB][32]
-    __shared__ float top[RB], sum[RB], acc_sm[RB * 32], fac[RB];      // fac: what the sums of the chunks before are worth
-    const int hblocks = (g.R + RB - 1) / RB;
-    const int hb = blockIdx.x % hblocks, tk = blockIdx.x / hblocks;
-    const int t = tk / g.G, kvh = tk % g.G, h0 = hb * RB, nh = min(RB, g.R - h0);
-    const int64_t i = g.pos0 + t, lo = wa_lo(g, i);
-    const int n = (int)(i - lo + 1), per_slice = (n + WV_SPLIT - 1) / WV_SPLIT;
-    const int s0 = min(n, (int)blockIdx.z * per_slice), m = min(n, s0 + per_slice) - s0;      // this CTA's keys: s0 .. s0 + m of the visible ones
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.y * 32 + lane;
-    const float* vb = vring + (int64_t)kvh * g.vhs + d;
-    float acc[RB];
-#pragma unroll
-    for (int hr = 0; hr < RB; hr++) acc[hr] = 0.0f;
-    int c0 = 0;
-    do {                                                      // (an empty slice: once, for its -inf and zeros)
-        const int mc = min(CHUNK, m - c0);
-        for (int hr = w; hr < RB; hr += WV_WARPS) {
-            const float* Sr = S + ((int64_t)t * g.H + kvh * g.R + h0 + hr) * g.cap + s0 + c0;
-            float* p = pr + (size_t)hr * CHUNK;
-            const bool on = hr < nh;
-            const float before = c0 ? top[hr] : -INFINITY;
-            float mx = -INFINITY;
-            for (int c = lane; c < mc; c += 32) { const float v = on ? Sr[c] : 0.0f; p[c] = v; mx = fmaxf(mx, v); }
-            mx = fmaxf(warp_max(mx), before);
-            float tot = 0.0f;
-            for (int c = lane; c < mc; c += 32) { const float e = expf(p[c] - mx); p[c] = e; tot += e; }
-            tot = warp_sum(tot);
-            if (lane == 0) {
-                if (c0) { fac[hr] = expf(before - mx); tot = fmaf(fac[hr], sum[hr], tot); }
-                top[hr] = mx; sum[hr] = tot;
-            }
-        }
-        __syncthreads();
-        if (c0) {
-#pragma unroll
-            for (int hr = 0; hr < RB; hr++) acc[hr] *= fac[hr];
-        }
-        const int per = (mc + WV_WARPS - 1) / WV_WARPS;
-        const int c_begin = min(mc, w * per), c_end = min(mc, c_begin + per);
-        if (d < g.dv) {
-            int r = (int)((lo + s0 + c0 + c_begin) % g.ring);
-#pragma unroll 8
-            for (int c = c_begin; c < c_end; c++) {
-                const float v = vb[(int64_t)r * g.vrs];
-#pragma unroll
-                for (int hr = 0; hr < RB; hr++) acc[hr] = fmaf(pr[(size_t)hr * CHUNK + c], v, acc[hr]);
-                if (++r == g.ring) r = 0;
-            }
-        }
-        c0 += CHUNK;
-        __syncthreads();                                      // the chunk has been read
-    } while (c0 < m);
-    wv_finish<RB>(acc, part, top, sum, acc_sm, out, g, sink, t, kvh, h0, nh, lane, w);
-}
-template <int RB>
-static int wa_launch_slices(cc_device* dev, const float* S, const float* v, float* out, const WaGeom& g, const float* sink, int64_t maxn) {
-    const int64_t slice = (maxn + WV_SPLIT - 1) / WV_SPLIT;
-    const bool whole = slice <= wv_chunk(RB);
-    const int smem = (int)((RB * (whole ? slice : wv_chunk(RB)) + WV_WARPS * RB * 32) * 4);
-    const dim3 grid((unsigned)(g.T * g.G * ((g.R + RB - 1) / RB)), (unsigned)((g.dv + 31) / 32), WV_SPLIT);
-    if (whole) {
-        if (smem > 40 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(wa_values_slices_kernel<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        cc_launch_alone(dev, wa_values_slices_kernel<RB>, grid, WV_THREADS, smem, S, v, out, g, sink, (int)slice);
-    } else {
-        CC_CUDA(dev, cudaFuncSetAttribute(wa_values_chunks_kernel<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        cc_launch_alone(dev, wa_values_chunks_kernel<RB>, grid, WV_THREADS, smem, S, v, out, g, sink);
-    }
-    CC_LAUNCH_CHECK(dev);
-    return CC_OK;
-}
+#include "attn_rows.cuh"
 // what a call's two ways share
 struct WaCall {
     float* q;
@@ -1282,22 +1066,11 @@ struct WaCall {
     float *o, scale;
     int64_t last, oldest, reach;                        // last position; first one anybody sees; the most keys one query sees
 };
-static int64_t wa_rows_smem(const WaGeom& g) { return (int64_t)(g.R < WS_HEADS ? g.R : WS_HEADS) * g.dk * 4; }
 // few rows: keys spread over the whole device
-static int wa_by_rows(cc_device* dev, WaGeom g, const WaCall& c) {
-    const size_t smem = (size_t)wa_rows_smem(g);
-    const int RB = g.R >= 8 ? 8 : g.R >= 3 ? 4 : g.R;        // query heads a cluster of the value kernel takes together
-    if (smem > 48 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(wa_scores_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    g.cap = (int)c.reach;
-    void* S = nullptr; size_t cls = 0;
-    int rc = cc_pool_alloc(dev, (size_t)g.T * g.H * g.cap * 4, &S, &cls);
-    if (rc) return rc;
-    cc_launch_pdl(dev, wa_scores_row_kernel, dim3((unsigned)((c.reach + 15) / 16), (unsigned)g.T, (unsigned)(g.G * ((g.R + WS_HEADS - 1) / WS_HEADS))), 256, smem, c.q, c.k, (float*)S, g, c.scale, c.r1, c.r2);
-    dev->launches++;
-    rc = RB == 8 ? wa_launch_slices<8>(dev, (const float*)S, c.v, c.o, g, c.sink, c.reach) : RB == 4 ? wa_launch_slices<4>(dev, (const float*)S, c.v, c.o, g, c.sink, c.reach)
-         : RB == 2 ? wa_launch_slices<2>(dev, (const float*)S, c.v, c.o, g, c.sink, c.reach) : wa_launch_slices<1>(dev, (const float*)S, c.v, c.o, g, c.sink, c.reach);
-    cc_pool_free(dev, S, cls);
-    return rc;
+static int wa_by_rows(cc_device* dev, const WaGeom& g, const WaCall& c) {
+    ArArgs A{};
+    A.q = c.q; A.k = c.k; A.v = c.v; A.r1 = c.r1; A.r2 = c.r2; A.sink = c.sink; A.out = c.o; A.scale = c.scale;
+    return attn_rows(dev, g, A, (int)c.reach);
 }
 // many rows: key/value heads in equal groups, so that the workspace -- scores and cut planes of a group -- is at most twice what the scores of all heads take
 // or WA_WORKSPACE, whichever is more (one head at least).  *room: false when the device had none and nothing was launched
@@ -1397,11 +1170,15 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
     g.T = (int)T; g.H = H; g.G = G; g.R = R; g.dk = dk; g.dv = dv; g.ring = (int)ring; g.QT = WA_ROWS / R; g.pos0 = pos0; g.pos0_row = (int)(pos0 % ring);
     g.krs = G * dk; g.vrs = vring ? G * dv : G * dk; g.vhs = vring ? dv : dk;
     const WaCall c = {fptr(q), fptr(kring), vptr, r1 ? fptr(r1) : nullptr, r2 ? fptr(r2) : nullptr, sink ? fptr(sink) : nullptr, (float*)o->base, scale, last, oldest, reach};
-    // Row by row the cache is read once per query and 8 heads of a key head; a tile's share of cutting it is the same up to 128 rows.  us by rows / by tiles, heads
-    // x queries over 300, 2000, 16000 keys: 16 x 4 (a key head each) 26 / 28, 65 / 57, 437 / 354 ; 16 x 8 42 / 27, 121 / 57, 817 / 353 ; 128 x 1 (keys of 192) 42 / 80,
-    // 139 / 320 ; 128 x 2 75 / 80, 254 / 320 ; 128 x 4 147 / 79, 499 / 320 ; 64 x 1 (32 a key head: 4 reads) 17 / 24, 28 / 38, 139 / 197 ; 64 x 2 18 / 20, 42 / 38, 239 / 197
-    const bool can_rows = T <= 65535 && wa_rows_smem(g) <= 160 * 1024;
-    const bool few_rows = can_rows && (T * H <= 64 || (T <= 2 && T * ((R + 7) / 8) <= 4) || ring >= (1 << 30));
+    // Row by row the cache is read once per query and 16 heads of a key head, and a key takes about 3e-9 us for each of
+    //     cost = T * (key heads x blocks of heads) * (dk + dv in whole 128s + 128 for the sums across lanes) * (2, 3, 4, 7 or 12 for up to 1, 2, 4, 8 or 16 heads);
+    // a tile's work is the same up to 128 rows, 20 to 30 us and 0.012 us a key.  More than 64 rows are tiles whatever they cost (one or two queries of few blocks of heads
+    // aside), so that a query of a prompt keeps its bits however the prompt is cut.  us by rows / by tiles over 300, 2000, 4000, 16000 keys, heads on key heads x queries:
+    // 16 on 16 x 4 13 / 27, 30 / 57, 50 / 103, 138 / 352 ; 8 on 1 (latent, 576) x 8 18 / 31, 41 / 51, 70 / 73, 222 / 223 ; 4 on 1 (latent) x 16 22 / 31, 52 / 52, 87 / 73, 229 / 223 ;
+    // 1 on 1 (latent) x 32 19 / 31, 57 / 51, 104 / 73, 275 / 222 ; 128 on 128 (192, 128) x 2 34 / 79, 120 / 319, 209 / 632
+    const bool can_rows = T <= 65535 && (int64_t)(R < 8 ? R : 8) * dk * 4 <= 160 * 1024;
+    const int64_t cost = T * G * ((R + 15) / 16) * ((((int64_t)dk + 127) & ~127) + (((int64_t)dv + 127) & ~127) + 128) * (R > 8 ? 12 : R > 4 ? 7 : R > 2 ? 4 : R + 1);
+    const bool few_rows = can_rows && ((T * H <= 64 && cost <= 72000 + 12000000 / reach) || (T <= 2 && T * ((R + 7) / 8) <= 4) || ring >= (1 << 30));
     if (qnw) {             // the query norm, in place: q is this call's private projection output in every caller of the runner; a caller that
                            // needs its q untouched passes a copy
         cc_launch_pdl(dev, head_rms_norm_kernel, (unsigned)((T * H + 7) / 8), 256, 0, c.q, fptr(qnw), T * H, dk, eps);

@@ -249,6 +249,37 @@ def test_attention_of_few_queries(dev, T, pos0, H, G, d, window, sink):
         np.testing.assert_array_equal(call(t, t + 1)[0].view(np.uint32), got[t].view(np.uint32))
 
 
+@pytest.mark.parametrize("T,n,H,G,dk,dv,latent", [
+    (1, 1, 1, 1, 1, 1, False), (2, 3, 3, 1, 7, 5, False), (3, 130, 8, 8, 33, 34, False),      # rows that are no multiple of 16 bytes
+    (1, 127, 4, 1, 128, 128, False), (1, 128, 4, 1, 128, 128, False), (1, 129, 4, 1, 128, 128, False), (2, 129, 4, 1, 128, 128, False),      # one slice, or two
+    (1, 700, 2, 1, 64, 64, False), (1, 9000, 2, 1, 16, 16, False),                             # weights in one piece, in several
+    (2, 31, 8, 1, 576, 512, True), (1, 32, 5, 1, 576, 512, True), (1, 500, 16, 1, 576, 512, True), (1, 65, 17, 1, 132, 131, True), (1, 1200, 64, 1, 80, 80, False),
+    (1, 13000, 16, 1, 576, 512, True),                                                         # slices too long to stay in shared memory
+    (1, 300, 9, 1, 256, 256, False), (1, 40, 2, 1, 64, 1500, False), (1, 40, 2, 1, 5000, 64, False), (1, 40, 16, 1, 2000, 40, True)])
+def test_attention_of_few_queries_at_the_edges_of_its_slices(dev, T, n, H, G, dk, dv, latent):
+    """Edges of slices, tiles and blocks of heads and columns, a ring that wraps around, and the order of a row's sums beside other rows"""
+    from crabml_b200 import seqops
+    rng = np.random.default_rng(n + H + dk)
+    q, k = rng.standard_normal((T, H, dk)).astype(np.float32), rng.standard_normal((n, G, dk)).astype(np.float32)
+    v = k[..., :dv] if latent else rng.standard_normal((n, G, dv)).astype(np.float32)
+    sk = rng.standard_normal(H).astype(np.float32)
+    ring = n + 3                                   # a ring that wraps: position p lies in row p % ring, and positions start at 2 ring - 5
+    first = 2 * ring - 5
+    order = np.argsort(np.r_[(first + np.arange(n)) % ring, np.setdiff1d(np.arange(ring), (first + np.arange(n)) % ring)])
+    kt, vt = (tensor(dev, np.concatenate([x, np.full((3,) + x.shape[1:], np.nan, np.float32)])[order].reshape(ring, -1)) for x in (k, v))
+    vt, st = None if latent else vt, tensor(dev, sk)
+    window = n - T + 1                             # the first query sees the oldest row
+
+    def call(a, b):
+        return seqops.masked_attention(tensor(dev, q[a:b].reshape(b - a, -1)), kt, vt, first + n - T + a, H, G, dk, dv, dk ** -0.5, window=window, sink=st).export().reshape(b - a, H, dv)
+    got = call(0, T)
+    want = np.stack([attend(q[t:t + 1], k[t:n - T + 1 + t], v[t:n - T + 1 + t], dk ** -0.5, n - T, 0, 0, 0.0, sk)[0] for t in range(T)])
+    # as above: 1e-5 of the values' size
+    assert np.abs(got - want).max() <= 1e-5
+    for t in range(T):
+        np.testing.assert_array_equal(call(t, t + 1)[0].view(np.uint32), got[t].view(np.uint32))
+
+
 def test_attention_of_many_rows_over_a_long_cache_takes_its_heads_in_groups(dev):
     """16 heads over 40,000 keys: 820 MB of scores and cut planes where the scores of 33 queries take 84"""
     from crabml_b200 import seqops

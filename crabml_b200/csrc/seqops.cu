@@ -1405,30 +1405,21 @@ struct QkPrepArgs {
     int64_t pos0;
 };
 #define QKP_THREADS 256
-// grid (tokens, blocks of heads); a norm over the whole projection takes one block.  First the inverse root mean squares -- one per head (a warp per head: lane-strided sum, butterfly) or one per projection
-// (thread-strided sums, butterfly, the warps' sums in warp order) -- then every element once: a rotated pair by the thread of its first
-// column, which reads both raw values and writes both results; all raw values were read for the sums before the barrier, so q may be
-// overwritten in place.
+// grid (tokens, blocks of heads); a norm over the whole projection takes one block, whose sums (thread-strided, butterfly, the warps' sums in warp order) come
+// first.  A warp takes a head: its inverse root mean square (lane-strided sum, butterfly), then every element once, a rotated pair by the lane of its
+// first column, which reads both raw values and writes both results, so q may be overwritten in place.  (With the heads' factors passed through shared memory and an
+// integer division per element: 4.9 us a decoded token and 8.5 us for 512 rows of 8 + 2 heads of 128; now 3.1 and 5.2.)
 __global__ void __launch_bounds__(QKP_THREADS) qk_prepare_kernel(QkPrepArgs a) {
     pdl_enter();
-    extern __shared__ float qkp_sm[];               // inv[H + G], red[8]
-    float* inv = qkp_sm;
-    float* red = qkp_sm + a.H + a.G;
+    __shared__ float red[QKP_THREADS / 32];
+    float inv[2];
     const int t = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int units_all = a.H + a.G, per_block = (units_all + gridDim.y - 1) / gridDim.y;
     const int u0 = min(units_all, (int)blockIdx.y * per_block), u1 = min(units_all, u0 + per_block);       // this CTA's heads: queries', then keys'
     const float* qr = a.q + t * a.qrs;
     const float* kr = a.k + t * a.krs;
     float* qo = a.qo + (int64_t)t * a.H * a.dk;
-    if (a.norm == CC_QK_NORM_HEAD) {
-        for (int u = u0 + w; u < u1; u += QKP_THREADS / 32) {
-            const float* src = u < a.H ? qr + u * a.dk : kr + (u - a.H) * a.dk;
-            float ss = 0.0f;
-            for (int c = lane; c < a.dk; c += 32) ss = fmaf(src[c], src[c], ss);
-            ss = warp_sum(ss);
-            if (lane == 0) inv[u] = 1.0f / sqrtf(ss / (float)a.dk + a.eps);
-        }
-    } else if (a.norm == CC_QK_NORM_ROW) {
+    if (a.norm == CC_QK_NORM_ROW) {
         for (int side = 0; side < 2; side++) {
             const float* src = side ? kr : qr;
             const int n = (side ? a.G : a.H) * a.dk;
@@ -1441,41 +1432,38 @@ __global__ void __launch_bounds__(QKP_THREADS) qk_prepare_kernel(QkPrepArgs a) {
             float tot = 0.0f;
 #pragma unroll
             for (int i = 0; i < QKP_THREADS / 32; i++) tot += red[i];
-            const float v = 1.0f / sqrtf(tot / (float)n + a.eps);
-            for (int u = threadIdx.x; u < (side ? a.G : a.H); u += QKP_THREADS) inv[(side ? a.H : 0) + u] = v;
+            inv[side] = 1.0f / sqrtf(tot / (float)n + a.eps);
         }
-    } else {
-        for (int u = u0 + threadIdx.x; u < u1; u += QKP_THREADS) inv[u] = 1.0f;
+        __syncthreads();                             // all raw values have been read for the sums
     }
-    __syncthreads();
     const int64_t row = (a.pos0 + t) % a.ring;
     const float pos = (float)(a.pos0 + t);
-    for (int idx = threadIdx.x; idx < (u1 - u0) * a.dk; idx += QKP_THREADS) {
-        const int ub = idx / a.dk, c = idx - ub * a.dk, u = u0 + ub;
+    for (int u = u0 + w; u < u1; u += QKP_THREADS / 32) {
         const bool is_q = u < a.H;
         const int ul = is_q ? u : u - a.H;
         const float* src = is_q ? qr + u * a.dk : kr + ul * a.dk;
         float* dst = is_q ? qo + u * a.dk : a.kring + (row * a.G + ul) * a.dk;
         const float* wt = is_q ? a.qw : a.kw;
         if (wt && a.norm == CC_QK_NORM_ROW) wt += ul * a.dk;
-        const float f = inv[u];
-        const int rel = c - a.off;
-        int pair = -1;                               // index of the pair this thread owns, -2: the pair's second column (its owner writes it)
-        if (rel >= 0 && a.half > 0) {
-            if (a.step == 1) pair = rel < a.half ? rel : rel < 2 * a.half ? -2 : -1;
-            else if (rel < 2 * a.half) pair = (rel & 1) ? -2 : rel >> 1;
+        float f = a.norm == CC_QK_NORM_ROW ? inv[is_q ? 0 : 1] : 1.0f;
+        if (a.norm == CC_QK_NORM_HEAD) {
+            float ss = 0.0f;
+#pragma unroll 4
+            for (int c = lane; c < a.dk; c += 32) ss = fmaf(src[c], src[c], ss);
+            ss = warp_sum(ss);
+            f = 1.0f / sqrtf(ss / (float)a.dk + a.eps);
         }
-        if (pair == -2) continue;
-        const float x0 = wt ? src[c] * f * wt[c] : src[c] * f;
-        if (pair >= 0) {
-            const int c1 = c + a.gap;
-            const float x1 = wt ? src[c1] * f * wt[c1] : src[c1] * f;
+        // a rotated pair by the lane of its first column
+        const int first = a.half > 0 ? a.off : a.dk, behind = a.half > 0 ? a.off + 2 * a.half : a.dk;
+        for (int i = lane; i < a.half; i += 32) {
+            const int c = a.off + a.step * i, c1 = c + a.gap;
+            const float x0 = wt ? src[c] * f * wt[c] : src[c] * f, x1 = wt ? src[c1] * f * wt[c1] : src[c1] * f;
             float o0, o1;
-            rotate_pair(x0, x1, pos, a.freq[pair], a.mag, o0, o1);
+            rotate_pair(x0, x1, pos, a.freq[i], a.mag, o0, o1);
             dst[c] = o0; dst[c1] = o1;
-        } else {
-            dst[c] = x0;
         }
+        for (int c = lane; c < first; c += 32) dst[c] = wt ? src[c] * f * wt[c] : src[c] * f;
+        for (int c = behind + lane; c < a.dk; c += 32) dst[c] = wt ? src[c] * f * wt[c] : src[c] * f;
     }
     const float* vr = a.v + t * a.vrs;
     float* vd = a.vring + row * a.G * a.dv;
@@ -1502,10 +1490,9 @@ static int qk_prepare_impl(cc_device* dev, QkPrepArgs a, int64_t T, const cc_vie
     a.kring = fptr(kring); a.vring = fptr(vring); a.qw = q_w ? fptr(q_w) : nullptr; a.kw = k_w ? fptr(k_w) : nullptr;
     a.freq = freq ? fptr(freq) : nullptr; a.H = H; a.G = G; a.dk = dk; a.dv = dv; a.ring = (int)ring; a.norm = qk_norm; a.half = (int)half; a.off = offset;
     a.step = pairing == CC_ROPE_HALVES ? 1 : 2; a.gap = pairing == CC_ROPE_HALVES ? (int)half : 1; a.eps = eps; a.mag = mag; a.pos0 = pos0;
-    const size_t smem = (size_t)(H + G + QKP_THREADS / 32) * 4;
-    CC_REQUIRE(dev, smem <= 48 * 1024, "qk_prepare_append: too many heads");
+    CC_REQUIRE(dev, (H + G + 8) * 4 <= 48 * 1024, "qk_prepare_append: too many heads");
     const int blocks = qk_norm == CC_QK_NORM_ROW ? 1 : (H + G + QKP_THREADS / 32 - 1) / (QKP_THREADS / 32);       // a warp per head
-    cc_launch_pdl(dev, qk_prepare_kernel, dim3((unsigned)T, (unsigned)blocks), QKP_THREADS, smem, a);
+    cc_launch_pdl(dev, qk_prepare_kernel, dim3((unsigned)T, (unsigned)blocks), QKP_THREADS, 0, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1551,19 +1538,32 @@ struct LatAppend {
     int ring_rows, rank, rest, half, step, gap;      // pair i of the rotated part: its columns step * i and step * i + gap
     float eps, mag;
 };
+#define LA_KEEP 16
 __device__ __forceinline__ void latent_append_row(const LatAppend& a, int t, int lane) {
     const int rank = a.rank, cols = a.rank + a.rest, half = a.half;
     const int64_t pos0 = a.pos0;
     const float *nw = a.nw, *freq = a.freq, *src = a.ckv + t * a.rs;
     const float eps = a.eps, mag = a.mag;
     float* dst = a.ring + ((pos0 + t) % a.ring_rows) * cols;
-    float ss = 0.0f;
+    // the first 512 columns and their weights at once
+    float keep[LA_KEEP], wt[LA_KEEP], ss = 0.0f;
+#pragma unroll
+    for (int e = 0; e < LA_KEEP; e++) {
+        const int c = lane + e * 32;
+        keep[e] = c < rank ? src[c] : 0.0f;
+        wt[e] = nw && c < rank ? nw[c] : 1.0f;
+    }
+#pragma unroll
+    for (int e = 0; e < LA_KEEP; e++) ss = fmaf(keep[e], keep[e], ss);
 #pragma unroll 8
-    for (int c = lane; c < rank; c += 32) ss = fmaf(src[c], src[c], ss);
+    for (int c = lane + LA_KEEP * 32; c < rank; c += 32) ss = fmaf(src[c], src[c], ss);
     ss = warp_sum(ss);
     const float inv = 1.0f / sqrtf(ss / (float)rank + eps);
+#pragma unroll
+    for (int e = 0; e < LA_KEEP; e++)
+        if (lane + e * 32 < rank) dst[lane + e * 32] = keep[e] * inv * wt[e];
 #pragma unroll 8
-    for (int c = lane; c < rank; c += 32) dst[c] = src[c] * inv * (nw ? nw[c] : 1.0f);
+    for (int c = lane + LA_KEEP * 32; c < rank; c += 32) dst[c] = src[c] * inv * (nw ? nw[c] : 1.0f);
     for (int i = lane; i < half; i += 32) {
         float ou, ov;
         const int c = rank + a.step * i;
@@ -1596,7 +1596,6 @@ extern "C" CC_API int cc_latent_ring_append(cc_device* dev, const cc_view* ring,
 }
 
 // ---- per-head products: the up-projections of a latent cache, folded into the query and applied to the attention result ---------------------
-#define HP_TOK 8
 struct HpArgs {
     const float *x, *W;           // token t's row at x + t * xrs, head h's inputs at + h * (n_in + rest)
     float* out;
@@ -1606,66 +1605,97 @@ struct HpArgs {
     float mag;
     LatAppend app;                // app.ring != NULL: the grid has one more z plane, the first, whose CTAs of head 0 write the tokens' cache rows
 };
-// grid (ceil(T / 8), H, ceil(n_out / 4)): the CTA stages 8 tokens' x[t, h, :n_in]; a warp owns one output coordinate for those tokens:
-// lane-strided partial sums over n_in, then the butterfly -- one order per output, whatever T is.  W: [H * n_out, n_in], rows read
-// contiguously.  The `rest` columns behind a head's n_in inputs are copied behind its n_out outputs.
-__global__ void __launch_bounds__(128) head_project_kernel(HpArgs a) {
+// grid (ceil(T / TOK), H, ceil(n_out / (8 * ROWS))): a warp owns ROWS neighbouring outputs of TOK tokens; its lanes read 4 columns each of W's rows (VEC) or one, the
+// rows' pieces all at once, and the tokens' x from the cache: partial sums of every lane, then the butterfly -- one order per output, which n_in alone decides,
+// whatever T is.  W: [H * n_out, n_in].  The `rest` columns behind a head's n_in inputs are copied behind its n_out outputs.
+// Bound by latency: one token's 2 MB of W in 1024 warps, each with 4 loads of 16 bytes a lane in flight.  With 8 tokens staged in shared memory, whatever T was (32 turns of
+// an integer division for 512 inputs), and 4-byte loads, 8 heads x 128 outputs of 512 took 15.8 us in a decoded token, x 512 outputs of 128 6.9 us; now 3.1 each.
+#define HP_WARPS 8
+template <int TOK, int ROWS, bool VEC>
+__global__ void __launch_bounds__(HP_WARPS * 32) head_project_kernel(HpArgs a) {
+    const int t0 = blockIdx.x * TOK, h = blockIdx.y, T = a.T, H = a.H, n_in = a.n_in, rest = a.rest, n_out = a.n_out, half = a.half;
+    const int z = (int)blockIdx.z - (a.app.ring ? 1 : 0), lane = threadIdx.x & 31, v0 = (z * HP_WARPS + (threadIdx.x >> 5)) * ROWS;
+    const int xs = n_in + rest, os = n_out + rest, nv = min(ROWS, n_out - v0);
+    const float* W = a.W + ((int64_t)h * n_out + v0) * n_in;
+    // the rows start for L2 while the kernel before is still at work
+    if (z >= 0 && nv > 0)
+        for (int64_t c = lane * 32; c < (int64_t)nv * n_in; c += 1024) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + c));
     pdl_enter();
-    extern __shared__ float hp_sm[];
-    const int t0 = blockIdx.x * HP_TOK, h = blockIdx.y, T = a.T, H = a.H, n_in = a.n_in, rest = a.rest, n_out = a.n_out, half = a.half;
-    const int z = (int)blockIdx.z - (a.app.ring ? 1 : 0);
     if (z < 0) {
         if (h == 0)
-            for (int tt = threadIdx.x >> 5; tt < HP_TOK && t0 + tt < T; tt += 4) latent_append_row(a.app, t0 + tt, threadIdx.x & 31);
+            for (int tt = threadIdx.x >> 5; tt < TOK && t0 + tt < T; tt += HP_WARPS) latent_append_row(a.app, t0 + tt, lane);
         return;
     }
-    const int xs = n_in + rest, os = n_out + rest;
-    for (int i = threadIdx.x; i < HP_TOK * n_in; i += 128) {
-        const int tt = i / n_in, d = i - tt * n_in;
-        hp_sm[i] = t0 + tt < T ? a.x[(t0 + tt) * a.xrs + h * xs + d] : 0.0f;
+    const float* x = a.x + (int64_t)t0 * a.xrs + (int64_t)h * xs;
+    const int nt = min(TOK, T - t0);
+    if (nv > 0) {
+        float acc[TOK][ROWS];
+#pragma unroll
+        for (int tt = 0; tt < TOK; tt++)
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) acc[tt][r] = 0.0f;
+        if (VEC) {
+            const bool xvec = (((uintptr_t)x & 15) | (unsigned)(a.xrs & 3)) == 0;
+#pragma unroll 4
+            for (int d = lane * 4; d < n_in; d += 128) {
+                float4 wv[ROWS];
+#pragma unroll
+                for (int r = 0; r < ROWS; r++) wv[r] = __ldg((const float4*)(W + (int64_t)min(r, nv - 1) * n_in + d));
+#pragma unroll
+                for (int tt = 0; tt < TOK; tt++) {
+                    const float* xt = x + (int64_t)min(tt, nt - 1) * a.xrs + d;
+                    const float4 xv = xvec ? *(const float4*)xt : make_float4(xt[0], xt[1], xt[2], xt[3]);
+#pragma unroll
+                    for (int r = 0; r < ROWS; r++) {
+                        float y = acc[tt][r];
+                        y = fmaf(xv.x, wv[r].x, y); y = fmaf(xv.y, wv[r].y, y); y = fmaf(xv.z, wv[r].z, y); y = fmaf(xv.w, wv[r].w, y);
+                        acc[tt][r] = y;
+                    }
+                }
+            }
+        } else {
+            for (int d = lane; d < n_in; d += 32)
+#pragma unroll
+                for (int r = 0; r < ROWS; r++) {
+                    const float wv = W[(int64_t)min(r, nv - 1) * n_in + d];
+#pragma unroll
+                    for (int tt = 0; tt < TOK; tt++) acc[tt][r] = fmaf(x[(int64_t)min(tt, nt - 1) * a.xrs + d], wv, acc[tt][r]);
+                }
+        }
+#pragma unroll
+        for (int tt = 0; tt < TOK; tt++)
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) {
+                float sum = warp_sum(acc[tt][r]);
+                if (lane != 0 || tt >= nt || r >= nv) continue;
+                if (a.gate) sum *= seq_sigmoid(a.gate[(t0 + tt) * a.grs + h * a.ghs + (v0 + r) * a.gvs]);
+                a.out[((int64_t)(t0 + tt) * H + h) * os + v0 + r] = sum;
+            }
     }
-    if (z == 0) {
+    if (z == 0 && rest > 0) {
         // the carried columns: the first 2 * half of them are rotated on the way when a frequency table is given
-        for (int i = threadIdx.x; i < HP_TOK * half; i += 128) {
-            const int tt = i / half, p = i - tt * half;
-            if (t0 + tt >= T) continue;
-            const float* src = a.x + (t0 + tt) * a.xrs + h * xs + n_in + a.step * p;
-            float* dst = a.out + ((int64_t)(t0 + tt) * H + h) * os + n_out + a.step * p;
-            rotate_pair(src[0], src[a.gap], (float)(a.pos0 + t0 + tt), a.freq[p], a.mag, dst[0], dst[a.gap]);
+        for (int tt = 0; tt < nt; tt++) {
+            const float* src = x + tt * a.xrs + n_in;
+            float* dst = a.out + ((int64_t)(t0 + tt) * H + h) * os + n_out;
+            for (int p = threadIdx.x; p < half; p += HP_WARPS * 32)
+                rotate_pair(src[a.step * p], src[a.step * p + a.gap], (float)(a.pos0 + t0 + tt), a.freq[p], a.mag, dst[a.step * p], dst[a.step * p + a.gap]);
+            for (int j = 2 * half + threadIdx.x; j < rest; j += HP_WARPS * 32) dst[j] = src[j];
         }
-        const int plain = rest - 2 * half;
-        for (int i = threadIdx.x; i < HP_TOK * plain; i += 128) {
-            const int tt = i / plain, j = 2 * half + (i - tt * plain);
-            if (t0 + tt < T) a.out[((int64_t)(t0 + tt) * H + h) * os + n_out + j] = a.x[(t0 + tt) * a.xrs + h * xs + n_in + j];
-        }
-    }
-    __syncthreads();
-    const int v = z * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (v >= n_out) return;
-    const float* wp = a.W + ((int64_t)h * n_out + v) * n_in;
-    float acc[HP_TOK];
-#pragma unroll
-    for (int tt = 0; tt < HP_TOK; tt++) acc[tt] = 0.0f;
-    for (int d = lane; d < n_in; d += 32) {
-        const float wv = wp[d];
-#pragma unroll
-        for (int tt = 0; tt < HP_TOK; tt++) acc[tt] = fmaf(hp_sm[tt * n_in + d], wv, acc[tt]);
-    }
-#pragma unroll
-    for (int tt = 0; tt < HP_TOK; tt++) {
-        float sum = warp_sum(acc[tt]);
-        if (lane != 0 || t0 + tt >= T) continue;
-        if (a.gate) sum *= seq_sigmoid(a.gate[(t0 + tt) * a.grs + h * a.ghs + v * a.gvs]);
-        a.out[((int64_t)(t0 + tt) * H + h) * os + v] = sum;
     }
 }
-static int head_project_few(cc_device* dev, const HpArgs& a) {
-    const size_t smem = (size_t)HP_TOK * a.n_in * 4;
-    CC_REQUIRE(dev, smem <= 160 * 1024, "head_project: %d inputs per head do not fit shared memory", a.n_in);
-    if (smem > 48 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(head_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cc_launch_pdl(dev, head_project_kernel, dim3((unsigned)((a.T + HP_TOK - 1) / HP_TOK), (unsigned)a.H, (unsigned)((a.n_out + 3) / 4 + (a.app.ring ? 1 : 0))), 128, smem, a);
+template <int TOK, int ROWS, bool VEC>
+static int head_project_launch(cc_device* dev, const HpArgs& a) {
+    cc_launch_pdl(dev, head_project_kernel<TOK, ROWS, VEC>, dim3((unsigned)((a.T + TOK - 1) / TOK), (unsigned)a.H, (unsigned)((a.n_out + HP_WARPS * ROWS - 1) / (HP_WARPS * ROWS) + (a.app.ring ? 1 : 0))),
+                  HP_WARPS * 32, 0, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
+}
+static int head_project_few(cc_device* dev, const HpArgs& a) {
+    CC_REQUIRE(dev, (int64_t)8 * a.n_in * 4 <= 160 * 1024, "head_project: %d inputs per head are too many", a.n_in);
+    if (a.n_in & 3 || (uintptr_t)a.W & 15) return head_project_launch<4, 1, false>(dev, a);
+    // rows of fewer than 256 columns by fours: a lane's one or two pieces of a row are too little in flight
+    if (a.n_in < 256) return a.T == 1 ? head_project_launch<1, 4, true>(dev, a) : head_project_launch<4, 4, true>(dev, a);
+    return a.T == 1 ? head_project_launch<1, 1, true>(dev, a) : head_project_launch<4, 2, true>(dev, a);
 }
 // many rows and nothing carried: a 64 x 64 output tile of one head per CTA, 16-deep slices of the inputs through shared memory, 4 x 4 outputs
 // per thread, every sum over n_in in ascending order inside one thread.  grid (ceil(n_out / 64), ceil(T / 64), H)
@@ -1726,8 +1756,7 @@ extern "C" CC_API int cc_head_project(cc_device* dev, const cc_view* x, const cc
     CC_REQUIRE(dev, x->ndim == 2 && w->ndim == 2 && n_heads > 0 && rest >= 0 && w->shape[0] % n_heads == 0 && x->shape[1] == (int64_t)n_heads * (w->shape[1] + rest),
                "head_project: x must be [T, heads * (n_in + rest)] and w [heads * n_out, n_in]");
     const int64_t T = x->shape[0], n_in = w->shape[1], n_out = w->shape[0] / n_heads;
-    const size_t smem = (size_t)HP_TOK * n_in * 4;
-    CC_REQUIRE(dev, smem <= 160 * 1024, "head_project: %lld inputs per head do not fit shared memory", (long long)n_in);
+    CC_REQUIRE(dev, n_in * 32 <= 160 * 1024, "head_project: %lld inputs per head are too many", (long long)n_in);
     cc_buf* o = nullptr;
     int rc = cc_new_activation(dev, T * n_heads * (n_out + rest), CC_F32, false, &o);
     if (rc) return rc;

@@ -24,17 +24,17 @@ int cc_prefill_bf16_operand(cc_device* dev, int64_t b, int64_t k, void** out);
 int cc_launch_prefill_bf16_operand(cc_device* dev, const cc_buf* w, float* out, int64_t m, int64_t k, int64_t b, int accumulate);
 int cc_launch_dense_tile(cc_device* dev, const cc_buf* w, const float* x, float* out, int64_t m, int64_t k, int64_t b, int accumulate);                        // dense.cu
 
-#define PB_THREADS 1024
-#define PB_WARPS (PB_THREADS / 32)
-#define PB_DEPTH 4                         // 16-byte pieces of a weight row a lane has in flight
+#define PB_COLS 1024                       // columns of the operand that a warp holds, 32 a lane
+#define PB_TURNS 32                        // rows of a warp whose sums wait in shared memory
 #define PB_LN_THREADS 256
 
 // what the operand's rows are made of
 struct PbNorm {
     const float *x, *w, *b;                // x: [T, k] contiguous; b NULL: no bias
     float eps;
+    template <int THREADS>
     __device__ __forceinline__ void stage(float* dst, int t, int k, float* red, bool round) const {
-        layer_norm_row<PB_THREADS>(x + (int64_t)t * k, w, b, k, eps, red, [&](int c, float v) { dst[c] = round ? __bfloat162float(__float2bfloat16_rn(v)) : v; });
+        layer_norm_row<THREADS>(x + (int64_t)t * k, w, b, k, eps, red, [&](int c, float v) { dst[c] = round ? __bfloat162float(__float2bfloat16_rn(v)) : v; });
     }
 };
 struct PbJoin {
@@ -45,102 +45,137 @@ struct PbJoin {
     __device__ __forceinline__ float at(int t, int c) const {
         return c < ca ? a[(int64_t)t * ca + c] : glu_apply(g[t * rs + (c - ca)], u[t * rs + (c - ca)], P);
     }
+    template <int THREADS>
     __device__ __forceinline__ void stage(float* dst, int t, int k, float*, bool round) const {
-        for (int c = threadIdx.x; c < k; c += PB_THREADS) {
-            const float v = at(t, c);
-            dst[c] = round ? __bfloat162float(__float2bfloat16_rn(v)) : v;
+        constexpr int EACH = 4096 / THREADS;
+        for (int c0 = threadIdx.x; c0 < k; c0 += EACH * THREADS) {       // the numbers of EACH columns at once
+            float x[EACH], y[EACH];
+#pragma unroll
+            for (int e = 0; e < EACH; e++) {
+                const int c = c0 + e * THREADS;
+                x[e] = y[e] = 0.0f;
+                if (c < ca) x[e] = a[(int64_t)t * ca + c];
+                else if (c < k) { x[e] = g[t * rs + (c - ca)]; y[e] = u[t * rs + (c - ca)]; }
+            }
+#pragma unroll
+            for (int e = 0; e < EACH; e++) {
+                const int c = c0 + e * THREADS;
+                const float v = c < ca ? x[e] : glu_apply(x[e], y[e], P);
+                if (c < k) dst[c] = round ? __bfloat162float(__float2bfloat16_rn(v)) : v;
+            }
         }
     }
 };
 
-__device__ __forceinline__ float pb_dot8(const int4 v, const float* a, float acc) {
-    const float4 a0 = *(const float4*)a, a1 = *(const float4*)(a + 4);
-    acc = fmaf(__uint_as_float((unsigned)v.x << 16), a0.x, acc); acc = fmaf(__uint_as_float((unsigned)v.x & 0xFFFF0000u), a0.y, acc);
-    acc = fmaf(__uint_as_float((unsigned)v.y << 16), a0.z, acc); acc = fmaf(__uint_as_float((unsigned)v.y & 0xFFFF0000u), a0.w, acc);
-    acc = fmaf(__uint_as_float((unsigned)v.z << 16), a1.x, acc); acc = fmaf(__uint_as_float((unsigned)v.z & 0xFFFF0000u), a1.y, acc);
-    acc = fmaf(__uint_as_float((unsigned)v.w << 16), a1.z, acc); acc = fmaf(__uint_as_float((unsigned)v.w & 0xFFFF0000u), a1.w, acc);
-    return acc;
-}
-// grid (about one CTA per SM, T).  `split` warps (a power of two) share one weight row, each a contiguous stretch of its 16-byte pieces in
-// lane-strided order; a CTA owns PB_WARPS / split rows at a time.  A lane keeps the next PB_DEPTH pieces -- of this row or of the next one --
-// in flight while it multiplies the current ones, and the first pieces are fetched before the operand row is staged.  Partial sums: the
-// butterfly, then the row's warps in ascending order.  The order depends on the sizes alone, not on T.
-template <bool BF16W, class Op>
-__global__ void __launch_bounds__(PB_THREADS, 1) pb_matvec_kernel(const void* __restrict__ W, Op op, float* __restrict__ out, int m, int k, int split, int accumulate) {
+// grid (about one CTA per SM, T).  `split` warps (a power of two) share one weight row, each a contiguous stretch of its 16-byte pieces, PB_COLS columns or less at a time;
+// a CTA owns PB_WARPS / split rows at a time.  A lane holds its 32 columns of the operand in registers for all of the warp's rows and has the pieces of the
+// next row in flight while it multiplies those of this one; the first are fetched before the operand row is staged.  Sums of a row: each piece by itself, the pieces, the
+// butterfly, then the row's warps in ascending order, once for up to PB_TURNS rows.  The order depends on the sizes alone, not on T.
+// Bound by latency (norm, first pieces) and, in a model's head, by memory.  With the operand read from shared memory for every row, 32 warps took 4096 cycles of its ports for
+// 64 rows of 1024 columns (lanes 32 bytes apart: two turns each).  A decoded token's products, us: 7424 x 1024 behind the norm 8.5 -> 6.7, 1024 x 4096 behind the
+// gated units 5.9 -> 5.8, the head's 32000 x 1024 (cold) 26.7 -> 22.3.
+template <bool BF16W, class Op, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) pb_matvec_kernel(const void* __restrict__ W, Op op, float* __restrict__ out, int m, int k, int split, int accumulate) {
     extern __shared__ __align__(16) float pb_sm[];              // the operand row, k floats (rounded up to 4)
-    __shared__ float red[PB_WARPS];
+    constexpr int WARPS = THREADS / 32;
+    __shared__ float red[WARPS], part[PB_TURNS][WARPS];
+    constexpr bool AHEAD = THREADS <= 512;                       // registers for the next row's pieces
+    constexpr int PIECE = BF16W ? 8 : 4, DEPTH = PB_COLS / 32 / PIECE;      // columns of a piece ; pieces a lane holds
     const int t = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int per_cta = PB_WARPS / split, sub = warp % split, slot = warp / split;
+    const int per_cta = WARPS / split, sub = warp % split, slot = warp / split;
     const int rows_it = (m + gridDim.x * per_cta - 1) / (gridDim.x * per_cta);
     const int row0 = blockIdx.x * per_cta + slot, row_step = gridDim.x * per_cta;
     float* orow = out + (int64_t)t * m;
-    const bool vec = BF16W ? (k & 7) == 0 : (k & 3) == 0;
-    const int pieces = BF16W ? k >> 3 : k >> 2;                  // 16-byte pieces of a row
-    const int per_warp = (pieces + split - 1) / split;
-    const int p_begin = min(pieces, sub * per_warp), p_end = min(pieces, p_begin + per_warp);
-    const int batches = (per_warp + 32 * PB_DEPTH - 1) / (32 * PB_DEPTH);
-    const int total = rows_it * batches;
-    int4 cur[PB_DEPTH], nxt[PB_DEPTH];
-    auto fetch = [&](int4* v, int i) {
-        const int it = i / batches, p0 = p_begin + (i - it * batches) * 32 * PB_DEPTH + lane;
-        const int row = row0 + it * row_step;
+    const bool vec = k % PIECE == 0;
+    const int pieces = k / PIECE, per_warp = (pieces + split - 1) / split;
+    const int p_begin = min(pieces, sub * per_warp), p_end = min(pieces, p_begin + per_warp), blocks = vec ? (per_warp + 32 * DEPTH - 1) / (32 * DEPTH) : 1;
+    int4 cur[DEPTH], nxt[AHEAD ? DEPTH : 1];
+    auto fetch = [&](int4 (&v)[DEPTH], int it, int b) {
+        const int p0 = p_begin + b * 32 * DEPTH + lane, row = row0 + it * row_step;
 #pragma unroll
-        for (int e = 0; e < PB_DEPTH; e++) {
+        for (int e = 0; e < DEPTH; e++) {
             const int p = p0 + e * 32;
             v[e] = (row < m && p < p_end) ? ld_stream_16((const uint8_t*)W + ((int64_t)row * pieces + p) * 16) : make_int4(0, 0, 0, 0);
         }
     };
     // this CTA's weight rows start for L2 while the kernel before is still at work (a prefetch has no value that could be stale): with the rows of 15 MB
     // fetched only behind the norm, the product took 12.8 us for 2.3 us of memory time
-    {
-        const int64_t row_bytes = (int64_t)k * (BF16W ? 2 : 4);
-        for (int64_t i = threadIdx.x; i < (int64_t)rows_it * per_cta * ((row_bytes + 127) >> 7); i += PB_THREADS) {
-            const int64_t r = i / ((row_bytes + 127) >> 7), at = (i - r * ((row_bytes + 127) >> 7)) << 7, row = blockIdx.x * per_cta + (r / per_cta) * row_step + r % per_cta;
-            if (row < m && blockIdx.y == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"((const uint8_t*)W + row * row_bytes + at));
-        }
+    if (blockIdx.y == 0) {
+        const unsigned row_bytes = (unsigned)k * (BF16W ? 2 : 4), lines = (row_bytes + 127) >> 7;
+        for (int it = 0; it < rows_it; it++)
+            for (unsigned i = threadIdx.x; i < per_cta * lines; i += THREADS) {
+                const unsigned r = i / lines;
+                const int64_t row = blockIdx.x * per_cta + (int64_t)it * row_step + r;
+                if (row < m) asm volatile("prefetch.global.L2 [%0];" ::"l"((const uint8_t*)W + row * row_bytes + ((i - r * lines) << 7)));
+            }
     }
     pdl_enter();
-    if (vec) fetch(cur, 0);
-    op.stage(pb_sm, t, k, red, BF16W);
+    if (vec) fetch(cur, 0, 0);
+    op.template stage<THREADS>(pb_sm, t, k, red, BF16W);
     __syncthreads();
-    for (int it = 0; it < rows_it; it++) {
-        const int row = row0 + it * row_step;
-        float acc = 0.0f;
-        if (vec) {
-            for (int b = 0; b < batches; b++) {
-                const int i = it * batches + b;
-                if (i + 1 < total) fetch(nxt, i + 1);
-                const int p0 = p_begin + b * 32 * PB_DEPTH + lane;
+    for (int it0 = 0; it0 < rows_it; it0 += PB_TURNS) {
+        const int turns = min(PB_TURNS, rows_it - it0);
+        for (int b = 0; b < blocks; b++) {
+            float x[PB_COLS / 32];
 #pragma unroll
-                for (int e = 0; e < PB_DEPTH; e++) {
-                    const int p = p0 + e * 32;
-                    if (p < p_end) {
-                        if (BF16W) acc = pb_dot8(cur[e], pb_sm + p * 8, acc);
-                        else {
-                            const float4 a = *(const float4*)(pb_sm + p * 4);
-                            acc = fmaf(__int_as_float(cur[e].x), a.x, acc); acc = fmaf(__int_as_float(cur[e].y), a.y, acc);
-                            acc = fmaf(__int_as_float(cur[e].z), a.z, acc); acc = fmaf(__int_as_float(cur[e].w), a.w, acc);
-                        }
-                    }
+            for (int e = 0; e < DEPTH; e++) {
+                const int p = p_begin + b * 32 * DEPTH + lane + e * 32;
+                const bool in = vec && p < p_end;
+#pragma unroll
+                for (int c = 0; c < PIECE; c += 4) {
+                    const float4 v = in ? *(const float4*)(pb_sm + p * PIECE + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    x[e * PIECE + c] = v.x; x[e * PIECE + c + 1] = v.y; x[e * PIECE + c + 2] = v.z; x[e * PIECE + c + 3] = v.w;
                 }
+            }
+            for (int it = 0; it < turns; it++) {
+                float acc = 0.0f;
+                if (vec) {
+                    const bool more = it + 1 < turns;             // the next row of this block, or the first one of the next
+                    const int nb = more ? b : b + 1 < blocks ? b + 1 : 0, ni = more ? it0 + it + 1 : b + 1 < blocks ? it0 : it0 + PB_TURNS;
+                    if constexpr (AHEAD) { if (ni < rows_it) fetch(nxt, ni, nb); }
+                    float piece[DEPTH];
 #pragma unroll
-                for (int e = 0; e < PB_DEPTH; e++) cur[e] = nxt[e];
+                    for (int e = 0; e < DEPTH; e++) {
+                        const float* y = x + e * PIECE;
+                        float a = 0.0f;
+                        if (BF16W) {
+                            a = fmaf(__uint_as_float((unsigned)cur[e].x << 16), y[0], a); a = fmaf(__uint_as_float((unsigned)cur[e].x & 0xFFFF0000u), y[1], a);
+                            a = fmaf(__uint_as_float((unsigned)cur[e].y << 16), y[2], a); a = fmaf(__uint_as_float((unsigned)cur[e].y & 0xFFFF0000u), y[3], a);
+                            a = fmaf(__uint_as_float((unsigned)cur[e].z << 16), y[4 % PIECE], a); a = fmaf(__uint_as_float((unsigned)cur[e].z & 0xFFFF0000u), y[5 % PIECE], a);
+                            a = fmaf(__uint_as_float((unsigned)cur[e].w << 16), y[6 % PIECE], a); a = fmaf(__uint_as_float((unsigned)cur[e].w & 0xFFFF0000u), y[7 % PIECE], a);
+                        } else {
+                            a = fmaf(__int_as_float(cur[e].x), y[0], a); a = fmaf(__int_as_float(cur[e].y), y[1], a);
+                            a = fmaf(__int_as_float(cur[e].z), y[2], a); a = fmaf(__int_as_float(cur[e].w), y[3], a);
+                        }
+                        piece[e] = a;
+                    }
+#pragma unroll
+                    for (int n = DEPTH / 2; n >= 1; n /= 2)
+#pragma unroll
+                        for (int e = 0; e < n; e++) piece[e] += piece[e + n];
+                    acc = piece[0];
+                    if constexpr (AHEAD) {
+#pragma unroll
+                        for (int e = 0; e < DEPTH; e++) cur[e] = nxt[e];
+                    } else if (ni < rows_it) fetch(cur, ni, nb);
+                } else {
+                    const int row = row0 + (it0 + it) * row_step;
+                    if (row < m)
+                        for (int c = sub * 32 + lane; c < k; c += split * 32)
+                            acc = fmaf(BF16W ? __uint_as_float((unsigned)((const uint16_t*)W)[(int64_t)row * k + c] << 16) : ((const float*)W)[(int64_t)row * k + c], pb_sm[c], acc);
+                }
+                acc = warp_sum(acc);
+                if (lane == 0) part[it][warp] = b ? part[it][warp] + acc : acc;
             }
-        } else if (row < m) {
-            for (int c = sub * 32 + lane; c < k; c += split * 32)
-                acc = fmaf(BF16W ? __uint_as_float((unsigned)((const uint16_t*)W)[(int64_t)row * k + c] << 16) : ((const float*)W)[(int64_t)row * k + c], pb_sm[c], acc);
         }
-        acc = warp_sum(acc);
-        if (split > 1) {
-            __syncthreads();                                     // red may still be read
-            if (lane == 0) red[warp] = acc;
-            __syncthreads();
-            if (sub == 0) {
-                acc = 0.0f;
-                for (int s = 0; s < split; s++) acc += red[warp + s];
-            }
+        __syncthreads();
+        for (int i = threadIdx.x; i < turns * per_cta; i += THREADS) {
+            const int it = i / per_cta, r = i - it * per_cta, row = blockIdx.x * per_cta + r + (it0 + it) * row_step;
+            float a = 0.0f;
+            for (int y = 0; y < split; y++) a += part[it][r * split + y];
+            if (row < m) orow[row] = accumulate ? orow[row] + a : a;
         }
-        if (lane == 0 && sub == 0 && row < m) orow[row] = accumulate ? orow[row] + acc : acc;
+        if (it0 + PB_TURNS < rows_it) __syncthreads();            // part is written again
     }
 }
 // the bfloat16 operand of the tensor-core product: a CTA per row
@@ -172,16 +207,28 @@ __global__ void __launch_bounds__(256) pb_join_f32_kernel(PbJoin op, float* __re
 
 static const size_t PB_MAX_SMEM = 200 * 1024;
 static bool pb_few(int64_t T, int64_t k) { return T < 8 && (size_t)((k + 3) & ~3) * 4 <= PB_MAX_SMEM; }
-template <bool BF16W, class Op>
-static int pb_launch_matvec(cc_device* dev, const cc_buf* w, const Op& op, float* out, int64_t m, int64_t k, int64_t T, int accumulate) {
+template <bool BF16W, class Op, int THREADS>
+static int pb_launch_matvec_by(cc_device* dev, const cc_buf* w, const Op& op, float* out, int64_t m, int64_t k, int64_t T, int accumulate, int split) {
     const size_t smem = (size_t)((k + 3) & ~3) * 4;
-    if (smem > 40 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(pb_matvec_kernel<BF16W, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int split = 1;                                               // as many warps per row as there are too few rows for the device's warps
-    while (split < PB_WARPS && m * split * 2 <= (int64_t)dev->sm_count * PB_WARPS) split *= 2;
-    const int64_t per_cta = PB_WARPS / split, ctas = (m + per_cta - 1) / per_cta;
-    cc_launch_pdl(dev, pb_matvec_kernel<BF16W, Op>, dim3((unsigned)(ctas < dev->sm_count ? ctas : dev->sm_count), (unsigned)T), PB_THREADS, smem, w->plane[0], op, out, (int)m, (int)k, split, accumulate);
+    auto kernel = pb_matvec_kernel<BF16W, Op, THREADS>;
+    if (smem > 40 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t per_cta = THREADS / 32 / split, ctas = (m + per_cta - 1) / per_cta;
+    cc_launch_pdl(dev, kernel, dim3((unsigned)(ctas < dev->sm_count ? ctas : dev->sm_count), (unsigned)T), THREADS, smem, w->plane[0], op, out, (int)m, (int)k, split, accumulate);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
+}
+template <bool BF16W, class Op>
+static int pb_launch_matvec(cc_device* dev, const cc_buf* w, const Op& op, float* out, int64_t m, int64_t k, int64_t T, int accumulate) {
+    // as many warps per row as there are too few rows for the device's warps, and as the row's columns need for one block each.  32 warps a CTA where that makes one turn
+    // of the rows (1024 x 4096: 5.8 us; two turns of 16 warps 6.7), 16 with the next row's pieces in flight where there are more (7424 x 1024)
+    auto split_for = [&](int warps) {
+        int split = 1;
+        while (split < warps && (m * split * 2 <= (int64_t)dev->sm_count * warps || k > (int64_t)split * PB_COLS)) split *= 2;
+        return split;
+    };
+    const int wide = split_for(32);
+    if (BF16W && m * wide <= (int64_t)dev->sm_count * 32) return pb_launch_matvec_by<BF16W, Op, 1024>(dev, w, op, out, m, k, T, accumulate, wide);
+    return pb_launch_matvec_by<BF16W, Op, 512>(dev, w, op, out, m, k, T, accumulate, split_for(16));
 }
 static bool pb_tensor_cores(const cc_buf* w, int64_t m, int64_t k, int64_t T) {
     return w->dtype == CC_BF16 && cc_prefill_bf16_supported(m, k, T) && ((uintptr_t)w->plane[0] & 15) == 0;

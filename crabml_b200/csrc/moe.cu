@@ -49,7 +49,7 @@ struct RouteArgs {
 // by element when D or the pointers do not allow them; then the butterfly), then warp tt does token tt's softmax and choice.  The order of a
 // logit's sum does not depend on TOK.
 template <int TOK>
-__global__ void __launch_bounds__(TOK == 1 ? 1024 : 512) moe_route_kernel(RouteArgs a) {
+__global__ void __launch_bounds__(TOK == 1 ? 1024 : 512, TOK == 2 ? 2 : 1) moe_route_kernel(RouteArgs a) {
     pdl_enter();
     extern __shared__ float rt_sm[];
     __shared__ float sg_sm[TOK];                           // the shared gate's logit: row E of the same products
@@ -138,24 +138,28 @@ __global__ void __launch_bounds__(TOK == 1 ? 1024 : 512) moe_route_kernel(RouteA
         for (int e = lane; e < E; e += 32) if (gs[e / per] != INFINITY) c[e] = -INFINITY;
         __syncwarp();
     }
-    float wsum = 0.0f;
+    float wsum = 0.0f, mine = 0.0f;                         // lane r keeps the weight of choice r (of the first 32) until all are known
     const int slots = top + n_shared;
     for (int r = 0; r < top; r++) {
         float bv = -INFINITY; int bi = 0x7fffffff;
         for (int e = lane; e < E; e += 32) { const float v = c[e]; if (v > bv) { bv = v; bi = e; } }
         warp_argmax(bv, bi);
         if (bi == 0x7fffffff) bi = 0;                       // unreachable with finite scores (keep * group size >= top); never index out of range
+        const float w = s[bi];
+        if (r == lane) mine = w;
         if (lane == 0) {
             ids[(int64_t)t * slots + r] = bi;
-            wts[(int64_t)t * slots + r] = s[bi];
+            if (r >= 32) wts[(int64_t)t * slots + r] = w;
             c[bi] = -INFINITY;
         }
-        wsum += s[bi];
+        wsum += w;
         __syncwarp();
     }
-    if (lane == 0) {
-        if (a.renorm) for (int r = 0; r < top; r++) wts[(int64_t)t * slots + r] /= wsum + a.renorm_eps;
-        if (a.scale != 1.0f) for (int r = 0; r < top; r++) wts[(int64_t)t * slots + r] *= a.scale;
+    for (int r = lane; r < top; r += 32) {
+        float w = r < 32 ? mine : wts[(int64_t)t * slots + r];
+        if (a.renorm) w /= wsum + a.renorm_eps;
+        if (a.scale != 1.0f) w *= a.scale;
+        wts[(int64_t)t * slots + r] = w;
     }
     for (int r = lane; r < n_shared; r += 32) {
         ids[(int64_t)t * slots + top + r] = E + r;
@@ -201,7 +205,8 @@ extern "C" CC_API int cc_moe_route_shared(cc_device* dev, const cc_view* x, cons
     const int64_t rows = E + (shared_gate ? 1 : 0), most = tiled ? 16 : 32, rounds = (rows + most - 1) / most;
     const int64_t even = (rows + rounds - 1) / rounds;
     const unsigned threads = 32 * (unsigned)(even < 4 ? 4 : even);
-    if (tiled) cc_launch_pdl(dev, moe_route_kernel<4>, (unsigned)((T + 3) / 4), threads, 4 * one, a);
+    if (tiled && T <= 4 * (int64_t)dev->sm_count) cc_launch_pdl(dev, moe_route_kernel<2>, (unsigned)((T + 1) / 2), threads, 2 * one, a);      // two CTAs fit an SM
+    else if (tiled) cc_launch_pdl(dev, moe_route_kernel<4>, (unsigned)((T + 3) / 4), threads, 4 * one, a);
     else cc_launch_pdl(dev, moe_route_kernel<1>, (unsigned)T, threads, one, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
@@ -319,6 +324,8 @@ static int moe_launch(cc_device* dev, const float* x, const int* ids, const floa
 bool cc_grouped_bf16_supported(int64_t m, int64_t k);
 int cc_launch_grouped_bf16(cc_device* dev, const cc_buf* w_stack, int64_t n_groups, int64_t m, int64_t k, const void* x_bf16, int64_t n_rows, const int* groups_dev,
                            int max_tiles, int block_n, float* out);
+int cc_launch_grouped_glu_bf16(cc_device* dev, const cc_buf* gate_stack, const cc_buf* up_stack, int64_t n_groups, int64_t m, int64_t k, const void* x_bf16, int64_t n_rows, const int* groups_dev,
+                               int max_tiles, int block_n, cc_glu_params act, void* out);
 
 // one CTA: counts per expert (shared-memory atomics), exclusive offsets, the tile table {n_tiles | expert, first row, rows, 0 ...}, and
 // pos[i] = sorted row of entry i = (token, slot).  The order of the rows INSIDE an expert is arbitrary; no value depends on it.
@@ -346,41 +353,59 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) pos[i] += off[moe_clamp(ids[i], E)];
 }
-// xs[pos[i]][:] = bf16(x[i / top][:]) ; one warp per entry
+// xs[pos[i]][:] = bf16(x[i / top][:]) ; one warp per entry, 8 columns a lane where rows allow it (VEC)
+template <bool VEC>
 __global__ void moe_gather_bf16_kernel(const float* __restrict__ x, const int* __restrict__ pos, __nv_bfloat16* __restrict__ xs, int n, int top, int D) {
     pdl_enter();
     const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i >= n) return;
     const float* src = x + (int64_t)(i / top) * D;
     __nv_bfloat16* dst = xs + (int64_t)pos[i] * D;
-    for (int d = lane * 2; d < D; d += 64) *(__nv_bfloat162*)(dst + d) = __floats2bfloat162_rn(src[d], src[d + 1]);
+    if (VEC) {
+#pragma unroll 4
+        for (int d = lane * 8; d < D; d += 256) {
+            const float4 a = *(const float4*)(src + d), b = *(const float4*)(src + d + 4);
+            __nv_bfloat162 o[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w), __floats2bfloat162_rn(b.x, b.y), __floats2bfloat162_rn(b.z, b.w)};
+            *(uint4*)(dst + d) = *(const uint4*)o;
+        }
+    } else
+        for (int d = lane * 2; d < D; d += 64) *(__nv_bfloat162*)(dst + d) = __floats2bfloat162_rn(src[d], src[d + 1]);
 }
-__global__ void moe_glu_bf16_kernel(const float* __restrict__ g, const float* __restrict__ u, __nv_bfloat16* __restrict__ h, int64_t n, cc_glu_params act) {
+// plain units: h = bf16(act(u))
+__global__ void moe_units_bf16_kernel(const float* __restrict__ u, __nv_bfloat16* __restrict__ h, int64_t n, cc_glu_params act) {
     pdl_enter();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (i >= n) return;
     const float2 uv = *(const float2*)(u + i);
-    if (g) {
-        const float2 gv = *(const float2*)(g + i);
-        *(__nv_bfloat162*)(h + i) = __floats2bfloat162_rn(glu_apply(gv.x, uv.x, act), glu_apply(gv.y, uv.y, act));
-    } else {                                                  // a plain unit: act(u)
-        *(__nv_bfloat162*)(h + i) = __floats2bfloat162_rn(act_apply(uv.x, act.act, act.alpha), act_apply(uv.y, act.act, act.alpha));
-    }
+    *(__nv_bfloat162*)(h + i) = __floats2bfloat162_rn(act_apply(uv.x, act.act, act.alpha), act_apply(uv.y, act.act, act.alpha));
 }
 __global__ void moe_activate_kernel(float* __restrict__ x, int64_t n, int act) {
     pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = act_apply(x[i], act);
 }
-// out[t][d] = sum over the slots, in slot order, of weights[t][s] * y[pos[t * top + s]][d]
-__global__ void moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ pos, const float* __restrict__ wts, float* __restrict__ out, int64_t T, int top, int D) {
+// out[t][d] = sum over the slots, in slot order, of weights[t][s] * y[pos[t * top + s]][d].  grid (columns / (128 V), T), V neighbouring columns a thread (an element a thread by a
+// 64-bit division: 6.5 us for 512 tokens of 4 slots, 1024 columns, cold; now 5.0)
+template <int V>
+__global__ void __launch_bounds__(128) moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ pos, const float* __restrict__ wts, float* __restrict__ out, int top, int D) {
     pdl_enter();
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= T * D) return;
-    const int64_t t = i / D; const int d = (int)(i % D);
-    float acc = 0.0f;
-    for (int s = 0; s < top; s++) acc = fmaf(wts[t * top + s], y[(int64_t)pos[t * top + s] * D + d], acc);
-    out[i] = acc;
+    const int d = (blockIdx.x * 128 + threadIdx.x) * V;
+    const int64_t t = blockIdx.y;
+    if (d >= D) return;
+    float acc[V];
+#pragma unroll
+    for (int c = 0; c < V; c++) acc[c] = 0.0f;
+#pragma unroll 4
+    for (int s = 0; s < top; s++) {
+        const float w = wts[t * top + s];
+        const float* row = y + (int64_t)pos[t * top + s] * D + d;
+        if (V == 4) {
+            const float4 v = *(const float4*)row;
+            acc[0] = fmaf(w, v.x, acc[0]); acc[1 % V] = fmaf(w, v.y, acc[1 % V]); acc[2 % V] = fmaf(w, v.z, acc[2 % V]); acc[3 % V] = fmaf(w, v.w, acc[3 % V]);
+        } else acc[0] = fmaf(w, *row, acc[0]);
+    }
+    if (V == 4) *(float4*)(out + t * D + d) = make_float4(acc[0], acc[1 % V], acc[2 % V], acc[3 % V]);
+    else out[t * D + d] = acc[0];
 }
 
 static int moe_grouped(cc_device* dev, const float* x, const int* ids, const float* wts, const cc_buf* wg, const cc_buf* wu, const cc_buf* wd, float* out, int64_t T, int D,
@@ -388,29 +413,32 @@ static int moe_grouped(cc_device* dev, const float* x, const int* ids, const flo
     const int64_t n = T * top;
     const int block_n = n / E >= 96 ? 128 : 64;
     const int max_tiles = (int)((n + block_n - 1) / block_n) + E;
-    // one pool block: pos[n] | table[4 + 4 * max_tiles] | xs bf16 [n][D] | g f32 [n][ff] | u f32 [n][ff] | h bf16 [n][ff] | y f32 [n][D]
+    // one pool block: pos[n] | table[4 + 4 * max_tiles] | xs bf16 [n][D] | u f32 [n][ff] (plain units) | h bf16 [n][ff] | y f32 [n][D]
     auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
-    const size_t o_pos = 0, o_tab = al((size_t)n * 4), o_xs = o_tab + al((size_t)(4 + 4 * max_tiles) * 4), o_g = o_xs + al((size_t)n * D * 2), o_u = o_g + (wg ? al((size_t)n * ff * 4) : 0),
-                 o_h = o_u + al((size_t)n * ff * 4), o_y = o_h + al((size_t)n * ff * 2), total = o_y + al((size_t)n * D * 4);
+    const size_t o_pos = 0, o_tab = al((size_t)n * 4), o_xs = o_tab + al((size_t)(4 + 4 * max_tiles) * 4), o_u = o_xs + al((size_t)n * D * 2),
+                 o_h = o_u + (wg ? 0 : al((size_t)n * ff * 4)), o_y = o_h + al((size_t)n * ff * 2), total = o_y + al((size_t)n * D * 4);
     uint8_t* base = nullptr; size_t cls = 0;
     int rc = cc_pool_alloc(dev, total, (void**)&base, &cls);
     if (rc) return rc;
     int* pos = (int*)(base + o_pos); int* table = (int*)(base + o_tab);
-    __nv_bfloat16* xs = (__nv_bfloat16*)(base + o_xs); float* g = wg ? (float*)(base + o_g) : nullptr; float* u = (float*)(base + o_u);
+    __nv_bfloat16* xs = (__nv_bfloat16*)(base + o_xs); float* u = (float*)(base + o_u);
     __nv_bfloat16* h = (__nv_bfloat16*)(base + o_h); float* y = (float*)(base + o_y);
     cc_launch_pdl(dev, moe_sort_kernel, 1, 1024, (size_t)2 * E * 4, ids, (int)n, E, block_n, pos, table);
     dev->launches++;
-    cc_launch_pdl(dev, moe_gather_bf16_kernel, (unsigned)((n + 7) / 8), 256, 0, x, pos, xs, (int)n, top, D);
+    cc_launch_pdl(dev, D % 8 == 0 && ((uintptr_t)x & 15) == 0 ? moe_gather_bf16_kernel<true> : moe_gather_bf16_kernel<false>, (unsigned)((n + 7) / 8), 256, 0, x, pos, xs, (int)n, top, D);
     dev->launches++;
-    if (wg) rc = cc_launch_grouped_bf16(dev, wg, E, ff, D, xs, n, table, max_tiles, block_n, g);
-    if (!rc) rc = cc_launch_grouped_bf16(dev, wu, E, ff, D, xs, n, table, max_tiles, block_n, u);
-    if (!rc) {
-        cc_launch_pdl(dev, moe_glu_bf16_kernel, (unsigned)((n * ff / 2 + 255) / 256), 256, 0, g, u, h, n * ff, act);
-        dev->launches++;
-        rc = cc_launch_grouped_bf16(dev, wd, E, D, ff, h, n, table, max_tiles, block_n, y);
+    if (wg) rc = cc_launch_grouped_glu_bf16(dev, wg, wu, E, ff, D, xs, n, table, max_tiles, block_n, act, h);
+    else {
+        rc = cc_launch_grouped_bf16(dev, wu, E, ff, D, xs, n, table, max_tiles, block_n, u);
+        if (!rc) {
+            cc_launch_pdl(dev, moe_units_bf16_kernel, (unsigned)((n * ff / 2 + 255) / 256), 256, 0, u, h, n * ff, act);
+            dev->launches++;
+        }
     }
+    if (!rc) rc = cc_launch_grouped_bf16(dev, wd, E, D, ff, h, n, table, max_tiles, block_n, y);
     if (!rc) {
-        cc_launch_pdl(dev, moe_combine_kernel, (unsigned)((T * D + 255) / 256), 256, 0, y, pos, wts, out, T, top, D);
+        if (D % 4 == 0) cc_launch_pdl(dev, moe_combine_kernel<4>, dim3((unsigned)((D / 4 + 127) / 128), (unsigned)T), 128, 0, y, pos, wts, out, top, D);
+        else cc_launch_pdl(dev, moe_combine_kernel<1>, dim3((unsigned)((D + 127) / 128), (unsigned)T), 128, 0, y, pos, wts, out, top, D);
         CC_LAUNCH_CHECK(dev);
     }
     cc_pool_free(dev, base, cls);

@@ -199,6 +199,33 @@ __global__ void __launch_bounds__(256) pb_join_bf16_kernel(PbJoin op, __nv_bfloa
     const int c = (blockIdx.x * 256 + threadIdx.x) * 2, t = blockIdx.y;
     if (c < k) *(__nv_bfloat162*)(out + (int64_t)t * k + c) = __floats2bfloat162_rn(op.at(t, c), op.at(t, c + 1));
 }
+// the same, 8 neighbouring columns per thread, where both parts and the rows of all operands are whole pieces of 16 bytes (SWISH: units known to
+// be that, without the code of the others).
+// grid (columns / 1024, rows).  512 x (1024 + 3072), us: two columns a thread, any unit 6.6 ; here 4.9 (509 x (2048 + 6144): 11.4, 6.4)
+template <bool SWISH>
+__global__ void __launch_bounds__(128) pb_join8_bf16_kernel(PbJoin op, __nv_bfloat16* __restrict__ out, int k) {
+    pdl_enter();
+    const int c = (blockIdx.x * 128 + threadIdx.x) * 8, t = blockIdx.y;
+    if (c >= k) return;
+    float v[8];
+    if (c < op.ca) {
+        const float* a = op.a + (int64_t)t * op.ca + c;
+        *(float4*)v = *(const float4*)a; *(float4*)(v + 4) = *(const float4*)(a + 4);
+    } else {
+        const float *gp = op.g + t * op.rs + (c - op.ca), *up = op.u + t * op.rs + (c - op.ca);
+        float g[8], u[8];
+        *(float4*)g = *(const float4*)gp; *(float4*)(g + 4) = *(const float4*)(gp + 4);
+        *(float4*)u = *(const float4*)up; *(float4*)(u + 4) = *(const float4*)(up + 4);
+        cc_glu_params P = op.P;
+        if (SWISH) P.act = CC_ACT_SWISH;
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[e] = glu_apply(g[e], u[e], P);
+    }
+    __nv_bfloat162 o[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) o[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+    *(uint4*)(out + (int64_t)t * k + c) = *(const uint4*)o;
+}
 __global__ void __launch_bounds__(256) pb_join_f32_kernel(PbJoin op, float* __restrict__ out, int k) {
     pdl_enter();
     const int c = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
@@ -319,7 +346,9 @@ extern "C" CC_API int cc_joined_product_accumulate(cc_device* dev, const cc_view
         void* operand = nullptr;
         int rc = cc_prefill_bf16_operand(dev, T, k, &operand);
         if (rc) return rc;
-        cc_launch_pdl(dev, pb_join_bf16_kernel, dim3((unsigned)((k / 2 + 255) / 256), (unsigned)T), 256, 0, op, (__nv_bfloat16*)operand, (int)k);
+        const bool whole = op.ca % 8 == 0 && ff % 8 == 0 && op.rs % 4 == 0 && (((uintptr_t)op.a | (uintptr_t)op.g | (uintptr_t)op.u | (uintptr_t)operand) & 15) == 0;
+        if (whole) cc_launch_pdl(dev, op.P.act == CC_ACT_SWISH ? pb_join8_bf16_kernel<true> : pb_join8_bf16_kernel<false>, dim3((unsigned)((k / 8 + 127) / 128), (unsigned)T), 128, 0, op, (__nv_bfloat16*)operand, (int)k);
+        else cc_launch_pdl(dev, pb_join_bf16_kernel, dim3((unsigned)((k / 2 + 255) / 256), (unsigned)T), 256, 0, op, (__nv_bfloat16*)operand, (int)k);
         CC_LAUNCH_CHECK(dev);
         return cc_launch_prefill_bf16_operand(dev, w->buf, out, m, k, T, 1);
     }

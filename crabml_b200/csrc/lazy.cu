@@ -680,7 +680,13 @@ struct Fuser {
             bool quantized = false;
             if ((used = try_attention(i, &xb, &quantized))) {
                 i += used;
-                if (size_t u2 = try_stream(i, xb, quantized ? 1 : -1)) i += u2;      // wo consumes the (quantised) attention output
+                const size_t ph0 = P.phases.size();
+                if (size_t u2 = try_stream(i, xb, quantized ? 1 : -1)) {              // wo consumes the (quantised) attention output
+                    i += u2;
+                    // heads that are no whole number of blocks leave the row to be quantised: by every CTA of the product, as in front of the down projection, not in a
+                    // phase of its own (six layers of heads of 48: 3.7 us each and token)
+                    if (!quantized) merge_prologue(ph0);
+                }
                 continue;
             }
             if (is(i, L_MATVEC) && q[i].b.buf->dtype == CC_F32 && (q[i].b.ndim == 1 || q[i].b.shape[0] == 1)) {

@@ -8,6 +8,7 @@
 
 #include <atomic>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <set>
 #include <string>
@@ -90,6 +91,13 @@ struct CommDev {                         // by-value kernel argument: where ever
 };
 struct cc_comm;
 
+// rotation angles of a run of positions: [n][pairs] float2 in the pool, given back by the last who holds them
+struct CcRopeTable {
+    cc_device* dev; int mode; int64_t head_dim, pos, n; int pairs;
+    void* base = nullptr; size_t cls = 0;
+    ~CcRopeTable();
+    const void* rows(int64_t from) const { return (const uint8_t*)base + (size_t)(from - pos) * pairs * 8; }
+};
 struct cc_device {
     int ordinal = 0;
     cc_comm* comm = nullptr;
@@ -125,6 +133,8 @@ struct cc_device {
     size_t dev_idx_bytes = 0;
 
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;    // cc_bench_timer_*
+    std::vector<std::shared_ptr<CcRopeTable>> rope_tables;     // (exact.cu; under rope_mu), the last used behind
+    std::mutex rope_mu;
     // pinned staging of a prompt's rotation angles (exact.cu), two buffers by turns
     void* rope_pinned[2] = {nullptr, nullptr};
     size_t rope_bytes[2] = {0, 0};
@@ -335,8 +345,8 @@ int cc_launch_rms_norm_exact(cc_device* dev, float* x, int64_t rows, int64_t col
 int cc_launch_softmax_exact(cc_device* dev, float* x, int64_t rows, int64_t cols);
 int cc_launch_rope_exact(cc_device* dev, float* x, int64_t n_batch, int64_t batch_stride, int64_t head_dim, int mode,
                          int64_t pos, int64_t rope_dim);
-// the cos / sin of n rows from position pos on, [n][rope_dim / 2] float2 in the pool (the caller gives it back), and the rotation that reads them
-int cc_rope_angles(cc_device* dev, int64_t n, int64_t head_dim, int mode, int64_t pos, int64_t rope_dim, void** table, size_t* cls);
+// the cos / sin of the positions pos .. pos + n - 1 (and perhaps others), and the rotation that reads them
+int cc_rope_angles(cc_device* dev, int64_t n, int64_t head_dim, int mode, int64_t pos, int64_t rope_dim, std::shared_ptr<CcRopeTable>* table);
 int cc_launch_rope_rows(cc_device* dev, float* x, int64_t n_batch, int64_t batch_stride, int64_t head_dim, int mode, int64_t rope_dim, const void* table);
 int cc_launch_bmm_kcontig_exact(cc_device* dev, const float* a, const void* b, int b_dtype, float* c, int64_t ab, int64_t bb,
                                 int64_t m, int64_t k, int64_t n, int64_t sb0, int64_t sb2);

@@ -172,13 +172,12 @@ static uint64_t hash_sig(const std::vector<uint64_t>& s) {
     return h;
 }
 
-// the rotation angles of a prompt's rows: made by the first rotation of the flush that needs them, given back with the flush's steps
+// the rotation angles of a prompt's rows: asked for by the first rotation of the flush that needs them, held by the flush's steps
 struct RopeAngles {
     cc_device* dev; int64_t n, head_dim, pos, rope_dim; int mode;
-    void* table = nullptr; size_t cls = 0;
+    std::shared_ptr<CcRopeTable> table;
     RopeAngles(cc_device* d, int64_t n_, int64_t hd, int m, int64_t p, int64_t rd) : dev(d), n(n_), head_dim(hd), pos(p), rope_dim(rd), mode(m) {}
-    ~RopeAngles() { if (table) cc_pool_free(dev, table, cls); }
-    int ready() { return table ? CC_OK : cc_rope_angles(dev, n, head_dim, mode, pos, rope_dim, &table, &cls); }
+    int ready() { return table ? CC_OK : cc_rope_angles(dev, n, head_dim, mode, pos, rope_dim, &table); }
 };
 
 struct Fuser {
@@ -256,7 +255,7 @@ struct Fuser {
             case L_ROPE:
                 if (ra) {
                     int rc = ra->ready();
-                    return rc ? rc : cc_launch_rope_rows(d, (float*)a.buf->plane[0], op.i1, op.i2, a.shape[a.ndim - 1], (int)op.f, op.rows[0], ra->table);
+                    return rc ? rc : cc_launch_rope_rows(d, (float*)a.buf->plane[0], op.i1, op.i2, a.shape[a.ndim - 1], (int)op.f, op.rows[0], ra->table->rows(op.i0));
                 }
                 return cc_launch_rope_exact(d, (float*)a.buf->plane[0], op.i1, op.i2, a.shape[a.ndim - 1], (int)op.f, op.i0, op.rows[0]);
             case L_CONCAT:

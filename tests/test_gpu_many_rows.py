@@ -37,6 +37,18 @@ def test_rotation_of_many_rows_has_the_reference_bits(dev, mode, shape, pos, dim
         np.testing.assert_array_equal(tensor(dev, x).rope_inplace(mode, pos, dims).export().view(np.uint32), o.export().view(np.uint32))
 
 
+def test_rope_of_positions_asked_for_before_and_not(dev):
+    """Runs of positions inside a kept one, behind it, across its end, of other shapes, more than are kept, longer than one may be: the bits of the rows by themselves"""
+    rng = np.random.default_rng(3)
+    for mode, hd, dims, pos, n in ((0, 64, 64, 0, 40), (0, 64, 64, 5, 30), (0, 64, 64, 40, 24), (0, 64, 64, 30, 60), (0, 64, 32, 3, 20), (1, 64, 64, 3, 20), (0, 128, 128, 7, 20), (0, 64, 64, 900, 33),
+                                   (0, 64, 64, 0, 70), (0, 64, 64, 0, 16500), (0, 64, 64, 16490, 12), (0, 64, 64, 899, 2)):
+        x = rng.standard_normal((n, 2 * hd)).astype(np.float32)
+        got = tensor(dev, x.reshape(n, 2, hd)).rope_inplace(mode, pos, dims).export().reshape(n, 2, hd)
+        for r in {0, 1, n // 2, n - 1}:
+            one = tensor(dev, x[r:r + 1].reshape(1, 2, hd)).rope_inplace(mode, pos + r, dims).export().reshape(2, hd)
+            np.testing.assert_array_equal(got[r].view(np.uint32), one.view(np.uint32))
+
+
 # ---- softmax: many rows and one row at a time give the same bits ------------------------------------------------------------------------------
 @pytest.mark.parametrize("cols", [1, 31, 512, 513, 1025, 2048, 2049])
 def test_softmax_of_many_rows_has_the_bits_of_one(dev, cols):

@@ -291,6 +291,17 @@ __global__ void head_gate_kernel(float* __restrict__ x, const float* __restrict_
     const int64_t u = i / hs, t = u / heads;
     x[i] *= seq_act(g[t * grs + (u - t * heads)], act);
 }
+// the same, four neighbouring elements of a head per thread: grid (columns / 512, rows).  512 x 8 heads of 128, us: one element by 64-bit divisions 5.0 ; here 4.0
+__global__ void __launch_bounds__(128) head_gate4_kernel(float* __restrict__ x, const float* __restrict__ g, int cols, int hs, int64_t grs, int act) {
+    pdl_enter();
+    const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
+    if (c >= cols) return;
+    float4* at = (float4*)(x + (int64_t)blockIdx.y * cols + c);
+    float4 v = *at;
+    const float f = seq_act(g[blockIdx.y * grs + c / hs], act);
+    v.x *= f; v.y *= f; v.z *= f; v.w *= f;
+    *at = v;
+}
 // gate numbers in the columns col0 .. col0 + n_heads of g's rows
 static int head_gate_impl(cc_device* dev, const cc_view* x, const cc_view* g, int32_t col0, int32_t n_heads, int32_t act) {
     SEQ_F32(dev, x, "head_gate x"); SEQ_ROWS(dev, g, "head_gate g");
@@ -298,7 +309,10 @@ static int head_gate_impl(cc_device* dev, const cc_view* x, const cc_view* g, in
                "head_gate: x must be [rows, heads * head_size] and g hold %d columns from column %d on", n_heads, col0);
     const int64_t n = view_len(x);
     if (!n) return CC_OK;
-    cc_launch_pdl(dev, head_gate_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(x), fptr(g) + col0, n, (int)(x->shape[1] / n_heads), n_heads, g->strides[0], act);
+    const int64_t hs = x->shape[1] / n_heads, cols = x->shape[1];
+    if (hs % 4 == 0 && x->shape[0] <= 65535 && ((uintptr_t)fptr(x) & 15) == 0)
+        cc_launch_pdl(dev, head_gate4_kernel, dim3((unsigned)((cols / 4 + 127) / 128), (unsigned)x->shape[0]), 128, 0, fptr(x), fptr(g) + col0, (int)cols, (int)hs, g->strides[0], act);
+    else cc_launch_pdl(dev, head_gate_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(x), fptr(g) + col0, n, (int)hs, n_heads, g->strides[0], act);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1836,30 +1850,30 @@ extern "C" CC_API int cc_latent_query_append_paired(cc_device* dev, const cc_vie
     a.half = half; a.step = step; a.gap = gap; a.mag = mag; a.T = (int)T; a.H = n_heads; a.n_in = (int)dim; a.rest = rest; a.n_out = (int)rank;
     return head_project_few(dev, a);
 }
-// the same for a pass of many rows, whose queries are not folded: one CTA per token copies the queries out of their columns, rotating the last
-// `rest` columns of every head on the way (a pair by the thread of its first column), and warp 0 writes the token's cache row
-__global__ void __launch_bounds__(256) latent_prepare_kernel(const float* __restrict__ q, int64_t qrs, float* __restrict__ out, int H, int dim, LatAppend a) {
+// the same for a pass of many rows, whose queries are not folded: one CTA per token copies the queries out of their columns, a warp a head, rotating the last
+// `rest` columns on the way (a pair by the lane of its first column), and one more warp writes the token's cache row.  512 rows of 8 heads (128 + 64), cache rows of
+// 512 + 64, us: elements dealt to threads by a division, the cache row behind them 5.5 ; here 3.6
+#define LP_WARPS 8
+__global__ void __launch_bounds__(LP_WARPS * 32 + 32) latent_prepare_kernel(const float* __restrict__ q, int64_t qrs, float* __restrict__ out, int H, int dim, LatAppend a) {
     pdl_enter();
-    const int t = blockIdx.x, hs = dim + a.rest;
-    const float* qr = q + t * qrs;
-    float* o = out + (int64_t)t * H * hs;
-    for (int idx = threadIdx.x; idx < H * hs; idx += 256) {
-        const int rel = idx % hs - dim;
-        int pair = -1;                               // index of the pair this thread owns, -2: the pair's second column
-        if (rel >= 0 && rel < 2 * a.half) {
-            if (a.step == 1) pair = rel < a.half ? rel : -2;
-            else pair = (rel & 1) ? -2 : rel >> 1;
-        }
-        if (pair == -2) continue;
-        if (pair >= 0) {
-            float ou, ov;
-            rotate_pair(qr[idx], qr[idx + a.gap], (float)(a.pos0 + t), a.freq[pair], a.mag, ou, ov);
-            o[idx] = ou; o[idx + a.gap] = ov;
-        } else {
-            o[idx] = qr[idx];
-        }
+    const int t = blockIdx.x, hs = dim + a.rest, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w == LP_WARPS) {
+        if (a.ring) latent_append_row(a, t, lane);
+        return;
     }
-    if (a.ring && threadIdx.x < 32) latent_append_row(a, t, threadIdx.x);
+    for (int h = w; h < H; h += LP_WARPS) {
+        const float* src = q + t * qrs + (int64_t)h * hs;
+        float* dst = out + ((int64_t)t * H + h) * hs;
+        for (int i = lane; i < a.half; i += 32) {
+            float ou, ov;
+            const int c = dim + a.step * i;
+            rotate_pair(src[c], src[c + a.gap], (float)(a.pos0 + t), a.freq[i], a.mag, ou, ov);
+            dst[c] = ou; dst[c + a.gap] = ov;
+        }
+#pragma unroll 4
+        for (int c = lane; c < dim; c += 32) dst[c] = src[c];
+        for (int c = dim + 2 * a.half + lane; c < hs; c += 32) dst[c] = src[c];
+    }
 }
 extern "C" CC_API int cc_latent_prepare_append(cc_device* dev, const cc_view* q_src, int32_t q_col0, int32_t n_heads, int32_t dim, int32_t rest, const cc_view* freq, int32_t pairing,
                                                float mag, int64_t pos0, const cc_view* kv_src, int32_t kv_col0, const cc_view* ring, const cc_view* norm_w, float eps, cc_buf** out) {
@@ -1886,7 +1900,7 @@ extern "C" CC_API int cc_latent_prepare_append(cc_device* dev, const cc_view* q_
     if (rc) return rc;
     *out = o;
     if (T == 0) return CC_OK;
-    cc_launch_pdl(dev, latent_prepare_kernel, (unsigned)T, 256, 0, fptr(q_src) + q_col0, q_src->strides[0], (float*)o->base, n_heads, dim, a);
+    cc_launch_pdl(dev, latent_prepare_kernel, (unsigned)T, LP_WARPS * 32 + 32, 0, fptr(q_src) + q_col0, q_src->strides[0], (float*)o->base, n_heads, dim, a);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -1902,6 +1916,15 @@ __global__ void head_concat_shared_kernel(const float* __restrict__ a, const flo
     const int64_t jh = idx / hs, j = jh / H;
     out[idx] = c < dim ? a[jh * dim + c] : shared[j * scols + col0 + (c - dim)];
 }
+// the same, four neighbouring columns per thread: grid (columns of a row / 512, rows).  2048 rows of 8 x (128 + 64), us: one element by 64-bit divisions 14.1 ; here 6.9
+__global__ void __launch_bounds__(128) head_concat_shared4_kernel(const float* __restrict__ a, const float* __restrict__ shared, float* __restrict__ out, int H, int dim, int rest, int scols, int col0) {
+    pdl_enter();
+    const int hs = dim + rest, at = (blockIdx.x * 128 + threadIdx.x) * 4;
+    if (at >= H * hs) return;
+    const int h = at / hs, c = at - h * hs;
+    const int64_t j = blockIdx.y;
+    *(float4*)(out + j * H * hs + at) = c < dim ? *(const float4*)(a + (j * H + h) * dim + c) : *(const float4*)(shared + j * scols + col0 + (c - dim));
+}
 extern "C" CC_API int cc_head_concat_shared(cc_device* dev, const cc_view* a, const cc_view* shared, int32_t n_heads, int32_t col0, int32_t rest, cc_buf** out) {
     SEQ_ENTER(dev, "head_concat_shared");
     if (!out) return cc_fail(dev, CC_ERR_ARG, "head_concat_shared: out is NULL");
@@ -1916,7 +1939,10 @@ extern "C" CC_API int cc_head_concat_shared(cc_device* dev, const cc_view* a, co
     *out = o;
     const int64_t n = rows * n_heads * (dim + rest);
     if (n == 0) return CC_OK;
-    cc_launch_pdl(dev, head_concat_shared_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(a), fptr(shared), (float*)o->base, n, n_heads, (int)dim, rest, (int)shared->shape[1], col0);
+    const int scols = (int)shared->shape[1];
+    if (dim % 4 == 0 && rest % 4 == 0 && scols % 4 == 0 && col0 % 4 == 0 && rows <= 65535 && (((uintptr_t)fptr(a) | (uintptr_t)fptr(shared)) & 15) == 0)
+        cc_launch_pdl(dev, head_concat_shared4_kernel, dim3((unsigned)((n_heads * (dim + rest) / 4 + 127) / 128), (unsigned)rows), 128, 0, fptr(a), fptr(shared), (float*)o->base, n_heads, (int)dim, rest, scols, col0);
+    else cc_launch_pdl(dev, head_concat_shared_kernel, (unsigned)((n + 255) / 256), 256, 0, fptr(a), fptr(shared), (float*)o->base, n, n_heads, (int)dim, rest, scols, col0);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }

@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(MV_THREADS) matvec_kernel(WPlanes W, const voi
 
 // a few activation rows (2 .. 31: several sequences' next tokens): the grid above fetches and unpacks the weights once per row.  Here a warp takes two weight
 // rows and NB activations at a time (vecdot.cuh rows_dot); a CTA stages its NB activations once and walks over the weight rows.
-// Q4_K, 11008 x 4096, 8 rows: 58 -> 37 us (whole call 77 -> 48) for 25 MB of weights (3.9 us at the copy rate); bound by the integer dot products and the
+// Q5_K and Q6_K, and Q4_K up to 4 rows or of very long ones; with one row a time Q4_K, 11008 x 4096, 8 rows took 58 us, so 37; bound by the integer dot products and the
 // activation reads from shared memory (a 16-byte weight chunk meets 2 x NB 16-byte activation chunks)
 template <class T, int NB>
 __global__ void __launch_bounds__(MV_THREADS) matvec_few_kernel(WPlanes W, const void* act, int64_t n_total, float* __restrict__ out, int m, int k, int b) {
@@ -63,6 +63,134 @@ static int launch_few(cc_device* dev, const WPlanes& W, const void* act, int64_t
     int64_t ctas = most / groups > 0 ? most / groups : 1;
     if (ctas > need) ctas = need;
     cc_launch_pdl(dev, matvec_few_kernel<T, NB>, dim3((unsigned)ctas, (unsigned)groups), MV_THREADS, smem, W, act, n_total, out, (int)m, (int)k, (int)b);
+    CC_LAUNCH_CHECK(dev);
+    return CC_OK;
+}
+// The same for Q4_K on the integer tensor cores.  An mma of 16 x 8 x 16 sums the 16 weights of a chunk's nibbles for 16 weight rows and 8 activations: exactly the
+// integers of vecdot.cuh, whose terms follow from them in the same order.  There a lane (super-block mod 4, chunk) adds up its terms and the
+// butterfly the lanes; here warp q of four has the super-blocks q, q + 4, .. of the 16 rows and a sum for each of the 8 chunks, and the four warps' sums are
+// added up in shared memory in the butterfly's order: identical bits.  A lane holds the weights of two rows at 4 columns of a chunk; activations come by ldmatrix.
+// Bound by the latency of the weights (16 warps an SM, a super-block of 16 rows each ahead) and the 9 instructions an output and chunk behind the mma.
+// us with the quantisation of the rows, 11008 x 4096 x 8 / 16 / 31 rows: two weight rows a warp by dp4a 31.4 / 44.1 / 74.2 ; here 27.2 / 37.3 / 54.4 ; 32000 x 4096 61 / 103 / 184 ; 48 / 72 /
+// 128.  CTAs of one group of warps: 26.9 / 41.9 / 66.4.  Q6_K the same way: 31.6 by dp4a, 43.4 here (its numbers take twice the instructions to put together).
+#define MM_THREADS 256
+#define MM_GROUPS (MM_THREADS / 128)
+#define MM_OUT 128                         // outputs of four warps: 16 rows x 8 activations
+__device__ __forceinline__ void mm_mma(int (&c)[4], unsigned a0, unsigned a1, unsigned b) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(b));
+}
+__device__ __forceinline__ unsigned mm_word(const uint8_t* p) { return __ldg((const unsigned*)p); }
+// one super-block of rows ra, rb (of the plane's rows) against 8 activations: acc[chunk][output]
+struct MmBlock {
+    unsigned w[2][8];
+    int4 h[2];
+    __device__ __forceinline__ void load(const WPlanes& W, int64_t ra, int64_t rb, int nsb, int sb, int c) {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const uint8_t* blk = W.p[0] + ((r ? rb : ra) * nsb + sb) * 144;
+            h[r] = __ldg((const int4*)blk);
+#pragma unroll
+            for (int j = 0; j < 8; j++) w[r][j] = mm_word(blk + 16 + 16 * j + 4 * c);
+        }
+    }
+    __device__ __forceinline__ void add(float (&acc)[8][4], const unsigned (&b)[16], const uint8_t* const (&act)[2], int k, int sb) const {
+        unsigned s[2][2], mn[2][2];
+        float d[4], dm[4];
+        int4 bs[2][2];                                           // block sums of the two activations, two 16-bit numbers a word
+#pragma unroll
+        for (int n = 0; n < 2; n++) {
+            KAct A(act[n], k);
+            const int4* at = (const int4*)(A.bs + sb * 16);
+            bs[n][0] = at[0]; bs[n][1] = at[1];
+            const float da = A.d[sb];
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                d[r * 2 + n] = h2f_bits((uint16_t)(h[r].x & 0xFFFF)) * da;
+                dm[r * 2 + n] = h2f_bits((uint16_t)((unsigned)h[r].x >> 16)) * da;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; r++) k4_unpack((unsigned)h[r].y, (unsigned)h[r].z, (unsigned)h[r].w, s[r][0], s[r][1], mn[r][0], mn[r][1]);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0}, sums[2];
+            mm_mma(lo, w[0][j] & 0x0F0F0F0Fu, w[1][j] & 0x0F0F0F0Fu, b[j]);
+            mm_mma(hi, (w[0][j] >> 4) & 0x0F0F0F0Fu, (w[1][j] >> 4) & 0x0F0F0F0Fu, b[8 + j]);
+            const int g = j >> 1;
+#pragma unroll
+            for (int n = 0; n < 2; n++) {
+                const int4 v = bs[n][j >> 2];
+                const int x = (j & 3) == 0 ? v.x : (j & 3) == 1 ? v.y : (j & 3) == 2 ? v.z : v.w;
+                sums[n] = (int)(int16_t)(x & 0xFFFF) + (x >> 16);
+            }
+#pragma unroll
+            for (int o = 0; o < 4; o++) {
+                const int r = o >> 1, n = o & 1;
+                const int isum = byte_of(s[r][0], s[r][1], 2 * g) * lo[o] + byte_of(s[r][0], s[r][1], 2 * g + 1) * hi[o], msum = sums[n] * byte_of(mn[r][0], mn[r][1], j);
+                acc[j][o] += d[o] * (float)isum - dm[o] * (float)msum;
+            }
+        }
+    }
+};
+// distance of two activations in shared memory: an odd number of 16-byte pieces, so that 8 of them lie in different banks
+__host__ __device__ __forceinline__ int mm_stride(int bytes) { return (bytes & 16) ? bytes : bytes + 16; }
+__global__ void __launch_bounds__(MM_THREADS, 512 / MM_THREADS) matvec_mma_kernel(WPlanes W, const void* act, int64_t n_total, float* __restrict__ out, int m, int k, int b) {
+    pdl_enter();
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int b0 = blockIdx.y * 8, stride = mm_stride(TQ45_K<false>::smem_bytes(k)), nsb = k >> 8;
+    float* part = (float*)(smem + 8 * stride);                                 // [groups][4 warps][8 chunks][MM_OUT]
+    for (int n = 0; n < 8; n++) TQ45_K<false>::stage_act(act, n_total, min(b0 + n, b - 1), k, smem + n * stride);       // activations behind the last repeat it
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = warp & 3, group = warp >> 2, c = lane & 3;
+    const uint8_t* const mine[2] = {smem + 2 * c * stride, smem + (2 * c + 1) * stride};      // the activations of this lane's outputs
+    const unsigned rows = (unsigned)__cvta_generic_to_shared(smem + (lane & 7) * stride) + ((lane & 8) ? 128 : 0) + ((lane & 16) ? 16 : 0);      // ldmatrix: chunks j, j + 8, j + 1, j + 9
+    for (int t = blockIdx.x; t * (16 * MM_GROUPS) < m; t += gridDim.x) {
+        const int row0 = t * (16 * MM_GROUPS) + group * 16;
+        const int64_t ra = min(row0 + (lane >> 2), m - 1), rb = min(row0 + (lane >> 2) + 8, m - 1);
+        float acc[8][4];
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+        if (row0 < m) {
+            MmBlock blk;
+            if (q < nsb) blk.load(W, ra, rb, nsb, q, c);
+#pragma unroll 1
+            for (int sb = q; sb < nsb; sb += 4) {
+                unsigned bx[16];
+#pragma unroll
+                for (int j = 0; j < 8; j += 2)
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(bx[j]), "=r"(bx[8 + j]), "=r"(bx[j + 1]), "=r"(bx[9 + j]) : "r"(rows + sb * 256 + j * 16));
+                const MmBlock now = blk;
+                if (sb + 4 < nsb) blk.load(W, ra, rb, nsb, sb + 4, c);
+                now.add(acc, bx, mine, k, sb);
+            }
+        }
+        float* to = part + ((group * 4 + q) * 8) * MM_OUT + lane * 4;
+#pragma unroll
+        for (int j = 0; j < 8; j++) *(float4*)(to + j * MM_OUT) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+        __syncthreads();
+        const int o = threadIdx.x & (MM_OUT - 1);                              // output o of this thread's group: lane o / 4, number o % 4 of it
+        const float* from = part + (threadIdx.x / MM_OUT) * (32 * MM_OUT) + o;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = (from[j * MM_OUT] + from[(16 + j) * MM_OUT]) + (from[(8 + j) * MM_OUT] + from[(24 + j) * MM_OUT]);
+        const float sum = ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+        const int row = t * (16 * MM_GROUPS) + (threadIdx.x / MM_OUT) * 16 + (o >> 4) + ((o & 2) ? 8 : 0), n = b0 + ((o >> 2) & 3) * 2 + (o & 1);
+        if (row < m && n < b) out[(int64_t)n * m + row] = sum;
+        __syncthreads();                                                       // the next tile's sums go where these were
+    }
+}
+static bool mm_fits(int64_t k) { return 8 * (int64_t)(TQ45_K<false>::smem_bytes((int)k) + 16) + MM_GROUPS * 32 * MM_OUT * 4 <= 200 * 1024; }
+static int launch_mma(cc_device* dev, const cc_buf* w, const void* act, int64_t n_total, float* out, int64_t m, int64_t k, int64_t b) {
+    WPlanes W;
+    for (int i = 0; i < CC_MAX_PLANES; i++) W.p[i] = w->plane[i];
+    const int smem = 8 * mm_stride(TQ45_K<false>::smem_bytes((int)k)) + MM_GROUPS * 32 * MM_OUT * 4;
+    CC_CUDA(dev, cudaFuncSetAttribute(matvec_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const int64_t groups = (b + 7) / 8, need = (m + 16 * MM_GROUPS - 1) / (16 * MM_GROUPS), fit = 224 * 1024 / (smem + 1024), most = dev->sm_count * (fit < 512 / MM_THREADS ? fit : 512 / MM_THREADS);
+    int64_t ctas = most / groups > 0 ? most / groups : 1;
+    if (ctas > need) ctas = need;
+    cc_launch_pdl(dev, matvec_mma_kernel, dim3((unsigned)ctas, (unsigned)groups), MM_THREADS, smem, W, act, n_total, out, (int)m, (int)k, (int)b);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
@@ -111,7 +239,10 @@ int cc_launch_matvec(cc_device* dev, const cc_buf* w, const void* act, const flo
     case CC_Q5_1: return launch<TQx_1<true>>(dev, w, act, n_total, out, m, k, b);
     case CC_Q2_K: return launch<TQ2_K>(dev, w, act, n_total, out, m, k, b);
     case CC_Q3_K: return launch<TQ3_K>(dev, w, act, n_total, out, m, k, b);
-    case CC_Q4_K: return launch_rows<TQ45_K<false>>(dev, w, act, n_total, out, m, k, b);
+    case CC_Q4_K:
+        // (up to 4 rows the dp4a kernel: 11008 x 4096, 4 rows 20.1 us by it, 25.5 here ; from 5 on it takes 8 rows' time for each 8: 31.4 and 27.3)
+        if (b > 4 && mm_fits(k)) return launch_mma(dev, w, act, n_total, out, m, k, b);
+        return launch_rows<TQ45_K<false>>(dev, w, act, n_total, out, m, k, b);
     case CC_Q5_K: return launch_rows<TQ45_K<true>>(dev, w, act, n_total, out, m, k, b);
     case CC_Q6_K: return launch_rows<TQ6_K>(dev, w, act, n_total, out, m, k, b);
     case CC_Q8_K: return launch<TQ8_K>(dev, w, act, n_total, out, m, k, b);

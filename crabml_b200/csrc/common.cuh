@@ -367,7 +367,7 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 // early: false for a long kernel of fewer CTAs than SMs: started beside the one before, some SMs get two of its CTAs and others none (the delta rule's 128
-// CTAs: 397 -> 439 us a call; attention over a long cache 40 -> 52 us)
+// CTAs: 397 -> 439 us a call)
 template <class... K, class... A>
 static inline cudaError_t cc_launch_when(bool early, cc_device* dev, void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, A... args) {
     cudaLaunchConfig_t cfg = {};

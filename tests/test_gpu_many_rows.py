@@ -339,6 +339,12 @@ def test_few_rows_have_the_bits_of_one(dev, t, m, k, b):
         np.testing.assert_array_equal(got[i].view(np.uint32), w.matmul_vec(tensor(dev, x[i:i + 1])).export().view(np.uint32))
 
 
+@pytest.mark.parametrize("m,k,b", [(1, 256, 5), (16, 512, 6), (31, 768, 7), (32, 1280, 8), (47, 1536, 12), (9600, 256, 17), (4800, 2048, 5), (3, 18944, 31)])
+def test_few_rows_of_q4_k_have_the_bits_of_one(dev, m, k, b):
+    """Edges of the tiles of 16 and 32 rows and of 8 activations, super-blocks fewer than warps and no multiple of 4, more tiles than CTAs"""
+    test_few_rows_have_the_bits_of_one(dev, oc.Q4_K, m, k, b)
+
+
 @pytest.mark.parametrize("t", [oc.Q8_0, oc.Q4_0, oc.Q5_0])
 @pytest.mark.parametrize("m,k,b", [(1, 32, 2), (33, 288, 3), (40, 1056, 8), (257, 4096, 9), (17, 14336, 31), (16, 40960, 5)])
 def test_few_rows_against_the_oracle(dev, t, m, k, b):

@@ -254,3 +254,45 @@ def test_bad_arguments_are_tensor_errors(dev):
     kring = CudaTensor.alloc([4, 8], capi.F32, dev); vring = CudaTensor.alloc([4, 8], capi.F32, dev)
     with pytest.raises(TensorError):                                                                      # window 6 needs more rows than the ring has
         seqops.window_attention(T32(dev, np.zeros((1, 8))), None, 0.0, kring, vring, 10, 1, 1, 8, 8, 6, 1.0)
+
+
+@pytest.mark.parametrize("act,alpha,limit,shift", [(capi.ACT_SILU, 1.0, 0.0, 0.0), (capi.ACT_SWISH, 1.702, 1.0, 1.0), (capi.ACT_SILU, 1.0, 0.5, 0.0)])
+@pytest.mark.parametrize("T,E,ff,top", [(65, 2, 64, 2), (129, 3, 128, 3), (200, 2, 320, 1), (300, 3, 192, 2)])
+def test_grouped_gate_and_up_with_their_unit(dev, act, alpha, limit, shift, T, E, ff, top):
+    """Rows and units at the edges of 64- and 128-row tiles, every form of the unit, against the same steps in 64 bits with the roundings to bfloat16 in their places"""
+    from crabml_b200 import CudaTensor
+    D = 64
+    rng = np.random.default_rng(T + ff)
+    x = rng.standard_normal((T, D)).astype(np.float32)
+    wg, wu, wd = (bf16(rng.standard_normal(s) / np.sqrt(s[-1])) for s in ((E, ff, D), (E, ff, D), (E, D, ff)))
+    ids = np.stack([rng.permutation(E)[:top] for _ in range(T)]).astype(np.int32)
+    wts = rng.uniform(0.1, 0.6, (T, top)).astype(np.float32)
+    got = seqops.moe_experts_glu(T32(dev, x), CudaTensor.from_cpu(ids, [T, top], capi.I32, dev), T32(dev, wts), W(dev, wg.reshape(E * ff, D), capi.BF16), W(dev, wu.reshape(E * ff, D), capi.BF16),
+                                 W(dev, wd.reshape(E * D, ff), capi.BF16), E, ff, act=act, alpha=alpha, limit=limit, up_shift=shift).export().reshape(T, D)
+    want, xb = np.zeros((T, D)), bf16(x).astype(np.float64)
+    for e in range(E):
+        g, u = xb @ wg[e].astype(np.float64).T, xb @ wu[e].astype(np.float64).T
+        if limit > 0:
+            g, u = np.minimum(g, limit), np.clip(u, -limit, limit)
+        h = bf16((g / (1 + np.exp(-alpha * g)) * (u + shift)).astype(np.float32)).astype(np.float64)
+        want += (h @ wd[e].astype(np.float64).T) * (wts * (ids == e)).sum(-1, keepdims=True)
+    # a unit beside a rounding boundary of bfloat16 may fall to the other side: 2^-8 of a hidden number of order one, times a weight of 1 / sqrt(ff); a few of them
+    assert np.abs(got - want).max() < 2e-2
+
+
+@pytest.mark.parametrize("T", [127, 128, 591, 593])
+@pytest.mark.parametrize("top,renorm", [(1, 0), (4, 1), (40, 1)])
+def test_router_choices_and_their_weights(dev, T, top, renorm):
+    """Calls around the limits of one, two and four tokens a CTA; more choices than a warp has lanes; weights that are renormalised"""
+    D, E = 48, 48
+    rng = np.random.default_rng(T + top)
+    x, wr = rng.standard_normal((T, D)).astype(np.float32), (rng.standard_normal((E, D)) * 0.4).astype(np.float32)
+    ids, wts = seqops.moe_route(T32(dev, x), T32(dev, wr), None, top, 1, 1, bool(renorm))
+    ids, wts = ids.export().view(np.int32).reshape(T, top), wts.export().reshape(T, top)
+    s = x.astype(np.float64) @ wr.T.astype(np.float64)
+    p = np.exp(s - s.max(-1, keepdims=True))
+    p /= p.sum(-1, keepdims=True)
+    got = np.take_along_axis(p, ids, 1)
+    best = -np.sort(-p, -1)[:, :top]
+    assert np.abs(got - best).max() < 1e-6 and all(len(set(r)) == top for r in ids)
+    assert np.abs(wts - (got / got.sum(-1, keepdims=True) if renorm else got)).max() < 2e-6

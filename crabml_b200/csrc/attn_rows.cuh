@@ -16,10 +16,8 @@
 // What bounds it: for few heads a key head the cache's bytes; for 16 heads over one latent row the reads of shared memory (12 of 16 bytes for 128 multiply-adds of
 // a lane), and for short caches the chain launch, first load, sums.
 #pragma once
+#include "attn_rows_lanes.cuh"
 
-#define AR_THREADS 512
-#define AR_WARPS (AR_THREADS / 32)
-#define AR_COLS 1024                     // value columns of a unit
 #define AR_MACS (1 << 18)                // a slice has this many multiply-adds or AR_BYTES bytes, whichever are fewer keys, as long as there are SMs without one
 #define AR_BYTES (1 << 17)
 #define AR_LEAST 4                       // long caches: 4 slices at least, so that 64 sums or more of few terms are added up whatever the number of heads
@@ -98,7 +96,7 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned kcb = blockIdx.z / (unsigned)A.cblocks, ukv = kcb / (unsigned)A.hblocks;
     const int slice = blockIdx.x, t = blockIdx.y, cb = (int)(blockIdx.z - kcb * A.cblocks), hb = (int)(kcb - ukv * A.hblocks), kvh = (int)ukv;
-    const int h0 = kvh * g.R + hb * HB, nh = min(HB, g.R - hb * HB), c_first = cb * AR_COLS, cols = min(AR_COLS, g.dv - c_first);
+    const int h0 = kvh * g.R + hb * HB, nh = min(HB, g.R - hb * HB), c_first = cb * AR_COLS, cols = ar_cols(g.dv, cb);
     const int64_t i = g.pos0 + t, lo = wa_lo(g, i);
     const int n = (int)(i - lo) + 1, slices = ar_slices(n, A.quantum, A.cap);     // n: at most the ring's rows
     if (slice >= slices) return;
@@ -106,10 +104,9 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
     const float* kbase = A.k + (int64_t)kvh * g.dk;
     const float* vbase = A.v + (int64_t)kvh * g.vhs + c_first;
     const float* qrow = A.q + ((int64_t)t * g.H + h0) * g.dk;
-    // a warp's part of the values: 128 columns, HS heads, every kgs-th key of a tile
-    const int cgs = (A.dvp + 127) / 128, kgs = AR_WARPS / (cgs * HG), cg = w % cgs, hg = w / cgs % HG, kg = w / (cgs * HG);
-    const int col = cg * 128 + lane * 4;
-    const bool on = kg < kgs && col < A.dvp;
+    const ArLane at_v = ar_lane(w, lane, A.dvp, cols, HG);
+    const int kgs = at_v.kgs, hg = at_v.hg, kg = at_v.kg, col = at_v.col;
+    const bool loads = at_v.loads;
     pdl_enter();                                                   // up to here nothing but the arguments
     float4 acc[HS];
 #pragma unroll
@@ -208,7 +205,7 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
         if constexpr (HB <= 2) {
 #pragma unroll
             for (int x = 0; x < EARLY; x++)
-                if (on && kg + x * kgs < mc) early[x] = value4(kg + x * kgs);
+                if (loads && kg + x * kgs < mc) early[x] = value4(kg + x * kgs);
         }
         __syncthreads();
         for (int h = w; h < HB; h += AR_WARPS) {                   // scores -> weights relative to the largest so far; none where there is no score but -inf
@@ -250,7 +247,7 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
             }
         };
         if constexpr (DIRECT) {
-            if (on) {
+            if (loads) {
                 int c = kg;
                 if constexpr (HB <= 2) {
 #pragma unroll
@@ -270,7 +267,7 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
                 }
                 const float* vt = ring + (size_t)((A.keep ? j : nk + j) % A.stages) * A.tile * A.rs;
                 const int at = j * A.tile, rows = min(A.tile, mc - at);
-                if (on) {
+                if (loads) {
 #pragma unroll 4
                     for (int c = kg; c < rows; c += kgs) add(*(const float4*)(vt + (size_t)c * A.rs + col), sc + (at + c) * PS + hg * HS);
                 }
@@ -283,7 +280,7 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
     // the warps' sums, in the order of the key groups
     const int row4 = A.dvp / 4, items = HB * row4;             // float4 numbers
     float4* red = (float4*)ring;
-    if (on) {
+    if (at_v.sums) {
 #pragma unroll
         for (int h = 0; h < HS; h++) red[kg * items + (hg * HS + h) * row4 + col / 4] = acc[h];
     }
@@ -395,7 +392,7 @@ static int attn_rows(cc_device* dev, const WaGeom& g, ArArgs A, int reach) {
     const bool lat = A.v == A.k && g.vrs == g.krs;
     A.dkp = (g.dk + 3) & ~3;
     A.cblocks = (g.dv + AR_COLS - 1) / AR_COLS;
-    A.dvp = ((A.cblocks > 1 ? AR_COLS : g.dv) + 3) & ~3;
+    A.dvp = ar_dvp(g.dv);
     A.vec = g.dk % 4 == 0 && g.krs % 4 == 0 && g.vrs % 4 == 0 && g.vhs % 4 == 0 && g.dv % 4 == 0 && (((uintptr_t)A.k | (uintptr_t)A.v) & 15) == 0;
     A.qvec = g.dk % 4 == 0 && ((uintptr_t)A.q & 15) == 0;
     int HB = g.R > 8 ? 16 : g.R > 4 ? 8 : g.R > 2 ? 4 : g.R;

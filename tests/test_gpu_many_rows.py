@@ -267,6 +267,7 @@ def test_attention_of_few_queries(dev, T, pos0, H, G, d, window, sink):
     (1, 700, 2, 1, 64, 64, False), (1, 9000, 2, 1, 16, 16, False),                             # weights in one piece, in several
     (2, 31, 8, 1, 576, 512, True), (1, 32, 5, 1, 576, 512, True), (1, 500, 16, 1, 576, 512, True), (1, 65, 17, 1, 132, 131, True), (1, 1200, 64, 1, 80, 80, False),
     (1, 13000, 16, 1, 576, 512, True),                                                         # slices too long to stay in shared memory
+    (1, 40, 1, 1, 64, 1025, False), (1, 40, 2, 1, 64, 1028, False), (2, 40, 4, 1, 64, 1025, False), (1, 300, 8, 2, 32, 1028, False), (1, 40, 8, 1, 64, 1028, False), (1, 5, 1, 1, 64, 2049, False),      # a last block of few columns
     (1, 300, 9, 1, 256, 256, False), (1, 40, 2, 1, 64, 1500, False), (1, 40, 2, 1, 5000, 64, False), (1, 40, 16, 1, 2000, 40, True)])
 def test_attention_of_few_queries_at_the_edges_of_its_slices(dev, T, n, H, G, dk, dv, latent):
     """Edges of slices, tiles and blocks of heads and columns, a ring that wraps around, and the order of a row's sums beside other rows"""

@@ -384,13 +384,13 @@ __global__ void moe_activate_kernel(float* __restrict__ x, int64_t n, int act) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = act_apply(x[i], act);
 }
-// out[t][d] = sum over the slots, in slot order, of weights[t][s] * y[pos[t * top + s]][d].  grid (columns / (128 V), T), V neighbouring columns a thread (an element a thread by a
-// 64-bit division: 6.5 us for 512 tokens of 4 slots, 1024 columns, cold; now 5.0)
+// out[t][d] = sum over the slots, in slot order, of weights[t][s] * y[pos[t * top + s]][d].  grid (T, columns / (128 V)) -- only the first may be more than 65535 --, V neighbouring columns a
+// thread (an element a thread by a 64-bit division: 6.5 us for 512 tokens of 4 slots, 1024 columns, cold; now 5.0)
 template <int V>
 __global__ void __launch_bounds__(128) moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ pos, const float* __restrict__ wts, float* __restrict__ out, int top, int D) {
     pdl_enter();
-    const int d = (blockIdx.x * 128 + threadIdx.x) * V;
-    const int64_t t = blockIdx.y;
+    const int d = (blockIdx.y * 128 + threadIdx.x) * V;
+    const int64_t t = blockIdx.x;
     if (d >= D) return;
     float acc[V];
 #pragma unroll
@@ -437,8 +437,8 @@ static int moe_grouped(cc_device* dev, const float* x, const int* ids, const flo
     }
     if (!rc) rc = cc_launch_grouped_bf16(dev, wd, E, D, ff, h, n, table, max_tiles, block_n, y);
     if (!rc) {
-        if (D % 4 == 0) cc_launch_pdl(dev, moe_combine_kernel<4>, dim3((unsigned)((D / 4 + 127) / 128), (unsigned)T), 128, 0, y, pos, wts, out, top, D);
-        else cc_launch_pdl(dev, moe_combine_kernel<1>, dim3((unsigned)((D + 127) / 128), (unsigned)T), 128, 0, y, pos, wts, out, top, D);
+        if (D % 4 == 0) cc_launch_pdl(dev, moe_combine_kernel<4>, dim3((unsigned)T, (unsigned)((D / 4 + 127) / 128)), 128, 0, y, pos, wts, out, top, D);
+        else cc_launch_pdl(dev, moe_combine_kernel<1>, dim3((unsigned)T, (unsigned)((D + 127) / 128)), 128, 0, y, pos, wts, out, top, D);
         CC_LAUNCH_CHECK(dev);
     }
     cc_pool_free(dev, base, cls);

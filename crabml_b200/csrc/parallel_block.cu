@@ -26,13 +26,15 @@ int cc_launch_dense_tile(cc_device* dev, const cc_buf* w, const float* x, float*
 
 #define PB_COLS 1024                       // columns of the operand that a warp holds, 32 a lane
 #define PB_TURNS 32                        // rows of a warp whose sums wait in shared memory
+#define PB_DEPTH 4                         // 16-byte pieces of a weight row that a lane has in flight where the operand stays in shared memory
 #define PB_LN_THREADS 256
 
 // what the operand's rows are made of
 struct PbNorm {
     const float *x, *w, *b;                // x: [T, k] contiguous; b NULL: no bias
     float eps;
-    template <int THREADS>
+    static constexpr bool NORM = true;
+    template <int THREADS, int EACH>
     __device__ __forceinline__ void stage(float* dst, int t, int k, float* red, bool round) const {
         layer_norm_row<THREADS>(x + (int64_t)t * k, w, b, k, eps, red, [&](int c, float v) { dst[c] = round ? __bfloat162float(__float2bfloat16_rn(v)) : v; });
     }
@@ -45,9 +47,16 @@ struct PbJoin {
     __device__ __forceinline__ float at(int t, int c) const {
         return c < ca ? a[(int64_t)t * ca + c] : glu_apply(g[t * rs + (c - ca)], u[t * rs + (c - ca)], P);
     }
-    template <int THREADS>
+    static constexpr bool NORM = false;
+    template <int THREADS, int EACH>
     __device__ __forceinline__ void stage(float* dst, int t, int k, float*, bool round) const {
-        constexpr int EACH = 4096 / THREADS;
+        if constexpr (EACH == 1) {
+            for (int c = threadIdx.x; c < k; c += THREADS) {
+                const float v = at(t, c);
+                dst[c] = round ? __bfloat162float(__float2bfloat16_rn(v)) : v;
+            }
+            return;
+        }
         for (int c0 = threadIdx.x; c0 < k; c0 += EACH * THREADS) {       // the numbers of EACH columns at once
             float x[EACH], y[EACH];
 #pragma unroll
@@ -111,7 +120,7 @@ __global__ void __launch_bounds__(THREADS, 1) pb_matvec_kernel(const void* __res
     }
     pdl_enter();
     if (vec) fetch(cur, 0, 0);
-    op.template stage<THREADS>(pb_sm, t, k, red, BF16W);
+    op.template stage<THREADS, 4>(pb_sm, t, k, red, BF16W);
     __syncthreads();
     for (int it0 = 0; it0 < rows_it; it0 += PB_TURNS) {
         const int turns = min(PB_TURNS, rows_it - it0);
@@ -178,6 +187,95 @@ __global__ void __launch_bounds__(THREADS, 1) pb_matvec_kernel(const void* __res
         if (it0 + PB_TURNS < rows_it) __syncthreads();            // part is written again
     }
 }
+__device__ __forceinline__ float pb_dot8(const int4 v, const float* a, float acc) {
+    const float4 a0 = *(const float4*)a, a1 = *(const float4*)(a + 4);
+    acc = fmaf(__uint_as_float((unsigned)v.x << 16), a0.x, acc); acc = fmaf(__uint_as_float((unsigned)v.x & 0xFFFF0000u), a0.y, acc);
+    acc = fmaf(__uint_as_float((unsigned)v.y << 16), a0.z, acc); acc = fmaf(__uint_as_float((unsigned)v.y & 0xFFFF0000u), a0.w, acc);
+    acc = fmaf(__uint_as_float((unsigned)v.z << 16), a1.x, acc); acc = fmaf(__uint_as_float((unsigned)v.z & 0xFFFF0000u), a1.y, acc);
+    acc = fmaf(__uint_as_float((unsigned)v.w << 16), a1.z, acc); acc = fmaf(__uint_as_float((unsigned)v.w & 0xFFFF0000u), a1.w, acc);
+    return acc;
+}
+// The same with the operand row in shared memory, where one batch of PB_DEPTH pieces a lane is all of a warp's part or a CTA has few rows (pb_launch_matvec): half the
+// registers, 32 warps, a sum of one chain.  `split` warps share a row, each a contiguous stretch of its pieces in lane-strided order; a lane keeps the next pieces -- of
+// this row or of the next one -- in flight while it multiplies the current ones.  Partial sums: the butterfly, then the row's warps in ascending order.
+template <bool BF16W, class Op>
+__global__ void __launch_bounds__(1024, 1) pb_matvec_shared_kernel(const void* __restrict__ W, Op op, float* __restrict__ out, int m, int k, int split, int accumulate) {
+    extern __shared__ __align__(16) float pb_sm[];              // the operand row, k floats (rounded up to 4)
+    __shared__ float red[32];
+    const int t = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per_cta = 32 / split, sub = warp % split, slot = warp / split;
+    const int rows_it = (m + gridDim.x * per_cta - 1) / (gridDim.x * per_cta);
+    const int row0 = blockIdx.x * per_cta + slot, row_step = gridDim.x * per_cta;
+    float* orow = out + (int64_t)t * m;
+    const bool vec = BF16W ? (k & 7) == 0 : (k & 3) == 0;
+    const int pieces = BF16W ? k >> 3 : k >> 2;                  // 16-byte pieces of a row
+    const int per_warp = (pieces + split - 1) / split;
+    const int p_begin = min(pieces, sub * per_warp), p_end = min(pieces, p_begin + per_warp);
+    const int batches = (per_warp + 32 * PB_DEPTH - 1) / (32 * PB_DEPTH);
+    const int total = rows_it * batches;
+    int4 cur[PB_DEPTH], nxt[PB_DEPTH];
+    auto fetch = [&](int4* v, int i) {
+        const int it = i / batches, p0 = p_begin + (i - it * batches) * 32 * PB_DEPTH + lane;
+        const int row = row0 + it * row_step;
+#pragma unroll
+        for (int e = 0; e < PB_DEPTH; e++) {
+            const int p = p0 + e * 32;
+            v[e] = (row < m && p < p_end) ? ld_stream_16((const uint8_t*)W + ((int64_t)row * pieces + p) * 16) : make_int4(0, 0, 0, 0);
+        }
+    };
+    // this CTA's weight rows start for L2 while the kernel before is still at work (a prefetch has no value that could be stale): with the rows of 15 MB
+    // fetched only behind the norm, the product took 12.8 us for 2.3 us of memory time
+    {
+        const int64_t row_bytes = (int64_t)k * (BF16W ? 2 : 4);
+        for (int64_t i = threadIdx.x; i < (int64_t)rows_it * per_cta * ((row_bytes + 127) >> 7); i += 1024) {
+            const int64_t r = i / ((row_bytes + 127) >> 7), at = (i - r * ((row_bytes + 127) >> 7)) << 7, row = blockIdx.x * per_cta + (r / per_cta) * row_step + r % per_cta;
+            if (row < m && blockIdx.y == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"((const uint8_t*)W + row * row_bytes + at));
+        }
+    }
+    pdl_enter();
+    if (vec) fetch(cur, 0);
+    op.template stage<1024, 1>(pb_sm, t, k, red, BF16W);
+    __syncthreads();
+    for (int it = 0; it < rows_it; it++) {
+        const int row = row0 + it * row_step;
+        float acc = 0.0f;
+        if (vec) {
+            for (int b = 0; b < batches; b++) {
+                const int i = it * batches + b;
+                if (i + 1 < total) fetch(nxt, i + 1);
+                const int p0 = p_begin + b * 32 * PB_DEPTH + lane;
+#pragma unroll
+                for (int e = 0; e < PB_DEPTH; e++) {
+                    const int p = p0 + e * 32;
+                    if (p < p_end) {
+                        if (BF16W) acc = pb_dot8(cur[e], pb_sm + p * 8, acc);
+                        else {
+                            const float4 a = *(const float4*)(pb_sm + p * 4);
+                            acc = fmaf(__int_as_float(cur[e].x), a.x, acc); acc = fmaf(__int_as_float(cur[e].y), a.y, acc);
+                            acc = fmaf(__int_as_float(cur[e].z), a.z, acc); acc = fmaf(__int_as_float(cur[e].w), a.w, acc);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < PB_DEPTH; e++) cur[e] = nxt[e];
+            }
+        } else if (row < m) {
+            for (int c = sub * 32 + lane; c < k; c += split * 32)
+                acc = fmaf(BF16W ? __uint_as_float((unsigned)((const uint16_t*)W)[(int64_t)row * k + c] << 16) : ((const float*)W)[(int64_t)row * k + c], pb_sm[c], acc);
+        }
+        acc = warp_sum(acc);
+        if (split > 1) {
+            __syncthreads();                                     // red may still be read
+            if (lane == 0) red[warp] = acc;
+            __syncthreads();
+            if (sub == 0) {
+                acc = 0.0f;
+                for (int s = 0; s < split; s++) acc += red[warp + s];
+            }
+        }
+        if (lane == 0 && sub == 0 && row < m) orow[row] = accumulate ? orow[row] + acc : acc;
+    }
+}
 // the bfloat16 operand of the tensor-core product: a CTA per row
 __global__ void __launch_bounds__(PB_LN_THREADS) pb_norm_bf16_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, __nv_bfloat16* __restrict__ out,
                                                                      int k, float eps) {
@@ -234,28 +332,48 @@ __global__ void __launch_bounds__(256) pb_join_f32_kernel(PbJoin op, float* __re
 
 static const size_t PB_MAX_SMEM = 200 * 1024;
 static bool pb_few(int64_t T, int64_t k) { return T < 8 && (size_t)((k + 3) & ~3) * 4 <= PB_MAX_SMEM; }
-template <bool BF16W, class Op, int THREADS>
-static int pb_launch_matvec_by(cc_device* dev, const cc_buf* w, const Op& op, float* out, int64_t m, int64_t k, int64_t T, int accumulate, int split) {
+template <class Op>
+static int pb_launch_matvec_by(cc_device* dev, void (*kernel)(const void*, Op, float*, int, int, int, int), int threads, const cc_buf* w, const Op& op, float* out, int64_t m, int64_t k, int64_t T,
+                               int accumulate, int split) {
     const size_t smem = (size_t)((k + 3) & ~3) * 4;
-    auto kernel = pb_matvec_kernel<BF16W, Op, THREADS>;
     if (smem > 40 * 1024) CC_CUDA(dev, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int64_t per_cta = THREADS / 32 / split, ctas = (m + per_cta - 1) / per_cta;
-    cc_launch_pdl(dev, kernel, dim3((unsigned)(ctas < dev->sm_count ? ctas : dev->sm_count), (unsigned)T), THREADS, smem, w->plane[0], op, out, (int)m, (int)k, split, accumulate);
+    // one CTA fits an SM, and staging the operand is most of a short call: the T rows share the SMs, so that no SM stages twice.  us with all SMs for each row / here,
+    // 7424 x 1024 behind the norm: 2 rows 13.1 / 9.8, 7 rows 41 / 20 ; 1024 x 4096 behind the gated units: 10.8 / 7.1, 33 / 12
+    const int64_t per_cta = threads / 32 / split, need = (m + per_cta - 1) / per_cta, ctas = dev->sm_count / T < 1 ? 1 : dev->sm_count / T;
+    cc_launch_pdl(dev, kernel, dim3((unsigned)(need < ctas ? need : ctas), (unsigned)T), threads, smem, w->plane[0], op, out, (int)m, (int)k, split, accumulate);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;
 }
+// Which kernel follows from the sizes and the weights' type alone, so that a row has the same bits in every call.  us of one row, operand in shared memory with 32 warps /
+// in registers with 16 / in registers with 32:
+//   norm, bfloat16    2000 x 384 5.2 / 4.0 / 5.9 ; 7424 x 1024 9.5 / 7.6 / 8.6 ; 18432 x 1024 15.4 / 12.5 / 12.4 ; 32000 x 1024 23.3 / 18.1 / 16.7 ; 6000 x 2048 13.1 / 10.1 / 10.5 ;
+//                     12288 x 2048 18.2 / 15.1 / 14.8 ; 32000 x 1536 28.5 / 31.2 / 24.4 ; 18432 x 3072 30.1 / 35.6 / 27.1: 16 warps stage sooner, 32 ask for more at a time
+//   norm, 32 bits     4000 x 512 5.7 / 5.4 ; 12288 x 512 9.3 / 9.3 ; 32000 x 512 16.0 / 16.9 ; 7424 x 1024 10.3 / 9.3 ; 32000 x 1024 25.7 / 23.6 ; 32000 x 1536 35.8 / 36.9  (32 warps spill)
+//   units, bfloat16   512 x 2048 4.4 / 4.0 / 4.7 ; 768 x 3072 5.4 / 6.4 / 5.7 ; 1024 x 4096 6.6 / 6.6 / 6.2 ; 1280 x 7680 12.4 / 11.9 / 10.5 ; 1536 x 9216 14.4 / 18.0 / 15.1 ;
+//                     2048 x 6144 11.7 / 12.4 / 11.5 ; 3072 x 9216 21.5 / 27.2 / 21.3 ; 4096 x 16384 38.3 / 40.4 / 30.7
+//   units, 32 bits    1024 x 4096 7.3 / 7.5 ; 1536 x 6144 11.6 / 12.9 ; 2048 x 8192 18.0 / 17.0 ; 3072 x 9216 31.3 / 30.1 ; 4096 x 24576 83.9 / 87.8
 template <bool BF16W, class Op>
 static int pb_launch_matvec(cc_device* dev, const cc_buf* w, const Op& op, float* out, int64_t m, int64_t k, int64_t T, int accumulate) {
-    // as many warps per row as there are too few rows for the device's warps, and as the row's columns need for one block each.  32 warps a CTA where that makes one turn
-    // of the rows (1024 x 4096: 5.8 us; two turns of 16 warps 6.7), 16 with the next row's pieces in flight where there are more (7424 x 1024)
-    auto split_for = [&](int warps) {
+    const int64_t sms = dev->sm_count;
+    // as many warps per row as there are too few rows for the device's warps, and, for the operand in registers, as the row's columns need for one block each
+    auto split_for = [&](int warps, bool in_registers) {
         int split = 1;
-        while (split < warps && (m * split * 2 <= (int64_t)dev->sm_count * warps || k > (int64_t)split * PB_COLS)) split *= 2;
+        while (split < warps && (m * split * 2 <= sms * warps || (in_registers && k > (int64_t)split * PB_COLS))) split *= 2;
         return split;
     };
-    const int wide = split_for(32);
-    if (BF16W && m * wide <= (int64_t)dev->sm_count * 32) return pb_launch_matvec_by<BF16W, Op, 1024>(dev, w, op, out, m, k, T, accumulate, wide);
-    return pb_launch_matvec_by<BF16W, Op, 512>(dev, w, op, out, m, k, T, accumulate, split_for(16));
+    const int half = split_for(16, true), full = split_for(32, true);
+    bool registers;
+    if (Op::NORM) registers = BF16W || k > PB_COLS / 2 || m <= 64 * sms;
+    else registers = m >= 2048 || (BF16W && k > (int64_t)full * (PB_COLS * 3 / 4));
+    if (!registers) return pb_launch_matvec_by<Op>(dev, pb_matvec_shared_kernel<BF16W, Op>, 1024, w, op, out, m, k, T, accumulate, split_for(32, false));
+    auto by = [&](auto threads, int split) {
+        return pb_launch_matvec_by<Op>(dev, pb_matvec_kernel<BF16W, Op, decltype(threads)::value>, decltype(threads)::value, w, op, out, m, k, T, accumulate, split);
+    };
+    if constexpr (BF16W && !Op::NORM) return by(std::integral_constant<int, 1024>{}, full);
+    else {
+        if constexpr (BF16W) { if (m * half > 8 * 16 * sms) return by(std::integral_constant<int, 1024>{}, full); }      // more than 8 turns of 16 warps
+        return by(std::integral_constant<int, 512>{}, half);
+    }
 }
 static bool pb_tensor_cores(const cc_buf* w, int64_t m, int64_t k, int64_t T) {
     return w->dtype == CC_BF16 && cc_prefill_bf16_supported(m, k, T) && ((uintptr_t)w->plane[0] & 15) == 0;

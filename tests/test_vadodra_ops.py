@@ -115,6 +115,32 @@ def test_a_row_gives_the_same_bits_in_every_call_of_few_rows(dev):
             assert np.array_equal(out(seqops.layer_norm_product(T32(dev, x[t:t + 1]), T32(dev, g), None, 1e-5, wd), 1, 90)[0], whole[t])
 
 
+@pytest.mark.parametrize("dtype", [capi.F32, capi.BF16])
+@pytest.mark.parametrize("k,m", [(64, 9472), (64, 9473), (520, 9473), (64, 18944), (64, 18945), (1032, 9472), (1032, 9473), (2056, 300), (9000, 40)])
+def test_norm_and_product_at_the_limits_between_their_kernels(dev, dtype, k, m):
+    """Operand in registers or in shared memory, 16 warps or 32, one block of columns or several: right, and the same bits whatever shares the call"""
+    test_norm_and_product(dev, dtype, k, m)
+    rng = np.random.default_rng(k)
+    x, g, wd = f32(rng.standard_normal((7, k))), f32(rng.standard_normal(k)), W(dev, bf16(rng.standard_normal((m, k))), dtype)
+    whole = out(seqops.layer_norm_product(T32(dev, x), T32(dev, g), None, 1e-5, wd), 7, m)
+    for a, b in ((0, 1), (2, 4), (4, 7)):
+        assert np.array_equal(out(seqops.layer_norm_product(T32(dev, x[a:b]), T32(dev, g), None, 1e-5, wd), b - a, m), whole[a:b])
+
+
+@pytest.mark.parametrize("dtype", [capi.F32, capi.BF16])
+@pytest.mark.parametrize("ca,ff,m", [(512, 64, 2047), (512, 64, 2048), (1024, 2048, 640), (1024, 2056, 640), (3000, 3144, 130), (40, 24, 3), (1000, 16000, 2050)])
+def test_joined_product_at_the_limits_between_its_kernels(dev, dtype, ca, ff, m):
+    test_joined_product_with_gated_units(dev, dtype, ca, ff, m)
+    rng = np.random.default_rng(m)
+    a, src, wd = f32(rng.standard_normal((7, ca))), f32(rng.standard_normal((7, 2 * ff))), W(dev, bf16(rng.standard_normal((m, ca + ff))), dtype)
+
+    def call(lo, hi):
+        return out(seqops.joined_product_accumulate(zeros(dev, hi - lo, m), wd, T32(dev, a[lo:hi]), T32(dev, src[lo:hi]), 0, ff, ff), hi - lo, m)
+    whole = call(0, 7)
+    for lo, hi in ((0, 1), (2, 4), (4, 7)):
+        assert np.array_equal(call(lo, hi), whole[lo:hi])
+
+
 def test_products_refuse_what_does_not_fit(dev):
     x, g, w = zeros(dev, 3, 8), zeros(dev, 8), zeros(dev, 5, 8)
     for bad in ((zeros(dev, 3, 7), g, None, w), (x, zeros(dev, 7), None, w), (x, g, zeros(dev, 9), w)):

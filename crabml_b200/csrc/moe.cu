@@ -47,9 +47,10 @@ struct RouteArgs {
 };
 // one CTA per TOK tokens: its warps share the experts' logits (a warp per expert and all TOK tokens: lanes striding D in 16-byte pieces, or element
 // by element when D or the pointers do not allow them; then the butterfly), then warp tt does token tt's softmax and choice.  The order of a
-// logit's sum does not depend on TOK.
+// logit's sum does not depend on TOK.  (Four tokens have 64 registers where nothing is asked for, so that two CTAs of 512 threads fit an SM; with one CTA asked for they
+// took 128: 1500 tokens of 16 experts, 1024 columns 14.4 -> 16.4 us.)
 template <int TOK>
-__global__ void __launch_bounds__(TOK == 1 ? 1024 : 512, TOK == 2 ? 2 : 1) moe_route_kernel(RouteArgs a) {
+__global__ void __launch_bounds__(TOK == 1 ? 1024 : 512, TOK == 4 ? 0 : TOK) moe_route_kernel(RouteArgs a) {
     pdl_enter();
     extern __shared__ float rt_sm[];
     __shared__ float sg_sm[TOK];                           // the shared gate's logit: row E of the same products
@@ -205,7 +206,9 @@ extern "C" CC_API int cc_moe_route_shared(cc_device* dev, const cc_view* x, cons
     const int64_t rows = E + (shared_gate ? 1 : 0), most = tiled ? 16 : 32, rounds = (rows + most - 1) / most;
     const int64_t even = (rows + rounds - 1) / rounds;
     const unsigned threads = 32 * (unsigned)(even < 4 ? 4 : even);
-    if (tiled && T <= 4 * (int64_t)dev->sm_count) cc_launch_pdl(dev, moe_route_kernel<2>, (unsigned)((T + 1) / 2), threads, 2 * one, a);      // two CTAs fit an SM
+    // two tokens a CTA as long as all of them are on the device at once (64 registers a thread); us by two / by four: 900 tokens of 8 experts, 2048 columns 7.1 / 11.6, 600
+    // tokens of 16 experts, 1024 columns 10.0 / 8.5
+    if (tiled && T <= 2 * (int64_t)dev->sm_count * (1024 / threads)) cc_launch_pdl(dev, moe_route_kernel<2>, (unsigned)((T + 1) / 2), threads, 2 * one, a);
     else if (tiled) cc_launch_pdl(dev, moe_route_kernel<4>, (unsigned)((T + 3) / 4), threads, 4 * one, a);
     else cc_launch_pdl(dev, moe_route_kernel<1>, (unsigned)T, threads, one, a);
     CC_LAUNCH_CHECK(dev);

@@ -284,7 +284,7 @@ def test_grouped_experts_of_more_tokens_than_a_grid_has_rows(dev):
     test_grouped_gate_and_up_with_their_unit(dev, capi.ACT_SILU, 1.0, 0.0, 0.0, 65537, 2, 64, 1)
 
 
-@pytest.mark.parametrize("T", [127, 128, 591, 593])
+@pytest.mark.parametrize("T", [127, 128, 591, 592, 593, 1184, 1185])
 @pytest.mark.parametrize("top,renorm", [(1, 0), (4, 1), (40, 1)])
 def test_router_choices_and_their_weights(dev, T, top, renorm):
     """Calls around the limits of one, two and four tokens a CTA; more choices than a warp has lanes; weights that are renormalised"""

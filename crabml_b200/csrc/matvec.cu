@@ -33,8 +33,8 @@ __global__ void __launch_bounds__(MV_THREADS) matvec_kernel(WPlanes W, const voi
 
 // a few activation rows (2 .. 31: several sequences' next tokens): the grid above fetches and unpacks the weights once per row.  Here a warp takes two weight
 // rows and NB activations at a time (vecdot.cuh rows_dot); a CTA stages its NB activations once and walks over the weight rows.
-// Q5_K and Q6_K, and Q4_K up to 4 rows or of very long ones; with one row a time Q4_K, 11008 x 4096, 8 rows took 58 us, so 37; bound by the integer dot products and the
-// activation reads from shared memory (a 16-byte weight chunk meets 2 x NB 16-byte activation chunks)
+// It takes Q8_0, Q4_0, Q5_K and Q6_K, and of Q4_K up to 4 rows or rows so long that the kernel below has no room for them.  Q4_K, 11008 x 4096, 8 rows: one row at a time
+// 58 us, this way 31.  Bound by the integer dot products and the activation reads from shared memory (a 16-byte weight chunk meets 2 x NB 16-byte activation chunks)
 template <class T, int NB>
 __global__ void __launch_bounds__(MV_THREADS) matvec_few_kernel(WPlanes W, const void* act, int64_t n_total, float* __restrict__ out, int m, int k, int b) {
     pdl_enter();
@@ -185,11 +185,14 @@ static bool mm_fits(int64_t k) { return 8 * (int64_t)(TQ45_K<false>::smem_bytes(
 static int launch_mma(cc_device* dev, const cc_buf* w, const void* act, int64_t n_total, float* out, int64_t m, int64_t k, int64_t b) {
     WPlanes W;
     for (int i = 0; i < CC_MAX_PLANES; i++) W.p[i] = w->plane[i];
-    const int smem = 8 * mm_stride(TQ45_K<false>::smem_bytes((int)k)) + MM_GROUPS * 32 * MM_OUT * 4;
-    CC_CUDA(dev, cudaFuncSetAttribute(matvec_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    int smem = 8 * mm_stride(TQ45_K<false>::smem_bytes((int)k)) + MM_GROUPS * 32 * MM_OUT * 4;
     const int64_t groups = (b + 7) / 8, need = (m + 16 * MM_GROUPS - 1) / (16 * MM_GROUPS), fit = 224 * 1024 / (smem + 1024), most = dev->sm_count * (fit < 512 / MM_THREADS ? fit : 512 / MM_THREADS);
     int64_t ctas = most / groups > 0 ? most / groups : 1;
     if (ctas > need) ctas = need;
+    // no more CTAs than SMs: each gets an SM of its own by asking for more than half of its shared memory.  Started while the kernel before is still there, some SMs took two
+    // and others none: 4096 x 8192, 8 rows 31.8 us, now 23.8 (by dp4a 27.6) ; 4096 x 4096, 5 rows 18.1, now 14.3 (17.2)
+    if (ctas * groups <= dev->sm_count && smem < 116 * 1024) smem = 116 * 1024;
+    CC_CUDA(dev, cudaFuncSetAttribute(matvec_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cc_launch_pdl(dev, matvec_mma_kernel, dim3((unsigned)ctas, (unsigned)groups), MM_THREADS, smem, W, act, n_total, out, (int)m, (int)k, (int)b);
     CC_LAUNCH_CHECK(dev);
     return CC_OK;

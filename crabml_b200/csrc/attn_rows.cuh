@@ -27,14 +27,24 @@ struct ArArgs {
     float *out, *part;                   // part: [unit][most][HB][dvp] sums of a slice
     float2* ml;                          // [unit][most][HB]: a slice's largest score and its sum of weights
     float scale;
-    int most, cap, quantum;              // slices of a unit: at most `most` in this call; by ar_slices(n, quantum, cap)
+    int most, cap, quantum, fine, late;  // slices of a unit: at most `most` in this call; by ar_slices
     int hblocks, cblocks;
     int dkp, dvp, rs, tile, stages, chunk, keep, vec, qvec;      // padded row lengths, floats; rs: floats of a ring row; keep: the ring holds the slice and its rows are the values
 };
-__host__ __device__ __forceinline__ int ar_slices(int n, int quantum, int cap) {
-    int c = n / quantum + (n % quantum != 0);
-    if (c > 1 && c < 8) c = 2 * c < 8 ? 2 * c : 8;           // the device is far from full: shorter ones
-    return c < cap ? c : cap;
+// how many slices n visible keys are dealt out in: `quantum` keys each; fewer than 8 of them leave the device far from full: twice as many, or `fine` keys each, up to 8;
+// beyond 40 `late` keys each.  It never falls as n grows.
+__host__ __device__ __forceinline__ int ar_parts(int n, int each) { return (int)(((unsigned)n + (unsigned)each - 1u) / (unsigned)each); }
+__host__ __device__ __forceinline__ int ar_slices(int n, const ArArgs& A) {
+    int c = ar_parts(n, A.quantum);
+    if (c < 8) {
+        c = c > 1 ? 2 * c : 1;
+        if (A.fine != A.quantum) { const int f = ar_parts(n, A.fine); c = c > f ? c : f; }
+        if (c > 8) c = 8;
+    } else if (c > 40 && A.late != A.quantum) {
+        const int l = ar_parts(n, A.late);
+        c = l > 40 ? l : 40;
+    }
+    return c < A.cap ? c : A.cap;
 }
 __host__ __device__ constexpr int ar_stride(int HB) { return HB >= 8 ? HB + 4 : HB; }      // of a key's scores: whole float4, few bank conflicts down a head
 __device__ __forceinline__ void ar_wait(int pending) {       // all but the newest `pending` groups of this thread's copies have arrived
@@ -98,7 +108,7 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
     const int slice = blockIdx.x, t = blockIdx.y, cb = (int)(blockIdx.z - kcb * A.cblocks), hb = (int)(kcb - ukv * A.hblocks), kvh = (int)ukv;
     const int h0 = kvh * g.R + hb * HB, nh = min(HB, g.R - hb * HB), c_first = cb * AR_COLS, cols = ar_cols(g.dv, cb);
     const int64_t i = g.pos0 + t, lo = wa_lo(g, i);
-    const int n = (int)(i - lo) + 1, slices = ar_slices(n, A.quantum, A.cap);     // n: at most the ring's rows
+    const int n = (int)(i - lo) + 1, slices = ar_slices(n, A);     // n: at most the ring's rows
     if (slice >= slices) return;
     const int per = (int)((unsigned)(n + slices - 1) / (unsigned)slices), s0 = min(n, slice * per), m = min(n - s0, per);
     const float* kbase = A.k + (int64_t)kvh * g.dk;
@@ -310,14 +320,14 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
 #define AR_GROUPS (AR_THREADS / 8)
 #define AR_EACH 5
 __global__ void __launch_bounds__(AR_THREADS) attn_rows_sum_kernel(ArArgs A, WaGeom g, int HB) {
-    pdl_enter();
     __shared__ float4 sa[AR_WARPS][8];
     __shared__ float sm[AR_WARPS][8], st[AR_WARPS][8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, row4 = A.dvp / 4, items = HB * row4, x = lane & 7, z0 = threadIdx.x >> 3;
     const unsigned kcb = blockIdx.z / (unsigned)A.cblocks, ukv = kcb / (unsigned)A.hblocks;
     const int t = blockIdx.y, cb = (int)(blockIdx.z - kcb * A.cblocks), hb = (int)(kcb - ukv * A.hblocks), kvh = (int)ukv;
     const int64_t i = g.pos0 + t;
-    const int n = (int)(i - wa_lo(g, i)) + 1, slices = ar_slices(n, A.quantum, A.cap);
+    const int n = (int)(i - wa_lo(g, i)) + 1, slices = ar_slices(n, A);
+    pdl_enter();                                                   // up to here nothing but the arguments
     if (slices <= 1) return;
     const int e = min((int)blockIdx.x * 8 + x, items - 1), h = e / row4;
     const size_t unit = ((size_t)t * gridDim.z + blockIdx.z) * A.most;
@@ -405,9 +415,15 @@ static int attn_rows(cc_device* dev, const WaGeom& g, ArArgs A, int reach) {
         A.cap = (int)(cap < AR_LEAST ? AR_LEAST : cap < AR_GROUPS * AR_EACH ? cap : AR_GROUPS * AR_EACH);
         A.quantum = (int)(by_macs < by_bytes ? by_macs : by_bytes);
         A.quantum = A.quantum < 8 ? 8 : A.quantum;
-        A.most = ar_slices(reach, A.quantum, A.cap);
+        // through the ring of tiles a slice of many narrow rows takes longer than the kernel that adds up several.  us as one slice / in up to 8: 8 heads a key head (2 of 64) over 200
+        // keys 18.0 / 10.2, over 500 14.6 / 10.3 (2 / 8 slices) ; 16 heads a key head (2 of 64) over 100 16.1 / 9.5.  Up to 4 heads a second kernel costs more: 200 keys of 64 9.3 / 10.0
+        A.fine = HB > 4 && A.quantum > 512 / HB ? 512 / HB : A.quantum;
+        // few heads over wide rows: a CTA of 30 rows is short, and several queries are more of them than fit the device at once.  2300 latent rows, us by 30 / by 45 keys: 1 head, 1 query
+        // 12.4 / 12.7, 4 queries 19.2 / 13.6, 5 20.4 / 13.8, 12 34 / 30, 25 59 / 49 ; 4 heads, 2 queries 15.8 / 17.2, 5 26.4 / 19.7, 6 27.6 / 29.8
+        A.late = HB <= 4 && cols > 512 ? A.quantum * 3 / 2 : A.quantum;
+        A.most = ar_slices(reach, A);
         // the longest slice of a row that sees up to `reach` keys
-        const int last = (reach + A.most - 1) / A.most, slice = A.most > 1 && A.quantum > last ? A.quantum : last;      // (a row of one slice: up to the quantum)
+        const int last = (reach + A.most - 1) / A.most, slice = A.most > 1 && A.late > last ? A.late : last;      // (a row of fewer keys: no more than `late` a slice)
         const int chunk_most = HB == 16 ? 512 : HB == 8 ? 1024 : 2048 / HB;
         A.chunk = slice < chunk_most ? (slice + 3) & ~3 : chunk_most;
         const size_t fixed = ((size_t)HB * A.dkp + (size_t)A.chunk * ar_stride(HB)) * 4, sums = (size_t)AR_WARPS * (HB < 8 ? HB : 8) * 128 * 4;

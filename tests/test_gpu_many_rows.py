@@ -266,6 +266,7 @@ def test_attention_of_few_queries(dev, T, pos0, H, G, d, window, sink):
     (1, 127, 4, 1, 128, 128, False), (1, 128, 4, 1, 128, 128, False), (1, 129, 4, 1, 128, 128, False), (2, 129, 4, 1, 128, 128, False),      # one slice, or two
     (1, 700, 2, 1, 64, 64, False), (1, 9000, 2, 1, 16, 16, False),                             # weights in one piece, in several
     (2, 31, 8, 1, 576, 512, True), (1, 32, 5, 1, 576, 512, True), (1, 500, 16, 1, 576, 512, True), (1, 65, 17, 1, 132, 131, True), (1, 1200, 64, 1, 80, 80, False),
+    (1, 64, 8, 1, 64, 64, False), (2, 66, 8, 1, 64, 64, False), (1, 32, 16, 1, 64, 80, False), (2, 34, 16, 1, 64, 80, False), (1, 200, 2, 2, 64, 64, False), (1, 46, 1, 1, 576, 512, True),      # one slice, or several
     (1, 13000, 16, 1, 576, 512, True),                                                         # slices too long to stay in shared memory
     (1, 40, 1, 1, 64, 1025, False), (1, 40, 2, 1, 64, 1028, False), (2, 40, 4, 1, 64, 1025, False), (1, 300, 8, 2, 32, 1028, False), (1, 40, 8, 1, 64, 1028, False), (1, 5, 1, 1, 64, 2049, False),      # a last block of few columns
     (1, 300, 9, 1, 256, 256, False), (1, 40, 2, 1, 64, 1500, False), (1, 40, 2, 1, 5000, 64, False), (1, 40, 16, 1, 2000, 40, True)])

@@ -32,7 +32,7 @@ struct ArArgs {
     int dkp, dvp, rs, tile, stages, chunk, keep, vec, qvec;      // padded row lengths, floats; rs: floats of a ring row; keep: the ring holds the slice and its rows are the values
 };
 // how many slices n visible keys are dealt out in: `quantum` keys each; fewer than 8 of them leave the device far from full: twice as many, or `fine` keys each, up to 8;
-// beyond 40 `late` keys each.  It never falls as n grows.
+// beyond 56 (5 queries of which fit the device at once) `late` keys each.  It never falls as n grows.
 __host__ __device__ __forceinline__ int ar_parts(int n, int each) { return (int)(((unsigned)n + (unsigned)each - 1u) / (unsigned)each); }
 __host__ __device__ __forceinline__ int ar_slices(int n, const ArArgs& A) {
     int c = ar_parts(n, A.quantum);
@@ -40,9 +40,9 @@ __host__ __device__ __forceinline__ int ar_slices(int n, const ArArgs& A) {
         c = c > 1 ? 2 * c : 1;
         if (A.fine != A.quantum) { const int f = ar_parts(n, A.fine); c = c > f ? c : f; }
         if (c > 8) c = 8;
-    } else if (c > 40 && A.late != A.quantum) {
+    } else if (c > 56 && A.late != A.quantum) {
         const int l = ar_parts(n, A.late);
-        c = l > 40 ? l : 40;
+        c = l > 56 ? l : 56;
     }
     return c < A.cap ? c : A.cap;
 }
@@ -419,7 +419,7 @@ static int attn_rows(cc_device* dev, const WaGeom& g, ArArgs A, int reach) {
         // keys 18.0 / 10.2, over 500 14.6 / 10.3 (2 / 8 slices) ; 16 heads a key head (2 of 64) over 100 16.1 / 9.5.  Up to 4 heads a second kernel costs more: 200 keys of 64 9.3 / 10.0
         A.fine = HB > 4 && A.quantum > 512 / HB ? 512 / HB : A.quantum;
         // few heads over wide rows: a CTA of 30 rows is short, and several queries are more of them than fit the device at once.  2300 latent rows, us by 30 / by 45 keys: 1 head, 1 query
-        // 12.4 / 12.7, 4 queries 19.2 / 13.6, 5 20.4 / 13.8, 12 34 / 30, 25 59 / 49 ; 4 heads, 2 queries 15.8 / 17.2, 5 26.4 / 19.7, 6 27.6 / 29.8
+        // 12.6 / 12.7, 4 queries 19.2 / 13.6, 5 20.4 / 13.6, 6 21.3 / 20.8, 12 34 / 29.5, 25 59 / 51 ; 4 heads, 2 queries 15.8 / 16.8, 5 26.5 / 19.2, 6 27.4 / 28.8, 12 47 / 42
         A.late = HB <= 4 && cols > 512 ? A.quantum * 3 / 2 : A.quantum;
         A.most = ar_slices(reach, A);
         // the longest slice of a row that sees up to `reach` keys

@@ -20,6 +20,7 @@
 
 #define AR_MACS (1 << 18)                // a slice has this many multiply-adds or AR_BYTES bytes, whichever are fewer keys, as long as there are SMs without one
 #define AR_BYTES (1 << 17)
+#define AR_WORKSPACE ((size_t)64 << 20)  // bytes of the slices' sums that a call has at a time
 #define AR_LEAST 4                       // long caches: 4 slices at least, so that 64 sums or more of few terms are added up whatever the number of heads
 
 struct ArArgs {
@@ -28,7 +29,7 @@ struct ArArgs {
     float2* ml;                          // [unit][most][HB]: a slice's largest score and its sum of weights
     float scale;
     int most, cap, quantum, fine, late;  // slices of a unit: at most `most` in this call; by ar_slices
-    int hblocks, cblocks;
+    int hblocks, cblocks, kv0;           // kv0: key/value head of the launch's first unit
     int dkp, dvp, rs, tile, stages, chunk, keep, vec, qvec;      // padded row lengths, floats; rs: floats of a ring row; keep: the ring holds the slice and its rows are the values
 };
 // how many slices n visible keys are dealt out in: `quantum` keys each; fewer than 8 of them leave the device far from full: twice as many, or `fine` keys each, up to 8;
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
     float* ring = sc + (size_t)A.chunk * PS;                       // [stages][tile][rs]; behind the last tile the warps' sums [key group][HB][dvp]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned kcb = blockIdx.z / (unsigned)A.cblocks, ukv = kcb / (unsigned)A.hblocks;
-    const int slice = blockIdx.x, t = blockIdx.y, cb = (int)(blockIdx.z - kcb * A.cblocks), hb = (int)(kcb - ukv * A.hblocks), kvh = (int)ukv;
+    const int slice = blockIdx.x, t = blockIdx.y, cb = (int)(blockIdx.z - kcb * A.cblocks), hb = (int)(kcb - ukv * A.hblocks), kvh = A.kv0 + (int)ukv;
     const int h0 = kvh * g.R + hb * HB, nh = min(HB, g.R - hb * HB), c_first = cb * AR_COLS, cols = ar_cols(g.dv, cb);
     const int64_t i = g.pos0 + t, lo = wa_lo(g, i);
     const int n = (int)(i - lo) + 1, slices = ar_slices(n, A);     // n: at most the ring's rows
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(AR_THREADS) attn_rows_sum_kernel(ArArgs A, WaG
     __shared__ float sm[AR_WARPS][8], st[AR_WARPS][8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, row4 = A.dvp / 4, items = HB * row4, x = lane & 7, z0 = threadIdx.x >> 3;
     const unsigned kcb = blockIdx.z / (unsigned)A.cblocks, ukv = kcb / (unsigned)A.hblocks;
-    const int t = blockIdx.y, cb = (int)(blockIdx.z - kcb * A.cblocks), hb = (int)(kcb - ukv * A.hblocks), kvh = (int)ukv;
+    const int t = blockIdx.y, cb = (int)(blockIdx.z - kcb * A.cblocks), hb = (int)(kcb - ukv * A.hblocks), kvh = A.kv0 + (int)ukv;
     const int64_t i = g.pos0 + t;
     const int n = (int)(i - wa_lo(g, i)) + 1, slices = ar_slices(n, A);
     pdl_enter();                                                   // up to here nothing but the arguments
@@ -444,20 +445,31 @@ static int attn_rows(cc_device* dev, const WaGeom& g, ArArgs A, int reach) {
         if (HB <= 4 || smem <= most) break;
     }
     // short caches: a CTA a head.  The slices, and with them the order of every sum, stay those of the larger block
-    if (HB <= 4 && A.chunk < 512 && g.T * g.G * A.hblocks * HB * A.most <= 2 * dev->sm_count) {
+    if (HB <= 4 && A.chunk < 512 && (int64_t)g.T * g.G * A.hblocks * HB * A.most <= 2 * dev->sm_count) {
         HB = 1; A.hblocks = g.R;
         smem = (size_t)(A.dkp + A.chunk + AR_WARPS * 128) * 4;
     }
-    const int64_t units = (int64_t)g.T * g.G * A.hblocks * A.cblocks;
+    // queries in portions whose partial sums take AR_WORKSPACE at most (many of them come here where tiles have no room), key heads in as many as a grid has units.  A query's
+    // slices, and its bits, are the same in any portion
+    const int64_t blocks = (int64_t)A.hblocks * A.cblocks, fit = 65535 / blocks > 0 ? 65535 / blocks : 1, heads = g.G < fit ? g.G : fit;
+    const size_t part = (size_t)(heads * blocks) * A.most * HB * A.dvp * 4, ml = (size_t)(heads * blocks) * A.most * HB * 8;      // of one query
+    const int64_t room = A.most > 1 && AR_WORKSPACE / (part + ml) < (size_t)g.T ? (int64_t)(AR_WORKSPACE / (part + ml)) : g.T, portion = room > 0 ? room : 1;
     void* ws = nullptr; size_t cls = 0;
     if (A.most > 1) {
-        const size_t part = (size_t)units * A.most * HB * A.dvp * 4, ml = (size_t)units * A.most * HB * 8;
-        int rc = cc_pool_alloc(dev, part + ml, &ws, &cls);
+        int rc = cc_pool_alloc(dev, (size_t)portion * (part + ml), &ws, &cls);
         if (rc) return rc;
-        A.part = (float*)ws; A.ml = (float2*)((uint8_t*)ws + part);
+        A.part = (float*)ws; A.ml = (float2*)((uint8_t*)ws + portion * part);
     }
-    const int rc = HB == 16 ? ar_launch<16>(dev, A, g, smem) : HB == 8 ? ar_launch<8>(dev, A, g, smem) : HB == 4 ? ar_launch<4>(dev, A, g, smem)
-                   : HB == 2 ? ar_launch<2>(dev, A, g, smem) : ar_launch<1>(dev, A, g, smem);
+    int rc = CC_OK;
+    for (int64_t t0 = 0; t0 < g.T && rc == CC_OK; t0 += portion)
+        for (int64_t kv0 = 0; kv0 < g.G && rc == CC_OK; kv0 += heads) {
+            ArArgs B = A;
+            WaGeom p = g;
+            B.q += t0 * g.H * g.dk; B.out += t0 * g.H * g.dv; B.kv0 = (int)kv0;
+            p.pos0 += t0; p.T = (int)(g.T - t0 < portion ? g.T - t0 : portion); p.G = (int)(g.G - kv0 < heads ? g.G - kv0 : heads);
+            rc = HB == 16 ? ar_launch<16>(dev, B, p, smem) : HB == 8 ? ar_launch<8>(dev, B, p, smem) : HB == 4 ? ar_launch<4>(dev, B, p, smem)
+                 : HB == 2 ? ar_launch<2>(dev, B, p, smem) : ar_launch<1>(dev, B, p, smem);
+        }
     if (ws) cc_pool_free(dev, ws, cls);
     return rc;
 }

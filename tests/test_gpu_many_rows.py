@@ -294,6 +294,29 @@ def test_attention_of_few_queries_at_the_edges_of_its_slices(dev, T, n, H, G, dk
         np.testing.assert_array_equal(call(t, t + 1)[0].view(np.uint32), got[t].view(np.uint32))
 
 
+@pytest.mark.parametrize("T,n,G,dk,dv", [(2, 18, 1050, 1024, 4096), (1, 2, 33000, 1, 1025)])
+def test_attention_of_few_queries_in_portions(dev, T, n, G, dk, dv):
+    """Slices of two queries whose sums take 69 MB each, and more blocks of value columns than a grid has units: portions of queries and of heads"""
+    from crabml_b200 import seqops
+    rng = np.random.default_rng(G)
+    q, k, v = (rng.standard_normal(s, np.float32) for s in ((T, G, dk), (n, G, dk), (n, G, dv)))
+    kt, vt = tensor(dev, k.reshape(n, -1)), tensor(dev, v.reshape(n, -1))
+    qt, launches = tensor(dev, q.reshape(T, -1)), dev.launch_count()
+    got = seqops.masked_attention(qt, kt, vt, n - T, G, G, dk, dv, dk ** -0.5)
+    assert dev.launch_count() - launches == (4 if T == 2 else 2)
+    got = got.export().reshape(T, G, dv)
+    for t in range(T):
+        seen = n - T + 1 + t
+        s = np.einsum("gd,ngd->gn", q[t].astype(np.float64), k[:seen].astype(np.float64)) * dk ** -0.5
+        w = np.exp(s - s.max(1, keepdims=True))
+        want = np.einsum("gn,ngd->gd", (w / w.sum(1, keepdims=True)).astype(np.float32), v[:seen], optimize=True)
+        # scores stay below 7 (one product: below 20, two keys), whose up to 1024 products and sums are off by 2^-24 of 7 a few times over; a weight moves by that share, a result by that share of values below 7.  (Scores
+        # of 70, by a scale of 1/2, are off by 1e-5 and with them the results.)
+        assert np.abs(got[t] - want).max() <= 1e-5
+    one = seqops.masked_attention(tensor(dev, q[T - 1:].reshape(1, -1)), kt, vt, n - 1, G, G, dk, dv, dk ** -0.5).export().reshape(G, dv)
+    np.testing.assert_array_equal(one.view(np.uint32), got[T - 1].view(np.uint32))
+
+
 def test_attention_of_many_rows_over_a_long_cache_takes_its_heads_in_groups(dev):
     """16 heads over 40,000 keys: 820 MB of scores and cut planes where the scores of 33 queries take 84"""
     from crabml_b200 import seqops

@@ -110,7 +110,6 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
     const int h0 = kvh * g.R + hb * HB, nh = min(HB, g.R - hb * HB), c_first = cb * AR_COLS, cols = ar_cols(g.dv, cb);
     const int64_t i = g.pos0 + t, lo = wa_lo(g, i);
     const int n = (int)(i - lo) + 1, slices = ar_slices(n, A);     // n: at most the ring's rows
-    if (slice >= slices) return;
     const int per = (int)((unsigned)(n + slices - 1) / (unsigned)slices), s0 = min(n, slice * per), m = min(n - s0, per);
     const float* kbase = A.k + (int64_t)kvh * g.dk;
     const float* vbase = A.v + (int64_t)kvh * g.vhs + c_first;
@@ -119,6 +118,7 @@ __global__ void __launch_bounds__(AR_THREADS, HB <= 4 ? 2 : 1) attn_rows_kernel(
     const int kgs = at_v.kgs, hg = at_v.hg, kg = at_v.kg, col = at_v.col;
     const bool loads = at_v.loads;
     pdl_enter();                                                   // up to here nothing but the arguments
+    if (slice >= slices) return;
     float4 acc[HS];
 #pragma unroll
     for (int h = 0; h < HS; h++) acc[h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);

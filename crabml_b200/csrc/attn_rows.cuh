@@ -9,7 +9,7 @@
 // rows straight into registers (through the ring 16 heads of 128 over 4000 keys took 48 us, 2 barriers and 32 wavefronts of shared memory for 4 keys).
 //
 // A token, us, as a kernel of scores and one of values (the cache read once per 32 value columns) / here: 16 heads over 4000 latent rows (576, 512; 9.2 MB) 29 / 14.5, over
-// 16000 72 / 38 ; 16 heads of their own (128) over 4000 keys (65 MB) 34 / 16, over 16000 113 / 51 ; 32 heads on 8 over 16000 (131 MB) 106 / 41 ; 128 heads (192, 128)
+// 16000 72 / 38 ; 16 heads of their own (128) over 4000 keys (65 MB) 34 / 16, over 16000 113 / 51 ; 32 heads on 8 over 16000 (131 MB) 106 / 37 ; 128 heads (192, 128)
 // over 4000 (655 MB) 240 / 130.  As a cluster of 8 CTAs a unit, the slices meeting in its shared memory and clusters through counters, the first took 21.5: 15 clusters are
 // resident at a time (120 of 148 SMs), and the last cluster adds up what the others left.
 //

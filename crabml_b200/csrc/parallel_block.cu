@@ -77,12 +77,11 @@ struct PbJoin {
 };
 
 // grid (about one CTA per SM, T).  `split` warps (a power of two) share one weight row, each a contiguous stretch of its 16-byte pieces, PB_COLS columns or less at a time;
-// a CTA owns PB_WARPS / split rows at a time.  A lane holds its 32 columns of the operand in registers for all of the warp's rows and has the pieces of the
+// a CTA owns WARPS / split rows at a time.  A lane holds its 32 columns of the operand in registers for all of the warp's rows and has the pieces of the
 // next row in flight while it multiplies those of this one; the first are fetched before the operand row is staged.  Sums of a row: each piece by itself, the pieces, the
 // butterfly, then the row's warps in ascending order, once for up to PB_TURNS rows.  The order depends on the sizes alone, not on T.
 // Bound by latency (norm, first pieces) and, in a model's head, by memory.  With the operand read from shared memory for every row, 32 warps took 4096 cycles of its ports for
-// 64 rows of 1024 columns (lanes 32 bytes apart: two turns each).  A decoded token's products, us: 7424 x 1024 behind the norm 8.5 -> 6.7, 1024 x 4096 behind the
-// gated units 5.9 -> 5.8, the head's 32000 x 1024 (cold) 26.7 -> 22.3.
+// 64 rows of 1024 columns (lanes 32 bytes apart: two turns each).  What both kernels measured, and where the line between them lies: pb_launch_matvec.
 template <bool BF16W, class Op, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) pb_matvec_kernel(const void* __restrict__ W, Op op, float* __restrict__ out, int m, int k, int split, int accumulate) {
     extern __shared__ __align__(16) float pb_sm[];              // the operand row, k floats (rounded up to 4)

@@ -1184,10 +1184,11 @@ static int masked_attention_impl(cc_device* dev, const cc_view* q, const cc_view
     g.T = (int)T; g.H = H; g.G = G; g.R = R; g.dk = dk; g.dv = dv; g.ring = (int)ring; g.QT = WA_ROWS / R; g.pos0 = pos0; g.pos0_row = (int)(pos0 % ring);
     g.krs = G * dk; g.vrs = vring ? G * dv : G * dk; g.vhs = vring ? dv : dk;
     const WaCall c = {fptr(q), fptr(kring), vptr, r1 ? fptr(r1) : nullptr, r2 ? fptr(r2) : nullptr, sink ? fptr(sink) : nullptr, (float*)o->base, scale, last, oldest, reach};
-    // Row by row the cache is read once per query and 16 heads of a key head, and a key takes about 3e-9 us for each of
+    // Row by row the cache is read once per query and 16 heads of a key head, and a key takes about 2e-7 us for each of
     //     cost = T * (key heads x blocks of heads) * (dk + dv in whole 128s + 128 for the sums across lanes) * (2, 3, 4, 7 or 12 for up to 1, 2, 4, 8 or 16 heads);
     // a tile's work is the same up to 128 rows, 20 to 30 us and 0.012 us a key.  More than 64 rows are tiles whatever they cost (one or two queries of few blocks of heads
-    // aside), so that a query of a prompt keeps its bits however the prompt is cut.  us by rows / by tiles over 300, 2000, 4000, 16000 keys, heads on key heads x queries:
+    // aside): the portions of a prompt that have more take the same way and a query its bits with them, however the prompt is cut.  Portions of 64 rows or fewer may take the other one,
+    // by how many queries they have and how long the cache is, and the two ways' bits differ.  us by rows / by tiles over 300, 2000, 4000, 16000 keys, heads on key heads x queries:
     // 16 on 16 x 4 13 / 27, 30 / 57, 50 / 103, 138 / 352 ; 8 on 1 (latent, 576) x 8 18 / 31, 41 / 51, 70 / 73, 222 / 223 ; 4 on 1 (latent) x 16 22 / 31, 52 / 52, 87 / 73, 229 / 223 ;
     // 1 on 1 (latent) x 32 19 / 31, 57 / 51, 104 / 73, 275 / 222 ; 128 on 128 (192, 128) x 2 34 / 79, 120 / 319, 209 / 632
     const bool can_rows = T <= 65535 && (int64_t)(R < 8 ? R : 8) * dk * 4 <= 160 * 1024;

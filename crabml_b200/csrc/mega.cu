@@ -434,7 +434,7 @@ bool cc_mega_generic_supported(int type, int64_t k) {
 }
 
 // developer A/B switches: CRABML_MEGA_FLAGS replaces the default flag word (see MK_F_* and the L2 budget byte)
-#define MK_DEFAULT_FLAGS (MK_F_LOOK | MK_F_WSTAGE | MK_F_POLLCNT | MK_F_XEARLY | MK_F_RING | MK_F_RPAIR)      // ring + pairs: profiles/r02n (2227 us vs 2386 us per 7B Q8_0 token, same box)      // profiles/r02c: 2407 us vs 2586 us (0x5) on the same box
+#define MK_DEFAULT_FLAGS (MK_F_LOOK | MK_F_WSTAGE | MK_F_POLLCNT | MK_F_XEARLY | MK_F_RING | MK_F_RPAIR)      // ring + pairs: 2227 us vs 2386 us per 7B Q8_0 token ; without them 2407 us vs 2586 us (0x5), each on one box
 int cc_mega_flags() {
     static const int f = getenv("CRABML_MEGA_FLAGS") ? (int)strtol(getenv("CRABML_MEGA_FLAGS"), nullptr, 0) : MK_DEFAULT_FLAGS;
     return f;

@@ -29,7 +29,7 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
 }
 __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) { asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
 
-// Split grid barrier (measured with tools/barrier_floor.py on B200, 148 CTAs: 2.1 us per phase; the two-level
+// Split grid barrier (measured with cc_test_mega_barrier_floor on B200, 148 CTAs: 2.1 us per phase; the two-level
 // acq_rel-atomic version cost 3.1 us, relaxed polling + fence 2.6 us):
 //   arrive : bar.sync, then ONE thread does a fire-and-forget red.release.gpu.add on a flat monotonic counter
 //            (the release publishes the CTA's phase output; that thread never issues prefetch loads);

@@ -98,7 +98,7 @@ __device__ __forceinline__ int mr_locate(const StreamMats& M, const MrGeo& g, in
 // slot's "full" barrier with the byte count, issues the two bulk copies (quants, scales) and publishes the entry number in the slot's
 // sequence word.  Consumers check that word before they look at the barrier: an mbarrier parity alone cannot tell "this use has not
 // landed" from "the previous use has not landed" when a warp gets more than one lap ahead (16 warps x 3 segments > 40 slots).
-// (Measured, profiles/r02q: 1 / 2 / 4 / 8 producer warps = 2859 / 2782 / 2262 / 2435 us per token -- a warp's probe-and-issue trip takes ~400
+// (Measured: 1 / 2 / 4 / 8 producer warps = 2859 / 2782 / 2262 / 2435 us per token -- a warp's probe-and-issue trip takes ~400
 // cycles, so the number of polling warps bounds the refill rate, and at 8 the 80-register cap starts to cost.  Sleeping after a failed probe,
 // SIMT-wide parameter computation, in-order probe loops and fence-free hand-back words changed nothing.)
 __device__ void mr_producer(const MkPhase* __restrict__ phases, int n_phases, const MrRing R, unsigned full0, unsigned done0, unsigned ring0,
@@ -238,7 +238,7 @@ __device__ __forceinline__ void mr_seg_lds(MkSeg& S, const uint8_t* sp, int seg,
 
 // Activation quants in shared memory, per group of 32 blocks: the 16-byte first halves of all 32 blocks, then the second halves (the layout of
 // the Q8_0 weight plane) -- lane l reads block 32 g + l with two conflict-free LDS.128 (block-major, 32 bytes apart, is a 2-way bank conflict:
-// 64 instead of 32 shared-memory wavefronts per segment, and the ring's throughput is bounded by shared-memory bandwidth, profiles/r02n)
+// 64 instead of 32 shared-memory wavefronts per segment, and the ring's throughput is bounded by shared-memory bandwidth)
 __device__ __forceinline__ int mr_act_word(int i) {           // i = 4-byte word index in block-major order (block i >> 3, word i & 7)
     const int b = i >> 3, w = i & 7;
     return (b >> 5) * 256 + (w >> 2) * 128 + (b & 31) * 4 + (w & 3);

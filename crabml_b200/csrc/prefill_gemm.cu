@@ -63,7 +63,7 @@ __device__ __forceinline__ void pg_tmem_load8(unsigned taddr, unsigned (&v)[8]) 
 // grid: (ceil(m / (128 * MT)), ceil(b / BLOCK_N), parts of the depth); dynamic smem: 1024-aligned ring of STAGES x (A tile MT x 16 KB + B tile BLOCK_N*128 B)
 // MT = 2: the CTA owns a 256-row weight tile as TWO M = 128 accumulators (2 x BLOCK_N TMEM columns) that share every B tile -- 1.5x
 // fewer operand bytes per FLOP than 128 x 256 tiles, which matters because 148 CTAs pulling 48 KB per 128x256x64 step ask more of L2
-// than it delivers (profiles/r02e: 47 % tensor pipe with MT = 1).
+// than it delivers (47 % tensor pipe with MT = 1).
 template <int BLOCK_N, int MT, int FMT = 0>
 __global__ void __launch_bounds__(PG_THREADS, 1) umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                                                                   float* C, int m, int b, int k, const int* __restrict__ groups = nullptr,
@@ -446,7 +446,7 @@ static int pg_launch(cc_device* dev, const CUtensorMap& tw, const CUtensorMap& t
 }
 
 // Dequantised weights are kept: with 180 GB of HBM a 7B model's f16 tile source (2 bytes per weight, 13-14 GB) fits many times over,
-// and dequantising 58 MB per matrix on every call costs as much as the GEMM itself (profiles/r02e).  CRABML_PREFILL_NOCACHE=1 keeps
+// and dequantising 58 MB per matrix on every call costs as much as the GEMM itself.  CRABML_PREFILL_NOCACHE=1 keeps
 // the round-trip through one reusable scratch buffer instead (memory-constrained deployments).
 static int pg_weight_f16(cc_device* dev, const cc_buf* w, int64_t m, int64_t k, PgScratch* s, const void** out) {
     static const bool nocache = getenv("CRABML_PREFILL_NOCACHE") != nullptr;

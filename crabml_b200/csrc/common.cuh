@@ -20,7 +20,7 @@
 #define QK_K 256
 
 // ------------------------------------------------------------------------------------------
-// Device-side storage layouts (DESIGN.md "Data layout in HBM").  GGUF stores a weight matrix
+// Device-side storage layouts.  GGUF stores a weight matrix
 // as rows of AoS blocks whose size is only 2-byte aligned (34 / 18 / 22 / 210 ... bytes).
 // from_cpu repacks each matrix ONCE into planes so that every hot-loop load is a 16-byte,
 // fully coalesced LDG.128; total bytes are unchanged (the f16 scales move to their own plane).

@@ -107,7 +107,7 @@ CC_API void* cc_device_stream(cc_device* dev);
 /* ---- storage: Tensor::from_cpu / alloc / Clone / Drop (api.rs:14-23) -------------------- */
 /* from_cpu: copies `nbytes` host bytes of GGUF-layout data (row-major rows of quant blocks,
  * model.rs:462-477).  `shape` is [rows, cols] (or 1-D).  Quantized types are repacked once
- * into the device layout documented in DESIGN.md (same algorithmic bytes). */
+ * into the device layout of the kernels (same algorithmic bytes). */
 CC_API int cc_tensor_from_cpu(cc_device* dev, const void* bytes, size_t nbytes, const int64_t* shape,
                        int32_t ndim, int32_t ggml_type, cc_buf** out);
 /* alloc: F32 zero-filled, or F16 (cpu_tensor.rs:138-165); other dtypes -> CC_ERR_TENSOR */

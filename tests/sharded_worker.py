@@ -1,4 +1,4 @@
-"""Worker of the multi-process tests of the sharded decode path (SURVEY §8e).  Launched by tests/test_sharded_gloo.py
+"""Worker of the multi-process tests of the sharded decode path.  Launched by tests/test_sharded_gloo.py
 (CPU, gloo, oracle tensors: validates the shard plan + replay) and tests/test_gpu_sharded.py (one process per GPU: the
 product path -- p2p one-shot exchange in eager mode, in the CUDA-graph mode and inside the megakernel, and the NCCL
 baseline) under `python -m torch.distributed.run --nproc-per-node N tests/sharded_worker.py --mode cpu|gpu`.

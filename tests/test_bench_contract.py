@@ -1,4 +1,4 @@
-"""The bench.py contract (SURVEY §8d): the reference arm runs here on CPU (small workload) and must print ONE JSON line
+"""The bench.py contract: the reference arm runs here on CPU (small workload) and must print ONE JSON line
 with the agreed keys; the committed B200 line of the round (profiles/) must carry the same keys plus the GPU-only ones."""
 import json
 import os

@@ -1,4 +1,4 @@
-"""The other architectures' forwards (SURVEY 8f-4; llama2.rs:283-352 qwen2, :455-524 gemma) through the C++ runner on the GPU:
+"""The other architectures' forwards (llama2.rs:283-352 qwen2, :455-524 gemma) through the C++ runner on the GPU:
 q/k/v bias adds, Neox RoPE, GeLU ffn through the f16 LUT, the sqrt(dim) embedding scale and the tied classifier, with grouped-query
 attention.  exact_order mode must reproduce the oracle replay of the same forward bit for bit; the fast modes must agree with each
 other bit for bit and stay close to the oracle."""

@@ -1,6 +1,6 @@
 """End-to-end parity on the reference's own GGUF fixtures: the Llama2Runner replay
-(llama2.rs:184-281,527-638) over CudaTensor vs the same replay over the CPU oracle.
-north_star: logits within 1e-3 relative; golden generations of llama2.rs:673-703 reproduced."""
+(llama2.rs:184-281,527-638) over CudaTensor vs the same replay over the CPU oracle:
+logits within 1e-3 relative; golden generations of llama2.rs:673-703 reproduced."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,7 @@ from tests.test_oracle_golden_text import CASES, PROMPT, PROMPT_IDS
 
 pytestmark = pytest.mark.gpu
 
-REL_TOL = 1e-3      # north_star bar (relative to max |logit|); met -- with equality -- in exact_order mode
+REL_TOL = 1e-3      # relative to max |logit|; met -- with equality -- in exact_order mode
 
 
 def _band():
@@ -91,7 +91,7 @@ def test_fast_mode_generation_and_band(fixture_path, fname, text, ids):
 
 
 def test_long_decode_positions(fixture_path):
-    """100 decode steps (BASELINE config 1/2): positions up to ~110 exercise the RoPE recurrence and
+    """100 decode steps: positions up to ~110 exercise the RoPE recurrence and
     a growing KV cache; logits must stay within the bar at every step."""
     from crabml_b200 import CudaTensor
     gm = GGUFModel(fixture_path("tinyllamas-stories-15m-q8_0.gguf"))

@@ -1,4 +1,4 @@
-"""THE hot path: matmul_vec for every GGUF quant type vs the oracle's gemv (SURVEY §8a a1-a11)."""
+"""THE hot path: matmul_vec for every GGUF quant type vs the oracle's gemv."""
 import numpy as np
 import pytest
 

@@ -1,4 +1,4 @@
-"""Parity of the small ops (SURVEY §8a a12-a19) through the C ABI vs the CPU oracle.
+"""Parity of the small ops through the C ABI vs the CPU oracle.
 Structure follows the reference's per-backend op tests (crabml-wgpu/src/wgpu_tensor.rs:749-1099)."""
 import numpy as np
 import pytest
@@ -208,7 +208,7 @@ def test_batch_matmul_attention_shapes(gdev, odev, kv_dtype, heads, kv_heads, hd
 
 @pytest.mark.parametrize("t", oc.QUANT_TYPES)
 def test_block_unpack_bit_exact(gdev, odev, t):
-    """north_star: 'block unpack bit-exact'.  copy_rows_from dequantises rows of the repacked device
+    """Block unpack is bit-exact.  copy_rows_from dequantises rows of the repacked device
     layout; must equal BlockQ*::dequantize bit for bit, and the repack must round-trip the GGUF bytes."""
     from crabml_b200 import CudaTensor
     rng = np.random.default_rng(100 + t)

@@ -1,6 +1,6 @@
 """The C++ Llama2Runner replay (crabml_b200/csrc/host/llama2_runner.cpp, the product's host side) end to end:
 golden generations of the reference (llama2.rs:673-703), bit-identical logits in exact_order mode, and a
-Llama-2-7B-SHAPED layer on the synthetic weights bench.py uses (BASELINE.json configs 2-4 at full size)."""
+Llama-2-7B-SHAPED layer on the synthetic weights bench.py uses."""
 import os
 import subprocess
 import sys
@@ -343,7 +343,7 @@ def test_fast_mode_logits_inside_the_reference_order_band_on_7b_shapes():
     """The benchmarked configuration (megakernel, warp-parallel reductions) on Llama-2-7B SHAPES, 8 layers, 32 decode positions:
     per position, the distance of the GPU logits from the reference's AVX2-order logits is compared with the distance between the
     reference's OWN two code paths (scalar vs AVX2 order, both restated in the oracle, both passing every KAT) on the same weights.
-    The truncating activation quantiser (buf_q8_0.rs:117-126) makes logits chaotic in the summation order (DESIGN.md section 2), so the
+    The truncating activation quantiser (buf_q8_0.rs:117-126) makes logits chaotic in the summation order, so the
     band of the reference itself is the meaningful yardstick; the distribution over the 32 positions is printed."""
     import os
     from crabml_b200 import runner as R

@@ -16,7 +16,7 @@ def f16b(x):
 
 def test_block_sizes():
     # size_of assertions: buf_q4_0.rs:263, buf_q4_1.rs:289, buf_q5_0.rs:188, buf_q5_1.rs:186,
-    # buf_q8_1.rs:139, buf_q8_k.rs:236, buf_q6_k.rs:250; Appendix A of SURVEY.md
+    # buf_q8_1.rs:139, buf_q8_k.rs:236, buf_q6_k.rs:250
     want = {oc.Q8_0: 34, oc.Q4_0: 18, oc.Q4_1: 20, oc.Q5_0: 22, oc.Q5_1: 24, oc.Q8_1: 36,
             oc.Q2_K: 84, oc.Q3_K: 110, oc.Q4_K: 144, oc.Q5_K: 176, oc.Q6_K: 210, oc.Q8_K: 292}
     for t, n in want.items():

@@ -1,6 +1,6 @@
 """Second, independent pin for block unpack: python `gguf.quants.dequantize` (ggml layouts)
-must agree BIT-EXACTLY with the oracle's dequantize on random valid blocks (SURVEY §8c,
-Appendix D-5), and vec_dot must agree with the dot of the dequantized operands."""
+must agree BIT-EXACTLY with the oracle's dequantize on random valid blocks,
+and vec_dot must agree with the dot of the dequantized operands."""
 import numpy as np
 import pytest
 

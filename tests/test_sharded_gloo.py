@@ -1,4 +1,4 @@
-"""world_size-2 gloo test of the sharded decode path on CPU (SURVEY §8e): two processes, each holding its shard
+"""world_size-2 gloo test of the sharded decode path on CPU: two processes, each holding its shard
 (crabml_b200/sharding.py) of a small synthetic model as oracle tensors, replay the sharded op sequence with the exchange
 step over torch.distributed/gloo; logits must agree on both ranks bit for bit and with the unsharded replay."""
 import os

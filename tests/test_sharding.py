@@ -1,4 +1,4 @@
-"""Host logic of the sharded decode path (crabml_b200/sharding.py, SURVEY §8e): the shard plan and the GGUF byte slicing.
+"""Host logic of the sharded decode path (crabml_b200/sharding.py): the shard plan and the GGUF byte slicing.
 CPU only; the oracle's dequantiser is the checker."""
 import numpy as np
 import pytest
@@ -19,7 +19,7 @@ def test_deal_covers_everything_once():
 
 
 def test_llama2_7b_plans():
-    # Q8_0: 11008 / 8 = 1376 = 43 blocks of 32 each (SURVEY §8e)
+    # Q8_0: 11008 / 8 = 1376 = 43 blocks of 32 each
     plans = [S.make_plan(32, 32, 4096, 11008, 32000, oc.Q8_0, r, 8) for r in range(8)]
     assert all(p.hidden_local == 1376 and p.q_rows[1] == 512 and p.vocab_rows[1] == 4000 for p in plans)
     # K-quants: 43 super-blocks of 256 -> 6,6,6,5,5,5,5,5

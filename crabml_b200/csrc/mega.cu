@@ -1,7 +1,7 @@
 // mega.cu -- one persistent kernel per token ("megakernel") for the fused decode path: the variant whose weight stream runs through
 // REGISTERS (two segments per warp in flight, look-ahead prefetch across the grid barrier).  The default is the variant in
 // mega_ring.cu (weights through a TMA-fed shared-memory ring); this one is the fallback (CRABML_MEGA_FLAGS without
-// MK_F_RING, or a phase table whose working area leaves the ring fewer than 12 slots) and the A/B baseline.  The phase bodies both
+// MK_F_RING, or a phase table whose working area leaves the ring fewer than 6 slots) and the A/B baseline.  The phase bodies both
 // kernels share live in mega_phases.cuh; the host side at the bottom of this file serves both.
 //
 // Why: profiles/r01c -- on B200 a kernel boundary costs ~4-5 us for a full-GPU streaming kernel (drain, launch latency,
@@ -434,7 +434,7 @@ bool cc_mega_generic_supported(int type, int64_t k) {
 }
 
 // developer A/B switches: CRABML_MEGA_FLAGS replaces the default flag word (see MK_F_* and the L2 budget byte)
-#define MK_DEFAULT_FLAGS (MK_F_LOOK | MK_F_WSTAGE | MK_F_POLLCNT | MK_F_XEARLY | MK_F_RING | MK_F_RPAIR)      // ring + pairs: 2227 us vs 2386 us per 7B Q8_0 token ; without them 2407 us vs 2586 us (0x5), each on one box
+#define MK_DEFAULT_FLAGS (MK_F_LOOK | MK_F_WSTAGE | MK_F_POLLCNT | MK_F_XEARLY | MK_F_RING)
 int cc_mega_flags() {
     static const int f = getenv("CRABML_MEGA_FLAGS") ? (int)strtol(getenv("CRABML_MEGA_FLAGS"), nullptr, 0) : MK_DEFAULT_FLAGS;
     return f;

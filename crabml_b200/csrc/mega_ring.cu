@@ -4,26 +4,31 @@
 // boundary (slowest warp -> grid barrier -> activation prologue, 6-9 us) no warp issues loads, so only the 2 look-ahead segments per
 // warp (20 MB per GPU, 3 us of HBM time) cover the bubble and HBM idles for the rest: 2.36 ms per Llama-2-7B Q8_0 token against
 // 1.07 ms of pure streaming.  Weights are immutable, so nothing forces the weight stream to follow the phase order of the compute:
-//   * warps 16-19 of every CTA are PRODUCERS: their threads walk the phase table on their own, ahead of the compute warps, and
-//     issue cp.async.bulk (TMA) copies of row segments (4 groups of 32 blocks: 4096 B of Q8_0 quants + 256 B of f16 scales) into a
-//     ring of shared-memory slots -- as many as fit beside the per-phase working area (~37-47 slots = 160-200 KB per SM, 24-30 MB
-//     per GPU in flight or landed).  It never waits for a barrier or an activation: whenever a slot is free the next segment of
-//     this CTA's rows -- of this phase or any later one -- is already being fetched.
-//   * warps 0-15 are CONSUMERS: same row dealing (row r -> CTA r % 148, rows of a CTA -> its warps round-robin), same per-lane
-//     block order, same arithmetic as mega.cu / matvec_stream.cu (bit-identical results), but a segment is read from the ring with
-//     LDS.128 after waiting on the slot's "full" mbarrier, and the slot is handed back through its "empty" mbarrier.  No weight
-//     registers live across phases -> no register pipe, no look-ahead bookkeeping, 96 registers are enough.
-//   * the activation prologue works from registers (x row: <= 4 float4 per thread straight from L2) instead of a shared-memory
-//     staging copy: the working area shrinks from 78 KB to ~18 KB (matvec) and the ring takes the rest.
-// The 512 compute threads synchronise on named barrier 1 (MK_SYNC); the producer warp never joins it.
+//   * warps 16-18 of every CTA are PRODUCERS: their threads walk the phase table on their own, ahead of the compute warps, and issue cp.async.bulk (TMA) copies
+//     of items -- two rows' segment of 128 blocks: 8192 B of Q8_0 quants + 512 B of f16 scales -- into a ring of shared-memory slots, as many as fit beside
+//     the per-phase working area (18 to 20 = 160-174 KB per SM, 25 MB per GPU).  They never wait for a barrier or an activation: whenever a slot is free the
+//     next item of this CTA's rows -- of this phase or any later one -- is being fetched.
+//   * warp 19 asks L2 for the items behind the ring, up to 224 KB of them per SM (33 MB per GPU), at 20 B per cycle and SM: a full ring is 4 us of HBM time, the
+//     time between one phase's last row and the next one's first 5 to 7 us, the attention phase 7.  A 7B Q8_0 token 2130 -> 1980 us (150, 224, 280, 330 KB and 16 to
+//     24 B the same within 1 %; 417 KB = 62 MB per GPU 2514: more than the L2 holds of it).  Without a pace the requests queue in front of the barrier's own
+//     traffic: with 19 MB under way a barrier takes 20 us instead of 2 (measured by itself; at 6.3 TB/s with 7 MB under way 3.4).
+//   * warps 0-15 are CONSUMERS: the CTA's rows are one contiguous run, pairs of rows dealt round-robin; same per-lane block order, same arithmetic as mega.cu /
+//     matvec_stream.cu (bit-identical results), but a segment is read from the ring with LDS.128 after waiting on the slot's "full" mbarrier, and the slot is
+//     handed back through its "done" word.  No weight registers live across phases, 96 registers are enough -- barely: a spilled register is a trip to L2 (the
+//     ring leaves no L1), and the same phases with the activation in registers, 600 bytes of spills, took 2540 us a token.
+// The 512 compute threads synchronise on named barrier 1 (MK_SYNC); the producer warps never join it.
 // 20 warps: five per SM sub-partition, so its 16384 registers allow 96 per thread (what __launch_bounds__(640, 1) yields).
 #define MK_SYNC() asm volatile("bar.sync 1, 512;" ::: "memory")
 #define MK_GENERIC_NOINLINE 1
 #include "mega_phases.cuh"
+#include "quotients.cuh"
 
 #define MR_PRODUCER_WARPS 4        // 20 warps: five per SM sub-partition, still 96 registers per thread
+#define MR_ISSUERS 96                // threads that issue copies: three warps (two: +1 %); the fourth warp prefetches
+#define MR_L2_LEAD (224 * 1024)       // bytes of items asked into L2 behind the ring, per SM
+#define MR_L2_RATE 20                 // bytes per cycle and SM at which they are asked for: 5.8 TB/s
 #define MR_THREADS (MK_THREADS + 32 * MR_PRODUCER_WARPS)
-#define MR_MAX_SLOTS 112
+#define MR_MAX_SLOTS 56
 #define MR_DESC_WORDS ((int)(sizeof(MkPhase) / 4))
 #define MR_DESC_PER_LANE ((MR_DESC_WORDS + 31) / 32)
 
@@ -48,7 +53,7 @@ __device__ __forceinline__ bool mr_test_wait(unsigned bar, unsigned parity) {
     asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Slot hand-back: the consumer stores (entry number + 1) into the slot's "done" word (release), the producer polls it (acquire) for
+// Slot hand-back: the consumer stores (item number + 1) into the slot's "done" word (release), the producer polls it (acquire) for
 // exactly the previous tenant's number -- an mbarrier parity could not tell one lap from two.  `dep` ties the store behind the
 // arithmetic that consumed the slot's data.
 __device__ __forceinline__ void mr_release(unsigned done_addr, unsigned v, float dep) { asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(done_addr), "r"(v), "f"(dep) : "memory"); }
@@ -58,11 +63,11 @@ __device__ __forceinline__ unsigned mr_ld_acquire_shared(unsigned addr) {
     return v;
 }
 
-// rows of a streaming MATVEC phase that belong to this CTA, as "units": unit u -> concatenated row first + u * stride, consumed by
-// warp u % 16; a unit is V virtual rows (2 for the gate/up pair, else 1) of NSEG segments each.  Producer and consumers derive the
-// same entry sequence from this.
+// Rows of a streaming MATVEC phase that belong to this CTA: one contiguous run.  They go through the ring as ITEMS of two virtual rows -- two rows next to
+// each other, or the gate and the up row of one unit -- and one segment of them; group (row pair) P is consumed by warp P % 16, segment after segment.
+// Producer and consumers derive the same item sequence from this: item of group P, segment s = P * NSEG + s.
 struct MrGeo {
-    int nb, GR, NSEG, V, E, n_units, first, stride, last_half_off, m_cat;
+    int nb, GR, NSEG, n_rows, groups, first, last_half_off;
     bool pair;
 };
 __device__ __forceinline__ MrGeo mr_geo(const StreamArgs& A) {
@@ -70,46 +75,65 @@ __device__ __forceinline__ MrGeo mr_geo(const StreamArgs& A) {
     g.nb = A.k >> 5; g.GR = (g.nb + 31) >> 5; g.NSEG = (g.GR + MK_SEG - 1) / MK_SEG;
     g.pair = A.epilogue == 2;
     const StreamMats& M = A.mats;
-    g.m_cat = g.pair ? M.m[0] : M.m[0] + (M.n > 1 ? M.m[1] : 0) + (M.n > 2 ? M.m[2] : 0);
-    if (A.epilogue == 3) {             // exchange phases: one contiguous block of rows per CTA (mega.cu mk_geo)
-        const int rpc = (((g.m_cat + (int)gridDim.x - 1) / (int)gridDim.x) + 3) & ~3;
-        g.first = (int)blockIdx.x * rpc; g.stride = 1;
-        g.n_units = min(rpc, max(0, g.m_cat - g.first));
+    const int m_cat = g.pair ? M.m[0] : M.m[0] + (M.n > 1 ? M.m[1] : 0) + (M.n > 2 ? M.m[2] : 0);
+    if (A.epilogue == 3) {             // exchange phases: blocks of a multiple of 4 rows (mega.cu mk_geo)
+        const int rpc = (((m_cat + (int)gridDim.x - 1) / (int)gridDim.x) + 3) & ~3;
+        g.first = (int)blockIdx.x * rpc;
+        g.n_rows = min(rpc, max(0, m_cat - g.first));
     } else {
-        g.first = (int)blockIdx.x; g.stride = (int)gridDim.x;
-        g.n_units = g.first < g.m_cat ? (g.m_cat - g.first + g.stride - 1) / g.stride : 0;
+        const int each = m_cat / (int)gridDim.x, more = m_cat - each * (int)gridDim.x;
+        g.first = (int)blockIdx.x * each + min((int)blockIdx.x, more);
+        g.n_rows = each + ((int)blockIdx.x < more ? 1 : 0);
     }
-    g.V = g.pair ? 2 : 1;
-    g.E = g.V * g.NSEG;
+    g.groups = g.pair ? g.n_rows : (g.n_rows + 1) >> 1;
     g.last_half_off = 16 * (g.nb - 32 * (g.GR - 1));
     return g;
 }
-__device__ __forceinline__ int mr_locate(const StreamMats& M, const MrGeo& g, int rc, int v, int& mat) {
+// concatenated row -> (matrix, row of it)
+__device__ __forceinline__ int mr_locate(const StreamMats& M, int rc, int& mat) {
     mat = 0;
     int r = rc;
-    if (g.pair) { mat = v; return r; }
     if (M.n > 1 && r >= M.m[0]) { r -= M.m[0]; mat = 1; if (M.n > 2 && r >= M.m[1]) { r -= M.m[1]; mat = 2; } }
     return r;
 }
 
-// ---- producer warp: runs ahead of everybody ---------------------------------------------------------------------------------------------
-// All 32 lanes issue (a single issuing thread manages ~1 entry per 350 cycles -- profiles/r02m: 1.8 TB/s); lane l owns the entries l, l + 32, ...
-// of a phase: it decomposes the entry index into (unit, virtual row, segment), waits until the slot's previous tenant has been consumed, arms the
-// slot's "full" barrier with the byte count, issues the two bulk copies (quants, scales) and publishes the entry number in the slot's
-// sequence word.  Consumers check that word before they look at the barrier: an mbarrier parity alone cannot tell "this use has not
-// landed" from "the previous use has not landed" when a warp gets more than one lap ahead (16 warps x 3 segments > 40 slots).
-// (Measured: 1 / 2 / 4 / 8 producer warps = 2859 / 2782 / 2262 / 2435 us per token -- a warp's probe-and-issue trip takes ~400
-// cycles, so the number of polling warps bounds the refill rate, and at 8 the 80-register cap starts to cost.  Sleeping after a failed probe,
-// SIMT-wide parameter computation, in-order probe loops and fence-free hand-back words changed nothing.)
+// where item j of a phase comes from: quants and scales of its two rows (two = false: one row, or two rows of one matrix next to each other as one run)
+struct MrItem { const uint8_t* q[2]; const uint16_t* d[2]; unsigned qbytes, dbytes; bool two; };
+__device__ __forceinline__ MrItem mr_item(const StreamMats& M, const MrGeo& g, unsigned BB, int j) {
+    MrItem it;
+    const int P = j / g.NSEG, sg = j - P * g.NSEG;
+    int mat, matB = 1;
+    const int rA = mr_locate(M, g.first + (g.pair ? P : 2 * P), mat);
+    int rB = rA;
+    it.two = g.pair || 2 * P + 1 < g.n_rows;
+    if (!g.pair && it.two) rB = mr_locate(M, g.first + 2 * P + 1, matB);
+    if (!it.two) matB = mat;
+    const size_t at = (size_t)sg * (MK_SEG * 32), d_row = (size_t)CC_D_STRIDE(g.nb);
+    const unsigned nbe = (unsigned)min(MK_SEG * 32, g.nb - MK_SEG * 32 * sg);
+    it.qbytes = nbe * BB;
+    it.dbytes = (nbe * 2u + 15u) & ~15u;               // the scale rows are padded to 16 bytes (CC_D_STRIDE): a short last segment copies its padding
+    it.q[0] = M.qs[mat] + ((size_t)rA * g.nb + at) * BB; it.d[0] = M.d[mat] + (size_t)rA * d_row + at;
+    it.q[1] = M.qs[matB] + ((size_t)rB * g.nb + at) * BB; it.d[1] = M.d[matB] + (size_t)rB * d_row + at;
+    if (it.two && g.NSEG == 1 && it.q[1] == it.q[0] + it.qbytes && (const uint8_t*)it.d[1] == (const uint8_t*)it.d[0] + it.dbytes) { it.qbytes *= 2; it.dbytes *= 2; it.two = false; }
+    return it;
+}
+
+// ---- producer warps: run ahead of everybody ---------------------------------------------------------------------------------------------
+// All lanes issue (a single issuing thread manages ~1 copy pair per 570 cycles): thread t owns the items whose number over the whole launch is t mod 96; it
+// decomposes the item into rows and a segment, waits until the slot's previous tenant has been consumed, arms the slot's "full" barrier with the byte
+// count, issues the bulk copies (two rows of one matrix that lie next to each other: one for the quants, one for the scales) and publishes the item number in
+// the slot's sequence word.  Consumers check that word before they look at the barrier: an mbarrier parity alone cannot tell "this use has not landed" from
+// "the use before has not been consumed" when one warp is laps ahead of another.
 __device__ void mr_producer(const MkPhase* __restrict__ phases, int n_phases, const MrRing R, unsigned full0, unsigned done0, unsigned ring0,
-                            MkPhase* s_pd, volatile unsigned* s_seq, volatile int* s_abort, int* s_prod_done, unsigned long long* prof_tail, const bool pairs, const bool kvpf, const uint8_t* __restrict__ dyn) {
+                            MkPhase* s_pd, volatile unsigned* s_seq, volatile int* s_abort, volatile int* s_dead, volatile int* s_issued, int* s_prod_done, const bool kvpf, const uint8_t* __restrict__ dyn) {
     const int lane = threadIdx.x & 31;
-    const int pt = (int)threadIdx.x - MK_THREADS;          // producer thread 0 .. 32 * MR_PRODUCER_WARPS - 1: owns the entries pt, pt + 128, ... of every phase
-    unsigned long long p_trips = 0, p_cyc = 0, p_iss = 0;       // developer profiling (CTA 0 / lane 0)
+    const int pt = (int)threadIdx.x - MK_THREADS;          // producer thread 0 .. 32 * MR_PRODUCER_WARPS - 1
     for (int i = lane; i < MR_DESC_WORDS; i += 32) ((int*)&s_pd[0])[i] = ((const int*)phases)[i];
     __syncwarp();
     unsigned ent = 0;
     bool dead = false;
+    long long t_last = clock64();          // the prefetcher's
+    unsigned idle = 0;
     for (int p = 0; p < n_phases && !dead; p++) {
         int nw[MR_DESC_PER_LANE];
 #pragma unroll
@@ -138,48 +162,55 @@ __device__ void mr_producer(const MkPhase* __restrict__ phases, int n_phases, co
             const StreamMats& M = A.mats;
             const MrGeo g = mr_geo(A);
             const unsigned BB = ph.wtype == CC_Q8_0 ? 32u : 16u;
-            const unsigned doff = MK_SEG * 32u * BB;
-            const int N = g.n_units * g.E, twoE = 2 * g.E, Npair = (g.n_units >> 1) * twoE;
-            // a flat loop, one probe of the thread's own slot per trip (a load of the slot's "done" word: no suspension): thread t serves the entries
-            // t, t + 128, ... at its own pace, so a slot is refilled as soon as it is released, not when the slowest lane of a batch is ready
-            int j = pt;
+            const unsigned doff = 2u * MK_SEG * 32u * BB;
+            const int N = g.groups * g.NSEG;
+            if (pt >= MR_ISSUERS) {                // the L2 prefetcher
+                const int item = (int)(2u * MK_SEG * 32u * (BB + 2u)), pace = item / MR_L2_RATE, lead = R.nslots + MR_L2_LEAD / item;
+                for (int j = 0; j < N && !dead;) {
+                    const int issued = __shfl_sync(0xffffffffu, *s_issued, 0) - (int)ent;
+                    if (j < issued) { j = min(issued, N); continue; }
+                    const long long now = __shfl_sync(0xffffffffu, clock64(), 0);
+                    if (t_last < now - 2 * pace) t_last = now - 2 * pace;
+                    const int n = min(min(N - j, issued + lead - j), (int)((now - t_last) / pace));          // (two items at most)
+                    if (n <= 0) { dead = (++idle & 0x3FFu) == 0 && __any_sync(0xffffffffu, *s_abort || *s_dead); continue; }
+                    if (lane < 4 * n) {                // four lanes an item
+                        const MrItem im = mr_item(M, g, BB, j + (lane >> 2));
+                        const int row = lane & 1;
+                        const void* src = lane & 2 ? (row ? (const void*)im.d[1] : (const void*)im.d[0]) : (row ? (const void*)im.q[1] : (const void*)im.q[0]);
+                        if (!row || im.two) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(lane & 2 ? im.dbytes : im.qbytes) : "memory");
+                    }
+                    __syncwarp();
+                    j += n; t_last += (long long)n * pace;
+                }
+                ent += (unsigned)N;
+            } else {
+            // a flat loop, one probe of the thread's own slot per trip (a load of the slot's "done" word: no suspension), so a slot is refilled as soon as it is
+            // released, not when the slowest lane of a batch is ready
+            int j = (pt + MR_ISSUERS - (int)(ent % MR_ISSUERS)) % MR_ISSUERS;
             bool have = false, mydead = false;
-            const uint8_t* q0 = nullptr; const uint16_t* d0 = nullptr;
-            unsigned nbe = 0, e = 0, slot = 0, use = 0, it = 0;
-            const long long pc0 = clock64();
+            MrItem im = {};
+            unsigned e = 0, slot = 0, use = 0, it = 0;
             while (j < N) {
-                p_trips++;
                 if (!have) {
-                    // ring order: the units of a CTA go in PAIRS whose entries alternate (A v0 s0, B v0 s0, A v0 s1, B v0 s1, ...): the consumer warp that
-                    // takes a pair always works on two ADJACENT entries and hands them back at once (16 warps x 2 entries < the ring); an odd last unit
-                    // follows on its own
-                    int u, vs;
-                    if (!pairs) { u = j / g.E; vs = j - u * g.E; }
-                    else if (j < Npair) { const int P = j / twoE, w = j - P * twoE; u = 2 * P + (w & 1); vs = w >> 1; }
-                    else { u = g.n_units - 1; vs = j - Npair; }
-                    const int v = vs / g.NSEG, sg = vs - v * g.NSEG;
-                    int mat;
-                    const int r = mr_locate(M, g, g.first + u * g.stride, v, mat);
-                    q0 = M.qs[mat] + ((size_t)r * g.nb + (size_t)sg * (MK_SEG * 32)) * BB;
-                    d0 = M.d[mat] + (size_t)r * CC_D_STRIDE(g.nb) + sg * (MK_SEG * 32);
-                    nbe = (unsigned)min(MK_SEG * 32, g.nb - MK_SEG * 32 * sg);
+                    im = mr_item(M, g, BB, j);
                     e = ent + (unsigned)j; slot = e % (unsigned)R.nslots; use = e / (unsigned)R.nslots;
                     have = true;
                 }
                 if (!use || mr_ld_acquire_shared(done0 + 4u * slot) == e - (unsigned)R.nslots + 1u) {      // the slot's previous tenant has been consumed
                     const unsigned fb = full0 + 8u * slot, dst = ring0 + slot * (unsigned)R.slot_bytes;
-                    const unsigned dbytes = (nbe * 2u + 15u) & ~15u;        // the scale rows are padded to 16 bytes (CC_D_STRIDE): a short last segment copies its padding
-                    mr_expect_tx(fb, nbe * BB + dbytes);
-                    mr_bulk_g2s(dst, q0, nbe * BB, fb);
-                    mr_bulk_g2s(dst + doff, d0, dbytes, fb);
+                    mr_expect_tx(fb, (im.qbytes + im.dbytes) << (im.two ? 1 : 0));
+                    mr_bulk_g2s(dst, im.q[0], im.qbytes, fb);
+                    if (im.two) mr_bulk_g2s(dst + im.qbytes, im.q[1], im.qbytes, fb);
+                    mr_bulk_g2s(dst + doff, im.d[0], im.dbytes, fb);
+                    if (im.two) mr_bulk_g2s(dst + doff + im.dbytes, im.d[1], im.dbytes, fb);
                     __threadfence_block();
                     s_seq[slot] = e + 1u;
-                    j += 32 * MR_PRODUCER_WARPS; have = false; p_iss++;
-                } else if ((++it & 0x3FFu) == 0 && *s_abort) { mydead = true; break; }
+                    j += MR_ISSUERS; have = false; atomicAdd((int*)s_issued, 1);
+                } else if ((++it & 0x3FFu) == 0 && (*s_abort || *s_dead)) { mydead = true; break; }
             }
-            p_cyc += (unsigned long long)(clock64() - pc0);
             dead = __any_sync(0xffffffffu, mydead);
             ent += (unsigned)N;
+            }
         }
         __syncwarp();
 #pragma unroll
@@ -187,11 +218,10 @@ __device__ void mr_producer(const MkPhase* __restrict__ phases, int n_phases, co
         __syncwarp();
     }
     if (lane == 0) { __threadfence_block(); atomicAdd(s_prod_done, 1); }
-    if (pt == 0 && prof_tail && blockIdx.x == 0) { prof_tail[1] = p_trips; prof_tail[2] = p_cyc; prof_tail[3] = p_iss; }
 }
 
 // ---- consumer side of a streaming MATVEC phase ------------------------------------------------------------------------------------------
-struct MrCons { bool pairs; unsigned full0, done0; const uint8_t* ring; int slot_bytes, nslots; unsigned ent_base; int* s_unit; volatile unsigned* s_seq; volatile int* s_dead; unsigned* err_dev; unsigned* err_host; };
+struct MrCons { unsigned full0, done0; const uint8_t* ring; int slot_bytes, nslots; unsigned ent_base; volatile unsigned* s_seq; volatile int* s_dead; unsigned* err_dev; unsigned* err_host; };
 
 // Bounded wait for a slot to fill.  A wait that does not end within 2 s (it takes microseconds) raises the error words (code 4, reported by
 // cc_check_async_error) and marks the ring dead for the whole CTA: every later wait returns at once, the launch drains with garbage
@@ -216,26 +246,6 @@ __device__ __forceinline__ void mr_wait_full(const MrCons& RC, unsigned slot, un
     }
 }
 
-template <int TYPE>
-__device__ __forceinline__ void mr_seg_lds(MkSeg& S, const uint8_t* sp, int seg, int nb, int GR, int last_half_off, int lane) {
-    constexpr int GB = TYPE == CC_Q8_0 ? 1024 : 512;
-    const uint8_t* q = sp + lane * 16;
-    const uint16_t* d = (const uint16_t*)(sp + MK_SEG * GB) + lane;
-#pragma unroll
-    for (int g = 0; g < MK_SEG; g++) {
-        const int gi = seg * MK_SEG + g;
-        const bool on = gi * 32 + lane < nb;
-        if constexpr (TYPE == CC_Q8_0) {
-            const int hoff = gi == GR - 1 ? last_half_off : 512;
-            if (on) { S.a[g] = *(const int4*)(q + g * GB); S.b[g] = *(const int4*)(q + g * GB + hoff); S.s[g] = d[g * 32]; }
-            else { S.a[g] = make_int4(0, 0, 0, 0); S.b[g] = S.a[g]; S.s[g] = 0; }
-        } else {
-            if (on) { S.a[g] = *(const int4*)(q + g * GB); S.s[g] = d[g * 32]; }
-            else { S.a[g] = make_int4(0, 0, 0, 0); S.s[g] = 0; }
-        }
-    }
-}
-
 // Activation quants in shared memory, per group of 32 blocks: the 16-byte first halves of all 32 blocks, then the second halves (the layout of
 // the Q8_0 weight plane) -- lane l reads block 32 g + l with two conflict-free LDS.128 (block-major, 32 bytes apart, is a 2-way bank conflict:
 // 64 instead of 32 shared-memory wavefronts per segment, and the ring's throughput is bounded by shared-memory bandwidth)
@@ -248,40 +258,34 @@ __device__ __forceinline__ int mr_act_int4(int i) {           // i = 16-byte ind
     return (b >> 5) * 64 + (i & 1) * 32 + (b & 31);
 }
 
-// One segment (4 groups) of TWO rows against the same activation segment: the activation quants and scales are read once for both rows
-// (shared-memory wavefronts per 4352-byte entry: 34 TMA write + 34 weight read + 16 activation, against 64 + for one row at a time).
-// Per row the arithmetic is mk_seg_dot's, term by term (bit-identical to matvec_stream.cu).
+// One segment (up to 4 groups of 32 blocks) of two rows against one activation: it is read once for both (shared-memory wavefronts per item: 68 to fill it, 72 for
+// the weights, 36 for the activation).  `left` = blocks of the row from this segment on: a lane behind them reads what the slot happens to hold (always
+// inside the slot) against zero quants and a scale it sets to zero.  Per row the arithmetic is mk_seg_dot's, term by term (bit-identical to matvec_stream.cu).
 template <int TYPE>
-__device__ __forceinline__ void mr_dot2(const uint8_t* spA, const uint8_t* spB, int seg, int nb, int GR, int last_half_off, int lane,
-                                        const int4* aq_l, const float* ad_l, const int* as_l, float& partA, float& partB) {
+__device__ __forceinline__ void mr_dot2(const uint8_t* sp, unsigned b_off, const uint8_t* dp, unsigned db_off, int left, int last_half_off, int lane,
+                                        const int4* aq, const float* ad, const int* as, float& partA, float& partB) {
     constexpr int GB = TYPE == CC_Q8_0 ? 1024 : 512;
-    const uint8_t* qA = spA + lane * 16;
-    const uint8_t* qB = spB + lane * 16;
-    const uint16_t* dA = (const uint16_t*)(spA + MK_SEG * GB) + lane;
-    const uint16_t* dB = (const uint16_t*)(spB + MK_SEG * GB) + lane;
-    const int4* aq = aq_l + seg * (MK_SEG * 64);
-    const float* ad = ad_l + seg * (MK_SEG * 32);
-    const int4 z4 = make_int4(0, 0, 0, 0);
+    const uint8_t* qA = sp + lane * 16;
+    const uint16_t* dA = (const uint16_t*)dp + lane;
     float accA = 0.0f, accB = 0.0f;
+    left -= lane;
 #pragma unroll
     for (int g = 0; g < MK_SEG; g++) {
-        const int gi = seg * MK_SEG + g;
-        const bool on = gi * 32 + lane < nb;
-        const int4 alo = aq[g * 64], ahi = aq[g * 64 + 32];
-        const float adv = ad[g * 32];
+        const bool on = left > 0;
+        const uint16_t sA = on ? dA[0] : (uint16_t)0, sB = on ? dA[db_off >> 1] : (uint16_t)0;
+        const int4 alo = aq[0], ahi = aq[32];
+        const float adv = ad[0];
         if constexpr (TYPE == CC_Q8_0) {
-            const int hoff = gi == GR - 1 ? last_half_off : 512;
-            int4 a0 = z4, a1 = z4, b0 = z4, b1 = z4; uint16_t sA = 0, sB = 0;
-            if (on) { a0 = *(const int4*)(qA + g * GB); a1 = *(const int4*)(qA + g * GB + hoff); sA = dA[g * 32];
-                      b0 = *(const int4*)(qB + g * GB); b1 = *(const int4*)(qB + g * GB + hoff); sB = dB[g * 32]; }
+            const int hoff = left + lane <= 32 ? last_half_off : 512;
+            const int4 a0 = *(const int4*)qA, a1 = *(const int4*)(qA + hoff);
+            const int4 b0 = *(const int4*)(qA + b_off), b1 = *(const int4*)(qA + b_off + hoff);
             const int sumA = mk_dp16(a0, alo) + mk_dp16(a1, ahi);
             const int sumB = mk_dp16(b0, alo) + mk_dp16(b1, ahi);
             accA += (float)sumA * h2f_bits(sA) * adv;
             accB += (float)sumB * h2f_bits(sB) * adv;
         } else {
-            int4 wA = z4, wB = z4; uint16_t sA = 0, sB = 0;
-            if (on) { wA = *(const int4*)(qA + g * GB); sA = dA[g * 32]; wB = *(const int4*)(qB + g * GB); sB = dB[g * 32]; }
-            const int asv = as_l[(seg * MK_SEG + g) * 32];
+            const int asv = as[0];
+            const int4 wA = *(const int4*)qA, wB = *(const int4*)(qA + b_off);
             const int4 loA = make_int4(wA.x & 0x0F0F0F0F, wA.y & 0x0F0F0F0F, wA.z & 0x0F0F0F0F, wA.w & 0x0F0F0F0F);
             const int4 hiA = make_int4((wA.x >> 4) & 0x0F0F0F0F, (wA.y >> 4) & 0x0F0F0F0F, (wA.z >> 4) & 0x0F0F0F0F, (wA.w >> 4) & 0x0F0F0F0F);
             const int4 loB = make_int4(wB.x & 0x0F0F0F0F, wB.y & 0x0F0F0F0F, wB.z & 0x0F0F0F0F, wB.w & 0x0F0F0F0F);
@@ -290,18 +294,117 @@ __device__ __forceinline__ void mr_dot2(const uint8_t* spA, const uint8_t* spB, 
             const int sumB = mk_dp16(loB, alo) + mk_dp16(hiB, ahi) - 8 * asv;
             accA += (float)sumA * h2f_bits(sA) * adv;
             accB += (float)sumB * h2f_bits(sB) * adv;
+            as += 32;
         }
+        qA += GB; dA += 32; aq += 64; ad += 32; left -= 32;
     }
     partA = accA; partB = accB;
 }
 
-// shared memory of the phase: quants [nbp * 32] | f32 scales [nbp] | block sums [nbp] | reduction scratch 256 B | exchange stage 2 KB
+__device__ __forceinline__ bool mr_tiny(float x) { return fabsf(x) < 0x1p-60f && x != 0.0f; }
+// Fused prologue: [exchange reduction] + [rms_norm * w] + Q8_0 quantisation of x by EVERY CTA: thread t owns the float4 chunks t, t + 512, ... (the
+// canonical reduction order of common.cuh, and 8 consecutive threads = one 32-block).  All chunks of a thread are asked for at once, into shared memory, and the
+// loops over them are short: the phases of a layer do not stay in the near instruction caches, and the kernel's 96 registers have no room for a row (a spilled
+// register is a trip to L2 here, the ring leaves no L1).  The divisions are multiplications with the same bits (quotients.cuh).
+#define MR_ROW_PIECE 12288             // elements (whole passes of 512 threads x 4)
+template <int TYPE>
+__device__ __forceinline__ void mr_prologue(const MkPhase& ph, int k, int nbp, int* s_q32, float* s_d, int* s_s, float* s_red, float4* s_x, const CommDev& comm, unsigned xseq) {
+    const int n4 = k >> 2, nch = nbp << 3;                              // chunks of the row; with the zeros behind it (nbp % 128 == 0: whole passes of 512 threads)
+    const int piece = min(n4, MR_ROW_PIECE / 4);                        // a longer row goes through the staging area in pieces
+    const float* nw = ph.norm_w;
+    float4* s_w = s_x + piece;
+    const float* xbase = ph.red_n ? comm.data[comm.rank] + (size_t)(xseq & 1u) * CC_COMM_MAX_RANKS * CC_COMM_MAX_ELEMS : ph.x;
+    auto fetch = [&](int i0) {
+        const int n = min(piece, n4 - i0);
+#pragma unroll 2
+        for (int i = threadIdx.x; i < n; i += MK_THREADS) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(s_x + i)), "l"((const float4*)xbase + i0 + i) : "memory");
+            if (nw) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(s_w + i)), "l"((const float4*)nw + i0 + i) : "memory");
+        }
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");     // (a thread reads only what it asked for itself)
+        if (ph.red_n) {                                                 // sum over ranks in rank order (+ residual): comm.cu
+#pragma unroll 1
+            for (int i = threadIdx.x; i < n; i += MK_THREADS) {
+                float4 a = s_x[i];
+                for (int p = 1; p < comm.world; p++) {
+                    const float4 t = __ldcg((const float4*)(xbase + (size_t)p * CC_COMM_MAX_ELEMS) + i0 + i);
+                    a.x += t.x; a.y += t.y; a.z += t.z; a.w += t.w;
+                }
+                if (ph.red_res) { const float4 r = __ldcg((const float4*)ph.red_res + i0 + i); a.x += r.x; a.y += r.y; a.z += r.z; a.w += r.w; }
+                s_x[i] = a;
+            }
+        }
+    };
+    float rms = 1.0f, rr = 1.0f;
+    if (nw) {
+        float ss = 0.0f;
+        for (int i0 = 0; i0 < n4; i0 += piece) {
+            fetch(i0);
+#pragma unroll 2
+            for (int i = threadIdx.x; i < min(piece, n4 - i0); i += MK_THREADS) ss += cc_sq4(s_x[i]);
+        }
+        ss = warp_sum(ss);
+        if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = ss;
+        MK_SYNC();
+        float t = 0.0f;
+#pragma unroll
+        for (int w = 0; w < MK_WARPS; w++) t += s_red[w];
+        rms = sqrtf(t / (float)k + ph.eps);
+        rr = 1.0f / rms;
+    }
+    const bool rms_ok = cc_quot_range(rms);
+    int i0 = 0;
+    if (!nw || n4 > piece) fetch(0);
+#pragma unroll 1
+    for (int i = threadIdx.x; i < nch; i += MK_THREADS) {               // chunk i = 4 elements of block i >> 3
+        if (i - i0 >= piece && i0 + piece < n4) { i0 += piece; fetch(i0); }             // (whole passes of 512 threads: all of them together)
+        const bool live = i < n4;
+        float4 v = live ? s_x[i - i0] : make_float4(0, 0, 0, 0);
+        if (ph.orig && blockIdx.x == 0 && live) ((float4*)ph.orig)[i] = v;              // Tensor::dup of the un-normalised row (llama2.rs:227,607)
+        const float4 x = v;
+        bool doubt = false;
+        if (nw && live) {
+            const float4 w = s_w[i - i0];
+            doubt = !rms_ok || mr_tiny(v.x) || mr_tiny(v.y) || mr_tiny(v.z) || mr_tiny(v.w);
+            v = make_float4(cc_quot_by(v.x, rms, rr) * w.x, cc_quot_by(v.y, rms, rr) * w.y, cc_quot_by(v.z, rms, rr) * w.z, cc_quot_by(v.w, rms, rr) * w.w);
+        }
+        float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if (!live) amax = 1.0f;                                         // (blocks behind the row: zeros)
+        doubt = doubt || !cc_quot_range(amax);
+        float d = cc_q8_0_scale(amax), rcp;
+        const int top = cc_q8_0_top(amax, d);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp) : "f"(d));        // within one unit in the last place
+        int q0 = cc_q8_0_quant(v.x, amax, top, rcp, doubt), q1 = cc_q8_0_quant(v.y, amax, top, rcp, doubt);
+        int q2 = cc_q8_0_quant(v.z, amax, top, rcp, doubt), q3 = cc_q8_0_quant(v.w, amax, top, rcp, doubt);
+        if (__any_sync(0xffffffffu, doubt)) {                           // rare: the whole warp's chunk with its divisions
+            v = x;
+            if (nw && live) { const float4 w = s_w[i - i0]; v = make_float4((v.x / rms) * w.x, (v.y / rms) * w.y, (v.z / rms) * w.z, (v.w / rms) * w.w); }
+            amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            d = amax / 127.0f;
+            q0 = live ? __float2int_rz(v.x / d) : 0; q1 = live ? __float2int_rz(v.y / d) : 0; q2 = live ? __float2int_rz(v.z / d) : 0; q3 = live ? __float2int_rz(v.w / d) : 0;
+        }
+        s_q32[mr_act_word(i)] = (q0 & 255) | ((q1 & 255) << 8) | ((q2 & 255) << 16) | (q3 << 24);
+        if constexpr (TYPE == CC_Q4_0) {
+            int sq = q0 + q1 + q2 + q3;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            if ((threadIdx.x & 7) == 0) s_s[i >> 3] = sq;
+        }
+        if ((threadIdx.x & 7) == 0) s_d[i >> 3] = live ? __half2float(__float2half_rn(d)) : 0.0f;
+    }
+}
+
+// shared memory of the phase: quants [nbp * 32] | f32 scales [nbp] | block sums [nbp] | reduction scratch 256 B | exchange stage 2 KB | fused prologue: the row and its norm weights
 template <int TYPE>
 __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16_t* exp_lut, MrCons& RC, const CommDev& comm, unsigned xseq, unsigned long long* stamp1) {
     const StreamArgs& A = ph.mv;
     const int k = A.k;
     const MrGeo g = mr_geo(A);
-    const int nb = g.nb, GR = g.GR, NSEG = g.NSEG;
+    const int nb = g.nb, NSEG = g.NSEG;
     const bool pair = g.pair;
     const int nbp = NSEG * MK_SEG * 32;
     int8_t* s_q = (int8_t*)smem;
@@ -311,94 +414,8 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
     float* s_part = (float*)(smem + (size_t)nbp * 40 + 256);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const StreamMats& M = A.mats;
-    if (threadIdx.x == 0) *RC.s_unit = 0;          // ordered before the row loop by the MK_SYNC that ends the prologue
     if (ph.x) {
-        // Fused prologue: [exchange reduction] + [rms_norm * w] + Q8_0 quantisation of x by EVERY CTA, from registers: thread t owns the
-        // float4 chunks t, t + 512, ... (the canonical reduction order of common.cuh, and 8 consecutive threads = one 32-block)
-        const int n4 = k >> 2;
-        const int npass = nbp >> 6;                                    // 64 blocks per pass of 512 threads (nbp % 128 == 0)
-        const float4 z4 = make_float4(0, 0, 0, 0);
-        const float* xbase = ph.red_n ? comm.data[comm.rank] + (size_t)(xseq & 1u) * CC_COMM_MAX_RANKS * CC_COMM_MAX_ELEMS : ph.x;
-        auto load_x = [&](int i) -> float4 {                            // chunk i of the input row
-            if (i >= n4) return z4;
-            float4 a4 = __ldcg((const float4*)xbase + i);
-            if (ph.red_n) {                                             // sum over ranks in rank order (+ residual): comm.cu
-                for (int p = 1; p < comm.world; p++) {
-                    const float4 t4 = __ldcg((const float4*)(xbase + (size_t)p * CC_COMM_MAX_ELEMS) + i);
-                    a4.x += t4.x; a4.y += t4.y; a4.z += t4.z; a4.w += t4.w;
-                }
-                if (ph.red_res) { const float4 r4 = __ldcg((const float4*)ph.red_res + i); a4.x += r4.x; a4.y += r4.y; a4.z += r4.z; a4.w += r4.w; }
-            }
-            return a4;
-        };
-        float rms = 1.0f;
-        const bool in_regs = npass <= 4;
-        float4 xr[4], wr[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) { xr[j] = z4; wr[j] = z4; }
-        if (in_regs) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int i = j * MK_THREADS + (int)threadIdx.x;
-                if (j < npass) { xr[j] = load_x(i); if (ph.norm_w && i < n4) wr[j] = __ldg((const float4*)ph.norm_w + i); }
-            }
-        }
-        if (stamp1) stamp1[3] = globaltimer_ns();
-        if (ph.norm_w) {
-            float ss = 0.0f;
-            if (in_regs) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) if (j * MK_THREADS + (int)threadIdx.x < n4) ss += cc_sq4(xr[j]);
-            } else {
-                for (int i = threadIdx.x; i < n4; i += MK_THREADS) { const float4 v = load_x(i); ss += cc_sq4(v); }
-            }
-            ss = warp_sum(ss);
-            if (lane == 0) s_red[warp] = ss;
-            MK_SYNC();
-            float t = 0.0f;
-#pragma unroll
-            for (int w = 0; w < MK_WARPS; w++) t += s_red[w];
-            rms = sqrtf(t / (float)k + ph.eps);
-        }
-        if (stamp1) stamp1[4] = globaltimer_ns();
-        const int sub = threadIdx.x & 7;
-        int* s_q32 = (int*)s_q;
-        auto quant_chunk = [&](int i, float4 v, const float4& w4) {      // i = chunk index (block i >> 3), v = its 4 elements (zeros past the row)
-            const bool live = i < n4;
-            if (ph.orig && blockIdx.x == 0 && live) ((float4*)ph.orig)[i] = v;      // Tensor::dup of the un-normalised row (llama2.rs:227,607)
-            if (ph.norm_w && live) { v.x = (v.x / rms) * w4.x; v.y = (v.y / rms) * w4.y; v.z = (v.z / rms) * w4.z; v.w = (v.w / rms) * w4.w; }
-            float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-            const float d = amax / 127.0f;
-            v = make_float4(v.x / d, v.y / d, v.z / d, v.w / d);
-            const int q0 = live ? __float2int_rz(v.x) : 0, q1 = live ? __float2int_rz(v.y) : 0;
-            const int q2 = live ? __float2int_rz(v.z) : 0, q3 = live ? __float2int_rz(v.w) : 0;
-            s_q32[mr_act_word(i)] = (q0 & 255) | ((q1 & 255) << 8) | ((q2 & 255) << 16) | (q3 << 24);
-            if constexpr (TYPE == CC_Q4_0) {
-                int sq = q0 + q1 + q2 + q3;
-#pragma unroll
-                for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-                if (sub == 0) s_s[i >> 3] = sq;
-            }
-            if (sub == 0) s_d[i >> 3] = live ? __half2float(__float2half_rn(d)) : 0.0f;
-        };
-        if (in_regs) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) if (j < npass) quant_chunk(j * MK_THREADS + (int)threadIdx.x, xr[j], wr[j]);
-        } else {
-            for (int j0 = 0; j0 < npass; j0 += 4) {                      // four chunks requested before the first is quantised
-                float4 v[4], w4[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int i = (j0 + j) * MK_THREADS + (int)threadIdx.x;
-                    v[j] = j0 + j < npass ? load_x(i) : z4;
-                    w4[j] = (ph.norm_w && j0 + j < npass && i < n4) ? __ldg((const float4*)ph.norm_w + i) : z4;
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) if (j0 + j < npass) quant_chunk((j0 + j) * MK_THREADS + (int)threadIdx.x, v[j], w4[j]);
-            }
-        }
+        mr_prologue<TYPE>(ph, k, nbp, (int*)s_q, s_d, s_s, s_red, (float4*)(smem + (size_t)nbp * 40 + 256 + 2048), comm, xseq);
     } else {   // stage the quantised activation (written by other CTAs in the previous phase: L2 loads)
         const uint8_t* act = (const uint8_t*)A.act;
         const int4* gq = (const int4*)act;
@@ -428,89 +445,68 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
     const int4* aq_l = (const int4*)s_q + lane;
     const float* ad_l = s_d + lane;
     const int* as_l = s_s + lane;
-    // Epilogues that need a value from memory (the residual, or the exp LUT entry of silu) are finished one round later (mega.cu); lane 0 only
-    float pend_a[2] = {0.0f, 0.0f}, pend_b[2] = {0.0f, 0.0f}, pend_res[2] = {0.0f, 0.0f};
-    unsigned short pend_lut[2] = {0, 0};
-    int pend_row[2] = {-1, -1};
+    // silu's exp LUT entry comes from memory: the row is finished one round later (lane 0)
+    float pend_a = 0.0f, pend_b = 0.0f;
+    unsigned short pend_lut = 0;
+    int pend_row = -1;
     auto flush_pending = [&]() {
-#pragma unroll
-        for (int t = 0; t < 2; t++) {
-            if (lane == 0 && pend_row[t] >= 0) {
-                if (pair) M.out[0][pend_row[t]] = (pend_a[t] / (1.0f + h2f_bits(pend_lut[t]))) * pend_b[t];
-                else M.out[0][pend_row[t]] = pend_a[t] + pend_res[t];
-            }
-            pend_row[t] = -1;
-        }
+        if (pend_row >= 0) M.out[0][pend_row] = (pend_a / (1.0f + h2f_bits(pend_lut))) * pend_b;      // silu(gate) * up
+        pend_row = -1;
     };
-    long long c_wait = 0, c_all = 0; int c_n = 0, c_fill = 0;  // developer profiling (CTA 0 / warp 0): cycles waiting for slots, cycles in the row loop, entries, ring fill
-    if (stamp1) c_all = clock64();
     const unsigned NS = (unsigned)RC.nslots;
-    // Pairs of units are dealt dynamically in ring order (the CTA's pair counter): no warp idles while another still has rows left, and the
-    // two rows of a pair share every activation load.  Which warp computes a row does not change its bits.
-    const int npairs = g.n_units >> 1, twoE = 2 * g.E;
-    for (;;) {
-        int P = 0;
-        if (lane == 0) P = atomicAdd(RC.s_unit, 1);
-        P = __shfl_sync(0xffffffffu, P, 0);
-        // pairs off: one unit per round, entries in plain (unit, virtual row, segment) order -- a slot is held for one row's arithmetic only
-        const bool two = RC.pairs && P < npairs;
-        if (RC.pairs ? (!two && !(P == npairs && (g.n_units & 1))) : P >= g.n_units) break;
-        const int u0 = !RC.pairs ? P : two ? 2 * P : g.n_units - 1;
-        const unsigned step = two ? 2u : 1u;
-        unsigned eA = RC.ent_base + (unsigned)(!RC.pairs ? P * g.E : two ? P * twoE : npairs * twoE);
-        unsigned slotA = eA % NS, parA = (eA / NS) & 1u;
-        float first[2] = {0.0f, 0.0f};
-        for (int v = 0; v < g.V; v++) {
-            float accA = 0.0f, accB = 0.0f;
-            for (int sg = 0; sg < NSEG; sg++) {
-                unsigned slotB = slotA + 1u, parB = parA;
-                if (slotB == NS) { slotB = 0; parB ^= 1u; }
-                long long t0 = 0;
-                if (stamp1) t0 = clock64();
-                mr_wait_full(RC, slotA, eA, parA);
-                if (two) mr_wait_full(RC, slotB, eA + 1u, parB);
-                if (stamp1) { c_wait += clock64() - t0; c_n += two ? 2 : 1; }
-                const uint8_t* spA = RC.ring + (size_t)slotA * RC.slot_bytes;
-                const uint8_t* spB = two ? RC.ring + (size_t)slotB * RC.slot_bytes : spA;
-                float partA, partB;
-                mr_dot2<TYPE>(spA, spB, sg, nb, GR, g.last_half_off, lane, aq_l, ad_l, as_l, partA, partB);
-                accA += partA; accB += partB;
-                __syncwarp();
-                if (lane == 0) { mr_release(RC.done0 + 4u * slotA, eA + 1u, partA); if (two) mr_release(RC.done0 + 4u * slotB, eA + 2u, partB); }
-                eA += step; slotA += step;
-                if (slotA >= NS) { slotA -= NS; parA ^= 1u; }
-            }
-            const float rA = warp_sum(accA), rB = warp_sum(accB);
-            if (pair && v == 0) { first[0] = rA; first[1] = rB; continue; }
-            if (pair || A.epilogue == 1) flush_pending();
+    constexpr unsigned DOFF = 2u * MK_SEG * (TYPE == CC_Q8_0 ? 1024u : 512u);
+    unsigned e = RC.ent_base + (unsigned)(warp * NSEG), slot = e % NS, par = (e / NS) & 1u;
+    for (int P = warp; P < g.groups; P += MK_WARPS) {
+        const bool half = lane >= 16;                          // lanes 0 .. 15 end up with the first row's sum, the others with the second's
+        const int rc = g.first + (pair ? P : 2 * P + (half ? 1 : 0));
+        const bool two = pair || 2 * P + 1 < g.n_rows;
+        const bool owner = (lane & 15) == 0 && (two || !half);
+        float res = 0.0f;
+        if (A.epilogue == 1 && owner) res = ldcg_f(A.residual + rc);              // + residual (llama2.rs:266,636)
+        float accA = 0.0f, accB = 0.0f;
+        for (int sg = 0; sg < NSEG; sg++) {
+            const int left = nb - sg * (MK_SEG * 32), nbe = min(MK_SEG * 32, left);
+            mr_wait_full(RC, slot, e, par);
+            const uint8_t* sp = RC.ring + (size_t)slot * RC.slot_bytes;
+            float partA, partB;
+            mr_dot2<TYPE>(sp, two ? (unsigned)nbe * (TYPE == CC_Q8_0 ? 32u : 16u) : 0u, sp + DOFF, two ? (unsigned)((nbe * 2 + 15) & ~15) : 0u, left, g.last_half_off, lane,
+                          aq_l + sg * (MK_SEG * 64), ad_l + sg * (MK_SEG * 32), as_l + sg * (MK_SEG * 32), partA, partB);
+            accA += partA; accB += partB;
+            __syncwarp();
+            if (lane == 0) mr_release(RC.done0 + 4u * slot, e + 1u, partA);
+            e++; slot++;
+            if (slot == NS) { slot = 0; par ^= 1u; }
+        }
+        e += (unsigned)((MK_WARPS - 1) * NSEG);
+        if (P + MK_WARPS < g.groups) { slot = e % NS; par = (e / NS) & 1u; }
+        // both rows in one butterfly (the same pairs of lanes are added as in warp_sum)
+        float r = half ? accB : accA;
+        r += __shfl_xor_sync(0xffffffffu, half ? accA : accB, 16);
 #pragma unroll
-            for (int t = 0; t < 2; t++) {
-                if (t == 1 && !two) break;
-                const float r = t ? rB : rA;
-                const int u = u0 + t, rc = g.first + u * g.stride;
-                if (lane != 0) continue;
-                if (pair) { pend_a[t] = first[t]; pend_b[t] = r; pend_row[t] = rc; pend_lut[t] = exp_lut[f2h_bits(-first[t])]; }      // silu(gate) * up
-                else if (A.epilogue == 1) { pend_a[t] = r; pend_row[t] = rc; pend_res[t] = ldcg_f(A.residual + rc); }              // + residual (llama2.rs:266,636)
-                else if (A.epilogue == 3) s_part[u] = r;                                                                            // partial row -> this CTA's exchange stage
-                else {
-                    int mat;
-                    const int rr = mr_locate(M, g, rc, 0, mat);
-                    float* o = mat == 0 ? M.out[0] : mat == 1 ? M.out[1] : M.out[2];
-                    o[rr] = r;
-                }
+        for (int o = 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        if (pair) {
+            const float up = __shfl_sync(0xffffffffu, r, 16);
+            if (lane == 0) { flush_pending(); pend_a = r; pend_b = up; pend_row = rc; pend_lut = exp_lut[f2h_bits(-r)]; }
+        } else if (owner) {
+            if (A.epilogue == 1) M.out[0][rc] = r + res;
+            else if (A.epilogue == 3) s_part[rc - g.first] = r;                    // partial row -> this CTA's exchange stage
+            else {
+                int mat;
+                const int rr = mr_locate(M, rc, mat);
+                float* o = mat == 0 ? M.out[0] : mat == 1 ? M.out[1] : M.out[2];
+                o[rr] = r;
             }
         }
     }
     flush_pending();
-    if (stamp1) { stamp1[5] = (unsigned long long)c_wait; stamp1[6] = ((unsigned long long)(clock64() - c_all) << 20) | ((unsigned long long)c_fill << 12) | (unsigned long long)c_n; }
-    RC.ent_base += (unsigned)(g.n_units * g.E);
+    RC.ent_base += (unsigned)(g.groups * NSEG);
     if (A.epilogue == 3) {
         // the CTA's block of partial rows -> slot[rank] of every GPU's exchange window: warp p serves peer p with coalesced 16-byte
         // NVLink stores (mega.cu)
         MK_SYNC();
         if (warp < comm.world) {
             const size_t off = ((size_t)((xseq + 1u) & 1u) * CC_COMM_MAX_RANKS + comm.rank) * CC_COMM_MAX_ELEMS + g.first;
-            for (int c4 = lane * 4; c4 < g.n_units; c4 += 128) *(float4*)(comm.data[warp] + off + c4) = *(const float4*)(s_part + c4);
+            for (int c4 = lane * 4; c4 < g.n_rows; c4 += 128) *(float4*)(comm.data[warp] + off + c4) = *(const float4*)(s_part + c4);
         }
     }
 }
@@ -518,7 +514,7 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
 template <bool GEN>
 __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase* __restrict__ phases, int n_phases, const uint8_t* dyn, unsigned* bar,
                                                                   const uint16_t* exp_lut, unsigned long long* prof, int flags, int wtop_off, unsigned* err_host,
-                                                                  const CommDev comm, const MrRing R) {
+                                                                  const __grid_constant__ CommDev comm, const __grid_constant__ MrRing R) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float s_red[MK_WARPS];
     __shared__ MkPhase s_phs[2];             // phase descriptors of the compute warps, double-buffered
@@ -526,11 +522,11 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
     __shared__ int s_abort;
     __shared__ int s_prod_done;
     __shared__ int s_ring_dead;
-    __shared__ int s_unit;                   // dynamic dealing of a phase's units to the consumer warps
+    __shared__ int s_issued;                 // items under way or landed since the launch began
     __shared__ __align__(8) unsigned long long s_abar[AT_NBUF];
     __shared__ __align__(8) unsigned long long s_full[MR_MAX_SLOTS];
-    __shared__ unsigned s_done[MR_MAX_SLOTS];     // entry number + 1 of the slot's last consumed tenant
-    __shared__ unsigned s_seq[MR_MAX_SLOTS];      // entry number + 1 of the slot's current tenant
+    __shared__ unsigned s_done[MR_MAX_SLOTS];     // item number + 1 of the slot's last consumed tenant
+    __shared__ unsigned s_seq[MR_MAX_SLOTS];      // item number + 1 of the slot's current tenant
     unsigned apar = 0u;
     const unsigned abar0 = (unsigned)__cvta_generic_to_shared(&s_abar[0]);
     const unsigned full0 = (unsigned)__cvta_generic_to_shared(&s_full[0]);
@@ -538,19 +534,19 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
     if (threadIdx.x == 0) {
         for (int i = 0; i < AT_NBUF; i++) mbar_init(abar0 + 8u * i, 1u);
         for (int i = 0; i < R.nslots; i++) { mbar_init(full0 + 8u * i, 1u); s_done[i] = 0u; s_seq[i] = 0u; }
-        s_abort = 0; s_prod_done = 0; s_ring_dead = 0;
+        s_abort = 0; s_prod_done = 0; s_ring_dead = 0; s_issued = 0;
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();                         // the only barrier all 640 threads share
     if (threadIdx.x >= MK_THREADS) {
-        mr_producer(phases, n_phases, R, full0, done0, (unsigned)__cvta_generic_to_shared(smem + R.ring_off), s_pd[(threadIdx.x - MK_THREADS) >> 5], s_seq, &s_abort, &s_prod_done,
-                    prof ? prof + (size_t)n_phases * MK_PROF_SLOTS : nullptr, (flags & MK_F_RPAIR) != 0, (flags & MK_F_KVPF) != 0, dyn);
+        mr_producer(phases, n_phases, R, full0, done0, (unsigned)__cvta_generic_to_shared(smem + R.ring_off), s_pd[(threadIdx.x - MK_THREADS) >> 5], s_seq, &s_abort, &s_ring_dead, &s_issued, &s_prod_done,
+                    (flags & MK_F_KVPF) != 0, dyn);
         return;
     }
     MrCons RC;
     RC.full0 = full0; RC.done0 = done0; RC.ring = smem + R.ring_off; RC.slot_bytes = R.slot_bytes; RC.nslots = R.nslots; RC.ent_base = 0u;
-    RC.pairs = (flags & MK_F_RPAIR) != 0; RC.s_unit = &s_unit; RC.s_seq = s_seq; RC.s_dead = &s_ring_dead; RC.err_dev = &bar[MK_BAR_ERR]; RC.err_host = err_host;
+    RC.s_seq = s_seq; RC.s_dead = &s_ring_dead; RC.err_dev = &bar[MK_BAR_ERR]; RC.err_host = err_host;
     AtPre at_pre = {0, 0, 0.0f, 0.0f};
     uint8_t* work = smem;
     float* s_w = (float*)(smem + wtop_off);  // generic phases: staging of the norm weights
@@ -621,7 +617,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
     // a launch that gave up: the producer stops at its next look at s_abort; bulk copies it has already issued must land before
     // the CTA's shared memory goes away
     MK_SYNC();
-    if (s_abort && threadIdx.x == 0) {
+    if ((s_abort || s_ring_dead) && threadIdx.x == 0) {
         at_drain(at_pre.jobs, abar0, apar);
         while (*(volatile int*)&s_prod_done < MR_PRODUCER_WARPS) {}
         for (unsigned sl = 0; sl < (unsigned)R.nslots; sl++) {               // every slot's latest tenant has landed
@@ -651,14 +647,14 @@ size_t cc_mega_ring_smem_for_phase(const MkPhase& ph) {
     if (ph.type == MK_MATVEC && ph.act_type == CC_Q8_K) return cc_mega_smem_for_phase(ph);
     if (ph.type == MK_MATVEC) {
         const size_t k = (size_t)ph.mv.k, nb = k / 32, GR = (nb + 31) / 32, NSEG = (GR + MK_SEG - 1) / MK_SEG, nbp = NSEG * MK_SEG * 32;
-        return nbp * 40 + 256 + 2048;
+        return nbp * 40 + 256 + 2048 + (ph.x ? (k < MR_ROW_PIECE ? k : MR_ROW_PIECE) * 4 * (ph.norm_w ? 2 : 1) : 0);
     }
     if (ph.type == MK_ATTN) return (size_t)(3 * ph.at.hd + ((ph.at.max_len + 8 + 3) & ~3)) * 4 + (size_t)AT_NBUF * cc_mega_ring_at_ch(ph) * ph.at.hd * (ph.at.kv_f16 ? 2 : 4) + 64;
     return 1024;
 }
 // slots the ring would get beside a working area of `smem_work` (+ `smem_wstage`) bytes; lazy.cu falls back to the register-pipe kernel
 // (mega.cu) below MR_MIN_SLOTS -- e.g. a 32 K-token context, whose attention phase needs 128 KB for the score row alone
-#define MR_MIN_SLOTS 12
+#define MR_MIN_SLOTS 6
 static size_t mr_ring_off(size_t smem_work, size_t smem_wstage) { return ((((smem_work + 15) & ~(size_t)15) + smem_wstage) + 127) & ~(size_t)127; }
 int cc_mega_ring_slots(size_t smem_work, size_t smem_wstage, int slot_bytes, bool generic) {
     cudaFuncAttributes fa;

@@ -1,18 +1,17 @@
-"""The ring order of mega_ring.cu, restated in Python: the producer warps enumerate a CTA's entries of a streaming MATVEC phase in one
-order (mr_producer), the consumer warps claim pairs of units and walk the same entries by index arithmetic (phase_matvec_ring).  Both
-sides must agree on which (unit, virtual row, segment) sits in entry e, every entry must be produced exactly once, and the two entries a
-pair round touches must be adjacent.  This test pins the arithmetic (a change on one side of the CUDA file has to be mirrored here and on
-the other side); the CUDA code itself is checked on the GPU by the bit-identity tests (tests/test_gpu_runner.py)."""
-import itertools
-
+"""The ring order of mega_ring.cu, restated in Python: the producer warps enumerate a CTA's items of a streaming MATVEC phase in one
+order (mr_item), the consumer warps take groups of two rows round-robin and walk the same items by index arithmetic (phase_matvec_ring).  Both
+sides must agree on which (group, segment) sits in item e, and every (unit, virtual row, segment) must be produced exactly once.  This test pins the
+arithmetic (a change on one side of the CUDA file has to be mirrored here and on the other side); the CUDA code itself is checked on the GPU by the
+bit-identity tests (tests/test_gpu_runner.py, tests/test_gpu_ring_rows.py)."""
 import pytest
 
 MK_SEG = 4
+WARPS = 16
 GRID = 148
 
 
 def geo(m, n_mats, k, epilogue, cta, grid=GRID):
-    """mr_geo: rows of the phase that belong to CTA `cta` as units (unit u -> concatenated row first + u * stride)."""
+    """mr_geo: rows of the phase that belong to CTA `cta`, one contiguous run; a group is a pair of rows or the gate and up row of one unit."""
     nb = k // 32
     gr = (nb + 31) // 32
     nseg = (gr + MK_SEG - 1) // MK_SEG
@@ -20,56 +19,43 @@ def geo(m, n_mats, k, epilogue, cta, grid=GRID):
     m_cat = m if pair else m * n_mats
     if epilogue == 3:
         rpc = ((m_cat + grid - 1) // grid + 3) & ~3
-        first, stride = cta * rpc, 1
-        n_units = min(rpc, max(0, m_cat - first))
+        first = cta * rpc
+        n_rows = min(rpc, max(0, m_cat - first))
     else:
-        first, stride = cta, grid
-        n_units = (m_cat - first + stride - 1) // stride if first < m_cat else 0
-    v = 2 if pair else 1
-    return dict(nb=nb, nseg=nseg, V=v, E=v * nseg, n_units=n_units, first=first, stride=stride)
+        each, more = divmod(m_cat, grid)
+        first = cta * each + min(cta, more)
+        n_rows = each + (1 if cta < more else 0)
+    return dict(nb=nb, nseg=nseg, V=2 if pair else 1, n_units=n_rows, first=first, stride=1, groups=n_rows if pair else (n_rows + 1) // 2)
 
 
-def producer_order(g, pairs):
-    """mr_producer: entry index j -> (unit, virtual row, segment)."""
-    n, e, two_e = g["n_units"] * g["E"], g["E"], 2 * g["E"]
-    npair = (g["n_units"] >> 1) * two_e
+def rows_of(g, P):
+    """the (unit, virtual row) pairs of group P"""
+    if g["V"] == 2:
+        return [(P, 0), (P, 1)]
+    return [(u, 0) for u in (2 * P, 2 * P + 1) if u < g["n_units"]]
+
+
+def producer_order(g):
+    """mr_item: item index j -> [(unit, virtual row, segment)] of its one or two rows."""
     out = []
-    for j in range(n):
-        if not pairs:
-            u, vs = divmod(j, e)
-        elif j < npair:
-            p, w = divmod(j, two_e)
-            u, vs = 2 * p + (w & 1), w >> 1
-        else:
-            u, vs = g["n_units"] - 1, j - npair
-        v, sg = divmod(vs, g["nseg"])
-        out.append((u, v, sg))
+    for j in range(g["groups"] * g["nseg"]):
+        P, sg = divmod(j, g["nseg"])
+        out.append([(u, v, sg) for u, v in rows_of(g, P)])
     return out
 
 
-def consumer_walk(g, pairs):
-    """phase_matvec_ring: for every claim P the list of (entry index, unit, virtual row, segment) it consumes, in order."""
-    e, two_e, npairs = g["E"], 2 * g["E"], g["n_units"] >> 1
-    claims = []
-    for p in itertools.count():
-        two = pairs and p < npairs
-        if pairs:
-            if not two and not (p == npairs and (g["n_units"] & 1)):
-                break
-        elif p >= g["n_units"]:
-            break
-        u0 = p if not pairs else (2 * p if two else g["n_units"] - 1)
-        step = 2 if two else 1
-        ea = (p * e) if not pairs else (p * two_e if two else npairs * two_e)
-        walk = []
-        for v in range(g["V"]):
+def consumer_walk(g):
+    """phase_matvec_ring: for every warp the list of (item index, [(unit, virtual row, segment)]) it consumes, in order."""
+    walks = []
+    for warp in range(WARPS):
+        walk, e = [], warp * g["nseg"]
+        for P in range(warp, g["groups"], WARPS):
             for sg in range(g["nseg"]):
-                walk.append((ea, u0, v, sg))
-                if two:
-                    walk.append((ea + 1, u0 + 1, v, sg))
-                ea += step
-        claims.append(walk)
-    return claims
+                walk.append((e, [(u, v, sg) for u, v in rows_of(g, P)]))
+                e += 1
+            e += (WARPS - 1) * g["nseg"]
+        walks.append(walk)
+    return walks
 
 
 SHAPES = [  # (rows per matrix, matrices, k, epilogue)
@@ -80,24 +66,21 @@ SHAPES = [  # (rows per matrix, matrices, k, epilogue)
 ]
 
 
-@pytest.mark.parametrize("pairs", [True, False])
 @pytest.mark.parametrize("m,n_mats,k,epilogue", SHAPES)
-def test_producer_and_consumers_agree_on_the_ring_order(m, n_mats, k, epilogue, pairs):
+def test_producer_and_consumers_agree_on_the_ring_order(m, n_mats, k, epilogue):
     covered_rows = set()
     for cta in (0, 1, 37, 146, 147):
         g = geo(m, n_mats, k, epilogue, cta)
-        order = producer_order(g, pairs)
+        order = producer_order(g)
         # every (unit, virtual row, segment) of the CTA exactly once
         want = {(u, v, s) for u in range(g["n_units"]) for v in range(g["V"]) for s in range(g["nseg"])}
-        assert len(order) == len(want) and set(order) == want
+        got = [x for item in order for x in item]
+        assert len(got) == len(want) and set(got) == want
         seen = []
-        for walk in consumer_walk(g, pairs):
-            for idx, (e, u, v, s) in enumerate(walk):
-                assert order[e] == (u, v, s), (cta, e, order[e], (u, v, s))
+        for walk in consumer_walk(g):
+            for e, rows in walk:
+                assert order[e] == rows, (cta, e, order[e], rows)
                 seen.append(e)
-            if pairs and len(walk) == 2 * g["E"]:                       # a pair round: its two entries of every step are adjacent in the ring
-                for a, b in zip(walk[0::2], walk[1::2]):
-                    assert b[0] == a[0] + 1
         assert sorted(seen) == list(range(len(order)))                # the consumers release every slot exactly once
         covered_rows.update(g["first"] + u * g["stride"] for u in range(g["n_units"]))
     assert covered_rows                                               # (the sampled CTAs own rows)

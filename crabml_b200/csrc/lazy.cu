@@ -40,12 +40,16 @@ struct LOp {
 // on every hit (a colliding key must re-capture, never replay another plan's baked pointers); `last_use` drives the LRU bound.
 struct GraphEntry { cudaGraphExec_t exec = nullptr; size_t dyn_bytes = 0; uint64_t launches = 0; MkPhase* phases_dev = nullptr;
                     std::vector<uint64_t> sig; uint64_t last_use = 0; int mega_variant = 0; };
-#define LZ_MAX_GRAPHS 128                            // cached token graphs per device: 64 token shapes (sequences with caches of their own) of two parts each
+#define LZ_MAX_GRAPHS 192                            // cached token graphs per device: 64 token shapes (sequences with caches of their own) of three parts each
+
+#define LZ_FIRST_OPS 64                              // the first part of a token: three layers, work for the GPU until the next part is recorded and fused
+#define LZ_PART_GROWTH 4                             // and each part so much longer than the one before: an op of a 7B layer keeps the GPU for 2.2 us and the host
+                                                     // for 0.5, so the 776 ops behind the first part (180 us of GPU) left the GPU idle for some 200 us a token
 
 struct LazyState {
     std::vector<LOp> q;
     std::unordered_map<cc_buf*, int> qrefs;
-#define LZ_DYN_SLOTS 16                              // the host may run eight tokens of two parts ahead of the GPU (absorbs host scheduling hiccups)
+#define LZ_DYN_SLOTS 24                              // the host may run eight tokens of three parts ahead of the GPU (absorbs host scheduling hiccups)
     uint8_t* dyn_host[LZ_DYN_SLOTS] = {nullptr};   // pinned, rotated so the host can build tokens t+1.. while t runs
     cudaEvent_t dyn_ev[LZ_DYN_SLOTS] = {nullptr};
     int dyn_slot = 0;
@@ -60,7 +64,7 @@ struct LazyState {
     uint64_t flushes = 0, graph_hits = 0, captures = 0, uncached = 0, evictions = 0, collisions = 0;
     uint64_t ns_record = 0, ns_fuse = 0, ns_submit = 0, n_ops = 0;      // host-side cost accounting
     int mega_variant = 0;            // persistent kernel of the last megakernel flush: 1 mega_kernel, 2 mega_ring_kernel
-    bool head_done = false;          // the token being recorded has started already
+    size_t part_ops = LZ_FIRST_OPS;  // queued ops from which the token being recorded starts, or goes on
 };
 
 static LView mkview(const cc_view* v) {
@@ -114,9 +118,6 @@ void cc_lazy_destroy(cc_device* dev) {
 }
 
 static int cc_lazy_flush_part(cc_device* dev, bool whole);
-#define LZ_HEAD_OPS 64                               // three layers: work for the GPU until the rest of a 7B token is recorded and fused.  16 tokens with 12 / 22 / 40 / 64 ops,
-                                                     // ms: 7B 41.2 / 40.6 / 40.5 / 39.8 (42.0 in one part), 15M 5.46 / 5.24 / 5.03 / 5.13 (5.93), four 7B layers of
-                                                     // K-quants 7.30 / 7.15 / 7.35 / 7.53 (7.97): a short token would go earlier, one count for all costs it 5 %
 static int64_t view_rows(const cc_view* v) { return v->ndim < 2 ? 1 : v->shape[0]; }
 
 // ---- recording ---------------------------------------------------------------------------------------------------
@@ -126,10 +127,10 @@ int cc_lazy_record(cc_device* dev, int kind, const cc_view* a, const cc_view* b,
                    const int64_t* rows, int n_rows) {
     LazyState* lz = dev->lz;
     // a long token starts while the rest of it is still being recorded: at the first copy of a layer's input (attention's or the feed-forward's) behind
-    // LZ_HEAD_OPS ops the queue so far runs, once per token -- the GPU used to wait some 180 us for the 840 ops of a 7B token.  No fused
-    // pattern spans that copy, so the phases are the same ones in two kernels.  Ranks that exchange keep one part: their launches stay paired.  So does a profiled token
-    if (kind == L_DUP && !lz->head_done && lz->q.size() >= LZ_HEAD_OPS && !cc_comm_dev(dev) && !lz->prof_dev && a && a->ndim <= 2 && view_rows(a) == 1) {
-        lz->head_done = true;
+    // part_ops ops the queue so far runs, and the next part may be longer.  No fused pattern spans that copy, so the phases are the same ones in several
+    // kernels.  Ranks that exchange keep one part: their launches stay paired.  So does a profiled token
+    if (kind == L_DUP && lz->q.size() >= lz->part_ops && !cc_comm_dev(dev) && !lz->prof_dev && a && a->ndim <= 2 && view_rows(a) == 1) {
+        lz->part_ops *= LZ_PART_GROWTH;
         int rc = cc_lazy_flush_part(dev, false);
         if (rc) return rc;
     }
@@ -699,7 +700,7 @@ struct Fuser {
 };
 
 int cc_lazy_flush(cc_device* dev) {
-    if (dev->lz) dev->lz->head_done = false;
+    if (dev->lz) dev->lz->part_ops = LZ_FIRST_OPS;
     return cc_lazy_flush_part(dev, true);
 }
 static int cc_lazy_flush_part(cc_device* dev, bool whole) {

@@ -9,13 +9,15 @@
 //     the per-phase working area (18 to 20 = 160-174 KB per SM, 25 MB per GPU).  They never wait for a barrier or an activation: whenever a slot is free the
 //     next item of this CTA's rows -- of this phase or any later one -- is being fetched.
 //   * warp 19 asks L2 for the items behind the ring, up to 224 KB of them per SM (33 MB per GPU), at 20 B per cycle and SM: a full ring is 4 us of HBM time, the
-//     time between one phase's last row and the next one's first 5 to 7 us, the attention phase 7.  A 7B Q8_0 token 2130 -> 1980 us (150, 224, 280, 330 KB and 16 to
-//     24 B the same within 1 %; 417 KB = 62 MB per GPU 2514: more than the L2 holds of it).  Without a pace the requests queue in front of the barrier's own
+//     time between one phase's last row and the next one's first 5 to 7 us, the attention phase 7.  A 7B Q8_0 token 1862 -> 1814 us (120 KB 1830; 224 and 300 KB, 20
+//     and 26 B alike; 417 KB = 62 MB per GPU was 30 % slower: more than L2 holds of it).  Without a pace the requests queue in front of the barrier's own
 //     traffic: with 19 MB under way a barrier takes 20 us instead of 2 (measured by itself; at 6.3 TB/s with 7 MB under way 3.4).
-//   * warps 0-15 are CONSUMERS: the CTA's rows are one contiguous run, pairs of rows dealt round-robin; same per-lane block order, same arithmetic as mega.cu /
-//     matvec_stream.cu (bit-identical results), but a segment is read from the ring with LDS.128 after waiting on the slot's "full" mbarrier, and the slot is
-//     handed back through its "done" word.  No weight registers live across phases, 96 registers are enough -- barely: a spilled register is a trip to L2 (the
-//     ring leaves no L1), and the same phases with the activation in registers, 600 bytes of spills, took 2540 us a token.
+//   * warps 0-15 are CONSUMERS: the CTA's rows are one contiguous run, two neighbouring rows an item, a warp each; same per-lane block order, same arithmetic as
+//     mega.cu / matvec_stream.cu (bit-identical results), but a segment is read from the ring with LDS.128 after waiting on the slot's "full" mbarrier, and
+//     the slot is handed back through its "done" words.  The activation stays in registers, lanes' sums are added up behind the row loop.  (One warp on both
+//     rows of an item, activation from shared memory: 16 of the 19 slots were being read and only the others under way, 1950 us a token; now 1814.)
+//     96 registers a thread are enough, but nothing may spill: a spilled register is a trip to L2, the ring leaves no L1 (the same rows with a prologue that
+//     kept its row in registers, 600 bytes of spills: 2540 us).
 // The 512 compute threads synchronise on named barrier 1 (MK_SYNC); the producer warps never join it.
 // 20 warps: five per SM sub-partition, so its 16384 registers allow 96 per thread (what __launch_bounds__(640, 1) yields).
 #define MK_SYNC() asm volatile("bar.sync 1, 512;" ::: "memory")
@@ -63,9 +65,10 @@ __device__ __forceinline__ unsigned mr_ld_acquire_shared(unsigned addr) {
     return v;
 }
 
-// Rows of a streaming MATVEC phase that belong to this CTA: one contiguous run.  They go through the ring as ITEMS of two virtual rows -- two rows next to
-// each other, or the gate and the up row of one unit -- and one segment of them; group (row pair) P is consumed by warp P % 16, segment after segment.
-// Producer and consumers derive the same item sequence from this: item of group P, segment s = P * NSEG + s.
+// Rows of a streaming MATVEC phase that belong to this CTA: one contiguous run.  They go through the ring as ITEMS: one segment of a GROUP, two rows next to each
+// other in one matrix (gate and up rows of two units are two groups, one behind the other).  Where a segment is a whole row the two lie in one run: two copies
+// an item, quants and scales -- the copy engine takes 30 M requests/s and SM, and a gate row beside an up row, four copies an item, was bound by that (10.3 us of
+// 75 items).  Producer and consumers derive the same item sequence from this: group P, segment s = item P * NSEG + s.
 struct MrGeo {
     int nb, GR, NSEG, n_rows, groups, first, last_half_off;
     bool pair;
@@ -85,10 +88,12 @@ __device__ __forceinline__ MrGeo mr_geo(const StreamArgs& A) {
         g.first = (int)blockIdx.x * each + min((int)blockIdx.x, more);
         g.n_rows = each + ((int)blockIdx.x < more ? 1 : 0);
     }
-    g.groups = g.pair ? g.n_rows : (g.n_rows + 1) >> 1;
+    g.groups = ((g.n_rows + 1) >> 1) << (g.pair ? 1 : 0);
     g.last_half_off = 16 * (g.nb - 32 * (g.GR - 1));
     return g;
 }
+// first row of a group, counted from the CTA's first
+__device__ __forceinline__ int mr_unit(const MrGeo& g, int P) { return g.pair ? P & ~1 : 2 * P; }
 // concatenated row -> (matrix, row of it)
 __device__ __forceinline__ int mr_locate(const StreamMats& M, int rc, int& mat) {
     mat = 0;
@@ -102,12 +107,10 @@ struct MrItem { const uint8_t* q[2]; const uint16_t* d[2]; unsigned qbytes, dbyt
 __device__ __forceinline__ MrItem mr_item(const StreamMats& M, const MrGeo& g, unsigned BB, int j) {
     MrItem it;
     const int P = j / g.NSEG, sg = j - P * g.NSEG;
-    int mat, matB = 1;
-    const int rA = mr_locate(M, g.first + (g.pair ? P : 2 * P), mat);
-    int rB = rA;
-    it.two = g.pair || 2 * P + 1 < g.n_rows;
-    if (!g.pair && it.two) rB = mr_locate(M, g.first + 2 * P + 1, matB);
-    if (!it.two) matB = mat;
+    const int u = mr_unit(g, P);
+    it.two = u + 1 < g.n_rows;
+    int mat = P & 1, matB = mat, rA = g.first + u, rB = rA + (it.two ? 1 : 0);
+    if (!g.pair) { const int rc = rA; rA = mr_locate(M, rc, mat); rB = mr_locate(M, rc + (it.two ? 1 : 0), matB); }
     const size_t at = (size_t)sg * (MK_SEG * 32), d_row = (size_t)CC_D_STRIDE(g.nb);
     const unsigned nbe = (unsigned)min(MK_SEG * 32, g.nb - MK_SEG * 32 * sg);
     it.qbytes = nbe * BB;
@@ -196,7 +199,7 @@ __device__ void mr_producer(const MkPhase* __restrict__ phases, int n_phases, co
                     e = ent + (unsigned)j; slot = e % (unsigned)R.nslots; use = e / (unsigned)R.nslots;
                     have = true;
                 }
-                if (!use || mr_ld_acquire_shared(done0 + 4u * slot) == e - (unsigned)R.nslots + 1u) {      // the slot's previous tenant has been consumed
+                if (!use || (mr_ld_acquire_shared(done0 + 8u * slot) == e - (unsigned)R.nslots + 1u && mr_ld_acquire_shared(done0 + 8u * slot + 4u) == e - (unsigned)R.nslots + 1u)) {      // the slot's previous tenant has been consumed
                     const unsigned fb = full0 + 8u * slot, dst = ring0 + slot * (unsigned)R.slot_bytes;
                     mr_expect_tx(fb, (im.qbytes + im.dbytes) << (im.two ? 1 : 0));
                     mr_bulk_g2s(dst, im.q[0], im.qbytes, fb);
@@ -258,50 +261,43 @@ __device__ __forceinline__ int mr_act_int4(int i) {           // i = 16-byte ind
     return (b >> 5) * 64 + (i & 1) * 32 + (b & 31);
 }
 
-// One segment (up to 4 groups of 32 blocks) of two rows against one activation: it is read once for both (shared-memory wavefronts per item: 68 to fill it, 72 for
-// the weights, 36 for the activation).  `left` = blocks of the row from this segment on: a lane behind them reads what the slot happens to hold (always
-// inside the slot) against zero quants and a scale it sets to zero.  Per row the arithmetic is mk_seg_dot's, term by term (bit-identical to matvec_stream.cu).
+// The activation of one segment in a lane's registers: its blocks of the four groups.  A warp keeps it for all rows of a phase, so an item costs the shared
+// memory 72 wavefronts to read and 68 to fill, and no more: the ring is consumed at shared-memory speed.
 template <int TYPE>
-__device__ __forceinline__ void mr_dot2(const uint8_t* sp, unsigned b_off, const uint8_t* dp, unsigned db_off, int left, int last_half_off, int lane,
-                                        const int4* aq, const float* ad, const int* as, float& partA, float& partB) {
-    constexpr int GB = TYPE == CC_Q8_0 ? 1024 : 512;
-    const uint8_t* qA = sp + lane * 16;
-    const uint16_t* dA = (const uint16_t*)dp + lane;
-    float accA = 0.0f, accB = 0.0f;
-    left -= lane;
+struct MrAct { int4 lo[MK_SEG], hi[MK_SEG]; float d[MK_SEG]; int s[TYPE == CC_Q4_0 ? MK_SEG : 1]; };
+template <int TYPE>
+__device__ __forceinline__ void mr_act_load(MrAct<TYPE>& a, int seg, const int4* aq_l, const float* ad_l, const int* as_l) {
 #pragma unroll
     for (int g = 0; g < MK_SEG; g++) {
-        const bool on = left > 0;
-        const uint16_t sA = on ? dA[0] : (uint16_t)0, sB = on ? dA[db_off >> 1] : (uint16_t)0;
-        const int4 alo = aq[0], ahi = aq[32];
-        const float adv = ad[0];
-        if constexpr (TYPE == CC_Q8_0) {
-            const int hoff = left + lane <= 32 ? last_half_off : 512;
-            const int4 a0 = *(const int4*)qA, a1 = *(const int4*)(qA + hoff);
-            const int4 b0 = *(const int4*)(qA + b_off), b1 = *(const int4*)(qA + b_off + hoff);
-            const int sumA = mk_dp16(a0, alo) + mk_dp16(a1, ahi);
-            const int sumB = mk_dp16(b0, alo) + mk_dp16(b1, ahi);
-            accA += (float)sumA * h2f_bits(sA) * adv;
-            accB += (float)sumB * h2f_bits(sB) * adv;
-        } else {
-            const int asv = as[0];
-            const int4 wA = *(const int4*)qA, wB = *(const int4*)(qA + b_off);
-            const int4 loA = make_int4(wA.x & 0x0F0F0F0F, wA.y & 0x0F0F0F0F, wA.z & 0x0F0F0F0F, wA.w & 0x0F0F0F0F);
-            const int4 hiA = make_int4((wA.x >> 4) & 0x0F0F0F0F, (wA.y >> 4) & 0x0F0F0F0F, (wA.z >> 4) & 0x0F0F0F0F, (wA.w >> 4) & 0x0F0F0F0F);
-            const int4 loB = make_int4(wB.x & 0x0F0F0F0F, wB.y & 0x0F0F0F0F, wB.z & 0x0F0F0F0F, wB.w & 0x0F0F0F0F);
-            const int4 hiB = make_int4((wB.x >> 4) & 0x0F0F0F0F, (wB.y >> 4) & 0x0F0F0F0F, (wB.z >> 4) & 0x0F0F0F0F, (wB.w >> 4) & 0x0F0F0F0F);
-            const int sumA = mk_dp16(loA, alo) + mk_dp16(hiA, ahi) - 8 * asv;
-            const int sumB = mk_dp16(loB, alo) + mk_dp16(hiB, ahi) - 8 * asv;
-            accA += (float)sumA * h2f_bits(sA) * adv;
-            accB += (float)sumB * h2f_bits(sB) * adv;
-            as += 32;
-        }
-        qA += GB; dA += 32; aq += 64; ad += 32; left -= 32;
+        const int gi = seg * MK_SEG + g;
+        a.lo[g] = aq_l[gi * 64]; a.hi[g] = aq_l[gi * 64 + 32]; a.d[g] = ad_l[gi * 32];
+        if constexpr (TYPE == CC_Q4_0) a.s[g] = as_l[gi * 32];
     }
-    partA = accA; partB = accB;
+}
+// One segment of one row.  `left` = blocks of the row from this segment on: a lane behind them reads what the slot happens to hold (always inside the slot)
+// against zero quants and a scale it sets to zero.  The arithmetic is mk_seg_dot's, term by term (bit-identical to matvec_stream.cu).
+template <int TYPE>
+__device__ __forceinline__ float mr_dot(const uint8_t* q, const uint16_t* d, int left, int last_half_off, int lane, const MrAct<TYPE>& act) {
+    constexpr int GB = TYPE == CC_Q8_0 ? 1024 : 512;
+    float acc = 0.0f;
+#pragma unroll
+    for (int g = 0; g < MK_SEG; g++) {
+        const int4 w = *(const int4*)(q + lane * 16 + g * GB);
+        const uint16_t s = g * 32 + lane < left ? d[g * 32 + lane] : (uint16_t)0;
+        int sum;
+        if constexpr (TYPE == CC_Q8_0) {
+            const int4 w1 = *(const int4*)(q + lane * 16 + g * GB + (left <= (g + 1) * 32 ? last_half_off : 512));
+            sum = mk_dp16(w, act.lo[g]) + mk_dp16(w1, act.hi[g]);
+        } else {
+            const int4 lo = make_int4(w.x & 0x0F0F0F0F, w.y & 0x0F0F0F0F, w.z & 0x0F0F0F0F, w.w & 0x0F0F0F0F);
+            const int4 hi = make_int4((w.x >> 4) & 0x0F0F0F0F, (w.y >> 4) & 0x0F0F0F0F, (w.z >> 4) & 0x0F0F0F0F, (w.w >> 4) & 0x0F0F0F0F);
+            sum = mk_dp16(lo, act.lo[g]) + mk_dp16(hi, act.hi[g]) - 8 * act.s[g];
+        }
+        acc += (float)sum * h2f_bits(s) * act.d[g];
+    }
+    return acc;
 }
 
-__device__ __forceinline__ bool mr_tiny(float x) { return fabsf(x) < 0x1p-60f && x != 0.0f; }
 // Fused prologue: [exchange reduction] + [rms_norm * w] + Q8_0 quantisation of x by EVERY CTA: thread t owns the float4 chunks t, t + 512, ... (the
 // canonical reduction order of common.cuh, and 8 consecutive threads = one 32-block).  All chunks of a thread are asked for at once, into shared memory, and the
 // loops over them are short: the phases of a layer do not stay in the near instruction caches, and the kernel's 96 registers have no room for a row (a spilled
@@ -355,30 +351,37 @@ __device__ __forceinline__ void mr_prologue(const MkPhase& ph, int k, int nbp, i
     const bool rms_ok = cc_quot_range(rms);
     int i0 = 0;
     if (!nw || n4 > piece) fetch(0);
+    // chunk i = 4 elements of block i >> 3.  512 chunks on are 64 blocks on: two groups of 32 in s_q32
+    int* out = s_q32 + mr_act_word(threadIdx.x);
 #pragma unroll 1
-    for (int i = threadIdx.x; i < nch; i += MK_THREADS) {               // chunk i = 4 elements of block i >> 3
+    for (int i = threadIdx.x; i < nch; i += MK_THREADS, out += 512) {
         if (i - i0 >= piece && i0 + piece < n4) { i0 += piece; fetch(i0); }             // (whole passes of 512 threads: all of them together)
         const bool live = i < n4;
+        if (!__any_sync(0xffffffffu, live)) {                           // behind the row: zeros (a segment is 128 blocks, a row of 288 has nine)
+            *out = 0;
+            if ((threadIdx.x & 7) == 0) { s_d[i >> 3] = 0.0f; if constexpr (TYPE == CC_Q4_0) s_s[i >> 3] = 0; }
+            continue;
+        }
         float4 v = live ? s_x[i - i0] : make_float4(0, 0, 0, 0);
         if (ph.orig && blockIdx.x == 0 && live) ((float4*)ph.orig)[i] = v;              // Tensor::dup of the un-normalised row (llama2.rs:227,607)
         const float4 x = v;
-        bool doubt = false;
+        bool sure = true;
         if (nw && live) {
             const float4 w = s_w[i - i0];
-            doubt = !rms_ok || mr_tiny(v.x) || mr_tiny(v.y) || mr_tiny(v.z) || mr_tiny(v.w);
+            sure = rms_ok && cc_quot_no_tiny(v.x, v.y, v.z, v.w);
             v = make_float4(cc_quot_by(v.x, rms, rr) * w.x, cc_quot_by(v.y, rms, rr) * w.y, cc_quot_by(v.z, rms, rr) * w.z, cc_quot_by(v.w, rms, rr) * w.w);
         }
         float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+        const float nan = (v.x + v.y) + (v.z + v.w);                    // (the maximum leaves one out; infinities are out of range)
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        if (!live) amax = 1.0f;                                         // (blocks behind the row: zeros)
-        doubt = doubt || !cc_quot_range(amax);
+        if (!live) amax = 1.0f;
+        sure = sure && cc_quot_range(amax) && nan == nan;
         float d = cc_q8_0_scale(amax), rcp;
-        const int top = cc_q8_0_top(amax, d);
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp) : "f"(d));        // within one unit in the last place
-        int q0 = cc_q8_0_quant(v.x, amax, top, rcp, doubt), q1 = cc_q8_0_quant(v.y, amax, top, rcp, doubt);
-        int q2 = cc_q8_0_quant(v.z, amax, top, rcp, doubt), q3 = cc_q8_0_quant(v.w, amax, top, rcp, doubt);
-        if (__any_sync(0xffffffffu, doubt)) {                           // rare: the whole warp's chunk with its divisions
+        const float half = 0.5f * d;
+        int q0 = cc_q8_0_quant(v.x, d, half, rcp), q1 = cc_q8_0_quant(v.y, d, half, rcp), q2 = cc_q8_0_quant(v.z, d, half, rcp), q3 = cc_q8_0_quant(v.w, d, half, rcp);
+        if (__any_sync(0xffffffffu, !sure)) {                           // rare: the whole warp's chunk with its divisions
             v = x;
             if (nw && live) { const float4 w = s_w[i - i0]; v = make_float4((v.x / rms) * w.x, (v.y / rms) * w.y, (v.z / rms) * w.z, (v.w / rms) * w.w); }
             amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
@@ -387,7 +390,7 @@ __device__ __forceinline__ void mr_prologue(const MkPhase& ph, int k, int nbp, i
             d = amax / 127.0f;
             q0 = live ? __float2int_rz(v.x / d) : 0; q1 = live ? __float2int_rz(v.y / d) : 0; q2 = live ? __float2int_rz(v.z / d) : 0; q3 = live ? __float2int_rz(v.w / d) : 0;
         }
-        s_q32[mr_act_word(i)] = (q0 & 255) | ((q1 & 255) << 8) | ((q2 & 255) << 16) | (q3 << 24);
+        *out = (int)__byte_perm(__byte_perm((unsigned)q0, (unsigned)q1, 0x0040), __byte_perm((unsigned)q2, (unsigned)q3, 0x0040), 0x5410);
         if constexpr (TYPE == CC_Q4_0) {
             int sq = q0 + q1 + q2 + q3;
 #pragma unroll
@@ -398,7 +401,15 @@ __device__ __forceinline__ void mr_prologue(const MkPhase& ph, int k, int nbp, i
     }
 }
 
-// shared memory of the phase: quants [nbp * 32] | f32 scales [nbp] | block sums [nbp] | reduction scratch 256 B | exchange stage 2 KB | fused prologue: the row and its norm weights
+// Lanes' sums are added up behind the row loop, all rows of the CTA at once, where they find room in shared memory.  One segment: a thread adds up a row's 32
+// (the butterfly took 320 of 1350 cycles a row).  Two to four segments (k <= 16384): warps keep to one segment, so that its activation stays in registers, and a
+// warp adds up a row's.  Else a warp takes a row's segments one after another, reads the activation for each and adds up itself.
+#define MR_PART_BYTES 30720
+__host__ __device__ __forceinline__ int mr_part_bytes(int nseg, int vrows) {
+    const int n = nseg == 1 ? vrows * 132 : nseg <= 4 ? vrows * nseg * 128 : 0;
+    return n <= MR_PART_BYTES ? n : 0;
+}
+// shared memory of the phase: quants [nbp * 32] | f32 scales [nbp] | block sums [nbp] | reduction scratch 256 B | sums of the CTA's virtual rows | lanes' sums | fused prologue (over the sums): the row and its norm weights
 template <int TYPE>
 __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16_t* exp_lut, MrCons& RC, const CommDev& comm, unsigned xseq, unsigned long long* stamp1) {
     const StreamArgs& A = ph.mv;
@@ -411,11 +422,13 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
     float* s_d = (float*)(smem + (size_t)nbp * 32);
     int* s_s = (int*)(smem + (size_t)nbp * 32 + (size_t)nbp * 4);
     float* s_red = (float*)(smem + (size_t)nbp * 40);
-    float* s_part = (float*)(smem + (size_t)nbp * 40 + 256);
+    float* s_sum = (float*)(smem + (size_t)nbp * 40 + 256);
+    const int vrows = pair ? 2 * g.n_rows : g.n_rows;
+    float* s_part = s_sum + ((vrows + 31) & ~31);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const StreamMats& M = A.mats;
     if (ph.x) {
-        mr_prologue<TYPE>(ph, k, nbp, (int*)s_q, s_d, s_s, s_red, (float4*)(smem + (size_t)nbp * 40 + 256 + 2048), comm, xseq);
+        mr_prologue<TYPE>(ph, k, nbp, (int*)s_q, s_d, s_s, s_red, (float4*)s_sum, comm, xseq);
     } else {   // stage the quantised activation (written by other CTAs in the previous phase: L2 loads)
         const uint8_t* act = (const uint8_t*)A.act;
         const int4* gq = (const int4*)act;
@@ -445,68 +458,94 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
     const int4* aq_l = (const int4*)s_q + lane;
     const float* ad_l = s_d + lane;
     const int* as_l = s_s + lane;
-    // silu's exp LUT entry comes from memory: the row is finished one round later (lane 0)
-    float pend_a = 0.0f, pend_b = 0.0f;
-    unsigned short pend_lut = 0;
-    int pend_row = -1;
-    auto flush_pending = [&]() {
-        if (pend_row >= 0) M.out[0][pend_row] = (pend_a / (1.0f + h2f_bits(pend_lut))) * pend_b;      // silu(gate) * up
-        pend_row = -1;
-    };
-    const unsigned NS = (unsigned)RC.nslots;
+    // Warps 2 i and 2 i + 1 take the two rows of an item.  One warp on both rows held sixteen of the twenty slots at a time, so few copies were under way
+    const int duo = warp >> 1, half = warp & 1;
+    const bool parts = mr_part_bytes(NSEG, vrows) > 0, split = parts && NSEG > 1;
+    const int s0 = split ? duo % NSEG : 0, ns = split ? 1 : NSEG;
+    const int P0 = split ? duo / NSEG : duo, dP = split ? (MK_WARPS / 2 - s0 + NSEG - 1) / NSEG : MK_WARPS / 2;
     constexpr unsigned DOFF = 2u * MK_SEG * (TYPE == CC_Q8_0 ? 1024u : 512u);
-    unsigned e = RC.ent_base + (unsigned)(warp * NSEG), slot = e % NS, par = (e / NS) & 1u;
-    for (int P = warp; P < g.groups; P += MK_WARPS) {
-        const bool half = lane >= 16;                          // lanes 0 .. 15 end up with the first row's sum, the others with the second's
-        const int rc = g.first + (pair ? P : 2 * P + (half ? 1 : 0));
-        const bool two = pair || 2 * P + 1 < g.n_rows;
-        const bool owner = (lane & 15) == 0 && (two || !half);
-        float res = 0.0f;
-        if (A.epilogue == 1 && owner) res = ldcg_f(A.residual + rc);              // + residual (llama2.rs:266,636)
-        float accA = 0.0f, accB = 0.0f;
-        for (int sg = 0; sg < NSEG; sg++) {
+    const unsigned NS = (unsigned)RC.nslots;
+    MrAct<TYPE> act;
+    mr_act_load<TYPE>(act, s0, aq_l, ad_l, as_l);
+    unsigned e = RC.ent_base + (unsigned)(P0 * NSEG + s0), slot = e % NS, par = (e / NS) & 1u;
+    for (int P = P0; P < g.groups; P += dP) {
+        const int u = mr_unit(g, P) + half, v = pair ? 2 * u + (P & 1) : u;
+        const bool row = u < g.n_rows;
+        float acc = 0.0f;
+        for (int s = 0; s < ns; s++) {
+            const int sg = s0 + s;
+            if (ns > 1) mr_act_load<TYPE>(act, sg, aq_l, ad_l, as_l);
             const int left = nb - sg * (MK_SEG * 32), nbe = min(MK_SEG * 32, left);
             mr_wait_full(RC, slot, e, par);
-            const uint8_t* sp = RC.ring + (size_t)slot * RC.slot_bytes;
-            float partA, partB;
-            mr_dot2<TYPE>(sp, two ? (unsigned)nbe * (TYPE == CC_Q8_0 ? 32u : 16u) : 0u, sp + DOFF, two ? (unsigned)((nbe * 2 + 15) & ~15) : 0u, left, g.last_half_off, lane,
-                          aq_l + sg * (MK_SEG * 64), ad_l + sg * (MK_SEG * 32), as_l + sg * (MK_SEG * 32), partA, partB);
-            accA += partA; accB += partB;
-            __syncwarp();
-            if (lane == 0) mr_release(RC.done0 + 4u * slot, e + 1u, partA);
-            e++; slot++;
-            if (slot == NS) { slot = 0; par ^= 1u; }
-        }
-        e += (unsigned)((MK_WARPS - 1) * NSEG);
-        if (P + MK_WARPS < g.groups) { slot = e % NS; par = (e / NS) & 1u; }
-        // both rows in one butterfly (the same pairs of lanes are added as in warp_sum)
-        float r = half ? accB : accA;
-        r += __shfl_xor_sync(0xffffffffu, half ? accA : accB, 16);
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-        if (pair) {
-            const float up = __shfl_sync(0xffffffffu, r, 16);
-            if (lane == 0) { flush_pending(); pend_a = r; pend_b = up; pend_row = rc; pend_lut = exp_lut[f2h_bits(-r)]; }
-        } else if (owner) {
-            if (A.epilogue == 1) M.out[0][rc] = r + res;
-            else if (A.epilogue == 3) s_part[rc - g.first] = r;                    // partial row -> this CTA's exchange stage
-            else {
-                int mat;
-                const int rr = mr_locate(M, rc, mat);
-                float* o = mat == 0 ? M.out[0] : mat == 1 ? M.out[1] : M.out[2];
-                o[rr] = r;
+            float part = 0.0f;
+            if (row) {
+                const uint8_t* sp = RC.ring + (size_t)slot * RC.slot_bytes;
+                part = mr_dot<TYPE>(sp + (half ? (unsigned)nbe * (TYPE == CC_Q8_0 ? 32u : 16u) : 0u), (const uint16_t*)(sp + DOFF + (half ? (unsigned)((nbe * 2 + 15) & ~15) : 0u)), left,
+                                    g.last_half_off, lane, act);
             }
+            acc += part;
+            __syncwarp();
+            if (lane == 0) mr_release(RC.done0 + 8u * slot + 4u * (unsigned)half, e + 1u, part);
+            const unsigned step = s + 1 < ns ? 1u : (unsigned)((dP - 1) * NSEG) + (split ? (unsigned)NSEG : 1u);
+            e += step; slot += step;
+            while (slot >= NS) { slot -= NS; par ^= 1u; }
+        }
+        if (!row) continue;
+        if (split) s_part[(v * NSEG + s0) * 32 + lane] = acc;
+        else if (parts) s_part[v * 33 + lane] = acc;
+        else { const float r = warp_sum(acc); if (lane == 0) s_sum[v] = r; }
+    }
+    RC.ent_base += (unsigned)(g.groups * NSEG);
+    float res = 0.0f;                                                  // + residual (llama2.rs:266,636)
+    if (A.epilogue == 1 && (int)threadIdx.x < g.n_rows) res = ldcg_f(A.residual + g.first + threadIdx.x);
+    MK_SYNC();
+    if (split) {                                                       // a row's segments in their order, then the butterfly
+        for (int v = warp; v < vrows; v += MK_WARPS) {
+            float acc = 0.0f;
+            for (int s = 0; s < NSEG; s++) acc += s_part[((size_t)v * NSEG + s) * 32 + lane];
+            const float r = warp_sum(acc);
+            if (lane == 0) s_sum[v] = r;
+        }
+        MK_SYNC();
+    }
+    // a row per thread, neighbouring rows side by side in memory; gate and up of a unit on neighbouring threads
+    for (int v = threadIdx.x; v - lane < vrows; v += MK_THREADS) {
+        float r = 0.0f;
+        if (v < vrows) {
+            if (parts && !split) {                                     // the butterfly's sum, its pairs in its order (stride 33: no bank conflicts)
+                const float* p = s_part + v * 33;
+                float t[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) t[i] = p[i] + p[i + 16];
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < o; i++) t[i] += t[i + o];
+                r = t[0];
+            } else r = s_sum[v];
+        }
+        const float up = __shfl_down_sync(0xffffffffu, r, 1);
+        if (v >= vrows) continue;
+        if (pair) {                                                    // silu(gate) * up
+            if (!(v & 1)) M.out[0][g.first + (v >> 1)] = (r / (1.0f + h2f_bits(exp_lut[f2h_bits(-r)]))) * up;
+        } else if (A.epilogue == 1) {
+            if (v >= MK_THREADS) res = ldcg_f(A.residual + g.first + v);
+            M.out[0][g.first + v] = r + res;
+        } else if (A.epilogue == 3) s_sum[v] = r;
+        else {
+            int mat;
+            const int rr = mr_locate(M, g.first + v, mat);
+            float* o = mat == 0 ? M.out[0] : mat == 1 ? M.out[1] : M.out[2];
+            o[rr] = r;
         }
     }
-    flush_pending();
-    RC.ent_base += (unsigned)(g.groups * NSEG);
     if (A.epilogue == 3) {
         // the CTA's block of partial rows -> slot[rank] of every GPU's exchange window: warp p serves peer p with coalesced 16-byte
         // NVLink stores (mega.cu)
         MK_SYNC();
         if (warp < comm.world) {
             const size_t off = ((size_t)((xseq + 1u) & 1u) * CC_COMM_MAX_RANKS + comm.rank) * CC_COMM_MAX_ELEMS + g.first;
-            for (int c4 = lane * 4; c4 < g.n_rows; c4 += 128) *(float4*)(comm.data[warp] + off + c4) = *(const float4*)(s_part + c4);
+            for (int c4 = lane * 4; c4 < g.n_rows; c4 += 128) *(float4*)(comm.data[warp] + off + c4) = *(const float4*)(s_sum + c4);
         }
     }
 }
@@ -525,7 +564,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
     __shared__ int s_issued;                 // items under way or landed since the launch began
     __shared__ __align__(8) unsigned long long s_abar[AT_NBUF];
     __shared__ __align__(8) unsigned long long s_full[MR_MAX_SLOTS];
-    __shared__ unsigned s_done[MR_MAX_SLOTS];     // item number + 1 of the slot's last consumed tenant
+    __shared__ unsigned s_done[2 * MR_MAX_SLOTS]; // item number + 1 of the slot's last consumed tenant, a word per row
     __shared__ unsigned s_seq[MR_MAX_SLOTS];      // item number + 1 of the slot's current tenant
     unsigned apar = 0u;
     const unsigned abar0 = (unsigned)__cvta_generic_to_shared(&s_abar[0]);
@@ -533,7 +572,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) mega_ring_kernel(const MkPhase*
     const unsigned done0 = (unsigned)__cvta_generic_to_shared(&s_done[0]);
     if (threadIdx.x == 0) {
         for (int i = 0; i < AT_NBUF; i++) mbar_init(abar0 + 8u * i, 1u);
-        for (int i = 0; i < R.nslots; i++) { mbar_init(full0 + 8u * i, 1u); s_done[i] = 0u; s_seq[i] = 0u; }
+        for (int i = 0; i < R.nslots; i++) { mbar_init(full0 + 8u * i, 1u); s_done[2 * i] = 0u; s_done[2 * i + 1] = 0u; s_seq[i] = 0u; }
         s_abort = 0; s_prod_done = 0; s_ring_dead = 0; s_issued = 0;
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -643,11 +682,15 @@ int cc_mega_ring_at_ch(const MkPhase& ph) {       // 48 KB of cache rows in flig
     if (env >= 8 && env <= 64) return env;
     return ph.at.kv_f16 ? 64 : 32;
 }
-size_t cc_mega_ring_smem_for_phase(const MkPhase& ph) {
+size_t cc_mega_ring_smem_for_phase(const MkPhase& ph, int ctas) {
     if (ph.type == MK_MATVEC && ph.act_type == CC_Q8_K) return cc_mega_smem_for_phase(ph);
     if (ph.type == MK_MATVEC) {
         const size_t k = (size_t)ph.mv.k, nb = k / 32, GR = (nb + 31) / 32, NSEG = (GR + MK_SEG - 1) / MK_SEG, nbp = NSEG * MK_SEG * 32;
-        return nbp * 40 + 256 + 2048 + (ph.x ? (k < MR_ROW_PIECE ? k : MR_ROW_PIECE) * 4 * (ph.norm_w ? 2 : 1) : 0);
+        const size_t m = ph.mv.epilogue == 2 ? (size_t)ph.mv.mats.m[0] : (size_t)ph.mv.mats.m[0] + (ph.mv.mats.n > 1 ? ph.mv.mats.m[1] : 0) + (ph.mv.mats.n > 2 ? ph.mv.mats.m[2] : 0);
+        const size_t rows = ((m + (size_t)ctas - 1) / (size_t)ctas + 3) & ~(size_t)3, vrows = ph.mv.epilogue == 2 ? 2 * rows : rows;
+        const size_t sums = ((vrows + 31) & ~(size_t)31) * 4 + (size_t)mr_part_bytes((int)NSEG, (int)vrows);
+        const size_t row = ph.x ? (k < MR_ROW_PIECE ? k : MR_ROW_PIECE) * 4 * (ph.norm_w ? 2 : 1) : 0;
+        return nbp * 40 + 256 + (sums > row ? sums : row);
     }
     if (ph.type == MK_ATTN) return (size_t)(3 * ph.at.hd + ((ph.at.max_len + 8 + 3) & ~3)) * 4 + (size_t)AT_NBUF * cc_mega_ring_at_ch(ph) * ph.at.hd * (ph.at.kv_f16 ? 2 : 4) + 64;
     return 1024;

@@ -4,11 +4,13 @@
 //   * a quotient by a divisor b that many numbers share: r = RN(1 / b) once, then two corrections q + (x - q b) r with fused multiply-adds.  The second starts
 //     from a quotient within one unit in the last place, so it rounds correctly (P. Markstein, "Computation of elementary functions on the IBM RISC
 //     System/6000 processor", 1990), as long as nothing underflows or overflows: cc_quot_range.
-//   * trunc(RN(v / d)): with any reciprocal within two units, v * rcp is within 127 * 2^-22 of the quotient, so its truncation is right unless a whole number lies
-//     that close; then (and for the block's own maximum, whose quotient is 127 within a unit) the truth is worked out.
+//   * trunc(RN(v / d)) for |v / d| <= 128: m = the whole number nearest to |v| * rcp, for a reciprocal within a few units; the remainder |v| - m d is exact (a
+//     multiple of d's unit, small), and the rounded quotient reaches m if it is not below m by more than half a unit of the floats under m (a tie rounds to
+//     m, whose mantissa is even).  Else the answer is m - 1.
 // Plain C++ beside CUDA: the CPU test compiles this file.
 #pragma once
 #include <math.h>
+#include <string.h>
 
 #ifdef __CUDACC__
 #define CC_QUOT_FN __host__ __device__ __forceinline__
@@ -23,19 +25,36 @@ CC_QUOT_FN float cc_quot_by(float x, float b, float r /* RN(1 / b) */) {
     q = fmaf(fmaf(-b, q, x), r, q);
     return fmaf(fmaf(-b, q, x), r, q);
 }
-// d of a block, and the quant of its largest magnitude: amax / d is 127 or less than it by more than half of its unit 2^-17 (then 126)
-CC_QUOT_FN float cc_q8_0_scale(float amax) { return cc_quot_by(amax, 127.0f, 1.0f / 127.0f); }
-CC_QUOT_FN int cc_q8_0_top(float amax, float d) { return fmaf(d, 127.0f, -amax) > d * 0x1p-18f ? 126 : 127; }
-// quant of v by a reciprocal of d; `doubt` is raised when a whole number is too close to tell
-CC_QUOT_FN int cc_q8_0_quant(float v, float amax, int top, float rcp, bool& doubt) {
-    const float t = v * rcp;
-    const float whole = (t + 12582912.0f) - 12582912.0f;          // nearest whole number (|t| < 128)
-    const bool is_top = fabsf(v) == amax;
-    if (fabsf(t - whole) < 0x1p-14f && whole != 0.0f && !is_top) doubt = true;
+CC_QUOT_FN float cc_quot_float(int b) {
 #ifdef __CUDA_ARCH__
-    const int q = __float2int_rz(t);
+    return __int_as_float(b);
 #else
-    const int q = t == t ? (int)t : 0;
+    float f; memcpy(&f, &b, 4); return f;
 #endif
-    return is_top ? (v < 0.0f ? -top : top) : q;
+}
+CC_QUOT_FN int cc_quot_bits(float f) {
+#ifdef __CUDA_ARCH__
+    return __float_as_int(f);
+#else
+    int b; memcpy(&b, &f, 4); return b;
+#endif
+}
+// no non-zero number of the four below 2^-60 (doubled bits less one: zero becomes the largest)
+CC_QUOT_FN bool cc_quot_no_tiny(float x, float y, float z, float w) {
+    const unsigned a = ((unsigned)cc_quot_bits(x) << 1) - 1u, b = ((unsigned)cc_quot_bits(y) << 1) - 1u, c = ((unsigned)cc_quot_bits(z) << 1) - 1u, d = ((unsigned)cc_quot_bits(w) << 1) - 1u;
+    const unsigned ab = a < b ? a : b, cd = c < d ? c : d;
+    return (ab < cd ? ab : cd) >= (((127u - 60u) << 24) - 1u);
+}
+// d of a block
+CC_QUOT_FN float cc_q8_0_scale(float amax) { return cc_quot_by(amax, 127.0f, 1.0f / 127.0f); }
+// quant of v by d = RN(amax / 127), half = d / 2 and a reciprocal of d.  No number at all (NaN): 0, as the conversion of one
+CC_QUOT_FN int cc_q8_0_quant(float v, float d, float half, float rcp) {
+    const float a = fabsf(v);
+    const float sh = a * rcp + 12582912.0f;                          // 1.5 * 2^23: the nearest whole number in the low bits
+    const float m = sh - 12582912.0f;
+    const float below = (cc_quot_float(cc_quot_bits(m) - 1) - m) * half;            // minus half a unit under m, times d (m = 0: NaN, nothing is below)
+    int q = cc_quot_bits(sh) - 0x4B400000;
+    if (fmaf(-m, d, a) < below) q--;
+    const int sign = cc_quot_bits(v) >> 31;
+    return (q ^ sign) - sign;
 }

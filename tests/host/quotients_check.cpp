@@ -11,12 +11,12 @@ static float from_bits(uint32_t u) { float f; memcpy(&f, &u, 4); return f; }
 static uint32_t bits(float f) { uint32_t u; memcpy(&u, &f, 4); return u; }
 
 int main() {
-    long bad_scale = 0, bad_top = 0, bad_by = 0, bad_quant = 0, doubts = 0, n_quant = 0;
-    for (uint32_t m = 0; m < (1u << 23); m++)                                        // every mantissa, several exponents: the scale and the largest quant
+    long bad_scale = 0, bad_by = 0, bad_quant = 0, n_quant = 0, bad_tiny = 0;
+    for (uint32_t m = 0; m < (1u << 23); m++)                                        // every mantissa, several exponents: the scale and the quant of the largest number
         for (uint32_t e : {68u, 127u, 128u, 186u}) {
             const float a = from_bits(e << 23 | m), d = a / 127.0f;
             if (bits(cc_q8_0_scale(a)) != bits(d)) bad_scale++;
-            if (cc_q8_0_top(a, d) != (int)(a / d)) bad_top++;
+            if (cc_q8_0_quant(e & 1 ? a : -a, d, 0.5f * d, 1.0f / d) != (e & 1 ? 1 : -1) * (int)(a / d)) bad_quant++;
         }
     std::mt19937 g(7);
     auto value = [&](int lo, int hi) { return from_bits((uint32_t)(127 + lo + (int)(g() % (uint32_t)(hi - lo))) << 23 | (g() & 0x7FFFFF) | (g() & 1u) << 31); };
@@ -36,15 +36,15 @@ int main() {
             if (i % 2) v = from_bits(bits(d * (float)(g() % 127 + 1)) + (g() % 9) - 4) * (g() & 1 ? 1.0f : -1.0f);
             if (i % 5 == 0) v = wobble & 1 ? amax : -amax;
             if (std::fabs(v) > amax) continue;
-            bool doubt = false;
-            const int q = cc_q8_0_quant(v, amax, cc_q8_0_top(amax, d), rcp, doubt);
             n_quant++;
-            if (doubt) doubts++;
-            else if (q != (int)(v / d)) bad_quant++;
+            if (cc_q8_0_quant(v, d, 0.5f * d, rcp) != (int)(v / d)) bad_quant++;
         }
     }
-    bool doubt = false;
-    const int nan_q = cc_q8_0_quant(NAN, 1.0f, 127, 127.0f, doubt);
-    printf("%ld %ld %ld %ld %ld %ld %d\n", bad_scale, bad_top, bad_by, bad_quant, doubts, n_quant, nan_q || doubt);
+    for (long i = 0; i < 1000000; i++) {
+        float x[4]; bool tiny = false;
+        for (float& f : x) { f = g() % 5 ? value(-64, -56) : 0.0f * (float)((int)(g() % 3) - 1); tiny = tiny || (f != 0.0f && std::fabs(f) < 0x1p-60f); }
+        if (cc_quot_no_tiny(x[0], x[1], x[2], x[3]) == tiny) bad_tiny++;
+    }
+    printf("%ld %ld %ld %ld %ld\n", bad_scale, bad_by, bad_quant, bad_tiny, n_quant);
     return 0;
 }

@@ -11,7 +11,7 @@ GRID = 148
 
 
 def geo(m, n_mats, k, epilogue, cta, grid=GRID):
-    """mr_geo: rows of the phase that belong to CTA `cta`, one contiguous run; a group is a pair of rows or the gate and up row of one unit."""
+    """mr_geo: rows of the phase that belong to CTA `cta`, one contiguous run; a group is two neighbouring rows of one matrix (gate and up: in turn)."""
     nb = k // 32
     gr = (nb + 31) // 32
     nseg = (gr + MK_SEG - 1) // MK_SEG
@@ -25,14 +25,13 @@ def geo(m, n_mats, k, epilogue, cta, grid=GRID):
         each, more = divmod(m_cat, grid)
         first = cta * each + min(cta, more)
         n_rows = each + (1 if cta < more else 0)
-    return dict(nb=nb, nseg=nseg, V=2 if pair else 1, n_units=n_rows, first=first, stride=1, groups=n_rows if pair else (n_rows + 1) // 2)
+    return dict(nb=nb, nseg=nseg, V=2 if pair else 1, n_units=n_rows, first=first, stride=1, groups=(n_rows + 1) // 2 * (2 if pair else 1))
 
 
 def rows_of(g, P):
     """the (unit, virtual row) pairs of group P"""
-    if g["V"] == 2:
-        return [(P, 0), (P, 1)]
-    return [(u, 0) for u in (2 * P, 2 * P + 1) if u < g["n_units"]]
+    u, v = (P & ~1, P & 1) if g["V"] == 2 else (2 * P, 0)
+    return [(x, v) for x in (u, u + 1) if x < g["n_units"]]
 
 
 def producer_order(g):
@@ -45,15 +44,19 @@ def producer_order(g):
 
 
 def consumer_walk(g):
-    """phase_matvec_ring: for every warp the list of (item index, [(unit, virtual row, segment)]) it consumes, in order."""
-    walks = []
-    for warp in range(WARPS):
-        walk, e = [], warp * g["nseg"]
-        for P in range(warp, g["groups"], WARPS):
-            for sg in range(g["nseg"]):
-                walk.append((e, [(u, v, sg) for u, v in rows_of(g, P)]))
-                e += 1
-            e += (WARPS - 1) * g["nseg"]
+    """phase_matvec_ring: for every pair of warps the list of (item index, [(unit, virtual row, segment)]) it consumes, in order."""
+    walks, nseg, duos = [], g["nseg"], WARPS // 2
+    vrows = g["n_units"] * g["V"]
+    part_bytes = vrows * 132 if nseg == 1 else vrows * nseg * 128 if nseg <= 4 else 0
+    split = nseg > 1 and 0 < part_bytes <= 30720                       # warps keep to one segment
+    for duo in range(duos):
+        s0, ns = (duo % nseg, 1) if split else (0, nseg)
+        p0, dp = (duo // nseg, (duos - s0 + nseg - 1) // nseg) if split else (duo, duos)
+        walk, e = [], p0 * nseg + s0
+        for P in range(p0, g["groups"], dp):
+            for s in range(ns):
+                walk.append((e, [(u, v, s0 + s) for u, v in rows_of(g, P)]))
+                e += 1 if s + 1 < ns else (dp - 1) * nseg + (nseg if split else 1)
         walks.append(walk)
     return walks
 
@@ -62,6 +65,7 @@ SHAPES = [  # (rows per matrix, matrices, k, epilogue)
     (4096, 3, 4096, 0), (4096, 1, 4096, 1), (11008, 2, 4096, 2), (4096, 1, 11008, 1), (32000, 1, 4096, 0),      # Llama-2-7B, one GPU
     (4096, 1, 2048, 3), (4096, 1, 5504, 3), (16000, 1, 4096, 3),                                                    # shards at N = 2 (exchange phases)
     (512, 3, 4096, 0), (4096, 1, 512, 3), (1376, 2, 4096, 2), (4096, 1, 1376, 3), (4000, 1, 4096, 3),               # shards at N = 8
+    (4096, 1, 14336, 1), (8192, 1, 28672, 1), (256000, 1, 8192, 0),                                               # four segments, seven, and more rows than their sums find room for
     (288, 3, 288, 0), (288, 1, 288, 1), (768, 2, 288, 2), (288, 1, 768, 1), (32000, 1, 288, 0),                     # tinyllamas-15M (ragged groups)
 ]
 

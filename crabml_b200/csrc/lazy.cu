@@ -324,6 +324,12 @@ struct Fuser {
         P.S(0x2001); P.SP(x); P.SP(og); P.SP(w); P.SP(act); P.S((uint64_t)n); uint32_t eb; memcpy(&eb, &eps, 4); P.S(eb); P.S(write_back);
         P.steps.push_back([=](uint8_t*) { return cc_launch_normq(d, x, og, w, eps, n, act, write_back); });
         { MkPhase ph = {}; ph.type = MK_NORMQ; ph.write_back = write_back; ph.x = x; ph.orig = og; ph.norm_w = w; ph.eps = eps; ph.n = (int)n; ph.act = cc_act_q8_0(act, n); P.phases.push_back(ph); }
+        // the final norm: its row is copied (the last of one) and only the copy's product reads it (llama2.rs:195-208) -> merge_picked
+        if (write_back && !orig && is(j + 2, L_COPY_ROWS) && is(j + 3, L_MATVEC)) {
+            const LOp &cr = q[j + 2], &mv = q[j + 3];
+            if (cr.b.buf == rn.a.buf && rn.a.buf->dtype == CC_F32 && cr.i2 == 0 && cr.rows.size() == 1 && cr.rows[0] == 0 && cr.a.buf->dtype == CC_F32 && vlen(cr.a) == n && vcontig(cr.a) && mv.b.buf == cr.a.buf &&
+                vlen(mv.b) == n && dead_after(rn.a.buf, j + 3) && dead_after(cr.a.buf, j + 4)) { picked = P.phases.size() - 1; P.S(0x2008); }
+        }
         *xbuf = rn.a.buf;
         size_t used = (j + 2) - i;
         for (size_t t = i; t < i + used; t++) q[t].done = true;
@@ -657,6 +663,18 @@ struct Fuser {
         }
     }
 
+    // megakernel only: [picked] NORMQ, ROWS that copies its row, MATVEC of the copy -> one MATVEC phase with the norm in its prologue (a 7B token's two phases
+    // of 6 and 7 us, at every model once a token)
+    size_t picked = (size_t)-1;
+    void merge_picked() {
+        if (picked == (size_t)-1 || picked + 2 >= P.phases.size()) return;
+        const MkPhase nq = P.phases[picked], cp = P.phases[picked + 1];
+        MkPhase& mv = P.phases[picked + 2];
+        if (nq.type != MK_NORMQ || cp.type != MK_ROWS || mv.type != MK_MATVEC || cp.rows_dev || cp.planes.p[0] != (const uint8_t*)nq.x || mv.x != (float*)cp.dst || mv.norm_w || mv.mv.k != nq.n) return;
+        mv.x = nq.x; mv.norm_w = nq.norm_w; mv.eps = nq.eps; mv.n = nq.n;
+        P.phases.erase(P.phases.begin() + picked, P.phases.begin() + picked + 2);
+    }
+
     void run() {
         index_uses();
         size_t i = 0;
@@ -696,6 +714,7 @@ struct Fuser {
             fallback(i);
             i++;
         }
+        merge_picked();
     }
 };
 

@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(MV_THREADS) matvec_kernel(WPlanes W, const voi
     extern __shared__ __align__(16) uint8_t smem[];
     const int bi = blockIdx.y;
     T::stage_act(act, n_total, bi, k, smem);
+    stage_wait();
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int row = blockIdx.x * MV_WARPS + warp; row < m; row += gridDim.x * MV_WARPS) {
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(MV_THREADS) matvec_few_kernel(WPlanes W, const
     extern __shared__ __align__(16) uint8_t smem[];
     const int b0 = blockIdx.y * NB, stride = T::smem_bytes(k);
     for (int n = 0; n < NB; n++) T::stage_act(act, n_total, min(b0 + n, b - 1), k, smem + n * stride);       // activations behind the last repeat it
+    stage_wait();
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int row = (blockIdx.x * MV_WARPS + warp) * 2; row < m; row += gridDim.x * MV_WARPS * 2) {
@@ -70,34 +72,29 @@ static int launch_few(cc_device* dev, const WPlanes& W, const void* act, int64_t
 // integers of vecdot.cuh, whose terms follow from them in the same order.  There a lane (super-block mod 4, chunk) adds up its terms and the
 // butterfly the lanes; here warp q of four has the super-blocks q, q + 4, .. of the 16 rows and a sum for each of the 8 chunks, and the four warps' sums are
 // added up in shared memory in the butterfly's order: identical bits.  A lane holds the weights of two rows at 4 columns of a chunk; activations come by ldmatrix.
-// Bound by the latency of the weights (16 warps an SM, a super-block of 16 rows each ahead) and the 9 instructions an output and chunk behind the mma.
-// us with the quantisation of the rows, 11008 x 4096 x 8 / 16 / 31 rows: two weight rows a warp by dp4a 31.4 / 44.1 / 74.2 ; here 27.2 / 37.3 / 54.4 ; 32000 x 4096 61 / 103 / 184 ; 48 / 72 /
-// 128.  CTAs of one group of warps: 26.9 / 41.9 / 66.4.  Q6_K the same way: 31.6 by dp4a, 43.4 here (its numbers take twice the instructions to put together).
+// A warp copies its super-blocks (16 rows x 144 B, which lie in memory as in shared memory) four ahead by cp.async (two, where activations of 40 super-blocks leave no
+// more room); rows of 144 B put the words of eight rows in different banks.  One CTA of two groups of four warps an SM: bound by the instructions, the mma among
+// them, and more warps only stage later (two CTAs an SM 11008 x 4096 x 8 25.1 us, CTAs of 3 / 4 / 5 groups 24.0 / 27.1 / 21.8).
+// us with the quantisation of the rows, 11008 x 4096 x 8 / 16 / 31 rows: two weight rows a warp by dp4a 31.4 / 44.1 / 74.2 ; weights by 4-byte loads one super-block ahead and activations
+// staged one after another 28.0 / 37.3 / 54.3 ; here 20.4 / 28.9 / 49.8 ; 32000 x 4096 48 / 72 / 128, now 39 / 68 / 128 ; 4096 x 4096 x 8 17.7, now 12.1.  Q6_K the same
+// way: 31.6 by dp4a, 43.4 (its numbers take twice the instructions to put together).
 #define MM_THREADS 256
 #define MM_GROUPS (MM_THREADS / 128)
 #define MM_OUT 128                         // outputs of four warps: 16 rows x 8 activations
+#define MM_SB 2304                         // a super-block of 16 rows
 __device__ __forceinline__ void mm_mma(int (&c)[4], unsigned a0, unsigned a1, unsigned b) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                  : "r"(a0), "r"(a1), "r"(b));
 }
-__device__ __forceinline__ unsigned mm_word(const uint8_t* p) { return __ldg((const unsigned*)p); }
-// one super-block of rows ra, rb (of the plane's rows) against 8 activations: acc[chunk][output]
+// one super-block of a lane's two rows (their copies in shared memory) against 8 activations: acc[chunk][output]
 struct MmBlock {
-    unsigned w[2][8];
-    int4 h[2];
-    __device__ __forceinline__ void load(const WPlanes& W, int64_t ra, int64_t rb, int nsb, int sb, int c) {
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const uint8_t* blk = W.p[0] + ((r ? rb : ra) * nsb + sb) * 144;
-            h[r] = __ldg((const int4*)blk);
-#pragma unroll
-            for (int j = 0; j < 8; j++) w[r][j] = mm_word(blk + 16 + 16 * j + 4 * c);
-        }
-    }
+    const uint8_t *ra, *rb;                // row lane / 4 and the one 8 behind it
+    int c;
     __device__ __forceinline__ void add(float (&acc)[8][4], const unsigned (&b)[16], const uint8_t* const (&act)[2], int k, int sb) const {
         unsigned s[2][2], mn[2][2];
         float d[4], dm[4];
+        const int4 h[2] = {*(const int4*)ra, *(const int4*)rb};
         int4 bs[2][2];                                           // block sums of the two activations, two 16-bit numbers a word
 #pragma unroll
         for (int n = 0; n < 2; n++) {
@@ -116,8 +113,9 @@ struct MmBlock {
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0}, sums[2];
-            mm_mma(lo, w[0][j] & 0x0F0F0F0Fu, w[1][j] & 0x0F0F0F0Fu, b[j]);
-            mm_mma(hi, (w[0][j] >> 4) & 0x0F0F0F0Fu, (w[1][j] >> 4) & 0x0F0F0F0Fu, b[8 + j]);
+            const unsigned w0 = *(const unsigned*)(ra + 16 + 16 * j + 4 * c), w1 = *(const unsigned*)(rb + 16 + 16 * j + 4 * c);
+            mm_mma(lo, w0 & 0x0F0F0F0Fu, w1 & 0x0F0F0F0Fu, b[j]);
+            mm_mma(hi, (w0 >> 4) & 0x0F0F0F0Fu, (w1 >> 4) & 0x0F0F0F0Fu, b[8 + j]);
             const int g = j >> 1;
 #pragma unroll
             for (int n = 0; n < 2; n++) {
@@ -136,36 +134,57 @@ struct MmBlock {
 };
 // distance of two activations in shared memory: an odd number of 16-byte pieces, so that 8 of them lie in different banks
 __host__ __device__ __forceinline__ int mm_stride(int bytes) { return (bytes & 16) ? bytes : bytes + 16; }
-__global__ void __launch_bounds__(MM_THREADS, 512 / MM_THREADS) matvec_mma_kernel(WPlanes W, const void* act, int64_t n_total, float* __restrict__ out, int m, int k, int b) {
+// shared memory: 8 activations | the warps' super-blocks, S a warp; behind a tile's last one: the warps' sums [groups][4 warps][8 chunks][MM_OUT]
+template <int S>
+__global__ void __launch_bounds__(MM_THREADS, 1) matvec_mma_kernel(WPlanes W, const void* act, int64_t n_total, float* __restrict__ out, int m, int k, int b) {
     pdl_enter();
     extern __shared__ __align__(16) uint8_t smem[];
-    const int b0 = blockIdx.y * 8, stride = mm_stride(TQ45_K<false>::smem_bytes(k)), nsb = k >> 8;
-    float* part = (float*)(smem + 8 * stride);                                 // [groups][4 warps][8 chunks][MM_OUT]
-    for (int n = 0; n < 8; n++) TQ45_K<false>::stage_act(act, n_total, min(b0 + n, b - 1), k, smem + n * stride);       // activations behind the last repeat it
-    __syncthreads();
+    const int b0 = blockIdx.y * 8, there = min(8, b - b0), stride = mm_stride(TQ45_K<false>::smem_bytes(k)), nsb = k >> 8;
+    float* part = (float*)(smem + 8 * stride);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = warp & 3, group = warp >> 2, c = lane & 3;
-    const uint8_t* const mine[2] = {smem + 2 * c * stride, smem + (2 * c + 1) * stride};      // the activations of this lane's outputs
-    const unsigned rows = (unsigned)__cvta_generic_to_shared(smem + (lane & 7) * stride) + ((lane & 8) ? 128 : 0) + ((lane & 16) ? 16 : 0);      // ldmatrix: chunks j, j + 8, j + 1, j + 9
+    uint8_t* ring = smem + 8 * stride + warp * (S * MM_SB);
+    const int nq = (nsb - q + 3) >> 2;                                         // this warp's super-blocks of a tile: q, q + 4, ..
+    auto ask = [&](int row0, int i) {                                          // the i-th of them; a group every time, empty behind the last
+        if (row0 < m && i < nq) {
+            const unsigned to = (unsigned)__cvta_generic_to_shared(ring + (i % S) * MM_SB) + lane * 16;
+#pragma unroll
+            for (int p = 0; p < 5; p++) {
+                const int x = lane + 32 * p, row = x / 9;                      // 9 pieces of 16 B a row
+                if (x < 144) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 512 * p), "l"(W.p[0] + ((int64_t)min(row0 + row, m - 1) * nsb + q + 4 * i) * 144 + (x - 9 * row) * 16) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int n = 0; n < there; n++) TQ45_K<false>::stage_act(act, n_total, b0 + n, k, smem + n * stride);       // (columns behind the last read it: eight copies of one row made 600 requests a line)
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int i = 0; i < S; i++) ask((int)(blockIdx.x * MM_GROUPS + group) * 16, i);
+    asm volatile("cp.async.wait_group %0;" ::"n"(S) : "memory");              // the activations
+    __syncthreads();
+    const uint8_t* const mine[2] = {smem + min(2 * c, there - 1) * stride, smem + min(2 * c + 1, there - 1) * stride};      // the activations of this lane's outputs
+    const unsigned rows = (unsigned)__cvta_generic_to_shared(smem + min(lane & 7, there - 1) * stride) + ((lane & 8) ? 128 : 0) + ((lane & 16) ? 16 : 0);      // ldmatrix: chunks j, j + 8, j + 1, j + 9
     for (int t = blockIdx.x; t * (16 * MM_GROUPS) < m; t += gridDim.x) {
-        const int row0 = t * (16 * MM_GROUPS) + group * 16;
-        const int64_t ra = min(row0 + (lane >> 2), m - 1), rb = min(row0 + (lane >> 2) + 8, m - 1);
+        const int row0 = (t * MM_GROUPS + group) * 16;
         float acc[8][4];
 #pragma unroll
         for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
         if (row0 < m) {
-            MmBlock blk;
-            if (q < nsb) blk.load(W, ra, rb, nsb, q, c);
 #pragma unroll 1
-            for (int sb = q; sb < nsb; sb += 4) {
+            for (int i = 0; i < nq; i++) {
+                const int sb = q + 4 * i;
                 unsigned bx[16];
 #pragma unroll
                 for (int j = 0; j < 8; j += 2)
                     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(bx[j]), "=r"(bx[8 + j]), "=r"(bx[j + 1]), "=r"(bx[9 + j]) : "r"(rows + sb * 256 + j * 16));
-                const MmBlock now = blk;
-                if (sb + 4 < nsb) blk.load(W, ra, rb, nsb, sb + 4, c);
-                now.add(acc, bx, mine, k, sb);
+                asm volatile("cp.async.wait_group %0;" ::"n"(S - 1) : "memory");
+                __syncwarp();
+                MmBlock blk;
+                blk.ra = ring + (i % S) * MM_SB + (lane >> 2) * 144; blk.rb = blk.ra + 8 * 144; blk.c = c;
+                blk.add(acc, bx, mine, k, sb);
+                __syncwarp();
+                ask(row0, i + S);
             }
         }
+        __syncthreads();                                                       // the sums go where the super-blocks were
         float* to = part + ((group * 4 + q) * 8) * MM_OUT + lane * 4;
 #pragma unroll
         for (int j = 0; j < 8; j++) *(float4*)(to + j * MM_OUT) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
@@ -176,26 +195,33 @@ __global__ void __launch_bounds__(MM_THREADS, 512 / MM_THREADS) matvec_mma_kerne
 #pragma unroll
         for (int j = 0; j < 8; j++) v[j] = (from[j * MM_OUT] + from[(16 + j) * MM_OUT]) + (from[(8 + j) * MM_OUT] + from[(24 + j) * MM_OUT]);
         const float sum = ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
-        const int row = t * (16 * MM_GROUPS) + (threadIdx.x / MM_OUT) * 16 + (o >> 4) + ((o & 2) ? 8 : 0), n = b0 + ((o >> 2) & 3) * 2 + (o & 1);
+        const int row = (t * MM_GROUPS + (int)threadIdx.x / MM_OUT) * 16 + (o >> 4) + ((o & 2) ? 8 : 0), n = b0 + ((o >> 2) & 3) * 2 + (o & 1);
         if (row < m && n < b) out[(int64_t)n * m + row] = sum;
-        __syncthreads();                                                       // the next tile's sums go where these were
+        if ((t + (int)gridDim.x) * (16 * MM_GROUPS) < m) {
+            __syncthreads();
+            for (int i = 0; i < S; i++) ask(row0 + (int)gridDim.x * (16 * MM_GROUPS), i);
+        }
     }
 }
-static bool mm_fits(int64_t k) { return 8 * (int64_t)(TQ45_K<false>::smem_bytes((int)k) + 16) + MM_GROUPS * 32 * MM_OUT * 4 <= 200 * 1024; }
+static int mm_act_bytes(int64_t k) { return 8 * mm_stride(TQ45_K<false>::smem_bytes((int)k)); }
+static int mm_smem(int64_t k, int stages) { const int part = MM_GROUPS * 32 * MM_OUT * 4, ring = MM_GROUPS * 4 * stages * MM_SB; return mm_act_bytes(k) + (part > ring ? part : ring); }
+#define MM_MOST (224 * 1024)
+static bool mm_fits(int64_t k) { return mm_act_bytes(k) <= 168 * 1024; }
+template <int S>
+static int launch_mma_as(cc_device* dev, const WPlanes& W, const void* act, int64_t n_total, float* out, int64_t m, int64_t k, int64_t b, int64_t ctas) {
+    int smem = mm_smem(k, S);
+    // an SM for each CTA: more than half of its shared memory.  Started while the kernel before is still there, some SMs took two and others none
+    if (smem < 116 * 1024) smem = 116 * 1024;
+    CC_CUDA(dev, cudaFuncSetAttribute(matvec_mma_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cc_launch_pdl(dev, matvec_mma_kernel<S>, dim3((unsigned)ctas, (unsigned)((b + 7) / 8)), MM_THREADS, smem, W, act, n_total, out, (int)m, (int)k, (int)b);
+    CC_LAUNCH_CHECK(dev);
+    return CC_OK;
+}
 static int launch_mma(cc_device* dev, const cc_buf* w, const void* act, int64_t n_total, float* out, int64_t m, int64_t k, int64_t b) {
     WPlanes W;
     for (int i = 0; i < CC_MAX_PLANES; i++) W.p[i] = w->plane[i];
-    int smem = 8 * mm_stride(TQ45_K<false>::smem_bytes((int)k)) + MM_GROUPS * 32 * MM_OUT * 4;
-    const int64_t groups = (b + 7) / 8, need = (m + 16 * MM_GROUPS - 1) / (16 * MM_GROUPS), fit = 224 * 1024 / (smem + 1024), most = dev->sm_count * (fit < 512 / MM_THREADS ? fit : 512 / MM_THREADS);
-    int64_t ctas = most / groups > 0 ? most / groups : 1;
-    if (ctas > need) ctas = need;
-    // no more CTAs than SMs: each gets an SM of its own by asking for more than half of its shared memory.  Started while the kernel before is still there, some SMs took two
-    // and others none: 4096 x 8192, 8 rows 31.8 us, now 23.8 (by dp4a 27.6) ; 4096 x 4096, 5 rows 18.1, now 14.3 (17.2)
-    if (ctas * groups <= dev->sm_count && smem < 116 * 1024) smem = 116 * 1024;
-    CC_CUDA(dev, cudaFuncSetAttribute(matvec_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    cc_launch_pdl(dev, matvec_mma_kernel, dim3((unsigned)ctas, (unsigned)groups), MM_THREADS, smem, W, act, n_total, out, (int)m, (int)k, (int)b);
-    CC_LAUNCH_CHECK(dev);
-    return CC_OK;
+    const int64_t groups = (b + 7) / 8, most = dev->sm_count / groups > 0 ? dev->sm_count / groups : 1, tiles = (m + 16 * MM_GROUPS - 1) / (16 * MM_GROUPS), ctas = tiles < most ? tiles : most;
+    return mm_smem(k, 4) <= MM_MOST ? launch_mma_as<4>(dev, W, act, n_total, out, m, k, b, ctas) : launch_mma_as<2>(dev, W, act, n_total, out, m, k, b, ctas);
 }
 template <class T>
 static int launch(cc_device* dev, const cc_buf* w, const void* act, int64_t n_total, float* out, int64_t m, int64_t k, int64_t b) {

@@ -22,18 +22,19 @@ __device__ __forceinline__ int4 shl4(const int4& v, int s) { return make_int4(v.
 __device__ __forceinline__ int spread4(unsigned bits) { return (int)((((bits & 0xF) * 0x00204081u) & 0x01010101u) << 4); }
 __device__ __forceinline__ int byte_of(unsigned w0, unsigned w1, int idx) { return (int)(((idx < 4 ? w0 : w1) >> (8 * (idx & 3))) & 0xFF); }
 
-// cooperative global -> shared copy of `bytes` (multiple of 4) bytes
+// cooperative global -> shared copy of `bytes` (multiple of 4) bytes.  The copies of a whole activation, of eight of them, are under way together: as loads and
+// stores each waited for the one before (in-order issue), 24 round trips to L2 in front of a product of 8 rows.  stage_wait, then a barrier, before it is read.
+__device__ __forceinline__ void stage_16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void stage_4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void stage(void* dst, const void* src, int bytes) {
-    if (((uintptr_t)src & 15) != 0) {          // batched activations: row bi may start 4-byte aligned only
-        for (int i = threadIdx.x; i < (bytes >> 2); i += blockDim.x) ((int*)dst)[i] = ((const int*)src)[i];
-        return;
-    }
-    int n16 = bytes >> 4;
-    const int4* s = (const int4*)src;
-    int4* d = (int4*)dst;
-    for (int i = threadIdx.x; i < n16; i += blockDim.x) d[i] = s[i];
-    int rem = (bytes & 15) >> 2;
-    if ((int)threadIdx.x < rem) ((int*)dst)[n16 * 4 + threadIdx.x] = ((const int*)src)[n16 * 4 + threadIdx.x];
+    const int n16 = ((uintptr_t)src & 15) ? 0 : bytes >> 4;                     // batched activations: row bi may start 4-byte aligned only
+    for (int i = threadIdx.x; i < n16; i += blockDim.x) stage_16((int4*)dst + i, (const int4*)src + i);
+    for (int i = n16 * 4 + (int)threadIdx.x; i < (bytes >> 2); i += blockDim.x) stage_4((int*)dst + i, (const int*)src + i);
 }
 __host__ __device__ inline int al16i(int v) { return (v + 15) & ~15; }
 
@@ -248,7 +249,7 @@ struct TKBase {
         const uint8_t* p = (const uint8_t*)scratch;
         int64_t o1 = (n_total + 15) & ~15ll, o2 = o1 + ((n_total / 256 * 4 + 15) & ~15ll);
         const int4* q = (const int4*)(p + (int64_t)bi * k);
-        for (int i = threadIdx.x; i < (k >> 4); i += blockDim.x) ((int4*)sm)[T::act_at(i)] = q[i];
+        for (int i = threadIdx.x; i < (k >> 4); i += blockDim.x) stage_16((int4*)sm + T::act_at(i), q + i);
         stage(sm + al16i(k), p + o1 + (int64_t)bi * (k / 256) * 4, k / 256 * 4);
         stage(sm + al16i(k) + al16i(k / 256 * 4), p + o2 + (int64_t)bi * (k / 16) * 2, k / 16 * 2);
     }

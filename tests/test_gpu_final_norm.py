@@ -46,3 +46,29 @@ def test_final_norm_and_classifier(wt, m, k):
     finally:
         fused.close()
         eager.close()
+
+
+@pytest.mark.parametrize("lazy", [1, 2])
+@pytest.mark.parametrize("rows,k,at", [(2, 32, 0), (5, 288, 4), (40, 512, 17)])
+def test_a_prompts_row_is_normed_alone_only_where_the_others_are_dropped(lazy, rows, k, at):
+    from crabml_b200 import CudaTensor as T
+    rng = np.random.default_rng(rows)
+    nw = (1.0 + 0.1 * rng.standard_normal(k)).astype(np.float32)
+    devs = make_device(lazy=lazy), make_device(lazy=0)
+    try:
+        for keep in (False, True, False):
+            x = rng.standard_normal((rows, k)).astype(np.float32)
+            got = []
+            for d in devs:
+                t = T.new(x.reshape(-1).copy(), [rows, k], d).rms_norm_inplace(1e-5).mul_inplace(T.from_cpu(nw, [k], oc.F32, d))
+                last = T.alloc([k], oc.F32, d)
+                last.copy_rows_from(t, [at])
+                if not keep:
+                    del t
+                got.append([last.export().copy()] + ([t.export().copy()] if keep else []))
+            for a, b in zip(*got):
+                np.testing.assert_array_equal(a.view(np.uint32), b.view(np.uint32))
+            t = last = None
+    finally:
+        for d in devs:
+            d.close()

@@ -42,9 +42,10 @@ struct GraphEntry { cudaGraphExec_t exec = nullptr; size_t dyn_bytes = 0; uint64
                     std::vector<uint64_t> sig; uint64_t last_use = 0; int mega_variant = 0; };
 #define LZ_MAX_GRAPHS 192                            // cached token graphs per device: 64 token shapes (sequences with caches of their own) of three parts each
 
-#define LZ_FIRST_OPS 64                              // the first part of a token: three layers, work for the GPU until the next part is recorded and fused
-#define LZ_PART_GROWTH 4                             // and each part so much longer than the one before: an op of a 7B layer keeps the GPU for 2.2 us and the host
-                                                     // for 0.5, so the 776 ops behind the first part (180 us of GPU) left the GPU idle for some 200 us a token
+#define LZ_FIRST_OPS 30                              // the first part of a token: more than a layer, work for the GPU until the next part is recorded and fused
+#define LZ_PART_GROWTH 5                             // and each part so much longer than the one before: an op of a 7B layer keeps the GPU for 2.2 us and the host for
+                                                     // 0.25.  16 tokens with first / growth 64 / 4, 40 / 4, 30 / 5, 22 / 6, ms: 7B 30.6 / 30.5 / 30.4 / 30.7 (two parts, before: 3 ms more), four 7B
+                                                     // layers of K-quants 7.39 / 7.19 / 7.18 / 6.97, 15M 4.23 / 4.34 / 4.32 / 4.61 (its kernels are short: a third part costs it more than it hides)
 
 struct LazyState {
     std::vector<LOp> q;

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("wt,ct", [(oc.Q8_0, oc.Q8_0), (oc.Q4_K, oc.Q6_K)])
 def test_a_token_of_three_parts_has_the_eager_bits(wt, ct):
     from crabml_b200 import runner as R
-    conf = R.LlamaConfig(4, 2, 16, 256, 512, 64, 512, 1e-5, 64)        # 16 layers of 26 ops: parts of 64, 256 and the rest
+    conf = R.LlamaConfig(4, 2, 16, 256, 512, 64, 512, 1e-5, 64)        # 16 layers of 26 ops: parts of 30, 150 and the rest
     res = {}
     for lazy in (0, 2):
         dev = make_device(lazy=lazy)

@@ -71,6 +71,7 @@ __device__ __forceinline__ unsigned mr_ld_acquire_shared(unsigned addr) {
 // 75 items).  Producer and consumers derive the same item sequence from this: group P, segment s = item P * NSEG + s.
 struct MrGeo {
     int nb, GR, NSEG, n_rows, groups, first, last_half_off;
+    int most;              // virtual rows of the CTA that has the most: what is laid out in shared memory goes by it, in every CTA and on the host
     bool pair;
 };
 __device__ __forceinline__ MrGeo mr_geo(const StreamArgs& A) {
@@ -83,10 +84,12 @@ __device__ __forceinline__ MrGeo mr_geo(const StreamArgs& A) {
         const int rpc = (((m_cat + (int)gridDim.x - 1) / (int)gridDim.x) + 3) & ~3;
         g.first = (int)blockIdx.x * rpc;
         g.n_rows = min(rpc, max(0, m_cat - g.first));
+        g.most = rpc;
     } else {
         const int each = m_cat / (int)gridDim.x, more = m_cat - each * (int)gridDim.x;
         g.first = (int)blockIdx.x * each + min((int)blockIdx.x, more);
         g.n_rows = each + ((int)blockIdx.x < more ? 1 : 0);
+        g.most = (each + (more ? 1 : 0)) << (g.pair ? 1 : 0);
     }
     g.groups = ((g.n_rows + 1) >> 1) << (g.pair ? 1 : 0);
     g.last_half_off = 16 * (g.nb - 32 * (g.GR - 1));
@@ -424,7 +427,7 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
     float* s_red = (float*)(smem + (size_t)nbp * 40);
     float* s_sum = (float*)(smem + (size_t)nbp * 40 + 256);
     const int vrows = pair ? 2 * g.n_rows : g.n_rows;
-    float* s_part = s_sum + ((vrows + 31) & ~31);
+    float* s_part = s_sum + ((g.most + 31) & ~31);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const StreamMats& M = A.mats;
     if (ph.x) {
@@ -460,7 +463,7 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
     const int* as_l = s_s + lane;
     // Warps 2 i and 2 i + 1 take the two rows of an item.  One warp on both rows held sixteen of the twenty slots at a time, so few copies were under way
     const int duo = warp >> 1, half = warp & 1;
-    const bool parts = mr_part_bytes(NSEG, vrows) > 0, split = parts && NSEG > 1;
+    const bool parts = mr_part_bytes(NSEG, g.most) > 0, split = parts && NSEG > 1;
     const int s0 = split ? duo % NSEG : 0, ns = split ? 1 : NSEG;
     const int P0 = split ? duo / NSEG : duo, dP = split ? (MK_WARPS / 2 - s0 + NSEG - 1) / NSEG : MK_WARPS / 2;
     constexpr unsigned DOFF = 2u * MK_SEG * (TYPE == CC_Q8_0 ? 1024u : 512u);
@@ -687,8 +690,8 @@ size_t cc_mega_ring_smem_for_phase(const MkPhase& ph, int ctas) {
     if (ph.type == MK_MATVEC) {
         const size_t k = (size_t)ph.mv.k, nb = k / 32, GR = (nb + 31) / 32, NSEG = (GR + MK_SEG - 1) / MK_SEG, nbp = NSEG * MK_SEG * 32;
         const size_t m = ph.mv.epilogue == 2 ? (size_t)ph.mv.mats.m[0] : (size_t)ph.mv.mats.m[0] + (ph.mv.mats.n > 1 ? ph.mv.mats.m[1] : 0) + (ph.mv.mats.n > 2 ? ph.mv.mats.m[2] : 0);
-        const size_t rows = ((m + (size_t)ctas - 1) / (size_t)ctas + 3) & ~(size_t)3, vrows = ph.mv.epilogue == 2 ? 2 * rows : rows;
-        const size_t sums = ((vrows + 31) & ~(size_t)31) * 4 + (size_t)mr_part_bytes((int)NSEG, (int)vrows);
+        const size_t rows = (m + (size_t)ctas - 1) / (size_t)ctas, most = ph.mv.epilogue == 2 ? 2 * rows : ph.mv.epilogue == 3 ? (rows + 3) & ~(size_t)3 : rows;      // mr_geo
+        const size_t sums = ((most + 31) & ~(size_t)31) * 4 + (size_t)mr_part_bytes((int)NSEG, (int)most);
         const size_t row = ph.x ? (k < MR_ROW_PIECE ? k : MR_ROW_PIECE) * 4 * (ph.norm_w ? 2 : 1) : 0;
         return nbp * 40 + 256 + (sums > row ? sums : row);
     }

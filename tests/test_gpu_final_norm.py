@@ -29,7 +29,7 @@ def tail(dev, w, norm, x, wt, m, k, keep):
     return out
 
 
-@pytest.mark.parametrize("wt,m,k", [(oc.Q8_0, 1000, 288), (oc.Q4_0, 512, 4096), (oc.Q4_K, 300, 512), (oc.Q6_K, 300, 1024)])
+@pytest.mark.parametrize("wt,m,k", [(oc.Q8_0, 1000, 288), (oc.Q8_0, 34386, 288), (oc.Q4_0, 512, 4096), (oc.Q4_K, 300, 512), (oc.Q6_K, 300, 1024)])
 def test_final_norm_and_classifier(wt, m, k):
     from crabml_b200 import CudaTensor as T
     rng = np.random.default_rng(k)

@@ -21,11 +21,13 @@ def geo(m, n_mats, k, epilogue, cta, grid=GRID):
         rpc = ((m_cat + grid - 1) // grid + 3) & ~3
         first = cta * rpc
         n_rows = min(rpc, max(0, m_cat - first))
+        most = rpc
     else:
         each, more = divmod(m_cat, grid)
         first = cta * each + min(cta, more)
         n_rows = each + (1 if cta < more else 0)
-    return dict(nb=nb, nseg=nseg, V=2 if pair else 1, n_units=n_rows, first=first, stride=1, groups=(n_rows + 1) // 2 * (2 if pair else 1))
+        most = (each + (1 if more else 0)) * (2 if pair else 1)
+    return dict(most=most, nb=nb, nseg=nseg, V=2 if pair else 1, n_units=n_rows, first=first, stride=1, groups=(n_rows + 1) // 2 * (2 if pair else 1))
 
 
 def rows_of(g, P):
@@ -46,8 +48,7 @@ def producer_order(g):
 def consumer_walk(g):
     """phase_matvec_ring: for every pair of warps the list of (item index, [(unit, virtual row, segment)]) it consumes, in order."""
     walks, nseg, duos = [], g["nseg"], WARPS // 2
-    vrows = g["n_units"] * g["V"]
-    part_bytes = vrows * 132 if nseg == 1 else vrows * nseg * 128 if nseg <= 4 else 0
+    part_bytes = g["most"] * 132 if nseg == 1 else g["most"] * nseg * 128 if nseg <= 4 else 0
     split = nseg > 1 and 0 < part_bytes <= 30720                       # warps keep to one segment
     for duo in range(duos):
         s0, ns = (duo % nseg, 1) if split else (0, nseg)
@@ -66,6 +67,7 @@ SHAPES = [  # (rows per matrix, matrices, k, epilogue)
     (4096, 1, 2048, 3), (4096, 1, 5504, 3), (16000, 1, 4096, 3),                                                    # shards at N = 2 (exchange phases)
     (512, 3, 4096, 0), (4096, 1, 512, 3), (1376, 2, 4096, 2), (4096, 1, 1376, 3), (4000, 1, 4096, 3),               # shards at N = 8
     (4096, 1, 14336, 1), (8192, 1, 28672, 1), (256000, 1, 8192, 0),                                               # four segments, seven, and more rows than their sums find room for
+    (34386, 1, 4096, 0), (4440, 2, 14336, 2),                                                                      # CTAs on both sides of the room for lanes' sums
     (288, 3, 288, 0), (288, 1, 288, 1), (768, 2, 288, 2), (288, 1, 768, 1), (32000, 1, 288, 0),                     # tinyllamas-15M (ragged groups)
 ]
 
@@ -88,6 +90,16 @@ def test_producer_and_consumers_agree_on_the_ring_order(m, n_mats, k, epilogue):
         assert sorted(seen) == list(range(len(order)))                # the consumers release every slot exactly once
         covered_rows.update(g["first"] + u * g["stride"] for u in range(g["n_units"]))
     assert covered_rows                                               # (the sampled CTAs own rows)
+
+
+@pytest.mark.parametrize("m,n_mats,k,epilogue", SHAPES)
+def test_no_cta_has_more_rows_than_the_layout_in_shared_memory_allows(m, n_mats, k, epilogue):
+    """the layout (and whether lanes' sums have room) goes by the CTA with the most rows: the same in every CTA and on the host (cc_mega_ring_smem_for_phase)"""
+    geos = [geo(m, n_mats, k, epilogue, cta) for cta in range(GRID)]
+    rows = -(-(m if epilogue == 2 else m * n_mats) // GRID)
+    host = 2 * rows if epilogue == 2 else (rows + 3) & ~3 if epilogue == 3 else rows
+    assert {g["most"] for g in geos} == {host}
+    assert max(g["n_units"] * g["V"] for g in geos) <= host
 
 
 @pytest.mark.parametrize("m,n_mats,k,epilogue", SHAPES)

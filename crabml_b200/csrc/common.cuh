@@ -321,7 +321,7 @@ int cc_launch_mega(cc_device* dev, const MkPhase* phases_dev, int n_phases, cons
 int cc_mega_flags();
 bool cc_mega_ring_enabled();
 bool cc_mega_ring_phase_ok(const MkPhase& ph);
-static inline int cc_mega_ring_slot(int wtype) { return wtype == CC_Q8_0 ? 8704 : 4608; }      // an item of the ring: two rows' segment of 128 blocks, quants and f16 scales
+static inline int cc_mega_ring_slot(int wtype) { return wtype == CC_Q8_0 ? 9216 : 4608; }      // an item of the ring: two rows' segment of 128 blocks, quants and room for their f16 scales
 int cc_mega_ring_at_ch(const MkPhase& ph);
 size_t cc_mega_ring_smem_for_phase(const MkPhase& ph, int ctas);
 bool cc_mega_ring_fits(size_t smem_work, size_t smem_wstage, int slot_bytes, bool generic);

@@ -5,8 +5,8 @@
 // warp (20 MB per GPU, 3 us of HBM time) cover the bubble and HBM idles for the rest: 2.36 ms per Llama-2-7B Q8_0 token against
 // 1.07 ms of pure streaming.  Weights are immutable, so nothing forces the weight stream to follow the phase order of the compute:
 //   * warps 16-18 of every CTA are PRODUCERS: their threads walk the phase table on their own, ahead of the compute warps, and issue cp.async.bulk (TMA) copies
-//     of items -- two rows' segment of 128 blocks: 8192 B of Q8_0 quants + 512 B of f16 scales -- into a ring of shared-memory slots, as many as fit beside
-//     the per-phase working area (18 to 20 = 160-174 KB per SM, 25 MB per GPU).  They never wait for a barrier or an activation: whenever a slot is free the
+//     of items -- two rows' segment of 128 blocks: 8192 B of Q8_0 quants + 512 B of f16 scales (1024 B are theirs) -- into a ring of shared-memory slots, as many as fit beside
+//     the per-phase working area (17 to 19 = 160-174 KB per SM, 25 MB per GPU).  They never wait for a barrier or an activation: whenever a slot is free the
 //     next item of this CTA's rows -- of this phase or any later one -- is being fetched.
 //   * warp 19 asks L2 for the items behind the ring, up to 224 KB of them per SM (33 MB per GPU), at 20 B per cycle and SM: a full ring is 4 us of HBM time, the
 //     time between one phase's last row and the next one's first 5 to 7 us, the attention phase 7.  A 7B Q8_0 token 1862 -> 1814 us (120 KB 1830; 224 and 300 KB, 20
@@ -106,7 +106,14 @@ __device__ __forceinline__ int mr_locate(const StreamMats& M, int rc, int& mat) 
 }
 
 // where item j of a phase comes from: quants and scales of its two rows (two = false: one row, or two rows of one matrix next to each other as one run)
-struct MrItem { const uint8_t* q[2]; const uint16_t* d[2]; unsigned qbytes, dbytes; bool two; };
+struct MrItem { const uint8_t* q[2]; const uint16_t* d[2]; unsigned qbytes, dbytes, dspan; bool two; };       // dspan: both rows' scales as one copy, what lies between them included (0: a copy each)
+// Where the second row's scales lie behind the first's: beside them, or, where Q8_0 rows are longer than a segment and both fit, as far as in the plane: one copy of
+// both and of what lies between them, an item in three copies (11008 x 4096: 14.3 -> 14.0 us, a token 1806 -> 1777; Q4_0 waits for its consumers, larger slots only cost it 0.7 %)
+#define MR_SCALES 1024
+__device__ __forceinline__ unsigned mr_scale_off(const MrGeo& g, unsigned BB, unsigned dbytes) {
+    const unsigned row = 2u * CC_D_STRIDE(g.nb);
+    return BB == 32u && g.NSEG > 1 && row + 2u * MK_SEG * 32u <= MR_SCALES ? row : dbytes;
+}
 __device__ __forceinline__ MrItem mr_item(const StreamMats& M, const MrGeo& g, unsigned BB, int j) {
     MrItem it;
     const int P = j / g.NSEG, sg = j - P * g.NSEG;
@@ -121,6 +128,7 @@ __device__ __forceinline__ MrItem mr_item(const StreamMats& M, const MrGeo& g, u
     it.q[0] = M.qs[mat] + ((size_t)rA * g.nb + at) * BB; it.d[0] = M.d[mat] + (size_t)rA * d_row + at;
     it.q[1] = M.qs[matB] + ((size_t)rB * g.nb + at) * BB; it.d[1] = M.d[matB] + (size_t)rB * d_row + at;
     if (it.two && g.NSEG == 1 && it.q[1] == it.q[0] + it.qbytes && (const uint8_t*)it.d[1] == (const uint8_t*)it.d[0] + it.dbytes) { it.qbytes *= 2; it.dbytes *= 2; it.two = false; }
+    it.dspan = it.two && (const uint8_t*)it.d[1] == (const uint8_t*)it.d[0] + mr_scale_off(g, BB, it.dbytes) ? mr_scale_off(g, BB, it.dbytes) + it.dbytes : 0u;
     return it;
 }
 
@@ -204,11 +212,11 @@ __device__ void mr_producer(const MkPhase* __restrict__ phases, int n_phases, co
                 }
                 if (!use || (mr_ld_acquire_shared(done0 + 8u * slot) == e - (unsigned)R.nslots + 1u && mr_ld_acquire_shared(done0 + 8u * slot + 4u) == e - (unsigned)R.nslots + 1u)) {      // the slot's previous tenant has been consumed
                     const unsigned fb = full0 + 8u * slot, dst = ring0 + slot * (unsigned)R.slot_bytes;
-                    mr_expect_tx(fb, (im.qbytes + im.dbytes) << (im.two ? 1 : 0));
+                    mr_expect_tx(fb, im.dspan ? 2u * im.qbytes + im.dspan : (im.qbytes + im.dbytes) << (im.two ? 1 : 0));
                     mr_bulk_g2s(dst, im.q[0], im.qbytes, fb);
                     if (im.two) mr_bulk_g2s(dst + im.qbytes, im.q[1], im.qbytes, fb);
-                    mr_bulk_g2s(dst + doff, im.d[0], im.dbytes, fb);
-                    if (im.two) mr_bulk_g2s(dst + doff + im.dbytes, im.d[1], im.dbytes, fb);
+                    mr_bulk_g2s(dst + doff, im.d[0], im.dspan ? im.dspan : im.dbytes, fb);
+                    if (im.two && !im.dspan) mr_bulk_g2s(dst + doff + mr_scale_off(g, BB, im.dbytes), im.d[1], im.dbytes, fb);
                     __threadfence_block();
                     s_seq[slot] = e + 1u;
                     j += MR_ISSUERS; have = false; atomicAdd((int*)s_issued, 1);
@@ -483,7 +491,7 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
             float part = 0.0f;
             if (row) {
                 const uint8_t* sp = RC.ring + (size_t)slot * RC.slot_bytes;
-                part = mr_dot<TYPE>(sp + (half ? (unsigned)nbe * (TYPE == CC_Q8_0 ? 32u : 16u) : 0u), (const uint16_t*)(sp + DOFF + (half ? (unsigned)((nbe * 2 + 15) & ~15) : 0u)), left,
+                part = mr_dot<TYPE>(sp + (half ? (unsigned)nbe * (TYPE == CC_Q8_0 ? 32u : 16u) : 0u), (const uint16_t*)(sp + DOFF + (half ? mr_scale_off(g, TYPE == CC_Q8_0 ? 32u : 16u, (unsigned)((nbe * 2 + 15) & ~15)) : 0u)), left,
                                     g.last_half_off, lane, act);
             }
             acc += part;

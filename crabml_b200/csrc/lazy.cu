@@ -40,7 +40,8 @@ struct LOp {
 // on every hit (a colliding key must re-capture, never replay another plan's baked pointers); `last_use` drives the LRU bound.
 struct GraphEntry { cudaGraphExec_t exec = nullptr; size_t dyn_bytes = 0; uint64_t launches = 0; MkPhase* phases_dev = nullptr;
                     std::vector<uint64_t> sig; uint64_t last_use = 0; int mega_variant = 0; };
-#define LZ_MAX_GRAPHS 192                            // cached token graphs per device: 64 token shapes (sequences with caches of their own) of three parts each
+#define LZ_MAX_PARTS 4                               // parts of a token: three grow, the fourth runs to its end (models of 36 layers and more have one)
+#define LZ_MAX_GRAPHS (64 * LZ_MAX_PARTS)            // cached token graphs per device: 64 token shapes (sequences with caches of their own), a graph a part
 
 #define LZ_FIRST_OPS 30                              // the first part of a token: more than a layer, work for the GPU until the next part is recorded and fused
 #define LZ_PART_GROWTH 5                             // and each part so much longer than the one before: an op of a 7B layer keeps the GPU for 2.2 us and the host for
@@ -50,7 +51,7 @@ struct GraphEntry { cudaGraphExec_t exec = nullptr; size_t dyn_bytes = 0; uint64
 struct LazyState {
     std::vector<LOp> q;
     std::unordered_map<cc_buf*, int> qrefs;
-#define LZ_DYN_SLOTS 24                              // the host may run eight tokens of three parts ahead of the GPU (absorbs host scheduling hiccups)
+#define LZ_DYN_SLOTS (8 * LZ_MAX_PARTS)              // a slot a part: the host may run eight tokens ahead of the GPU (absorbs host scheduling hiccups)
     uint8_t* dyn_host[LZ_DYN_SLOTS] = {nullptr};   // pinned, rotated so the host can build tokens t+1.. while t runs
     cudaEvent_t dyn_ev[LZ_DYN_SLOTS] = {nullptr};
     int dyn_slot = 0;
@@ -66,6 +67,7 @@ struct LazyState {
     uint64_t ns_record = 0, ns_fuse = 0, ns_submit = 0, n_ops = 0;      // host-side cost accounting
     int mega_variant = 0;            // persistent kernel of the last megakernel flush: 1 mega_kernel, 2 mega_ring_kernel
     size_t part_ops = LZ_FIRST_OPS;  // queued ops from which the token being recorded starts, or goes on
+    int parts = 0;                   // of it that run already
 };
 
 static LView mkview(const cc_view* v) {
@@ -130,8 +132,9 @@ int cc_lazy_record(cc_device* dev, int kind, const cc_view* a, const cc_view* b,
     // a long token starts while the rest of it is still being recorded: at the first copy of a layer's input (attention's or the feed-forward's) behind
     // part_ops ops the queue so far runs, and the next part may be longer.  No fused pattern spans that copy, so the phases are the same ones in several
     // kernels.  Ranks that exchange keep one part: their launches stay paired.  So does a profiled token
-    if (kind == L_DUP && lz->q.size() >= lz->part_ops && !cc_comm_dev(dev) && !lz->prof_dev && a && a->ndim <= 2 && view_rows(a) == 1) {
+    if (kind == L_DUP && lz->parts < LZ_MAX_PARTS - 1 && lz->q.size() >= lz->part_ops && !cc_comm_dev(dev) && !lz->prof_dev && a && a->ndim <= 2 && view_rows(a) == 1) {
         lz->part_ops *= LZ_PART_GROWTH;
+        lz->parts++;
         int rc = cc_lazy_flush_part(dev, false);
         if (rc) return rc;
     }
@@ -745,7 +748,7 @@ struct Fuser {
 };
 
 int cc_lazy_flush(cc_device* dev) {
-    if (dev->lz) dev->lz->part_ops = LZ_FIRST_OPS;
+    if (dev->lz) { dev->lz->part_ops = LZ_FIRST_OPS; dev->lz->parts = 0; }
     return cc_lazy_flush_part(dev, true);
 }
 static int cc_lazy_flush_part(cc_device* dev, bool whole) {

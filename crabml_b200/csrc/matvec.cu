@@ -72,7 +72,7 @@ static int launch_few(cc_device* dev, const WPlanes& W, const void* act, int64_t
 // integers of vecdot.cuh, whose terms follow from them in the same order.  There a lane (super-block mod 4, chunk) adds up its terms and the
 // butterfly the lanes; here warp q of four has the super-blocks q, q + 4, .. of the 16 rows and a sum for each of the 8 chunks, and the four warps' sums are
 // added up in shared memory in the butterfly's order: identical bits.  A lane holds the weights of two rows at 4 columns of a chunk; activations come by ldmatrix.
-// A warp copies its super-blocks (16 rows x 144 B, which lie in memory as in shared memory) four ahead by cp.async (two, where activations of 40 super-blocks leave no
+// A warp copies its super-blocks (16 rows x 144 B, which lie in memory as in shared memory) four ahead by cp.async (two, where activations of 67 to 73 super-blocks leave no
 // more room); rows of 144 B put the words of eight rows in different banks.  One CTA of two groups of four warps an SM: bound by the instructions, the mma among
 // them, and more warps only stage later (two CTAs an SM 11008 x 4096 x 8 25.1 us, CTAs of 3 / 4 / 5 groups 24.0 / 27.1 / 21.8).
 // us with the quantisation of the rows, 11008 x 4096 x 8 / 16 / 31 rows: two weight rows a warp by dp4a 31.4 / 44.1 / 74.2 ; weights by 4-byte loads one super-block ahead and activations

@@ -370,6 +370,12 @@ def test_few_rows_of_q4_k_have_the_bits_of_one(dev, m, k, b):
     test_few_rows_have_the_bits_of_one(dev, oc.Q4_K, m, k, b)
 
 
+@pytest.mark.parametrize("m,k,b", [(33, 16896, 8), (1, 17152, 5), (45, 17152, 12), (1217, 17152, 31), (31, 18688, 31), (50, 18688, 7), (20, 18944, 8)])
+def test_few_rows_of_q4_k_with_long_activations_have_the_bits_of_one(dev, m, k, b):
+    """66 super-blocks are the most that leave room for four stages of weights a warp, 67 to 73 have two (1217 rows: more tiles than CTAs, so the stages fill again), 74 go without the tensor cores"""
+    test_few_rows_have_the_bits_of_one(dev, oc.Q4_K, m, k, b)
+
+
 @pytest.mark.parametrize("t", [oc.Q8_0, oc.Q4_0, oc.Q5_0])
 @pytest.mark.parametrize("m,k,b", [(1, 32, 2), (33, 288, 3), (40, 1056, 8), (257, 4096, 9), (17, 14336, 31), (16, 40960, 5)])
 def test_few_rows_against_the_oracle(dev, t, m, k, b):

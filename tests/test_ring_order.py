@@ -110,3 +110,13 @@ def test_every_row_of_a_phase_belongs_to_exactly_one_cta(m, n_mats, k, epilogue)
         rows += [g["first"] + u * g["stride"] for u in range(g["n_units"])]
     m_cat = m if epilogue == 2 else m * n_mats
     assert sorted(rows) == list(range(m_cat))
+
+
+def test_items_that_come_free_together_are_issued_by_different_warps():
+    """mr_producer: thread 3 * lane + warp owns item t mod 96; of any ring's worth of neighbouring items no warp has more than a third (its lanes issue one after another)"""
+    owner = {lane * 3 + warp: warp for warp in range(3) for lane in range(32)}
+    assert sorted(owner) == list(range(96))
+    for first in range(96):
+        for items in (8, 17, 24, 48):
+            share = [sum(owner[e % 96] == w for e in range(first, first + items)) for w in range(3)]
+            assert max(share) <= -(-items // 3), (first, items, share)

@@ -296,10 +296,10 @@ struct DeqPlanes { const uint8_t* p[CC_MAX_PLANES]; int64_t cols; };
 enum { MK_NORMQ = 0, MK_MATVEC = 1, MK_ATTN = 2, MK_ROWS = 3, MK_REDUCE = 4, MK_GATHER = 5, MK_ARGMAX = 6 };
 struct MkPhase {
     int type, wtype, write_back, next_matvec;
-    int xgpu, red_n, next_matvec2, spare; float* red_dst; const float* red_res;   // cross-GPU barrier after this phase ; REDUCE/GATHER phase operands   // next_matvec / next_matvec2: index of the next MATVEC phase and of the one after it (look-ahead prefetch), -1 if none
+    int xgpu, red_n, next_matvec2, ring_sums; float* red_dst; const float* red_res;   // cross-GPU barrier after this phase ; REDUCE/GATHER phase operands   // next_matvec / next_matvec2: index of the next MATVEC phase and of the one after it (look-ahead prefetch), -1 if none
     // NORMQ (and the output quantisation of ATTN)
     float* x; float* orig; const float* norm_w; float eps; int n; ActQ8_0 act;
-    int act_type, spare2;               // MATVEC: CC_Q8_0 (streaming phases) or CC_Q8_K (generic phases: K-quant weights)
+    int act_type, ring_parts;           // MATVEC: CC_Q8_0 (streaming phases) or CC_Q8_K (generic phases: K-quant weights) ; ring_sums, ring_parts: cc_mega_ring_layout
     StreamArgs mv;                      // MATVEC
     AttnArgs at;                        // ATTN
     unsigned long long dyn_off, rope_off;   // ATTN {pos, kv_len} / ROWS row list ; RoPE table
@@ -323,7 +323,7 @@ bool cc_mega_ring_enabled();
 bool cc_mega_ring_phase_ok(const MkPhase& ph);
 static inline int cc_mega_ring_slot(int wtype) { return wtype == CC_Q8_0 ? 9216 : 4608; }      // an item of the ring: two rows' segment of 128 blocks, quants and room for their f16 scales
 int cc_mega_ring_at_ch(const MkPhase& ph);
-size_t cc_mega_ring_smem_for_phase(const MkPhase& ph, int ctas);
+size_t cc_mega_ring_layout(MkPhase& ph, int ctas);      // working area of the phase on so many CTAs; how a streaming phase's sums lie in it
 bool cc_mega_ring_fits(size_t smem_work, size_t smem_wstage, int slot_bytes, bool generic);
 int cc_launch_mega_ring(cc_device* dev, const MkPhase* phases_dev, int n_phases, const uint8_t* dyn_dev, unsigned* bar_dev, size_t smem_work, size_t smem_wstage,
                         unsigned long long* prof, const CommDev* comm, bool generic, int slot_bytes, int at_ch, int flags);

@@ -852,7 +852,7 @@ static int cc_lazy_flush_part(cc_device* dev, bool whole) {
                 if (P.mega_ring) {              // is there room for a useful ring beside the working area?  else: the register-pipe kernel
                     size_t work = 0, wst = 0; int slot = 0;
                     for (auto& ph : P.phases) {
-                        work = std::max(work, cc_mega_ring_smem_for_phase(ph, dev->sm_count));
+                        work = std::max(work, cc_mega_ring_layout(ph, dev->sm_count));
                         if (ph.type == MK_MATVEC && ph.act_type == CC_Q8_K && ph.x && ph.norm_w) wst = std::max(wst, (size_t)ph.n * 4);
                         if (ph.type == MK_MATVEC && ph.act_type != CC_Q8_K) slot = std::max(slot, cc_mega_ring_slot(ph.wtype));
                     }
@@ -860,7 +860,7 @@ static int cc_lazy_flush_part(cc_device* dev, bool whole) {
                 }
                 for (auto& ph : P.phases) {
                     if (P.mega_ring) {
-                        P.mega_smem = std::max(P.mega_smem, cc_mega_ring_smem_for_phase(ph, dev->sm_count));
+                        P.mega_smem = std::max(P.mega_smem, cc_mega_ring_layout(ph, dev->sm_count));
                         if (ph.type == MK_MATVEC && ph.act_type == CC_Q8_K && ph.x && ph.norm_w) P.mega_wstage = std::max(P.mega_wstage, (size_t)ph.n * 4);
                         if (ph.type == MK_MATVEC && ph.act_type != CC_Q8_K) P.ring_slot = std::max(P.ring_slot, cc_mega_ring_slot(ph.wtype));
                         if (ph.type == MK_ATTN) P.ring_at_ch = cc_mega_ring_at_ch(ph);

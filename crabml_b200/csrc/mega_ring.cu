@@ -71,7 +71,6 @@ __device__ __forceinline__ unsigned mr_ld_acquire_shared(unsigned addr) {
 // 75 items).  Producer and consumers derive the same item sequence from this: group P, segment s = item P * NSEG + s.
 struct MrGeo {
     int nb, GR, NSEG, n_rows, groups, first, last_half_off;
-    int most;              // virtual rows of the CTA that has the most: what is laid out in shared memory goes by it, in every CTA and on the host
     bool pair;
 };
 __device__ __forceinline__ MrGeo mr_geo(const StreamArgs& A) {
@@ -84,12 +83,10 @@ __device__ __forceinline__ MrGeo mr_geo(const StreamArgs& A) {
         const int rpc = (((m_cat + (int)gridDim.x - 1) / (int)gridDim.x) + 3) & ~3;
         g.first = (int)blockIdx.x * rpc;
         g.n_rows = min(rpc, max(0, m_cat - g.first));
-        g.most = rpc;
     } else {
         const int each = m_cat / (int)gridDim.x, more = m_cat - each * (int)gridDim.x;
         g.first = (int)blockIdx.x * each + min((int)blockIdx.x, more);
         g.n_rows = each + ((int)blockIdx.x < more ? 1 : 0);
-        g.most = (each + (more ? 1 : 0)) << (g.pair ? 1 : 0);
     }
     g.groups = ((g.n_rows + 1) >> 1) << (g.pair ? 1 : 0);
     g.last_half_off = 16 * (g.nb - 32 * (g.GR - 1));
@@ -415,14 +412,14 @@ __device__ __forceinline__ void mr_prologue(const MkPhase& ph, int k, int nbp, i
     }
 }
 
-// Lanes' sums are added up behind the row loop, all rows of the CTA at once, where they find room in shared memory.  One segment: a thread adds up a row's 32
-// (the butterfly took 320 of 1350 cycles a row).  Two to four segments (k <= 16384): warps keep to one segment, so that its activation stays in registers, and a
-// warp adds up a row's.  Else a warp takes a row's segments one after another, reads the activation for each and adds up itself.
-#define MR_PART_BYTES 30720
-__host__ __device__ __forceinline__ int mr_part_bytes(int nseg, int vrows) {
-    const int n = nseg == 1 ? vrows * 132 : nseg <= 4 ? vrows * nseg * 128 : 0;
-    return n <= MR_PART_BYTES ? n : 0;
-}
+// Lanes' sums are added up behind the row loop, all rows of the CTA at once, where they find room in shared memory (ph.ring_parts, decided by the host for all CTAs
+// alike).  One segment: a thread adds up a row's 32 (the butterfly took 320 of 1350 cycles a row).  Several: warps keep to one segment, so that its activation stays in
+// registers, and a warp adds up a row's.  Else a warp takes a row's segments one after another, reads the activation for each and adds up itself.
+// The room is taken from the ring.  30 KB are 232 rows of one segment (a vocabulary of 32000; one of 128256 comes at 7.3 TB/s all the same).  Rows of five segments and more
+// have 56 KB (8192 rows of eight): without it the ring holds the items of two or three pairs of rows, and as many pairs of warps work: 8192 x 28672 58.6 -> 45.2 us in
+// Q8_0, 42.7 -> 34.4 in Q4_0; four layers of 6144 x 20480 494 -> 476 and 423 -> 431 (five segments, eight pairs of warps).  86 KB (12288 x 32768) cost a
+// token of two such layers more than it gave, 680 -> 742.
+#define MR_PART_BYTES(nseg) ((nseg) > 4 ? 57344 : 30720)
 // shared memory of the phase: quants [nbp * 32] | f32 scales [nbp] | block sums [nbp] | reduction scratch 256 B | sums of the CTA's virtual rows | lanes' sums | fused prologue (over the sums): the row and its norm weights
 template <int TYPE>
 __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16_t* exp_lut, MrCons& RC, const CommDev& comm, unsigned xseq, unsigned long long* stamp1) {
@@ -438,7 +435,7 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
     float* s_red = (float*)(smem + (size_t)nbp * 40);
     float* s_sum = (float*)(smem + (size_t)nbp * 40 + 256);
     const int vrows = pair ? 2 * g.n_rows : g.n_rows;
-    float* s_part = s_sum + ((g.most + 31) & ~31);
+    float* s_part = s_sum + ph.ring_sums;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const StreamMats& M = A.mats;
     if (ph.x) {
@@ -474,7 +471,7 @@ __device__ void phase_matvec_ring(const MkPhase& ph, uint8_t* smem, const uint16
     const int* as_l = s_s + lane;
     // Warps 2 i and 2 i + 1 take the two rows of an item.  One warp on both rows held sixteen of the twenty slots at a time, so few copies were under way
     const int duo = warp >> 1, half = warp & 1;
-    const bool parts = mr_part_bytes(NSEG, g.most) > 0, split = parts && NSEG > 1;
+    const bool parts = ph.ring_parts != 0, split = parts && NSEG > 1;
     const int s0 = split ? duo % NSEG : 0, ns = split ? 1 : NSEG;
     const int P0 = split ? duo / NSEG : duo, dP = split ? (MK_WARPS / 2 - s0 + NSEG - 1) / NSEG : MK_WARPS / 2;
     constexpr unsigned DOFF = 2u * MK_SEG * (TYPE == CC_Q8_0 ? 1024u : 512u);
@@ -696,13 +693,15 @@ int cc_mega_ring_at_ch(const MkPhase& ph) {       // 48 KB of cache rows in flig
     if (env >= 8 && env <= 64) return env;
     return ph.at.kv_f16 ? 64 : 32;
 }
-size_t cc_mega_ring_smem_for_phase(const MkPhase& ph, int ctas) {
+size_t cc_mega_ring_layout(MkPhase& ph, int ctas) {
     if (ph.type == MK_MATVEC && ph.act_type == CC_Q8_K) return cc_mega_smem_for_phase(ph);
     if (ph.type == MK_MATVEC) {
         const size_t k = (size_t)ph.mv.k, nb = k / 32, GR = (nb + 31) / 32, NSEG = (GR + MK_SEG - 1) / MK_SEG, nbp = NSEG * MK_SEG * 32;
         const size_t m = ph.mv.epilogue == 2 ? (size_t)ph.mv.mats.m[0] : (size_t)ph.mv.mats.m[0] + (ph.mv.mats.n > 1 ? ph.mv.mats.m[1] : 0) + (ph.mv.mats.n > 2 ? ph.mv.mats.m[2] : 0);
-        const size_t rows = (m + (size_t)ctas - 1) / (size_t)ctas, most = ph.mv.epilogue == 2 ? 2 * rows : ph.mv.epilogue == 3 ? (rows + 3) & ~(size_t)3 : rows;      // mr_geo
-        const size_t sums = ((most + 31) & ~(size_t)31) * 4 + (size_t)mr_part_bytes((int)NSEG, (int)most);
+        const size_t rows = (m + (size_t)ctas - 1) / (size_t)ctas, most = ph.mv.epilogue == 2 ? 2 * rows : ph.mv.epilogue == 3 ? (rows + 3) & ~(size_t)3 : rows;      // the CTA with the most rows: mr_geo
+        const size_t own = ((most + 31) & ~(size_t)31) * 4, parts = NSEG == 1 ? most * 132 : most * NSEG * 128;
+        ph.ring_sums = (int)(own / 4); ph.ring_parts = NSEG <= MK_WARPS / 2 && parts <= MR_PART_BYTES(NSEG);
+        const size_t sums = own + (ph.ring_parts ? parts : 0);
         const size_t row = ph.x ? (k < MR_ROW_PIECE ? k : MR_ROW_PIECE) * 4 * (ph.norm_w ? 2 : 1) : 0;
         return nbp * 40 + 256 + (sums > row ? sums : row);
     }

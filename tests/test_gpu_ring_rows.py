@@ -1,5 +1,5 @@
 """The streaming phases of the ring kernel at the edges of their tiles: rows that do not divide by the CTAs or pair up, rows of one to several segments with
-ragged ends, rows longer than the prologue's staging area, and activations on which the quantiser's shortcuts do not hold.  A feed-forward block
+ragged ends, rows longer than the prologue's staging area, more rows than their lanes' sums find room for, and activations on which the quantiser's shortcuts do not hold.  A feed-forward block
 (norm, gate / up, silu * mul, down, residual) of the persistent kernel must equal the eager kernels bit for bit: both sum in one canonical order."""
 import numpy as np
 import pytest
@@ -42,7 +42,7 @@ def block(dev, wt, dim, hid, x, w):
 
 
 @pytest.mark.parametrize("wt", [oc.Q8_0, oc.Q4_0])
-@pytest.mark.parametrize("dim,hid", [(32, 32), (288, 768), (512, 4128), (4096, 12320), (4128, 2976), (12320, 160), (16448, 64)])
+@pytest.mark.parametrize("dim,hid", [(32, 32), (288, 768), (512, 4128), (4096, 12320), (4128, 2976), (12320, 160), (16448, 64), (320, 20000), (64, 24608), (32, 28672), (608, 29568), (96, 32768), (4128, 20000), (20512, 1216)])
 def test_feed_forward_block_equals_the_eager_kernels(wt, dim, hid):
     rng = np.random.default_rng(dim * 7 + hid + wt)
     w = {"gate": random_weight(wt, hid, dim, rng), "up": random_weight(wt, hid, dim, rng), "down": random_weight(wt, dim, hid, rng),

@@ -48,8 +48,8 @@ def producer_order(g):
 def consumer_walk(g):
     """phase_matvec_ring: for every pair of warps the list of (item index, [(unit, virtual row, segment)]) it consumes, in order."""
     walks, nseg, duos = [], g["nseg"], WARPS // 2
-    part_bytes = g["most"] * 132 if nseg == 1 else g["most"] * nseg * 128 if nseg <= 4 else 0
-    split = nseg > 1 and 0 < part_bytes <= 30720                       # warps keep to one segment
+    part_bytes = g["most"] * 132 if nseg == 1 else g["most"] * nseg * 128            # cc_mega_ring_layout
+    split = 1 < nseg <= duos and part_bytes <= (57344 if nseg > 4 else 30720)        # warps keep to one segment
     for duo in range(duos):
         s0, ns = (duo % nseg, 1) if split else (0, nseg)
         p0, dp = (duo // nseg, (duos - s0 + nseg - 1) // nseg) if split else (duo, duos)
@@ -66,7 +66,8 @@ SHAPES = [  # (rows per matrix, matrices, k, epilogue)
     (4096, 3, 4096, 0), (4096, 1, 4096, 1), (11008, 2, 4096, 2), (4096, 1, 11008, 1), (32000, 1, 4096, 0),      # Llama-2-7B, one GPU
     (4096, 1, 2048, 3), (4096, 1, 5504, 3), (16000, 1, 4096, 3),                                                    # shards at N = 2 (exchange phases)
     (512, 3, 4096, 0), (4096, 1, 512, 3), (1376, 2, 4096, 2), (4096, 1, 1376, 3), (4000, 1, 4096, 3),               # shards at N = 8
-    (4096, 1, 14336, 1), (8192, 1, 28672, 1), (256000, 1, 8192, 0),                                               # four segments, seven, and more rows than their sums find room for
+    (4096, 1, 14336, 1), (8192, 1, 28672, 1), (256000, 1, 8192, 0), (28672, 2, 8192, 2),                          # four segments, seven, and more rows than their sums find room for
+    (8192, 1, 18432, 1), (8192, 1, 24576, 1), (8192, 1, 29568, 1), (12288, 1, 32768, 1), (148, 1, 65536, 1),      # five, six, eight with room and without, sixteen
     (34386, 1, 4096, 0), (4440, 2, 14336, 2),                                                                      # CTAs on both sides of the room for lanes' sums
     (288, 3, 288, 0), (288, 1, 288, 1), (768, 2, 288, 2), (288, 1, 768, 1), (32000, 1, 288, 0),                     # tinyllamas-15M (ragged groups)
 ]
@@ -94,7 +95,7 @@ def test_producer_and_consumers_agree_on_the_ring_order(m, n_mats, k, epilogue):
 
 @pytest.mark.parametrize("m,n_mats,k,epilogue", SHAPES)
 def test_no_cta_has_more_rows_than_the_layout_in_shared_memory_allows(m, n_mats, k, epilogue):
-    """the layout (and whether lanes' sums have room) goes by the CTA with the most rows: the same in every CTA and on the host (cc_mega_ring_smem_for_phase)"""
+    """the host lays shared memory out (and decides whether lanes' sums have room) by the CTA with the most rows (cc_mega_ring_layout)"""
     geos = [geo(m, n_mats, k, epilogue, cta) for cta in range(GRID)]
     rows = -(-(m if epilogue == 2 else m * n_mats) // GRID)
     host = 2 * rows if epilogue == 2 else (rows + 3) & ~3 if epilogue == 3 else rows

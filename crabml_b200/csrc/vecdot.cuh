@@ -24,8 +24,12 @@ __device__ __forceinline__ int byte_of(unsigned w0, unsigned w1, int idx) { retu
 
 // cooperative global -> shared copy of `bytes` (multiple of 4) bytes.  The copies of a whole activation, of eight of them, are under way together: as loads and
 // stores each waited for the one before (in-order issue), 24 round trips to L2 in front of a product of 8 rows.  stage_wait, then a barrier, before it is read.
+// By way of L1 (.ca): up to eight CTAs of an SM read the same activation; past it each went to L2 for itself (Q4_K 4096 x 11008, a row: 12.2 us by loads, 16.2, now 10.3).
+// In loops that are not unrolled: the compiler takes other registers for the rows behind them (Q5_K 2048 x 28672, 31 rows 143 us by loads, 179 unrolled, now 143).
+// Of 918 products (12 types, 9 sizes, 1 to 31 rows) 68 had become more than 3 % slower than with loads, by up to 33 %; now 19, by up to 11 % but for one (Q8_0
+// 4096 x 4096, 5 rows: 15 or 18 us by how the CTAs fall).  In the mean they take 0.92 of the loads' time (0.94 past L1)
 __device__ __forceinline__ void stage_16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void stage_4(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -33,7 +37,9 @@ __device__ __forceinline__ void stage_4(void* dst, const void* src) {
 __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void stage(void* dst, const void* src, int bytes) {
     const int n16 = ((uintptr_t)src & 15) ? 0 : bytes >> 4;                     // batched activations: row bi may start 4-byte aligned only
+#pragma unroll 1
     for (int i = threadIdx.x; i < n16; i += blockDim.x) stage_16((int4*)dst + i, (const int4*)src + i);
+#pragma unroll 1
     for (int i = n16 * 4 + (int)threadIdx.x; i < (bytes >> 2); i += blockDim.x) stage_4((int*)dst + i, (const int*)src + i);
 }
 __host__ __device__ inline int al16i(int v) { return (v + 15) & ~15; }
@@ -249,6 +255,7 @@ struct TKBase {
         const uint8_t* p = (const uint8_t*)scratch;
         int64_t o1 = (n_total + 15) & ~15ll, o2 = o1 + ((n_total / 256 * 4 + 15) & ~15ll);
         const int4* q = (const int4*)(p + (int64_t)bi * k);
+#pragma unroll 1
         for (int i = threadIdx.x; i < (k >> 4); i += blockDim.x) stage_16((int4*)sm + T::act_at(i), q + i);
         stage(sm + al16i(k), p + o1 + (int64_t)bi * (k / 256) * 4, k / 256 * 4);
         stage(sm + al16i(k) + al16i(k / 256 * 4), p + o2 + (int64_t)bi * (k / 16) * 2, k / 16 * 2);

@@ -102,7 +102,7 @@ LazyState* cc_lazy_create(cc_device* dev) {
     for (int i = 0; i < LZ_DYN_SLOTS; i++)
         if (cudaMallocHost(&lz->dyn_host[i], lz->dyn_cap) != cudaSuccess || cudaEventCreateWithFlags(&lz->dyn_ev[i], cudaEventDisableTiming) != cudaSuccess) { delete lz; return nullptr; }
     if (cudaMalloc(&lz->dyn_dev, lz->dyn_cap) != cudaSuccess) { delete lz; return nullptr; }
-    if (getenv("CRABML_MEGA_PROF") && cudaMalloc(&lz->prof_dev, 8 * 8 * 4097) == cudaSuccess) cudaMemset(lz->prof_dev, 0, 8 * 8 * 4097);     // (the ring kernel stamps phases only)
+    if (getenv("CRABML_MEGA_PROF")) cudaMalloc(&lz->prof_dev, 8 * 8 * 4097);
     if (cudaMalloc(&lz->bar_dev, 4096) != cudaSuccess || cudaMemset(lz->bar_dev, 0, 4096) != cudaSuccess) { delete lz; return nullptr; }
     return lz;
 }

@@ -73,8 +73,9 @@ static int launch_few(cc_device* dev, const WPlanes& W, const void* act, int64_t
 // butterfly the lanes; here warp q of four has the super-blocks q, q + 4, .. of the 16 rows and a sum for each of the 8 chunks, and the four warps' sums are
 // added up in shared memory in the butterfly's order: identical bits.  A lane holds the weights of two rows at 4 columns of a chunk; activations come by ldmatrix.
 // A warp copies its super-blocks (16 rows x 144 B, which lie in memory as in shared memory) four ahead by cp.async (two, where activations of 67 to 73 super-blocks leave no
-// more room); rows of 144 B put the words of eight rows in different banks.  One CTA of two groups of four warps an SM: bound by the instructions, the mma among
-// them, and more warps only stage later (two CTAs an SM 11008 x 4096 x 8 25.1 us, CTAs of 3 / 4 / 5 groups 24.0 / 27.1 / 21.8).
+// more room); rows of 144 B put the words of eight rows in different banks.  One CTA of two groups of four warps an SM.  Half of the
+// issue slots are busy (51 %: 707 warp instructions per 16 rows and super-block, the mma among them, two warps a scheduler), the rest are their latencies; more warps only
+// stage later (two CTAs an SM 11008 x 4096 x 8 25.1 us, CTAs of 3 / 4 / 5 groups 24.0 / 27.1 / 21.8).
 // us with the quantisation of the rows, 11008 x 4096 x 8 / 16 / 31 rows: two weight rows a warp by dp4a 31.4 / 44.1 / 74.2 ; weights by 4-byte loads one super-block ahead and activations
 // staged one after another 28.0 / 37.3 / 54.3 ; here 18.8 / 28 / 49.5 ; 32000 x 4096 48 / 72 / 128, now 37 / 67 / 128 ; 4096 x 4096 x 8 17.7, now 10.4.  Q6_K the same
 // way: 31.6 by dp4a, 43.4 (its numbers take twice the instructions to put together).

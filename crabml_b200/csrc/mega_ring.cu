@@ -8,16 +8,18 @@
 //     of items -- two rows' segment of 128 blocks: 8192 B of Q8_0 quants + 512 B of f16 scales (1024 B are theirs) -- into a ring of shared-memory slots, as many as fit beside
 //     the per-phase working area (17 to 19 = 160-174 KB per SM, 25 MB per GPU).  They never wait for a barrier or an activation: whenever a slot is free the
 //     next item of this CTA's rows -- of this phase or any later one -- is being fetched.
-//   * warp 19 asks L2 for the items behind the ring, up to 224 KB of them per SM (33 MB per GPU), at 20 B per cycle and SM: a full ring is 4 us of HBM time, the
-//     time between one phase's last row and the next one's first 5 to 7 us, the attention phase 7.  A 7B Q8_0 token 1862 -> 1814 us (120 KB 1830; 224 and 300 KB, 20
-//     and 26 B alike; 417 KB = 62 MB per GPU was 30 % slower: more than L2 holds of it).  Without a pace the requests queue in front of the barrier's own
-//     traffic: with 19 MB under way a barrier takes 20 us instead of 2 (measured by itself; at 6.3 TB/s with 7 MB under way 3.4).
+//   * warp 19 asks L2 for the items behind the ring: it is ahead of the copies by a ring's size and 224 KB (390 KB per SM, 58 MB per GPU) at most, at 20 B per cycle and
+//     SM: a full ring is 4 us of HBM time, the time between one phase's last row and the next one's first 5 to 7 us, the attention phase 7.  A 7B Q8_0 token 1862 ->
+//     1814 us (with 120 KB instead of the 224 1830; 224 and 300 KB, 20 and 26 B alike; 417 KB, 86 MB per GPU with the ring's size, was 30 % slower: more than L2 keeps).
+//     Lead and pace count every item as a full one: items of rows of 288 are charged 14 times their bytes, the copies overtake the requests, and short rows come by the
+//     ring alone.  Without a pace the requests queue in front of the barrier's own traffic: with 19 MB under way a barrier takes 20 us instead of 2 (measured by
+//     itself; at 6.3 TB/s with 7 MB under way 3.4).
 //   * warps 0-15 are CONSUMERS: the CTA's rows are one contiguous run, two neighbouring rows an item, a warp each; same per-lane block order, same arithmetic as
 //     mega.cu / matvec_stream.cu (bit-identical results), but a segment is read from the ring with LDS.128 after waiting on the slot's "full" mbarrier, and
 //     the slot is handed back through its "done" words.  The activation stays in registers, lanes' sums are added up behind the row loop.  (One warp on both
 //     rows of an item, activation from shared memory: 16 of the 19 slots were being read and only the others under way, 1950 us a token; now 1814.)
-//     96 registers a thread are enough, but nothing may spill: a spilled register is a trip to L2, the ring leaves no L1 (the same rows with a prologue that
-//     kept its row in registers, 600 bytes of spills: 2540 us).
+//     96 registers a thread are enough, and next to nothing may spill (4 bytes do, 84 where the K-quant phases are compiled in): a spilled register is a trip to L2,
+//     the ring leaves no L1 (the same rows with a prologue that kept its row in registers, 600 bytes of spills: 2540 us).
 // The 512 compute threads synchronise on named barrier 1 (MK_SYNC); the producer warps never join it.
 // 20 warps: five per SM sub-partition, so its 16384 registers allow 96 per thread (what __launch_bounds__(640, 1) yields).
 #define MK_SYNC() asm volatile("bar.sync 1, 512;" ::: "memory")
@@ -27,7 +29,7 @@
 
 #define MR_PRODUCER_WARPS 4        // 20 warps: five per SM sub-partition, still 96 registers per thread
 #define MR_ISSUERS 96                // threads that issue copies: three warps (two: +1 %); the fourth warp prefetches
-#define MR_L2_LEAD (224 * 1024)       // bytes of items asked into L2 behind the ring, per SM
+#define MR_L2_LEAD (224 * 1024)       // bytes of items, beside a ring's size, that the requests to L2 are ahead of the copies, per SM
 #define MR_L2_RATE 20                 // bytes per cycle and SM at which they are asked for: 5.8 TB/s
 #define MR_THREADS (MK_THREADS + 32 * MR_PRODUCER_WARPS)
 #define MR_MAX_SLOTS 56
@@ -48,11 +50,6 @@ __device__ __forceinline__ void mr_bulk_g2s(unsigned dst, const void* src, unsig
 __device__ __forceinline__ bool mr_try_wait(unsigned bar, unsigned parity) {
     unsigned ok;
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mr_test_wait(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
 // Slot hand-back: the consumer stores (item number + 1) into the slot's "done" word (release), the producer polls it (acquire) for
@@ -105,7 +102,8 @@ __device__ __forceinline__ int mr_locate(const StreamMats& M, int rc, int& mat) 
 // where item j of a phase comes from: quants and scales of its two rows (two = false: one row, or two rows of one matrix next to each other as one run)
 struct MrItem { const uint8_t* q[2]; const uint16_t* d[2]; unsigned qbytes, dbytes, dspan; bool two; };       // dspan: both rows' scales as one copy, what lies between them included (0: a copy each)
 // Where the second row's scales lie behind the first's: beside them, or, where Q8_0 rows are longer than a segment and both fit, as far as in the plane: one copy of
-// both and of what lies between them, an item in three copies (11008 x 4096: 14.3 -> 14.0 us, a token 1806 -> 1777; Q4_0 waits for its consumers, larger slots only cost it 0.7 %)
+// both and of what lies between them, an item in three copies (11008 x 4096: 14.3 -> 14.0 us, a token 1806 -> 1777; Q4_0 waits for its consumers, larger slots only cost it 0.7 %).
+// Slots with room for rows of 14336 too (1152 B) give nothing: four layers of 4096 x 14336 340 -> 342 us, of 5120 x 13824 394 -> 395, 24 of 8192 x 28672 4012 -> 3983
 #define MR_SCALES 1024
 __device__ __forceinline__ unsigned mr_scale_off(const MrGeo& g, unsigned BB, unsigned dbytes) {
     const unsigned row = 2u * CC_D_STRIDE(g.nb);

@@ -137,7 +137,9 @@ __global__ void scale_kernel(float* x, int64_t n, float s) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = x[i] * s;
 }
-// 16 bytes a thread: [32, 512, 128] 10.6 us by single numbers, 5.1
+// 16 bytes a thread: [32, 512, 128] 10.6 us by single numbers, 5.1.  Call after call it takes 1.05 million numbers 4.6 and 3.9 us; below that a call waits for the
+// host, whose launch of this kernel takes 0.4 us longer (512 numbers 3.8 and 4.3 us), so a decoded token's few thousand go by single numbers
+#define SCALE4_FROM ((int64_t)1 << 19)
 __global__ void __launch_bounds__(256) scale4_kernel(float4* x, unsigned n4, float s) {
     pdl_enter();
     const unsigned i = blockIdx.x * 256u + threadIdx.x;
@@ -147,7 +149,7 @@ __global__ void __launch_bounds__(256) scale4_kernel(float4* x, unsigned n4, flo
 }
 int cc_launch_scale(cc_device* dev, float* x, int64_t n, float s) {     // cpu_tensor.rs:404-410
     if (n == 0) return CC_OK;
-    if (n % 4 == 0 && n < ((int64_t)1 << 32) && ((uintptr_t)x & 15) == 0) {
+    if (n >= SCALE4_FROM && n % 4 == 0 && n < ((int64_t)1 << 32) && ((uintptr_t)x & 15) == 0) {
         cc_launch_pdl(dev, scale4_kernel, (unsigned)((n / 4 + 255) / 256), 256, 0, (float4*)x, (unsigned)(n / 4), s);
         CC_LAUNCH_CHECK(dev);
         return CC_OK;

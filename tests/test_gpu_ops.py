@@ -256,3 +256,16 @@ def test_activation_quantize_bit_exact(gdev, act):
     if act == oc.Q8_1:       # zero block: reference gives qs=-128 with d=0 (B2); compare everything
         pass
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1, 510, (1 << 19) - 4, (1 << 19) - 1, 1 << 19, (1 << 19) + 2, (1 << 19) + 4, (1 << 20) + 256])
+def test_scale_by_single_numbers_and_by_sixteen_bytes(n):
+    """both sides of the size from which a thread takes four numbers, and sizes that are no multiple of four: a product each, so the bits are numpy's"""
+    from crabml_b200 import CudaTensor
+    dev = make_device()
+    try:
+        x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
+        got = CudaTensor.new(x, [n], dev).scale_inplace(0.0883883461).export()
+        np.testing.assert_array_equal(got.view(np.uint32), (x * np.float32(0.0883883461)).view(np.uint32))
+    finally:
+        dev.close()

@@ -46,7 +46,9 @@ struct GraphEntry { cudaGraphExec_t exec = nullptr; size_t dyn_bytes = 0; uint64
 #define LZ_FIRST_OPS 30                              // the first part of a token: more than a layer, work for the GPU until the next part is recorded and fused
 #define LZ_PART_GROWTH 5                             // and each part so much longer than the one before: an op of a 7B layer keeps the GPU for 2.2 us and the host for
                                                      // 0.25.  16 tokens with first / growth 64 / 4, 40 / 4, 30 / 5, 22 / 6, ms: 7B 30.6 / 30.5 / 30.4 / 30.7 (two parts, before: 3 ms more), four 7B
-                                                     // layers of K-quants 7.39 / 7.19 / 7.18 / 6.97, 15M 4.23 / 4.34 / 4.32 / 4.61 (its kernels are short: a third part costs it more than it hides)
+                                                     // layers of K-quants 7.39 / 7.19 / 7.18 / 6.97, 15M 4.23 / 4.34 / 4.32 / 4.61 (its kernels are short: a third part costs it more than it hides).
+                                                     // Mode 1, a token with its read-back, one part of 64 and the rest / 64 / 4 / 30 / 5, us: 15M 242 / 242 / 252, 8 layers of 2048 x 5632 367 / 367 / 384,
+                                                     // 12 of 288 x 768 457 / 457 / 421, 16 of 1024 x 2816 613 / 585 / 551, 40 of 512 x 1536 1397 / 1208 / 1270
 
 struct LazyState {
     std::vector<LOp> q;

@@ -58,8 +58,8 @@ WORKLOADS = {
     "vadodra-w2048": ("VADODRA", "BF16", "BF16"),
     "vadodra-w4096": ("VADODRA", "BF16", "BF16"),
 }
-# dram bytes per megakernel launch from the committed ncu --set full capture (profiles/); None until captured
-TRAFFIC = {("llama2-7b-q8_0", 1): 7040893000 + 49879296}     # profiles/r02p_mega_ring_q8_0_ncu_summary.txt (mega_ring_kernel: dram__bytes_read.sum + dram__bytes_write.sum)
+# dram bytes of a token's persistent launches from the committed ncu capture (profiles/); None until captured
+TRAFFIC = {("llama2-7b-q8_0", 1): 7035444480 + 21546496}     # profiles/ring_phases.txt (mega_ring_kernel, three launches: dram__bytes_read.sum + dram__bytes_write.sum)
 MEGA_NAMES = {1: ("mega_kernel", "mega.cu, weights through registers"), 2: ("mega_ring_kernel", "mega_ring.cu, weights through a TMA-fed shared-memory ring")}
 TYPE_ID = {"Q4_0": 2, "Q4_1": 3, "Q5_0": 6, "Q5_1": 7, "Q8_0": 8, "Q2_K": 10, "Q3_K": 11, "Q4_K": 12, "Q5_K": 13, "Q6_K": 14}
 
@@ -414,7 +414,7 @@ def run_b200(args, rank, world, local_rank):
             traffic = TRAFFIC.get((args.workload, world))
             roofline = {"bound": "hbm", "kernel": f"{mk_name} ({mk_file}): {parts:g} persistent launch(es) per decoded token, all matvec/attention/norm phases",
                         "achieved": mega_gbs, "peak": peaks["hbm_gbs"], "peak_source": peak_src, "unit": "GB/s", "frac": mega_gbs / peaks["hbm_gbs"],
-                        "traffic": traffic / parts if traffic else None, "traffic_source": "profiles/ (dram__bytes_read.sum + dram__bytes_write.sum of a token in one launch, shared evenly by its launches)" if traffic else None,
+                        "traffic": traffic / parts if traffic else None, "traffic_source": "profiles/ (dram__bytes_read.sum + dram__bytes_write.sum of a token, shared evenly by its launches)" if traffic else None,
                         "algorithmic_bytes_per_launch": bytes_per_token / parts, "us_per_launch": val_ms / K * 1e3 / parts, "frac_of_8TBs_nominal": mega_gbs / 8000.0}
         else:
             roofline = {"bound": "hbm", "kernel": f"matvec_stream_kernel<{wt_name}> {m}x{k} (+ activation quantize: {launches_per_mv:.0f} launches per matmul_vec)",

@@ -86,3 +86,37 @@ def test_prefill_small_batches_keep_the_exact_block_path(gdev):
     """b below the dense threshold still takes the per-row quantised dot (1e-6 * sum|terms| parity, test_gpu_matvec.py)"""
     from tests.test_gpu_matvec import run_case
     run_case(gdev, oc.Q8_0, 33, 1024, b=3, seed=301)
+
+
+@pytest.mark.parametrize("b,k", [(32, 64), (33, 320), (257, 1088)])
+@pytest.mark.parametrize("kind", ["plain", "whole quotients", "beside whole quotients", "zeros and extremes", "tiny", "no numbers"])
+def test_operand_of_plain_rows_has_the_bits_of_a_division(gdev, kind, b, k):
+    """Against the unit matrix the dense product returns its operand, f16(q * f16(d)), with d = max|x| / 127 and q = trunc(x / d): also where the quantiser's
+    multiplications do not stand for the divisions, and in the last, ragged CTA of rows."""
+    from crabml_b200 import CudaTensor
+    rng = np.random.default_rng(b + k)
+    x = rng.standard_normal((b, k)).astype(np.float32)
+    if "whole" in kind:                                   # every number a whole multiple of its block's step, or the float next to one
+        x = rng.integers(-127, 128, (b, k)).astype(np.float32) * np.float32(0.37)
+        x[:, ::32] = np.float32(127) * np.float32(0.37)
+        if "beside" in kind:
+            x[:, 1::2] = np.nextafter(x[:, 1::2], np.where(rng.random(x[:, 1::2].shape) < 0.5, -1e9, 1e9).astype(np.float32))
+    elif kind == "zeros and extremes":
+        x[:, :32] = 0
+        x[:, 32::3] *= np.float32(1e-30)
+        x[:, k - 1] = 3e4
+    elif kind == "tiny":
+        x *= np.float32(1e-39)
+    elif kind == "no numbers":
+        x[:, ::7] = np.nan
+    raw = np.zeros((k, k // 32, 34), np.uint8)            # Q8_0 blocks of the unit matrix: d = 1, a single 1
+    raw[:, :, :2] = np.frombuffer(np.float16(1).tobytes(), np.uint8)
+    raw[np.arange(k), np.arange(k) // 32, 2 + np.arange(k) % 32] = 1
+    got = CudaTensor.from_cpu(raw.reshape(-1), [k, k], oc.Q8_0, gdev).matmul_vec(CudaTensor.new(x.reshape(-1), [b, k], gdev)).export().reshape(b, k)
+    blk = x.reshape(b, k // 32, 32)
+    with np.errstate(all="ignore"):
+        d = np.nanmax(np.abs(blk), axis=2, keepdims=True) / np.float32(127)
+        q = np.trunc(blk / d)
+        q = np.where(np.isnan(q), np.float32(0), q)
+        want = (q * d.astype(np.float16).astype(np.float32)).astype(np.float16).astype(np.float32).reshape(b, k)
+    np.testing.assert_array_equal(got, want)
